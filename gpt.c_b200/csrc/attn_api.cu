@@ -261,7 +261,7 @@ int attn_sm100_backward(const void *saved, const float *out, const float *lse, c
         e = attn::launch_fast_backward(map_x, map_do, map_dx, lse, delta, dqkv, B, T, H, ds->num_sms, sched, ds->status, s);
     } else {
         if (prepare) {
-            e = attn::launch_bwd_prepare(dout, out, delta, nullptr, nullptr, nullptr, nullptr, B, T, H, D, s);
+            e = attn::launch_bwd_prepare(dout, out, delta, nullptr, nullptr, dqkv, nullptr, B, T, H, D, s);
             if (e != cudaSuccess) return (int)e;
         }
         if (!core) return ATTN_OK;

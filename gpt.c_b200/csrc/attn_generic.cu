@@ -1,4 +1,4 @@
-// General-shape causal attention kernels (fp32 SIMT, one warp per row) and the elementwise
+// General-shape causal attention kernels (fp32 SIMT, tiled) and the elementwise
 // preparation kernels shared with the tensor-core path.
 //
 // These kernels accept any head size D <= 256 and any T <= 8192.  They are the correctness
@@ -14,28 +14,11 @@ namespace {
 
 constexpr int kWarp = 32;
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-
-// Element accessors: plain fp32, or the sum of the two bf16 planes written by the split kernel.
-struct XF32 {
-    const float *p;
-    __device__ __forceinline__ float at(size_t i) const { return __ldg(p + i); }
-};
-struct XSplit {
-    const __nv_bfloat16 *hi, *lo;
-    __device__ __forceinline__ float at(size_t i) const {
-        return __bfloat162float(hi[i]) + __bfloat162float(lo[i]);
-    }
-};
 
 // ---------------------------------------------------------------------------------------
 // split: x -> hi, lo
@@ -72,14 +55,14 @@ __global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ x,
 }
 
 // ---------------------------------------------------------------------------------------
-// backward preparation: delta[b,h,t] = sum_d dout*out, optional split of dout, optional
-// zero-fill of the dq third of dqkv (the tensor-core backward accumulates dq with atomics).
-// One warp per (b, t, h): D elements.
+// backward preparation for the general kernels: delta[b,h,t] = sum_d dout*out, and zero-fill of the
+// dq third of dqkv (the backward accumulates dq with atomics).  One warp per (b, t, h): D elements.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) bwd_prepare_kernel(const float *__restrict__ dout, const float *__restrict__ out,
-                                                           float *__restrict__ delta, __nv_bfloat16 *__restrict__ dhi,
-                                                           __nv_bfloat16 *__restrict__ dlo, float *__restrict__ dq_zero,
+                                                           float *__restrict__ delta, float *__restrict__ dq_zero,
                                                            int B, int T, int H, int D) {
+    tc05::pdl_launch_dependents();
+    tc05::pdl_wait();
     const int lane = threadIdx.x & 31;
     const size_t nrows = (size_t)B * T * H;
     const size_t wstride = (size_t)gridDim.x * (blockDim.x >> 5);
@@ -94,12 +77,7 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const float *__restric
         for (int d = lane; d < D; d += kWarp) {
             const float g = dout[base + d];
             acc += g * out[base + d];
-            if (dhi) {
-                const __nv_bfloat16 hh = __float2bfloat16_rn(g);
-                dhi[base + d] = hh;
-                dlo[base + d] = __float2bfloat16_rn(g - __bfloat162float(hh));
-            }
-            if (dq_zero) dq_zero[bt * 3 * C + (size_t)h * D + d] = 0.f;
+            dq_zero[bt * 3 * C + (size_t)h * D + d] = 0.f;
         }
         acc = warp_sum(acc);
         if (lane == 0) delta[((size_t)b * H + h) * T + t] = acc;
@@ -159,178 +137,549 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
 }
 
 // ---------------------------------------------------------------------------------------
-// generic forward: one warp per query row (b, h, i)
-// shared memory per warp: T scores + D query values
+// General kernels: causal attention in fp32 for any head size, tiled over queries and keys.
+//
+// What bounds them is the fp32 pipe, so they are built around register tiles: a thread owns kR rows and
+// several columns of every product and reads its operands from shared memory in 16-byte words, 16 packed
+// multiply-adds (fma.rn.f32x2) for each such word of a score tile and 6 for each word of an output tile.
+// A warp covers 4 row groups x 8 column groups, which lets the 8 (or 4) lanes that want the same word get
+// it in one access; rows are padded to an odd number of 16-byte words, so 8 rows in a column do not collide.
+//   score products (contraction over the head size, contiguous in both operands): the two halves of a packed
+//     accumulator hold the sums over even and odd head columns, added once at the end;
+//   output products (contraction over keys or queries): they hold two neighbouring head columns, the other
+//     operand is broadcast into both halves.
+// kNI = head columns in blocks of 32 (the output tile's width), so D = 80 does 96 columns of output work; the
+// score products run over exactly the 4-column words that hold data.
+// The kernels they replace (one warp per row, K and V read again from L2 for every row) took 83 ms for forward
+// and backward of B=4 T=1024 H=6 D=128; these take 0.74 ms (23 GFLOP of fp32 products, a third of the fp32 rate
+// of 148 SMs).
 // ---------------------------------------------------------------------------------------
-template <class X>
-__global__ void __launch_bounds__(128) generic_fwd_kernel(X x, float *__restrict__ out, float *__restrict__ out_copy,
-                                                           float *__restrict__ lse, int B, int T, int H, int D,
-                                                           float scale) {
-    extern __shared__ float sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nw = blockDim.x >> 5;
-    const size_t row = (size_t)blockIdx.x * nw + warp;
-    if (row >= (size_t)B * H * T) return;
-    // longest rows first inside each (b, h)
-    const int i = T - 1 - (int)(row % T);
-    const size_t bh = row / T;
-    const int h = (int)(bh % H), b = (int)(bh / H);
-    const int C = H * D, C3 = 3 * C;
-    float *s = sm + (size_t)warp * (T + D);
-    float *q = s + T;
-    const size_t base = (size_t)b * T * C3;
+typedef unsigned long long f32x2;  // two floats of a packed instruction
 
-    for (int d = lane; d < D; d += kWarp) q[d] = x.at(base + (size_t)i * C3 + (size_t)h * D + d);
-    __syncwarp();
-
-    float m = -INFINITY;
-    for (int j = lane; j <= i; j += kWarp) {
-        const size_t kp = base + (size_t)j * C3 + C + (size_t)h * D;
-        float acc = 0.f;
-        for (int d = 0; d < D; d++) acc = fmaf(q[d], x.at(kp + d), acc);
-        acc *= scale;
-        s[j] = acc;
-        m = fmaxf(m, acc);
-    }
-    m = warp_max(m);
-    float l = 0.f;
-    for (int j = lane; j <= i; j += kWarp) {
-        const float e = expf(s[j] - m);
-        s[j] = e;
-        l += e;
-    }
-    l = warp_sum(l);
-    __syncwarp();
-    const float inv = 1.0f / l;
-    for (int d = lane; d < D; d += kWarp) {
-        const size_t vp = base + 2 * (size_t)C + (size_t)h * D + d;
-        float acc = 0.f;
-        for (int j = 0; j <= i; j++) acc = fmaf(s[j], x.at(vp + (size_t)j * C3), acc);
-        const size_t op = ((size_t)b * T + i) * C + (size_t)h * D + d;
-        const float o = acc * inv;
-        out[op] = o;
-        if (out_copy) out_copy[op] = o;
-    }
-    if (lane == 0) lse[bh * T + i] = m + logf(l);
+__device__ __forceinline__ f32x2 fma_x2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
 }
+__device__ __forceinline__ f32x2 mul_x2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 both(float v) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+    return d;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ ulonglong2 lds_x4(const float *p) { return *reinterpret_cast<const ulonglong2 *>(p); }
 
-// ---------------------------------------------------------------------------------------
-// generic backward, part 1: one warp per query row -> dq
-// shared memory per warp: T values of dS + D (q) + D (dout row)
-// ---------------------------------------------------------------------------------------
-template <class X>
-__global__ void __launch_bounds__(128) generic_bwd_dq_kernel(X x, const float *__restrict__ lse,
-                                                              const float *__restrict__ delta,
-                                                              const float *__restrict__ dout, float *__restrict__ dqkv,
-                                                              int B, int T, int H, int D, float scale) {
-    extern __shared__ float sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nw = blockDim.x >> 5;
-    const size_t row = (size_t)blockIdx.x * nw + warp;
-    if (row >= (size_t)B * H * T) return;
-    const int i = T - 1 - (int)(row % T);
-    const size_t bh = row / T;
-    const int h = (int)(bh % H), b = (int)(bh / H);
-    const int C = H * D, C3 = 3 * C;
-    float *ds = sm + (size_t)warp * (T + 2 * D);
-    float *q = ds + T;
-    float *g = q + D;
-    const size_t base = (size_t)b * T * C3;
-    for (int d = lane; d < D; d += kWarp) {
-        q[d] = x.at(base + (size_t)i * C3 + (size_t)h * D + d);
-        g[d] = dout[((size_t)b * T + i) * C + (size_t)h * D + d];
-    }
-    __syncwarp();
-    const float lse_i = lse[bh * T + i], delta_i = delta[bh * T + i];
-    for (int j = lane; j <= i; j += kWarp) {
-        const size_t kp = base + (size_t)j * C3 + C + (size_t)h * D;
-        const size_t vp = kp + C;
-        float sacc = 0.f, dp = 0.f;
-        for (int d = 0; d < D; d++) {
-            sacc = fmaf(q[d], x.at(kp + d), sacc);
-            dp = fmaf(g[d], x.at(vp + d), dp);
+// Row pitch of a tile in shared memory, in floats: wide enough for the output product's columns, an odd number
+// of 16-byte words.
+template <int kNI>
+struct Pitch {
+    static constexpr int value = 32 * kNI + 4;
+};
+
+// Rows r0 .. r0+kRows-1 of one head (D columns starting at src, rows `stride` apart) into a shared-memory tile, by
+// asynchronous copies; rows at or past `rows` and the columns that fill the last 16-byte word become zeros.
+template <int kRows, int kPitch, int kThreads, bool kVec>
+__device__ __forceinline__ void load_rows_async(float *tile, const float *src, size_t stride, int r0, int rows, int D) {
+    const int words = (D + 3) >> 2;
+    for (int r = threadIdx.x >> 3; r < kRows; r += kThreads / 8) {
+        const bool in = r0 + r < rows;
+        const float *row = src + (size_t)(in ? r0 + r : 0) * stride;
+        const uint32_t dst = tc05::smem_u32(tile + r * kPitch);
+        for (int w = threadIdx.x & 7; w < words; w += 8) {
+            if (kVec) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16 * w), "l"(row + 4 * w),
+                             "r"(in ? 16 : 0)
+                             : "memory");
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int c = 4 * w + e;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * c),
+                                 "l"(row + (c < D ? c : 0)), "r"(in && c < D ? 4 : 0)
+                                 : "memory");
+                }
+            }
         }
-        const float p = expf(sacc * scale - lse_i);
-        ds[j] = p * (dp - delta_i);
     }
-    __syncwarp();
-    for (int d = lane; d < D; d += kWarp) {
-        const size_t kp = base + C + (size_t)h * D + d;
-        float acc = 0.f;
-        for (int j = 0; j <= i; j++) acc = fmaf(ds[j], x.at(kp + (size_t)j * C3), acc);
-        dqkv[base + (size_t)i * C3 + (size_t)h * D + d] = acc * scale;
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
+// The same for rows held as two bf16 planes: the sum of the two is stored.
+template <int kRows, int kPitch, int kThreads, bool kVec>
+__device__ __forceinline__ void load_rows_split(float *tile, const __nv_bfloat16 *hi, const __nv_bfloat16 *lo, size_t stride,
+                                                int r0, int rows, int D) {
+    const int words = (D + 3) >> 2;
+#pragma unroll 2
+    for (int r = threadIdx.x >> 3; r < kRows; r += kThreads / 8) {
+        const bool in = r0 + r < rows;
+        const size_t at = (size_t)(in ? r0 + r : 0) * stride;
+#pragma unroll 2
+        for (int w = threadIdx.x & 7; w < words; w += 8) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in) {
+                if (kVec) {
+                    const uint2 h = __ldg(reinterpret_cast<const uint2 *>(hi + at) + w);
+                    const uint2 l = __ldg(reinterpret_cast<const uint2 *>(lo + at) + w);
+                    v.x = __uint_as_float(h.x << 16) + __uint_as_float(l.x << 16);
+                    v.y = __uint_as_float(h.x & 0xffff0000u) + __uint_as_float(l.x & 0xffff0000u);
+                    v.z = __uint_as_float(h.y << 16) + __uint_as_float(l.y << 16);
+                    v.w = __uint_as_float(h.y & 0xffff0000u) + __uint_as_float(l.y & 0xffff0000u);
+                } else {
+                    float f[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int c = 4 * w + e;
+                        f[e] = c < D ? __bfloat162float(hi[at + c]) + __bfloat162float(lo[at + c]) : 0.f;
+                    }
+                    v = make_float4(f[0], f[1], f[2], f[3]);
+                }
+            }
+            *reinterpret_cast<float4 *>(tile + r * kPitch + 4 * w) = v;
+        }
+    }
+}
+
+// acc[r][c] += rows a0 + 4 r of A (pitch floats apart) times rows b0 + 8 c of B, over `words` 4-column words.
+template <int kR, int kC, int kPitch>
+__device__ __forceinline__ void score_product(f32x2 (&acc)[kR][kC], const float *a0, const float *b0, int words) {
+#pragma unroll
+    for (int r = 0; r < kR; r++)
+#pragma unroll
+        for (int c = 0; c < kC; c++) acc[r][c] = 0ull;
+#pragma unroll 2
+    for (int w = 0; w < words; w++) {
+        ulonglong2 a[kR], b[kC];
+#pragma unroll
+        for (int r = 0; r < kR; r++) a[r] = lds_x4(a0 + 4 * r * kPitch + 4 * w);
+#pragma unroll
+        for (int c = 0; c < kC; c++) b[c] = lds_x4(b0 + 8 * c * kPitch + 4 * w);
+#pragma unroll
+        for (int r = 0; r < kR; r++)
+#pragma unroll
+            for (int c = 0; c < kC; c++) {
+                acc[r][c] = fma_x2(a[r].x, b[c].x, acc[r][c]);
+                acc[r][c] = fma_x2(a[r].y, b[c].y, acc[r][c]);
+            }
+    }
+}
+__device__ __forceinline__ float total(f32x2 v) {
+    const float2 h = halves(v);
+    return h.x + h.y;
+}
+
+template <bool kVec>
+__device__ __forceinline__ void store_cols(float *row, int col, int D, float4 v) {
+    if (kVec) {
+        if (col < D) *reinterpret_cast<float4 *>(row + col) = v;  // D is a multiple of 4
+    } else {
+        if (col < D) row[col] = v.x;
+        if (col + 1 < D) row[col + 1] = v.y;
+        if (col + 2 < D) row[col + 2] = v.z;
+        if (col + 3 < D) row[col + 3] = v.w;
     }
 }
 
 // ---------------------------------------------------------------------------------------
-// generic backward, part 2: one warp per key row -> dk, dv
-// shared memory per warp: (T p values) + (T dS values) + D (k) + D (v)
+// forward: one block per (b, h, 64 queries), key tiles of 8 kC, online softmax.  4 warps: two blocks share an SM
+// (100 KB of shared memory each at D = 128) and cover each other's loads.
 // ---------------------------------------------------------------------------------------
-template <class X>
-__global__ void __launch_bounds__(128) generic_bwd_dkv_kernel(X x, const float *__restrict__ lse,
-                                                               const float *__restrict__ delta,
-                                                               const float *__restrict__ dout, float *__restrict__ dqkv,
-                                                               int B, int T, int H, int D, float scale) {
-    extern __shared__ float sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nw = blockDim.x >> 5;
-    const size_t row = (size_t)blockIdx.x * nw + warp;
-    if (row >= (size_t)B * H * T) return;
-    const int j = (int)(row % T);  // smallest j = longest column first
-    const size_t bh = row / T;
-    const int h = (int)(bh % H), b = (int)(bh / H);
-    const int C = H * D, C3 = 3 * C;
-    float *ps = sm + (size_t)warp * (2 * T + 2 * D);
-    float *dss = ps + T;
-    float *kk = dss + T;
-    float *vv = kk + D;
-    const size_t base = (size_t)b * T * C3;
-    for (int d = lane; d < D; d += kWarp) {
-        kk[d] = x.at(base + (size_t)j * C3 + C + (size_t)h * D + d);
-        vv[d] = x.at(base + (size_t)j * C3 + 2 * (size_t)C + (size_t)h * D + d);
+constexpr int kFwdThreads = 128, kFwdRows = 64;
+
+template <int kNI, int kC>
+struct FwdTile {
+    static constexpr int kPitch = Pitch<kNI>::value, kKeys = 8 * kC, kPPitch = kKeys + 4;
+    static constexpr int kQ = kFwdRows * kPitch;
+    static constexpr int kKP = kKeys * kPitch > kFwdRows * kPPitch ? kKeys * kPitch : kFwdRows * kPPitch;  // K, then P
+    static constexpr int kV = kKeys * kPitch;
+    static constexpr size_t kBytes = (size_t)(kQ + kKP + kV) * sizeof(float);
+};
+
+template <int kNI, int kC, bool kVec>
+__global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *__restrict__ qkv, float *__restrict__ out,
+                                                                  float *__restrict__ out_copy, float *__restrict__ lse,
+                                                                  int T, int H, int D, float scale) {
+    using S = FwdTile<kNI, kC>;
+    constexpr int kR = 4, kPitch = S::kPitch, kKeys = S::kKeys, kPPitch = S::kPPitch;
+    extern __shared__ __align__(16) float sm[];
+    float *sq = sm, *sk = sm + S::kQ, *sp = sk, *sv = sk + S::kKP;
+    const int lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
+    const int row0 = 16 * (threadIdx.x >> 5) + ty;  // this thread's rows: row0 + 4 r
+    const int nq = (T + kFwdRows - 1) / kFwdRows;
+    const int nbh = gridDim.x / nq;
+    const int q0 = (nq - 1 - (int)blockIdx.x / nbh) * kFwdRows;  // longest rows first
+    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
+    const int C = H * D;
+    const size_t C3 = 3 * (size_t)C;
+    const int words = (D + 3) >> 2;
+    const float *head = qkv + (size_t)b * T * C3 + (size_t)h * D;
+
+    tc05::pdl_launch_dependents();
+    tc05::pdl_wait();
+    load_rows_async<kFwdRows, kPitch, kFwdThreads, kVec>(sq, head, C3, q0, T, D);
+    f32x2 o[kR][2 * kNI];
+    float m[kR], l[kR];
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+        m[r] = -INFINITY, l[r] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 2 * kNI; i++) o[r][i] = 0ull;
     }
-    __syncwarp();
-    for (int i = j + lane; i < T; i += kWarp) {
-        const size_t qp = base + (size_t)i * C3 + (size_t)h * D;
-        const size_t gp = ((size_t)b * T + i) * C + (size_t)h * D;
-        float sacc = 0.f, dp = 0.f;
-        for (int d = 0; d < D; d++) {
-            sacc = fmaf(x.at(qp + d), kk[d], sacc);
-            dp = fmaf(dout[gp + d], vv[d], dp);
+    const int last = min(q0 + kFwdRows, T) - 1;
+    for (int j0 = 0; j0 <= last; j0 += kKeys) {
+        load_rows_async<kKeys, kPitch, kFwdThreads, kVec>(sk, head + C, C3, j0, T, D);
+        async_commit();
+        load_rows_async<kKeys, kPitch, kFwdThreads, kVec>(sv, head + 2 * C, C3, j0, T, D);
+        async_commit();
+        async_wait<1>();
+        __syncthreads();
+        float p[kR][kC];
+        {
+            f32x2 acc[kR][kC];
+            score_product<kR, kC, kPitch>(acc, sq + row0 * kPitch, sk + tx * kPitch, words);
+#pragma unroll
+            for (int r = 0; r < kR; r++)
+#pragma unroll
+                for (int c = 0; c < kC; c++) p[r][c] = total(acc[r][c]) * scale;
         }
-        const float p = expf(sacc * scale - lse[bh * T + i]);
-        ps[i - j] = p;
-        dss[i - j] = p * (dp - delta[bh * T + i]);
+        if (j0 + kKeys > q0) {  // the diagonal passes through this tile
+#pragma unroll
+            for (int r = 0; r < kR; r++)
+#pragma unroll
+                for (int c = 0; c < kC; c++)
+                    if (j0 + tx + 8 * c > q0 + row0 + 4 * r) p[r][c] = -INFINITY;
+        }
+#pragma unroll
+        for (int r = 0; r < kR; r++) {
+            float mx = p[r][0];
+#pragma unroll
+            for (int c = 1; c < kC; c++) mx = fmaxf(mx, p[r][c]);
+#pragma unroll
+            for (int s = 1; s < 8; s <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+            mx = fmaxf(mx, m[r]);  // finite: key 0 of the first tile is never masked
+            const float alpha = expf(m[r] - mx);
+            m[r] = mx;
+            l[r] *= alpha;
+            const f32x2 a2 = both(alpha);
+#pragma unroll
+            for (int i = 0; i < 2 * kNI; i++) o[r][i] = mul_x2(o[r][i], a2);
+#pragma unroll
+            for (int c = 0; c < kC; c++) {
+                p[r][c] = expf(p[r][c] - mx);
+                l[r] += p[r][c];
+            }
+        }
+        __syncthreads();  // K has been read by everybody: its place takes P
+#pragma unroll
+        for (int r = 0; r < kR; r++)
+#pragma unroll
+            for (int c = 0; c < kC; c++) sp[(row0 + 4 * r) * kPPitch + tx + 8 * c] = p[r][c];
+        async_wait<0>();
+        __syncthreads();
+#pragma unroll 1
+        for (int j = 0; j < kKeys; j += 4) {
+            float4 pr[kR];
+#pragma unroll
+            for (int r = 0; r < kR; r++) pr[r] = *reinterpret_cast<const float4 *>(sp + (row0 + 4 * r) * kPPitch + j);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                ulonglong2 v[kNI];
+#pragma unroll
+                for (int i = 0; i < kNI; i++) v[i] = lds_x4(sv + (j + e) * kPitch + 4 * tx + 32 * i);
+#pragma unroll
+                for (int r = 0; r < kR; r++) {
+                    const f32x2 pe = both(e == 0 ? pr[r].x : e == 1 ? pr[r].y : e == 2 ? pr[r].z : pr[r].w);
+#pragma unroll
+                    for (int i = 0; i < kNI; i++) {
+                        o[r][2 * i] = fma_x2(pe, v[i].x, o[r][2 * i]);
+                        o[r][2 * i + 1] = fma_x2(pe, v[i].y, o[r][2 * i + 1]);
+                    }
+                }
+            }
+        }
+        __syncthreads();  // P and V have been read: the next tile may overwrite them
     }
-    __syncwarp();
-    for (int d = lane; d < D; d += kWarp) {
-        float dk = 0.f, dv = 0.f;
-        for (int i = j; i < T; i++) {
-            dk = fmaf(dss[i - j], x.at(base + (size_t)i * C3 + (size_t)h * D + d), dk);
-            dv = fmaf(ps[i - j], dout[((size_t)b * T + i) * C + (size_t)h * D + d], dv);
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+        const int t = q0 + row0 + 4 * r;
+        float sum = l[r];
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+        if (t >= T) continue;
+        const float inv = 1.0f / sum;
+        const size_t at = ((size_t)b * T + t) * C + (size_t)h * D;
+#pragma unroll
+        for (int i = 0; i < kNI; i++) {
+            const float2 lo = halves(o[r][2 * i]), hi = halves(o[r][2 * i + 1]);
+            const float4 v = make_float4(lo.x * inv, lo.y * inv, hi.x * inv, hi.y * inv);
+            store_cols<kVec>(out + at, 4 * tx + 32 * i, D, v);
+            if (out_copy) store_cols<kVec>(out_copy + at, 4 * tx + 32 * i, D, v);
         }
-        dqkv[base + (size_t)j * C3 + C + (size_t)h * D + d] = dk * scale;
-        dqkv[base + (size_t)j * C3 + 2 * (size_t)C + (size_t)h * D + d] = dv;
+        if (tx == 0) lse[(size_t)bh * T + t] = m[r] + logf(sum);
     }
 }
 
-int warps_for(size_t floats_per_warp) {
-    const size_t bytes = floats_per_warp * sizeof(float);
-    int nw = (int)(kGenericSmemLimit / bytes);
-    return nw > 4 ? 4 : nw;
+// ---------------------------------------------------------------------------------------
+// backward: one block per (b, h, key tile of 8 kC keys), query tiles from the diagonal on.  K, V, the query tile's Q
+// and dO, P and dS sit in shared memory (171 KB at D = 128, so one block of 8 warps per SM).  Two groups of four
+// warps share the five products: one computes S and then dV, the other dP, dS and then dK; each keeps its gradient
+// tile in registers over all query tiles; dQ of the query tile is shared out by blocks of 32 head columns and added
+// to memory with fp32 atomics (a second kernel that owns the queries would do S and dP again, seven products
+// instead of five).  dq has been zero-filled by the preparation kernel.
+// ---------------------------------------------------------------------------------------
+constexpr int kBwdThreads = 256;
+
+template <int kNI, int kC>
+struct BwdTile {
+    static constexpr int kPitch = Pitch<kNI>::value, kRows = 8 * kC, kPPitch = kRows + 4;
+    static constexpr int kX = kRows * kPitch, kP = kRows * kPPitch;
+    static constexpr size_t kBytes = (size_t)(4 * kX + 2 * kP + 2 * kRows) * sizeof(float);
+};
+
+// g[k][..] += sum over the query tile of p[q][key k] * x[q][columns of this thread]
+template <int kR, int kNI, int kRows, int kPPitch, int kPitch>
+__device__ __forceinline__ void key_gradient(f32x2 (&g)[kR][2 * kNI], const float *p, const float *x) {
+#pragma unroll 2
+    for (int q = 0; q < kRows; q++) {
+        float pk[kR];
+        if (kR == 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(p + q * kPPitch);
+            pk[0] = v.x, pk[1] = v.y, pk[2 % kR] = v.z, pk[3 % kR] = v.w;
+        } else {
+            const float2 v = *reinterpret_cast<const float2 *>(p + q * kPPitch);
+            pk[0] = v.x, pk[1] = v.y;
+        }
+        ulonglong2 xv[kNI];
+#pragma unroll
+        for (int i = 0; i < kNI; i++) xv[i] = lds_x4(x + q * kPitch + 32 * i);
+#pragma unroll
+        for (int k = 0; k < kR; k++) {
+            const f32x2 pe = both(pk[k]);
+#pragma unroll
+            for (int i = 0; i < kNI; i++) {
+                g[k][2 * i] = fma_x2(pe, xv[i].x, g[k][2 * i]);
+                g[k][2 * i + 1] = fma_x2(pe, xv[i].y, g[k][2 * i + 1]);
+            }
+        }
+    }
 }
+
+template <int kNI, int kC, bool kVec>
+__global__ void __launch_bounds__(kBwdThreads) generic_bwd_kernel(const __nv_bfloat16 *__restrict__ xhi,
+                                                                  const __nv_bfloat16 *__restrict__ xlo,
+                                                                  const float *__restrict__ lse,
+                                                                  const float *__restrict__ delta,
+                                                                  const float *__restrict__ dout,
+                                                                  float *__restrict__ dqkv, int T, int H, int D,
+                                                                  float scale) {
+    using S = BwdTile<kNI, kC>;
+    constexpr int kR = kC / 2;  // 16 row groups cover the tile
+    constexpr int kPitch = S::kPitch, kRows = S::kRows, kPPitch = S::kPPitch;
+    constexpr int kQI = (kNI + 1) / 2;  // column blocks of dQ per group
+    extern __shared__ __align__(16) float sm[];
+    float *sk = sm, *sv = sk + S::kX, *sq = sv + S::kX, *sg = sq + S::kX;
+    float *sp = sg + S::kX, *sd = sp + S::kP, *s_lse = sd + S::kP, *s_delta = s_lse + kRows;
+    const int lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
+    const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3;
+    const int row0 = 4 * kR * warp + ty;  // score tiles: rows row0 + 4 r, columns tx + 8 c
+    const int key0 = 4 * kR * warp + kR * ty;  // gradient tiles: keys key0 .. key0 + kR - 1, columns 4 tx + 32 i
+    const int nt = (T + kRows - 1) / kRows;
+    const int nbh = gridDim.x / nt;
+    const int k0 = (int)blockIdx.x / nbh * kRows;  // the first keys are seen by the most queries
+    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
+    const int C = H * D;
+    const size_t C3 = 3 * (size_t)C;
+    const int words = (D + 3) >> 2;
+    const size_t head = (size_t)b * T * C3 + (size_t)h * D;
+    const float *dhead = dout + (size_t)b * T * C + (size_t)h * D;
+
+    tc05::pdl_launch_dependents();
+    tc05::pdl_wait();
+    load_rows_split<kRows, kPitch, kBwdThreads, kVec>(sk, xhi + head + C, xlo + head + C, C3, k0, T, D);
+    load_rows_split<kRows, kPitch, kBwdThreads, kVec>(sv, xhi + head + 2 * C, xlo + head + 2 * C, C3, k0, T, D);
+    f32x2 grad[kR][2 * kNI];  // dV in group 0, dK in group 1
+#pragma unroll
+    for (int r = 0; r < kR; r++)
+#pragma unroll
+        for (int i = 0; i < 2 * kNI; i++) grad[r][i] = 0ull;
+
+    for (int q0 = k0; q0 < T; q0 += kRows) {
+        load_rows_async<kRows, kPitch, kBwdThreads, kVec>(sg, dhead, (size_t)C, q0, T, D);
+        async_commit();
+        load_rows_split<kRows, kPitch, kBwdThreads, kVec>(sq, xhi + head, xlo + head, C3, q0, T, D);
+        if (threadIdx.x < 2 * kRows) {
+            const int r = threadIdx.x % kRows;
+            const float *src = threadIdx.x < kRows ? lse : delta;
+            s_lse[threadIdx.x] = q0 + r < T ? src[(size_t)bh * T + q0 + r] : 0.f;
+        }
+        async_wait<0>();
+        __syncthreads();
+        {
+            f32x2 acc[kR][kC];
+            if (group == 0) {
+                score_product<kR, kC, kPitch>(acc, sq + row0 * kPitch, sk + tx * kPitch, words);
+#pragma unroll
+                for (int r = 0; r < kR; r++) {
+                    const int q = q0 + row0 + 4 * r;
+#pragma unroll
+                    for (int c = 0; c < kC; c++) {
+                        const float e = expf(total(acc[r][c]) * scale - s_lse[row0 + 4 * r]);
+                        sp[(row0 + 4 * r) * kPPitch + tx + 8 * c] = q < T && k0 + tx + 8 * c <= q ? e : 0.f;
+                    }
+                }
+            } else {
+                score_product<kR, kC, kPitch>(acc, sg + row0 * kPitch, sv + tx * kPitch, words);
+            }
+            __syncthreads();  // P is complete
+            if (group == 1) {
+#pragma unroll
+                for (int r = 0; r < kR; r++)
+#pragma unroll
+                    for (int c = 0; c < kC; c++) {
+                        const int at = (row0 + 4 * r) * kPPitch + tx + 8 * c;
+                        sd[at] = sp[at] * (total(acc[r][c]) - s_delta[row0 + 4 * r]);
+                    }
+                asm volatile("bar.sync 1, 128;" ::: "memory");  // dS is complete for the warps of this group
+            }
+        }
+        if (group == 0) key_gradient<kR, kNI, kRows, kPPitch, kPitch>(grad, sp + key0, sg + 4 * tx);
+        else key_gradient<kR, kNI, kRows, kPPitch, kPitch>(grad, sd + key0, sq + 4 * tx);
+        __syncthreads();  // dS is complete for everybody
+        {
+            f32x2 dq[kR][2 * kQI];
+#pragma unroll
+            for (int r = 0; r < kR; r++)
+#pragma unroll
+                for (int i = 0; i < 2 * kQI; i++) dq[r][i] = 0ull;
+#pragma unroll 1
+            for (int j = 0; j < kRows; j += 4) {
+                float4 ds[kR];
+#pragma unroll
+                for (int r = 0; r < kR; r++) ds[r] = *reinterpret_cast<const float4 *>(sd + (row0 + 4 * r) * kPPitch + j);
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    ulonglong2 kv[kQI];
+#pragma unroll
+                    for (int i = 0; i < kQI; i++) {
+                        const int block = min(group + 2 * i, kNI - 1);  // an odd last block is done by group 0
+                        kv[i] = lds_x4(sk + (j + e) * kPitch + 4 * tx + 32 * block);
+                    }
+#pragma unroll
+                    for (int r = 0; r < kR; r++) {
+                        const f32x2 de = both(e == 0 ? ds[r].x : e == 1 ? ds[r].y : e == 2 ? ds[r].z : ds[r].w);
+#pragma unroll
+                        for (int i = 0; i < kQI; i++) {
+                            dq[r][2 * i] = fma_x2(de, kv[i].x, dq[r][2 * i]);
+                            dq[r][2 * i + 1] = fma_x2(de, kv[i].y, dq[r][2 * i + 1]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kR; r++) {
+                const int t = q0 + row0 + 4 * r;
+                if (t >= T) continue;
+                float *dst = dqkv + head + (size_t)t * C3;
+#pragma unroll
+                for (int i = 0; i < kQI; i++) {
+                    const int col = 4 * tx + 32 * (group + 2 * i);
+                    const float2 lo = halves(dq[r][2 * i]), hi = halves(dq[r][2 * i + 1]);
+                    if (group + 2 * i >= kNI || col >= D) continue;
+                    if (kVec) {
+                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + col), "f"(lo.x * scale),
+                                     "f"(lo.y * scale), "f"(hi.x * scale), "f"(hi.y * scale)
+                                     : "memory");
+                    } else {
+                        const float v[4] = {lo.x * scale, lo.y * scale, hi.x * scale, hi.y * scale};
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            if (col + e < D) atomicAdd(dst + col + e, v[e]);
+                    }
+                }
+            }
+        }
+        __syncthreads();  // Q, dO, P and dS may be overwritten
+    }
+    const float by = group == 0 ? 1.0f : scale;
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+        const int t = k0 + key0 + r;
+        if (t >= T) continue;
+        float *dst = dqkv + head + (size_t)t * C3 + (group == 0 ? 2 * C : C);
+#pragma unroll
+        for (int i = 0; i < kNI; i++) {
+            const float2 lo = halves(grad[r][2 * i]), hi = halves(grad[r][2 * i + 1]);
+            store_cols<kVec>(dst, 4 * tx + 32 * i, D, make_float4(lo.x * by, lo.y * by, hi.x * by, hi.y * by));
+        }
+    }
+}
+
+template <int kNI>
+struct Generic {
+    // key tiles of 64; head sizes above 128 take 32, whose wider rows need as much shared memory and registers
+    static constexpr int kC = kNI <= 4 ? 8 : 4;
+    using F = FwdTile<kNI, kC>;
+    using G = BwdTile<kNI, kC>;
+
+    static cudaError_t set_attributes() {
+        cudaError_t e;
+        const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if ((e = cudaFuncSetAttribute(generic_fwd_kernel<kNI, kC, true>, a, (int)F::kBytes)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(generic_fwd_kernel<kNI, kC, false>, a, (int)F::kBytes)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(generic_bwd_kernel<kNI, kC, true>, a, (int)G::kBytes)) != cudaSuccess) return e;
+        return cudaFuncSetAttribute(generic_bwd_kernel<kNI, kC, false>, a, (int)G::kBytes);
+    }
+    static cudaError_t forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H, int D,
+                               cudaStream_t s) {
+        const dim3 grid((unsigned)((size_t)B * H * ((T + kFwdRows - 1) / kFwdRows)));
+        return launch_after_previous(D % 4 == 0 ? generic_fwd_kernel<kNI, kC, true> : generic_fwd_kernel<kNI, kC, false>, grid,
+                                     dim3(kFwdThreads), F::kBytes, s, qkv, out, out_copy, lse, T, H, D,
+                                     1.0f / sqrtf((float)D));
+    }
+    static cudaError_t backward(const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse, const float *delta,
+                                const float *dout, float *dqkv, int B, int T, int H, int D, cudaStream_t s) {
+        const dim3 grid((unsigned)((size_t)B * H * ((T + G::kRows - 1) / G::kRows)));
+        return launch_after_previous(D % 4 == 0 ? generic_bwd_kernel<kNI, kC, true> : generic_bwd_kernel<kNI, kC, false>, grid,
+                                     dim3(kBwdThreads), G::kBytes, s, xhi, xlo, lse, delta, dout, dqkv, T, H, D,
+                                     1.0f / sqrtf((float)D));
+    }
+};
 
 }  // namespace
 
+// f(Generic<n>{}) for n = 1 .. 8, the number of 32-column blocks of the head size
+template <class Fn>
+static cudaError_t with_blocks(int n, Fn f) {
+    switch (n) {
+        case 1: return f(Generic<1>{});
+        case 2: return f(Generic<2>{});
+        case 3: return f(Generic<3>{});
+        case 4: return f(Generic<4>{});
+        case 5: return f(Generic<5>{});
+        case 6: return f(Generic<6>{});
+        case 7: return f(Generic<7>{});
+        default: return f(Generic<8>{});
+    }
+}
+
 cudaError_t generic_set_attributes() {
-    cudaError_t e;
-    e = cudaFuncSetAttribute(generic_fwd_kernel<XF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGenericSmemLimit);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(generic_bwd_dq_kernel<XSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kGenericSmemLimit);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(generic_bwd_dkv_kernel<XSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kGenericSmemLimit);
+    for (int n = 1; n <= kGenericMaxD / 32; n++) {
+        const cudaError_t e = with_blocks(n, [](auto g) { return decltype(g)::set_attributes(); });
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t n, cudaStream_t s) {
@@ -343,7 +692,7 @@ cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, s
 
 cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta, __nv_bfloat16 *dhi,
                                __nv_bfloat16 *dlo, float *dq_zero, int *sched, int B, int T, int H, int D, cudaStream_t s) {
-    if (D == 64 && dhi && dlo && dq_zero) {
+    if (D == 64 && dhi && dlo) {
         const size_t nvec = (size_t)B * T * H * 8;
         size_t blocks = (nvec + 255) / 256;
         if (blocks > 148 * 16) blocks = 148 * 16;
@@ -353,45 +702,22 @@ cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta
     const size_t rows = (size_t)B * T * H;
     size_t blocks = (rows + 7) / 8;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    bwd_prepare_kernel<<<(unsigned)blocks, 256, 0, s>>>(dout, out, delta, dhi, dlo, dq_zero, B, T, H, D);
-    return cudaGetLastError();
+    return launch_after_previous(bwd_prepare_kernel, dim3((unsigned)blocks), dim3(256), 0, s, dout, out, delta, dq_zero, B, T,
+                                 H, D);
 }
 
 cudaError_t launch_generic_forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H,
                                    int D, cudaStream_t s) {
-    const size_t per_warp = (size_t)T + D;
-    const int nw = warps_for(per_warp);
-    if (nw < 1) return cudaErrorInvalidValue;
-    const size_t rows = (size_t)B * H * T;
-    const size_t blocks = (rows + nw - 1) / nw;
-    generic_fwd_kernel<XF32><<<(unsigned)blocks, nw * 32, nw * per_warp * sizeof(float), s>>>(
-        XF32{qkv}, out, out_copy, lse, B, T, H, D, 1.0f / sqrtf((float)D));
-    return cudaGetLastError();
+    return with_blocks((D + 31) / 32,
+                       [&](auto g) { return decltype(g)::forward(qkv, out, out_copy, lse, B, T, H, D, s); });
 }
 
 cudaError_t launch_generic_backward(const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse,
                                     const float *delta, const float *dout, float *dqkv, int B, int T, int H, int D,
                                     cudaStream_t s) {
-    const size_t rows = (size_t)B * H * T;
-    const float scale = 1.0f / sqrtf((float)D);
-    XSplit x{xhi, xlo};
-    {
-        const size_t per_warp = (size_t)T + 2 * D;
-        const int nw = warps_for(per_warp);
-        if (nw < 1) return cudaErrorInvalidValue;
-        generic_bwd_dq_kernel<XSplit><<<(unsigned)((rows + nw - 1) / nw), nw * 32, nw * per_warp * sizeof(float), s>>>(
-            x, lse, delta, dout, dqkv, B, T, H, D, scale);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    {
-        const size_t per_warp = 2 * (size_t)T + 2 * D;
-        const int nw = warps_for(per_warp);
-        if (nw < 1) return cudaErrorInvalidValue;
-        generic_bwd_dkv_kernel<XSplit><<<(unsigned)((rows + nw - 1) / nw), nw * 32, nw * per_warp * sizeof(float), s>>>(
-            x, lse, delta, dout, dqkv, B, T, H, D, scale);
-    }
-    return cudaGetLastError();
+    return with_blocks((D + 31) / 32, [&](auto g) {
+        return decltype(g)::backward(xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, s);
+    });
 }
 
 }  // namespace attn

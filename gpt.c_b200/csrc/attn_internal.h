@@ -11,7 +11,6 @@ namespace attn {
 
 constexpr int kGenericMaxD = 256;
 constexpr int kGenericMaxT = 8192;
-constexpr int kGenericSmemLimit = 200 * 1024;
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -21,9 +20,9 @@ inline size_t plane_bytes(size_t n) { return align_up(n * sizeof(__nv_bfloat16),
 // fp32 -> (hi, lo) bf16 planes, hi = bf16(x), lo = bf16(x - hi).
 cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t n, cudaStream_t s);
 
-// rowsum(dout * out) per (b, h, t) -> delta [B, H, T]; also splits dout into bf16 planes when
-// dhi/dlo are given, zero-fills the dq third of `dq_zero` ([B, T, 3C]) when it is given, and zeroes the
-// two ints at `sched` (the item counter of the tensor-core backward kernel) when that is given.
+// rowsum(dout * out) per (b, h, t) -> delta [B, H, T], and zero-fill of the dq third of `dq_zero` ([B, T, 3C]);
+// also splits dout into bf16 planes when dhi/dlo are given and zeroes the two ints at `sched` (the item counter
+// of the tensor-core backward kernel) when that is given.
 cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta, __nv_bfloat16 *dhi,
                                __nv_bfloat16 *dlo, float *dq_zero, int *sched, int B, int T, int H, int D, cudaStream_t s);
 

@@ -78,6 +78,19 @@ def test_generic_vs_oracle(pkg, gpu, oracle, shape):
     assert np.abs(dx - oracle.backward(x, g, H)).max() < GENERIC_TOL
 
 
+@pytest.mark.parametrize("D", [1, 4, 31, 32, 33, 63, 96, 100, 128, 129, 132, 200, 256])
+@pytest.mark.parametrize("T", [1, 63, 65, 130])
+def test_generic_tile_edges(pkg, gpu, oracle, T, D):
+    """Query and key tiles of 64 (32 above D = 128), head columns in blocks of 32, rows read in words of four
+    columns when D allows it."""
+    x, g = seeded(23 + T + D, 2, T, 2, D)
+    out, lse, dx = run_cuda(pkg, gpu, x, g, 2, flags=pkg.FLAG_FORCE_GENERIC)
+    ref_out, ref_lse = oracle.forward(x, 2, want_lse=True)
+    assert np.abs(out - ref_out).max() < GENERIC_TOL
+    assert np.abs(lse - ref_lse).max() < GENERIC_TOL
+    assert np.abs(dx - oracle.backward(x, g, 2)).max() < GENERIC_TOL
+
+
 # ---------------------------------------------------------------------------------------------
 # tensor-core kernels (D = 64)
 # ---------------------------------------------------------------------------------------------
