@@ -2,7 +2,8 @@
 
 The product is the C-ABI library declared in ``include/attn_sm100.h`` (hand-written sm_100a CUDA).
 This package only loads it and offers a thin convenience layer that takes ``torch`` CUDA tensors
-for device memory and streams; every call goes through the C ABI with raw pointers.  There is no
+for device memory and streams; every call goes through the C ABI with raw pointers, the tensor-level
+ones by way of a small extension module (``csrc/torch_calls.cpp``).  There is no
 CPU or PyTorch fallback: if the library is missing or the device is not an sm_100 GPU the calls
 raise.
 
@@ -17,6 +18,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libattn_sm100.so")
+CALLS_PATH = os.path.join(HERE, "lib", "gptc_b200_calls.so")
 HEADER_PATH = os.path.join(HERE, "..", "include", "attn_sm100.h")
 
 FLAG_FORCE_GENERIC = 1
@@ -54,6 +56,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_calls_module = None
 
 
 class AttnError(RuntimeError):
@@ -79,13 +82,33 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def _calls():
+    """The extension module over the C ABI (once).  Raises if it has not been built."""
+    global _calls_module
+    if _calls_module is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+
+        lib()
+        if not os.path.exists(CALLS_PATH):
+            raise FileNotFoundError(
+                f"{CALLS_PATH} is missing: build it with `python gpt.c_b200/build.py`; there is no fallback path")
+        spec = importlib.util.spec_from_file_location("gptc_b200_calls", CALLS_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_error(AttnError)
+        _calls_module = mod
+    return _calls_module
+
+
+def _raw(stream):
+    return None if stream is None else stream.cuda_stream
+
+
 def _check(code: int, where: str) -> None:
     if code != 0:
         raise AttnError(code, where)
-
-
-def _ptr(t) -> int:
-    return 0 if t is None else t.data_ptr()
 
 
 def init() -> None:
@@ -127,55 +150,22 @@ class Saved:
 
 def forward_into(qkv, out, out_copy, lse, saved, n_heads: int, flags: int = 0, stream=None) -> None:
     """Raw call: every buffer is supplied by the caller (torch CUDA tensors or None)."""
-    import torch
-
-    B, T, C3 = qkv.shape
-    D = C3 // 3 // n_heads
-    s = torch.cuda.current_stream() if stream is None else stream
-    _check(lib().attn_sm100_forward(_ptr(qkv), _ptr(out), _ptr(out_copy), _ptr(lse), _ptr(saved), B, T, n_heads, D,
-                                    flags, s.cuda_stream), "attn_sm100_forward")
+    _calls().forward_into(qkv, out, out_copy, lse, saved, n_heads, flags, _raw(stream))
 
 
 def backward_into(saved, out, lse, dout, dqkv, scratch, n_heads: int, flags: int = 0, stream=None) -> None:
-    import torch
-
-    B, T, C = dout.shape
-    D = C // n_heads
-    s = torch.cuda.current_stream() if stream is None else stream
-    _check(lib().attn_sm100_backward(_ptr(saved), _ptr(out), _ptr(lse), _ptr(dout), _ptr(dqkv), _ptr(scratch), B, T,
-                                     n_heads, D, flags, s.cuda_stream), "attn_sm100_backward")
+    _calls().backward_into(saved, out, lse, dout, dqkv, scratch, n_heads, flags, _raw(stream))
 
 
 def forward(qkv, n_heads: int, flags: int = 0, keep_copy: bool = False):
     """qkv [B, T, 3C] fp32 CUDA tensor -> (out [B, T, C], Saved)."""
-    import torch
-
-    if not (qkv.is_cuda and qkv.dtype == torch.float32 and qkv.is_contiguous() and qkv.dim() == 3):
-        raise ValueError("qkv must be a contiguous fp32 CUDA tensor of shape [B, T, 3C]")
-    B, T, C3 = qkv.shape
-    if C3 % (3 * n_heads) != 0:
-        raise ValueError("last dimension must be 3 * n_heads * head_size")
-    C = C3 // 3
-    D = C // n_heads
-    out = torch.empty((B, T, C), device=qkv.device, dtype=torch.float32)
-    out_copy = torch.empty_like(out) if keep_copy else None
-    lse = torch.empty((B, n_heads, T), device=qkv.device, dtype=torch.float32)
-    saved = torch.empty(saved_bytes(B, T, n_heads, D), device=qkv.device, dtype=torch.uint8)
-    forward_into(qkv, out, out_copy, lse, saved, n_heads, flags)
-    return out, Saved(saved, out_copy if keep_copy else out, lse, (B, T, n_heads, D), flags)
+    out, out_copy, lse, saved, shape = _calls().forward(qkv, n_heads, flags, keep_copy)
+    return out, Saved(saved, out if out_copy is None else out_copy, lse, shape, flags)
 
 
 def backward(ctx: Saved, dout):
     """dout [B, T, C] -> dqkv [B, T, 3C] = [dq | dk | dv]."""
-    import torch
-
-    B, T, H, D = ctx.shape
-    if not (dout.is_cuda and dout.dtype == torch.float32 and dout.is_contiguous() and tuple(dout.shape) == (B, T, H * D)):
-        raise ValueError("dout must be a contiguous fp32 CUDA tensor of shape [B, T, C]")
-    dqkv = torch.empty((B, T, 3 * H * D), device=dout.device, dtype=torch.float32)
-    scratch = torch.empty(backward_scratch_bytes(B, T, H, D), device=dout.device, dtype=torch.uint8)
-    backward_into(ctx.saved, ctx.out, ctx.lse, dout, dqkv, scratch, H, ctx.flags)
-    return dqkv
+    return _calls().backward(ctx.saved, ctx.out, ctx.lse, dout, ctx.shape, ctx.flags)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -185,33 +175,13 @@ def backward(ctx: Saved, dout):
 def linear_forward(x, w, bias=None, planes=None, stream=None):
     """y[..., N] = x[..., K] @ w[N, K].T + bias.  `planes`: optional uint8 CUDA tensor of
     saved_bytes(...) bytes that receives y as bf16 hi/lo planes for the attention kernels."""
-    import torch
-
-    K = x.shape[-1]
-    N = w.shape[0]
-    M = x.numel() // K
-    y = torch.empty((*x.shape[:-1], N), device=x.device, dtype=torch.float32)
-    s = torch.cuda.current_stream() if stream is None else stream
-    _check(lib().linear_sm100_forward(_ptr(x), _ptr(w), _ptr(bias), _ptr(y), _ptr(planes), M, N, K, s.cuda_stream),
-           "linear_sm100_forward")
-    return y
+    return _calls().linear_forward(x, w, bias, planes, _raw(stream))
 
 
 def linear_backward(dy, x, w, dw, db=None, stream=None, want_dx=True):
     """Returns dx = dy @ w (None when want_dx is false); accumulates dy.T @ x into dw (skipped when dw is
     None) and the column sums of dy into db."""
-    import torch
-
-    K = x.shape[-1]
-    N = w.shape[0]
-    M = x.numel() // K
-    dx = torch.empty_like(x) if want_dx else None
-    s = torch.cuda.current_stream() if stream is None else stream
-    nbytes = lib().linear_sm100_backward_scratch_bytes(M, N, K)
-    scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8) if nbytes else None
-    _check(lib().linear_sm100_backward(_ptr(dy), _ptr(x), _ptr(w), _ptr(dx), _ptr(dw), _ptr(db), _ptr(scratch), M, N, K,
-                                       s.cuda_stream), "linear_sm100_backward")
-    return dx
+    return _calls().linear_backward(dy, x, w, dw, db, _raw(stream), want_dx)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -220,25 +190,9 @@ def linear_backward(dy, x, w, dw, db=None, stream=None, want_dx=True):
 # ---------------------------------------------------------------------------------------------
 def layernorm_forward(x, w, b=None, eps: float = 1e-5, stream=None):
     """Returns (y, mean, rstd) for x [..., C]."""
-    import torch
-
-    C = x.shape[-1]
-    rows = x.numel() // C
-    y = torch.empty_like(x)
-    mean = torch.empty(rows, device=x.device, dtype=torch.float32)
-    rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
-    s = torch.cuda.current_stream() if stream is None else stream
-    _check(lib().layernorm_sm100_forward(_ptr(x), _ptr(w), _ptr(b), eps, _ptr(mean), _ptr(rstd), _ptr(y), rows, C,
-                                         s.cuda_stream), "layernorm_sm100_forward")
-    return y, mean, rstd
+    return _calls().layernorm_forward(x, w, b, eps, _raw(stream))
 
 
 def layernorm_backward(dy, x, mean, rstd, w, dw, db, dx, stream=None) -> None:
     """Accumulates into dw, db (may be None) and dx, like the reference."""
-    import torch
-
-    C = x.shape[-1]
-    rows = x.numel() // C
-    s = torch.cuda.current_stream() if stream is None else stream
-    _check(lib().layernorm_sm100_backward(_ptr(dy), _ptr(x), _ptr(mean), _ptr(rstd), _ptr(w), _ptr(dw), _ptr(db), _ptr(dx),
-                                          rows, C, s.cuda_stream), "layernorm_sm100_backward")
+    _calls().layernorm_backward(dy, x, mean, rstd, w, dw, db, dx, _raw(stream))
