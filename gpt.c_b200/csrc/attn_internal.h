@@ -47,20 +47,30 @@ cudaError_t launch_fast_backward(const CUtensorMap &map_x, const CUtensorMap &ma
 
 // Launches `kernel` so that it may begin (up to its pdl_wait(), tc05.cuh) while the previous kernel of the
 // stream is still running: its launch latency and set-up overlap that kernel's tail.
+// cluster > 1: in clusters of that many CTAs along x.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                         Args &&...args) {
+inline cudaError_t launch_clusters_after_previous(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, unsigned cluster,
+                                                  cudaStream_t s, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                         Args &&...args) {
+    return launch_clusters_after_previous(kernel, grid, block, smem, 1, s, static_cast<Args &&>(args)...);
 }
 
 // Helpers shared with the Linear kernels (linear_sm100.cu).

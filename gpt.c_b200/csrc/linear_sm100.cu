@@ -12,20 +12,25 @@
 //     forward  y [M,N]  = x [M,K] . W[N,K]^T        A: x, K-major          B: W,  K-major
 //     dx       dx[M,K]  = dy[M,N] . W[N,K]          A: dy, K-major (over N) B: W,  MN-major
 //     dW       dW[N,K] += dy[M,N]^T . x[M,K]        A: dy, MN-major         B: x,  MN-major  (split over M)
-// (K-major: the contraction index is the contiguous one.)  Tiles are 128 x 128 with contraction
-// blocks of 32 fp32 values (one 128-byte swizzled row), four stages.
+// (K-major: the contraction index is the contiguous one.)  Contraction blocks are 32 fp32 values (one 128-byte
+// swizzled row).  A tile is 128 rows of one CTA, or 256 rows of a CTA pair (cta_group::2), by 128, 192 or 256
+// columns, with as many pipeline stages as shared memory holds; plan_tiles picks the shape.
+//
+// What bounds the kernel: at 256 x 256 a pair needs 32 KB per CTA and contraction block, which takes 512 cycles of
+// the tensor core and arrives at the 55 to 62 bytes per cycle an SM gets from L2 when all of them ask; a CTA on its
+// own needs 48 KB for half the work (64 % tensor pipe active).  The result is written straight from registers, a row
+// per lane in 32-byte sectors: staging it for the copy engine costs shared memory that the pipeline wants (7 stages
+// instead of 6), bandwidth, and hand-overs between warps.  8192 x 3072 x 768: forward 67.0 -> 58.4 us, dx of the
+// same layer 69 -> 61 us, dW 61 -> 53 us; with bf16 planes (QKV) 62.7 -> 56 us.
 //
 // Warp roles (384 threads, one CTA per SM, grid = number of SMs, tiles handed out round robin):
 //   warp 0      TMA producer
-//   warp 1      MMA issuer (kind::tf32, M128 N128 K8, one elected lane)
-//   warp 2      tensor-memory allocation (2 accumulators of 128 columns: the epilogue of one tile
-//               overlaps the main loop of the next)
-//   warps 4-11  epilogue, two warps per tensor-memory lane quarter: accumulator -> registers ->
-//               (+bias, bf16 split) -> swizzled staging tile in shared memory
-//   warp 3      bulk tensor store (forward, dx) or bulk tensor reduction (dW) of each staged chunk
+//   warp 1      MMA issuer (kind::tf32, one elected lane; of a pair, the leader's)
+//   warp 2      tensor-memory allocation (2 accumulators: the epilogue of one tile overlaps the main loop of the next)
+//   warps 4-11  epilogue: 32 rows and half of the columns each, (+ bias, bf16 split) -> global memory, or through a
+//               staging buffer of the warp's own to a bulk tensor reduction (dW) or unaligned rows (vocabulary)
 // All waits are bounded (see tc05.cuh).
-#include "attn_internal.h"
-#include "tc05.cuh"
+#include "linear_tf32.cuh"
 
 #include "../../include/linear_sm100.h"
 #include "../../include/tensor_sm100.h"
@@ -35,27 +40,18 @@ namespace {
 
 using namespace tc05;
 
-constexpr int kBM = 128, kBK = 32;
-constexpr int kATileBytes = kBM * kBK * 4;  // A tile of one stage: 16 KiB
 constexpr int kThreads = 384;
-constexpr int kEpiThreads = 256;
+constexpr int kEpiWarps = 8;
 
 // Tile width kBN (128 or 256 columns) and pipeline depth are chosen per problem: wide tiles halve the
 // shared-memory and L2 traffic per flop, narrow ones fill the SMs better when there are few tiles.
-template <int kBN, int kStages, bool kPlanes>
+template <int kBN, int kStages, bool kPair, bool kStage>
 struct __align__(1024) SmemT {
     uint8_t a[kStages][kATileBytes];
-    uint8_t b[kStages][kBN * kBK * 4];
-    // 64 output columns of a tile on their way out: fp32 columns 0-31 and fp32 columns 32-63; when the bf16
-    // planes are wanted, the same two buffers then carry the hi plane (64 columns) and the lo plane of the
-    // chunk (a second round through the copy engine: two more buffers would cost a pipeline stage, and the
-    // depth of the operand pipeline is what bounds this kernel); each [128 rows x 128 bytes], swizzled
-    // 192-wide tiles without planes stage through ONE buffer (32 columns per round): that leaves room for a
-    // fifth pipeline stage of 40 KB
-    uint8_t out[(kBN == 192 && !kPlanes) ? 1 : 2][16384];
+    uint8_t b[kStages][kBN * kBK * 4 / (kPair ? 2 : 1)];  // a pair's CTAs hold half of the columns each
+    uint8_t out[kStage ? kEpiWarps : 1][kStage ? 4096 : 16];  // output staging of the epilogue warps: 32 rows x 128 bytes
     uint64_t full[kStages], empty[kStages];
     uint64_t acc_full[2], acc_empty[2];
-    uint64_t out_ready, out_free;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -63,51 +59,23 @@ struct __align__(1024) SmemT {
 struct Problem {
     int M, N, K;  // C is [M, N]; K is the contraction length
     int bn;       // tile width
+    int pair;     // tiles of 256 rows on CTA pairs (else of 128 rows on single CTAs)
     int a_one, b_one;  // MN-major operand fetched with one 3-D copy per stage (else one copy per 32-row block)
     int tiles_m, tiles_n, splits, kb_total, kb_per_split, total;
+    int wide, wide_planes;  // rows of C / of the planes start on 32-byte boundaries
+    size_t plane_words;     // distance from the hi to the lo plane
     int m_fast;  // consecutive work items walk down the rows of C (else along its columns)
 };
 
 enum Site : int {
-    SITE_EMPTY = 201, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_OUT_READY, SITE_OUT_FREE, SITE_SMEM_ALIGN
+    SITE_EMPTY = 201, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_SMEM_ALIGN
 };
-
-// Instruction descriptor for kind::tf32 (A and B formats = 2), fp32 accumulation.
-__host__ __device__ constexpr uint32_t idesc_tf32(int M, int N, int a_mn_major, int b_mn_major) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) |
-           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_tf32_lead(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                              uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, e;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 e, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-        "}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
-
-// Shared-memory descriptor for 32-bit operands read MN-major: layout type 1 (128-byte swizzle with
-// 32-byte atoms); rows of 32 values along M/N, LBO = distance between 32-value blocks, SBO = distance
-// between groups of 4 contraction steps.
-__device__ __forceinline__ uint64_t smem_desc_sw128_base32(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)1 << 61;
-    return d;
-}
 
 struct Work {
-    int m0, n0, kb0, kb1;
+    int m0, n0, kb0, kb1;  // first row of this CTA's 128, first column of the tile, contraction blocks
 };
-__device__ __forceinline__ Work decode(const Problem &p, int w) {
+template <bool kPair>
+__device__ __forceinline__ Work decode(const Problem &p, int w, int rank) {
     const int split = w % p.splits;
     const int t = w / p.splits;
     // The operand whose tile index changes slowest is read from HBM once; the other one is streamed again for
@@ -115,26 +83,49 @@ __device__ __forceinline__ Work decode(const Problem &p, int w) {
     const int tn = p.m_fast ? t / p.tiles_m : t % p.tiles_n;
     const int tm = p.m_fast ? t % p.tiles_m : t / p.tiles_n;
     Work r;
-    r.m0 = tm * kBM;
+    r.m0 = kPair ? (2 * tm + rank) * kBM : tm * kBM;
     r.n0 = tn * p.bn;
     r.kb0 = split * p.kb_per_split;
     r.kb1 = min(p.kb_total, r.kb0 + p.kb_per_split);
     return r;
 }
 
+// Writes 4 * kQuads consecutive 32-bit words to dst, as far as `left` words go (a multiple of
+// 4): 32 bytes per store where dst allows it, else 16.
+template <int kQuads>
+__device__ __forceinline__ void store_words(void *dst, int left, int wide, const uint32_t *r) {
+    uint32_t *d = static_cast<uint32_t *>(dst);
+    if (wide) {
+#pragma unroll
+        for (int q = 0; q < kQuads / 2; q++)
+            if (8 * q < left)
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(d + 8 * q), "r"(r[8 * q]),
+                             "r"(r[8 * q + 1]), "r"(r[8 * q + 2]), "r"(r[8 * q + 3]), "r"(r[8 * q + 4]), "r"(r[8 * q + 5]),
+                             "r"(r[8 * q + 6]), "r"(r[8 * q + 7])
+                             : "memory");
+    } else {
+#pragma unroll
+        for (int q = 0; q < kQuads; q++)
+            if (4 * q < left) *reinterpret_cast<uint4 *>(d + 4 * q) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+    }
+}
+
 // kEpi 0: C = acc (+ bias), optional bf16 planes; kEpi 1: C += acc (bulk reduction)
 // kDirect: the result goes out with plain coalesced 4-byte stores instead of the copy engine, for outputs
 // whose row pitch is not a multiple of 16 bytes (the 50257-wide vocabulary projection).
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect = false>
+// kPair: two CTAs of a cluster share a tile of 256 rows.  Each loads its 128 rows of A and half of the kBN columns
+// of B, 32 KB per contraction block of a 256 x 256 tile where a CTA on its own needs 48 KB for a 128 x 256 one.
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                   const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_planes,
-                   const float *__restrict__ bias, float *__restrict__ c_direct, Problem p, int *status) {
+                   const __grid_constant__ CUtensorMap map_c, const float *__restrict__ bias, float *__restrict__ c_direct,
+                   uint32_t *__restrict__ planes, Problem p, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    using Smem = SmemT<kBN, kStages, kPlanes>;
+    using Smem = SmemT<kBN, kStages, kPair, kEpi == 1 || kDirect>;
     constexpr uint32_t kTmemCols = 2 * kBN <= 256 ? 256 : 512;  // a power of two that holds two accumulators
-    constexpr int kBTileBytes = kBN * kBK * 4;
-    constexpr bool kOut1 = kBN == 192 && !kPlanes;  // one output staging buffer (see SmemT)
+    constexpr int kBRows = kPair ? kBN / 2 : kBN;  // columns of the result whose B rows this CTA loads
+    constexpr int kBTileBytes = kBRows * kBK * 4;
+    constexpr int kCtas = kPair ? 2 : 1;
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     if ((smem_u32(smem_raw) & 1023u) != 0) {
         if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE_SMEM_ALIGN);
@@ -142,29 +133,35 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WaitCtx ctx{&sm.abort_flag, status};
-    pdl_launch_dependents();
+    const int rank = kPair ? (int)cluster_rank() : 0;
+    const int first = (int)blockIdx.x / kCtas, step = (int)gridDim.x / kCtas;  // work items of this CTA or pair
 
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         for (int i = 0; i < kStages; i++) {
-            mbar_init(&sm.full[i], 1);
+            mbar_init(&sm.full[i], 1);  // a pair uses the leader's: its arrival, and the bytes of both CTAs
             mbar_init(&sm.empty[i], 1);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&sm.acc_full[i], 1);
-            mbar_init(&sm.acc_empty[i], kEpiThreads);
+            mbar_init(&sm.acc_empty[i], kEpiWarps * kCtas);  // one arrival per epilogue warp
         }
-        mbar_init(&sm.out_ready, kEpiThreads);
-        mbar_init(&sm.out_free, kDirect ? kEpiThreads : 1);
         fence_barrier_init();
     }
     if (warp == 2) {
-        tmem_alloc(&sm.tmem_base, kTmemCols);
-        tmem_relinquish();
+        if (kPair) {
+            tmem_alloc_pair(&sm.tmem_base, kTmemCols);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(&sm.tmem_base, kTmemCols);
+            tmem_relinquish();
+        }
     }
+    pdl_launch_dependents();
     pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();
-    __syncthreads();
+    if (kPair) cluster_sync_all();  // the other CTA's barriers are initialised too
+    else __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = sm.tmem_base;
 
@@ -175,50 +172,56 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             tma_prefetch_desc(&map_b);
             int it = 0;
             bool ok = true;
-            for (int w = blockIdx.x; ok && w < p.total; w += gridDim.x) {
-                const Work wk = decode(p, w);
+            for (int w = first; ok && w < p.total; w += step) {
+                const Work wk = decode<kPair>(p, w, rank);
                 for (int kb = wk.kb0; kb < wk.kb1; kb++, it++) {
                     const int st = it % kStages;
                     if (it >= kStages && !mbar_wait(&sm.empty[st], ((it / kStages) - 1) & 1, ctx, SITE_EMPTY)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(&sm.full[st], kATileBytes + kBTileBytes);
+                    if (rank == 0) mbar_expect_tx(&sm.full[st], kCtas * (kATileBytes + kBTileBytes));
+                    const uint32_t full_at = kPair ? mapa(smem_u32(&sm.full[st]), 0) : 0;
+                    auto load = [&](void *dst, const CUtensorMap *map, int c0, int c1, int c2) {
+                        if (kPair) tma_load_4d_pair(dst, map, full_at, c0, c1, c2, 0);
+                        else tma_load_4d(dst, map, &sm.full[st], c0, c1, c2, 0);
+                    };
+                    const int b0 = wk.n0 + rank * kBRows;
                     // K-major: map {contraction, rows}, one box {32, 128}.  MN-major: map {rows, contraction},
                     // four boxes {32, 32}: blocks of 32 rows, each [32 contraction steps x 128 bytes].
                     if (kAMN) {
                         if (p.a_one) {
-                            tma_load_4d(sm.a[st], &map_a, &sm.full[st], 0, kb * kBK, wk.m0 / 32, 0);
+                            load(sm.a[st], &map_a, 0, kb * kBK, wk.m0 / 32);
                         } else {
 #pragma unroll
                             for (int i = 0; i < 4; i++)
-                                tma_load_4d(sm.a[st] + i * 4096, &map_a, &sm.full[st], wk.m0 + 32 * i, kb * kBK, 0, 0);
+                                load(sm.a[st] + i * 4096, &map_a, wk.m0 + 32 * i, kb * kBK, 0);
                         }
                     } else {
-                        tma_load_4d(sm.a[st], &map_a, &sm.full[st], kb * kBK, wk.m0, 0, 0);
+                        load(sm.a[st], &map_a, kb * kBK, wk.m0, 0);
                     }
                     if (kBMN) {
                         if (p.b_one) {
-                            tma_load_4d(sm.b[st], &map_b, &sm.full[st], 0, kb * kBK, wk.n0 / 32, 0);
+                            load(sm.b[st], &map_b, 0, kb * kBK, b0 / 32);
                         } else {
 #pragma unroll
-                            for (int i = 0; i < kBN / 32; i++)
-                                tma_load_4d(sm.b[st] + i * 4096, &map_b, &sm.full[st], wk.n0 + 32 * i, kb * kBK, 0, 0);
+                            for (int i = 0; i < kBRows / 32; i++)
+                                load(sm.b[st] + i * 4096, &map_b, b0 + 32 * i, kb * kBK, 0);
                         }
                     } else {
-                        tma_load_4d(sm.b[st], &map_b, &sm.full[st], kb * kBK, wk.n0, 0, 0);  // the B map's box is kBN rows
+                        load(sm.b[st], &map_b, kb * kBK, b0, 0);  // the B map's box is kBRows rows
                     }
                 }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 && rank == 0) {
         // ------------------------------ MMA issuer ------------------------------
-        constexpr uint32_t idesc = idesc_tf32(kBM, kBN, kAMN ? 1 : 0, kBMN ? 1 : 0);
+        constexpr uint32_t idesc = idesc_tf32(kBM * kCtas, kBN, kAMN ? 1 : 0, kBMN ? 1 : 0);
         const uint32_t leader = elect_leader();
         int it = 0, j = 0;
         bool ok = true;
-        for (int w = blockIdx.x; ok && w < p.total; w += gridDim.x, j++) {
-            const Work wk = decode(p, w);
+        for (int w = first; ok && w < p.total; w += step, j++) {
+            const Work wk = decode<kPair>(p, w, rank);
             const int acc = j & 1;
             if (j >= 2 && !mbar_wait_warp(&sm.acc_empty[acc], ((j >> 1) - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
             tc_fence_after_sync();
@@ -236,208 +239,117 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const uint64_t bd = kBMN ? smem_desc_sw128_base32(smem_u32(sm.b[st]), 4096, 512)
                                          : smem_desc_sw128(smem_u32(sm.b[st]), 16, 1024);
 #pragma unroll
-                for (int k = 0; k < kBK / 8; k++)
-                    mma_tf32_lead(leader, d, desc_advance(ad, k * (kAMN ? 1024 : 32)),
-                                  desc_advance(bd, k * (kBMN ? 1024 : 32)), idesc, (kb > wk.kb0 || k > 0) ? 1u : 0u);
-                tc_commit_lead(leader, &sm.empty[st]);
+                for (int k = 0; k < kBK / 8; k++) {
+                    const uint64_t ak = desc_advance(ad, k * (kAMN ? 1024 : 32)), bk = desc_advance(bd, k * (kBMN ? 1024 : 32));
+                    const uint32_t add = (kb > wk.kb0 || k > 0) ? 1u : 0u;
+                    if (kPair) mma_tf32_pair_lead(leader, d, ak, bk, idesc, add);
+                    else mma_tf32_lead(leader, d, ak, bk, idesc, add);
+                }
+                if (kPair) tc_commit_pair_lead(leader, &sm.empty[st]);
+                else tc_commit_lead(leader, &sm.empty[st]);
             }
-            if (ok) tc_commit_lead(leader, &sm.acc_full[acc]);
+            if (!ok) break;
+            if (kPair) tc_commit_pair_lead(leader, &sm.acc_full[acc]);
+            else tc_commit_lead(leader, &sm.acc_full[acc]);
         }
     } else if (warp >= 4) {
         // ------------------------------ epilogue ------------------------------
-        // Two warps per tensor-memory lane quarter: each thread owns one row and 32 of the 64 columns
-        // of a chunk.  Warp 3 drives the copy engine.
+        // Every warp takes 32 rows (its tensor-memory lane quarter) and half of the columns, 32 at a time, through
+        // a staging buffer of its own: accumulator -> registers (+ bias) -> shared memory -> copy engine.  No warp
+        // waits for another one.
         const int quarter = warp & 3;
         const int half = (warp - 4) >> 2;
-        const int row = (quarter << 5) | lane;
+        uint8_t *buf = sm.out[kEpi == 1 || kDirect ? warp - 4 : 0];
         const uint32_t lane_addr = (uint32_t)(quarter << 5) << 16;
-        int j = 0, chunk_count = 0;
-        int sub = 0;  // stagings handed to the copy engine so far (one per chunk, two with the planes)
-        bool ok = true;
-        for (int w = blockIdx.x; ok && w < p.total; w += gridDim.x, j++) {
-            const Work wk = decode(p, w);
+        constexpr int kChunks = kBN / 64;
+        int j = 0;
+        for (int w = first; w < p.total; w += step, j++) {
+            const Work wk = decode<kPair>(p, w, rank);
             const int acc = j & 1;
+            const int row0 = wk.m0 + 32 * quarter;
+            float bv[kChunks];  // bias of the columns col0 + lane, fetched while the tile is still being computed
+#pragma unroll
+            for (int c = 0; c < kChunks; c++) {
+                const int col = wk.n0 + half * (kBN / 2) + 32 * c + lane;
+                bv[c] = kEpi == 0 && bias != nullptr && col < p.N ? __ldg(bias + col) : 0.f;
+            }
             if (!mbar_wait_warp(&sm.acc_full[acc], (j >> 1) & 1, ctx, SITE_ACC_FULL)) break;
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < kBN / 64; c++, chunk_count++) {
-                const int col0 = wk.n0 + 64 * c + 32 * half;  // first of this thread's 32 columns
-                uint32_t r2[2][16];
-#define R(i) r2[(i) >> 4][(i) & 15]
-#pragma unroll
-                for (int q = 0; q < 2; q++)
-                    tmem_ld16(tmem + lane_addr + (uint32_t)acc * kBN + 64 * c + 32 * half + 16 * q, r2[q]);
+            for (int c = 0; c < kChunks; c++) {
+                const int off = half * (kBN / 2) + 32 * c, col0 = wk.n0 + off;
+                uint32_t r[32];
+                tmem_ld32(tmem + lane_addr + (uint32_t)acc * kBN + off, r);
                 tmem_wait_ld();
-                if (c == kBN / 64 - 1) {  // the accumulator has been read out: the tensor cores may reuse it
+                if (c == kChunks - 1) {  // the accumulator has been read out: the tensor cores may reuse it
                     tc_fence_before_sync();
-                    mbar_arrive(&sm.acc_empty[acc]);
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (kPair) mbar_arrive_cluster(mapa(smem_u32(&sm.acc_empty[acc]), 0));
+                        else mbar_arrive(&sm.acc_empty[acc]);
+                    }
                 }
                 if (kEpi == 0 && bias != nullptr) {
+                    const float mine = c == 0 ? bv[0] : c == 1 ? bv[1] : c == 2 ? bv[2 % kChunks] : bv[3 % kChunks];
 #pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        if (kDirect) {  // N need not be a multiple of 4: element-wise and guarded
-#pragma unroll
-                            for (int e = 0; e < 4; e++)
-                                if (col0 + 4 * q + e < p.N)
-                                    R(4 * q + e) = __float_as_uint(__uint_as_float(R(4 * q + e)) + __ldg(bias + col0 + 4 * q + e));
-                        } else if (col0 + 4 * q < p.N) {  // N is a multiple of 4
-                            const float4 bv = __ldg(reinterpret_cast<const float4 *>(bias + col0) + q);
-                            R(4 * q) = __float_as_uint(__uint_as_float(R(4 * q)) + bv.x);
-                            R(4 * q + 1) = __float_as_uint(__uint_as_float(R(4 * q + 1)) + bv.y);
-                            R(4 * q + 2) = __float_as_uint(__uint_as_float(R(4 * q + 2)) + bv.z);
-                            R(4 * q + 3) = __float_as_uint(__uint_as_float(R(4 * q + 3)) + bv.w);
-                        }
-                    }
+                    for (int e = 0; e < 32; e++)
+                        r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, mine, e));
                 }
-                uint32_t hp[16], lp[16];  // packed bf16 pairs of the two planes
-                if (kEpi == 0 && kPlanes) {
+                if (kEpi == 0 && !kDirect) {
+                    // straight from the registers: this lane's row, 32-byte sectors
+                    const int row = row0 + lane;
+                    if (row < p.M) {
+                        store_words<8>(c_direct + (size_t)row * p.N + col0, p.N - col0, p.wide, r);
+                        if (kPlanes) {
+                            uint32_t hp[16], lp[16];
 #pragma unroll
-                    for (int e = 0; e < 16; e++) {
-                        const float f0 = __uint_as_float(R(2 * e)), f1 = __uint_as_float(R(2 * e + 1));
-                        const __nv_bfloat162 hh = __floats2bfloat162_rn(f0, f1);
-                        const __nv_bfloat162 ll = __floats2bfloat162_rn(f0 - __low2float(hh), f1 - __high2float(hh));
-                        hp[e] = *reinterpret_cast<const uint32_t *>(&hh);
-                        lp[e] = *reinterpret_cast<const uint32_t *>(&ll);
-                    }
-                }
-                if (kOut1) {
-                    // one staging buffer: the two column halves of the chunk go through it one after the other
-#pragma unroll 1
-                    for (int hsel = 0; hsel < 2; hsel++) {
-                        if (sub >= 1 && !mbar_wait_warp(&sm.out_free, (sub - 1) & 1, ctx, SITE_OUT_FREE)) {
-                            ok = false;
-                            break;
+                            for (int e = 0; e < 16; e++)
+                                split_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]), hp[e], lp[e]);
+                            uint32_t *hi = planes + ((size_t)row * p.N + col0) / 2;
+                            store_words<4>(hi, (p.N - col0) / 2, p.wide_planes, hp);
+                            store_words<4>(hi + p.plane_words, (p.N - col0) / 2, p.wide_planes, lp);
                         }
-                        if (half == hsel) {
-#pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                uint8_t *dst = sm.out[0] + row * 128 + ((q ^ (row & 7)) << 4);
-                                *reinterpret_cast<uint4 *>(dst) = make_uint4(R(4 * q), R(4 * q + 1), R(4 * q + 2), R(4 * q + 3));
-                            }
-                        }
-                        fence_proxy_async_smem();
-                        mbar_arrive(&sm.out_ready);
-                        sub++;
                     }
-                    if (!ok) break;
                     continue;
                 }
-                // the copy engine must have read the previous staging out of the two buffers
-                if (sub >= 1 && !mbar_wait_warp(&sm.out_free, (sub - 1) & 1, ctx, SITE_OUT_FREE)) {
-                    ok = false;
-                    break;
-                }
+                if (!kDirect && lane == 0) bulk_wait_read_all();  // the copy engine has read the buffer out
+                __syncwarp();
 #pragma unroll
-                for (int q = 0; q < 8; q++) {  // fp32: this half's box of 32 columns, 8 chunks of 16 bytes per row
-                    uint8_t *dst = sm.out[kOut1 ? 0 : half] + row * 128 + ((q ^ (row & 7)) << 4);
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(R(4 * q), R(4 * q + 1), R(4 * q + 2), R(4 * q + 3));
-                }
-#undef R
+                for (int q = 0; q < 8; q++)  // one row of 128 bytes per lane, 16-byte words swizzled
+                    *reinterpret_cast<uint4 *>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                        make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
                 if (kDirect) {
-                    // every row of the staged chunk is written by one warp instruction: 32 consecutive floats
-                    mbar_arrive(&sm.out_ready);
-                    if (!mbar_wait_warp(&sm.out_ready, sub & 1, ctx, SITE_OUT_READY)) {
-                        ok = false;
-                        break;
+                    // every row leaves as 32 consecutive floats in one warp instruction
+                    __syncwarp();
+#pragma unroll 8
+                    for (int rr = 0; rr < 32; rr++) {
+                        const float v = *reinterpret_cast<const float *>(buf + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) +
+                                                                         ((lane & 3) << 2));
+                        if (row0 + rr < p.M && col0 + lane < p.N) c_direct[(size_t)(row0 + rr) * p.N + col0 + lane] = v;
                     }
-                    const int et = threadIdx.x - 128;  // 0..255
-                    const int cbase = wk.n0 + 64 * c;
-#pragma unroll 4
-                    for (int k = 0; k < (128 * 64) / kEpiThreads; k++) {
-                        const int e = et + kEpiThreads * k;
-                        const int rr = e >> 6, cc = e & 63;
-                        const float v = *reinterpret_cast<const float *>(sm.out[kOut1 ? 0 : (cc >> 5)] + rr * 128 +
-                                                                         ((((cc & 31) >> 2) ^ (rr & 7)) << 4) + ((cc & 3) << 2));
-                        if (wk.m0 + rr < p.M && cbase + cc < p.N) c_direct[(size_t)(wk.m0 + rr) * p.N + cbase + cc] = v;
-                    }
-                    mbar_arrive(&sm.out_free);
-                    sub++;
-                } else {
-                    fence_proxy_async_smem();
-                    mbar_arrive(&sm.out_ready);
-                    sub++;
-                    if (kEpi == 0 && kPlanes) {
-                        // second round: once the fp32 tiles have been read, the same buffers take the planes
-                        if (!mbar_wait_warp(&sm.out_free, (sub - 1) & 1, ctx, SITE_OUT_FREE)) {
-                            ok = false;
-                            break;
-                        }
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {  // this half's 32 columns = 4 chunks of 8 bf16 values
-                            const int off = row * 128 + (((4 * half + q) ^ (row & 7)) << 4);
-                            *reinterpret_cast<uint4 *>(sm.out[0] + off) =
-                                make_uint4(hp[4 * q], hp[4 * q + 1], hp[4 * q + 2], hp[4 * q + 3]);
-                            *reinterpret_cast<uint4 *>(sm.out[kOut1 ? 0 : 1] + off) =
-                                make_uint4(lp[4 * q], lp[4 * q + 1], lp[4 * q + 2], lp[4 * q + 3]);
-                        }
-                        fence_proxy_async_smem();
-                        mbar_arrive(&sm.out_ready);
-                        sub++;
-                    }
+                    continue;
                 }
-            }
-        }
-    } else if (warp == 3 && !kDirect) {
-        // ------------------------------ output copies ------------------------------
-        if (lane == 0) {
-            int sub = 0;
-            bool ok = true;
-            for (int w = blockIdx.x; ok && w < p.total; w += gridDim.x) {
-                const Work wk = decode(p, w);
-                for (int c = 0; c < kBN / 64; c++) {
-                    const int col0 = wk.n0 + 64 * c;
-                    if (!mbar_wait(&sm.out_ready, sub & 1, ctx, SITE_OUT_READY)) {
-                        ok = false;
-                        break;
-                    }
-                    sub++;
-                    if (kOut1) {  // one buffer, two rounds of 32 columns
-                        if (kEpi == 0) tma_store_3d(sm.out[0], &map_c, col0, wk.m0, 0);
-                        else tma_reduce_add_3d(sm.out[0], &map_c, col0, wk.m0, 0);
-                        bulk_commit();
-                        bulk_wait_read_all();
-                        mbar_arrive(&sm.out_free);
-                        if (!mbar_wait(&sm.out_ready, sub & 1, ctx, SITE_OUT_READY)) {
-                            ok = false;
-                            break;
-                        }
-                        sub++;
-                        if (kEpi == 0) tma_store_3d(sm.out[0], &map_c, col0 + 32, wk.m0, 0);
-                        else tma_reduce_add_3d(sm.out[0], &map_c, col0 + 32, wk.m0, 0);
-                    } else if (kEpi == 0) {
-                        tma_store_3d(sm.out[0], &map_c, col0, wk.m0, 0);
-                        tma_store_3d(sm.out[kOut1 ? 0 : 1], &map_c, col0 + 32, wk.m0, 0);
-                        if (kPlanes) {  // second round through the same buffers: hi plane, lo plane
-                            bulk_commit();
-                            bulk_wait_read_all();
-                            mbar_arrive(&sm.out_free);
-                            if (!mbar_wait(&sm.out_ready, sub & 1, ctx, SITE_OUT_READY)) {
-                                ok = false;
-                                break;
-                            }
-                            sub++;
-                            tma_store_3d(sm.out[0], &map_planes, col0, wk.m0, 0);
-                            tma_store_3d(sm.out[kOut1 ? 0 : 1], &map_planes, col0, wk.m0, 1);
-                        }
-                    } else {
-                        tma_reduce_add_3d(sm.out[0], &map_c, col0, wk.m0, 0);
-                        tma_reduce_add_3d(sm.out[kOut1 ? 0 : 1], &map_c, col0 + 32, wk.m0, 0);
-                    }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_reduce_add_3d(buf, &map_c, col0, row0, 0);
                     bulk_commit();
-                    bulk_wait_read_all();
-                    mbar_arrive(&sm.out_free);
                 }
             }
         }
+        if (kEpi == 1 && lane == 0) bulk_wait_read_all();  // shared memory stays until it has been read
     }
 
     // ------------------------------ tear-down ------------------------------
     if (sm.abort_flag) __nanosleep(50000);
     tc_fence_before_sync();
+    // neither CTA of a pair leaves, or frees tensor memory, while the other may still signal or compute into it
     __syncthreads();
+    if (kPair) cluster_sync_all();
     if (warp == 2) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem, kTmemCols);
+        if (kPair) tmem_dealloc_pair(tmem, kTmemCols);
+        else tmem_dealloc(tmem, kTmemCols);
     }
 }
 
@@ -536,52 +448,20 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(float *__restrict__ dst, 
 
 // ---- host side ----
 
-// Operand read K-major: matrix [rows, kc] row-major (kc contiguous = contraction); boxes of 32 x box_rows.
-int map_k_major(CUtensorMap *map, const float *base, int rows, int kc, int box_rows) {
-    const cuuint64_t dims[4] = {(cuuint64_t)kc, (cuuint64_t)rows, 1, 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)kc * 4, (cuuint64_t)kc * 4 * (cuuint64_t)rows, (cuuint64_t)kc * 4 * (cuuint64_t)rows};
-    const cuuint32_t box[4] = {32, (cuuint32_t)box_rows, 1, 1};
-    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box);
-}
-// Operand read MN-major, whole tile in one copy: the matrix [kc, rows] seen as {32 values, kc, rows / 32 blocks}
-// with the block index as the slowest box dimension, box {32, 32, nblocks}: shared memory receives
-// [block][contraction step][32 values], the layout the descriptor expects.  rows % 32 == 0.
-int map_mn_major_blocks(CUtensorMap *map, const float *base, int kc, int rows, int nblocks) {
-    const cuuint64_t dims[4] = {32, (cuuint64_t)kc, (cuuint64_t)(rows / 32), 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)rows * 4, 128, (cuuint64_t)rows * 4 * (cuuint64_t)kc};
-    const cuuint32_t box[4] = {32, 32, (cuuint32_t)nblocks, 1};
-    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
-                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
-}
-// Operand read MN-major: matrix [kc, rows] row-major (rows contiguous, kc = contraction), boxes of 32 x 32.
-int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows) {
-    const cuuint64_t dims[4] = {(cuuint64_t)rows, (cuuint64_t)kc, 1, 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)rows * 4, (cuuint64_t)rows * 4 * (cuuint64_t)kc, (cuuint64_t)rows * 4 * (cuuint64_t)kc};
-    const cuuint32_t box[4] = {32, 32, 1, 1};
-    // 32-bit operands read MN-major need the 128-byte swizzle with 32-byte atoms (rows of 128 bytes, the
-    // 32-byte quarter of a row XORed with the row index modulo 4)
-    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
-                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
-}
 int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols) {
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
     const cuuint64_t strides[2] = {(cuuint64_t)cols * 4, (cuuint64_t)cols * 4 * (cuuint64_t)rows};
-    const cuuint32_t box[3] = {32, 128, 1};
+    const cuuint32_t box[3] = {32, 32, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
 }
-int map_out_planes(CUtensorMap *map, const void *base, int rows, int cols) {
-    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 2};
-    const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)attn::plane_bytes((size_t)rows * cols)};
-    const cuuint32_t box[3] = {64, 128, 1};
-    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box);
-}
+int tile_rows(int pair) { return pair ? 2 * kBM : kBM; }
 
-Problem make_problem(int M, int N, int K, int bn, int splits) {
+Problem make_problem(int M, int N, int K, int bn, int pair, int splits) {
     Problem p;
-    p.M = M, p.N = N, p.K = K, p.bn = bn;
+    p.M = M, p.N = N, p.K = K, p.bn = bn, p.pair = pair;
     p.a_one = p.b_one = 0;
     p.m_fast = 0;
-    p.tiles_m = (M + kBM - 1) / kBM;
+    p.tiles_m = (M + tile_rows(pair) - 1) / tile_rows(pair);
     p.tiles_n = (N + bn - 1) / bn;
     p.kb_total = (K + kBK - 1) / kBK;
     if (splits < 1) splits = 1;
@@ -598,58 +478,110 @@ int sm_count() {
     return sms;
 }
 
-// Tile width for a [M, N] result: the candidate with the fewest (rounds over the SMs) x (tile width),
-// with a fixed charge per tile that makes narrow tiles pay for their higher operand traffic per flop.
-int pick_bn(int M, int N, int splits, int sms) {
-    const int cand[3] = {256, 192, 128};
-    int best = 128;
-    long long best_cost = -1;
-    for (int i = 0; i < 3; i++) {
-        const int bn = cand[i];
-        if (bn > 128 && N < bn) continue;
-        const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + bn - 1) / bn) * splits;
-        const long long rounds = (tiles + sms - 1) / sms;
-        const long long cost = rounds * (bn + 192);  // measured: a 192-wide tile costs ~0.9 of a 256-wide one
-        if (best_cost < 0 || cost < best_cost) best = bn, best_cost = cost;
+// Tile shape and number of pieces of the contraction for a [M, N] result of kb contraction blocks, chosen by expected
+// time: rounds over the SMs (or pairs) x (a charge per round + contraction blocks x nanoseconds per block) + a fixed
+// part.  The constants are a fit to the kernel's measured times on 224 shapes of 100 to 8192 rows and 512 to 6400
+// columns (mean error 5 %; the choice is within 1 % of the best of the six on average).  What stands behind them: a
+// block of a 256 x 256 tile takes its 512 tensor-core cycles, narrower or single-CTA tiles are bound by the
+// 12 to 17 TB/s at which L2 feeds the SMs and cost nearly as much per block.
+struct Plan {
+    int pair, bn, splits;
+    int ns;
+};
+struct Cost {
+    int pair, bn, fixed, round, block;
+};
+constexpr Cost kCosts[6] = {{1, 256, 4890, 2250, 306}, {1, 192, 4300, 1580, 272}, {1, 128, 4220, 840, 262},
+                            {0, 256, 860, 4770, 316},  {0, 192, 1360, 3230, 262}, {0, 128, 2690, 1300, 238}};
+
+// What does not fit in L2 arrives from HBM at 5.0 TB/s, after a start of 6 us.
+Plan plan_tiles(int M, int N, int kb, int sms) {
+    Plan best{0, 128, 1, 0};
+    const long long bytes = 4ll * ((long long)M * N + (long long)kb * kBK * (M + N));
+    const long long least = bytes > (100ll << 20) ? 6000 + bytes / 5000 : 0;
+    for (const Cost &c : kCosts) {
+        if (c.bn > 128 && N < c.bn) continue;
+        const long long tiles = (long long)((M + tile_rows(c.pair) - 1) / tile_rows(c.pair)) * ((N + c.bn - 1) / c.bn);
+        const int units = c.pair ? sms / 2 : sms;
+        long long t = c.fixed + (tiles + units - 1) / units * (c.round + (long long)kb * c.block);
+        if (t < least) t = least;
+        if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, 1, (int)(t < 0x7fffffff ? t : 0x7fffffff)};
     }
     return best;
 }
 
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect = false>
-int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const CUtensorMap &mp,
-               const float *bias, const Problem &p, int *status, cudaStream_t s, float *c_direct = nullptr) {
-    using Smem = SmemT<kBN, kStages, kPlanes>;
+// The same with the contraction cut into up to 32 pieces that add into the result with bulk reductions (dW, and dx when
+// its contraction is very long); those cost 43 (pairs) or 80 ns per megabyte and make a block 15 % slower.
+Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks) {
+    Plan best{0, 128, 1, 0};
+    for (const Cost &c : kCosts) {
+        if (c.bn > 128 && N < c.bn) continue;
+        const long long tiles = (long long)((M + tile_rows(c.pair) - 1) / tile_rows(c.pair)) * ((N + c.bn - 1) / c.bn);
+        const int units = c.pair ? sms / 2 : sms;
+        const long long tile_bytes = (long long)tile_rows(c.pair) * c.bn * 4;
+        for (int s = 1; s <= 32 && s <= kb; s++) {
+            const int per = (kb + s - 1) / s;
+            if (s > 1 && per < least_blocks) break;
+            const long long rounds = (tiles * s + units - 1) / units;
+            const long long t = (c.pair ? 5800 : 4200) + rounds * ((c.pair ? 550 : 160) + (long long)per * c.block * 115 / 100) +
+                                tiles * s * tile_bytes / 1000 * (c.pair ? 43 : 80) / 1000;
+            if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, s, (int)(t < 0x7fffffff ? t : 0x7fffffff)};
+        }
+    }
+    return best;
+}
+
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
+int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
+               Problem p, int *status, cudaStream_t s) {
+    using Smem = SmemT<kBN, kStages, kPair, kEpi == 1 || kDirect>;
     static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear kernel");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect>;
+    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair>;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return (int)e;
         attr_done[dev] = true;
     }
-    const int sms = sm_count();
-    const int grid = p.total < sms ? p.total : sms;
-    return (int)attn::launch_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), s, ma, mb, mc, mp, bias, c_direct, p,
-                                            status);
+    p.wide = p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(c) & 31u) == 0;
+    p.wide_planes = p.N % 16 == 0 && (reinterpret_cast<uintptr_t>(planes) & 31u) == 0;
+    p.plane_words = attn::plane_bytes((size_t)p.M * p.N) / 4;
+    constexpr int kCtas = kPair ? 2 : 1;
+    const int most = sm_count() / kCtas;
+    const int grid = (p.total < most ? p.total : most) * kCtas;
+    return (int)attn::launch_clusters_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), kCtas, s, ma, mb, mc, bias, c,
+                                                     static_cast<uint32_t *>(planes), p, status);
 }
 
 // Pipeline depth by what fits in 227 KiB next to the output staging tile.
 template <bool kAMN, bool kBMN, int kEpi>
-int launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const CUtensorMap &mp, const float *bias,
-           bool planes, const Problem &p, int *status, cudaStream_t s) {
-    if (p.bn == 256) {
-        if (planes) return launch_one<kAMN, kBMN, kEpi, 256, 4, true>(ma, mb, mc, mp, bias, p, status, s);
-        return launch_one<kAMN, kBMN, kEpi, 256, 4, false>(ma, mb, mc, mp, bias, p, status, s);
+int launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
+           const Problem &p, int *status, cudaStream_t s) {
+#define GO(bn, stages, with_planes, pair) \
+    return launch_one<kAMN, kBMN, kEpi, bn, stages, with_planes, false, pair>(ma, mb, mc, bias, c, planes, p, status, s)
+    constexpr bool kCanPlanes = !kAMN && !kBMN && kEpi == 0;  // only the forward product writes planes
+    if (p.pair) {
+        if constexpr (kCanPlanes) {
+            if (planes && p.bn == 256) GO(256, 7, true, true);
+            if (planes && p.bn == 192) GO(192, 7, true, true);
+            if (planes) GO(128, 6, true, true);
+        }
+        if (p.bn == 256) GO(256, kEpi == 1 ? 6 : 7, false, true);
+        if (p.bn == 192) GO(192, kEpi == 1 ? 6 : 7, false, true);
+        GO(128, 6, false, true);
     }
-    if (p.bn == 192) {
-        if (planes) return launch_one<kAMN, kBMN, kEpi, 192, 4, true>(ma, mb, mc, mp, bias, p, status, s);
-        return launch_one<kAMN, kBMN, kEpi, 192, 5, false>(ma, mb, mc, mp, bias, p, status, s);
+    if constexpr (kCanPlanes) {
+        if (planes && p.bn == 256) GO(256, 4, true, false);
+        if (planes && p.bn == 192) GO(192, 5, true, false);
+        if (planes) GO(128, 6, true, false);
     }
-    if (planes) return launch_one<kAMN, kBMN, kEpi, 128, 6, true>(ma, mb, mc, mp, bias, p, status, s);
-    return launch_one<kAMN, kBMN, kEpi, 128, 6, false>(ma, mb, mc, mp, bias, p, status, s);
+    if (p.bn == 256) GO(256, 4, false, false);
+    if (p.bn == 192) GO(192, kEpi == 1 ? 4 : 5, false, false);
+    GO(128, 6, false, false);
+#undef GO
 }
 
 // C[M, N] = A[M, K] . B[N, K]^T: true when B (the weight) is too large to stay in L2 while every tile row of
@@ -660,34 +592,30 @@ int stream_rows_of_c(int M, int N, int K) {
     return b_bytes > ((size_t)48 << 20) && b_bytes > a_bytes ? 1 : 0;
 }
 
-// Number of pieces the contraction of a [M, N] result is cut into when it is very long and the tiles do not
-// fill the SMs evenly (dx of the vocabulary projection: 192 tiles on 148 SMs, 1571 steps each).  Each piece
-// pays a fixed charge for its epilogue; 1 = no split.
-int pick_splits(int tiles, int kb_total, int sms) {
-    if (kb_total < 512) return 1;
-    int best = 1;
-    long long best_cost = -1;
-    for (int s = 1; s <= 8; s++) {
-        const long long rounds = ((long long)tiles * s + sms - 1) / sms;
-        const long long cost = rounds * ((kb_total + s - 1) / s + 24);
-        if (best_cost < 0 || cost < best_cost) best = s, best_cost = cost;
-    }
-    return best;
-}
-
-// The same choice for dW, whose contraction (the rows of dy) is always cut: up to 32 pieces.
-int pick_splits_dw(int tiles, int kb_total, int sms, int overhead) {
-    int best = 1;
-    long long best_cost = -1;
-    for (int s = 1; s <= 32 && s <= kb_total; s++) {
-        const long long rounds = ((long long)tiles * s + sms - 1) / sms;
-        const long long cost = rounds * ((kb_total + s - 1) / s + overhead);
-        if (best_cost < 0 || cost < best_cost) best = s, best_cost = cost;
-    }
-    return best;
-}
-
 bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
+
+// dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
+int input_gradient(const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status, cudaStream_t s) {
+    const int kb = np / kBK;
+    Plan plan = plan_tiles(M, K, kb, sms);
+    if (kb >= 512) {  // very long (the vocabulary projection): pieces may pay, although dx has to be zeroed first
+        Plan cut = plan_pieces(M, K, kb, sms, 32);
+        cut.ns += 2500 + (int)((long long)M * K * 4 / 5500);
+        if (cut.splits > 1 && cut.ns < plan.ns) plan = cut;
+    }
+    int split = 1, rc;
+    if (plan_split(M, K, np, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, status, s);
+    CUtensorMap ma, mb, mc;
+    Problem p = make_problem(M, K, np, plan.bn, plan.pair, plan.splits);
+    if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
+    p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 / (p.pair ? 2 : 1)) == 0;
+    if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
+    if (p.splits == 1) return launch<false, true, 0>(ma, mb, ma, nullptr, dx, nullptr, p, status, s);
+    // the pieces of the contraction add into dx with bulk reductions: start from zeros
+    if ((rc = map_out_f32(&mc, dx, M, K)) != 0) return rc;
+    if ((rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
+    return launch<false, true, 1>(ma, mb, mc, nullptr, dx, nullptr, p, status, s);
+}
 
 }  // namespace
 }  // namespace lin
@@ -707,22 +635,21 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     int *status = nullptr;
     int rc = attn::device_status_word(&status);
     if (rc != ATTN_OK) return rc;
-    CUtensorMap ma, mb, mc, mp;
-    const int bn = direct ? 256 : pick_bn(M, N, 1, sm_count());
-    if ((rc = map_k_major(&ma, x, M, K, 128)) != 0) return rc;
-    if ((rc = map_k_major(&mb, w, N, K, bn)) != 0) return rc;
-    if (direct) {
-        Problem pd = make_problem(M, N, K, 256, 1);
-        pd.m_fast = stream_rows_of_c(M, N, K);
-        return launch_one<false, false, 0, 256, 4, false, true>(ma, mb, ma, ma, bias, pd, status,
-                                                                static_cast<cudaStream_t>(stream), y);
-    }
-    if ((rc = map_out_f32(&mc, y, M, N)) != 0) return rc;
-    mp = mc;
-    if (planes && (rc = map_out_planes(&mp, planes, M, N)) != 0) return rc;
-    Problem p = make_problem(M, N, K, bn, 1);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const Plan plan = plan_tiles(M, N, (K + kBK - 1) / kBK, sm_count());
+    int split = 1;
+    if (plan_split(M, N, K, &split) < plan.ns) return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, status, s);
+    CUtensorMap ma, mb;
+    // with plain stores (N not a multiple of 4) only the widest tiles are built
+    Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, direct ? M > kBM : plan.pair, 1);
     p.m_fast = stream_rows_of_c(M, N, K);
-    return launch<false, false, 0>(ma, mb, mc, mp, bias, planes != nullptr, p, status, static_cast<cudaStream_t>(stream));
+    if ((rc = map_k_major(&ma, x, M, K, 128)) != 0) return rc;
+    if ((rc = map_k_major(&mb, w, N, K, p.bn / (p.pair ? 2 : 1))) != 0) return rc;
+    if (direct) {
+        if (p.pair) return launch_one<false, false, 0, 256, 6, false, true, true>(ma, mb, ma, bias, y, nullptr, p, status, s);
+        return launch_one<false, false, 0, 256, 4, false, true, false>(ma, mb, ma, bias, y, nullptr, p, status, s);
+    }
+    return launch<false, false, 0>(ma, mb, ma, bias, y, planes, p, status, s);
 }
 
 size_t linear_sm100_backward_scratch_bytes(int M, int N, int K) {
@@ -758,51 +685,19 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         if (rc != 0) return rc;
         g = static_cast<const float *>(scratch);
     }
+    if (dx && (rc = input_gradient(g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
     CUtensorMap ma, mb, mc;
-    if (dx) {
-        // dx[M,K] = dy[M,N] . w[N,K]: contraction over N (rows of w past N read as zeros)
-        if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
-        int bn_dx = pick_bn(M, K, 1, sms), splits_dx = 1;
-        if (np / kBK >= 512) {  // very long contraction: tile width and number of pieces together
-            const int cand[3] = {256, 192, 128};
-            long long best_cost = -1;
-            for (int i = 0; i < 3; i++) {
-                if (cand[i] > 128 && K < cand[i]) continue;
-                const int tiles = ((M + kBM - 1) / kBM) * ((K + cand[i] - 1) / cand[i]);
-                const int sp = pick_splits(tiles, np / kBK, sms);
-                const long long rounds = ((long long)tiles * sp + sms - 1) / sms;
-                const long long cost = rounds * ((np / kBK + sp - 1) / sp + 24) * (cand[i] + 192);
-                if (best_cost < 0 || cost < best_cost) best_cost = cost, bn_dx = cand[i], splits_dx = sp;
-            }
-        }
-        Problem pdx = make_problem(M, K, np, bn_dx, splits_dx);
-        pdx.b_one = map_mn_major_blocks(&mb, w, N, K, pdx.bn / 32) == 0;
-        if (!pdx.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
-        if ((rc = map_out_f32(&mc, dx, M, K)) != 0) return rc;
-        if (pdx.splits > 1) {
-            // the pieces of the contraction add into dx with bulk reductions: start from zeros
-            if ((rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, stream)) != 0) return rc;
-            rc = launch<false, true, 1>(ma, mb, mc, mc, nullptr, false, pdx, status, s);
-        } else {
-            rc = launch<false, true, 0>(ma, mb, mc, mc, nullptr, false, pdx, status, s);
-        }
-        if (rc != 0) return rc;
-    }
     if (dw) {
         // dw[N,K] += dy[M,N]^T . x[M,K]: contraction over M, split so that every SM has work (rows of the
         // result past N are dropped by the copy engine)
-        const int bn = K % 256 == 0 ? 256 : (K % 192 == 0 ? 192 : 128);
-        const int tiles = ((N + kBM - 1) / kBM) * ((K + bn - 1) / bn);
-        // pieces of the contraction: whole rounds over the SMs cost (steps per piece + a fixed charge for the
-        // piece's epilogue and reduction) each; e.g. QKV: 54 tiles, 256 steps -> 5 pieces in 2 rounds of 52 steps
-        const int splits = pick_splits_dw(tiles, (M + kBK - 1) / kBK, sms, 8);
-        Problem pdw = make_problem(N, K, M, bn, splits);
+        const Plan plan = plan_pieces(N, K, (M + kBK - 1) / kBK, sms, 1);
+        Problem pdw = make_problem(N, K, M, plan.bn, plan.pair, plan.splits);
         pdw.a_one = map_mn_major_blocks(&ma, g, M, np, 4) == 0;
         if (!pdw.a_one && (rc = map_mn_major(&ma, g, M, np)) != 0) return rc;
-        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, bn / 32) == 0;
+        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32 / (plan.pair ? 2 : 1)) == 0;
         if (!pdw.b_one && (rc = map_mn_major(&mb, x, M, K)) != 0) return rc;
         if ((rc = map_out_f32(&mc, dw, N, K)) != 0) return rc;
-        rc = launch<true, true, 1>(ma, mb, mc, mc, nullptr, false, pdw, status, s);
+        rc = launch<true, true, 1>(ma, mb, mc, nullptr, dw, nullptr, pdw, status, s);
         if (rc != 0) return rc;
     }
     if (db) {

@@ -1,0 +1,94 @@
+// What the two Linear kernels share: TF32 tensor-core instructions, operand descriptors and tensor maps.
+#pragma once
+
+#include "attn_internal.h"
+#include "tc05.cuh"
+
+namespace lin {
+
+constexpr int kBM = 128, kBK = 32;
+constexpr int kATileBytes = kBM * kBK * 4;  // A tile of one stage: 16 KiB
+
+// Instruction descriptor for kind::tf32 (A and B formats = 2), fp32 accumulation.
+__host__ __device__ constexpr uint32_t idesc_tf32(int M, int N, int a_mn_major, int b_mn_major) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) |
+           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_tf32_pair_lead(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                   uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+        "}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
+}
+
+__device__ __forceinline__ void mma_tf32_lead(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                              uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+        "}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
+}
+
+// Shared-memory descriptor for 32-bit operands read MN-major: layout type 1 (128-byte swizzle with
+// 32-byte atoms); rows of 32 values along M/N, LBO = distance between 32-value blocks, SBO = distance
+// between groups of 4 contraction steps.
+__device__ __forceinline__ uint64_t smem_desc_sw128_base32(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
+    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)1 << 61;
+    return d;
+}
+
+// ---- host side ----
+
+// Operand read K-major: matrix [rows, kc] row-major (kc contiguous = contraction); boxes of 32 x box_rows.
+inline int map_k_major(CUtensorMap *map, const float *base, int rows, int kc, int box_rows) {
+    const cuuint64_t dims[4] = {(cuuint64_t)kc, (cuuint64_t)rows, 1, 1};
+    const cuuint64_t strides[3] = {(cuuint64_t)kc * 4, (cuuint64_t)kc * 4 * (cuuint64_t)rows, (cuuint64_t)kc * 4 * (cuuint64_t)rows};
+    const cuuint32_t box[4] = {32, (cuuint32_t)box_rows, 1, 1};
+    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box);
+}
+// Operand read MN-major, whole tile in one copy: the matrix [kc, rows] seen as {32 values, kc, rows / 32 blocks}
+// with the block index as the slowest box dimension, box {32, 32, nblocks}: shared memory receives
+// [block][contraction step][32 values], the layout the descriptor expects.  rows % 32 == 0.
+inline int map_mn_major_blocks(CUtensorMap *map, const float *base, int kc, int rows, int nblocks) {
+    const cuuint64_t dims[4] = {32, (cuuint64_t)kc, (cuuint64_t)(rows / 32), 1};
+    const cuuint64_t strides[3] = {(cuuint64_t)rows * 4, 128, (cuuint64_t)rows * 4 * (cuuint64_t)kc};
+    const cuuint32_t box[4] = {32, 32, (cuuint32_t)nblocks, 1};
+    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
+                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
+}
+// Operand read MN-major: matrix [kc, rows] row-major (rows contiguous, kc = contraction), boxes of 32 x 32.
+inline int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows) {
+    const cuuint64_t dims[4] = {(cuuint64_t)rows, (cuuint64_t)kc, 1, 1};
+    const cuuint64_t strides[3] = {(cuuint64_t)rows * 4, (cuuint64_t)rows * 4 * (cuuint64_t)kc, (cuuint64_t)rows * 4 * (cuuint64_t)kc};
+    const cuuint32_t box[4] = {32, 32, 1, 1};
+    // 32-bit operands read MN-major need the 128-byte swizzle with 32-byte atoms (rows of 128 bytes, the
+    // 32-byte quarter of a row XORed with the row index modulo 4)
+    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
+                              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
+}
+// The kernel for results of few tiles (linear_split_sm100.cu): out[M, cols] = act[M, kc] . w^T + bias, with w [cols, kc],
+// or with w_mn_major [w_rows, cols] (its rows past w_rows, up to kc, read as zeros); optionally the bf16 planes of out.
+// `split` CTAs share the contraction of a tile.  Returns ATTN_OK or an error.
+int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, const float *bias, float *out, void *planes, int M,
+                 int cols, int kc, int split, int *status, cudaStream_t s);
+// The best `split` and the time in nanoseconds it is expected to take.
+int plan_split(int M, int cols, int kc, int *split);
+
+}  // namespace lin

@@ -106,6 +106,30 @@ def test_linear_backward_vs_cpu(pkg, M, N, K):
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (1, 96, 64), (16, 128, 32), (17, 260, 96),   # one tile of 16 or 32 activation rows, one CTA or two
+    (48, 1001, 128), (129, 384, 512), (250, 130, 1024), (348, 768, 3072),  # clusters of 6 and 8 CTAs, unaligned columns
+    (2600, 3000, 512), (6000, 1104, 256), (8192, 1152, 384), (3000, 520, 1600),  # CTA pairs 256 and 192 columns wide
+])
+def test_linear_tile_shapes(pkg, M, N, K):
+    """Forward with bias and planes, dx, dW and db where the choice of kernel, tile shape and split changes."""
+    x, w, b, dy = inputs(M, N, K, 47)
+    xt, wt, bt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, b, dy))
+    planes = torch.zeros(2 * ((M * N * 2 + 255) // 256 * 256), dtype=torch.uint8, device="cuda") if N % 8 == 0 else None
+    y = pkg.linear_forward(xt, wt, bt, planes=planes)
+    within(y.cpu().numpy(), ops.linear_forward(x, w, b), x, w.T)
+    if planes is not None:
+        hi, lo = (p[: M * N * 2].view(torch.bfloat16).view(M, N) for p in planes.chunk(2))
+        assert torch.equal(hi, y.bfloat16()) and torch.equal(lo, (y - hi.float()).bfloat16())
+    dw, db = torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda")
+    dx = pkg.linear_backward(dyt, xt, wt, dw, db)
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, np.zeros_like(w), np.zeros_like(b))
+    within(dx.cpu().numpy(), dx_ref, dy, w)
+    within(dw.cpu().numpy(), dw_ref, dy.T, x)
+    assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+
+
 def test_linear_backward_parts_can_be_skipped(pkg):
     M, N, K = 512, 768, 768
     x, w, b, dy = inputs(M, N, K, 31)
