@@ -479,20 +479,35 @@ int sm_count() {
 }
 
 // Tile shape and number of pieces of the contraction for a [M, N] result of kb contraction blocks, chosen by expected
-// time: rounds over the SMs (or pairs) x (a charge per round + contraction blocks x nanoseconds per block) + a fixed
-// part.  The constants are a fit to the kernel's measured times on 224 shapes of 100 to 8192 rows and 512 to 6400
-// columns (mean error 5 %; the choice is within 1 % of the best of the six on average).  What stands behind them: a
-// block of a 256 x 256 tile takes its 512 tensor-core cycles, narrower or single-CTA tiles are bound by the
-// 12 to 17 TB/s at which L2 feeds the SMs and cost nearly as much per block.
+// time: a fixed part, and for every round over the SMs (or pairs) a charge and kb blocks at the slower of what one
+// CTA takes when it is alone (`block`) and what L2 needs to feed all CTAs of the round.  The constants are a fit to
+// the kernel's times on 224 shapes of 100 to 8192 rows and 512 to 6400 columns (mean error 5 %; the choice is within
+// 1 % of the best of the six on average).  Wide pair tiles read the least per flop and win when there are many
+// tiles, narrow ones and single CTAs leave a smaller last round.
 struct Plan {
     int pair, bn, splits;
     int ns;
 };
 struct Cost {
-    int pair, bn, fixed, round, block;
+    int pair, bn, fixed, round, block;  // nanoseconds
 };
-constexpr Cost kCosts[6] = {{1, 256, 4890, 2250, 306}, {1, 192, 4300, 1580, 272}, {1, 128, 4220, 840, 262},
-                            {0, 256, 860, 4770, 316},  {0, 192, 1360, 3230, 262}, {0, 128, 2690, 1300, 238}};
+constexpr Cost kCosts[6] = {{1, 256, 5090, 2300, 298}, {1, 192, 4440, 1660, 264}, {1, 128, 4350, 840, 258},
+                            {0, 256, 4470, 2030, 283}, {0, 192, 4450, 900, 232},  {0, 128, 3920, 400, 226}};
+constexpr int kL2BytesPerNs = 18190;
+
+// Time of `tiles` tiles of kb contraction blocks each, without the fixed part.
+long long rounds_ns(const Cost &c, long long tiles, int kb, int sms) {
+    const int ctas = c.pair ? 2 : 1, units = sms / ctas;
+    const long long bytes = kATileBytes + (long long)c.bn / ctas * kBK * 4;  // a CTA's operands of one block
+    auto round = [&](long long busy) {
+        const long long fed = bytes * busy * ctas / kL2BytesPerNs;
+        return c.round + kb * (fed > c.block ? fed : c.block);
+    };
+    const long long rest = tiles % units;
+    return tiles / units * round(units) + (rest ? round(rest) : 0);
+}
+
+int at_most_int(long long v) { return v < 0x7fffffff ? (int)v : 0x7fffffff; }
 
 // What does not fit in L2 arrives from HBM at 5.0 TB/s, after a start of 6 us.
 Plan plan_tiles(int M, int N, int kb, int sms) {
@@ -502,10 +517,9 @@ Plan plan_tiles(int M, int N, int kb, int sms) {
     for (const Cost &c : kCosts) {
         if (c.bn > 128 && N < c.bn) continue;
         const long long tiles = (long long)((M + tile_rows(c.pair) - 1) / tile_rows(c.pair)) * ((N + c.bn - 1) / c.bn);
-        const int units = c.pair ? sms / 2 : sms;
-        long long t = c.fixed + (tiles + units - 1) / units * (c.round + (long long)kb * c.block);
+        long long t = c.fixed + rounds_ns(c, tiles, kb, sms);
         if (t < least) t = least;
-        if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, 1, (int)(t < 0x7fffffff ? t : 0x7fffffff)};
+        if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, 1, at_most_int(t)};
     }
     return best;
 }
@@ -517,15 +531,13 @@ Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks) {
     for (const Cost &c : kCosts) {
         if (c.bn > 128 && N < c.bn) continue;
         const long long tiles = (long long)((M + tile_rows(c.pair) - 1) / tile_rows(c.pair)) * ((N + c.bn - 1) / c.bn);
-        const int units = c.pair ? sms / 2 : sms;
         const long long tile_bytes = (long long)tile_rows(c.pair) * c.bn * 4;
         for (int s = 1; s <= 32 && s <= kb; s++) {
             const int per = (kb + s - 1) / s;
             if (s > 1 && per < least_blocks) break;
-            const long long rounds = (tiles * s + units - 1) / units;
-            const long long t = (c.pair ? 5800 : 4200) + rounds * ((c.pair ? 550 : 160) + (long long)per * c.block * 115 / 100) +
+            const long long t = c.fixed + rounds_ns(c, tiles * s, per, sms) * 115 / 100 +
                                 tiles * s * tile_bytes / 1000 * (c.pair ? 43 : 80) / 1000;
-            if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, s, (int)(t < 0x7fffffff ? t : 0x7fffffff)};
+            if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, s, at_most_int(t)};
         }
     }
     return best;
