@@ -115,6 +115,17 @@ def test_fast_forward_vs_oracle(pkg, gpu, oracle, shape):
     assert np.abs(lse - ref_lse).max() < 1e-4
 
 
+@pytest.mark.parametrize("B,T,H", [(41, 60, 16), (41, 64, 15), (20, 130, 16), (7, 700, 20)])
+def test_fast_forward_takes_over_items(pkg, gpu, oracle, B, T, H):
+    """More query tiles than two per SM, so that thread blocks take over those of blocks that have not started: one
+    key step per tile, one or two, many; more than four items per block wrap the slots of the answers."""
+    x, _ = seeded(33, B, T, H, 64)
+    out, lse, _ = run_cuda(pkg, gpu, x, None, H)
+    ref_out, ref_lse = oracle.forward(x, H, want_lse=True)
+    assert np.abs(out - ref_out).max() < EXPECT_OUT
+    assert np.abs(lse - ref_lse).max() < 1e-4
+
+
 @pytest.mark.parametrize("shape", FAST_SHAPES, ids=lambda s: "B%d_T%d_H%d" % s)
 def test_fast_backward_vs_oracle(pkg, gpu, oracle, shape):
     B, T, H = shape
