@@ -218,10 +218,64 @@ __device__ __forceinline__ void store_ds(uint8_t *tile_h, uint8_t *tile_l, int r
     }
 }
 
+// What the prepare kernel works from and leaves behind, for the variant that does its work (take_dout).
+struct Dout {
+    const float *dout, *out;
+    __nv_bfloat16 *hi, *lo;
+    float *delta;
+};
+
+// Sequences of at most 128 tokens, one (batch, head) per CTA: dO and O come as fp32, the compute warps split dO into the
+// planes the tensor cores read (ring slots 0 and 1: the two halves of the only query tile) and form rowsum(dO * O).
+// The prepare kernel, its launch and a trip through memory go out of a pass that is all latency; its results are
+// written to the scratch buffer as well, where a later core-only call expects them.  Thread: a quarter of a row.
+__device__ __forceinline__ void take_dout(BwdSmem &sm, const Dout &d, int b, int h, int H, int T) {
+    const int tid = (int)threadIdx.x - 128, r = tid >> 2, c0 = 16 * (tid & 3);
+    float4 g[4], o[4];
+    const size_t at = ((size_t)b * T + r) * H * kD + h * kD + c0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        g[i] = r < T ? __ldcs(reinterpret_cast<const float4 *>(d.dout + at) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        o[i] = r < T ? __ldcs(reinterpret_cast<const float4 *>(d.out + at) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) sum += g[i].x * o[i].x + g[i].y * o[i].y + g[i].z * o[i].z + g[i].w * o[i].w;
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    uint8_t *th = sm.in[r >> 6][2] + (r & 63) * 128, *tl = sm.in[r >> 6][3] + (r & 63) * 128;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        uint4 vh, vl;
+        split_bf16x2(g[2 * i].x, g[2 * i].y, vh.x, vl.x);
+        split_bf16x2(g[2 * i].z, g[2 * i].w, vh.y, vl.y);
+        split_bf16x2(g[2 * i + 1].x, g[2 * i + 1].y, vh.z, vl.z);
+        split_bf16x2(g[2 * i + 1].z, g[2 * i + 1].w, vh.w, vl.w);
+        const int chunk = ((2 * (tid & 3) + i) ^ (r & 7)) << 4;
+        *reinterpret_cast<uint4 *>(th + chunk) = vh;
+        *reinterpret_cast<uint4 *>(tl + chunk) = vl;
+        if (r < T) {
+            *reinterpret_cast<uint4 *>(d.hi + at + 8 * i) = vh;
+            *reinterpret_cast<uint4 *>(d.lo + at + 8 * i) = vl;
+        }
+    }
+    if ((tid & 3) == 0) {
+        sm.delta[0][r] = -sum;
+        if (r < T) d.delta[((size_t)b * H + h) * T + r] = sum;
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        mbar_arrive(&sm.in_full[r >> 6]);  // a warp's 8 rows are in one half
+        mbar_arrive(&sm.stats_full[0]);
+    }
+}
+
+template <bool kFp32>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_do,
                 const __grid_constant__ CUtensorMap map_dx, const float *__restrict__ lse, const float *__restrict__ delta,
-                float *__restrict__ dqkv, int B, int T, int H, float scale, float scale_log2, int *sched, int *status) {
+                float *__restrict__ dqkv, Dout src, int B, int T, int H, float scale, float scale_log2, int *sched, int *status) {
     // The structure fills the whole 227 KiB, so there is no room to round the base up: the
     // swizzled tiles need 1024-byte alignment and the kernel refuses to run without it.
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -254,11 +308,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             mbar_init(&sm.st_full[i], 1);
             mbar_init(&sm.pds_full[i], kComputeThreads);
             mbar_init(&sm.dq_full[i], 1);
-            mbar_init(&sm.stats_full[i], 32);
+            mbar_init(&sm.stats_full[i], kFp32 ? 32 + kComputeThreads / 32 : 32);
             mbar_init(&sm.stats_free[i], kComputeThreads / 32);
         }
         for (int i = 0; i < kSlots; i++) {
-            mbar_init(&sm.in_full[i], 1);
+            mbar_init(&sm.in_full[i], kFp32 ? 1 + kComputeThreads / 64 : 1);
             mbar_init(&sm.in_empty[i], 1);
         }
         mbar_init(&sm.ds_full, kComputeThreads);
@@ -301,11 +355,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 }
                 const int b = it.bh / H, h = it.bh % H;
                 const int y = (it.jt + (t >> 1)) * kTile + (t & 1) * kHalf;
-                mbar_expect_tx(&sm.in_full[slot], 4 * kPlaneHalf);
+                mbar_expect_tx(&sm.in_full[slot], (kFp32 ? 2 : 4) * kPlaneHalf);
                 tma_load_4d(sm.in[slot][0], &map_x, &sm.in_full[slot], h * kD, y, b, 0);
                 tma_load_4d(sm.in[slot][1], &map_x, &sm.in_full[slot], h * kD, y, b, 1);
-                tma_load_4d(sm.in[slot][2], &map_do, &sm.in_full[slot], h * kD, y, b, 0);
-                tma_load_4d(sm.in[slot][3], &map_do, &sm.in_full[slot], h * kD, y, b, 1);
+                if (!kFp32) {
+                    tma_load_4d(sm.in[slot][2], &map_do, &sm.in_full[slot], h * kD, y, b, 0);
+                    tma_load_4d(sm.in[slot][3], &map_do, &sm.in_full[slot], h * kD, y, b, 1);
+                }
                 g++;
             };
             auto load_kv = [&](const Work &it, uint8_t (*dst)[kPlaneTile], int x0) {
@@ -460,7 +516,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             for (int k = 0; k < kTile / 32; k++) {
                 const int r = lane + 32 * k, t = (c.w.jt + c.m) * kTile + r;
                 sm.lse2[buf][r] = t < T ? -lse[(size_t)c.w.bh * T + t] * 1.4426950408889634f : 0.f;
-                sm.delta[buf][r] = t < T ? -delta[(size_t)c.w.bh * T + t] : 0.f;
+                if (!kFp32) sm.delta[buf][r] = t < T ? -delta[(size_t)c.w.bh * T + t] : 0.f;
             }
             mbar_arrive(&sm.stats_full[buf]);
         };
@@ -515,8 +571,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         auto reduce_dq = [&](const Work &it, int qt) {
             if (lane == 0) {
                 const int b = it.bh / H, xq = (it.bh % H) * kD;
-                tma_reduce_add_3d(sm.ds[0][0], &map_dx, xq, qt * kTile, b);
-                tma_reduce_add_3d(sm.ds[0][1], &map_dx, xq + 32, qt * kTile, b);
+                if (kFp32) {  // the only contribution
+                    tma_store_3d(sm.ds[0][0], &map_dx, xq, qt * kTile, b);
+                    tma_store_3d(sm.ds[0][1], &map_dx, xq + 32, qt * kTile, b);
+                } else {
+                    tma_reduce_add_3d(sm.ds[0][0], &map_dx, xq, qt * kTile, b);
+                    tma_reduce_add_3d(sm.ds[0][1], &map_dx, xq + 32, qt * kTile, b);
+                }
                 bulk_commit();
                 bulk_wait_read_all();
                 mbar_arrive(&sm.out_free);
@@ -579,6 +640,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         const float2 sc2 = make_float2(scale_log2, scale_log2);
         bool ok = true;
         uint32_t n = 0;  // query tiles processed so far in this launch
+        if (kFp32) take_dout(sm, src, (int)blockIdx.x / H, (int)blockIdx.x % H, H, T);
 
         // One row (16 of its 64 columns) of an fp32 output tile into the staging layout the copy
         // engine expects: two 32-column halves, 128-byte rows, 16-byte chunks swizzled by row % 8.
@@ -775,7 +837,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         tmem_dealloc(sm.tmem_base, kTmemCols);
     }
     // the last CTA to finish leaves the item counter as the next launch expects it
-    if (threadIdx.x == 0 && atomicAdd(sched + 1, 1) == (int)gridDim.x - 1) {
+    if (threadIdx.x == 0 && (kFp32 ? blockIdx.x == 0 : atomicAdd(sched + 1, 1) == (int)gridDim.x - 1)) {
         sched[0] = 0;
         sched[1] = 0;
     }
@@ -787,7 +849,9 @@ static size_t bwd_smem_bytes() { return sizeof(BwdSmem); }
 static_assert(sizeof(BwdSmem) <= 227 * 1024, "backward kernel shared memory");
 
 cudaError_t fast_bwd_set_attributes() {
-    return cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem_bytes());
+    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem_bytes());
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem_bytes());
 }
 
 // map_x / map_do must have boxes of 64 rows (see the producer warp); map_dx covers dqkv as fp32
@@ -803,8 +867,17 @@ cudaError_t launch_fast_backward(const CUtensorMap &map_x, const CUtensorMap &ma
     if (items >= (long long)kMoreBit) return cudaErrorInvalidValue;  // an item number and a flag share one int
     const unsigned grid = (unsigned)(items < num_sms ? items : num_sms);
     const float scale = 0.125f;  // 1/sqrt(64)
-    return launch_after_previous(attn_bwd_kernel, dim3(grid), dim3(kThreads), bwd_smem_bytes(), s, map_x, map_do, map_dx, lse,
-                                 delta, dqkv, B, T, H, scale, scale * 1.4426950408889634f, sched, status);
+    return launch_after_previous(attn_bwd_kernel<false>, dim3(grid), dim3(kThreads), bwd_smem_bytes(), s, map_x, map_do, map_dx,
+                                 lse, delta, dqkv, Dout{}, B, T, H, scale, scale * 1.4426950408889634f, sched, status);
+}
+
+cudaError_t launch_fast_backward_fp32(const CUtensorMap &map_x, const CUtensorMap &map_dx, const float *dout, const float *out,
+                                      const float *lse, float *delta, __nv_bfloat16 *dhi, __nv_bfloat16 *dlo, float *dqkv, int B,
+                                      int T, int H, int *sched, int *status, cudaStream_t s) {
+    const float scale = 0.125f;  // 1/sqrt(64)
+    return launch_after_previous(attn_bwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), bwd_smem_bytes(), s, map_x, map_x,
+                                 map_dx, lse, nullptr, dqkv, Dout{dout, out, dhi, dlo, delta}, B, T, H, scale,
+                                 scale * 1.4426950408889634f, sched, status);
 }
 
 }  // namespace attn

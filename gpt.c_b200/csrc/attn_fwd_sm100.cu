@@ -224,9 +224,53 @@ __device__ __forceinline__ void store_row(float *dst, const uint32_t (&r)[32], f
     }
 }
 
+// Sequences of at most 64 tokens: the (only) item's Q, K and V come from the fp32 tensor, every thread splits its share
+// into the two bf16 planes, in shared memory where the tensor cores read them and in `saved` for the backward.
+// That takes the split kernel, its launch and a second trip through memory out of a pass that is all latency.
+__device__ __forceinline__ void take_fp32(FwdSmem &sm, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ hi,
+                                          __nv_bfloat16 *__restrict__ lo, int b, int h, int T, int C) {
+    constexpr int kBatch = 4;  // 32 bytes each, all on their way before the first is used
+    for (int i0 = threadIdx.x; i0 < 3 * 8 * kStep; i0 += kBatch * kThreads) {
+        float4 a[kBatch][2];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int i = i0 + u * kThreads, part = i >> 9, row = (i >> 3) & 63, c = i & 7;
+            a[u][0] = a[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < 3 * 8 * kStep && row < T) {
+                const float4 *src = reinterpret_cast<const float4 *>(qkv + ((size_t)b * T + row) * 3 * C + part * C + h * kD) + 2 * c;
+                a[u][0] = __ldcs(src);
+                a[u][1] = __ldcs(src + 1);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int i = i0 + u * kThreads, part = i >> 9, row = (i >> 3) & 63, c = i & 7;
+            if (i >= 3 * 8 * kStep) break;
+            uint4 vh, vl;
+            split_bf16x2(a[u][0].x, a[u][0].y, vh.x, vl.x);
+            split_bf16x2(a[u][0].z, a[u][0].w, vh.y, vl.y);
+            split_bf16x2(a[u][1].x, a[u][1].y, vh.z, vl.z);
+            split_bf16x2(a[u][1].z, a[u][1].w, vh.w, vl.w);
+            const int at = row * 128 + ((c ^ (row & 7)) << 4);
+            uint8_t *dh = part == 0 ? sm.q[0] : (part == 1 ? sm.k[0][0] : sm.v[0][0]);
+            uint8_t *dl = part == 0 ? sm.q[1] : (part == 1 ? sm.k[0][1] : sm.v[0][1]);
+            *reinterpret_cast<uint4 *>(dh + at) = vh;
+            *reinterpret_cast<uint4 *>(dl + at) = vl;
+            if (row < T) {
+                const size_t g = ((size_t)b * T + row) * 3 * C + part * C + h * kD + 8 * c;
+                *reinterpret_cast<uint4 *>(hi + g) = vh;
+                *reinterpret_cast<uint4 *>(lo + g) = vl;
+            }
+        }
+    }
+    fence_proxy_async_smem();
+}
+
+template <bool kFp32>
 __global__ void __launch_bounds__(kThreads, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, float *__restrict__ out, float *__restrict__ out_copy,
-                float *__restrict__ lse, int B, int T, int H, float scale_log2, int *status) {
+attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ hi,
+                __nv_bfloat16 *__restrict__ lo, float *__restrict__ out, float *__restrict__ out_copy, float *__restrict__ lse,
+                int B, int T, int H, float scale_log2, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     FwdSmem &sm = *reinterpret_cast<FwdSmem *>(smem_raw);
     if ((smem_u32(smem_raw) & 1023u) != 0) {
@@ -258,12 +302,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, float *__restrict__ o
         fence_barrier_init();
         // This thread is also the Q/K producer: the first Q and K tiles are requested right away, while the other
         // warps are still setting up (but not before the kernel that wrote them has completed).
-        pdl_wait();
-        fence_proxy_async_smem();
-        tma_prefetch_desc(&map_x);
-        const Item w = decode((int)blockIdx.x, B, T, H);
-        load_q(sm, map_x, w);
-        for (int j = 0; j < min(2, w.nsteps); j++) load_k(sm, map_x, w, C, j, j);
+        if (!kFp32) {
+            pdl_wait();
+            fence_proxy_async_smem();
+            tma_prefetch_desc(&map_x);
+            const Item w = decode((int)blockIdx.x, B, T, H);
+            load_q(sm, map_x, w);
+            for (int j = 0; j < min(2, w.nsteps); j++) load_k(sm, map_x, w, C, j, j);
+        }
     }
     if (warp == 1) {
         tmem_alloc(&sm.tmem_base, kTmemCols);
@@ -271,6 +317,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, float *__restrict__ o
     }
     pdl_launch_dependents();
     pdl_wait();  // every thread, before its first access to global memory
+    if (kFp32) {
+        const Item w = decode((int)blockIdx.x, B, T, H);
+        take_fp32(sm, qkv, hi, lo, w.b, w.h, T, C);
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -280,11 +330,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, float *__restrict__ o
     // items of this CTA, `n` their key steps; both number the phases of the barriers (the answer that names item t
     // is the t-th one, in slot (t - 1) % 4).
     auto next_item = [&](int t) -> int {
+        if (kFp32) return -1;
         if (!mbar_wait_warp(&sm.next_full[(t - 1) & 3], ((t - 1) >> 2) & 1, ctx, SITE_NEXT)) return -1;
         return item_of(&sm.next[(t - 1) & 3]);
     };
 
-    if (warp == 0) {
+    if (kFp32 && threadIdx.x == 0) {  // what the copy engine signals otherwise
+        mbar_arrive(&sm.q_full);
+        mbar_arrive(&sm.k_full[0]);
+        mbar_arrive(&sm.v_full[0]);
+    }
+
+    if (kFp32 && (warp == 0 || warp == 3)) {
+        // no loads to request
+    } else if (warp == 0) {
         // ------------------------------ TMA producer: Q and K; requests ------------------------------
         int n = 0;
         bool ok = true;
@@ -507,16 +566,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, float *__restrict__ o
 }  // namespace
 
 cudaError_t fast_fwd_set_attributes() {
-    return cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
+    const cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(attn_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
 }
+
+static const float kScaleLog2 = 0.125f * 1.4426950408889634f;  // 1/sqrt(64) * log2(e)
 
 cudaError_t launch_fast_forward(const CUtensorMap &map_x, float *out, float *out_copy, float *lse, int B, int T, int H,
                                 int *status, cudaStream_t s) {
     const int nqt = (T + kTile - 1) / kTile;
-    const unsigned grid = (unsigned)(nqt * B * H);
-    const float scale_log2 = 0.125f * 1.4426950408889634f;  // 1/sqrt(64) * log2(e)
-    return launch_after_previous(attn_fwd_kernel, dim3(grid), dim3(kThreads), sizeof(FwdSmem), s, map_x, out, out_copy, lse, B, T, H,
-                                 scale_log2, status);
+    return launch_after_previous(attn_fwd_kernel<false>, dim3((unsigned)(nqt * B * H)), dim3(kThreads), sizeof(FwdSmem), s, map_x,
+                                 nullptr, nullptr, nullptr, out, out_copy, lse, B, T, H, kScaleLog2, status);
+}
+
+cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy,
+                                     float *lse, int B, int T, int H, int *status, cudaStream_t s) {
+    const CUtensorMap none = {};
+    return launch_after_previous(attn_fwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), sizeof(FwdSmem), s, none, qkv, hi,
+                                 lo, out, out_copy, lse, B, T, H, kScaleLog2, status);
 }
 
 }  // namespace attn

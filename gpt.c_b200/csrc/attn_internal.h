@@ -9,6 +9,7 @@
 
 namespace attn {
 
+constexpr int kShortT = 128;  // one query and key tile: the kernels that read the fp32 tensors themselves
 constexpr int kGenericMaxD = 256;
 constexpr int kGenericMaxT = 8192;
 
@@ -41,6 +42,14 @@ cudaError_t fast_fwd_set_attributes();
 cudaError_t fast_bwd_set_attributes();
 cudaError_t launch_fast_forward(const CUtensorMap &map_x, float *out, float *out_copy, float *lse, int B, int T, int H,
                                 int *status, cudaStream_t s);
+// T <= kShortT / 2 only: splits qkv itself (hi, lo receive the planes), in place of launch_split and launch_fast_forward.
+cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy,
+                                     float *lse, int B, int T, int H, int *status, cudaStream_t s);
+// T <= kShortT and B * H <= num_sms only: prepares dout itself (everything launch_bwd_prepare leaves in the scratch
+// buffer is written too), in place of launch_bwd_prepare and launch_fast_backward.
+cudaError_t launch_fast_backward_fp32(const CUtensorMap &map_x, const CUtensorMap &map_dx, const float *dout, const float *out,
+                                      const float *lse, float *delta, __nv_bfloat16 *dhi, __nv_bfloat16 *dlo, float *dqkv, int B,
+                                      int T, int H, int *sched, int *status, cudaStream_t s);
 cudaError_t launch_fast_backward(const CUtensorMap &map_x, const CUtensorMap &map_do, const CUtensorMap &map_dx,
                                  const float *lse, const float *delta, float *dqkv, int B, int T, int H, int num_sms,
                                  int *sched, int *status, cudaStream_t s);
