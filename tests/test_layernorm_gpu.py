@@ -16,9 +16,10 @@ from oracle import ops_oracle as ops  # noqa: E402
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(8 * 128, 768), (1000, 768), (333, 1024), (64, 1600), (17, 64), (256, 2048), (5, 4)]
+EDGES = [(2368, 516), (2369, 516), (3000, 768), (9, 2044), (2500, 8)]  # either side of the row count and width of the dispatch
 
 
-@pytest.mark.parametrize("rows,C", SHAPES)
+@pytest.mark.parametrize("rows,C", SHAPES + EDGES)
 @pytest.mark.parametrize("with_bias", [True, False])
 def test_layernorm_forward_and_backward_vs_cpu(pkg, rows, C, with_bias):
     rng = np.random.default_rng(rows * 7 + C)
