@@ -64,6 +64,9 @@ struct Problem {
     int tiles_m, tiles_n, splits, kb_total, kb_per_split, total;
     int wide, wide_planes;  // rows of C / of the planes start on 32-byte boundaries
     size_t plane_words;     // distance from the hi to the lo plane
+    size_t ldc;             // floats from one row of C to the next
+    int b_shift;            // B's contraction index runs this far behind A's (see RowClasses)
+    int a_shift[4];         // columns of A's views before the first column of dy (dW from row classes)
     int m_fast;  // consecutive work items walk down the rows of C (else along its columns)
 };
 
@@ -71,7 +74,30 @@ enum Site : int {
     SITE_EMPTY = 201, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_SMEM_ALIGN
 };
 
+// Tensors the copy engine fetches from; four views of each operand for dW from row classes.
+template <bool kClasses>
+struct Maps {
+    CUtensorMap a[kClasses ? 4 : 1], b[kClasses ? 4 : 1], c;
+};
+
+// Rows of dy whose pitch is not a multiple of 16 bytes (the vocabulary projection: 50257 floats) cannot be tiled by the
+// copy engine as they are, but every fourth row can: the rows m = 4 i + j form a matrix with a pitch of 4 N floats, whose
+// base is moved down to a 16-byte boundary, by a_shift = (j N) mod 4 floats.  The view's column c is then column
+// c - a_shift of dy.  In dx that is the contraction index, and W is fetched at rows c - a_shift (rows before the first
+// and past the last read as zeros); one product per class, which leaves every fourth row of dx.  In dW it is the row of
+// the result: each class is a piece of the contraction, added into dW a_shift rows higher up.  What this replaces is a
+// copy of dy with padded rows, 536 us for the 1.65 GB of 8192 x 50257.
+struct RowClass {
+    const float *dy;  // base of the view
+    int rows, shift;
+};
+RowClass row_class(const float *dy, int M, int N, int j) {
+    const int shift = (int)(((long long)j * N) & 3);
+    return RowClass{dy + (size_t)j * N - shift, (M - j + 3) / 4, shift};
+}
+
 struct Work {
+    int cls;  // row class
     int m0, n0, kb0, kb1;  // first row of this CTA's 128, first column of the tile, contraction blocks
 };
 template <bool kPair>
@@ -85,6 +111,7 @@ __device__ __forceinline__ Work decode(const Problem &p, int w, int rank) {
     Work r;
     r.m0 = kPair ? (2 * tm + rank) * kBM : tm * kBM;
     r.n0 = tn * p.bn;
+    r.cls = split;  // only looked at where the pieces of the contraction are row classes
     r.kb0 = split * p.kb_per_split;
     r.kb1 = min(p.kb_total, r.kb0 + p.kb_per_split);
     return r;
@@ -115,10 +142,9 @@ __device__ __forceinline__ void store_words(void *dst, int left, int wide, const
 // whose row pitch is not a multiple of 16 bytes (the 50257-wide vocabulary projection).
 // kPair: two CTAs of a cluster share a tile of 256 rows.  Each loads its 128 rows of A and half of the kBN columns
 // of B, 32 KB per contraction block of a 256 x 256 tile where a CTA on its own needs 48 KB for a 128 x 256 one.
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair, bool kClasses>
 __global__ void __launch_bounds__(kThreads, 1)
-linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                   const __grid_constant__ CUtensorMap map_c, const float *__restrict__ bias, float *__restrict__ c_direct,
+linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__restrict__ bias, float *__restrict__ c_direct,
                    uint32_t *__restrict__ planes, Problem p, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     using Smem = SmemT<kBN, kStages, kPair, kEpi == 1 || kDirect>;
@@ -168,12 +194,16 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
         if (lane == 0) {
-            tma_prefetch_desc(&map_a);
-            tma_prefetch_desc(&map_b);
+            for (int i = 0; i < (kClasses ? 4 : 1); i++) {
+                tma_prefetch_desc(&maps.a[i]);
+                tma_prefetch_desc(&maps.b[i]);
+            }
             int it = 0;
             bool ok = true;
             for (int w = first; ok && w < p.total; w += step) {
-                const Work wk = decode<kPair>(p, w, rank);
+                Work wk = decode<kPair>(p, w, rank);
+                const CUtensorMap &map_a = maps.a[kClasses ? wk.cls : 0], &map_b = maps.b[kClasses ? wk.cls : 0];
+                if (kClasses) wk.kb0 = 0, wk.kb1 = p.kb_total;
                 for (int kb = wk.kb0; kb < wk.kb1; kb++, it++) {
                     const int st = it % kStages;
                     if (it >= kStages && !mbar_wait(&sm.empty[st], ((it / kStages) - 1) & 1, ctx, SITE_EMPTY)) {
@@ -202,11 +232,11 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     }
                     if (kBMN) {
                         if (p.b_one) {
-                            load(sm.b[st], &map_b, 0, kb * kBK, b0 / 32);
+                            load(sm.b[st], &map_b, 0, kb * kBK - p.b_shift, b0 / 32);
                         } else {
 #pragma unroll
                             for (int i = 0; i < kBRows / 32; i++)
-                                load(sm.b[st] + i * 4096, &map_b, b0 + 32 * i, kb * kBK, 0);
+                                load(sm.b[st] + i * 4096, &map_b, b0 + 32 * i, kb * kBK - p.b_shift, 0);
                         }
                     } else {
                         load(sm.b[st], &map_b, kb * kBK, b0, 0);  // the B map's box is kBRows rows
@@ -221,7 +251,8 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         int it = 0, j = 0;
         bool ok = true;
         for (int w = first; ok && w < p.total; w += step, j++) {
-            const Work wk = decode<kPair>(p, w, rank);
+            Work wk = decode<kPair>(p, w, rank);
+            if (kClasses) wk.kb0 = 0, wk.kb1 = p.kb_total;
             const int acc = j & 1;
             if (j >= 2 && !mbar_wait_warp(&sm.acc_empty[acc], ((j >> 1) - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
             tc_fence_after_sync();
@@ -299,7 +330,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     // straight from the registers: this lane's row, 32-byte sectors
                     const int row = row0 + lane;
                     if (row < p.M) {
-                        store_words<8>(c_direct + (size_t)row * p.N + col0, p.N - col0, p.wide, r);
+                        store_words<8>(c_direct + (size_t)row * p.ldc + col0, p.N - col0, p.wide, r);
                         if (kPlanes) {
                             uint32_t hp[16], lp[16];
 #pragma unroll
@@ -309,6 +340,23 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             store_words<4>(hi, (p.N - col0) / 2, p.wide_planes, hp);
                             store_words<4>(hi + p.plane_words, (p.N - col0) / 2, p.wide_planes, lp);
                         }
+                    }
+                    continue;
+                }
+                const int up = kClasses ? p.a_shift[wk.cls] : 0;
+                if (kClasses && row0 < up) {
+                    // The first 32 rows of the result: up to three of them do not exist, and a copy must not start at a
+                    // negative coordinate.
+                    const int row = row0 + lane - up;
+                    if (row >= 0 && row < p.M) {
+                        float *dst = c_direct + (size_t)row * p.ldc + col0;
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            if (col0 + 4 * q < p.N)
+                                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * q),
+                                             "f"(__uint_as_float(r[4 * q])), "f"(__uint_as_float(r[4 * q + 1])),
+                                             "f"(__uint_as_float(r[4 * q + 2])), "f"(__uint_as_float(r[4 * q + 3]))
+                                             : "memory");
                     }
                     continue;
                 }
@@ -332,7 +380,7 @@ linear_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_reduce_add_3d(buf, &map_c, col0, row0, 0);
+                    tma_reduce_add_3d(buf, &maps.c, col0, row0 - up, 0);
                     bulk_commit();
                 }
             }
@@ -448,9 +496,10 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(float *__restrict__ dst, 
 
 // ---- host side ----
 
-int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols) {
+int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, size_t pitch = 0) {
+    if (pitch == 0) pitch = (size_t)cols;
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
-    const cuuint64_t strides[2] = {(cuuint64_t)cols * 4, (cuuint64_t)cols * 4 * (cuuint64_t)rows};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * 4 * (cuuint64_t)rows};
     const cuuint32_t box[3] = {32, 32, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
 }
@@ -461,6 +510,9 @@ Problem make_problem(int M, int N, int K, int bn, int pair, int splits) {
     p.M = M, p.N = N, p.K = K, p.bn = bn, p.pair = pair;
     p.a_one = p.b_one = 0;
     p.m_fast = 0;
+    p.ldc = (size_t)N;
+    p.b_shift = 0;
+    for (int i = 0; i < 4; i++) p.a_shift[i] = 0;
     p.tiles_m = (M + tile_rows(pair) - 1) / tile_rows(pair);
     p.tiles_n = (N + bn - 1) / bn;
     p.kb_total = (K + kBK - 1) / kBK;
@@ -543,29 +595,35 @@ Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks) {
     return best;
 }
 
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
-int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
-               Problem p, int *status, cudaStream_t s) {
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair, bool kClasses = false>
+int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *planes, Problem p, int *status, cudaStream_t s) {
     using Smem = SmemT<kBN, kStages, kPair, kEpi == 1 || kDirect>;
     static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear kernel");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair>;
+    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair, kClasses>;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return (int)e;
         attr_done[dev] = true;
     }
-    p.wide = p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(c) & 31u) == 0;
+    p.wide = p.ldc % 8 == 0 && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(c) & 31u) == 0;
     p.wide_planes = p.N % 16 == 0 && (reinterpret_cast<uintptr_t>(planes) & 31u) == 0;
     p.plane_words = attn::plane_bytes((size_t)p.M * p.N) / 4;
     constexpr int kCtas = kPair ? 2 : 1;
     const int most = sm_count() / kCtas;
     const int grid = (p.total < most ? p.total : most) * kCtas;
-    return (int)attn::launch_clusters_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), kCtas, s, ma, mb, mc, bias, c,
+    return (int)attn::launch_clusters_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), kCtas, s, maps, bias, c,
                                                      static_cast<uint32_t *>(planes), p, status);
+}
+
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
+int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
+               const Problem &p, int *status, cudaStream_t s) {
+    const Maps<false> maps = {{ma}, {mb}, mc};
+    return launch_maps<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair>(maps, bias, c, planes, p, status, s);
 }
 
 // Pipeline depth by what fits in 227 KiB next to the output staging tile.
@@ -605,6 +663,54 @@ int stream_rows_of_c(int M, int N, int K) {
 }
 
 bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
+
+// dx and dW (either may be NULL) straight from a dy whose rows are not 16-byte aligned.
+int gradients_by_row_class(const float *dy, const float *x, const float *w, float *dx, float *dw, int M, int N, int K, int sms,
+                           int *status, cudaStream_t s) {
+    int rc;
+    CUtensorMap ma, mb, mc;
+    if (dx) {
+        const int kb = (N + 3 + kBK - 1) / kBK;
+        Plan plan = plan_tiles((M + 3) / 4, K, kb, sms), cut = plan_pieces((M + 3) / 4, K, kb, sms, 32);
+        cut.ns += (2500 + (int)((long long)M * K * 4 / 5500)) / 4;
+        if (cut.splits > 1 && cut.ns < plan.ns) plan = cut;
+        if (plan.splits > 1 && (rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
+        for (int j = 0; j < 4; j++) {
+            const RowClass c = row_class(dy, M, N, j);
+            Problem p = make_problem(c.rows, K, N + c.shift, plan.bn, plan.pair, plan.splits);
+            p.ldc = 4 * (size_t)K, p.b_shift = c.shift;
+            if ((rc = map_k_major(&ma, c.dy, c.rows, N + c.shift, 128, 4 * (size_t)N)) != 0) return rc;
+            p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 / (p.pair ? 2 : 1)) == 0;
+            if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
+            float *out = dx + (size_t)j * K;
+            if (p.splits > 1) {
+                if ((rc = map_out_f32(&mc, out, c.rows, K, p.ldc)) != 0) return rc;
+                rc = launch<false, true, 1>(ma, mb, mc, nullptr, out, nullptr, p, status, s);
+            } else {
+                rc = launch<false, true, 0>(ma, mb, ma, nullptr, out, nullptr, p, status, s);
+            }
+            if (rc != 0) return rc;
+        }
+    }
+    if (!dw) return ATTN_OK;
+    // the four classes of a tile follow each other, so that the tile of dW they add into stays in L2
+    Maps<true> maps;
+    Problem p = make_problem(N, K, (M + 3) / 4, K % 256 == 0 ? 256 : 128, 1, 1);
+    p.splits = 4, p.total *= 4;
+    p.a_one = 0, p.b_one = 1;
+    for (int j = 0; j < 4; j++) {
+        const RowClass c = row_class(dy, M, N, j);
+        p.a_shift[j] = c.shift;
+        if ((rc = map_mn_major(&maps.a[j], c.dy, c.rows, N + c.shift, 4 * (size_t)N)) != 0) return rc;
+        if ((rc = map_mn_major_blocks(&maps.b[j], x + (size_t)j * K, c.rows, K, p.bn / 64, 4 * (size_t)K)) != 0) return rc;
+    }
+    // up to three rows of the last tile may only be reached through the shifted views
+    p.tiles_m = (N + 3 + tile_rows(1) - 1) / tile_rows(1);
+    p.total = p.tiles_m * p.tiles_n * p.splits;
+    if ((rc = map_out_f32(&maps.c, dw, N, K)) != 0) return rc;
+    if (p.bn == 256) return launch_maps<true, true, 1, 256, 6, false, false, true, true>(maps, nullptr, dw, nullptr, p, status, s);
+    return launch_maps<true, true, 1, 128, 6, false, false, true, true>(maps, nullptr, dw, nullptr, p, status, s);
+}
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
 int input_gradient(const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status, cudaStream_t s) {
@@ -690,6 +796,8 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     if (rc != ATTN_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int sms = sm_count();
+    // From 1024 rows on the copy with padded rows costs more than four products on every fourth row do.
+    if (N % 4 != 0 && M >= 1024 && !db) return gradients_by_row_class(dy, x, w, dx, dw, M, N, K, sms, status, s);
     const float *g = dy;  // [M, np] from here on
     if (padded) {
         rc = (int)attn::launch_after_previous(pad_rows_kernel, dim3(sms * 16), dim3(256), 0, s, static_cast<float *>(scratch), dy, M,

@@ -57,26 +57,30 @@ __device__ __forceinline__ uint64_t smem_desc_sw128_base32(uint32_t smem_addr, u
 // ---- host side ----
 
 // Operand read K-major: matrix [rows, kc] row-major (kc contiguous = contraction); boxes of 32 x box_rows.
-inline int map_k_major(CUtensorMap *map, const float *base, int rows, int kc, int box_rows) {
+// `pitch`: floats from one row to the next (0: kc).
+inline int map_k_major(CUtensorMap *map, const float *base, int rows, int kc, int box_rows, size_t pitch = 0) {
+    if (pitch == 0) pitch = (size_t)kc;
     const cuuint64_t dims[4] = {(cuuint64_t)kc, (cuuint64_t)rows, 1, 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)kc * 4, (cuuint64_t)kc * 4 * (cuuint64_t)rows, (cuuint64_t)kc * 4 * (cuuint64_t)rows};
+    const cuuint64_t strides[3] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * 4 * (cuuint64_t)rows, (cuuint64_t)pitch * 4 * (cuuint64_t)rows};
     const cuuint32_t box[4] = {32, (cuuint32_t)box_rows, 1, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box);
 }
 // Operand read MN-major, whole tile in one copy: the matrix [kc, rows] seen as {32 values, kc, rows / 32 blocks}
 // with the block index as the slowest box dimension, box {32, 32, nblocks}: shared memory receives
 // [block][contraction step][32 values], the layout the descriptor expects.  rows % 32 == 0.
-inline int map_mn_major_blocks(CUtensorMap *map, const float *base, int kc, int rows, int nblocks) {
+inline int map_mn_major_blocks(CUtensorMap *map, const float *base, int kc, int rows, int nblocks, size_t pitch = 0) {
+    if (pitch == 0) pitch = (size_t)rows;
     const cuuint64_t dims[4] = {32, (cuuint64_t)kc, (cuuint64_t)(rows / 32), 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)rows * 4, 128, (cuuint64_t)rows * 4 * (cuuint64_t)kc};
+    const cuuint64_t strides[3] = {(cuuint64_t)pitch * 4, 128, (cuuint64_t)pitch * 4 * (cuuint64_t)kc};
     const cuuint32_t box[4] = {32, 32, (cuuint32_t)nblocks, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
 }
 // Operand read MN-major: matrix [kc, rows] row-major (rows contiguous, kc = contraction), boxes of 32 x 32.
-inline int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows) {
+inline int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows, size_t pitch = 0) {
+    if (pitch == 0) pitch = (size_t)rows;
     const cuuint64_t dims[4] = {(cuuint64_t)rows, (cuuint64_t)kc, 1, 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)rows * 4, (cuuint64_t)rows * 4 * (cuuint64_t)kc, (cuuint64_t)rows * 4 * (cuuint64_t)kc};
+    const cuuint64_t strides[3] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * 4 * (cuuint64_t)kc, (cuuint64_t)pitch * 4 * (cuuint64_t)kc};
     const cuuint32_t box[4] = {32, 32, 1, 1};
     // 32-bit operands read MN-major need the 128-byte swizzle with 32-byte atoms (rows of 128 bytes, the
     // 32-byte quarter of a row XORed with the row index modulo 4)

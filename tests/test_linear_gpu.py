@@ -130,6 +130,24 @@ def test_linear_tile_shapes(pkg, M, N, K):
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
 
 
+@pytest.mark.parametrize("M,N,K", [(1024, 257, 256), (1025, 1001, 96), (1026, 513, 384), (1027, 94, 512), (1300, 9999, 64), (1111, 16387, 32)])
+def test_linear_backward_from_every_fourth_row(pkg, M, N, K):
+    """Rows of dy that start on 4- or 8-byte boundaries, enough of them that no padded copy is made; dW has rows that only
+    the shifted views reach, dx a contraction that is cut into pieces (the last one)."""
+    x, w, _, dy = inputs(M, N, K, 53)
+    xt, wt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, dy))
+    dw0 = np.random.default_rng(3).standard_normal((N, K), dtype=np.float32)
+    pad = torch.full((N + 16, K), 7.0, device="cuda")  # rows either side of dW stay as they are
+    dw = pad[8:8 + N]
+    dw.copy_(torch.from_numpy(dw0))
+    dx = pkg.linear_backward(dyt, xt, wt, dw)
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, _ = ops.linear_backward(dy, x, w, dw0, np.zeros(N, np.float32))
+    within(dx.cpu().numpy(), dx_ref, dy, w)
+    within(dw.cpu().numpy(), dw_ref, dy.T, x)
+    assert bool((pad[:8] == 7.0).all()) and bool((pad[8 + N:] == 7.0).all())
+
+
 def test_linear_backward_parts_can_be_skipped(pkg):
     M, N, K = 512, 768, 768
     x, w, b, dy = inputs(M, N, K, 31)
