@@ -23,7 +23,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 // ---------------------------------------------------------------------------------------
 // split: x -> hi, lo
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ hi,
+// Small tensors, whose planes the next kernel reads from L2.
+__global__ void __launch_bounds__(256) split_small_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ hi,
                                                      __nv_bfloat16 *__restrict__ lo, size_t n) {
     tc05::pdl_launch_dependents();
     tc05::pdl_wait();
@@ -51,6 +52,53 @@ __global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ x,
         const __nv_bfloat16 hh = __float2bfloat16_rn(f);
         hi[i] = hh;
         lo[i] = __float2bfloat16_rn(f - __bfloat162float(hh));
+    }
+}
+
+// Read once and written once: HBM bound.  32 bytes per load, two of them in flight per thread, every block one piece;
+// results leave the cache first (the loop above, 16 bytes per load, took 133 us for 805 MB, this 121 us; 125 us at the
+// copy rate).  On small tensors it is no slower itself, but a forward of B=8 T=128 H=12 went from 10.7 to 12.3 us.
+__global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ hi,
+                                                     __nv_bfloat16 *__restrict__ lo, size_t n) {
+    tc05::pdl_launch_dependents();
+    tc05::pdl_wait();
+    constexpr int kU = 2;
+    const size_t n8 = n / 8, v0 = (size_t)blockIdx.x * (256 * kU) + threadIdx.x;
+    const bool wide = (reinterpret_cast<uintptr_t>(x) & 31u) == 0;
+    float f[kU][8];
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+        const size_t v = v0 + 256 * u;
+        if (v >= n8) break;
+        if (wide) {
+            asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=f"(f[u][0]), "=f"(f[u][1]), "=f"(f[u][2]), "=f"(f[u][3]), "=f"(f[u][4]), "=f"(f[u][5]), "=f"(f[u][6]),
+                           "=f"(f[u][7])
+                         : "l"(x + 8 * v));
+        } else {
+            const float4 a = __ldcs(reinterpret_cast<const float4 *>(x) + 2 * v), b = __ldcs(reinterpret_cast<const float4 *>(x) + 2 * v + 1);
+            f[u][0] = a.x, f[u][1] = a.y, f[u][2] = a.z, f[u][3] = a.w, f[u][4] = b.x, f[u][5] = b.y, f[u][6] = b.z, f[u][7] = b.w;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+        const size_t v = v0 + 256 * u;
+        if (v >= n8) break;
+        uint4 h, l;
+        tc05::split_bf16x2(f[u][0], f[u][1], h.x, l.x);
+        tc05::split_bf16x2(f[u][2], f[u][3], h.y, l.y);
+        tc05::split_bf16x2(f[u][4], f[u][5], h.z, l.z);
+        tc05::split_bf16x2(f[u][6], f[u][7], h.w, l.w);
+        __stcs(reinterpret_cast<uint4 *>(hi) + v, h);
+        __stcs(reinterpret_cast<uint4 *>(lo) + v, l);
+    }
+    // ragged tail (n not a multiple of 8)
+    if (blockIdx.x == 0 && n8 * 8 + threadIdx.x < n) {
+        const size_t i = n8 * 8 + threadIdx.x;
+        const float t = x[i];
+        const __nv_bfloat16 hh = __float2bfloat16_rn(t);
+        hi[i] = hh;
+        lo[i] = __float2bfloat16_rn(t - __bfloat162float(hh));
     }
 }
 
@@ -151,7 +199,7 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
 // kNI = head columns in blocks of 32 (the output tile's width), so D = 80 does 96 columns of output work; the
 // score products run over exactly the 4-column words that hold data.
 // The kernels they replace (one warp per row, K and V read again from L2 for every row) took 83 ms for forward
-// and backward of B=4 T=1024 H=6 D=128; these take 0.74 ms (23 GFLOP of fp32 products, a third of the fp32 rate
+// and backward of B=4 T=1024 H=6 D=128; these take 0.71 ms (23 GFLOP of fp32 products, a third of the fp32 rate
 // of 148 SMs).
 // ---------------------------------------------------------------------------------------
 typedef unsigned long long f32x2;  // two floats of a packed instruction
@@ -188,13 +236,13 @@ struct Pitch {
 // Rows r0 .. r0+kRows-1 of one head (D columns starting at src, rows `stride` apart) into a shared-memory tile, by
 // asynchronous copies; rows at or past `rows` and the columns that fill the last 16-byte word become zeros.
 template <int kRows, int kPitch, int kThreads, bool kVec>
-__device__ __forceinline__ void load_rows_async(float *tile, const float *src, size_t stride, int r0, int rows, int D) {
+__device__ __forceinline__ void load_rows_async(float *tile, const float *src, size_t stride, int r0, int rows, int D, int tid) {
     const int words = (D + 3) >> 2;
-    for (int r = threadIdx.x >> 3; r < kRows; r += kThreads / 8) {
+    for (int r = tid >> 3; r < kRows; r += kThreads / 8) {
         const bool in = r0 + r < rows;
         const float *row = src + (size_t)(in ? r0 + r : 0) * stride;
         const uint32_t dst = tc05::smem_u32(tile + r * kPitch);
-        for (int w = threadIdx.x & 7; w < words; w += 8) {
+        for (int w = tid & 7; w < words; w += 8) {
             if (kVec) {
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16 * w), "l"(row + 4 * w),
                              "r"(in ? 16 : 0)
@@ -212,6 +260,7 @@ __device__ __forceinline__ void load_rows_async(float *tile, const float *src, s
     }
 }
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <int kLeft>
 __device__ __forceinline__ void async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
@@ -293,10 +342,14 @@ __device__ __forceinline__ void store_cols(float *row, int col, int D, float4 v)
 }
 
 // ---------------------------------------------------------------------------------------
-// forward: one block per (b, h, 64 queries), key tiles of 8 kC, online softmax.  4 warps: two blocks share an SM
-// (100 KB of shared memory each at D = 128) and cover each other's loads.
+// forward: one block per (b, h, 64 queries), key tiles of 8 kC, online softmax.  Two groups of four warps take the
+// key tiles in turns, each with its own K, V and P tiles (168 KB of shared memory in all at D = 128), and the two
+// partial results are merged at the end: a block then has its SM to itself and the longest-first order balances the
+// SMs.  (With one group per block and two blocks per SM, the SMs were busy for 71 % of the launch on average, because
+// the long blocks that start together share an SM.)  B=4 T=1024 H=6 D=128 233 -> 192 us, B=2 T=2048 H=4 D=80
+// 395 -> 183 us.  Up to 64 head columns two blocks still fit.
 // ---------------------------------------------------------------------------------------
-constexpr int kFwdThreads = 128, kFwdRows = 64;
+constexpr int kFwdGroup = 128, kFwdThreads = 2 * kFwdGroup, kFwdRows = 64;
 
 template <int kNI, int kC>
 struct FwdTile {
@@ -304,19 +357,23 @@ struct FwdTile {
     static constexpr int kQ = kFwdRows * kPitch;
     static constexpr int kKP = kKeys * kPitch > kFwdRows * kPPitch ? kKeys * kPitch : kFwdRows * kPPitch;  // K, then P
     static constexpr int kV = kKeys * kPitch;
-    static constexpr size_t kBytes = (size_t)(kQ + kKP + kV) * sizeof(float);
+    static constexpr size_t kBytes = (size_t)(kQ + 2 * (kKP + kV)) * sizeof(float);
 };
 
+// one group's barrier
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
 template <int kNI, int kC, bool kVec>
-__global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *__restrict__ qkv, float *__restrict__ out,
+__global__ void __launch_bounds__(kFwdThreads, kNI <= 2 ? 2 : 1) generic_fwd_kernel(const float *__restrict__ qkv, float *__restrict__ out,
                                                                   float *__restrict__ out_copy, float *__restrict__ lse,
                                                                   int T, int H, int D, float scale) {
     using S = FwdTile<kNI, kC>;
     constexpr int kR = 4, kPitch = S::kPitch, kKeys = S::kKeys, kPPitch = S::kPPitch;
     extern __shared__ __align__(16) float sm[];
-    float *sq = sm, *sk = sm + S::kQ, *sp = sk, *sv = sk + S::kKP;
+    const int group = threadIdx.x / kFwdGroup, tid = threadIdx.x % kFwdGroup;
+    float *sq = sm, *sk = sm + S::kQ + group * (S::kKP + S::kV), *sp = sk, *sv = sk + S::kKP;
     const int lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
-    const int row0 = 16 * (threadIdx.x >> 5) + ty;  // this thread's rows: row0 + 4 r
+    const int row0 = 16 * (tid >> 5) + ty;  // this thread's rows: row0 + 4 r
     const int nq = (T + kFwdRows - 1) / kFwdRows;
     const int nbh = gridDim.x / nq;
     const int q0 = (nq - 1 - (int)blockIdx.x / nbh) * kFwdRows;  // longest rows first
@@ -328,7 +385,9 @@ __global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *_
 
     tc05::pdl_launch_dependents();
     tc05::pdl_wait();
-    load_rows_async<kFwdRows, kPitch, kFwdThreads, kVec>(sq, head, C3, q0, T, D);
+    load_rows_async<kFwdRows, kPitch, kFwdThreads, kVec>(sq, head, C3, q0, T, D, threadIdx.x);
+    async_wait_all();
+    __syncthreads();
     f32x2 o[kR][2 * kNI];
     float m[kR], l[kR];
 #pragma unroll
@@ -338,13 +397,13 @@ __global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *_
         for (int i = 0; i < 2 * kNI; i++) o[r][i] = 0ull;
     }
     const int last = min(q0 + kFwdRows, T) - 1;
-    for (int j0 = 0; j0 <= last; j0 += kKeys) {
-        load_rows_async<kKeys, kPitch, kFwdThreads, kVec>(sk, head + C, C3, j0, T, D);
+    for (int j0 = group * kKeys; j0 <= last; j0 += 2 * kKeys) {
+        load_rows_async<kKeys, kPitch, kFwdGroup, kVec>(sk, head + C, C3, j0, T, D, tid);
         async_commit();
-        load_rows_async<kKeys, kPitch, kFwdThreads, kVec>(sv, head + 2 * C, C3, j0, T, D);
+        load_rows_async<kKeys, kPitch, kFwdGroup, kVec>(sv, head + 2 * C, C3, j0, T, D, tid);
         async_commit();
         async_wait<1>();
-        __syncthreads();
+        group_sync(group);
         float p[kR][kC];
         {
             f32x2 acc[kR][kC];
@@ -368,9 +427,10 @@ __global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *_
             for (int c = 1; c < kC; c++) mx = fmaxf(mx, p[r][c]);
 #pragma unroll
             for (int s = 1; s < 8; s <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
-            mx = fmaxf(mx, m[r]);  // finite: key 0 of the first tile is never masked
-            const float alpha = expf(m[r] - mx);
+            mx = fmaxf(mx, m[r]);
+            const float alpha = mx == -INFINITY ? 1.f : expf(m[r] - mx);
             m[r] = mx;
+            if (mx == -INFINITY) mx = 0.f;  // group 1 may start with a tile that lies past all keys of a row
             l[r] *= alpha;
             const f32x2 a2 = both(alpha);
 #pragma unroll
@@ -381,13 +441,13 @@ __global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *_
                 l[r] += p[r][c];
             }
         }
-        __syncthreads();  // K has been read by everybody: its place takes P
+        group_sync(group);  // K has been read by everybody: its place takes P
 #pragma unroll
         for (int r = 0; r < kR; r++)
 #pragma unroll
             for (int c = 0; c < kC; c++) sp[(row0 + 4 * r) * kPPitch + tx + 8 * c] = p[r][c];
         async_wait<0>();
-        __syncthreads();
+        group_sync(group);
 #pragma unroll 1
         for (int j = 0; j < kKeys; j += 4) {
             float4 pr[kR];
@@ -409,15 +469,38 @@ __global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *_
                 }
             }
         }
-        __syncthreads();  // P and V have been read: the next tile may overwrite them
+        group_sync(group);  // P and V have been read: the next tile may overwrite them
     }
+#pragma unroll
+    for (int r = 0; r < kR; r++)
+#pragma unroll
+        for (int s = 1; s < 8; s <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], s);
+    // group 1 leaves its output sums in its own tiles, maximum and sum of every row in the Q tile
+    f32x2 *po = reinterpret_cast<f32x2 *>(sm + S::kQ + S::kKP + S::kV);
+    float *ml = sm;
+    __syncthreads();
+    if (group == 1) {
+#pragma unroll
+        for (int r = 0; r < kR; r++) {
+            ml[r * kFwdGroup + tid] = m[r];
+            ml[(kR + r) * kFwdGroup + tid] = l[r];
+#pragma unroll
+            for (int i = 0; i < 2 * kNI; i++) po[(r * 2 * kNI + i) * kFwdGroup + tid] = o[r][i];
+        }
+    }
+    __syncthreads();
+    if (group == 1) return;
 #pragma unroll
     for (int r = 0; r < kR; r++) {
         const int t = q0 + row0 + 4 * r;
-        float sum = l[r];
-#pragma unroll
-        for (int s = 1; s < 8; s <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
         if (t >= T) continue;
+        // the other group's thread of this number has the same rows and columns
+        const float m1 = ml[r * kFwdGroup + tid], top = fmaxf(m[r], m1);
+        const float by0 = expf(m[r] - top), by1 = expf(m1 - top);  // m1 is -inf when that group had no tile
+        const float sum = l[r] * by0 + ml[(kR + r) * kFwdGroup + tid] * by1;
+        const f32x2 w0 = both(by0), w1 = both(by1);
+#pragma unroll
+        for (int i = 0; i < 2 * kNI; i++) o[r][i] = fma_x2(o[r][i], w0, mul_x2(po[(r * 2 * kNI + i) * kFwdGroup + tid], w1));
         const float inv = 1.0f / sum;
         const size_t at = ((size_t)b * T + t) * C + (size_t)h * D;
 #pragma unroll
@@ -427,7 +510,7 @@ __global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *_
             store_cols<kVec>(out + at, 4 * tx + 32 * i, D, v);
             if (out_copy) store_cols<kVec>(out_copy + at, 4 * tx + 32 * i, D, v);
         }
-        if (tx == 0) lse[(size_t)bh * T + t] = m[r] + logf(sum);
+        if (tx == 0) lse[(size_t)bh * T + t] = top + logf(sum);
     }
 }
 
@@ -516,7 +599,7 @@ __global__ void __launch_bounds__(kBwdThreads) generic_bwd_kernel(const __nv_bfl
         for (int i = 0; i < 2 * kNI; i++) grad[r][i] = 0ull;
 
     for (int q0 = k0; q0 < T; q0 += kRows) {
-        load_rows_async<kRows, kPitch, kBwdThreads, kVec>(sg, dhead, (size_t)C, q0, T, D);
+        load_rows_async<kRows, kPitch, kBwdThreads, kVec>(sg, dhead, (size_t)C, q0, T, D, threadIdx.x);
         async_commit();
         load_rows_split<kRows, kPitch, kBwdThreads, kVec>(sq, xhi + head, xlo + head, C3, q0, T, D);
         if (threadIdx.x < 2 * kRows) {
@@ -683,11 +766,10 @@ cudaError_t generic_set_attributes() {
 }
 
 cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t n, cudaStream_t s) {
-    const size_t work = (n + 7) / 8;
-    size_t blocks = (work + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (blocks == 0) blocks = 1;
-    return launch_after_previous(split_kernel, dim3((unsigned)blocks), dim3(256), 0, s, x, hi, lo, n);
+    const size_t pieces = (n / 8 + 255) / 256;
+    if (pieces <= 148 * 16)  // one trip of the loop
+        return launch_after_previous(split_small_kernel, dim3((unsigned)(pieces ? pieces : 1)), dim3(256), 0, s, x, hi, lo, n);
+    return launch_after_previous(split_kernel, dim3((unsigned)((pieces + 1) / 2)), dim3(256), 0, s, x, hi, lo, n);
 }
 
 cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta, __nv_bfloat16 *dhi,
