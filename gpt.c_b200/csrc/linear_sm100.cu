@@ -20,8 +20,8 @@
 // the tensor core and arrives at the 55 to 62 bytes per cycle an SM gets from L2 when all of them ask; a CTA on its
 // own needs 48 KB for half the work (64 % tensor pipe active).  The result is written straight from registers, a row
 // per lane in 32-byte sectors: staging it for the copy engine costs shared memory that the pipeline wants (7 stages
-// instead of 6), bandwidth, and hand-overs between warps.  8192 x 3072 x 768: forward 67.0 -> 58.4 us, dx of the
-// same layer 69 -> 61 us, dW 61 -> 53 us; with bf16 planes (QKV) 62.7 -> 56 us.
+// instead of 6), bandwidth, and hand-overs between warps.  8192 x 3072 x 768: forward 67.0 -> 62.6 us, dW 61 -> 53.7 us;
+// 8192 x 768 x 3072: forward 70 -> 61.6 us, dx 69 -> 61.7 us; QKV with bf16 planes 62.7 -> 57.4 us.
 //
 // Warp roles (384 threads, one CTA per SM, grid = number of SMs, tiles handed out round robin):
 //   warp 0      TMA producer
