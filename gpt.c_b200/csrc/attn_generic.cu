@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
 // kNI = head columns in blocks of 32 (the output tile's width), so D = 80 does 96 columns of output work; the
 // score products run over exactly the 4-column words that hold data.
 // The kernels they replace (one warp per row, K and V read again from L2 for every row) took 83 ms for forward
-// and backward of B=4 T=1024 H=6 D=128; these take 0.71 ms (23 GFLOP of fp32 products, a third of the fp32 rate
+// and backward of B=4 T=1024 H=6 D=128; these take 0.68 ms (23 GFLOP of fp32 products, a third of the fp32 rate
 // of 148 SMs).
 // ---------------------------------------------------------------------------------------
 typedef unsigned long long f32x2;  // two floats of a packed instruction
@@ -598,17 +598,61 @@ __global__ void __launch_bounds__(kBwdThreads) generic_bwd_kernel(const __nv_bfl
 #pragma unroll
         for (int i = 0; i < 2 * kNI; i++) grad[r][i] = 0ull;
 
-    for (int q0 = k0; q0 < T; q0 += kRows) {
+    // A query tile is loaded while dQ of the one before it is computed, the last product, which reads neither: dO by
+    // asynchronous copies, Q (split rows) and the row statistics through registers.
+    constexpr int kRowsEach = kRows / (kBwdThreads / 8);
+    uint2 qh[kRowsEach][kNI], ql[kRowsEach][kNI];
+    float stat = 0.f;
+    auto request = [&](int q0) {
         load_rows_async<kRows, kPitch, kBwdThreads, kVec>(sg, dhead, (size_t)C, q0, T, D, threadIdx.x);
         async_commit();
-        load_rows_split<kRows, kPitch, kBwdThreads, kVec>(sq, xhi + head, xlo + head, C3, q0, T, D);
-        if (threadIdx.x < 2 * kRows) {
-            const int r = threadIdx.x % kRows;
-            const float *src = threadIdx.x < kRows ? lse : delta;
-            s_lse[threadIdx.x] = q0 + r < T ? src[(size_t)bh * T + q0 + r] : 0.f;
+        if (kVec) {
+#pragma unroll
+            for (int i = 0; i < kRowsEach; i++) {
+                const int r = q0 + ((int)threadIdx.x >> 3) + i * (kBwdThreads / 8);
+                const size_t at = head + (size_t)(r < T ? r : 0) * C3;
+#pragma unroll
+                for (int u = 0; u < kNI; u++) {
+                    const int w = (threadIdx.x & 7) + 8 * u;
+                    const bool in = r < T && w < words;
+                    qh[i][u] = in ? __ldg(reinterpret_cast<const uint2 *>(xhi + at) + w) : make_uint2(0, 0);
+                    ql[i][u] = in ? __ldg(reinterpret_cast<const uint2 *>(xlo + at) + w) : make_uint2(0, 0);
+                }
+            }
         }
+        if (threadIdx.x < 2 * kRows) {
+            const int t = q0 + (int)threadIdx.x % kRows;
+            const float *src = threadIdx.x < kRows ? lse : delta;
+            stat = t < T ? src[(size_t)bh * T + t] : 0.f;
+        }
+    };
+    auto place = [&](int q0) {  // what request() holds in registers; the tile is complete behind the next barrier
+        if (kVec) {
+#pragma unroll
+            for (int i = 0; i < kRowsEach; i++) {
+                float *row = sq + (((int)threadIdx.x >> 3) + i * (kBwdThreads / 8)) * kPitch;
+#pragma unroll
+                for (int u = 0; u < kNI; u++) {
+                    const int w = (threadIdx.x & 7) + 8 * u;
+                    const uint2 h = qh[i][u], l = ql[i][u];
+                    if (w < words)
+                        *reinterpret_cast<float4 *>(row + 4 * w) =
+                            make_float4(__uint_as_float(h.x << 16) + __uint_as_float(l.x << 16),
+                                        __uint_as_float(h.x & 0xffff0000u) + __uint_as_float(l.x & 0xffff0000u),
+                                        __uint_as_float(h.y << 16) + __uint_as_float(l.y << 16),
+                                        __uint_as_float(h.y & 0xffff0000u) + __uint_as_float(l.y & 0xffff0000u));
+                }
+            }
+        } else {
+            load_rows_split<kRows, kPitch, kBwdThreads, kVec>(sq, xhi + head, xlo + head, C3, q0, T, D);
+        }
+        if (threadIdx.x < 2 * kRows) s_lse[threadIdx.x] = stat;
         async_wait<0>();
-        __syncthreads();
+    };
+    request(k0);
+    place(k0);
+    __syncthreads();
+    for (int q0 = k0; q0 < T; q0 += kRows) {
         {
             f32x2 acc[kR][kC];
             if (group == 0) {
@@ -639,7 +683,9 @@ __global__ void __launch_bounds__(kBwdThreads) generic_bwd_kernel(const __nv_bfl
         }
         if (group == 0) key_gradient<kR, kNI, kRows, kPPitch, kPitch>(grad, sp + key0, sg + 4 * tx);
         else key_gradient<kR, kNI, kRows, kPPitch, kPitch>(grad, sd + key0, sq + 4 * tx);
-        __syncthreads();  // dS is complete for everybody
+        __syncthreads();  // dS is complete for everybody; Q, dO, P and the statistics have been read
+        const bool more = q0 + kRows < T;
+        if (more) request(q0 + kRows);
         {
             f32x2 dq[kR][2 * kQI];
 #pragma unroll
@@ -693,7 +739,8 @@ __global__ void __launch_bounds__(kBwdThreads) generic_bwd_kernel(const __nv_bfl
                 }
             }
         }
-        __syncthreads();  // Q, dO, P and dS may be overwritten
+        if (more) place(q0 + kRows);
+        __syncthreads();  // the next tile is in place, dS may be overwritten
     }
     const float by = group == 0 ? 1.0f : scale;
 #pragma unroll
