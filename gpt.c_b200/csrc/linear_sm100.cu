@@ -66,6 +66,7 @@ struct Problem {
     size_t plane_words;     // distance from the hi to the lo plane
     size_t ldc;             // floats from one row of C to the next
     int b_shift;            // B's contraction index runs this far behind A's (see RowClasses)
+    int a_whole[4];         // columns in whole blocks of A's views
     int a_shift[4];         // columns of A's views before the first column of dy (dW from row classes)
     int m_fast;  // consecutive work items walk down the rows of C (else along its columns)
 };
@@ -78,6 +79,9 @@ enum Site : int {
 template <bool kClasses>
 struct Maps {
     CUtensorMap a[kClasses ? 4 : 1], b[kClasses ? 4 : 1], c;
+    // row classes: A's 32-column blocks that are whole, fetched a tile at a time (`a` has the columns after them too,
+    // but takes four copies, and the thread that requests them is then the limit)
+    CUtensorMap a_whole[kClasses ? 4 : 1];
 };
 
 // Rows of dy whose pitch is not a multiple of 16 bytes (the vocabulary projection: 50257 floats) cannot be tiled by the
@@ -220,7 +224,9 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                     // K-major: map {contraction, rows}, one box {32, 128}.  MN-major: map {rows, contraction},
                     // four boxes {32, 32}: blocks of 32 rows, each [32 contraction steps x 128 bytes].
                     if (kAMN) {
-                        if (p.a_one) {
+                        if (kClasses && wk.m0 + kBM <= p.a_whole[wk.cls]) {
+                            load(sm.a[st], &maps.a_whole[kClasses ? wk.cls : 0], 0, kb * kBK, wk.m0 / 32);
+                        } else if (p.a_one) {
                             load(sm.a[st], &map_a, 0, kb * kBK, wk.m0 / 32);
                         } else {
 #pragma unroll
@@ -517,7 +523,7 @@ Problem make_problem(int M, int N, int K, int bn, int pair, int splits) {
     p.m_fast = 0;
     p.ldc = (size_t)N;
     p.b_shift = 0;
-    for (int i = 0; i < 4; i++) p.a_shift[i] = 0;
+    for (int i = 0; i < 4; i++) p.a_shift[i] = p.a_whole[i] = 0;
     p.tiles_m = (M + tile_rows(pair) - 1) / tile_rows(pair);
     p.tiles_n = (N + bn - 1) / bn;
     p.kb_total = (K + kBK - 1) / kBK;
@@ -627,7 +633,7 @@ int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *p
 template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
 int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
                const Problem &p, int *status, cudaStream_t s) {
-    const Maps<false> maps = {{ma}, {mb}, mc};
+    const Maps<false> maps = {{ma}, {mb}, mc, {ma}};
     return launch_maps<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair>(maps, bias, c, planes, p, status, s);
 }
 
@@ -706,6 +712,12 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
     for (int j = 0; j < 4; j++) {
         const RowClass c = row_class(dy, M, N, j);
         p.a_shift[j] = c.shift;
+        p.a_whole[j] = (N + c.shift) / 32 * 32;
+        if (p.a_whole[j] > 0) {
+            if ((rc = map_mn_major_blocks(&maps.a_whole[j], c.dy, c.rows, p.a_whole[j], 4, 4 * (size_t)N)) != 0) return rc;
+        } else {
+            maps.a_whole[j] = {};
+        }
         if ((rc = map_mn_major(&maps.a[j], c.dy, c.rows, N + c.shift, 4 * (size_t)N)) != 0) return rc;
         if ((rc = map_mn_major_blocks(&maps.b[j], x + (size_t)j * K, c.rows, K, p.bn / 64, 4 * (size_t)K)) != 0) return rc;
     }
