@@ -134,8 +134,14 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const float *__restric
 
 // ---------------------------------------------------------------------------------------
 // backward preparation for head size 64 (the tensor-core path): the same work as above with
-// 8 consecutive elements per thread, so 8 lanes cover one (b, t, h) row of 64 values.
+// 8 consecutive elements per thread, so 8 lanes cover one (b, t, h) row of 64 values.  HBM bound: 32 bytes per access,
+// one piece per block (1.68 GB: 283 us with 16-byte accesses in a grid-stride loop, 261 us now; 260 at the copy rate).
 // ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void load8_last_use(const float *p, float4 &a, float4 &b) {
+    asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
 __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restrict__ dout, const float *__restrict__ out,
                                                              float *__restrict__ delta, __nv_bfloat16 *__restrict__ dhi,
                                                              __nv_bfloat16 *__restrict__ dlo, float *__restrict__ dq_zero,
@@ -145,18 +151,22 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
     if (sched && blockIdx.x == 0 && threadIdx.x < 2) sched[threadIdx.x] = 0;  // item counter of the backward core
     const int C = H * 64;
     const size_t nvec = (size_t)B * T * C / 8;  // multiple of 8, so whole groups of 8 lanes stay together
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    // the loop bound is warp-uniform (shuffles below need every lane); memory accesses are guarded
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v - lane < nvec; v += stride) {
+    const bool wide = ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dq_zero)) & 31u) == 0;
+    const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v - lane < nvec) {  // warp-uniform (shuffles below need every lane); memory accesses are guarded
         const bool active = v < nvec;
         const size_t bt = v / (C / 8);
         const int c8 = (int)(v % (C / 8));
         const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 g0 = active ? __ldcs(reinterpret_cast<const float4 *>(dout) + 2 * v) : zero4;
-        const float4 g1 = active ? __ldcs(reinterpret_cast<const float4 *>(dout) + 2 * v + 1) : zero4;
-        const float4 o0 = active ? __ldcs(reinterpret_cast<const float4 *>(out) + 2 * v) : zero4;
-        const float4 o1 = active ? __ldcs(reinterpret_cast<const float4 *>(out) + 2 * v + 1) : zero4;
+        float4 g0 = zero4, g1 = zero4, o0 = zero4, o1 = zero4;
+        if (active && wide) {
+            load8_last_use(dout + 8 * v, g0, g1);
+            load8_last_use(out + 8 * v, o0, o1);
+        } else if (active) {
+            g0 = __ldcs(reinterpret_cast<const float4 *>(dout) + 2 * v), g1 = __ldcs(reinterpret_cast<const float4 *>(dout) + 2 * v + 1);
+            o0 = __ldcs(reinterpret_cast<const float4 *>(out) + 2 * v), o1 = __ldcs(reinterpret_cast<const float4 *>(out) + 2 * v + 1);
+        }
         float acc = g0.x * o0.x + g0.y * o0.y + g0.z * o0.z + g0.w * o0.w + g1.x * o1.x + g1.y * o1.y + g1.z * o1.z +
                     g1.w * o1.w;
         acc += __shfl_xor_sync(0xffffffffu, acc, 1);
@@ -171,12 +181,16 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
             hw[k] = *reinterpret_cast<uint32_t *>(&hh);
             lw[k] = *reinterpret_cast<uint32_t *>(&ll);
         }
-        if (!active) continue;
+        if (!active) return;
         reinterpret_cast<uint4 *>(dhi)[v] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
         reinterpret_cast<uint4 *>(dlo)[v] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         float4 *z = reinterpret_cast<float4 *>(dq_zero + bt * 3 * C + (size_t)c8 * 8);
-        z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-        z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (wide) {
+            asm volatile("st.global.v8.f32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"l"(z), "f"(0.f) : "memory");
+        } else {
+            z[0] = zero4;
+            z[1] = zero4;
+        }
         if ((c8 & 7) == 0) {
             const int h = c8 >> 3, t = (int)(bt % T), b = (int)(bt / T);
             delta[((size_t)b * H + h) * T + t] = acc;
@@ -823,8 +837,7 @@ cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta
                                __nv_bfloat16 *dlo, float *dq_zero, int *sched, int B, int T, int H, int D, cudaStream_t s) {
     if (D == 64 && dhi && dlo) {
         const size_t nvec = (size_t)B * T * H * 8;
-        size_t blocks = (nvec + 255) / 256;
-        if (blocks > 148 * 16) blocks = 148 * 16;
+        const size_t blocks = (nvec + 255) / 256;
         return launch_after_previous(bwd_prepare64_kernel, dim3((unsigned)blocks), dim3(256), 0, s, dout, out, delta, dhi,
                                      dlo, dq_zero, sched, B, T, H);
     }
