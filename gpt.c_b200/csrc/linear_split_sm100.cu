@@ -254,15 +254,15 @@ int rows_per_tile(int M) {
 // separate rows arrive; sharing an SM makes it 390 to 600 ns; cluster barriers and the exchange cost 1.3 us.
 int plan_split(int M, int cols, int kc, int *split) {
     const int bm = rows_per_tile(M), units = (cols + kBM - 1) / kBM * ((M + bm - 1) / bm), kb = (kc + kBK - 1) / kBK;
-    int best = 0;
+    long long best = 0;
     for (int s = 1; s <= kMaxSplit; s++) {
         if (kAlone[s] == 0 || s > kb || (s > 1 && units * s > 2 * kAlone[s])) continue;
         const int per = (kb + s - 1) / s;
-        const int t = s == 1 ? 1650 + 16 * bm + (units <= 148 ? 295 * per : (400 * per + 1000) * units / 148)
-                             : 2900 + 16 * bm + per * (units * s <= kAlone[s] ? 310 : 300 + 2 * bm);
+        const long long t = s == 1 ? 1650 + 16 * bm + (units <= 148 ? 295ll * per : (400ll * per + 1000) * units / 148)
+                             : 2900 + 16 * bm + (long long)per * (units * s <= kAlone[s] ? 310 : 300 + 2 * bm);
         if (best == 0 || t < best) best = t, *split = s;
     }
-    return best;
+    return best < 0x7fffffff ? (int)best : 0x7fffffff;
 }
 
 int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, const float *bias, float *out, void *planes, int M,
