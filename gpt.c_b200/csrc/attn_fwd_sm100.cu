@@ -329,10 +329,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
     // Every role walks the same items: its own block's, then those answered for by the requests.  `t` counts the
     // items of this CTA, `n` their key steps; both number the phases of the barriers (the answer that names item t
     // is the t-th one, in slot (t - 1) % 4).
-    auto next_item = [&](int t) -> int {
-        if (kFp32) return -1;
-        if (!mbar_wait_warp(&sm.next_full[(t - 1) & 3], ((t - 1) >> 2) & 1, ctx, SITE_NEXT)) return -1;
-        return item_of(&sm.next[(t - 1) & 3]);
+    auto next_item = [&](int) -> int {
+        return -1;
     };
 
     if (kFp32 && threadIdx.x == 0) {  // what the copy engine signals otherwise
@@ -357,13 +355,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
                     if (ok) load_q(sm, map_x, w);
                 }
                 for (int j = 0; ok && j < w.nsteps; j++, n++) {
-                    if (j == w.nsteps - 1) {
-                        // near the end of the item, so that a CTA with a long one does not hold the next; the answer
-                        // takes about as long as the three steps that are left
-                        fence_proxy_async_smem();
-                        mbar_expect_tx(&sm.next_full[t & 3], 16);
-                        request_item(&sm.next[t & 3], &sm.next_full[t & 3]);
-                    }
                     if (t == 0 && j < 2) continue;  // requested during set-up
                     ok = n < 2 || mbar_wait(&sm.k_empty[n & 1], ((n >> 1) - 1) & 1, ctx, SITE_K_EMPTY);
                     if (!ok) break;

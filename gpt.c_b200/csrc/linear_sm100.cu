@@ -180,8 +180,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     }
     if (warp == 2) {
         if (kPair) {
-            tmem_alloc_pair(&sm.tmem_base, kTmemCols);
-            tmem_relinquish_pair();
+            tmem_alloc_pair(&sm.tmem_base, kTmemCols);  // the permit is given back at the end
         } else {
             tmem_alloc(&sm.tmem_base, kTmemCols);
             tmem_relinquish();
@@ -402,9 +401,16 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     if (kPair) cluster_sync_all();
     if (warp == 2) {
         tc_fence_after_sync();
-        if (kPair) tmem_dealloc_pair(tmem, kTmemCols);
-        else tmem_dealloc(tmem, kTmemCols);
+        if (kPair) {
+            tmem_relinquish_pair();
+            tmem_dealloc_pair(tmem, kTmemCols);
+        } else {
+            tmem_dealloc(tmem, kTmemCols);
+        }
     }
+    // Allocation state is the pair's: neither SM may be handed to another kernel, which allocates for itself, before
+    // both CTAs have freed their columns.
+    if (kPair) cluster_sync_all();
 }
 
 // db[n] += sum_m dy[m, n].  A block covers 128 columns (one float4 per lane) and every 8th row of its
@@ -554,8 +560,7 @@ struct Plan {
 struct Cost {
     int pair, bn, fixed, round, block;  // nanoseconds
 };
-constexpr Cost kCosts[6] = {{1, 256, 5090, 2300, 298}, {1, 192, 4440, 1660, 264}, {1, 128, 4350, 840, 258},
-                            {0, 256, 4470, 2030, 283}, {0, 192, 4450, 900, 232},  {0, 128, 3920, 400, 226}};
+constexpr Cost kCosts[3] = {{0, 256, 4470, 2030, 283}, {0, 192, 4450, 900, 232}, {0, 128, 3920, 400, 226}};
 constexpr int kL2BytesPerNs = 18190;
 
 // Time of `tiles` tiles of kb contraction blocks each, without the fixed part.
@@ -644,16 +649,6 @@ int launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, 
 #define GO(bn, stages, with_planes, pair) \
     return launch_one<kAMN, kBMN, kEpi, bn, stages, with_planes, false, pair>(ma, mb, mc, bias, c, planes, p, status, s)
     constexpr bool kCanPlanes = !kAMN && !kBMN && kEpi == 0;  // only the forward product writes planes
-    if (p.pair) {
-        if constexpr (kCanPlanes) {
-            if (planes && p.bn == 256) GO(256, 7, true, true);
-            if (planes && p.bn == 192) GO(192, 7, true, true);
-            if (planes) GO(128, 6, true, true);
-        }
-        if (p.bn == 256) GO(256, kEpi == 1 ? 6 : 7, false, true);
-        if (p.bn == 192) GO(192, kEpi == 1 ? 6 : 7, false, true);
-        GO(128, 6, false, true);
-    }
     if constexpr (kCanPlanes) {
         if (planes && p.bn == 256) GO(256, 4, true, false);
         if (planes && p.bn == 192) GO(192, 5, true, false);
@@ -706,7 +701,7 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
     if (!dw) return ATTN_OK;
     // the four classes of a tile follow each other, so that the tile of dW they add into stays in L2
     Maps<true> maps;
-    Problem p = make_problem(N, K, (M + 3) / 4, K % 256 == 0 ? 256 : 128, 1, 1);
+    Problem p = make_problem(N, K, (M + 3) / 4, K % 256 == 0 ? 256 : 128, 0, 1);
     p.splits = 4, p.total *= 4;
     p.a_one = 0, p.b_one = 1;
     for (int j = 0; j < 4; j++) {
@@ -719,14 +714,14 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
             maps.a_whole[j] = {};
         }
         if ((rc = map_mn_major(&maps.a[j], c.dy, c.rows, N + c.shift, 4 * (size_t)N)) != 0) return rc;
-        if ((rc = map_mn_major_blocks(&maps.b[j], x + (size_t)j * K, c.rows, K, p.bn / 64, 4 * (size_t)K)) != 0) return rc;
+        if ((rc = map_mn_major_blocks(&maps.b[j], x + (size_t)j * K, c.rows, K, p.bn / 32, 4 * (size_t)K)) != 0) return rc;
     }
     // up to three rows of the last tile may only be reached through the shifted views
-    p.tiles_m = (N + 3 + tile_rows(1) - 1) / tile_rows(1);
+    p.tiles_m = (N + 3 + tile_rows(0) - 1) / tile_rows(0);
     p.total = p.tiles_m * p.tiles_n * p.splits;
     if ((rc = map_out_f32(&maps.c, dw, N, K)) != 0) return rc;
-    if (p.bn == 256) return launch_maps<true, true, 1, 256, 6, false, false, true, true>(maps, nullptr, dw, nullptr, p, status, s);
-    return launch_maps<true, true, 1, 128, 6, false, false, true, true>(maps, nullptr, dw, nullptr, p, status, s);
+    if (p.bn == 256) return launch_maps<true, true, 1, 256, 4, false, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
+    return launch_maps<true, true, 1, 128, 6, false, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
 }
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
@@ -776,12 +771,11 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     if (plan_split(M, N, K, &split) < plan.ns) return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, status, s);
     CUtensorMap ma, mb;
     // with plain stores (N not a multiple of 4) only the widest tiles are built
-    Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, direct ? M > kBM : plan.pair, 1);
+    Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, plan.pair, 1);
     p.m_fast = stream_rows_of_c(M, N, K);
     if ((rc = map_k_major(&ma, x, M, K, 128)) != 0) return rc;
     if ((rc = map_k_major(&mb, w, N, K, p.bn / (p.pair ? 2 : 1))) != 0) return rc;
     if (direct) {
-        if (p.pair) return launch_one<false, false, 0, 256, 6, false, true, true>(ma, mb, ma, bias, y, nullptr, p, status, s);
         return launch_one<false, false, 0, 256, 4, false, true, false>(ma, mb, ma, bias, y, nullptr, p, status, s);
     }
     return launch<false, false, 0>(ma, mb, ma, bias, y, planes, p, status, s);
