@@ -8,13 +8,8 @@
 // diagonal in steps of 64.  Inputs are the bf16 hi/lo planes of the fused QKV tensor; Q/K/V tiles are
 // addressed straight inside [B, T, 3C] by a 4-D tensor map (column, row, batch, plane).
 //
-// The grid has one CTA per item, heaviest first, but a CTA that runs takes over items of CTAs that have
-// not started (clusterlaunchcontrol.try_cancel), one request ahead: at the end of an item the next Q tile
-// is in shared memory, the first keys are in the ring, and the tensor cores start on the next scores while
-// the softmax warps still write the finished tile.  With a CTA per item, half of a CTA's life went into
-// being set up (first scores 1.6 us after the start), into its epilogue and exit (2 us).  Forward core alone,
-// before and after: B=32 T=1024 H=16 249 -> 225 us, B=8 T=1024 H=12 44.8 -> 41.4 us, B=64 T=128 H=12 25.4 -> 20.5 us,
-// B=1 T=40 H=2 5.7 -> 4.3 us (a single key step where two were taken).
+// The grid has one CTA per item, heaviest first.  The first Q and K tiles are requested while the CTA is still being set
+// up, the finished tile is written straight from registers.  A sequence of at most 64 tokens takes one key step.
 //
 // A CTA is deliberately small (about 100 KiB of shared memory, 256 columns of tensor memory,
 // 384 threads) so that TWO CTAs share an SM.  Inside a CTA two score buffers alternate, so the
@@ -22,7 +17,7 @@
 // In the steady state a step takes about 1000 cycles of an SM, 800 of which its 24 MMAs execute.
 //
 // Warp roles (384 threads):
-//   warp 0       TMA producer for Q and K (two-stage ring), requests the next item
+//   warp 0       TMA producer for Q and K (two-stage ring)
 //   warp 1       tensor-memory allocation / release
 //   warp 2       MMA issuer (not on the scheduler of the TMA warps: 2 % faster): S = Q K^T (Q from tensor memory, K K-major from shared memory) and O += P V (P from tensor memory,
 //                V MN-major from shared memory), each as hi*hi + hi*lo + lo*hi; the whole warp
@@ -61,9 +56,7 @@ struct __align__(1024) FwdSmem {
     uint8_t q[2][kPlaneTile];  // [plane]
     uint8_t k[2][2][kPlaneStep];  // [stage][plane]
     uint8_t v[2][2][kPlaneStep];
-    uint4 next[4];              // answers to the requests for items, by item number of this CTA
-    uint64_t next_full[4];
-    uint64_t q_full, q_free, q_tmem, k_full[2], k_empty[2], v_full[2], v_empty[2];
+    uint64_t q_full, q_tmem, k_full[2], k_empty[2], v_full[2], v_empty[2];
     uint64_t s_full[2], p_full[2], o_full;
     uint64_t pair_bar[4];       // [quarter]: the two halves of a row block meet here once per step
     uint64_t o_done;            // the last PV product of an item has completed
@@ -75,34 +68,8 @@ struct __align__(1024) FwdSmem {
 
 enum Site : int {
     SITE_K_EMPTY = 1, SITE_V_EMPTY, SITE_Q_FULL, SITE_K_FULL, SITE_V_FULL, SITE_P_FULL, SITE_S_FULL, SITE_O_FULL,
-    SITE_O_FULL_LAST, SITE_Q_TMEM, SITE_Q_FREE, SITE_NEXT, SITE_PAIR, SITE_SMEM_ALIGN
+    SITE_O_FULL_LAST, SITE_Q_TMEM, SITE_PAIR, SITE_SMEM_ALIGN
 };
-
-// Asks for an item whose CTA has not started; the 16-byte answer is counted on `bar`.
-__device__ __forceinline__ void request_item(uint4 *answer, uint64_t *bar) {
-    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
-                     smem_u32(answer)),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
-// The item number in an answer, or -1 when there was none left.
-__device__ __forceinline__ int item_of(const uint4 *answer) {
-    int item;
-    asm volatile(
-        "{\n\t"
-        ".reg .b128 r;\n\t"
-        ".reg .pred p;\n\t"
-        ".reg .b32 y, z, w;\n\t"
-        "ld.shared.b128 r, [%1];\n\t"
-        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
-        "mov.b32 %0, -1;\n\t"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, y, z, w}, r;\n\t"
-        "}"
-        : "=r"(item)
-        : "r"(smem_u32(answer))
-        : "memory");
-    return item;
-}
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -285,9 +252,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         mbar_init(&sm.q_full, 1);
-        mbar_init(&sm.q_free, kSoftmaxWarps);
         mbar_init(&sm.q_tmem, kSoftmaxWarps);
-        for (int i = 0; i < 4; i++) mbar_init(&sm.next_full[i], 1);
         for (int i = 0; i < 2; i++) {
             mbar_init(&sm.k_full[i], 1);
             mbar_init(&sm.k_empty[i], 1);
@@ -326,13 +291,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
 
-    // Every role walks the same items: its own block's, then those answered for by the requests.  `t` counts the
-    // items of this CTA, `n` their key steps; both number the phases of the barriers (the answer that names item t
-    // is the t-th one, in slot (t - 1) % 4).
-    auto next_item = [&](int) -> int {
-        return -1;
-    };
-
+    const Item w = decode((int)blockIdx.x, B, T, H);
     if (kFp32 && threadIdx.x == 0) {  // what the copy engine signals otherwise
         mbar_arrive(&sm.q_full);
         mbar_arrive(&sm.k_full[0]);
@@ -342,45 +301,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
     if (kFp32 && (warp == 0 || warp == 3)) {
         // no loads to request
     } else if (warp == 0) {
-        // ------------------------------ TMA producer: Q and K; requests ------------------------------
-        int n = 0;
-        bool ok = true;
-        for (int t = 0, item = (int)blockIdx.x; item >= 0; item = next_item(++t)) {
-            const Item w = decode(item, B, T, H);
-            if (lane == 0) {
-                if (t > 0) {
-                    // the Q tile before this one has been copied to tensor memory; by then every role has also read
-                    // the answer that the next request overwrites (it is four items old)
-                    ok = mbar_wait(&sm.q_free, (t - 1) & 1, ctx, SITE_Q_FREE);
-                    if (ok) load_q(sm, map_x, w);
-                }
-                for (int j = 0; ok && j < w.nsteps; j++, n++) {
-                    if (t == 0 && j < 2) continue;  // requested during set-up
-                    ok = n < 2 || mbar_wait(&sm.k_empty[n & 1], ((n >> 1) - 1) & 1, ctx, SITE_K_EMPTY);
-                    if (!ok) break;
-                    load_k(sm, map_x, w, C, j, n & 1);
-                }
+        // ------------------------------ TMA producer: K ------------------------------
+        if (lane == 0) {
+            for (int n = 2; n < w.nsteps; n++) {  // Q and the first two steps were requested during set-up
+                if (!mbar_wait(&sm.k_empty[n & 1], ((n >> 1) - 1) & 1, ctx, SITE_K_EMPTY)) break;
+                load_k(sm, map_x, w, C, n, n & 1);
             }
-            if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
         }
     } else if (warp == 3) {
         // ------------------------------ TMA producer: V ------------------------------
-        int n = 0;
-        bool ok = true;
-        for (int t = 0, item = (int)blockIdx.x; item >= 0; item = next_item(++t)) {
-            const Item w = decode(item, B, T, H);
-            if (lane == 0) {
-                const int xv = 2 * C + w.h * kD;
-                for (int j = 0; j < w.nsteps; j++, n++) {
-                    const int st = n & 1;
-                    ok = n < 2 || mbar_wait(&sm.v_empty[st], ((n >> 1) - 1) & 1, ctx, SITE_V_EMPTY);
-                    if (!ok) break;
-                    mbar_expect_tx(&sm.v_full[st], 2 * kPlaneStep);
-                    tma_load_4d(sm.v[st][0], &map_x, &sm.v_full[st], xv, j * kStep, w.b, 0);
-                    tma_load_4d(sm.v[st][1], &map_x, &sm.v_full[st], xv, j * kStep, w.b, 1);
-                }
+        if (lane == 0) {
+            const int xv = 2 * C + w.h * kD;
+            for (int n = 0; n < w.nsteps; n++) {
+                const int st = n & 1;
+                if (n >= 2 && !mbar_wait(&sm.v_empty[st], ((n >> 1) - 1) & 1, ctx, SITE_V_EMPTY)) break;
+                mbar_expect_tx(&sm.v_full[st], 2 * kPlaneStep);
+                tma_load_4d(sm.v[st][0], &map_x, &sm.v_full[st], xv, n * kStep, w.b, 0);
+                tma_load_4d(sm.v[st][1], &map_x, &sm.v_full[st], xv, n * kStep, w.b, 1);
             }
-            if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
         }
     } else if (warp == 2) {
         // ------------------------------ MMA issuer ------------------------------
@@ -411,52 +349,45 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
             tc_commit_lead(leader, &sm.k_empty[st]);
             return true;
         };
-        int n = 0;
-        bool ok = true;
-        for (int t = 0, item = (int)blockIdx.x; item >= 0; item = next_item(++t)) {
-            const int nsteps = decode(item, B, T, H).nsteps;
-            ok = mbar_wait_warp(&sm.q_tmem, t & 1, ctx, SITE_Q_TMEM) && issue_qk(n);
-            for (int j = 0; ok && j < nsteps; j++, n++) {
-                const int st = n & 1;
-                ok = (j + 1 == nsteps || issue_qk(n + 1)) &&
-                     // O += P_j V_j
-                     mbar_wait_warp(&sm.v_full[st], (n >> 1) & 1, ctx, SITE_V_FULL) &&
-                     mbar_wait_warp(&sm.p_full[st], (n >> 1) & 1, ctx, SITE_P_FULL);
-                if (!ok) break;
-                tc_fence_after_sync();
-                const uint64_t vd[2] = {smem_desc_sw128(smem_u32(sm.v[st][0]), 1024, 1024),
-                                        smem_desc_sw128(smem_u32(sm.v[st][1]), 1024, 1024)};
-                uint32_t acc = j >= 1 ? 1u : 0u;
-#pragma unroll
-                for (int term = 0; term < 3; term++) {
-                    const int pa = term == 2 ? 1 : 0, vb = term == 1 ? 1 : 0;  // hh, hl, lh
-#pragma unroll
-                    for (int kk = 0; kk < kStep / 16; kk++) {
-                        mma_ts_lead(leader, tmem + kColO, tmem + kColS + st * kStep + 16 * kk + 8 * pa,
-                                     desc_advance(vd[vb], kk * 2048), idesc_o, acc);
-                        acc = 1;
-                    }
-                }
-                tc_commit_lead(leader, &sm.o_full);
-                tc_commit_lead(leader, &sm.v_empty[st]);
-                if (j == nsteps - 1) tc_commit_lead(leader, &sm.o_done);
-            }
+        bool ok = mbar_wait_warp(&sm.q_tmem, 0, ctx, SITE_Q_TMEM) && issue_qk(0);
+        for (int n = 0; ok && n < w.nsteps; n++) {
+            const int st = n & 1;
+            ok = (n + 1 == w.nsteps || issue_qk(n + 1)) &&
+                 // O += P_n V_n
+                 mbar_wait_warp(&sm.v_full[st], (n >> 1) & 1, ctx, SITE_V_FULL) &&
+                 mbar_wait_warp(&sm.p_full[st], (n >> 1) & 1, ctx, SITE_P_FULL);
             if (!ok) break;
+            tc_fence_after_sync();
+            const uint64_t vd[2] = {smem_desc_sw128(smem_u32(sm.v[st][0]), 1024, 1024),
+                                    smem_desc_sw128(smem_u32(sm.v[st][1]), 1024, 1024)};
+            uint32_t acc = n >= 1 ? 1u : 0u;
+#pragma unroll
+            for (int term = 0; term < 3; term++) {
+                const int pa = term == 2 ? 1 : 0, vb = term == 1 ? 1 : 0;  // hh, hl, lh
+#pragma unroll
+                for (int kk = 0; kk < kStep / 16; kk++) {
+                    mma_ts_lead(leader, tmem + kColO, tmem + kColS + st * kStep + 16 * kk + 8 * pa,
+                                 desc_advance(vd[vb], kk * 2048), idesc_o, acc);
+                    acc = 1;
+                }
+            }
+            tc_commit_lead(leader, &sm.o_full);
+            tc_commit_lead(leader, &sm.v_empty[st]);
+            if (n == w.nsteps - 1) tc_commit_lead(leader, &sm.o_done);
         }
     } else if (warp >= 4) {
         // ------------------------------ softmax ------------------------------
         const int half = (warp - 4) >> 2;       // which 32 score columns / 32 output columns
         const int quarter = warp & 3;           // TMEM lane quarter this warp may access
         const int row = (quarter << 5) | lane;  // query row inside the tile == TMEM lane
-        uint64_t *pair_bar = &sm.pair_bar[quarter];  // one phase per step and one per item
+        uint64_t *pair_bar = &sm.pair_bar[quarter];  // one phase per step and one at the end
         const uint32_t lane_addr = (uint32_t)(quarter << 5) << 16;
         const uint32_t t_o = tmem + lane_addr + kColO + 32 * half;
 
         // Copies this thread's Q row (half 0: hi plane, half 1: lo plane) from the swizzled shared
-        // memory tile into tensor memory: 64 bf16 = 32 packed columns, lane = row.  The scores of the
-        // item before have all been computed by then (this thread has seen the last of them).
-        auto take_q = [&](int t) -> bool {
-            if (!mbar_wait_warp(&sm.q_full, t & 1, ctx, SITE_Q_FULL)) return false;
+        // memory tile into tensor memory: 64 bf16 = 32 packed columns, lane = row.
+        auto take_q = [&]() -> bool {
+            if (!mbar_wait_warp(&sm.q_full, 0, ctx, SITE_Q_FULL)) return false;
             const uint8_t *qrow = sm.q[half] + row * 128;
             uint32_t r[32];
 #pragma unroll
@@ -471,64 +402,53 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&sm.q_tmem);
-                mbar_arrive(&sm.q_free);
-            }
+            if (lane == 0) mbar_arrive(&sm.q_tmem);
             return true;
         };
 
-        int n = 0, item = (int)blockIdx.x;
-        bool ok = take_q(0);
-        for (int t = 0; ok && item >= 0; t++) {
-            const Item w = decode(item, B, T, H);
-            float m = -INFINITY, l = 0.f;
-            for (int j = 0; j < w.nsteps; j++, n++) {
-                const int st = n & 1;
-                const uint32_t t_s = tmem + lane_addr + kColS + st * kStep;
-                const int key0 = j * kStep - w.qt * kTile;  // first key of the step relative to the tile's first row
-                const bool diag = key0 + kStep - 1 > 0;     // some (row, key) pair of this step is above the diagonal
-                if (!mbar_wait_warp(&sm.s_full[st], (n >> 1) & 1, ctx, SITE_S_FULL)) { ok = false; break; }
+        bool ok = take_q();
+        float m = -INFINITY, l = 0.f;
+        for (int n = 0; ok && n < w.nsteps; n++) {
+            const int st = n & 1;
+            const uint32_t t_s = tmem + lane_addr + kColS + st * kStep;
+            const int key0 = n * kStep - w.qt * kTile;  // first key of the step relative to the tile's first row
+            const bool diag = key0 + kStep - 1 > 0;     // some (row, key) pair of this step is above the diagonal
+            if (!mbar_wait_warp(&sm.s_full[st], (n >> 1) & 1, ctx, SITE_S_FULL)) { ok = false; break; }
+            tc_fence_after_sync();
+            float alpha;
+            const bool step_ok = diag
+                ? max_pass<true>(sm, ctx, t_s, row, half, st, key0, pair_bar, n & 1, scale_log2, m, alpha)
+                : max_pass<false>(sm, ctx, t_s, row, half, st, key0, pair_bar, n & 1, scale_log2, m, alpha);
+            if (!step_ok) { ok = false; break; }
+            // When the reference maximum of some row of this warp moved, rescale the warp's 32 rows x
+            // 32 columns of O in place: after the previous PV product has finished, before P_j is
+            // published.  (The barrier completes once per step, and not for this one before P_j is there.)
+            if (n >= 1 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+                if (!mbar_wait_warp(&sm.o_full, (n - 1) & 1, ctx, SITE_O_FULL)) { ok = false; break; }
                 tc_fence_after_sync();
-                float alpha;
-                const bool step_ok = diag
-                    ? max_pass<true>(sm, ctx, t_s, row, half, st, key0, pair_bar, (n + t) & 1, scale_log2, m, alpha)
-                    : max_pass<false>(sm, ctx, t_s, row, half, st, key0, pair_bar, (n + t) & 1, scale_log2, m, alpha);
-                if (!step_ok) { ok = false; break; }
-                // When the reference maximum of some row of this warp moved, rescale the warp's 32 rows x
-                // 32 columns of O in place: after the previous PV product has finished, before P_j is
-                // published.  (The barrier completes once per step, and not for this one before P_j is there.)
-                if (j >= 1 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-                    if (!mbar_wait_warp(&sm.o_full, (n - 1) & 1, ctx, SITE_O_FULL)) { ok = false; break; }
-                    tc_fence_after_sync();
-                    uint32_t r[32];
-                    tmem_ld32(t_o, r);
-                    tmem_wait_ld();
+                uint32_t r[32];
+                tmem_ld32(t_o, r);
+                tmem_wait_ld();
 #pragma unroll
-                    for (int e = 0; e < 32; e++) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
-                    tmem_st32(t_o, r);
-                }
-                l = l * alpha + (diag ? exp_pass<true>(t_s, row, half, key0, scale_log2, m)
-                                      : exp_pass<false>(t_s, row, half, key0, scale_log2, m));
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive(&sm.p_full[st]);
+                for (int e = 0; e < 32; e++) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+                tmem_st32(t_o, r);
             }
-            if (!ok) break;
-            // hand the next Q to the tensor cores before finishing this item
-            item = next_item(t + 1);
-            if (item >= 0 && !take_q(t + 1)) { ok = false; break; }
-
-            // O / l for this thread's 32 columns, log-sum-exp by the first half
-            sm.lpart[half][row] = l;
-            mbar_arrive(pair_bar);
-            if (!mbar_wait_warp(pair_bar, (n + t) & 1, ctx, SITE_PAIR)) { ok = false; break; }
-            const float l_all = sm.lpart[0][row] + sm.lpart[1][row];
-            const float inv = 1.0f / l_all;
-            // The last product of an item has a barrier of its own: o_full completes once per key step and this
-            // thread has not followed its phases, so a parity wait on it could not tell the last product from the
-            // one before.
-            if (!mbar_wait_warp(&sm.o_done, t & 1, ctx, SITE_O_FULL_LAST)) { ok = false; break; }
+            l = l * alpha + (diag ? exp_pass<true>(t_s, row, half, key0, scale_log2, m)
+                                  : exp_pass<false>(t_s, row, half, key0, scale_log2, m));
+            tmem_wait_st();
+            tc_fence_before_sync();
+            mbar_arrive(&sm.p_full[st]);
+        }
+        // O / l for this thread's 32 columns, log-sum-exp by the first half
+        sm.lpart[half][row] = l;
+        mbar_arrive(pair_bar);
+        ok = ok && mbar_wait_warp(pair_bar, w.nsteps & 1, ctx, SITE_PAIR);
+        const float l_all = sm.lpart[0][row] + sm.lpart[1][row];
+        const float inv = 1.0f / l_all;
+        // The last product of an item has a barrier of its own: o_full completes once per key step and this
+        // thread has not followed its phases, so a parity wait on it could not tell the last product from the
+        // one before.
+        if (ok && mbar_wait_warp(&sm.o_done, 0, ctx, SITE_O_FULL_LAST)) {
             tc_fence_after_sync();
             uint32_t r[32];
             tmem_ld32(t_o, r);

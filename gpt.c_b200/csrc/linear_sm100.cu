@@ -13,19 +13,17 @@
 //     dx       dx[M,K]  = dy[M,N] . W[N,K]          A: dy, K-major (over N) B: W,  MN-major
 //     dW       dW[N,K] += dy[M,N]^T . x[M,K]        A: dy, MN-major         B: x,  MN-major  (split over M)
 // (K-major: the contraction index is the contiguous one.)  Contraction blocks are 32 fp32 values (one 128-byte
-// swizzled row).  A tile is 128 rows of one CTA, or 256 rows of a CTA pair (cta_group::2), by 128, 192 or 256
-// columns, with as many pipeline stages as shared memory holds; plan_tiles picks the shape.
+// swizzled row).  A tile is 128 rows by 128, 192 or 256 columns, with as many pipeline stages as shared memory holds;
+// plan_tiles picks the width.
 //
-// What bounds the kernel: at 256 x 256 a pair needs 32 KB per CTA and contraction block, which takes 512 cycles of
-// the tensor core and arrives at the 55 to 62 bytes per cycle an SM gets from L2 when all of them ask; a CTA on its
-// own needs 48 KB for half the work (64 % tensor pipe active).  The result is written straight from registers, a row
-// per lane in 32-byte sectors: staging it for the copy engine costs shared memory that the pipeline wants (7 stages
-// instead of 6), bandwidth, and hand-overs between warps.  8192 x 3072 x 768: forward 67.0 -> 62.6 us, dW 61 -> 53.7 us;
-// 8192 x 768 x 3072: forward 70 -> 61.6 us, dx 69 -> 61.7 us; QKV with bf16 planes 62.7 -> 57.4 us.
+// What bounds the kernel: a 128 x 256 tile needs 48 KB per contraction block, and the SMs get 15 to 18 TB/s from L2
+// together (64 % tensor pipe active).  The result is written straight from registers, a row per lane in 32-byte
+// sectors: staging it for the copy engine costs shared memory that the pipeline wants, bandwidth, and hand-overs
+// between warps (QKV forward with bf16 planes 72 -> 67 us at 192 columns).
 //
 // Warp roles (384 threads, one CTA per SM, grid = number of SMs, tiles handed out round robin):
 //   warp 0      TMA producer
-//   warp 1      MMA issuer (kind::tf32, one elected lane; of a pair, the leader's)
+//   warp 1      MMA issuer (kind::tf32, one elected lane)
 //   warp 2      tensor-memory allocation (2 accumulators: the epilogue of one tile overlaps the main loop of the next)
 //   warps 4-11  epilogue: 32 rows and half of the columns each, (+ bias, bf16 split) -> global memory, or through a
 //               staging buffer of the warp's own to a bulk tensor reduction (dW) or unaligned rows (vocabulary)
@@ -45,10 +43,10 @@ constexpr int kEpiWarps = 8;
 
 // Tile width kBN (128 or 256 columns) and pipeline depth are chosen per problem: wide tiles halve the
 // shared-memory and L2 traffic per flop, narrow ones fill the SMs better when there are few tiles.
-template <int kBN, int kStages, bool kPair, bool kStage>
+template <int kBN, int kStages, bool kStage>
 struct __align__(1024) SmemT {
     uint8_t a[kStages][kATileBytes];
-    uint8_t b[kStages][kBN * kBK * 4 / (kPair ? 2 : 1)];  // a pair's CTAs hold half of the columns each
+    uint8_t b[kStages][kBN * kBK * 4];
     uint8_t out[kStage ? kEpiWarps : 1][kStage ? 4096 : 16];  // output staging of the epilogue warps: 32 rows x 128 bytes
     uint64_t full[kStages], empty[kStages];
     uint64_t acc_full[2], acc_empty[2];
@@ -59,7 +57,6 @@ struct __align__(1024) SmemT {
 struct Problem {
     int M, N, K;  // C is [M, N]; K is the contraction length
     int bn;       // tile width
-    int pair;     // tiles of 256 rows on CTA pairs (else of 128 rows on single CTAs)
     int a_one, b_one;  // MN-major operand fetched with one 3-D copy per stage (else one copy per 32-row block)
     int tiles_m, tiles_n, splits, kb_total, kb_per_split, total;
     int wide, wide_planes;  // rows of C / of the planes start on 32-byte boundaries
@@ -104,8 +101,7 @@ struct Work {
     int cls;  // row class
     int m0, n0, kb0, kb1;  // first row of this CTA's 128, first column of the tile, contraction blocks
 };
-template <bool kPair>
-__device__ __forceinline__ Work decode(const Problem &p, int w, int rank) {
+__device__ __forceinline__ Work decode(const Problem &p, int w) {
     const int split = w % p.splits;
     const int t = w / p.splits;
     // The operand whose tile index changes slowest is read from HBM once; the other one is streamed again for
@@ -113,7 +109,7 @@ __device__ __forceinline__ Work decode(const Problem &p, int w, int rank) {
     const int tn = p.m_fast ? t / p.tiles_m : t % p.tiles_n;
     const int tm = p.m_fast ? t % p.tiles_m : t / p.tiles_n;
     Work r;
-    r.m0 = kPair ? (2 * tm + rank) * kBM : tm * kBM;
+    r.m0 = tm * kBM;
     r.n0 = tn * p.bn;
     r.cls = split;  // only looked at where the pieces of the contraction are row classes
     r.kb0 = split * p.kb_per_split;
@@ -144,18 +140,14 @@ __device__ __forceinline__ void store_words(void *dst, int left, int wide, const
 // kEpi 0: C = acc (+ bias), optional bf16 planes; kEpi 1: C += acc (bulk reduction)
 // kDirect: the result goes out with plain coalesced 4-byte stores instead of the copy engine, for outputs
 // whose row pitch is not a multiple of 16 bytes (the 50257-wide vocabulary projection).
-// kPair: two CTAs of a cluster share a tile of 256 rows.  Each loads its 128 rows of A and half of the kBN columns
-// of B, 32 KB per contraction block of a 256 x 256 tile where a CTA on its own needs 48 KB for a 128 x 256 one.
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair, bool kClasses>
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kClasses>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__restrict__ bias, float *__restrict__ c_direct,
                    uint32_t *__restrict__ planes, Problem p, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    using Smem = SmemT<kBN, kStages, kPair, kEpi == 1 || kDirect>;
+    using Smem = SmemT<kBN, kStages, kEpi == 1 || kDirect>;
     constexpr uint32_t kTmemCols = 2 * kBN <= 256 ? 256 : 512;  // a power of two that holds two accumulators
-    constexpr int kBRows = kPair ? kBN / 2 : kBN;  // columns of the result whose B rows this CTA loads
-    constexpr int kBTileBytes = kBRows * kBK * 4;
-    constexpr int kCtas = kPair ? 2 : 1;
+    constexpr int kBTileBytes = kBN * kBK * 4;
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     if ((smem_u32(smem_raw) & 1023u) != 0) {
         if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE_SMEM_ALIGN);
@@ -163,34 +155,28 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WaitCtx ctx{&sm.abort_flag, status};
-    const int rank = kPair ? (int)cluster_rank() : 0;
-    const int first = (int)blockIdx.x / kCtas, step = (int)gridDim.x / kCtas;  // work items of this CTA or pair
+    const int first = (int)blockIdx.x, step = (int)gridDim.x;  // work items of this CTA
 
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         for (int i = 0; i < kStages; i++) {
-            mbar_init(&sm.full[i], 1);  // a pair uses the leader's: its arrival, and the bytes of both CTAs
+            mbar_init(&sm.full[i], 1);
             mbar_init(&sm.empty[i], 1);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&sm.acc_full[i], 1);
-            mbar_init(&sm.acc_empty[i], kEpiWarps * kCtas);  // one arrival per epilogue warp
+            mbar_init(&sm.acc_empty[i], kEpiWarps);  // one arrival per epilogue warp
         }
         fence_barrier_init();
     }
     if (warp == 2) {
-        if (kPair) {
-            tmem_alloc_pair(&sm.tmem_base, kTmemCols);  // the permit is given back at the end
-        } else {
-            tmem_alloc(&sm.tmem_base, kTmemCols);
-            tmem_relinquish();
-        }
+        tmem_alloc(&sm.tmem_base, kTmemCols);
+        tmem_relinquish();
     }
     pdl_launch_dependents();
     pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();
-    if (kPair) cluster_sync_all();  // the other CTA's barriers are initialised too
-    else __syncthreads();
+    __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = sm.tmem_base;
 
@@ -204,7 +190,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
             int it = 0;
             bool ok = true;
             for (int w = first; ok && w < p.total; w += step) {
-                Work wk = decode<kPair>(p, w, rank);
+                Work wk = decode(p, w);
                 const CUtensorMap &map_a = maps.a[kClasses ? wk.cls : 0], &map_b = maps.b[kClasses ? wk.cls : 0];
                 if (kClasses) wk.kb0 = 0, wk.kb1 = p.kb_total;
                 for (int kb = wk.kb0; kb < wk.kb1; kb++, it++) {
@@ -213,13 +199,11 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                         ok = false;
                         break;
                     }
-                    if (rank == 0) mbar_expect_tx(&sm.full[st], kCtas * (kATileBytes + kBTileBytes));
-                    const uint32_t full_at = kPair ? mapa(smem_u32(&sm.full[st]), 0) : 0;
+                    mbar_expect_tx(&sm.full[st], kATileBytes + kBTileBytes);
                     auto load = [&](void *dst, const CUtensorMap *map, int c0, int c1, int c2) {
-                        if (kPair) tma_load_4d_pair(dst, map, full_at, c0, c1, c2, 0);
-                        else tma_load_4d(dst, map, &sm.full[st], c0, c1, c2, 0);
+                        tma_load_4d(dst, map, &sm.full[st], c0, c1, c2, 0);
                     };
-                    const int b0 = wk.n0 + rank * kBRows;
+                    const int b0 = wk.n0;
                     // K-major: map {contraction, rows}, one box {32, 128}.  MN-major: map {rows, contraction},
                     // four boxes {32, 32}: blocks of 32 rows, each [32 contraction steps x 128 bytes].
                     if (kAMN) {
@@ -240,23 +224,23 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                             load(sm.b[st], &map_b, 0, kb * kBK - p.b_shift, b0 / 32);
                         } else {
 #pragma unroll
-                            for (int i = 0; i < kBRows / 32; i++)
+                            for (int i = 0; i < kBN / 32; i++)
                                 load(sm.b[st] + i * 4096, &map_b, b0 + 32 * i, kb * kBK - p.b_shift, 0);
                         }
                     } else {
-                        load(sm.b[st], &map_b, kb * kBK, b0, 0);  // the B map's box is kBRows rows
+                        load(sm.b[st], &map_b, kb * kBK, b0, 0);  // the B map's box is kBN rows
                     }
                 }
             }
         }
-    } else if (warp == 1 && rank == 0) {
+    } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        constexpr uint32_t idesc = idesc_tf32(kBM * kCtas, kBN, kAMN ? 1 : 0, kBMN ? 1 : 0);
+        constexpr uint32_t idesc = idesc_tf32(kBM, kBN, kAMN ? 1 : 0, kBMN ? 1 : 0);
         const uint32_t leader = elect_leader();
         int it = 0, j = 0;
         bool ok = true;
         for (int w = first; ok && w < p.total; w += step, j++) {
-            Work wk = decode<kPair>(p, w, rank);
+            Work wk = decode(p, w);
             if (kClasses) wk.kb0 = 0, wk.kb1 = p.kb_total;
             const int acc = j & 1;
             if (j >= 2 && !mbar_wait_warp(&sm.acc_empty[acc], ((j >> 1) - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
@@ -278,15 +262,12 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                 for (int k = 0; k < kBK / 8; k++) {
                     const uint64_t ak = desc_advance(ad, k * (kAMN ? 1024 : 32)), bk = desc_advance(bd, k * (kBMN ? 1024 : 32));
                     const uint32_t add = (kb > wk.kb0 || k > 0) ? 1u : 0u;
-                    if (kPair) mma_tf32_pair_lead(leader, d, ak, bk, idesc, add);
-                    else mma_tf32_lead(leader, d, ak, bk, idesc, add);
+                    mma_tf32_lead(leader, d, ak, bk, idesc, add);
                 }
-                if (kPair) tc_commit_pair_lead(leader, &sm.empty[st]);
-                else tc_commit_lead(leader, &sm.empty[st]);
+                tc_commit_lead(leader, &sm.empty[st]);
             }
             if (!ok) break;
-            if (kPair) tc_commit_pair_lead(leader, &sm.acc_full[acc]);
-            else tc_commit_lead(leader, &sm.acc_full[acc]);
+            tc_commit_lead(leader, &sm.acc_full[acc]);
         }
     } else if (warp >= 4) {
         // ------------------------------ epilogue ------------------------------
@@ -300,7 +281,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
         constexpr int kChunks = kBN / 64;
         int j = 0;
         for (int w = first; w < p.total; w += step, j++) {
-            const Work wk = decode<kPair>(p, w, rank);
+            const Work wk = decode(p, w);
             const int acc = j & 1;
             const int row0 = wk.m0 + 32 * quarter;
             float bv[kChunks];  // bias of the columns col0 + lane, fetched while the tile is still being computed
@@ -320,10 +301,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                 if (c == kChunks - 1) {  // the accumulator has been read out: the tensor cores may reuse it
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) {
-                        if (kPair) mbar_arrive_cluster(mapa(smem_u32(&sm.acc_empty[acc]), 0));
-                        else mbar_arrive(&sm.acc_empty[acc]);
-                    }
+                    if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
                 }
                 if (kEpi == 0 && bias != nullptr) {
                     const float mine = c == 0 ? bv[0] : c == 1 ? bv[1] : c == 2 ? bv[2 % kChunks] : bv[3 % kChunks];
@@ -396,21 +374,11 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     // ------------------------------ tear-down ------------------------------
     if (sm.abort_flag) __nanosleep(50000);
     tc_fence_before_sync();
-    // neither CTA of a pair leaves, or frees tensor memory, while the other may still signal or compute into it
     __syncthreads();
-    if (kPair) cluster_sync_all();
     if (warp == 2) {
         tc_fence_after_sync();
-        if (kPair) {
-            tmem_relinquish_pair();
-            tmem_dealloc_pair(tmem, kTmemCols);
-        } else {
-            tmem_dealloc(tmem, kTmemCols);
-        }
+        tmem_dealloc(tmem, kTmemCols);
     }
-    // Allocation state is the pair's: neither SM may be handed to another kernel, which allocates for itself, before
-    // both CTAs have freed their columns.
-    if (kPair) cluster_sync_all();
 }
 
 // db[n] += sum_m dy[m, n].  A block covers 128 columns (one float4 per lane) and every 8th row of its
@@ -520,17 +488,15 @@ int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, size_t 
     const cuuint32_t box[3] = {32, 32, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
 }
-int tile_rows(int pair) { return pair ? 2 * kBM : kBM; }
-
-Problem make_problem(int M, int N, int K, int bn, int pair, int splits) {
+Problem make_problem(int M, int N, int K, int bn, int splits) {
     Problem p;
-    p.M = M, p.N = N, p.K = K, p.bn = bn, p.pair = pair;
+    p.M = M, p.N = N, p.K = K, p.bn = bn;
     p.a_one = p.b_one = 0;
     p.m_fast = 0;
     p.ldc = (size_t)N;
     p.b_shift = 0;
     for (int i = 0; i < 4; i++) p.a_shift[i] = p.a_whole[i] = 0;
-    p.tiles_m = (M + tile_rows(pair) - 1) / tile_rows(pair);
+    p.tiles_m = (M + kBM - 1) / kBM;
     p.tiles_n = (N + bn - 1) / bn;
     p.kb_total = (K + kBK - 1) / kBK;
     if (splits < 1) splits = 1;
@@ -548,27 +514,26 @@ int sm_count() {
 }
 
 // Tile shape and number of pieces of the contraction for a [M, N] result of kb contraction blocks, chosen by expected
-// time: a fixed part, and for every round over the SMs (or pairs) a charge and kb blocks at the slower of what one
-// CTA takes when it is alone (`block`) and what L2 needs to feed all CTAs of the round.  The constants are a fit to
-// the kernel's times on 224 shapes of 100 to 8192 rows and 512 to 6400 columns (mean error 5 %; the choice is within
-// 1 % of the best of the six on average).  Wide pair tiles read the least per flop and win when there are many
-// tiles, narrow ones and single CTAs leave a smaller last round.
+// time: a fixed part, and for every round over the SMs a charge and kb blocks at the slower of what one CTA takes when
+// it is alone (`block`) and what L2 needs to feed all CTAs of the round.  The constants are a fit to the kernel's times
+// on 224 shapes of 100 to 8192 rows and 512 to 6400 columns (mean error 5 %).  Wide tiles read the least per flop and
+// win when there are many, narrow ones leave a smaller last round.
 struct Plan {
-    int pair, bn, splits;
+    int bn, splits;
     int ns;
 };
 struct Cost {
-    int pair, bn, fixed, round, block;  // nanoseconds
+    int bn, fixed, round, block;  // nanoseconds
 };
-constexpr Cost kCosts[3] = {{0, 256, 4470, 2030, 283}, {0, 192, 4450, 900, 232}, {0, 128, 3920, 400, 226}};
+constexpr Cost kCosts[3] = {{256, 4470, 2030, 283}, {192, 4450, 900, 232}, {128, 3920, 400, 226}};
 constexpr int kL2BytesPerNs = 18190;
 
 // Time of `tiles` tiles of kb contraction blocks each, without the fixed part.
 long long rounds_ns(const Cost &c, long long tiles, int kb, int sms) {
-    const int ctas = c.pair ? 2 : 1, units = sms / ctas;
-    const long long bytes = kATileBytes + (long long)c.bn / ctas * kBK * 4;  // a CTA's operands of one block
+    const int units = sms;
+    const long long bytes = kATileBytes + (long long)c.bn * kBK * 4;  // a CTA's operands of one block
     auto round = [&](long long busy) {
-        const long long fed = bytes * busy * ctas / kL2BytesPerNs;
+        const long long fed = bytes * busy / kL2BytesPerNs;
         return c.round + kb * (fed > c.block ? fed : c.block);
     };
     const long long rest = tiles % units;
@@ -579,47 +544,47 @@ int at_most_int(long long v) { return v < 0x7fffffff ? (int)v : 0x7fffffff; }
 
 // What does not fit in L2 arrives from HBM at 5.0 TB/s, after a start of 6 us.
 Plan plan_tiles(int M, int N, int kb, int sms) {
-    Plan best{0, 128, 1, 0};
+    Plan best{128, 1, 0};
     const long long bytes = 4ll * ((long long)M * N + (long long)kb * kBK * (M + N));
     const long long least = bytes > (100ll << 20) ? 6000 + bytes / 5000 : 0;
     for (const Cost &c : kCosts) {
         if (c.bn > 128 && N < c.bn) continue;
-        const long long tiles = (long long)((M + tile_rows(c.pair) - 1) / tile_rows(c.pair)) * ((N + c.bn - 1) / c.bn);
+        const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + c.bn - 1) / c.bn);
         long long t = c.fixed + rounds_ns(c, tiles, kb, sms);
         if (t < least) t = least;
-        if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, 1, at_most_int(t)};
+        if (best.ns == 0 || t < best.ns) best = Plan{c.bn, 1, at_most_int(t)};
     }
     return best;
 }
 
 // The same with the contraction cut into up to 32 pieces that add into the result with bulk reductions (dW, and dx when
-// its contraction is very long); those cost 43 (pairs) or 80 ns per megabyte and make a block 15 % slower.
+// its contraction is very long); those cost 80 ns per megabyte and make a block 15 % slower.
 Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks) {
-    Plan best{0, 128, 1, 0};
+    Plan best{128, 1, 0};
     for (const Cost &c : kCosts) {
         if (c.bn > 128 && N < c.bn) continue;
-        const long long tiles = (long long)((M + tile_rows(c.pair) - 1) / tile_rows(c.pair)) * ((N + c.bn - 1) / c.bn);
-        const long long tile_bytes = (long long)tile_rows(c.pair) * c.bn * 4;
+        const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + c.bn - 1) / c.bn);
+        const long long tile_bytes = (long long)kBM * c.bn * 4;
         for (int s = 1; s <= 32 && s <= kb; s++) {
             const int per = (kb + s - 1) / s;
             if (s > 1 && per < least_blocks) break;
             const long long t = c.fixed + rounds_ns(c, tiles * s, per, sms) * 115 / 100 +
-                                tiles * s * tile_bytes / 1000 * (c.pair ? 43 : 80) / 1000;
-            if (best.ns == 0 || t < best.ns) best = Plan{c.pair, c.bn, s, at_most_int(t)};
+                                tiles * s * tile_bytes / 1000 * 80 / 1000;
+            if (best.ns == 0 || t < best.ns) best = Plan{c.bn, s, at_most_int(t)};
         }
     }
     return best;
 }
 
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair, bool kClasses = false>
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kClasses = false>
 int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *planes, Problem p, int *status, cudaStream_t s) {
-    using Smem = SmemT<kBN, kStages, kPair, kEpi == 1 || kDirect>;
+    using Smem = SmemT<kBN, kStages, kEpi == 1 || kDirect>;
     static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear kernel");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair, kClasses>;
+    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kClasses>;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return (int)e;
@@ -628,35 +593,34 @@ int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *p
     p.wide = p.ldc % 8 == 0 && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(c) & 31u) == 0;
     p.wide_planes = p.N % 16 == 0 && (reinterpret_cast<uintptr_t>(planes) & 31u) == 0;
     p.plane_words = attn::plane_bytes((size_t)p.M * p.N) / 4;
-    constexpr int kCtas = kPair ? 2 : 1;
-    const int most = sm_count() / kCtas;
-    const int grid = (p.total < most ? p.total : most) * kCtas;
-    return (int)attn::launch_clusters_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), kCtas, s, maps, bias, c,
+    const int most = sm_count();
+    const int grid = p.total < most ? p.total : most;
+    return (int)attn::launch_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), s, maps, bias, c,
                                                      static_cast<uint32_t *>(planes), p, status);
 }
 
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kPair>
+template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect>
 int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
                const Problem &p, int *status, cudaStream_t s) {
     const Maps<false> maps = {{ma}, {mb}, mc, {ma}};
-    return launch_maps<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kPair>(maps, bias, c, planes, p, status, s);
+    return launch_maps<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect>(maps, bias, c, planes, p, status, s);
 }
 
 // Pipeline depth by what fits in 227 KiB next to the output staging tile.
 template <bool kAMN, bool kBMN, int kEpi>
 int launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
            const Problem &p, int *status, cudaStream_t s) {
-#define GO(bn, stages, with_planes, pair) \
-    return launch_one<kAMN, kBMN, kEpi, bn, stages, with_planes, false, pair>(ma, mb, mc, bias, c, planes, p, status, s)
+#define GO(bn, stages, with_planes) \
+    return launch_one<kAMN, kBMN, kEpi, bn, stages, with_planes, false>(ma, mb, mc, bias, c, planes, p, status, s)
     constexpr bool kCanPlanes = !kAMN && !kBMN && kEpi == 0;  // only the forward product writes planes
     if constexpr (kCanPlanes) {
-        if (planes && p.bn == 256) GO(256, 4, true, false);
-        if (planes && p.bn == 192) GO(192, 5, true, false);
-        if (planes) GO(128, 6, true, false);
+        if (planes && p.bn == 256) GO(256, 4, true);
+        if (planes && p.bn == 192) GO(192, 5, true);
+        if (planes) GO(128, 6, true);
     }
-    if (p.bn == 256) GO(256, 4, false, false);
-    if (p.bn == 192) GO(192, kEpi == 1 ? 4 : 5, false, false);
-    GO(128, 6, false, false);
+    if (p.bn == 256) GO(256, 4, false);
+    if (p.bn == 192) GO(192, kEpi == 1 ? 4 : 5, false);
+    GO(128, 6, false);
 #undef GO
 }
 
@@ -683,10 +647,10 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
         if (plan.splits > 1 && (rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
         for (int j = 0; j < 4; j++) {
             const RowClass c = row_class(dy, M, N, j);
-            Problem p = make_problem(c.rows, K, N + c.shift, plan.bn, plan.pair, plan.splits);
+            Problem p = make_problem(c.rows, K, N + c.shift, plan.bn, plan.splits);
             p.ldc = 4 * (size_t)K, p.b_shift = c.shift;
             if ((rc = map_k_major(&ma, c.dy, c.rows, N + c.shift, 128, 4 * (size_t)N)) != 0) return rc;
-            p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 / (p.pair ? 2 : 1)) == 0;
+            p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 ) == 0;
             if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
             float *out = dx + (size_t)j * K;
             if (p.splits > 1) {
@@ -701,7 +665,7 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
     if (!dw) return ATTN_OK;
     // the four classes of a tile follow each other, so that the tile of dW they add into stays in L2
     Maps<true> maps;
-    Problem p = make_problem(N, K, (M + 3) / 4, K % 256 == 0 ? 256 : 128, 0, 1);
+    Problem p = make_problem(N, K, (M + 3) / 4, K % 256 == 0 ? 256 : 128, 1);
     p.splits = 4, p.total *= 4;
     p.a_one = 0, p.b_one = 1;
     for (int j = 0; j < 4; j++) {
@@ -717,11 +681,11 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
         if ((rc = map_mn_major_blocks(&maps.b[j], x + (size_t)j * K, c.rows, K, p.bn / 32, 4 * (size_t)K)) != 0) return rc;
     }
     // up to three rows of the last tile may only be reached through the shifted views
-    p.tiles_m = (N + 3 + tile_rows(0) - 1) / tile_rows(0);
+    p.tiles_m = (N + 3 + kBM - 1) / kBM;
     p.total = p.tiles_m * p.tiles_n * p.splits;
     if ((rc = map_out_f32(&maps.c, dw, N, K)) != 0) return rc;
-    if (p.bn == 256) return launch_maps<true, true, 1, 256, 4, false, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
-    return launch_maps<true, true, 1, 128, 6, false, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
+    if (p.bn == 256) return launch_maps<true, true, 1, 256, 4, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
+    return launch_maps<true, true, 1, 128, 6, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
 }
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
@@ -736,9 +700,9 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
     int split = 1, rc;
     if (plan_split(M, K, np, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, status, s);
     CUtensorMap ma, mb, mc;
-    Problem p = make_problem(M, K, np, plan.bn, plan.pair, plan.splits);
+    Problem p = make_problem(M, K, np, plan.bn, plan.splits);
     if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
-    p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 / (p.pair ? 2 : 1)) == 0;
+    p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 ) == 0;
     if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
     if (p.splits == 1) return launch<false, true, 0>(ma, mb, ma, nullptr, dx, nullptr, p, status, s);
     // the pieces of the contraction add into dx with bulk reductions: start from zeros
@@ -771,12 +735,12 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     if (plan_split(M, N, K, &split) < plan.ns) return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, status, s);
     CUtensorMap ma, mb;
     // with plain stores (N not a multiple of 4) only the widest tiles are built
-    Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, plan.pair, 1);
+    Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, 1);
     p.m_fast = stream_rows_of_c(M, N, K);
     if ((rc = map_k_major(&ma, x, M, K, 128)) != 0) return rc;
-    if ((rc = map_k_major(&mb, w, N, K, p.bn / (p.pair ? 2 : 1))) != 0) return rc;
+    if ((rc = map_k_major(&mb, w, N, K, p.bn )) != 0) return rc;
     if (direct) {
-        return launch_one<false, false, 0, 256, 4, false, true, false>(ma, mb, ma, bias, y, nullptr, p, status, s);
+        return launch_one<false, false, 0, 256, 4, false, true>(ma, mb, ma, bias, y, nullptr, p, status, s);
     }
     return launch<false, false, 0>(ma, mb, ma, bias, y, planes, p, status, s);
 }
@@ -822,10 +786,10 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         // dw[N,K] += dy[M,N]^T . x[M,K]: contraction over M, split so that every SM has work (rows of the
         // result past N are dropped by the copy engine)
         const Plan plan = plan_pieces(N, K, (M + kBK - 1) / kBK, sms, 1);
-        Problem pdw = make_problem(N, K, M, plan.bn, plan.pair, plan.splits);
+        Problem pdw = make_problem(N, K, M, plan.bn, plan.splits);
         pdw.a_one = map_mn_major_blocks(&ma, g, M, np, 4) == 0;
         if (!pdw.a_one && (rc = map_mn_major(&ma, g, M, np)) != 0) return rc;
-        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32 / (plan.pair ? 2 : 1)) == 0;
+        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32 ) == 0;
         if (!pdw.b_one && (rc = map_mn_major(&mb, x, M, K)) != 0) return rc;
         if ((rc = map_out_f32(&mc, dw, N, K)) != 0) return rc;
         rc = launch<true, true, 1>(ma, mb, mc, nullptr, dw, nullptr, pdw, status, s);

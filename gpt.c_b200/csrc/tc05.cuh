@@ -205,9 +205,7 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
 }
 
 // ------------------------------------------------------------------------------------------
-// CTA pairs: a cluster of two CTAs on one TPC that work on one tensor-core tile (cta_group::2).  The CTA of
-// rank 0 leads: it issues the MMAs, which read each CTA's own half of both operands and leave each CTA its
-// own rows of the result.
+// Clusters of CTAs.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -223,40 +221,6 @@ __device__ __forceinline__ uint32_t mapa(uint32_t smem_addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// Loads into this CTA's shared memory; the bytes are counted on a barrier of either CTA of the pair.
-__device__ __forceinline__ void tma_load_4d_pair(void *smem_dst, const CUtensorMap *map, uint32_t bar_cluster_addr, int c0,
-                                                 int c1, int c2, int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
-        "[%2];" ::"r"(smem_u32(smem_dst)),
-        "l"(map), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t *smem_result, uint32_t ncols) {  // one full warp of both CTAs
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// Arrives once on `bar` in both CTAs when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void tc_commit_pair_lead(uint32_t leader, uint64_t *bar) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred e;\n\t"
-        "setp.ne.b32 e, %1, 0;\n\t"
-        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t"
-        "}"
-        ::"r"(smem_u32(bar)), "r"(leader), "h"((uint16_t)3)
-        : "memory");
-}
-
 // ------------------------------------------------------------------------------------------
 // Descriptors
 // ------------------------------------------------------------------------------------------
