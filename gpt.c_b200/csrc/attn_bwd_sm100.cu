@@ -291,7 +291,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const int C = H * kD;
 
     WaitCtx ctx{&sm.abort_flag, status};
-    pdl_launch_dependents();
 
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
@@ -320,8 +319,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         fence_barrier_init();
     }
     if (warp == 2) {
-        tmem_alloc(&sm.tmem_base, kTmemCols);
-        tmem_relinquish();
+        tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
     pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();

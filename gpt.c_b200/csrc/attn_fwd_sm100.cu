@@ -50,6 +50,7 @@ constexpr int kPlaneStep = kStep * kD * 2;  // bytes of one bf16 plane of a K / 
 constexpr int kThreads = 384;
 constexpr int kSoftmaxWarps = 8;
 constexpr uint32_t kTmemCols = 256;
+static_assert(2 * kTmemCols <= 512, "the two CTAs of an SM have their columns at the same time");
 constexpr uint32_t kColS = 0, kColO = 128, kColQ = 192;  // Q: hi plane [192,224), lo plane [224,256)
 
 struct __align__(1024) FwdSmem {
@@ -277,10 +278,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
         }
     }
     if (warp == 1) {
-        tmem_alloc(&sm.tmem_base, kTmemCols);
-        tmem_relinquish();
+        tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
-    pdl_launch_dependents();
     pdl_wait();  // every thread, before its first access to global memory
     if (kFp32) {
         const Item w = decode((int)blockIdx.x, B, T, H);

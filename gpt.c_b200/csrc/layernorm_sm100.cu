@@ -10,7 +10,9 @@
 // One warp owns a row at a time and keeps it in registers (C <= 2048: up to 16 float4 per lane), so
 // every tensor is read once.  In the backward each warp also carries the dW / db partial sums of its
 // columns in registers over all the rows it visits; a block adds them up in shared memory and issues
-// one atomicAdd per column, which cuts the atomics from rows x C to blocks x C.
+// one atomicAdd per column, which cuts the atomics from rows x C to blocks x C.  The backwards' blocks work in clusters
+// whose barriers have no limit: every block reaches both of them, since none waits for anything else once the previous
+// kernel has completed.
 #include <cooperative_groups.h>
 
 #include "attn_internal.h"

@@ -27,7 +27,8 @@
 //   warp 2      tensor-memory allocation (2 accumulators: the epilogue of one tile overlaps the main loop of the next)
 //   warps 4-11  epilogue: 32 rows and half of the columns each, (+ bias, bf16 split) -> global memory, or through a
 //               staging buffer of the warp's own to a bulk tensor reduction (dW) or unaligned rows (vocabulary)
-// All waits are bounded (see tc05.cuh).
+// The waits on barriers are bounded (tc05.cuh).  Two others end for the reasons given there and need no limit: the
+// allocation of tensor memory, and the wait for the previous kernel of the stream.
 #include "linear_tf32.cuh"
 
 #include "../../include/linear_sm100.h"
@@ -170,10 +171,8 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
         fence_barrier_init();
     }
     if (warp == 2) {
-        tmem_alloc(&sm.tmem_base, kTmemCols);
-        tmem_relinquish();
+        tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
-    pdl_launch_dependents();
     pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();
     __syncthreads();

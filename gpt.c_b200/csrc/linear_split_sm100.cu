@@ -24,12 +24,17 @@ using namespace tc05;
 
 constexpr int kMaxStages = 12;
 constexpr int kMaxSplit = 8;  // CTAs on one tile: the portable cluster size
+constexpr int kMostTmemCols = 128;  // an accumulator of at most 128 columns
 // Epilogue warps (the first ones), one or two per tensor-memory lane quarter, then a TMA producer warp and a warp that
 // issues the MMAs.  Several CTAs share an SM when tiles are not split: four warps each are enough there.
 template <bool kSplit>
 struct Roles {
     static constexpr int kEpiWarps = kSplit ? 8 : 4, kWarpTma = kEpiWarps, kWarpMma = kEpiWarps + 1;
     static constexpr int kThreads = 32 * (kEpiWarps + 2);
+    static constexpr int kPerSm = kSplit ? 2 : 3;  // CTAs an SM's registers hold
+    // The CTAs of a cluster wait for each other while they hold tensor memory: were an SM's columns fewer than its CTAs
+    // want, two clusters could each hold what the other waits for.
+    static_assert(kPerSm * kMostTmemCols <= 512, "tensor memory for every CTA of an SM");
 };
 
 struct Params {
@@ -57,7 +62,7 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
 
 // kSplit: a cluster of CTAs per tile (else one CTA, several to an SM)
 template <bool kWMN, bool kSplit>
-__global__ void __launch_bounds__(Roles<kSplit>::kThreads, kSplit ? 2 : 3) linear_split_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(Roles<kSplit>::kThreads, Roles<kSplit>::kPerSm) linear_split_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                 const __grid_constant__ CUtensorMap map_act,
                                                                 const float *__restrict__ bias, float *__restrict__ out,
                                                                 __nv_bfloat16 *__restrict__ planes, Params p, int *status) {
@@ -82,8 +87,7 @@ __global__ void __launch_bounds__(Roles<kSplit>::kThreads, kSplit ? 2 : 3) linea
         fence_barrier_init();
     }
     if (warp == kWarpMma) {
-        tmem_alloc(&ct.tmem_base, p.tmem_cols);
-        tmem_relinquish();
+        tmem_alloc_then_launch_dependents(&ct.tmem_base, p.tmem_cols);
     }
     if (warp == kWarpTma && lane == 0) {
         tma_prefetch_desc(&map_w);
@@ -96,7 +100,6 @@ __global__ void __launch_bounds__(Roles<kSplit>::kThreads, kSplit ? 2 : 3) linea
                              : "memory");
         }
     }
-    pdl_launch_dependents();
     pdl_wait();
     tc_fence_before_sync();
     __syncthreads();
@@ -289,7 +292,7 @@ int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, 
     p.kb_total = (kc + kBK - 1) / kBK;
     p.kb_per_split = (p.kb_total + split - 1) / split;
     p.split = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;  // every CTA has a share
-    p.tmem_cols = p.bm <= 32 ? 32 : (p.bm <= 64 ? 64 : 128);
+    p.tmem_cols = p.bm <= 32 ? 32 : (p.bm <= 64 ? 64 : kMostTmemCols);
     p.plane_elems = attn::plane_bytes((size_t)M * cols) / sizeof(__nv_bfloat16);
     const int grid = (cols + kBM - 1) / kBM * p.tiles_m * p.split;
     const int stage = kATileBytes + p.bm * 128;

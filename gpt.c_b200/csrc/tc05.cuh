@@ -36,8 +36,9 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // Programmatic dependent launch: a kernel launched with launch_after_previous() (attn_internal.h) may
 // start while the kernel before it in the stream is still running.  It must not touch global memory
 // before pdl_wait() (returns once the previous kernel has completed and its writes are visible);
-// pdl_launch_dependents() lets the kernel after this one start its own set-up.  Both are no-ops for a
-// kernel launched the ordinary way.
+// pdl_launch_dependents() lets the kernel after this one start its own set-up, as soon as any one thread of
+// every CTA has executed it.  Both are no-ops for a kernel launched the ordinary way.  Kernels that allocate
+// tensor memory do not call it themselves: tmem_alloc_then_launch_dependents() does.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -96,7 +97,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Shared abort word of a CTA plus the device-global status word.  A wait that runs out sets
+// Every wait on an mbarrier is bounded.  Shared abort word of a CTA plus the device-global status word.  A wait that runs out sets
 // both; every later wait in the CTA returns false at once, so all roles fall through to the
 // common tear-down (tensor memory is freed there) instead of spinning for ever.
 struct WaitCtx {
@@ -177,13 +178,18 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // ------------------------------------------------------------------------------------------
 // Tensor memory (TMEM) allocation.  Addresses are (lane << 16) | column.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_alloc(uint32_t *smem_result, uint32_t ncols) {  // one full warp
+// One full warp.  An allocation waits, without a limit, until the columns are free.  That wait ends because the next
+// kernel of the stream is let start only behind the allocation, and by the thread that made it: a CTA of the next
+// kernel may share the SM and take columns before it waits for this kernel to complete, so with the two the other way
+// round (or the signal given by another warp, which counts for the whole CTA) this CTA could wait for columns of one
+// that waits for it.  As it is, whoever holds columns waits at most for kernels of which every CTA has its own.
+// Each CTA allocates once, so none holds columns while it waits for more.
+__device__ __forceinline__ void tmem_alloc_then_launch_dependents(uint32_t *smem_result, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
                  "r"(ncols)
                  : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  // same warp as alloc
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
@@ -212,6 +218,7 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+// Has no limit; ends because every CTA of the cluster gets here, also after one of its bounded waits has run out.
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
