@@ -86,8 +86,10 @@ struct Maps {
 // copy engine as they are, but every fourth row can: the rows m = 4 i + j form a matrix with a pitch of 4 N floats, whose
 // base is moved down to a 16-byte boundary, by a_shift = (j N) mod 4 floats.  The view's column c is then column
 // c - a_shift of dy.  In dx that is the contraction index, and W is fetched at rows c - a_shift (rows before the first
-// and past the last read as zeros); one product per class, which leaves every fourth row of dx.  In dW it is the row of
-// the result: each class is a piece of the contraction, added into dW a_shift rows higher up.  What this replaces is a
+// and past the last read as zeros); one product per class, which leaves every fourth row of dx.  What the first a_shift
+// columns hold is the end of the row of dy before: the MMA warp puts zeros there in shared memory (clear_leading), since
+// the zeros of W alone would turn a value that is not finite into NaN.  In dW the view's column is the row of the
+// result: each class is a piece of the contraction, added into dW a_shift rows higher up.  What this replaces is a
 // copy of dy with padded rows, 536 us for the 1.65 GB of 8192 x 50257.
 struct RowClass {
     const float *dy;  // base of the view
@@ -116,6 +118,20 @@ __device__ __forceinline__ Work decode(const Problem &p, int w) {
     r.kb0 = split * p.kb_per_split;
     r.kb1 = min(p.kb_total, r.kb0 + p.kb_per_split);
     return r;
+}
+
+// Zeros for the first `columns` (at most 3) of a K-major A tile's 128 rows: they are in the first 16 bytes of a row, which
+// the 128-byte swizzle puts at 16 * (row mod 8).  By a whole warp, one lane of which issues the tensor-core instructions
+// that read the tile.
+__device__ __forceinline__ void clear_leading(uint8_t *tile, int columns, int lane) {
+    for (int r = lane; r < kBM; r += 32) {
+        float *row = reinterpret_cast<float *>(tile + r * 128 + ((r & 7) << 4));
+        row[0] = 0.f;
+        if (columns > 1) row[1] = 0.f;
+        if (columns > 2) row[2] = 0.f;
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
 }
 
 // Writes 4 * kQuads consecutive 32-bit words to dst, as far as `left` words go (a multiple of
@@ -252,6 +268,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                     break;
                 }
                 tc_fence_after_sync();
+                if (!kAMN && kBMN && kb == 0 && p.b_shift > 0) clear_leading(sm.a[st], p.b_shift, lane);
                 // MN-major tiles: 32-row blocks 4096 bytes apart, groups of 4 contraction steps 512 bytes apart
                 const uint64_t ad = kAMN ? smem_desc_sw128_base32(smem_u32(sm.a[st]), 4096, 512)
                                          : smem_desc_sw128(smem_u32(sm.a[st]), 16, 1024);

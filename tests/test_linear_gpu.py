@@ -148,6 +148,26 @@ def test_linear_backward_from_every_fourth_row(pkg, M, N, K):
     assert bool((pad[:8] == 7.0).all()) and bool((pad[8 + N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("N", [257, 258, 1003, 16387])  # the last one: contraction in pieces
+def test_linear_input_gradient_keeps_rows_apart(pkg, N):
+    """Values of dy that are not finite stay in their own row of dx and their own column's row of dW, where dy's rows start
+    on 4- or 8-byte boundaries and every fourth one is read through a view that starts up to three values early."""
+    M, K = 1030, 96
+    x, w, _, dy = inputs(M, N, K, 61)
+    bad = {3: (N - 1, np.inf), 4: (N - 2, np.nan), 517: (N - 3, -np.inf), 1025: (N - 1, np.nan), M - 1: (N - 1, np.inf)}
+    for row, (col, value) in bad.items():
+        dy[row, col] = value
+    rest = np.setdiff1d(np.arange(M), list(bad))
+    dw = torch.zeros(N, K, device="cuda")
+    dx = pkg.linear_backward(*(torch.from_numpy(a).cuda() for a in (dy, x, w)), dw).cpu().numpy()
+    assert pkg.device_status() == 0
+    assert not np.isfinite(dx[list(bad)]).any()
+    within(dx[rest], dy[rest].astype(np.float64) @ w.astype(np.float64), dy[rest], w)
+    dw = dw.cpu().numpy()
+    assert not np.isfinite(dw[-3:]).any()
+    within(dw[:-3], dy[:, :-3].T.astype(np.float64) @ x.astype(np.float64), dy[:, :-3].T, x)
+
+
 def test_linear_backward_parts_can_be_skipped(pkg):
     M, N, K = 512, 768, 768
     x, w, b, dy = inputs(M, N, K, 31)
