@@ -397,15 +397,24 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     }
 }
 
-// db[n] += sum_m dy[m, n].  A block covers 128 columns (one float4 per lane) and every 8th row of its
-// share of the rows; four loads are in flight per thread.  N is a multiple of 4.
+// db[n] += sum_m dy[m, n].  A block covers 128 columns, four per lane, and every 8th row of its share of the rows; the
+// loads of four rows are in flight per thread.  kWords: a lane's columns are one float4 (the pitch is a multiple of 4),
+// else they are 32 apart and read one by one.
+template <bool kWords>
 __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict__ dy, float *__restrict__ db, int M, int N,
                                                         int pitch) {
     tc05::pdl_launch_dependents();
     tc05::pdl_wait();
     __shared__ float4 part[8][32];
     const int lane = threadIdx.x & 31, rl = threadIdx.x >> 5;
-    const int col = blockIdx.x * 128 + 4 * lane;
+    constexpr int kApart = kWords ? 1 : 32;
+    const int col = blockIdx.x * 128 + (kWords ? 4 * lane : lane);
+    auto load = [&](int m) -> float4 {
+        const float *at = dy + (size_t)m * pitch + col;
+        if (kWords) return __ldcs(reinterpret_cast<const float4 *>(at));
+        return make_float4(__ldcs(at), col + 32 < N ? __ldcs(at + 32) : 0.f, col + 64 < N ? __ldcs(at + 64) : 0.f,
+                           col + 96 < N ? __ldcs(at + 96) : 0.f);
+    };
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (col < N) {
         const int step = gridDim.y * 8;
@@ -413,12 +422,12 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict_
         for (; m + 3 * step < M; m += 4 * step) {
             float4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = __ldcs(reinterpret_cast<const float4 *>(dy + (size_t)(m + u * step) * pitch + col));
+            for (int u = 0; u < 4; u++) v[u] = load(m + u * step);
 #pragma unroll
             for (int u = 0; u < 4; u++) acc.x += v[u].x, acc.y += v[u].y, acc.z += v[u].z, acc.w += v[u].w;
         }
         for (; m < M; m += step) {
-            const float4 v = __ldcs(reinterpret_cast<const float4 *>(dy + (size_t)m * pitch + col));
+            const float4 v = load(m);
             acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
         }
     }
@@ -428,15 +437,15 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict_
         float4 t = part[0][lane];
 #pragma unroll
         for (int i = 1; i < 8; i++) t.x += part[i][lane].x, t.y += part[i][lane].y, t.z += part[i][lane].z, t.w += part[i][lane].w;
-        if (col + 3 < N && (reinterpret_cast<uintptr_t>(db + col) & 15u) == 0) {
+        if (kWords && col + 3 < N && (reinterpret_cast<uintptr_t>(db + col) & 15u) == 0) {
             asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(db + col), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w)
                          : "memory");
             return;
         }
         atomicAdd(db + col, t.x);
-        if (col + 1 < N) atomicAdd(db + col + 1, t.y);
-        if (col + 2 < N) atomicAdd(db + col + 2, t.z);
-        if (col + 3 < N) atomicAdd(db + col + 3, t.w);
+        if (col + kApart < N) atomicAdd(db + col + kApart, t.y);
+        if (col + 2 * kApart < N) atomicAdd(db + col + 2 * kApart, t.z);
+        if (col + 3 * kApart < N) atomicAdd(db + col + 3 * kApart, t.w);
     }
 }
 
@@ -650,6 +659,16 @@ int stream_rows_of_c(int M, int N, int K) {
 
 bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
+// Whether the gradients of a [M, N] result come from views of every fourth row of dy, whose rows are not 16-byte aligned,
+// and not from a copy with padded rows.  The copy is cheap as long as it stays in L2 (128 MB), and dx as four products
+// of a quarter of the rows wants at least eight row tiles in each.  dx and dW, copy -> views, in us (N, K; M):
+//     50257, 768; 1024: 398 -> 470, 2048: 675 -> 826, 4096: 1455 -> 1215, 8192: 3000 -> 2520
+//     50257, 384; 1024: 272 -> 293, 2048: 475 -> 503, 4096: 942 -> 902, 8192: 1930 -> 1662
+//     16387, 512; 1024: 102 -> 105, 2048: 186 -> 182, 4096: 349 -> 316, 8192: 720 -> 541
+//      4099, 768; 1024: 39 -> 74, 4096: 119 -> 134, 8192: 256 -> 218          1001, 768; 2048: 26 -> 63, 8192: 66 -> 87
+// The size of the scratch buffer follows from the shape alone, so this must too.
+bool by_row_class(int M, int N) { return N % 4 != 0 && M >= 4096 && (long long)M * N >= (32 << 20); }
+
 // dx and dW (either may be NULL) straight from a dy whose rows are not 16-byte aligned.
 int gradients_by_row_class(const float *dy, const float *x, const float *w, float *dx, float *dw, int M, int N, int K, int sms,
                            int *status, cudaStream_t s) {
@@ -763,7 +782,7 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
 
 size_t linear_sm100_backward_scratch_bytes(int M, int N, int K) {
     (void)K;
-    if (M <= 0 || N <= 0 || N % 32 == 0) return 0;
+    if (M <= 0 || N <= 0 || N % 32 == 0 || lin::by_row_class(M, N)) return 0;
     const size_t np = ((size_t)N + 31) / 32 * 32;
     return (size_t)M * np * sizeof(float);
 }
@@ -774,31 +793,32 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     if (!dy || !w || (!dx && !dw) || (dw && !x)) return ATTN_ERR_NULL;
     if (M <= 0 || N <= 0 || K <= 0 || (long long)M * N > 0x7fffffffLL || (long long)M * K > 0x7fffffffLL) return ATTN_ERR_SHAPE;
     if (K % 32 != 0) return ATTN_ERR_UNSUPPORTED;
-    const bool padded = N % 32 != 0;  // dy's rows cannot be tiles of the copy engine as they are: work on a padded copy
+    const bool classes = by_row_class(M, N);
+    const bool padded = N % 32 != 0 && !classes;  // dy's rows cannot be tiles of the copy engine: work on a padded copy
     const int np = (N + 31) / 32 * 32;
     if ((long long)M * np > 0x7fffffffLL) return ATTN_ERR_SHAPE;
     if (padded && !scratch) return ATTN_ERR_NULL;
     // dy itself must start on a 16-byte boundary in both cases: the padding kernel reads it in 16-byte words
     if (!aligned16(dy) || !aligned16(x) || !aligned16(w) || !aligned16(dx) || !aligned16(dw) ||
-        (!padded && !aligned16(db)) || !aligned16(scratch))
+        (N % 32 == 0 && !aligned16(db)) || !aligned16(scratch))
         return ATTN_ERR_ALIGN;
     int *status = nullptr;
     int rc = attn::device_status_word(&status);
     if (rc != ATTN_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int sms = sm_count();
-    // From 1024 rows on the copy with padded rows costs more than four products on every fourth row do.
-    if (N % 4 != 0 && M >= 1024 && !db) return gradients_by_row_class(dy, x, w, dx, dw, M, N, K, sms, status, s);
-    const float *g = dy;  // [M, np] from here on
-    if (padded) {
+    const float *g = dy;  // without row classes [M, np] from here on
+    if (classes) {
+        if ((rc = gradients_by_row_class(dy, x, w, dx, dw, M, N, K, sms, status, s)) != 0) return rc;
+    } else if (padded) {
         rc = (int)attn::launch_after_previous(pad_rows_kernel, dim3(sms * 16), dim3(256), 0, s, static_cast<float *>(scratch), dy, M,
                                               N, np);
         if (rc != 0) return rc;
         g = static_cast<const float *>(scratch);
     }
-    if (dx && (rc = input_gradient(g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
+    if (!classes && dx && (rc = input_gradient(g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
     CUtensorMap ma, mb, mc;
-    if (dw) {
+    if (!classes && dw) {
         // dw[N,K] += dy[M,N]^T . x[M,K]: contraction over M, split so that every SM has work (rows of the
         // result past N are dropped by the copy engine)
         const Plan plan = plan_pieces(N, K, (M + kBK - 1) / kBK, sms, 1);
@@ -816,7 +836,8 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         // 8192 x 768), but at least four rows for each of a block's eight row lanes
         const int across = (N + 127) / 128, fill = 8 * sms / across, by = (M + 31) / 32 < fill ? (M + 31) / 32 : (fill > 1 ? fill : 1);
         dim3 grid((unsigned)((N + 127) / 128), (unsigned)by);
-        rc = (int)attn::launch_after_previous(bias_grad_kernel, grid, dim3(256), 0, s, g, db, M, N, np);
+        rc = (int)attn::launch_after_previous(classes ? bias_grad_kernel<false> : bias_grad_kernel<true>, grid, dim3(256), 0, s, g,
+                                              db, M, N, classes ? N : np);
     }
     return rc;
 }

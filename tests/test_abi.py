@@ -51,6 +51,15 @@ def test_size_queries(pkg):
         assert pkg.backward_scratch_bytes(*bad) == 0
 
 
+def test_linear_scratch_is_only_asked_for_where_it_is_used(pkg):
+    size = pkg.lib().linear_sm100_backward_scratch_bytes
+    assert size(8192, 50257, 768) == 0 and size(4096, 8193, 64) == 0  # read as they are, every fourth row at a time
+    assert size(8192, 768, 768) == 0
+    # a padded copy: too few rows, a dy that stays in L2, rows on 16-byte boundaries
+    for M, N, pitch in ((4095, 50257, 50272), (1024, 50257, 50272), (4096, 8191, 8192), (8192, 100, 128), (8192, 50260, 50272)):
+        assert size(M, N, 768) == M * pitch * 4
+
+
 def test_argument_errors_are_reported_before_any_cuda_call(pkg):
     L = pkg.lib()
     one = ctypes.c_void_p(16)

@@ -130,29 +130,39 @@ def test_linear_tile_shapes(pkg, M, N, K):
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
 
 
-@pytest.mark.parametrize("M,N,K", [(1024, 257, 256), (1025, 1001, 96), (1026, 513, 384), (1027, 94, 512), (1300, 9999, 64), (1111, 16387, 32)])
+@pytest.mark.parametrize("M,N,K", [(1024, 257, 256), (1025, 1001, 96), (1026, 513, 384), (1027, 94, 512), (1300, 9999, 64), (1111, 16387, 32),
+                                   (4096, 8193, 256), (4097, 8195, 96), (4099, 8318, 384), (9999, 3357, 128), (4111, 16387, 32)])
 def test_linear_backward_from_every_fourth_row(pkg, M, N, K):
-    """Rows of dy that start on 4- or 8-byte boundaries, enough of them that no padded copy is made; dW has rows that only
-    the shifted views reach, dx a contraction that is cut into pieces (the last one)."""
+    """Rows of dy that start on 4- or 8-byte boundaries: from a padded copy, and from 4096 rows and 2^25 values on without
+    one; there dW has rows that only the shifted views reach, dx a contraction that is cut into pieces (the last one)."""
     x, w, _, dy = inputs(M, N, K, 53)
     xt, wt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, dy))
     dw0 = np.random.default_rng(3).standard_normal((N, K), dtype=np.float32)
     pad = torch.full((N + 16, K), 7.0, device="cuda")  # rows either side of dW stay as they are
     dw = pad[8:8 + N]
     dw.copy_(torch.from_numpy(dw0))
-    dx = pkg.linear_backward(dyt, xt, wt, dw)
+    db = torch.full((N + 8,), 0.5, device="cuda")
+    dx = torch.empty_like(xt)
+    need = pkg.lib().linear_sm100_backward_scratch_bytes(M, N, K)
+    assert (need == 0) == (M >= 4096)
+    scratch = torch.empty(need, dtype=torch.uint8, device="cuda")
+    assert pkg.lib().linear_sm100_backward(dyt.data_ptr(), xt.data_ptr(), wt.data_ptr(), dx.data_ptr(), dw.data_ptr(),
+                                           db[3:].data_ptr(), scratch.data_ptr() if need else None, M, N, K,
+                                           torch.cuda.current_stream().cuda_stream) == 0
     assert pkg.device_status() == 0
-    dx_ref, dw_ref, _ = ops.linear_backward(dy, x, w, dw0, np.zeros(N, np.float32))
+    dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, dw0, np.full(N, 0.5, np.float32))
+    assert np.abs(db.cpu().numpy()[3:3 + N] - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+    assert bool((db[:3] == 0.5).all()) and bool((db[3 + N:] == 0.5).all())
     within(dx.cpu().numpy(), dx_ref, dy, w)
     within(dw.cpu().numpy(), dw_ref, dy.T, x)
     assert bool((pad[:8] == 7.0).all()) and bool((pad[8 + N:] == 7.0).all())
 
 
-@pytest.mark.parametrize("N", [257, 258, 1003, 16387])  # the last one: contraction in pieces
+@pytest.mark.parametrize("N", [8193, 8194, 8195, 16387])  # the last one: contraction in pieces
 def test_linear_input_gradient_keeps_rows_apart(pkg, N):
     """Values of dy that are not finite stay in their own row of dx and their own column's row of dW, where dy's rows start
     on 4- or 8-byte boundaries and every fourth one is read through a view that starts up to three values early."""
-    M, K = 1030, 96
+    M, K = 4102, 96
     x, w, _, dy = inputs(M, N, K, 61)
     bad = {3: (N - 1, np.inf), 4: (N - 2, np.nan), 517: (N - 3, -np.inf), 1025: (N - 1, np.nan), M - 1: (N - 1, np.inf)}
     for row, (col, value) in bad.items():
