@@ -4,7 +4,10 @@ reference in oracle/ops_oracle.py, pinned to the reference's own CPU kernel by t
 accumulates the loss into its output, which is what the CUDA kernels here do too):
 log-softmax, mean negative log-likelihood accumulated into the loss, and the backward that works on what
 dout already holds.  Tolerance: fp32 with fast exponentials, 2e-6 absolute on log-softmax values of order
-10, 1e-6 relative on the loss, 1e-7 + 1e-5 relative on the gradient.
+10, 1e-7 + 1e-5 relative on the gradient.  On the loss 1e-6 relative for its terms, and what adding them up one by one
+rounds: the kernel's blocks add into one float in no fixed order, each addition is off by at most half a unit in the last
+place of the sum, and such errors, spread evenly, have a standard deviation of sqrt(rows / 12) units; six of them are
+allowed (7e-5 at 2048 rows and a loss of 10.5, where one in some dozen runs was more than 1.2e-5 off).
 """
 import numpy as np
 import pytest
@@ -34,7 +37,8 @@ def test_cross_entropy_forward_backward_vs_cpu(pkg, rows, C):
     loss = torch.full((1,), 0.25, device="cuda")  # accumulates on top of what is there
     assert L.xent_sm100_forward(lt.data_ptr(), tt.data_ptr(), logsm.data_ptr(), loss.data_ptr(), rows, C, stream()) == 0
     assert np.abs(logsm.cpu().numpy() - logsm_ref).max() <= 2e-6 * max(1.0, np.abs(logsm_ref).max())
-    assert abs(loss.item() - 0.25 - loss_ref) <= 1e-6 * max(1.0, abs(loss_ref)) + 2e-6
+    unit = float(np.spacing(np.float32(loss_ref + 0.25)))
+    assert abs(loss.item() - 0.25 - loss_ref) <= 1e-6 * max(1.0, abs(loss_ref)) + 2e-6 + 6 * np.sqrt(rows / 12) * unit
 
     # backward from a zero-filled dout (what the layer does) ...
     dout = torch.zeros_like(lt)
