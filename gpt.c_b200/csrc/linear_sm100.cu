@@ -673,6 +673,14 @@ bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) ==
 // The size of the scratch buffer follows from the shape alone, so this must too.
 bool by_row_class(int M, int N) { return N % 4 != 0 && M >= 4096 && (long long)M * N >= (32 << 20); }
 
+// Tile width of dW [N, K] from views of every fourth row: 256 unless tiles of 192 columns end more than a tenth earlier;
+// 128 is only for results that narrow.  8192 x 50257, K = 384: 764 / 724 / 822 us at 128 / 192 / 256 columns,
+// 512: 1128 / 1000 / 845, 576: 1352 / 1025 / 1181, 640: 1431 / 1297 / 1165, 768: 1615 / 1372 / 1218, 1600: 3222 / 3164 / 3007.
+int class_tile_width(int K) {
+    if (K <= 128) return 128;
+    return (K + 191) / 192 * 192 * 11 / 10 < (K + 255) / 256 * 256 ? 192 : 256;
+}
+
 // dx and dW (either may be NULL) straight from a dy whose rows are not 16-byte aligned.
 int gradients_by_row_class(const float *dy, const float *x, const float *w, float *dx, float *dw, int M, int N, int K, int sms,
                            int *status, cudaStream_t s) {
@@ -704,7 +712,7 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
     if (!dw) return ATTN_OK;
     // the four classes of a tile follow each other, so that the tile of dW they add into stays in L2
     Maps<true> maps;
-    Problem p = make_problem(N, K, (M + 3) / 4, K % 256 == 0 ? 256 : 128, 1);
+    Problem p = make_problem(N, K, (M + 3) / 4, class_tile_width(K), 1);
     p.splits = 4, p.total *= 4;
     p.a_one = 0, p.b_one = 1;
     for (int j = 0; j < 4; j++) {
@@ -723,6 +731,7 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
     p.tiles_m = (N + 3 + kBM - 1) / kBM;
     p.total = p.tiles_m * p.tiles_n * p.splits;
     if ((rc = map_out_f32(&maps.c, dw, N, K)) != 0) return rc;
+    if (p.bn == 192) return launch_maps<true, true, 1, 192, 4, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
     if (p.bn == 256) return launch_maps<true, true, 1, 256, 4, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
     return launch_maps<true, true, 1, 128, 6, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
 }

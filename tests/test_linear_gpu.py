@@ -131,10 +131,12 @@ def test_linear_tile_shapes(pkg, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(1024, 257, 256), (1025, 1001, 96), (1026, 513, 384), (1027, 94, 512), (1300, 9999, 64), (1111, 16387, 32),
-                                   (4096, 8193, 256), (4097, 8195, 96), (4099, 8318, 384), (9999, 3357, 128), (4111, 16387, 32)])
+                                   (4096, 8193, 256), (4097, 8195, 96), (4099, 8318, 384), (4101, 8190, 320), (4098, 8197, 640),
+                                   (9999, 3357, 128), (4111, 16387, 32)])
 def test_linear_backward_from_every_fourth_row(pkg, M, N, K):
     """Rows of dy that start on 4- or 8-byte boundaries: from a padded copy, and from 4096 rows and 2^25 values on without
-    one; there dW has rows that only the shifted views reach, dx a contraction that is cut into pieces (the last one)."""
+    one; there dW has rows that only the shifted views reach and tiles of each width, whole and not, dx a contraction that
+    is cut into pieces (the last one)."""
     x, w, _, dy = inputs(M, N, K, 53)
     xt, wt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, dy))
     dw0 = np.random.default_rng(3).standard_normal((N, K), dtype=np.float32)
