@@ -828,7 +828,7 @@ cudaError_t generic_set_attributes() {
 
 cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t n, cudaStream_t s) {
     const size_t pieces = (n / 8 + 255) / 256;
-    if (pieces <= 148 * 16)  // one trip of the loop
+    if (pieces <= (size_t)sm_count() * 16)  // one trip of the loop
         return launch_after_previous(split_small_kernel, dim3((unsigned)(pieces ? pieces : 1)), dim3(256), 0, s, x, hi, lo, n);
     return launch_after_previous(split_kernel, dim3((unsigned)((pieces + 1) / 2)), dim3(256), 0, s, x, hi, lo, n);
 }
@@ -842,8 +842,8 @@ cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta
                                      dlo, dq_zero, sched, B, T, H);
     }
     const size_t rows = (size_t)B * T * H;
-    size_t blocks = (rows + 7) / 8;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    const size_t most = (size_t)sm_count() * 16;
+    const size_t blocks = (rows + 7) / 8 < most ? (rows + 7) / 8 : most;
     return launch_after_previous(bwd_prepare_kernel, dim3((unsigned)blocks), dim3(256), 0, s, dout, out, delta, dq_zero, B, T,
                                  H, D);
 }

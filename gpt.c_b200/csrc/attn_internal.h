@@ -7,7 +7,21 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace attn {
+
+// SMs of the current device (1 when that cannot be found out: the launch that follows reports why).
+inline int sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    const bool slot = dev >= 0 && dev < 64;
+    if (slot && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+    if (slot) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
+}
 
 constexpr int kShortT = 128;  // one query and key tile: the kernels that read the fp32 tensors themselves
 constexpr int kGenericMaxD = 256;

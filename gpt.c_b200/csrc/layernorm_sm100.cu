@@ -204,7 +204,6 @@ __global__ void __launch_bounds__(kThreads, (kNV <= 6 ? 4 : 1)) ln_backward_kern
 // registers.  1500 x 1600: backward 20.8 -> 15.1 us; 300 x 1024: 6.5 -> 5.3 us, forward 3.6 -> 2.2 us; 1024 x 2048:
 // forward 6.5 -> 4.7 us.  At 8192 x 768 the barriers cost more than the occupancy brings (backward 23.6 -> 28.8 us).
 // ---------------------------------------------------------------------------------------
-constexpr int kFewRows = 16 * 148;  // up to here: fewer than 16 rows per SM
 constexpr int kMostThreads = 512;   // C <= 2048
 constexpr int kFewCluster = 8;
 
@@ -374,12 +373,14 @@ __global__ void __launch_bounds__(kMostThreads, 1) ln_backward_few_rows_kernel(c
     cluster.sync();  // a block's shared memory stays alive until the others have read it
 }
 
+// Fewer than 16 rows per SM.
+bool few_rows(int rows) { return rows <= 16 * attn::sm_count(); }
+
 int threads_for(int C) { return (C / 4 + 31) / 32 * 32; }
 
 // Blocks that fill the SMs at `regs` registers per thread, but no more than there are groups of rows.
 int few_rows_grid(int rows, int threads, int regs, int rows_at_a_time) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = attn::sm_count();
     int per_sm = 65536 / (regs * threads);
     if (per_sm > 2048 / threads) per_sm = 2048 / threads;
     if (per_sm > 32) per_sm = 32;
@@ -388,9 +389,7 @@ int few_rows_grid(int rows, int threads, int regs, int rows_at_a_time) {
 }
 
 int grid_for(int rows, int blocks_per_sm) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int grid = sms * blocks_per_sm;
+    int grid = attn::sm_count() * blocks_per_sm;
     const int need = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
     return grid < need ? grid : (need > 0 ? need : 1);
 }
@@ -445,7 +444,7 @@ int layernorm_sm100_forward(const float *x, const float *w, const float *b, floa
     if (C % 4 != 0 || C > 2048) return ATTN_ERR_UNSUPPORTED;
     if (!aligned16(x) || !aligned16(w) || !aligned16(b) || !aligned16(y)) return ATTN_ERR_ALIGN;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (rows <= kFewRows) {
+    if (few_rows(rows)) {
         const int threads = threads_for(C);
         return (int)attn::launch_after_previous(ln_forward_few_rows_kernel<2>, dim3(few_rows_grid(rows, threads, 40, 2)), dim3(threads),
                                                 0, s, x, w, b, eps, mean, rstd, y, rows, C);
@@ -467,7 +466,7 @@ int layernorm_sm100_backward(const float *dy, const float *x, const float *mean,
     if (C % 4 != 0 || C > 2048) return ATTN_ERR_UNSUPPORTED;
     if (!aligned16(dy) || !aligned16(x) || !aligned16(w) || !aligned16(dx)) return ATTN_ERR_ALIGN;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (rows <= kFewRows || C <= 512) {  // (8192 x 384: 15.1 -> 12.2 us)
+    if (few_rows(rows) || C <= 512) {  // (8192 x 384: 15.1 -> 12.2 us)
         // whole clusters (blocks without rows add zeros)
         const int threads = threads_for(C);
         const int grid = (few_rows_grid(rows, threads, 128, 4) + kFewCluster - 1) / kFewCluster * kFewCluster;

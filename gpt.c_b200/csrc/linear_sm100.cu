@@ -536,12 +536,6 @@ Problem make_problem(int M, int N, int K, int bn, int splits) {
     return p;
 }
 
-int sm_count() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // Tile shape and number of pieces of the contraction for a [M, N] result of kb contraction blocks, chosen by expected
 // time: a fixed part, and for every round over the SMs a charge and kb blocks at the slower of what one CTA takes when
 // it is alone (`block`) and what L2 needs to feed all CTAs of the round.  The constants are a fit to the kernel's times
@@ -622,7 +616,7 @@ int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *p
     p.wide = p.ldc % 8 == 0 && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(c) & 31u) == 0;
     p.wide_planes = p.N % 16 == 0 && (reinterpret_cast<uintptr_t>(planes) & 31u) == 0;
     p.plane_words = attn::plane_bytes((size_t)p.M * p.N) / 4;
-    const int most = sm_count();
+    const int most = attn::sm_count();
     const int grid = p.total < most ? p.total : most;
     return (int)attn::launch_after_previous(kernel, dim3(grid), dim3(kThreads), sizeof(Smem), s, maps, bias, c,
                                                      static_cast<uint32_t *>(planes), p, status);
@@ -746,7 +740,7 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
         if (cut.splits > 1 && cut.ns < plan.ns) plan = cut;
     }
     int split = 1, rc;
-    if (plan_split(M, K, np, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, status, s);
+    if (plan_split(M, K, np, sms, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, sms, status, s);
     CUtensorMap ma, mb, mc;
     Problem p = make_problem(M, K, np, plan.bn, plan.splits);
     if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
@@ -778,9 +772,11 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     int rc = attn::device_status_word(&status);
     if (rc != ATTN_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const Plan plan = plan_tiles(M, N, (K + kBK - 1) / kBK, sm_count());
+    const int sms = attn::sm_count();
+    const Plan plan = plan_tiles(M, N, (K + kBK - 1) / kBK, sms);
     int split = 1;
-    if (plan_split(M, N, K, &split) < plan.ns) return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, status, s);
+    if (plan_split(M, N, K, sms, &split) < plan.ns)
+        return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, sms, status, s);
     CUtensorMap ma, mb;
     // with plain stores (N not a multiple of 4) only the widest tiles are built
     Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, 1);
@@ -819,7 +815,7 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     int rc = attn::device_status_word(&status);
     if (rc != ATTN_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int sms = sm_count();
+    const int sms = attn::sm_count();
     const float *g = dy;  // without row classes [M, np] from here on
     if (classes) {
         if ((rc = gradients_by_row_class(dy, x, w, dx, dw, M, N, K, sms, status, s)) != 0) return rc;

@@ -241,9 +241,13 @@ __global__ void __launch_bounds__(Roles<kSplit>::kThreads, Roles<kSplit>::kPerSm
     if (kSplit) cluster_sync_all();  // this CTA's partial tile stays until the others have read it
 }
 
-// CTAs of clusters of that many that find an SM each at the same time (a cluster stays inside a GPC, so larger ones
-// leave SMs over; sizes that are not listed leave too many): beyond it a second wave, or sharing, sets in.
-constexpr int kAlone[kMaxSplit + 1] = {0, 148, 148, 117, 128, 120, 108, 0, 104};
+// CTAs of clusters of `split` that find an SM each at the same time; beyond it a second wave, or sharing, sets in.  A
+// cluster stays inside a GPC, so larger ones leave SMs over: the table is what a GPU of 148 SMs had room for (clusters of
+// seven leave too many), on one with fewer SMs it is taken in proportion.
+int alone(int split, int sms) {
+    constexpr int kOn148[kMaxSplit + 1] = {0, 148, 148, 117, 128, 120, 108, 0, 104};
+    return kOn148[split] * sms / 148;
+}
 
 int rows_per_tile(int M) {
     const int tiles = (M + 127) / 128;
@@ -255,21 +259,21 @@ int rows_per_tile(int M) {
 // Time of the product in nanoseconds as measured on shapes of 16 to 1500 rows and 512 to 6400 columns (within 10 %): a
 // CTA takes about 300 ns per contraction block, whatever the rows, because that is how fast one SM's loads of 128
 // separate rows arrive; sharing an SM makes it 390 to 600 ns; cluster barriers and the exchange cost 1.3 us.
-int plan_split(int M, int cols, int kc, int *split) {
+int plan_split(int M, int cols, int kc, int sms, int *split) {
     const int bm = rows_per_tile(M), units = (cols + kBM - 1) / kBM * ((M + bm - 1) / bm), kb = (kc + kBK - 1) / kBK;
     long long best = 0;
     for (int s = 1; s <= kMaxSplit; s++) {
-        if (kAlone[s] == 0 || s > kb || (s > 1 && units * s > 2 * kAlone[s])) continue;
+        if (alone(s, sms) == 0 || s > kb || (s > 1 && units * s > 2 * alone(s, sms))) continue;
         const int per = (kb + s - 1) / s;
-        const long long t = s == 1 ? 1650 + 16 * bm + (units <= 148 ? 295ll * per : (400ll * per + 1000) * units / 148)
-                             : 2900 + 16 * bm + (long long)per * (units * s <= kAlone[s] ? 310 : 300 + 2 * bm);
+        const long long t = s == 1 ? 1650 + 16 * bm + (units <= sms ? 295ll * per : (400ll * per + 1000) * units / sms)
+                             : 2900 + 16 * bm + (long long)per * (units * s <= alone(s, sms) ? 310 : 300 + 2 * bm);
         if (best == 0 || t < best) best = t, *split = s;
     }
     return best < 0x7fffffff ? (int)best : 0x7fffffff;
 }
 
 int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, const float *bias, float *out, void *planes, int M,
-                 int cols, int kc, int split, int *status, cudaStream_t s) {
+                 int cols, int kc, int split, int sms, int *status, cudaStream_t s) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -297,7 +301,7 @@ int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, 
     const int grid = (cols + kBM - 1) / kBM * p.tiles_m * p.split;
     const int stage = kATileBytes + p.bm * 128;
     // more CTAs than fit one to an SM: two or three share one, and its shared memory
-    const int sharing = grid > 2 * kAlone[p.split] ? 3 : (grid > kAlone[p.split] ? 2 : 1);
+    const int room = alone(p.split, sms), sharing = grid > 2 * room ? 3 : (grid > room ? 2 : 1);
     p.stages = kMostBytes / sharing / stage;
     if (p.stages > kMaxStages) p.stages = kMaxStages;
     if (p.stages > p.kb_per_split) p.stages = p.kb_per_split;

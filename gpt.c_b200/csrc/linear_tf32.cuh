@@ -78,8 +78,8 @@ inline int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows, s
 // or with w_mn_major [w_rows, cols] (its rows past w_rows, up to kc, read as zeros); optionally the bf16 planes of out.
 // `split` CTAs share the contraction of a tile.  Returns ATTN_OK or an error.
 int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, const float *bias, float *out, void *planes, int M,
-                 int cols, int kc, int split, int *status, cudaStream_t s);
+                 int cols, int kc, int split, int sms, int *status, cudaStream_t s);
 // The best `split` and the time in nanoseconds it is expected to take.
-int plan_split(int M, int cols, int kc, int *split);
+int plan_split(int M, int cols, int kc, int sms, int *split);
 
 }  // namespace lin

@@ -17,10 +17,8 @@ namespace {
 constexpr int kThreads = 256;
 
 int grid_for(size_t work_items) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t need = (work_items + kThreads - 1) / kThreads;
-    const size_t cap = (size_t)sms * 16;
+    const size_t cap = (size_t)attn::sm_count() * 16;
     return (int)(need < cap ? (need ? need : 1) : cap);
 }
 
