@@ -42,7 +42,7 @@ using namespace tc05;
 constexpr int kThreads = 384;
 constexpr int kEpiWarps = 8;
 
-// Tile width kBN (128 or 256 columns) and pipeline depth are chosen per problem: wide tiles halve the
+// Tile width kBN (128, 192 or 256 columns) and pipeline depth are chosen per problem: wide tiles halve the
 // shared-memory and L2 traffic per flop, narrow ones fill the SMs better when there are few tiles.
 template <int kBN, int kStages, bool kStage>
 struct __align__(1024) SmemT {
@@ -63,7 +63,7 @@ struct Problem {
     int wide, wide_planes;  // rows of C / of the planes start on 32-byte boundaries
     size_t plane_words;     // distance from the hi to the lo plane
     size_t ldc;             // floats from one row of C to the next
-    int b_shift;            // B's contraction index runs this far behind A's (see RowClasses)
+    int b_shift;            // B's contraction index runs this far behind A's (see RowClass)
     int a_whole[4];         // columns in whole blocks of A's views
     int a_shift[4];         // columns of A's views before the first column of dy (dW from row classes)
     int m_fast;  // consecutive work items walk down the rows of C (else along its columns)
@@ -155,8 +155,8 @@ __device__ __forceinline__ void store_words(void *dst, int left, int wide, const
 }
 
 // kEpi 0: C = acc (+ bias), optional bf16 planes; kEpi 1: C += acc (bulk reduction)
-// kDirect: the result goes out with plain coalesced 4-byte stores instead of the copy engine, for outputs
-// whose row pitch is not a multiple of 16 bytes (the 50257-wide vocabulary projection).
+// kDirect: the result goes out with plain coalesced 4-byte stores, for outputs whose row pitch is not a multiple of 16
+// bytes (the 50257-wide vocabulary projection).
 template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kClasses>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__restrict__ bias, float *__restrict__ c_direct,
@@ -291,9 +291,9 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
         }
     } else if (warp >= 4) {
         // ------------------------------ epilogue ------------------------------
-        // Every warp takes 32 rows (its tensor-memory lane quarter) and half of the columns, 32 at a time, through
-        // a staging buffer of its own: accumulator -> registers (+ bias) -> shared memory -> copy engine.  No warp
-        // waits for another one.
+        // Every warp takes 32 rows (its tensor-memory lane quarter) and half of the columns, 32 at a time: accumulator
+        // -> registers (+ bias) -> global memory; what is added into the result, and rows that are not 16-byte aligned,
+        // by way of a staging buffer of the warp's own.  No warp waits for another one.
         const int quarter = warp & 3;
         const int half = (warp - 4) >> 2;
         uint8_t *buf = sm.out[kEpi == 1 || kDirect ? warp - 4 : 0];
@@ -553,14 +553,13 @@ constexpr int kL2BytesPerNs = 18190;
 
 // Time of `tiles` tiles of kb contraction blocks each, without the fixed part.
 long long rounds_ns(const Cost &c, long long tiles, int kb, int sms) {
-    const int units = sms;
     const long long bytes = kATileBytes + (long long)c.bn * kBK * 4;  // a CTA's operands of one block
     auto round = [&](long long busy) {
         const long long fed = bytes * busy / kL2BytesPerNs;
         return c.round + kb * (fed > c.block ? fed : c.block);
     };
-    const long long rest = tiles % units;
-    return tiles / units * round(units) + (rest ? round(rest) : 0);
+    const long long rest = tiles % sms;
+    return tiles / sms * round(sms) + (rest ? round(rest) : 0);
 }
 
 int at_most_int(long long v) { return v < 0x7fffffff ? (int)v : 0x7fffffff; }
@@ -691,7 +690,7 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
             Problem p = make_problem(c.rows, K, N + c.shift, plan.bn, plan.splits);
             p.ldc = 4 * (size_t)K, p.b_shift = c.shift;
             if ((rc = map_k_major(&ma, c.dy, c.rows, N + c.shift, 128, 4 * (size_t)N)) != 0) return rc;
-            p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 ) == 0;
+            p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32) == 0;
             if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
             float *out = dx + (size_t)j * K;
             if (p.splits > 1) {
@@ -744,7 +743,7 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
     CUtensorMap ma, mb, mc;
     Problem p = make_problem(M, K, np, plan.bn, plan.splits);
     if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
-    p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32 ) == 0;
+    p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32) == 0;
     if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
     if (p.splits == 1) return launch<false, true, 0>(ma, mb, ma, nullptr, dx, nullptr, p, status, s);
     // the pieces of the contraction add into dx with bulk reductions: start from zeros
@@ -782,7 +781,7 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, 1);
     p.m_fast = stream_rows_of_c(M, N, K);
     if ((rc = map_k_major(&ma, x, M, K, 128)) != 0) return rc;
-    if ((rc = map_k_major(&mb, w, N, K, p.bn )) != 0) return rc;
+    if ((rc = map_k_major(&mb, w, N, K, p.bn)) != 0) return rc;
     if (direct) {
         return launch_one<false, false, 0, 256, 4, false, true>(ma, mb, ma, bias, y, nullptr, p, status, s);
     }
@@ -834,7 +833,7 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         Problem pdw = make_problem(N, K, M, plan.bn, plan.splits);
         pdw.a_one = map_mn_major_blocks(&ma, g, M, np, 4) == 0;
         if (!pdw.a_one && (rc = map_mn_major(&ma, g, M, np)) != 0) return rc;
-        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32 ) == 0;
+        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32) == 0;
         if (!pdw.b_one && (rc = map_mn_major(&mb, x, M, K)) != 0) return rc;
         if ((rc = map_out_f32(&mc, dw, N, K)) != 0) return rc;
         rc = launch<true, true, 1>(ma, mb, mc, nullptr, dw, nullptr, pdw, status, s);

@@ -116,9 +116,9 @@ def test_fast_forward_vs_oracle(pkg, gpu, oracle, shape):
 
 
 @pytest.mark.parametrize("B,T,H", [(41, 60, 16), (41, 64, 15), (20, 130, 16), (7, 700, 20)])
-def test_fast_forward_takes_over_items(pkg, gpu, oracle, B, T, H):
-    """More query tiles than two per SM, so that thread blocks take over those of blocks that have not started: one
-    key step per tile, one or two, many; more than four items per block wrap the slots of the answers."""
+def test_fast_forward_of_more_tiles_than_fit_at_once(pkg, gpu, oracle, B, T, H):
+    """More query tiles than two per SM, so that thread blocks follow others on an SM and reuse its tensor memory: one
+    key step per tile, one or two, many."""
     x, _ = seeded(33, B, T, H, 64)
     out, lse, _ = run_cuda(pkg, gpu, x, None, H)
     ref_out, ref_lse = oracle.forward(x, H, want_lse=True)

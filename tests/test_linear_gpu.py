@@ -109,7 +109,7 @@ def test_linear_backward_vs_cpu(pkg, M, N, K):
 @pytest.mark.parametrize("M,N,K", [
     (1, 96, 64), (16, 128, 32), (17, 260, 96),   # one tile of 16 or 32 activation rows, one CTA or two
     (48, 1001, 128), (129, 384, 512), (250, 130, 1024), (348, 768, 3072),  # clusters of 6 and 8 CTAs, unaligned columns
-    (2600, 3000, 512), (6000, 1104, 256), (8192, 1152, 384), (3000, 520, 1600),  # CTA pairs 256 and 192 columns wide
+    (2600, 3000, 512), (6000, 1104, 256), (8192, 1152, 384), (3000, 520, 1600),  # tiles of 256, 192 and 128 columns, several per CTA
 ])
 def test_linear_tile_shapes(pkg, M, N, K):
     """Forward with bias and planes, dx, dW and db where the choice of kernel, tile shape and split changes."""
