@@ -361,7 +361,10 @@ __device__ __forceinline__ void store_cols(float *row, int col, int D, float4 v)
 // partial results are merged at the end: a block then has its SM to itself and the longest-first order balances the
 // SMs.  (With one group per block and two blocks per SM, the SMs were busy for 71 % of the launch on average, because
 // the long blocks that start together share an SM.)  B=4 T=1024 H=6 D=128 233 -> 192 us, B=2 T=2048 H=4 D=80
-// 395 -> 183 us.  Up to 64 head columns two blocks still fit.
+// 395 -> 183 us.  Up to 64 head columns two blocks still fit, with 128 registers per thread and up to 144 bytes of
+// them spilled.  That pays when there are more blocks than SMs: B=4 T=1024 H=12 D=64 202 us against 212 with one block
+// and no spills, D=16 104 against 125, B=8 T=512 H=16 D=32 92 against 109.  With one block or less per SM it costs:
+// B=1 T=2048 H=4 D=64 219 against 143, B=8 T=128 H=12 D=64 22 against 17.
 // ---------------------------------------------------------------------------------------
 constexpr int kFwdGroup = 128, kFwdThreads = 2 * kFwdGroup, kFwdRows = 64;
 

@@ -17,9 +17,9 @@
 // plan_tiles picks the width.
 //
 // What bounds the kernel: a 128 x 256 tile needs 48 KB per contraction block, and the SMs get 15 to 18 TB/s from L2
-// together (64 % tensor pipe active).  The result is written straight from registers, a row per lane in 32-byte
-// sectors: staging it for the copy engine costs shared memory that the pipeline wants, bandwidth, and hand-overs
-// between warps (QKV forward with bf16 planes 72 -> 67 us at 192 columns).
+// together (tensor pipe active 48 % in the forward with bf16 planes, 76 % in dW).  The result is written straight from
+// registers, a row per lane in 32-byte sectors: staging it for the copy engine costs shared memory that the pipeline
+// wants, bandwidth, and hand-overs between warps (QKV forward with bf16 planes 72 -> 67 us at 192 columns).
 //
 // Warp roles (384 threads, one CTA per SM, grid = number of SMs, tiles handed out round robin):
 //   warp 0      TMA producer
