@@ -43,6 +43,8 @@ bool stages_ok(int flags) { return !((flags & ATTN_FLAG_PREPARE_ONLY) && (flags 
 
 bool use_fast(int D, int flags) { return D == 64 && !(flags & ATTN_FLAG_FORCE_GENERIC); }
 
+bool use_attn24(int D) { return D <= attn::kAttn24MaxD; }
+
 // bf16 planes of a [B, T, W] tensor as a 4-D map {W, T, B, plane}, box {64, box_rows, 1, 1}.
 int encode_planes(CUtensorMap *map, const void *base, int B, int T, int W, size_t plane_stride_bytes, int box_rows) {
     const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)T, (cuuint64_t)B, 2};
@@ -115,6 +117,13 @@ int encode_tiled(CUtensorMap *map, CUtensorMapDataType dtype, unsigned rank, con
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
+int attn24_rows_map(CUtensorMap *map, const void *base, int B, int T, int W, int D, int rows) {
+    const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)T, (cuuint64_t)B, 1};
+    const cuuint64_t strides[3] = {(cuuint64_t)W * 4, (cuuint64_t)W * 4 * (cuuint64_t)T, (cuuint64_t)W * 4 * (cuuint64_t)T * (cuuint64_t)B};
+    const cuuint32_t box[4] = {(cuuint32_t)D, (cuuint32_t)rows, 1, 1};
+    return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
 int device_status_word(int **status) {
     DeviceState *ds = nullptr;
     const int rc = current_device_state(&ds);
@@ -154,6 +163,8 @@ int attn_sm100_init(void) {
     if ((e = attn::generic_set_attributes()) != cudaSuccess) return (int)e;
     if ((e = attn::fast_fwd_set_attributes()) != cudaSuccess) return (int)e;
     if ((e = attn::fast_bwd_set_attributes()) != cudaSuccess) return (int)e;
+    if ((e = attn::attn24_fwd_set_attributes()) != cudaSuccess) return (int)e;
+    if ((e = attn::attn24_bwd_set_attributes()) != cudaSuccess) return (int)e;
 
     int sms = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
@@ -212,7 +223,8 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
         if (rc != 0) return rc;
         e = attn::launch_fast_forward(map_x, out, out_copy, lse, B, T, H, ds->status, s);
     } else {
-        e = attn::launch_generic_forward(qkv, out, out_copy, lse, B, T, H, D, s);
+        e = use_attn24(D) ? attn::launch_attn24_forward(qkv, out, out_copy, lse, B, T, H, D, ds->status, s)
+                          : attn::launch_generic_forward(qkv, out, out_copy, lse, B, T, H, D, s);
     }
     return (int)e;
 }
@@ -269,7 +281,10 @@ int attn_sm100_backward(const void *saved, const float *out, const float *lse, c
             if (e != cudaSuccess) return (int)e;
         }
         if (!core) return ATTN_OK;
-        e = attn::launch_generic_backward(xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, s);
+        CUtensorMap map_x = {};
+        if (use_attn24(D) && D % 16 == 0 && (rc = encode_planes(&map_x, saved, B, T, 3 * H * D, xplane, 64)) != 0) return rc;
+        e = use_attn24(D) ? attn::launch_attn24_backward(map_x, xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, ds->status, s)
+                          : attn::launch_generic_backward(xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, s);
     }
     return (int)e;
 }

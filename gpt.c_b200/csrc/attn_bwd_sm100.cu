@@ -72,6 +72,7 @@
 // operands in shared memory is limited by shared-memory bandwidth (48 instead of 32 cycles at
 // N = 64).  P^T and dS^T overwrite S^T and dP^T in place: each run of 16 columns becomes 8 columns
 // of packed bf16 hi parts followed by 8 columns of packed lo parts.
+#include "attn24.cuh"
 #include "attn_internal.h"
 #include "tc05.cuh"
 
@@ -841,6 +842,487 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// General backward: any head size up to 128; fp32 dO, P and dS as three bf16 terms (attn24.cuh), Q, K, V as the two the
+// forward saved.
+//
+// One CTA per (b, h, 128 keys), which walks the queries from the diagonal on in steps of 64:
+//     S^T = K Q^T, dP^T = V dO^T      (lanes = keys; 4 and 5 term products)
+//     dV += P^T dO, dK += dS^T Q      (P^T, dS^T from tensor memory; 6 and 5)
+//     dQ^T = K^T dS^T                 (lanes = head columns; 5)
+// The workers turn S^T and dP^T into P^T and dS^T (in tensor memory, dS^T also in shared memory), add dV and dK of the step
+// to their registers, and leave dQ in shared memory, from where the copy engine adds it to dqkv (zero-filled by the
+// preparation kernel) row by row.  Reductions from registers, a warp's lanes 32 consecutive floats, held the workers up for
+// 1700 (D = 64) to 3400 (D = 128) cycles per step.  Q and dO of the next step are on their way while the products that
+// still need the current ones run.
+//
+// One block of 64 head columns: dQ^T would need only half of the 128 rows a product has, so the two planes of K are stacked,
+// rows 64 to 127 hold the products with K's lo plane (3 passes instead of 5), and both halves are added to dqkv.
+// Two blocks: shared memory is full; dS^T takes dO's place once dV has been computed, and dQ leaves in two halves, the
+// second one (32 queries) in the next step.
+//
+// What bounds it: the tensor cores (25 bf16 passes over five products: 8400 cycles per step at D = 128).
+// ---------------------------------------------------------------------------------------
+namespace general {
+
+using namespace attn24;
+
+template <int kK>  // head columns in groups of 16
+struct __align__(1024) Bwd24Smem {
+    static constexpr int kBlocks = (kK + 3) / 4;  // of 64 columns
+    static constexpr int kKeyPlane = kBlocks * kTile * 128, kQueryPlane = kBlocks * kStep * 128, kDsPlane = kTile * 128;
+    static constexpr int kOutRows = kBlocks == 1 ? 2 * kStep : kStep / 2, kOuts = kK < 4 ? 2 : 1;
+    static constexpr int kDs = kBlocks == 1 ? 3 * kQueryPlane : 0;  // dS^T in g: behind dO, or in its place
+    uint8_t k[2][kKeyPlane], v[2][kKeyPlane], q[2][kQueryPlane];
+    uint8_t g[kDs + 3 * kDsPlane];  // dO [3][kQueryPlane], dS^T [3][kDsPlane]
+    // dQ on its way to memory, rows of D: [step parity][K plane, query], or half of the queries
+    __align__(128) float out[kOuts][kOutRows * 16 * kK];
+    // dO of the next step as it comes (two blocks: in g, over the last two planes of dO itself)
+    __align__(128) float raw_own[kBlocks == 1 ? kStep * 16 * kK : 32];
+    __device__ __forceinline__ float *raw() { return kBlocks == 1 ? raw_own : reinterpret_cast<float *>(g + kQueryPlane); }
+    float stat[2][2][kStep];               // [step parity][log-sum-exp, delta]
+    uint64_t go_s, go_dp, go_dv, go_dk, go_dq;  // operands are in place (one arrival per worker warp; Q from the copy engine)
+    uint64_t done_s, done_dp, done_dv, done_dk, done_dq;
+    uint64_t v_full, raw_full, raw_free, stat_full[2], stat_free[2];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+enum Site24 : int {
+    SITE24_GO_S = 321, SITE24_GO_DP, SITE24_GO_DV, SITE24_GO_DK, SITE24_GO_DQ, SITE24_S, SITE24_DP, SITE24_DV, SITE24_DK, SITE24_DQ, SITE24_V, SITE24_RAW_FULL,
+    SITE24_RAW_FREE, SITE24_STAT, SITE24_SMEM_ALIGN
+};
+
+// kTma: D = 16 kK, and the copy engine fetches Q, K, V and dO; else the workers do.
+template <int kK, bool kTma>
+__global__ void __launch_bounds__(attn24::kThreads, 1)
+attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_do,
+                  const __grid_constant__ CUtensorMap map_dq, const __nv_bfloat16 *__restrict__ xhi,
+                  const __nv_bfloat16 *__restrict__ xlo, const float *__restrict__ lse, const float *__restrict__ delta,
+                  const float *__restrict__ dout, float *__restrict__ dqkv, int T, int H, int D_arg, float scale, Scale scale_log2,
+                  int *status) {
+    using Smem = Bwd24Smem<kK>;
+    constexpr int kKeyPlane = Smem::kKeyPlane, kQueryPlane = Smem::kQueryPlane, kDsPlane = Smem::kDsPlane;
+    constexpr int kBlocks = Smem::kBlocks;
+    constexpr bool kOne = kBlocks == 1;
+    constexpr int kPiece = kOne ? 8 : 4;  // scores a worker has in registers at a time (four: fewer spilled)
+    constexpr uint32_t kColS = 0, kColDP = 96, kColDQ = 192, kColDV = 256, kColDK = 256 + 16 * kK;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    if ((smem_u32(smem_raw) & 1023u) != 0) {
+        if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE24_SMEM_ALIGN);
+        return;
+    }
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int D = kTma ? 16 * kK : D_arg;
+    const bool vec = kTma || D % 4 == 0;
+    WaitCtx ctx{&sm.abort_flag, status};
+    if (tid == 0) {
+        sm.abort_flag = 0;
+        mbar_init(&sm.go_s, kTma ? 1 : kWorkWarps);
+        mbar_init(&sm.go_dp, kWorkWarps);
+        mbar_init(&sm.go_dv, kWorkWarps);
+        mbar_init(&sm.go_dk, kWorkWarps);
+        mbar_init(&sm.go_dq, kWorkWarps);
+        mbar_init(&sm.done_s, 1);
+        mbar_init(&sm.done_dp, 1);
+        mbar_init(&sm.done_dv, 1);
+        mbar_init(&sm.done_dk, 1);
+        mbar_init(&sm.done_dq, 1);
+        mbar_init(&sm.v_full, 1);
+        mbar_init(&sm.raw_full, 1);
+        mbar_init(&sm.raw_free, kWorkWarps);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&sm.stat_full[i], 1);
+            mbar_init(&sm.stat_free[i], kWorkWarps);
+        }
+        fence_barrier_init();
+    }
+    if (warp == kWorkWarps) {
+        tmem_alloc_then_launch_dependents(&sm.tmem_base, 512);
+    }
+    pdl_wait();
+    const int nt = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nt;
+    const int k0 = (int)blockIdx.x / nbh * kTile;  // the first keys are seen by the most queries
+    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
+    const int C = H * D, nsteps = (T - k0 + kStep - 1) / kStep;
+    const size_t C3 = 3 * (size_t)C, head = (size_t)b * T * C3 + (size_t)h * D;
+    const float *dhead = dout + (size_t)b * T * C + (size_t)h * D;
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
+
+    if (warp == kWorkWarps + 1) {
+        // ------------------------------ producer: K, V, Q and dO ------------------------------
+        if (kTma && lane == 0) {
+            auto load_keys = [&](uint8_t *tile, uint64_t *bar, int x) {
+#pragma unroll 1
+                for (int plane = 0; plane < 2; plane++)
+#pragma unroll 1
+                    for (int i = 0; i < kBlocks; i++)
+#pragma unroll 1
+                        for (int half = 0; half < 2; half++)
+                            tma_load_4d(tile + plane * kKeyPlane + i * (kTile * 128) + half * (kStep * 128), &map_x, bar, x + 64 * i,
+                                        k0 + half * kStep, b, plane);
+            };
+            for (int n = 0; n < nsteps; n++) {
+                auto load_do = [&]() {
+                    mbar_expect_tx(&sm.raw_full, kStep * 16 * kK * 4);
+                    tma_load_4d(sm.raw(), &map_do, &sm.raw_full, h * D, k0 + n * kStep, b, 0);
+                };
+                if (kOne) {
+                    if (n > 0 && !await_thread(&sm.raw_free, (n - 1) & 1, ctx, SITE24_RAW_FREE)) break;
+                    load_do();
+                }
+                if (n > 0 && !await_thread(&sm.done_dk, (n - 1) & 1, ctx, SITE24_DK)) break;
+                mbar_expect_tx(&sm.go_s, 2 * kQueryPlane + (n == 0 ? 2 * kKeyPlane : 0));
+#pragma unroll 1
+                for (int plane = 0; plane < 2; plane++)
+#pragma unroll 1
+                    for (int i = 0; i < kBlocks; i++)
+                        tma_load_4d(sm.q[plane] + i * (kStep * 128), &map_x, &sm.go_s, h * D + 64 * i, k0 + n * kStep, b, plane);
+                if (!kOne) {  // its place is dS's
+                    if (n > 0 && !await_thread(&sm.done_dq, (n - 1) & 1, ctx, SITE24_DQ)) break;
+                    load_do();
+                }
+                if (n == 0) {
+                    load_keys(sm.k[0], &sm.go_s, C + h * D);
+                    mbar_expect_tx(&sm.v_full, 2 * kKeyPlane);
+                    load_keys(sm.v[0], &sm.v_full, 2 * C + h * D);
+                }
+            }
+        }
+    } else if (warp == kWorkWarps + 2) {
+        // ------------------------------ row statistics ------------------------------
+        for (int n = 0; n < nsteps; n++) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int t = k0 + n * kStep + 32 * (i & 1) + lane;
+                v[i] = t < T ? (i < 2 ? lse : delta)[(size_t)bh * T + t] : 0.f;
+            }
+            if (n > 1) await(&sm.stat_free[n & 1], ((n >> 1) - 1) & 1, ctx, SITE24_STAT);
+#pragma unroll
+            for (int i = 0; i < 4; i++) sm.stat[n & 1][i >> 1][32 * (i & 1) + lane] = v[i];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.stat_full[n & 1]);
+        }
+    } else if (warp > kWorkWarps) {
+        // the rest of the issuing group
+    } else if (warp == kWorkWarps) {
+        // ------------------------------ MMA issuer ------------------------------
+        constexpr uint32_t idesc_s = idesc_bf16_f32(kTile, kStep, 0, 0), idesc_g = idesc_bf16_f32(kTile, 16 * kK, 0, 1),
+                           idesc_q = idesc_bf16_f32(kTile, kStep, 1, 1);
+        const uint32_t leader = elect_leader();
+        const uint64_t k_km = smem_desc_sw128(smem_u32(sm.k[0]), 16, 1024), v_km = smem_desc_sw128(smem_u32(sm.v[0]), 16, 1024);
+        const uint64_t q_km = smem_desc_sw128(smem_u32(sm.q[0]), 16, 1024), g_km = smem_desc_sw128(smem_u32(sm.g), 16, 1024);
+        const uint64_t q_mn = smem_desc_sw128(smem_u32(sm.q[0]), kStep * 128, 1024);
+        const uint64_t g_mn = smem_desc_sw128(smem_u32(sm.g), kStep * 128, 1024);
+        // rows 64 to 127: the second block of head columns, or where there is one block, K's lo plane, which follows it
+        const uint64_t k_mn = smem_desc_sw128(smem_u32(sm.k[0]), kTile * 128, 1024);
+        const uint64_t ds_mn = smem_desc_sw128(smem_u32(sm.g + Smem::kDs), 1024, 1024);
+        // terms of the two operands, smallest products first
+        constexpr int kSA[4] = {1, 1, 0, 0}, kSB[4] = {1, 0, 1, 0};
+        constexpr int kPA[5] = {1, 0, 1, 0, 0}, kPB[5] = {1, 2, 0, 1, 0};
+        constexpr int kVA[6] = {2, 1, 0, 1, 0, 0}, kVB[6] = {0, 1, 2, 0, 1, 0};
+        constexpr int kKA[5] = {1, 2, 0, 1, 0}, kKB[5] = {1, 0, 1, 0, 0};
+        for (int n = 0; n < nsteps; n++) {
+            await(&sm.go_s, n & 1, ctx, SITE24_GO_S);
+#pragma unroll
+            for (int term = 0; term < 4; term++)
+#pragma unroll
+                for (int kk = 0; kk < kK; kk++)
+                    mma_ss_lead(leader, tmem + kColS, desc_advance(k_km, kSA[term] * kKeyPlane + (kk >> 2) * (kTile * 128) + (kk & 3) * 32),
+                                desc_advance(q_km, kSB[term] * kQueryPlane + (kk >> 2) * (kStep * 128) + (kk & 3) * 32), idesc_s,
+                                term > 0 || kk > 0 ? 1u : 0u);
+            tc_commit_lead(leader, &sm.done_s);
+            await(&sm.go_dp, n & 1, ctx, SITE24_GO_DP);
+            if (kTma && n == 0) await(&sm.v_full, 0, ctx, SITE24_V);
+#pragma unroll
+            for (int term = 0; term < 5; term++)
+#pragma unroll
+                for (int kk = 0; kk < kK; kk++)
+                    mma_ss_lead(leader, tmem + kColDP, desc_advance(v_km, kPA[term] * kKeyPlane + (kk >> 2) * (kTile * 128) + (kk & 3) * 32),
+                                desc_advance(g_km, kPB[term] * kQueryPlane + (kk >> 2) * (kStep * 128) + (kk & 3) * 32), idesc_s,
+                                term > 0 || kk > 0 ? 1u : 0u);
+            tc_commit_lead(leader, &sm.done_dp);
+            await(&sm.go_dv, n & 1, ctx, SITE24_GO_DV);
+#pragma unroll
+            for (int term = 0; term < 6; term++)
+#pragma unroll
+                for (int kk = 0; kk < kStep / 16; kk++)
+                    mma_ts_lead(leader, tmem + kColDV, tmem + kColS + term_column(kVA[term], kk),
+                                desc_advance(g_mn, kVB[term] * kQueryPlane + kk * 2048), idesc_g, term > 0 || kk > 0 ? 1u : 0u);
+            tc_commit_lead(leader, &sm.done_dv);
+            await(&sm.go_dk, n & 1, ctx, SITE24_GO_DK);
+#pragma unroll
+            for (int term = 0; term < 5; term++)
+#pragma unroll
+                for (int kk = 0; kk < kStep / 16; kk++)
+                    mma_ts_lead(leader, tmem + kColDK, tmem + kColDP + term_column(kKA[term], kk),
+                                desc_advance(q_mn, kKB[term] * kQueryPlane + kk * 2048), idesc_g, term > 0 || kk > 0 ? 1u : 0u);
+            tc_commit_lead(leader, &sm.done_dk);
+            if (!kOne) await(&sm.go_dq, n & 1, ctx, SITE24_GO_DQ);
+#pragma unroll
+            for (int term = 0; term < (kOne ? 3 : 5); term++) {
+                const int ka = kOne ? 0 : kKB[term], ds = kOne ? 2 - term : kKA[term];
+#pragma unroll
+                for (int kk = 0; kk < kTile / 16; kk++)
+                    mma_ss_lead(leader, tmem + kColDQ, desc_advance(k_mn, ka * kKeyPlane + kk * 2048),
+                                desc_advance(ds_mn, ds * kDsPlane + kk * 2048), idesc_q, term > 0 || kk > 0 ? 1u : 0u);
+            }
+            tc_commit_lead(leader, &sm.done_dq);
+        }
+    } else {
+        // ------------------------------ workers ------------------------------
+        const int quarter = warp & 3, cq = warp >> 2, row = 32 * quarter + lane;
+        const uint32_t lane_addr = (uint32_t)(quarter << 5) << 16;
+        const Chunk mine(tid);
+        auto put_q = [&](int n) {
+            if (kTma) return;
+            const int t = k0 + n * kStep + mine.r;
+            const size_t from = head + (size_t)t * C3;
+#pragma unroll
+            for (int i = 0; i < kBlocks; i++)
+                if (mine.has<kK>(i)) {
+                    copy8(sm.q[0] + mine.at + i * (kStep * 128), xhi + from, mine.col(i), D, t < T, vec);
+                    copy8(sm.q[1] + mine.at + i * (kStep * 128), xlo + from, mine.col(i), D, t < T, vec);
+                }
+            warp_arrive(&sm.go_s, lane);
+        };
+        // dO: from shared memory (kTma), or one step ahead in registers
+        float greg[kBlocks][8];
+        auto request_g = [&](int n) {
+            if (kTma) return;
+            const int t = k0 + n * kStep + mine.r;
+            const float *from = dhead + (size_t)t * C;
+#pragma unroll
+            for (int i = 0; i < kBlocks; i++)
+                if (mine.has<kK>(i)) load8(greg[i], from, mine.col(i), D, t < T, vec);
+        };
+        auto put_g = [&](int n) {
+            if (kTma) {
+                await(&sm.raw_full, n & 1, ctx, SITE24_RAW_FULL);
+#pragma unroll
+                for (int i = 0; i < kBlocks; i++)
+                    if (mine.has<kK>(i)) lds8(greg[i], sm.raw() + mine.r * D + mine.col(i), mine.c);
+                if (kOne) warp_arrive(&sm.raw_free, lane);  // its fence holds the copy engine back until these values are in registers
+                else named_sync(5, kWorkers);
+            }
+#pragma unroll
+            for (int i = 0; i < kBlocks; i++)
+                if (mine.has<kK>(i)) store_split3(sm.g, kQueryPlane, mine.at + i * (kStep * 128), greg[i]);
+            warp_arrive(&sm.go_dp, lane);
+        };
+        request_g(0);
+        if (!kTma) {
+#pragma unroll
+            for (int i = 0; i < kBlocks; i++) {  // K and V of this CTA's keys, 64 rows by 64 columns at a time
+                if (!mine.has<kK>(i)) continue;
+#pragma unroll 1
+                for (int half = 0; half < 2; half++) {
+                    const int t = k0 + mine.r + kStep * half, to = mine.at + half * (kStep * 128) + i * (kTile * 128), col = mine.col(i);
+                    const size_t from = head + (size_t)t * C3;
+                    copy8(sm.k[0] + to, xhi + from + C, col, D, t < T, vec);
+                    copy8(sm.k[1] + to, xlo + from + C, col, D, t < T, vec);
+                    copy8(sm.v[0] + to, xhi + from + 2 * C, col, D, t < T, vec);
+                    copy8(sm.v[1] + to, xlo + from + 2 * C, col, D, t < T, vec);
+                }
+            }
+        }
+        put_q(0);
+        put_g(0);
+
+        // dQ^T of this thread's head column and 16 queries of step n, from tensor memory on its way to dqkv.  Rows of dqkv
+        // that are not 16-byte aligned are added to from registers.
+        const int dq_col = kOne ? row % 64 : row;
+        auto take_dq = [&](int n) {
+            const int q0 = k0 + n * kStep + 16 * cq;
+            uint32_t r[16];
+            tmem_ld16(tmem + lane_addr + kColDQ + 16 * cq, r);
+            tmem_wait_ld();
+            if (dq_col >= D) return;
+            if (vec) {
+                float *dst = sm.out[n & (Smem::kOuts - 1)] + (kOne ? row / 64 * kStep + 16 * cq : 16 * (cq & 1)) * D + dq_col;
+#pragma unroll
+                for (int e = 0; e < 16; e++) dst[e * D] = __uint_as_float(r[e]) * scale;
+            } else {
+                float *dst = dqkv + head + (size_t)q0 * C3 + dq_col;
+#pragma unroll
+                for (int e = 0; e < 16; e++)
+                    if (q0 + e < T) atomicAdd(dst + e * C3, __uint_as_float(r[e]) * scale);
+            }
+        };
+        // the rows of sm.out are added to dqkv from row t of the sequence on (one thread)
+        auto send_dq = [&](int parity, int t) {
+#pragma unroll 1
+            for (int plane = 0; t < T && plane < (kOne ? 2 : 1); plane++)
+                tma_reduce_add_3d(sm.out[parity] + plane * kStep * D, &map_dq, h * D, t, b);
+            bulk_commit();
+        };
+
+        float dv[4 * kK], dk[4 * kK];
+#pragma unroll
+        for (int i = 0; i < 4 * kK; i++) dv[i] = dk[i] = 0.f;
+        const uint32_t t_s = tmem + lane_addr + kColS, t_dp = tmem + lane_addr + kColDP;
+        // eight queries (chunk c of this thread's row) of the three planes of dS^T
+        auto put_ds = [&](int c, const uint32_t *hi, const uint32_t *mid, const uint32_t *lo) {
+            uint8_t *to = sm.g + Smem::kDs + row * 128 + ((c ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4 *>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4 *>(to + kDsPlane) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+            *reinterpret_cast<uint4 *>(to + 2 * kDsPlane) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        };
+        for (int n = 0; n < nsteps; n++) {
+            const int q0 = k0 + n * kStep;
+            const bool more = n + 1 < nsteps;
+            await(&sm.stat_full[n & 1], (n >> 1) & 1, ctx, SITE24_STAT);
+            await(&sm.done_s, n & 1, ctx, SITE24_S);
+            const int first = k0 + row - (q0 + 16 * cq), end = T - (q0 + 16 * cq);  // of this thread's 16 queries
+            const bool edge = k0 + 32 * quarter + 31 > q0 + 16 * cq || end < 16;  // above the diagonal, or past the end
+            const float2 log2e = make_float2(-1.4426950408889634f, -1.4426950408889634f);
+            // P, while dP is being computed, and then dS, while dV is
+            float2 p[8];
+            uint32_t lo[8];  // its columns hold scores that are still to be read
+#pragma unroll
+            for (int piece = 0; piece < 16 / kPiece; piece++) {
+                const int c0 = 16 * cq + kPiece * piece;
+                constexpr int kPairs = kPiece / 2;
+                uint32_t s[kPiece], hi[kPairs], mid[kPairs];
+                tmem_load<kPiece>(t_s + c0, s);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < kPairs; e++) {
+                    const float2 l = mul2(*reinterpret_cast<const float2 *>(sm.stat[n & 1][0] + c0 + 2 * e), log2e);
+                    const float2 v = make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
+                    const float2 x = fma2(v, make_float2(scale_log2.lo, scale_log2.lo), fma2(v, make_float2(scale_log2.hi, scale_log2.hi), l));
+                    float2 y = make_float2(ex2f(x.x), ex2f(x.y));
+                    if (edge) {
+                        const int q = kPiece * piece + 2 * e;
+                        if (q < first || q >= end) y.x = 0.f;
+                        if (q + 1 < first || q + 1 >= end) y.y = 0.f;
+                    }
+                    p[kPairs * piece + e] = y;
+                    split3(y, hi[e], mid[e], lo[kPairs * piece + e]);
+                }
+                tmem_store<kPairs>(t_s + term_column(0, cq) + kPairs * piece, hi);
+                tmem_store<kPairs>(t_s + term_column(1, cq) + kPairs * piece, mid);
+            }
+            tmem_st8(t_s + term_column(2, cq), lo);
+            tmem_wait_st();
+            // The thread that sends dQ sees that the one whose place it takes has left sm.out before done_dv.
+            if (tid == 0) bulk_wait_read<Smem::kOuts - 1>();
+            warp_arrive(&sm.go_dv, lane);
+            await(&sm.done_dp, n & 1, ctx, SITE24_DP);
+#pragma unroll
+            for (int piece = 0; piece < 16 / kPiece; piece++) {
+                const int c0 = 16 * cq + kPiece * piece;
+                constexpr int kPairs = kPiece / 2;
+                uint32_t dp[kPiece], hi[kPairs], mid[kPairs];
+                tmem_load<kPiece>(t_dp + c0, dp);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < kPairs; e++) {
+                    const float2 d = *reinterpret_cast<const float2 *>(sm.stat[n & 1][1] + c0 + 2 * e);
+                    const float2 ds = mul2(p[kPairs * piece + e], make_float2(__uint_as_float(dp[2 * e]) - d.x, __uint_as_float(dp[2 * e + 1]) - d.y));
+                    split3(ds, hi[e], mid[e], lo[kPairs * piece + e]);
+                }
+                if (kOne) put_ds(2 * cq + piece, hi, mid, lo + 4 * piece);
+                tmem_store<kPairs>(t_dp + term_column(0, cq) + kPairs * piece, hi);
+                tmem_store<kPairs>(t_dp + term_column(1, cq) + kPairs * piece, mid);
+            }
+            tmem_st8(t_dp + term_column(2, cq), lo);
+            tmem_wait_st();
+            warp_arrive(&sm.go_dk, lane);
+            if (lane == 0) mbar_arrive(&sm.stat_free[n & 1]);
+
+            if (kOne && more) request_g(n + 1);
+            await(&sm.done_dv, n & 1, ctx, SITE24_DV);  // nothing reads dO any more
+            if (kOne) {
+                if (more) put_g(n + 1);
+            } else {
+                uint32_t w[3][8];
+#pragma unroll
+                for (int term = 0; term < 3; term++) tmem_ld8(t_dp + term_column(term, cq), w[term]);
+                tmem_wait_ld();
+                put_ds(2 * cq, w[0], w[1], w[2]);
+                put_ds(2 * cq + 1, w[0] + 4, w[1] + 4, w[2] + 4);
+                if (n > 0 && cq >= 2) take_dq(n - 1);
+                warp_arrive(&sm.go_dq, lane);
+                if (vec && n > 0 && cq >= 2) {
+                    named_sync(2, kWorkers / 2);
+                    if (tid == 256) send_dq(0, q0 - kStep / 2);
+                }
+            }
+            add_columns<kK>(dv, tmem + lane_addr + kColDV + 4 * kK * cq, 1.f);
+
+            await(&sm.done_dk, n & 1, ctx, SITE24_DK);  // nor Q
+            if (more) put_q(n + 1);
+            add_columns<kK>(dk, tmem + lane_addr + kColDK + 4 * kK * cq, 1.f);
+            if (!kOne && more) request_g(n + 1);
+            if (vec && !kOne && n > 0 && warp == 8) {
+                if (lane == 0) bulk_wait_read<0>();
+                __syncwarp();
+                named_arrive(3, kWorkers / 2 + 32);
+            }
+
+            await(&sm.done_dq, n & 1, ctx, SITE24_DQ);  // nor dS
+            if (kOne) {
+                take_dq(n);
+                if (vec) {
+                    fence_proxy_async_smem();
+                    named_sync(1, kWorkers);
+                    if (tid == 0) send_dq(n & (Smem::kOuts - 1), q0);
+                }
+            } else {
+                if (more) put_g(n + 1);
+                if (cq < 2) {
+                    if (vec && n > 0) named_sync(3, kWorkers / 2 + 32);  // the other half has left
+                    take_dq(n);
+                    if (vec) {
+                        fence_proxy_async_smem();
+                        named_sync(1, kWorkers / 2);
+                        if (tid == 0) send_dq(0, q0);
+                    }
+                }
+            }
+        }
+        if (!kOne) {
+            // the second half of the last dQ
+            if (vec && warp == 0) {
+                if (lane == 0) bulk_wait_read<0>();
+                __syncwarp();
+                named_arrive(4, kWorkers / 2 + 32);
+            }
+            if (cq >= 2) {
+                if (vec) named_sync(4, kWorkers / 2 + 32);  // its own: these warps may get here while the others still meet at 3
+                take_dq(nsteps - 1);
+                if (vec) {
+                    fence_proxy_async_smem();
+                    named_sync(2, kWorkers / 2);
+                    if (tid == 256) send_dq(0, k0 + nsteps * kStep - kStep / 2);
+                }
+            }
+        }
+        if (tid == 0 || tid == 256) bulk_wait_all();
+        const int t = k0 + row;
+        if (t < T) {
+            float *dst = dqkv + head + (size_t)t * C3;
+            store_columns<kK>(dst + C, 4 * kK * cq, D, dk, scale, vec);
+            store_columns<kK>(dst + 2 * C, 4 * kK * cq, D, dv, 1.f, vec);
+        }
+    }
+    if (sm.abort_flag) __nanosleep(50000);  // let copies and products that are still in flight end
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kWorkWarps) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+}  // namespace general
+
 }  // namespace
 
 static size_t bwd_smem_bytes() { return sizeof(BwdSmem); }
@@ -876,6 +1358,44 @@ cudaError_t launch_fast_backward_fp32(const CUtensorMap &map_x, const CUtensorMa
     return launch_after_previous(attn_bwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), bwd_smem_bytes(), s, map_x, map_x,
                                  map_dx, lse, nullptr, dqkv, Dout{dout, out, dhi, dlo, delta}, B, T, H, scale,
                                  scale * 1.4426950408889634f, sched, status);
+}
+
+cudaError_t attn24_bwd_set_attributes() {
+    for (int n = 1; n <= kAttn24MaxD / 16; n++) {
+        const cudaError_t e = attn24::with_groups(n, [](auto k) {
+            constexpr int kK = decltype(k)::value, kBytes = (int)sizeof(general::Bwd24Smem<kK>);
+            static_assert(kBytes <= 227 * 1024, "shared memory");
+            const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            const cudaError_t e = cudaFuncSetAttribute(general::attn24_bwd_kernel<kK, true>, a, kBytes);
+            return e != cudaSuccess ? e : cudaFuncSetAttribute(general::attn24_bwd_kernel<kK, false>, a, kBytes);
+        });
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse,
+                                   const float *delta, const float *dout, float *dqkv, int B, int T, int H, int D, int *status,
+                                   cudaStream_t s) {
+    CUtensorMap map_do = {}, map_dq = {};
+    const bool tma = D % 16 == 0;
+    int rc = 0;
+    if (tma) rc = attn24_rows_map(&map_do, dout, B, T, H * D, D, attn24::kStep);
+    if (rc != 0) return (cudaError_t)rc;
+    if (D % 4 == 0) {  // one head's rows of dq
+        const cuuint64_t width = (cuuint64_t)3 * H * D;
+        const cuuint64_t dims[3] = {width, (cuuint64_t)T, (cuuint64_t)B}, strides[2] = {width * 4, width * 4 * (cuuint64_t)T};
+        const cuuint32_t box[3] = {(cuuint32_t)D, (cuuint32_t)(D <= 64 ? attn24::kStep : attn24::kStep / 2), 1};
+        rc = encode_tiled(&map_dq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dqkv, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc != 0) return (cudaError_t)rc;
+    }
+    return attn24::with_groups((D + 15) / 16, [&](auto k) {
+        constexpr int kK = decltype(k)::value;
+        const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile)));
+        return launch_after_previous(tma ? general::attn24_bwd_kernel<kK, true> : general::attn24_bwd_kernel<kK, false>, grid,
+                                     dim3(attn24::kThreads), sizeof(general::Bwd24Smem<kK>), s, map_x, map_do, map_dq, xhi, xlo, lse,
+                                     delta, dout, dqkv, T, H, D, 1.0f / sqrtf((float)D), attn24::log2_scale(D), status);
+    });
 }
 
 }  // namespace attn

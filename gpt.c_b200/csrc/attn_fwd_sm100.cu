@@ -34,6 +34,7 @@
 // parts.  O accumulates in tensor memory across key tiles (the PV MMAs accumulate); the running
 // reference maximum only moves when a row maximum exceeds it by more than 2^8, and only then is
 // the accumulator rescaled in place.
+#include "attn24.cuh"
 #include "attn_internal.h"
 #include "tc05.cuh"
 
@@ -473,6 +474,249 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// General forward: any head size up to 128, fp32 operands as three bf16 terms (attn24.cuh).
+//
+// One CTA per (b, h, 128 queries), heaviest first; it walks the keys in steps of 64.  S = Q K^T with Q from tensor memory
+// and K from shared memory, P back to tensor memory as three terms, O_step = P V added to the running output in registers.
+// The 16 worker warps convert K of the next step and start its scores before they turn to the softmax of this one, and
+// convert V behind the softmax, so the tensor cores have the next scores and this step's P V ahead of them.
+//
+// What bounds it: the tensor cores, 12 bf16 passes over both products (3200 cycles per step at D = 128), with the
+// conversions, the softmax and the additions of the workers beneath them.
+// ---------------------------------------------------------------------------------------
+namespace general {
+
+using namespace attn24;
+
+template <int kK>  // head columns in groups of 16
+struct __align__(1024) Fwd24Smem {
+    static constexpr int kBlocks = (kK + 3) / 4, kPlane = kBlocks * kStep * 128;  // bytes of one term of a K or V tile
+    uint8_t k[3][kPlane], v[3][kPlane];  // before the first step: the three terms of Q, 128 rows each
+    float raw[2][kStep * 16 * kK];       // K, V of the next step as they come (rows of D); first the halves of Q
+    uint64_t raw_full[2], raw_free[2];
+    uint64_t go_s, go_pv, done_s, done_pv;
+    float part[2][4][kTile];  // [step parity][column quarter][row]: row maxima, at the end row sums
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+enum Site24 : int { SITE24_GO_S = 301, SITE24_GO_PV, SITE24_S, SITE24_PV, SITE24_RAW_FREE, SITE24_RAW_FULL, SITE24_SMEM_ALIGN };
+
+// kTma: D = 16 kK, and the copy engine fetches the rows; else the workers read them when they need them.
+template <int kK, bool kTma>
+__global__ void __launch_bounds__(attn24::kThreads, 1)
+attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ qkv, float *__restrict__ out,
+                  float *__restrict__ out_copy, float *__restrict__ lse, int T, int H, int D_arg, Scale scale_log2, int *status) {
+    using Smem = Fwd24Smem<kK>;
+    constexpr int kPlane = Smem::kPlane, kBlocks = Smem::kBlocks;
+    constexpr uint32_t kColS = 0, kColO = 192, kColQ = 192 + 16 * kK;  // S (96 columns) twice; P takes its place
+    constexpr uint32_t kCols = 192 + 40 * kK <= 256 ? 256 : 512;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    if ((smem_u32(smem_raw) & 1023u) != 0) {
+        if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE24_SMEM_ALIGN);
+        return;
+    }
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int D = kTma ? 16 * kK : D_arg;
+    const bool vec = kTma || D % 4 == 0;
+    WaitCtx ctx{&sm.abort_flag, status};
+    if (tid == 0) {
+        sm.abort_flag = 0;
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&sm.raw_full[i], 1);
+            mbar_init(&sm.raw_free[i], kWorkWarps);
+        }
+        mbar_init(&sm.go_s, kWorkWarps);
+        mbar_init(&sm.go_pv, kWorkWarps);
+        mbar_init(&sm.done_s, 1);
+        mbar_init(&sm.done_pv, 1);
+        fence_barrier_init();
+    }
+    if (warp == kWorkWarps) {
+        tmem_alloc_then_launch_dependents(&sm.tmem_base, kCols);
+    }
+    pdl_wait();
+    const int nq = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nq;
+    const int q0 = (nq - 1 - (int)blockIdx.x / nbh) * kTile;  // longest rows first
+    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
+    const int C = H * D, nsteps = (min(q0 + kTile, T) + kStep - 1) / kStep;
+    const size_t C3 = 3 * (size_t)C;
+    const float *head = qkv + (size_t)b * T * C3 + (size_t)h * D;
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
+
+    if (warp > kWorkWarps) {
+        // ------------------------------ producers: K, V (before the first step the halves of Q) ------------------------------
+        const int kv = warp - kWorkWarps - 1;
+        if (kTma && kv < 2 && lane == 0) {
+            for (int n = 0; n <= nsteps; n++) {
+                if (n > 0 && !await_thread(&sm.raw_free[kv], (n - 1) & 1, ctx, SITE24_RAW_FREE)) break;
+                mbar_expect_tx(&sm.raw_full[kv], kStep * 16 * kK * 4);
+                tma_load_4d(sm.raw[kv], &map_x, &sm.raw_full[kv], (n > 0 ? (kv + 1) * C : 0) + h * D,
+                            n > 0 ? (n - 1) * kStep : q0 + kv * kStep, b, 0);
+            }
+        }
+    } else if (warp == kWorkWarps) {
+        // ------------------------------ MMA issuer ------------------------------
+        constexpr uint32_t idesc_s = idesc_bf16_f32(kTile, kStep, 0, 0), idesc_o = idesc_bf16_f32(kTile, 16 * kK, 0, 1);
+        constexpr int kTermA[6] = {2, 1, 0, 1, 0, 0}, kTermB[6] = {0, 1, 2, 0, 1, 0};  // smallest first
+        const uint32_t leader = elect_leader();
+        const uint64_t kd = smem_desc_sw128(smem_u32(sm.k[0]), 16, 1024);
+        const uint64_t vd = smem_desc_sw128(smem_u32(sm.v[0]), kStep * 128, 1024);
+        auto issue_s = [&](int n) {
+            await(&sm.go_s, n & 1, ctx, SITE24_GO_S);
+#pragma unroll
+            for (int term = 0; term < 6; term++)
+#pragma unroll
+                for (int kk = 0; kk < kK; kk++)
+                    mma_ts_lead(leader, tmem + kColS + (n & 1) * 96, tmem + kColQ + 8 * kK * kTermA[term] + 8 * kk,
+                                desc_advance(kd, kTermB[term] * kPlane + (kk >> 2) * (kStep * 128) + (kk & 3) * 32), idesc_s,
+                                term > 0 || kk > 0 ? 1u : 0u);
+            tc_commit_lead(leader, &sm.done_s);
+        };
+        issue_s(0);
+        for (int n = 0; n < nsteps; n++) {
+            // S_n+1 goes where P_n-1 was, which P V of step n-1, earlier in the pipe, has read by then
+            if (n + 1 < nsteps) issue_s(n + 1);
+            await(&sm.go_pv, n & 1, ctx, SITE24_GO_PV);
+#pragma unroll
+            for (int term = 0; term < 6; term++)
+#pragma unroll
+                for (int kk = 0; kk < kStep / 16; kk++)
+                    mma_ts_lead(leader, tmem + kColO, tmem + kColS + (n & 1) * 96 + term_column(kTermA[term], kk),
+                                desc_advance(vd, kTermB[term] * kPlane + kk * 2048), idesc_o, term > 0 || kk > 0 ? 1u : 0u);
+            tc_commit_lead(leader, &sm.done_pv);
+        }
+    } else {
+        // ------------------------------ workers ------------------------------
+        const int quarter = warp & 3, cq = warp >> 2, row = 32 * quarter + lane;
+        const uint32_t lane_addr = (uint32_t)(quarter << 5) << 16;
+        const uint32_t t_o = tmem + lane_addr + kColO + 4 * kK * cq;
+        const Chunk mine(tid);
+        // This thread's values of a 64-row tile (rows from t0 on, the columns of one head at src) as three terms into the
+        // planes at `tile`; phase: how often the buffer has been filled before.
+        auto put = [&](uint8_t *tile, int plane, int block, int kv, const float *src, int t0, int phase) {
+            float f[kBlocks][8];
+            if (kTma) {
+                await(&sm.raw_full[kv], phase & 1, ctx, SITE24_RAW_FULL);
+#pragma unroll
+                for (int i = 0; i < kBlocks; i++)
+                    if (mine.has<kK>(i)) lds8(f[i], sm.raw[kv] + mine.r * D + mine.col(i), mine.c);
+                warp_arrive(&sm.raw_free[kv], lane);  // its fence holds the copy engine back until these values are in registers
+            } else {
+                const float *from = src + (size_t)(t0 + mine.r) * C3;
+#pragma unroll
+                for (int i = 0; i < kBlocks; i++)
+                    if (mine.has<kK>(i)) load8(f[i], from, mine.col(i), D, t0 + mine.r < T, vec);
+            }
+#pragma unroll
+            for (int i = 0; i < kBlocks; i++)
+                if (mine.has<kK>(i)) store_split3(tile, plane, mine.at + i * block, f[i]);
+        };
+        // Q: split like K and V, 128 rows where those will be, and from there into tensor memory
+        for (int half = 0; half < 2; half++)
+            put(sm.k[0] + half * (kStep * 128), 2 * kPlane, kTile * 128, half, head, q0 + half * kStep, 0);
+        named_sync(5, kWorkers);
+#pragma unroll
+        for (int i = 0; i < kK; i++) {
+            const int col = 4 * kK * cq + 4 * i;
+            const uint8_t *from = sm.k[0] + (col >> 6) * (kTile * 128) + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4) + (col & 4) * 2;
+            const uint32_t t_q = tmem + lane_addr + kColQ + 2 * kK * cq + 2 * i;
+#pragma unroll
+            for (int term = 0; term < 3; term++) {
+                const uint2 w = *reinterpret_cast<const uint2 *>(from + term * 2 * kPlane);
+                tmem_st2(t_q + term * 8 * kK, w.x, w.y);
+            }
+        }
+        tmem_wait_st();
+        named_sync(5, kWorkers);
+        put(sm.k[0], kPlane, kStep * 128, 0, head + C, 0, 1);
+        warp_arrive(&sm.go_s, lane);
+
+        float o[4 * kK], m = -INFINITY, l = 0.f, alpha_before = 1.f;
+#pragma unroll
+        for (int i = 0; i < 4 * kK; i++) o[i] = 0.f;
+        for (int n = 0; n < nsteps; n++) {
+            await(&sm.done_s, n & 1, ctx, SITE24_S);
+            if (n + 1 < nsteps) {
+                put(sm.k[0], kPlane, kStep * 128, 0, head + C, (n + 1) * kStep, n + 2);
+                warp_arrive(&sm.go_s, lane);
+            }
+            const uint32_t t_s = tmem + lane_addr + kColS + (n & 1) * 96;
+            uint32_t s[16];
+            tmem_ld16(t_s + 16 * cq, s);
+            tmem_wait_ld();
+            float mx = -INFINITY;
+            const int key0 = n * kStep + 16 * cq - q0;  // of this thread's columns, relative to the first query row
+            if (key0 + 15 > 32 * quarter) {
+#pragma unroll
+                for (int e = 0; e < 16; e++)
+                    if (key0 + e > row) s[e] = 0xff800000u;  // -inf
+            }
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) mx = max3(mx, __uint_as_float(s[e]), __uint_as_float(s[e + 1]));
+            sm.part[n & 1][cq][row] = mx;
+            named_sync(1 + quarter, 128);  // the four warps of these rows
+            mx = fmaxf(fmaxf(sm.part[n & 1][0][row], sm.part[n & 1][1][row]), fmaxf(sm.part[n & 1][2][row], sm.part[n & 1][3][row]));
+            mx = fmaxf(m, mx * scale_log2.hi);
+            const bool none = mx == -INFINITY;  // nothing but -inf so far
+            const float alpha = none ? 1.f : ex2f(m - mx);
+            m = mx;
+            const float2 by = make_float2(scale_log2.hi, scale_log2.hi), rest = make_float2(scale_log2.lo, scale_log2.lo);
+            const float2 minus = make_float2(none ? 0.f : -mx, none ? 0.f : -mx);
+            float2 sum = make_float2(0.f, 0.f);
+            uint32_t hi[8], mid[8], lo[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float2 v = make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
+                const float2 x = fma2(v, rest, fma2(v, by, minus));
+                const float2 p = make_float2(ex2f(x.x), ex2f(x.y));
+                sum = add2(sum, p);
+                split3(p, hi[e], mid[e], lo[e]);
+            }
+            l = l * alpha + (sum.x + sum.y);
+            tmem_st8(t_s + term_column(0, cq), hi);
+            tmem_st8(t_s + term_column(1, cq), mid);
+            tmem_st8(t_s + term_column(2, cq), lo);
+            tmem_wait_st();
+            if (n > 0) {
+                await(&sm.done_pv, (n - 1) & 1, ctx, SITE24_PV);
+                add_columns<kK>(o, t_o, alpha_before);
+            }
+            alpha_before = alpha;
+            put(sm.v[0], kPlane, kStep * 128, 1, head + 2 * C, n * kStep, n + 1);
+            warp_arrive(&sm.go_pv, lane);
+        }
+        sm.part[nsteps & 1][cq][row] = l;
+        named_sync(1 + quarter, 128);
+        l = (sm.part[nsteps & 1][0][row] + sm.part[nsteps & 1][1][row]) + (sm.part[nsteps & 1][2][row] + sm.part[nsteps & 1][3][row]);
+        await(&sm.done_pv, (nsteps - 1) & 1, ctx, SITE24_PV);
+        add_columns<kK>(o, t_o, alpha_before);
+        const int t = q0 + row;
+        if (t < T) {
+            const float inv = 1.0f / l;
+            const size_t at = ((size_t)b * T + t) * C + (size_t)h * D;
+            store_columns<kK>(out + at, 4 * kK * cq, D, o, inv, vec);
+            if (out_copy) store_columns<kK>(out_copy + at, 4 * kK * cq, D, o, inv, vec);
+            // m ln 2 + ln l, ln 2 in two parts
+            if (cq == 0) lse[(size_t)bh * T + t] = fmaf(m, 0.693147182464599609375f, fmaf(m, -1.904654299957768e-9f, logf(l)));
+        }
+    }
+    if (sm.abort_flag) __nanosleep(50000);  // let copies and products that are still in flight end
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kWorkWarps) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, kCols);
+    }
+}
+
+}  // namespace general
+
 }  // namespace
 
 cudaError_t fast_fwd_set_attributes() {
@@ -495,6 +739,37 @@ cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_b
     const CUtensorMap none = {};
     return launch_after_previous(attn_fwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), sizeof(FwdSmem), s, none, qkv, hi,
                                  lo, out, out_copy, lse, B, T, H, kScaleLog2, status);
+}
+
+cudaError_t attn24_fwd_set_attributes() {
+    for (int n = 1; n <= kAttn24MaxD / 16; n++) {
+        const cudaError_t e = attn24::with_groups(n, [](auto k) {
+            constexpr int kK = decltype(k)::value, kBytes = (int)sizeof(general::Fwd24Smem<kK>);
+            static_assert(kBytes <= 227 * 1024, "shared memory");
+            const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            const cudaError_t e = cudaFuncSetAttribute(general::attn24_fwd_kernel<kK, true>, a, kBytes);
+            return e != cudaSuccess ? e : cudaFuncSetAttribute(general::attn24_fwd_kernel<kK, false>, a, kBytes);
+        });
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_attn24_forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H, int D, int *status,
+                                  cudaStream_t s) {
+    CUtensorMap map_x = {};
+    const bool tma = D % 16 == 0;
+    if (tma) {
+        const int rc = attn24_rows_map(&map_x, qkv, B, T, 3 * H * D, D, attn24::kStep);
+        if (rc != 0) return (cudaError_t)rc;
+    }
+    return attn24::with_groups((D + 15) / 16, [&](auto k) {
+        constexpr int kK = decltype(k)::value;
+        const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile)));
+        return launch_after_previous(tma ? general::attn24_fwd_kernel<kK, true> : general::attn24_fwd_kernel<kK, false>, grid,
+                                     dim3(attn24::kThreads), sizeof(general::Fwd24Smem<kK>), s, map_x, qkv, out, out_copy, lse, T, H,
+                                     D, attn24::log2_scale(D), status);
+    });
 }
 
 }  // namespace attn

@@ -1,10 +1,8 @@
 // General-shape causal attention kernels (fp32 SIMT, tiled) and the elementwise
 // preparation kernels shared with the tensor-core path.
 //
-// These kernels accept any head size D <= 256 and any T <= 8192.  They are the correctness
-// anchor on the GPU and serve the shapes the tcgen05 kernels do not take (D != 64, e.g. the
-// D = 3 case of the reference's tests/test_self_attention.py).  They replace the same
-// reference code as the fast path: kernels/src/cuda/Attention.cu:170-324 of gpt.c.
+// These kernels serve the head sizes the tcgen05 kernels do not take, 129 to 256, and any T <= 8192.  They replace
+// the same reference code as those: kernels/src/cuda/Attention.cu:170-324 of gpt.c.
 #include "attn_internal.h"
 #include "tc05.cuh"
 
@@ -199,7 +197,7 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
 }
 
 // ---------------------------------------------------------------------------------------
-// General kernels: causal attention in fp32 for any head size, tiled over queries and keys.
+// General kernels: causal attention in fp32 for head sizes above 128, tiled over queries and keys.
 //
 // What bounds them is the fp32 pipe, so they are built around register tiles: a thread owns kR rows and
 // several columns of every product and reads its operands from shared memory in 16-byte words, 16 packed
@@ -210,11 +208,8 @@ __global__ void __launch_bounds__(256) bwd_prepare64_kernel(const float *__restr
 //     accumulator hold the sums over even and odd head columns, added once at the end;
 //   output products (contraction over keys or queries): they hold two neighbouring head columns, the other
 //     operand is broadcast into both halves.
-// kNI = head columns in blocks of 32 (the output tile's width), so D = 80 does 96 columns of output work; the
+// kNI = head columns in blocks of 32 (the output tile's width), so D = 140 does 160 columns of output work; the
 // score products run over exactly the 4-column words that hold data.
-// The kernels they replace (one warp per row, K and V read again from L2 for every row) took 83 ms for forward
-// and backward of B=4 T=1024 H=6 D=128; these take 0.68 ms (23 GFLOP of fp32 products, a third of the fp32 rate
-// of 148 SMs).
 // ---------------------------------------------------------------------------------------
 typedef unsigned long long f32x2;  // two floats of a packed instruction
 
@@ -357,14 +352,9 @@ __device__ __forceinline__ void store_cols(float *row, int col, int D, float4 v)
 
 // ---------------------------------------------------------------------------------------
 // forward: one block per (b, h, 64 queries), key tiles of 8 kC, online softmax.  Two groups of four warps take the
-// key tiles in turns, each with its own K, V and P tiles (168 KB of shared memory in all at D = 128), and the two
-// partial results are merged at the end: a block then has its SM to itself and the longest-first order balances the
-// SMs.  (With one group per block and two blocks per SM, the SMs were busy for 71 % of the launch on average, because
-// the long blocks that start together share an SM.)  B=4 T=1024 H=6 D=128 233 -> 192 us, B=2 T=2048 H=4 D=80
-// 395 -> 183 us.  Up to 64 head columns two blocks still fit, with 128 registers per thread and up to 144 bytes of
-// them spilled.  That pays when there are more blocks than SMs: B=4 T=1024 H=12 D=64 202 us against 212 with one block
-// and no spills, D=16 104 against 125, B=8 T=512 H=16 D=32 92 against 109.  With one block or less per SM it costs:
-// B=1 T=2048 H=4 D=64 219 against 143, B=8 T=128 H=12 D=64 22 against 17.
+// key tiles in turns, each with its own K, V and P tiles, and the two partial results are merged at the end: a block
+// then has its SM to itself and the longest-first order balances the SMs.  (With one group per block and two blocks per
+// SM, the SMs were busy for 71 % of the launch on average, because the long blocks that start together share an SM.)
 // ---------------------------------------------------------------------------------------
 constexpr int kFwdGroup = 128, kFwdThreads = 2 * kFwdGroup, kFwdRows = 64;
 
@@ -381,7 +371,7 @@ struct FwdTile {
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
 template <int kNI, int kC, bool kVec>
-__global__ void __launch_bounds__(kFwdThreads, kNI <= 2 ? 2 : 1) generic_fwd_kernel(const float *__restrict__ qkv, float *__restrict__ out,
+__global__ void __launch_bounds__(kFwdThreads) generic_fwd_kernel(const float *__restrict__ qkv, float *__restrict__ out,
                                                                   float *__restrict__ out_copy, float *__restrict__ lse,
                                                                   int T, int H, int D, float scale) {
     using S = FwdTile<kNI, kC>;
@@ -533,7 +523,7 @@ __global__ void __launch_bounds__(kFwdThreads, kNI <= 2 ? 2 : 1) generic_fwd_ker
 
 // ---------------------------------------------------------------------------------------
 // backward: one block per (b, h, key tile of 8 kC keys), query tiles from the diagonal on.  K, V, the query tile's Q
-// and dO, P and dS sit in shared memory (171 KB at D = 128, so one block of 8 warps per SM).  Two groups of four
+// and dO, P and dS sit in shared memory (one block of 8 warps per SM).  Two groups of four
 // warps share the five products: one computes S and then dV, the other dP, dS and then dK; each keeps its gradient
 // tile in registers over all query tiles; dQ of the query tile is shared out by blocks of 32 head columns and added
 // to memory with fp32 atomics (a second kernel that owns the queries would do S and dP again, seven products
@@ -554,13 +544,8 @@ __device__ __forceinline__ void key_gradient(f32x2 (&g)[kR][2 * kNI], const floa
 #pragma unroll 2
     for (int q = 0; q < kRows; q++) {
         float pk[kR];
-        if (kR == 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(p + q * kPPitch);
-            pk[0] = v.x, pk[1] = v.y, pk[2 % kR] = v.z, pk[3 % kR] = v.w;
-        } else {
-            const float2 v = *reinterpret_cast<const float2 *>(p + q * kPPitch);
-            pk[0] = v.x, pk[1] = v.y;
-        }
+        const float2 v = *reinterpret_cast<const float2 *>(p + q * kPPitch);
+        pk[0] = v.x, pk[1] = v.y;
         ulonglong2 xv[kNI];
 #pragma unroll
         for (int i = 0; i < kNI; i++) xv[i] = lds_x4(x + q * kPitch + 32 * i);
@@ -775,8 +760,7 @@ __global__ void __launch_bounds__(kBwdThreads) generic_bwd_kernel(const __nv_bfl
 
 template <int kNI>
 struct Generic {
-    // key tiles of 64; head sizes above 128 take 32, whose wider rows need as much shared memory and registers
-    static constexpr int kC = kNI <= 4 ? 8 : 4;
+    static constexpr int kC = 4;  // key tiles of 32: 64 would not fit with rows this wide
     using F = FwdTile<kNI, kC>;
     using G = BwdTile<kNI, kC>;
 
@@ -806,14 +790,10 @@ struct Generic {
 
 }  // namespace
 
-// f(Generic<n>{}) for n = 1 .. 8, the number of 32-column blocks of the head size
+// f(Generic<n>{}) for n = 5 .. 8, the number of 32-column blocks of the head size
 template <class Fn>
 static cudaError_t with_blocks(int n, Fn f) {
     switch (n) {
-        case 1: return f(Generic<1>{});
-        case 2: return f(Generic<2>{});
-        case 3: return f(Generic<3>{});
-        case 4: return f(Generic<4>{});
         case 5: return f(Generic<5>{});
         case 6: return f(Generic<6>{});
         case 7: return f(Generic<7>{});
@@ -822,7 +802,7 @@ static cudaError_t with_blocks(int n, Fn f) {
 }
 
 cudaError_t generic_set_attributes() {
-    for (int n = 1; n <= kGenericMaxD / 32; n++) {
+    for (int n = kAttn24MaxD / 32 + 1; n <= kGenericMaxD / 32; n++) {
         const cudaError_t e = with_blocks(n, [](auto g) { return decltype(g)::set_attributes(); });
         if (e != cudaSuccess) return e;
     }

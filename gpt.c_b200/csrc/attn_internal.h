@@ -24,6 +24,7 @@ inline int sm_count() {
 }
 
 constexpr int kShortT = 128;  // one query and key tile: the kernels that read the fp32 tensors themselves
+constexpr int kAttn24MaxD = 128;  // general kernels on the tensor cores; above, fp32 arithmetic
 constexpr int kGenericMaxD = 256;
 constexpr int kGenericMaxT = 8192;
 
@@ -41,13 +42,24 @@ cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, s
 cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta, __nv_bfloat16 *dhi,
                                __nv_bfloat16 *dlo, float *dq_zero, int *sched, int B, int T, int H, int D, cudaStream_t s);
 
-// General-shape SIMT kernels (any D <= kGenericMaxD, T <= kGenericMaxT).
+// General-shape SIMT kernels (kAttn24MaxD < D <= kGenericMaxD, T <= kGenericMaxT).
 cudaError_t generic_set_attributes();
 cudaError_t launch_generic_forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H,
                                    int D, cudaStream_t s);
 cudaError_t launch_generic_backward(const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse,
                                     const float *delta, const float *dout, float *dqkv, int B, int T, int H, int D,
                                     cudaStream_t s);
+
+// The general kernels on the tensor cores (D <= kAttn24MaxD, T <= kGenericMaxT), fp32 operands as three bf16 terms.
+// fp32 [B, T, W] as a 4-D map {W, T, B, 1} with boxes of D columns by `rows`, not swizzled.
+int attn24_rows_map(CUtensorMap *map, const void *base, int B, int T, int W, int D, int rows);
+cudaError_t attn24_fwd_set_attributes();
+cudaError_t attn24_bwd_set_attributes();
+cudaError_t launch_attn24_forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H, int D, int *status,
+                                  cudaStream_t s);
+// map_x: see launch_fast_backward below
+cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse, const float *delta,
+                                   const float *dout, float *dqkv, int B, int T, int H, int D, int *status, cudaStream_t s);
 
 // Tensor-core (tcgen05) kernels, D == 64.  The tensor maps cover the bf16 hi/lo planes:
 //   map_x : dims {3C, T, B, 2 planes}, box {64, 128, 1, 1}, 128-byte swizzle

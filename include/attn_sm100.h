@@ -42,7 +42,8 @@
  *
  * Precision: operands are split into two bf16 terms (x ~ hi + lo, 16 significant bits) and each
  * product is evaluated as hi*hi + hi*lo + lo*hi on the tensor cores with fp32 accumulation;
- * softmax statistics are fp32.  Head sizes other than 64 take a general fp32 SIMT kernel.
+ * softmax statistics are fp32.  Head sizes other than 64 take general kernels with fp32 operands (the
+ * backward reads q, k, v as the two saved planes).
  */
 #ifndef ATTN_SM100_H
 #define ATTN_SM100_H
@@ -63,7 +64,7 @@ extern "C" {
 #define ATTN_ERR_STATIC_CAPACITY (-7) /* attn_sm100_forward_static: the problem needs more than ATTN_STATIC_SCRATCH_BYTES */
 
 /* flags */
-#define ATTN_FLAG_FORCE_GENERIC 1 /* use the general SIMT kernels even when the tensor-core path applies */
+#define ATTN_FLAG_FORCE_GENERIC 1 /* use the general kernels even when those for D = 64 apply */
 /* forward and backward each enqueue a preparation kernel (the bf16 hi/lo split of qkv; the split
  * of dout with rowsum(dout*out) and the zero-fill of dq) followed by the core attention kernel.
  * These two flags enqueue only one of the two stages, e.g. to time them separately or to reuse a

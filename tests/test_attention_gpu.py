@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
 TOL_OUT, TOL_DX = 2e-3, 5e-3
 EXPECT_OUT, EXPECT_DX = 2e-4, 5e-4
-GENERIC_TOL = 1e-4  # fp32 SIMT kernels (backward reads the 16-bit hi+lo copy of qkv)
+GENERIC_TOL = 1e-4  # fp32 operands (backward reads the 16-bit hi+lo copy of qkv)
 
 
 @pytest.fixture(scope="module")
@@ -48,7 +48,7 @@ def seeded(seed, B, T, H, D):
 
 
 # ---------------------------------------------------------------------------------------------
-# general SIMT kernels
+# general kernels (tensor cores up to D = 128, fp32 arithmetic above)
 # ---------------------------------------------------------------------------------------------
 def test_generic_reference_own_test_case(pkg, gpu):
     z = np.load(os.path.join(GOLDEN, "ref_selfattn_case.npz"))
@@ -89,6 +89,34 @@ def test_generic_tile_edges(pkg, gpu, oracle, T, D):
     assert np.abs(out - ref_out).max() < GENERIC_TOL
     assert np.abs(lse - ref_lse).max() < GENERIC_TOL
     assert np.abs(dx - oracle.backward(x, g, 2)).max() < GENERIC_TOL
+
+
+@pytest.mark.parametrize("T,D", [(1, 16), (64, 48), (65, 64), (127, 80), (128, 96), (129, 112), (193, 128), (256, 32), (257, 96),
+                                 (2, 3), (64, 20), (129, 40), (191, 100), (320, 126)])
+def test_general_tensor_core_kernels_are_fp32_and_repeatable(pkg, gpu, oracle, T, D):
+    """Steps of 64 keys or queries, tiles of 128, head columns in groups of 16 and blocks of 64, rows fetched by the copy
+    engine (D a multiple of 16) or by the threads (a multiple of 4, and others).
+
+    Operands of 24 bits: a relative error of 2^-21 in the 2-norm leaves eight roundings of 2^-24, above all those of
+    exponents of up to eight and of exp2; operands of 16 bits give 4e-6.  The backward reads q, k, v with 16 bits: each of
+    three factors off by up to 2^-17.  What is not added up in memory is the same in every call."""
+    torch = gpu
+    x, g = seeded(29 + T + D, 3, T, 2, D)
+    out, lse, dx = run_cuda(pkg, gpu, x, g, 2, flags=pkg.FLAG_FORCE_GENERIC)
+    ref_out, ref_lse = oracle.forward(x, 2, want_lse=True)
+    ref_dx = oracle.backward(x, g, 2)
+    assert np.linalg.norm(out - ref_out) < 2.0 ** -21 * np.linalg.norm(ref_out)
+    assert np.linalg.norm(lse - ref_lse) < 2.0 ** -21 * max(np.linalg.norm(ref_lse), 1.0)
+    assert np.linalg.norm(dx - ref_dx) < 3 * 2.0 ** -17 * np.linalg.norm(ref_dx)
+    xd, gd = torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda()
+    flush = torch.empty(48 << 20, device="cuda")
+    for i in range(20):
+        if i % 2:
+            flush.fill_(float(i))  # the next call's first loads come from memory
+        o, ctx = pkg.forward(xd, 2, flags=pkg.FLAG_FORCE_GENERIC)
+        d = pkg.backward(ctx, gd)
+        assert np.array_equal(o.cpu().numpy(), out) and np.array_equal(ctx.lse.cpu().numpy().reshape(lse.shape), lse)
+        assert np.array_equal(d.cpu().numpy()[..., 2 * D:], dx[..., 2 * D:])
 
 
 # ---------------------------------------------------------------------------------------------
