@@ -57,7 +57,7 @@ int encode_planes(CUtensorMap *map, const void *base, int B, int T, int W, size_
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-// fp32 [B, T, W] tensor as a 3-D map {W, T, B}, box {32, 128, 1}: the output side of the backward kernel.
+// fp32 [B, T, W] tensor as a 3-D map {W, T, B}, box {32, 128, 1}: the output side of the tensor-core kernels.
 int encode_rows_f32(CUtensorMap *map, const void *base, int B, int T, int W) {
     const cuuint64_t dims[3] = {(cuuint64_t)W, (cuuint64_t)T, (cuuint64_t)B};
     const cuuint64_t strides[2] = {(cuuint64_t)W * 4, (cuuint64_t)W * 4 * (cuuint64_t)T};
@@ -206,11 +206,16 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
     __nv_bfloat16 *hi = static_cast<__nv_bfloat16 *>(saved);
     __nv_bfloat16 *lo = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(saved) + plane);
     cudaError_t e = cudaSuccess;
+    CUtensorMap map_o, map_copy;  // where the tensor-core kernels' result goes
+    if (fast && !(flags & ATTN_FLAG_PREPARE_ONLY)) {
+        if ((rc = encode_rows_f32(&map_o, out, B, T, H * D)) != 0) return rc;
+        if (out_copy && (rc = encode_rows_f32(&map_copy, out_copy, B, T, H * D)) != 0) return rc;
+    }
     // Both stages in one kernel for sequences of one key step and no more of them than SMs (6.7 -> 4.6 us for one of 40
     // tokens).  Beyond that the split kernel, which spreads the conversion over the whole GPU and overlaps its end with
     // the set-up of the next, is faster: B=8 T=128 H=12 9.5 us in two kernels, 14 us in one.
     if (fast && T <= attn::kShortT / 2 && B * H <= ds->num_sms && !(flags & (ATTN_FLAG_CORE_ONLY | ATTN_FLAG_PREPARE_ONLY)))
-        return (int)attn::launch_fast_forward_fp32(qkv, hi, lo, out, out_copy, lse, B, T, H, ds->status, s);
+        return (int)attn::launch_fast_forward_fp32(qkv, hi, lo, map_o, out_copy ? &map_copy : nullptr, lse, B, T, H, ds->status, s);
     if (!(flags & ATTN_FLAG_CORE_ONLY)) {
         e = attn::launch_split(qkv, hi, lo, n, s);
         if (e != cudaSuccess) return (int)e;
@@ -221,7 +226,7 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
         CUtensorMap map_x;
         rc = encode_planes(&map_x, saved, B, T, 3 * H * D, plane, 64);
         if (rc != 0) return rc;
-        e = attn::launch_fast_forward(map_x, out, out_copy, lse, B, T, H, ds->status, s);
+        e = attn::launch_fast_forward(map_x, map_o, out_copy ? &map_copy : nullptr, lse, B, T, H, ds->status, s);
     } else {
         e = use_attn24(D) ? attn::launch_attn24_forward(qkv, out, out_copy, lse, B, T, H, D, ds->status, s)
                           : attn::launch_generic_forward(qkv, out, out_copy, lse, B, T, H, D, s);

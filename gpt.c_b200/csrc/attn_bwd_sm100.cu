@@ -234,10 +234,14 @@ __device__ __forceinline__ void take_dout(BwdSmem &sm, const Dout &d, int b, int
     const int tid = (int)threadIdx.x - 128, r = tid >> 2, c0 = 16 * (tid & 3);
     float4 g[4], o[4];
     const size_t at = ((size_t)b * T + r) * H * kD + h * kD + c0;
+    const bool wide = aligned32(d.dout) && aligned32(d.out);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        g[i] = r < T ? __ldcs(reinterpret_cast<const float4 *>(d.dout + at) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        o[i] = r < T ? __ldcs(reinterpret_cast<const float4 *>(d.out + at) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < 4; i += 2) {
+        g[i] = g[i + 1] = o[i] = o[i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < T) {
+            load_f32x8(g[i], g[i + 1], d.dout + at + 4 * i, wide);
+            load_f32x8(o[i], o[i + 1], d.out + at + 4 * i, wide);
+        }
     }
     float sum = 0.f;
 #pragma unroll
@@ -245,30 +249,32 @@ __device__ __forceinline__ void take_dout(BwdSmem &sm, const Dout &d, int b, int
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     uint8_t *th = sm.in[r >> 6][2] + (r & 63) * 128, *tl = sm.in[r >> 6][3] + (r & 63) * 128;
+    uint4 vh[2], vl[2];
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-        uint4 vh, vl;
-        split_bf16x2(g[2 * i].x, g[2 * i].y, vh.x, vl.x);
-        split_bf16x2(g[2 * i].z, g[2 * i].w, vh.y, vl.y);
-        split_bf16x2(g[2 * i + 1].x, g[2 * i + 1].y, vh.z, vl.z);
-        split_bf16x2(g[2 * i + 1].z, g[2 * i + 1].w, vh.w, vl.w);
+        split_bf16x2(g[2 * i].x, g[2 * i].y, vh[i].x, vl[i].x);
+        split_bf16x2(g[2 * i].z, g[2 * i].w, vh[i].y, vl[i].y);
+        split_bf16x2(g[2 * i + 1].x, g[2 * i + 1].y, vh[i].z, vl[i].z);
+        split_bf16x2(g[2 * i + 1].z, g[2 * i + 1].w, vh[i].w, vl[i].w);
         const int chunk = ((2 * (tid & 3) + i) ^ (r & 7)) << 4;
-        *reinterpret_cast<uint4 *>(th + chunk) = vh;
-        *reinterpret_cast<uint4 *>(tl + chunk) = vl;
-        if (r < T) {
-            *reinterpret_cast<uint4 *>(d.hi + at + 8 * i) = vh;
-            *reinterpret_cast<uint4 *>(d.lo + at + 8 * i) = vl;
-        }
+        *reinterpret_cast<uint4 *>(th + chunk) = vh[i];
+        *reinterpret_cast<uint4 *>(tl + chunk) = vl[i];
     }
-    if ((tid & 3) == 0) {
-        sm.delta[0][r] = -sum;
-        if (r < T) d.delta[((size_t)b * H + h) * T + r] = sum;
-    }
+    if ((tid & 3) == 0) sm.delta[0][r] = -sum;
     fence_proxy_async_smem();
     __syncwarp();
     if ((threadIdx.x & 31) == 0) {
         mbar_arrive(&sm.in_full[r >> 6]);  // a warp's 8 rows are in one half
         mbar_arrive(&sm.stats_full[0]);
+    }
+    // what only a later call may want goes out behind that: the fence would wait for it
+    if (r < T) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            *reinterpret_cast<uint4 *>(d.hi + at + 8 * i) = vh[i];
+            *reinterpret_cast<uint4 *>(d.lo + at + 8 * i) = vl[i];
+        }
+        if ((tid & 3) == 0) d.delta[((size_t)b * H + h) * T + r] = sum;
     }
 }
 
@@ -291,8 +297,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const int nt = (T + kTile - 1) / kTile;
     const int C = H * kD;
 
+    // One tile in all (kFp32): a sequence of at most 64 tokens has no second half (T = 40: 0.9 us of a kernel of 6).
+    const int halves = kFp32 && T <= kHalf ? 1 : 2;
+
     WaitCtx ctx{&sm.abort_flag, status};
 
+    if (warp == kGradWarp && lane == 0) {
+        tma_prefetch_desc(&map_x);
+        if (!kFp32) tma_prefetch_desc(&map_do);
+        tma_prefetch_desc(&map_dx);
+    }
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         mbar_init(&sm.kv_full, 1);
@@ -340,8 +354,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     } else if (warp == 0) {
         // ------------------------------ TMA producer (boxes of 64 rows) ------------------------------
         if (lane == 0) {
-            tma_prefetch_desc(&map_x);
-            tma_prefetch_desc(&map_do);
             // Half tile number g of the whole launch goes to ring slot g % 3; the slot is free again once
             // the dV / dK products that read its previous content have completed.
             uint32_t g = 0;
@@ -377,7 +389,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             load_kv(w, sm.v, 2 * C + (w.bh % H) * kD);
             int pre = 0;  // half tiles of the current item already requested
             for (uint32_t item = 0; has && ok; item++) {
-                for (int t = pre; ok && t < 2 * w.niter; t++) load_half(w, t);
+                for (int t = pre; ok && t < halves * w.niter; t++) load_half(w, t);
                 // the next item: its entry is the (item + 1)-th post, made while the CTA worked on the item
                 // before this one
                 const bool has_next = feed.more;
@@ -428,7 +440,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (!ok) break;
             if (item > 0) feed.read(sm, item);
             w = decode_item(feed.p, BH, nt);
-            for (int t = 0; ok && t < 2 * w.niter; t++, g++) {
+            for (int t = 0; ok && t < halves * w.niter; t++, g++) {
                 const int hf = t & 1;
                 const uint32_t slot = g % kSlots;
                 if (g >= 2) ok = mbar_wait_warp(&sm.in_empty[(g - 2) % kSlots], ((g - 2) / kSlots) & 1, ctx, SITE_IN_EMPTY);
@@ -468,7 +480,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     }
                 }
                 tc_commit_lead(leader, &sm.st_full[hf]);
-                if (t == 2 * w.niter - 1) tc_commit_lead(leader, &sm.v_free);
+                if (t == halves * w.niter - 1) tc_commit_lead(leader, &sm.v_free);
             }
             if (!feed.more) break;
         }
@@ -481,7 +493,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         // reader.  (2) Staged dQ tiles are added into dqkv (several key tiles contribute to one query
         // tile), the dK / dV tiles of a finished item are plain stores; rows past the end of the sequence
         // are dropped by the copy engine.
-        if (lane == 0) tma_prefetch_desc(&map_dx);
         // The query tiles of this CTA's items, in processing order.  This warp hands the items out (below)
         // and reads their numbers from q_raw, which it has written itself.
         const int nitems = BH * nt, G = (int)gridDim.x;
@@ -714,19 +725,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     flush_dq();
                 }
                 // half B: queries 64..127
-                if (!mbar_wait_warp(&sm.st_full[1], n & 1, ctx, SITE_ST_FULL)) { ok = false; break; }
-                tc_fence_after_sync();
-                compute_run(sm, t_st + kHalf, t_dpt + kHalf, lb, kHalf + 16 * cq, row, diag, sc2, dh_b, dl_b);
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive(&sm.pds_full[1]);  // dV / dK of half B may start
+                if (halves == 2) {
+                    if (!mbar_wait_warp(&sm.st_full[1], n & 1, ctx, SITE_ST_FULL)) { ok = false; break; }
+                    tc_fence_after_sync();
+                    compute_run(sm, t_st + kHalf, t_dpt + kHalf, lb, kHalf + 16 * cq, row, diag, sc2, dh_b, dl_b);
+                    tmem_wait_st();
+                    tc_fence_before_sync();
+                    mbar_arrive(&sm.pds_full[1]);  // dV / dK of half B may start
+                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.stats_free[lb]);  // this warp has read the tile's statistics
                 // the staged dQ tile of the previous query tile (of this item or the one before) must have left
                 // shared memory
                 if (n >= 1 && !mbar_wait_warp(&sm.out_free, (n - 1) & 1, ctx, SITE_OUT_FREE)) { ok = false; break; }
                 store_ds(sm.ds[0][0], sm.ds[1][0], row, cq, dh_a, dl_a);
-                store_ds(sm.ds[0][1], sm.ds[1][1], row, cq, dh_b, dl_b);
+                if (halves == 2) store_ds(sm.ds[0][1], sm.ds[1][1], row, cq, dh_b, dl_b);
                 fence_proxy_async_smem();
                 mbar_arrive(&sm.ds_full);  // dQ may start
             }
@@ -773,7 +786,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (item > 0) feed.read(sm, item);
             w = decode_item(feed.p, BH, nt);
             for (int m = 0; ok && m < w.niter; m++, n++) {
-                for (int hf = 0; hf < 2; hf++, g++) {
+                for (int hf = 0; hf < halves; hf++, g++) {
                     if (!mbar_wait_warp(&sm.pds_full[hf], n & 1, ctx, SITE_PDS_FULL)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t slot = g % kSlots;
@@ -805,7 +818,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                         }
                     }
                     tc_commit_lead(leader, &sm.in_empty[slot]);
-                    if (m == w.niter - 1 && hf == 1) tc_commit_lead(leader, &sm.grads_done);
+                    if (m == w.niter - 1 && hf == halves - 1) tc_commit_lead(leader, &sm.grads_done);
                 }
                 if (!ok) break;
                 // dQ_i = dS K_j over all 128 keys
@@ -940,6 +953,13 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     if (warp == kWorkWarps) {
         tmem_alloc_then_launch_dependents(&sm.tmem_base, 512);
+    }
+    if (warp == kWorkWarps + 1 && lane == 0) {
+        if (kTma) {
+            tma_prefetch_desc(&map_x);
+            tma_prefetch_desc(&map_do);
+        }
+        if (vec) tma_prefetch_desc(&map_dq);
     }
     pdl_wait();
     const int nt = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nt;

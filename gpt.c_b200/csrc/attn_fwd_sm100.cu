@@ -9,7 +9,7 @@
 // addressed straight inside [B, T, 3C] by a 4-D tensor map (column, row, batch, plane).
 //
 // The grid has one CTA per item, heaviest first.  The first Q and K tiles are requested while the CTA is still being set
-// up, the finished tile is written straight from registers.  A sequence of at most 64 tokens takes one key step.
+// up, the finished tile leaves by the copy engine from where Q was.  A sequence of at most 64 tokens takes one key step.
 //
 // A CTA is deliberately small (about 100 KiB of shared memory, 256 columns of tensor memory,
 // 384 threads) so that TWO CTAs share an SM.  Inside a CTA two score buffers alternate, so the
@@ -62,6 +62,7 @@ struct __align__(1024) FwdSmem {
     uint64_t s_full[2], p_full[2], o_full;
     uint64_t pair_bar[4];       // [quarter]: the two halves of a row block meet here once per step
     uint64_t o_done;            // the last PV product of an item has completed
+    uint64_t staged[2];         // [half]: 32 columns of the output are where Q was
     float xmax[2][2][kTile];    // [step parity][half][row]: row maxima exchanged between halves
     float lpart[2][kTile];      // [half][row]: partial row sums for the epilogue
     uint32_t tmem_base;
@@ -70,7 +71,7 @@ struct __align__(1024) FwdSmem {
 
 enum Site : int {
     SITE_K_EMPTY = 1, SITE_V_EMPTY, SITE_Q_FULL, SITE_K_FULL, SITE_V_FULL, SITE_P_FULL, SITE_S_FULL, SITE_O_FULL,
-    SITE_O_FULL_LAST, SITE_Q_TMEM, SITE_PAIR, SITE_SMEM_ALIGN
+    SITE_O_FULL_LAST, SITE_Q_TMEM, SITE_PAIR, SITE_SMEM_ALIGN, SITE_STAGED
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -175,71 +176,60 @@ __device__ __forceinline__ void load_k(FwdSmem &sm, const CUtensorMap &map_x, co
     tma_load_4d(sm.k[st][1], &map_x, &sm.k_full[st], C + w.h * kD, j * kStep, w.b, 1);
 }
 
-// 32 columns of one row, scaled: 32 bytes per store when the pointer allows it.
-__device__ __forceinline__ void store_row(float *dst, const uint32_t (&r)[32], float by) {
-    if ((reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
-#pragma unroll
-        for (int c = 0; c < 32; c += 8)
-            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + c), "f"(__uint_as_float(r[c]) * by),
-                         "f"(__uint_as_float(r[c + 1]) * by), "f"(__uint_as_float(r[c + 2]) * by), "f"(__uint_as_float(r[c + 3]) * by),
-                         "f"(__uint_as_float(r[c + 4]) * by), "f"(__uint_as_float(r[c + 5]) * by), "f"(__uint_as_float(r[c + 6]) * by),
-                         "f"(__uint_as_float(r[c + 7]) * by)
-                         : "memory");
-    } else {
-#pragma unroll
-        for (int c = 0; c < 32; c += 4)
-            *reinterpret_cast<float4 *>(dst + c) = make_float4(__uint_as_float(r[c]) * by, __uint_as_float(r[c + 1]) * by,
-                                                               __uint_as_float(r[c + 2]) * by, __uint_as_float(r[c + 3]) * by);
-    }
-}
-
 // Sequences of at most 64 tokens: the (only) item's Q, K and V come from the fp32 tensor, every thread splits its share
 // into the two bf16 planes, in shared memory where the tensor cores read them and in `saved` for the backward.
 // That takes the split kernel, its launch and a second trip through memory out of a pass that is all latency.
-__device__ __forceinline__ void take_fp32(FwdSmem &sm, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ hi,
-                                          __nv_bfloat16 *__restrict__ lo, int b, int h, int T, int C) {
-    constexpr int kBatch = 4;  // 32 bytes each, all on their way before the first is used
-    for (int i0 = threadIdx.x; i0 < 3 * 8 * kStep; i0 += kBatch * kThreads) {
-        float4 a[kBatch][2];
+struct Chunks {  // this thread's 32-byte pieces of the 3 x 64 rows
+    static constexpr int kEach = 3 * 8 * kStep / kThreads;
+    static_assert(kEach * kThreads == 3 * 8 * kStep, "every thread has the same number");
+    uint4 hi[kEach], lo[kEach];
+    __device__ static int part(int u) { return ((int)threadIdx.x + u * kThreads) >> 9; }
+    __device__ static int row(int u) { return (((int)threadIdx.x + u * kThreads) >> 3) & 63; }
+    __device__ static int col() { return (int)threadIdx.x & 7; }
+    __device__ static size_t at(int u, int b, int h, int T, int C) {
+        return ((size_t)b * T + row(u)) * 3 * C + part(u) * C + h * kD + 8 * col();
+    }
+};
+__device__ __forceinline__ void take_fp32(FwdSmem &sm, Chunks &x, const float *__restrict__ qkv, int b, int h, int T, int C) {
+    float4 a[Chunks::kEach][2];  // all on their way before the first is used
+    const bool wide = aligned32(qkv);
 #pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-            const int i = i0 + u * kThreads, part = i >> 9, row = (i >> 3) & 63, c = i & 7;
-            a[u][0] = a[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < 3 * 8 * kStep && row < T) {
-                const float4 *src = reinterpret_cast<const float4 *>(qkv + ((size_t)b * T + row) * 3 * C + part * C + h * kD) + 2 * c;
-                a[u][0] = __ldcs(src);
-                a[u][1] = __ldcs(src + 1);
-            }
-        }
+    for (int u = 0; u < Chunks::kEach; u++) {
+        a[u][0] = a[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (Chunks::row(u) < T) load_f32x8(a[u][0], a[u][1], qkv + Chunks::at(u, b, h, T, C), wide);
+    }
 #pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-            const int i = i0 + u * kThreads, part = i >> 9, row = (i >> 3) & 63, c = i & 7;
-            if (i >= 3 * 8 * kStep) break;
-            uint4 vh, vl;
-            split_bf16x2(a[u][0].x, a[u][0].y, vh.x, vl.x);
-            split_bf16x2(a[u][0].z, a[u][0].w, vh.y, vl.y);
-            split_bf16x2(a[u][1].x, a[u][1].y, vh.z, vl.z);
-            split_bf16x2(a[u][1].z, a[u][1].w, vh.w, vl.w);
-            const int at = row * 128 + ((c ^ (row & 7)) << 4);
-            uint8_t *dh = part == 0 ? sm.q[0] : (part == 1 ? sm.k[0][0] : sm.v[0][0]);
-            uint8_t *dl = part == 0 ? sm.q[1] : (part == 1 ? sm.k[0][1] : sm.v[0][1]);
-            *reinterpret_cast<uint4 *>(dh + at) = vh;
-            *reinterpret_cast<uint4 *>(dl + at) = vl;
-            if (row < T) {
-                const size_t g = ((size_t)b * T + row) * 3 * C + part * C + h * kD + 8 * c;
-                *reinterpret_cast<uint4 *>(hi + g) = vh;
-                *reinterpret_cast<uint4 *>(lo + g) = vl;
-            }
-        }
+    for (int u = 0; u < Chunks::kEach; u++) {
+        split_bf16x2(a[u][0].x, a[u][0].y, x.hi[u].x, x.lo[u].x);
+        split_bf16x2(a[u][0].z, a[u][0].w, x.hi[u].y, x.lo[u].y);
+        split_bf16x2(a[u][1].x, a[u][1].y, x.hi[u].z, x.lo[u].z);
+        split_bf16x2(a[u][1].z, a[u][1].w, x.hi[u].w, x.lo[u].w);
+        const int part = Chunks::part(u), row = Chunks::row(u), at = row * 128 + ((Chunks::col() ^ (row & 7)) << 4);
+        uint8_t *dh = part == 0 ? sm.q[0] : (part == 1 ? sm.k[0][0] : sm.v[0][0]);
+        uint8_t *dl = part == 0 ? sm.q[1] : (part == 1 ? sm.k[0][1] : sm.v[0][1]);
+        *reinterpret_cast<uint4 *>(dh + at) = x.hi[u];
+        *reinterpret_cast<uint4 *>(dl + at) = x.lo[u];
     }
     fence_proxy_async_smem();
+}
+// The planes for the backward, once nothing waits for this thread's fence any more.
+__device__ __forceinline__ void save_planes(const Chunks &x, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, int b, int h,
+                                            int T, int C) {
+#pragma unroll
+    for (int u = 0; u < Chunks::kEach; u++) {
+        if (Chunks::row(u) >= T) continue;
+        const size_t at = Chunks::at(u, b, h, T, C);
+        *reinterpret_cast<uint4 *>(hi + at) = x.hi[u];
+        *reinterpret_cast<uint4 *>(lo + at) = x.lo[u];
+    }
 }
 
 template <bool kFp32>
 __global__ void __launch_bounds__(kThreads, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ hi,
-                __nv_bfloat16 *__restrict__ lo, float *__restrict__ out, float *__restrict__ out_copy, float *__restrict__ lse,
-                int B, int T, int H, float scale_log2, int *status) {
+attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_o,
+                const __grid_constant__ CUtensorMap map_copy, bool has_copy, const float *__restrict__ qkv,
+                __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, float *__restrict__ lse, int B, int T, int H,
+                float scale_log2, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     FwdSmem &sm = *reinterpret_cast<FwdSmem *>(smem_raw);
     if ((smem_u32(smem_raw) & 1023u) != 0) {
@@ -251,6 +241,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
     const int C = H * kD;
     WaitCtx ctx{&sm.abort_flag, status};
 
+    if (threadIdx.x == 96) {
+        if (!kFp32) tma_prefetch_desc(&map_x);
+        tma_prefetch_desc(&map_o);
+        if (has_copy) tma_prefetch_desc(&map_copy);
+    }
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         mbar_init(&sm.q_full, 1);
@@ -266,13 +261,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
         for (int i = 0; i < 4; i++) mbar_init(&sm.pair_bar[i], 64);
         mbar_init(&sm.o_full, 1);
         mbar_init(&sm.o_done, 1);
+        for (int i = 0; i < 2; i++) mbar_init(&sm.staged[i], kSoftmaxWarps / 2);
         fence_barrier_init();
         // This thread is also the Q/K producer: the first Q and K tiles are requested right away, while the other
         // warps are still setting up (but not before the kernel that wrote them has completed).
         if (!kFp32) {
             pdl_wait();
             fence_proxy_async_smem();
-            tma_prefetch_desc(&map_x);
             const Item w = decode((int)blockIdx.x, B, T, H);
             load_q(sm, map_x, w);
             for (int j = 0; j < min(2, w.nsteps); j++) load_k(sm, map_x, w, C, j, j);
@@ -282,9 +277,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
     pdl_wait();  // every thread, before its first access to global memory
+    Chunks chunks;
     if (kFp32) {
         const Item w = decode((int)blockIdx.x, B, T, H);
-        take_fp32(sm, qkv, hi, lo, w.b, w.h, T, C);
+        take_fp32(sm, chunks, qkv, w.b, w.h, T, C);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -297,6 +293,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
         mbar_arrive(&sm.k_full[0]);
         mbar_arrive(&sm.v_full[0]);
     }
+    if (kFp32) save_planes(chunks, hi, lo, w.b, w.h, T, C);
 
     if (kFp32 && (warp == 0 || warp == 3)) {
         // no loads to request
@@ -455,11 +452,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restri
             tmem_wait_ld();
             tc_fence_before_sync();
             const int tok = w.qt * kTile + row;
-            if (tok < T) {
-                if (half == 0) lse[((size_t)w.b * H + w.h) * T + tok] = (m + __log2f(l_all)) * 0.6931471805599453f;
-                const size_t at = ((size_t)w.b * T + tok) * C + (size_t)w.h * kD + 32 * half;
-                store_row(out + at, r, inv);
-                if (out_copy) store_row(out_copy + at, r, inv);
+            if (half == 0 && tok < T) lse[((size_t)w.b * H + w.h) * T + tok] = (m + __log2f(l_all)) * 0.6931471805599453f;
+            // This thread's own row and plane of Q, long in tensor memory, take its 32 columns, and the copy engine takes
+            // them from there (rows past the end are dropped).  Rows written from registers, a row per lane in 32-byte
+            // pieces, took 1640 cycles at the end of every CTA (B=8 T=128 H=12).
+            uint8_t *at = sm.q[half] + row * 128;
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                *reinterpret_cast<float4 *>(at + ((c ^ (row & 7)) << 4)) =
+                    make_float4(__uint_as_float(r[4 * c]) * inv, __uint_as_float(r[4 * c + 1]) * inv, __uint_as_float(r[4 * c + 2]) * inv,
+                                __uint_as_float(r[4 * c + 3]) * inv);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&sm.staged[half]);
+                if (quarter == 0 && mbar_wait(&sm.staged[half], 0, ctx, SITE_STAGED)) {
+                    tma_store_3d(sm.q[half], &map_o, w.h * kD + 32 * half, w.qt * kTile, w.b);
+                    if (has_copy) tma_store_3d(sm.q[half], &map_copy, w.h * kD + 32 * half, w.qt * kTile, w.b);
+                    bulk_commit();
+                    bulk_wait_read_all();  // shared memory stays alive until then
+                }
             }
         }
     }
@@ -537,6 +549,7 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     if (warp == kWorkWarps) {
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kCols);
     }
+    if (kTma && warp == kWorkWarps + 1 && lane == 0) tma_prefetch_desc(&map_x);
     pdl_wait();
     const int nq = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nq;
     const int q0 = (nq - 1 - (int)blockIdx.x / nbh) * kTile;  // longest rows first
@@ -727,18 +740,18 @@ cudaError_t fast_fwd_set_attributes() {
 
 static const float kScaleLog2 = 0.125f * 1.4426950408889634f;  // 1/sqrt(64) * log2(e)
 
-cudaError_t launch_fast_forward(const CUtensorMap &map_x, float *out, float *out_copy, float *lse, int B, int T, int H,
-                                int *status, cudaStream_t s) {
+cudaError_t launch_fast_forward(const CUtensorMap &map_x, const CUtensorMap &map_o, const CUtensorMap *map_copy, float *lse, int B,
+                                int T, int H, int *status, cudaStream_t s) {
     const int nqt = (T + kTile - 1) / kTile;
-    return launch_after_previous(attn_fwd_kernel<false>, dim3((unsigned)(nqt * B * H)), dim3(kThreads), sizeof(FwdSmem), s, map_x,
-                                 nullptr, nullptr, nullptr, out, out_copy, lse, B, T, H, kScaleLog2, status);
+    return launch_after_previous(attn_fwd_kernel<false>, dim3((unsigned)(nqt * B * H)), dim3(kThreads), sizeof(FwdSmem), s, map_x, map_o,
+                                 map_copy ? *map_copy : map_o, map_copy != nullptr, nullptr, nullptr, nullptr, lse, B, T, H, kScaleLog2,
+                                 status);
 }
 
-cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy,
-                                     float *lse, int B, int T, int H, int *status, cudaStream_t s) {
-    const CUtensorMap none = {};
-    return launch_after_previous(attn_fwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), sizeof(FwdSmem), s, none, qkv, hi,
-                                 lo, out, out_copy, lse, B, T, H, kScaleLog2, status);
+cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, const CUtensorMap &map_o,
+                                     const CUtensorMap *map_copy, float *lse, int B, int T, int H, int *status, cudaStream_t s) {
+    return launch_after_previous(attn_fwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), sizeof(FwdSmem), s, map_o, map_o,
+                                 map_copy ? *map_copy : map_o, map_copy != nullptr, qkv, hi, lo, lse, B, T, H, kScaleLog2, status);
 }
 
 cudaError_t attn24_fwd_set_attributes() {

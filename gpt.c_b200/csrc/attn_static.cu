@@ -109,7 +109,16 @@ extern "C" int attn_sm100_forward_static(const float *qkv, float *out, float *ls
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return (int)cudaErrorInvalidValue;
-    return (int)attn::launch_fast_forward(map_x, out, nullptr, lse, B, T, H, st.status, s);
+    CUtensorMap map_o;  // where the result goes: boxes of 32 columns by 128 rows
+    const int C = H * D;
+    const cuuint64_t odims[3] = {(cuuint64_t)C, (cuuint64_t)T, (cuuint64_t)B};
+    const cuuint64_t ostrides[2] = {(cuuint64_t)C * 4, (cuuint64_t)C * 4 * (cuuint64_t)T};
+    const cuuint32_t obox[3] = {32, 128, 1};
+    if (g_encode_static(&map_o, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, out, odims, ostrides, obox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return (int)cudaErrorInvalidValue;
+    return (int)attn::launch_fast_forward(map_x, map_o, nullptr, lse, B, T, H, st.status, s);
 }
 
 

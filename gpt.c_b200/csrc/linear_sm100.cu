@@ -189,6 +189,12 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     if (warp == 2) {
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
+    if (warp == 3 && lane == 0) {
+        for (int i = 0; i < (kClasses ? 4 : 1); i++) {
+            tma_prefetch_desc(&maps.a[i]);
+            tma_prefetch_desc(&maps.b[i]);
+        }
+    }
     pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();
     __syncthreads();
@@ -198,10 +204,6 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
         if (lane == 0) {
-            for (int i = 0; i < (kClasses ? 4 : 1); i++) {
-                tma_prefetch_desc(&maps.a[i]);
-                tma_prefetch_desc(&maps.b[i]);
-            }
             int it = 0;
             bool ok = true;
             for (int w = first; ok && w < p.total; w += step) {

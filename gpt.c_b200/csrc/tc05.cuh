@@ -146,6 +146,8 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, c
 // TMA: tiled loads global -> shared, completion signalled on an mbarrier (bytes).
 // The innermost coordinate times the element size must be a multiple of 16 bytes.
 // ------------------------------------------------------------------------------------------
+// Before pdl_wait() as a rule: a tensor map is an argument of the launch, and the first copy through it waits for the
+// fetch of the map otherwise.
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -435,6 +437,22 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
+}
+
+// ------------------------------------------------------------------------------------------
+// Global memory, 32 bytes per lane where the address allows it: whole sectors, where 16 bytes of every 32 ask for each
+// sector twice.
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
+__device__ __forceinline__ void load_f32x8(float4 &a, float4 &b, const float *p, bool wide) {
+    if (wide) {
+        asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                     : "l"(p));
+    } else {
+        a = __ldcs(reinterpret_cast<const float4 *>(p));
+        b = __ldcs(reinterpret_cast<const float4 *>(p) + 1);
+    }
 }
 
 // ------------------------------------------------------------------------------------------

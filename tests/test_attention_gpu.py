@@ -119,6 +119,35 @@ def test_general_tensor_core_kernels_are_fp32_and_repeatable(pkg, gpu, oracle, T
         assert np.array_equal(d.cpu().numpy()[..., 2 * D:], dx[..., 2 * D:])
 
 
+@pytest.mark.parametrize("T", [1, 40, 64, 65, 128])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_short_sequences_at_any_16_byte_address(pkg, gpu, oracle, T, offset):
+    """One key tile, with and without a second half; fp32 tensors read and written on 32-byte boundaries and off them."""
+    torch, B, H, D = gpu, 2, 3, 64
+    x, g = seeded(31 + T, B, T, H, D)
+
+    def at(values, shape):  # a tensor that starts `offset` floats behind a 512-byte boundary
+        n = int(np.prod(shape))
+        t = torch.full((n + offset,), 7.0, device="cuda")[offset:].view(shape)
+        return t if values is None else t.copy_(torch.from_numpy(values))
+
+    qkv, dout = at(x, x.shape), at(g, g.shape)
+    out, copy, dqkv = at(None, g.shape), at(None, g.shape), at(None, x.shape)
+    lse = torch.empty((B, H, T), device="cuda")
+    saved = torch.empty(pkg.saved_bytes(B, T, H, D), device="cuda", dtype=torch.uint8)
+    scratch = torch.empty(pkg.backward_scratch_bytes(B, T, H, D), device="cuda", dtype=torch.uint8)
+    pkg.forward_into(qkv, out, copy, lse, saved, H)
+    pkg.backward_into(saved, out, lse, dout, dqkv, scratch, H)
+    assert pkg.device_status() == 0
+    assert torch.equal(out, copy)
+    ref_dx = oracle.backward(x, g, H)
+    assert np.abs(out.cpu().numpy() - oracle.forward(x, H)).max() < EXPECT_OUT
+    assert np.abs(dqkv.cpu().numpy() - ref_dx).max() < EXPECT_DX
+    dqkv.zero_()
+    pkg.backward_into(saved, out, lse, dout, dqkv, scratch, H, flags=pkg.FLAG_CORE_ONLY)  # from what the call above left
+    assert np.abs(dqkv.cpu().numpy() - ref_dx).max() < EXPECT_DX
+
+
 # ---------------------------------------------------------------------------------------------
 # tensor-core kernels (D = 64)
 # ---------------------------------------------------------------------------------------------
