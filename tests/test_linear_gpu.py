@@ -196,6 +196,51 @@ def test_linear_backward_parts_can_be_skipped(pkg):
     within(dw_only.cpu().numpy(), dy.astype(np.float64).T @ x.astype(np.float64), dy.T, x)
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 96, 64), (37, 768, 768), (300, 2304, 768), (2048, 768, 768), (9, 16415, 32)])
+@pytest.mark.parametrize("want_dx,want_dw,want_db", [(True, True, True), (True, True, False), (True, False, True), (False, True, True)])
+def test_linear_backward_kernels_beside_each_other(pkg, M, N, K, want_dx, want_dw, want_db):
+    """dx, dW and db may run at the same time, but neither before what wrote dy, x and w nor after what reads the results:
+    back to back, with every input written by the kernel before and every result read by the kernel behind.  Small and
+    large tiles, clusters, pieces that add into zeros, a padded copy."""
+    L = pkg.lib()
+    rounds = 12
+    x, w, _, dy = inputs(M, N, K, 41)
+    st = torch.cuda.current_stream().cuda_stream
+    src = [torch.from_numpy(dy).cuda() * (i + 1) for i in range(rounds)]
+    xs = [torch.from_numpy(x).cuda() * 2.0 ** -i for i in range(rounds)]
+    wt = torch.from_numpy(w).cuda()
+
+    def copy(dst, source):
+        assert L.tensor_sm100_copy(dst.data_ptr(), source.data_ptr(), source.numel(), st) == 0
+
+    def once(i, g, xi):
+        copy(xi, xs[i])
+        copy(g, src[i])
+        dw = torch.zeros(N, K, device="cuda") if want_dw else None
+        db = torch.zeros(N, device="cuda") if want_db else None
+        dx = pkg.linear_backward(g, xi, wt, dw, db, want_dx=want_dx)
+        out = [torch.empty_like(t) if t is not None else None for t in (dx, dw, db)]
+        for o, t in zip(out, (dx, dw, db)):
+            if t is not None:
+                copy(o, t)
+                t.fill_(float("nan"))
+        return out
+
+    got, alone = [], []
+    g, xi = torch.empty_like(src[0]), torch.empty_like(xs[0])
+    for i in range(rounds):
+        got.append(once(i, g, xi))
+    torch.cuda.synchronize()
+    for i in range(rounds):
+        alone.append(once(i, g, xi))
+        torch.cuda.synchronize()
+    assert pkg.device_status() == 0
+    for a, b in zip(got, alone):
+        for u, v in zip(a, b):
+            # the order of additions in memory is free: up to 32 pieces, each within an ulp of the sum so far
+            assert (u is None and v is None) or (u - v).abs().max().item() <= 2.0 ** -19 * v.abs().max().item()
+
+
 def test_linear_argument_errors(pkg):
     L = pkg.lib()
     assert L.linear_sm100_forward(None, None, None, None, None, 1, 4, 4, None) == -1
