@@ -98,6 +98,7 @@ def _calls():
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         mod.set_error(AttnError)
+        mod.take_over(lib())
         _calls_module = mod
     return _calls_module
 

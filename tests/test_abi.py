@@ -94,3 +94,29 @@ def test_no_cpu_fallback_without_gpu(pkg):
     assert pkg.lib().attn_sm100_init() != 0
     with pytest.raises(pkg.AttnError):
         pkg.init()
+
+
+def test_extension_answers_like_ctypes(pkg):
+    """The entry points the extension puts in front of the ctypes functions: the same results for numbers, None, ctypes
+    objects and wrong arguments (all rejected or done before the GPU is touched), the same attributes."""
+    plain_lib = ctypes.CDLL(pkg.LIB_PATH)
+    for name, (res, args) in pkg.SIGNATURES.items():
+        getattr(plain_lib, name).restype, getattr(plain_lib, name).argtypes = res, args
+    pkg._calls()
+    fast = pkg.lib()
+    calls = [("tensor_sm100_axpy", (0, 1.0, None, None, None)), ("tensor_sm100_axpy", (5, 1.0, None, None, 0)),
+             ("tensor_sm100_axpy", (5, 1, None, None, None)), ("tensor_sm100_copy", (ctypes.c_void_p(0), None, ctypes.c_size_t(3), None)),
+             ("tensor_sm100_fill", (None, 2, 0.5, None)), ("tensor_sm100_arange", (None, 2, -1, -1, None)),
+             ("tensor_sm100_gelu_forward", (None, None, 1, None)), ("tensor_sm100_gelu_backward", (None, None, None, 1, None)),
+             ("xent_sm100_forward", (None, None, None, None, 1, 1, None)), ("xent_sm100_backward", (1, 1, 1, 1, -1, 2, None)),
+             ("attn_sm100_saved_bytes", (8, 1024, 12, 64)), ("attn_sm100_saved_bytes", (2 ** 32 + 1, 1, 1, 3)),
+             ("attn_sm100_backward_scratch_bytes", (1, -1, 1, 1)), ("attn_sm100_backward_scratch_bytes", (True, 7, 2, 64))]
+    for name, args in calls:
+        assert getattr(fast, name)(*args) == getattr(plain_lib, name)(*args), (name, args)
+    for args in ((1,), ("a", 1.0, None, None, None), (1, "a", None, None, None), (1.5, 1.0, None, None, None), (1, 1.0, 2.5, None, None)):
+        with pytest.raises((TypeError, ctypes.ArgumentError)) as ours:
+            fast.tensor_sm100_axpy(*args)
+        with pytest.raises((TypeError, ctypes.ArgumentError)) as plain:
+            plain_lib.tensor_sm100_axpy(*args)
+        assert ours.type is plain.type
+    assert fast.tensor_sm100_axpy.argtypes == pkg.SIGNATURES["tensor_sm100_axpy"][1]
