@@ -588,13 +588,13 @@ Plan plan_tiles(int M, int N, int kb, int sms) {
 
 // The same with the contraction cut into up to 32 pieces that add into the result with bulk reductions (dW, and dx when
 // its contraction is very long); those cost 80 ns per megabyte and make a block 15 % slower.
-Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks) {
+Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks, int most = 32) {
     Plan best{128, 1, 0};
     for (const Cost &c : kCosts) {
         if (c.bn > 128 && N < c.bn) continue;
         const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + c.bn - 1) / c.bn);
         const long long tile_bytes = (long long)kBM * c.bn * 4;
-        for (int s = 1; s <= 32 && s <= kb; s++) {
+        for (int s = 1; s <= most && s <= kb; s++) {
             const int per = (kb + s - 1) / s;
             if (s > 1 && per < least_blocks) break;
             const long long t = c.fixed + rounds_ns(c, tiles * s, per, sms) * 115 / 100 +
@@ -741,11 +741,14 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
                    cudaStream_t s) {
     const int kb = np / kBK;
     Plan plan = plan_tiles(M, K, kb, sms);
-    if (kb >= 512) {  // very long (the vocabulary projection): pieces may pay, although dx has to be zeroed first
-        Plan cut = plan_pieces(M, K, kb, sms, 32);
-        cut.ns += 2500 + (int)((long long)M * K * 4 / 5500);
-        if (cut.splits > 1 && cut.ns < plan.ns) plan = cut;
-    }
+    // Pieces of the contraction may fill the SMs better, although dx has to be zeroed first.  Any number where it is very long
+    // (the vocabulary projection), else two, whose sum does not depend on their order, and if they are expected to save more
+    // than the estimate's error (M, N, K: 900, 5120, 1280 52 -> 33 us, 3000, 12032, 512 96 -> 80; without a margin 6000, 9999,
+    // 768 214 -> 220).
+    const bool very_long = kb >= 512;
+    Plan cut = plan_pieces(M, K, kb, sms, 32, very_long ? 32 : 2);
+    cut.ns += 2500 + (int)((long long)M * K * 4 / 5500);
+    if (cut.splits > 1 && (very_long ? cut.ns : at_most_int(cut.ns * 21ll / 20)) < plan.ns) plan = cut;
     int split = 1, rc;
     if (plan_split(M, K, np, sms, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, sms, chain, status, s);
     CUtensorMap ma, mb, mc;

@@ -241,6 +241,18 @@ def test_linear_backward_kernels_beside_each_other(pkg, M, N, K, want_dx, want_d
             assert (u is None and v is None) or (u - v).abs().max().item() <= 2.0 ** -19 * v.abs().max().item()
 
 
+@pytest.mark.parametrize("M,N,K", [(900, 5120, 1280), (257, 4096, 512), (3000, 12001, 512)])
+def test_linear_input_gradient_in_two_pieces(pkg, M, N, K):
+    """A contraction in two pieces that add into zeros: within the bound, and the same in every call."""
+    x, w, _, dy = inputs(M, N, K, 43)
+    g, xt, wt = (torch.from_numpy(t).cuda() for t in (dy, x, w))
+    first = pkg.linear_backward(g, xt, wt, None, None)
+    assert pkg.device_status() == 0
+    within(first.cpu().numpy(), dy.astype(np.float64) @ w.astype(np.float64), dy, w)
+    for _ in range(5):
+        assert torch.equal(pkg.linear_backward(g, xt, wt, None, None), first)
+
+
 def test_linear_argument_errors(pkg):
     L = pkg.lib()
     assert L.linear_sm100_forward(None, None, None, None, None, 1, 4, 4, None) == -1
