@@ -99,6 +99,32 @@ __device__ __forceinline__ void lds8(float (&f)[8], const float *src, int c) {
     f[0] = x.x, f[1] = x.y, f[2] = x.z, f[3] = x.w, f[4] = y.x, f[5] = y.y, f[6] = y.z, f[7] = y.w;
 }
 
+// Eight values from column col of a row as the two bf16 planes the backward reads, rounded as launch_split rounds them.
+__device__ __forceinline__ void save8(__nv_bfloat16 *hi, __nv_bfloat16 *lo, int col, int width, const float (&f)[8], bool vec) {
+    if (col >= width) return;
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) split_bf16x2(f[2 * e], f[2 * e + 1], h[e], l[e]);
+    if (vec && width % 8 == 0) {
+        *reinterpret_cast<uint4 *>(hi + col) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4 *>(lo + col) = make_uint4(l[0], l[1], l[2], l[3]);
+    } else if (vec) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            if (col + 4 * i >= width) break;
+            *reinterpret_cast<uint2 *>(hi + col + 4 * i) = make_uint2(h[2 * i], h[2 * i + 1]);
+            *reinterpret_cast<uint2 *>(lo + col + 4 * i) = make_uint2(l[2 * i], l[2 * i + 1]);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            if (col + e >= width) break;
+            reinterpret_cast<uint16_t *>(hi)[col + e] = (uint16_t)(h[e >> 1] >> (16 * (e & 1)));
+            reinterpret_cast<uint16_t *>(lo)[col + e] = (uint16_t)(l[e >> 1] >> (16 * (e & 1)));
+        }
+    }
+}
+
 // Tiles in shared memory: planes of 64-column blocks, in a block a row of 128 bytes per row, with the 128-byte swizzle.
 // A worker moves eight values at a time: column 8 c of row r (of 64) and, from 64 columns on, the same in the next block.
 struct Chunk {

@@ -216,7 +216,9 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
     // the set-up of the next, is faster: B=8 T=128 H=12 9.5 us in two kernels, 14 us in one.
     if (fast && T <= attn::kShortT / 2 && B * H <= ds->num_sms && !(flags & (ATTN_FLAG_CORE_ONLY | ATTN_FLAG_PREPARE_ONLY)))
         return (int)attn::launch_fast_forward_fp32(qkv, hi, lo, map_o, out_copy ? &map_copy : nullptr, lse, B, T, H, ds->status, s);
-    if (!(flags & ATTN_FLAG_CORE_ONLY)) {
+    // the general kernel on the tensor cores writes the planes itself
+    const bool planes_too = !fast && use_attn24(D) && !(flags & (ATTN_FLAG_CORE_ONLY | ATTN_FLAG_PREPARE_ONLY));
+    if (!(flags & ATTN_FLAG_CORE_ONLY) && !planes_too) {
         e = attn::launch_split(qkv, hi, lo, n, s);
         if (e != cudaSuccess) return (int)e;
     }
@@ -228,7 +230,7 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
         if (rc != 0) return rc;
         e = attn::launch_fast_forward(map_x, map_o, out_copy ? &map_copy : nullptr, lse, B, T, H, ds->status, s);
     } else {
-        e = use_attn24(D) ? attn::launch_attn24_forward(qkv, out, out_copy, lse, B, T, H, D, ds->status, s)
+        e = use_attn24(D) ? attn::launch_attn24_forward(qkv, planes_too ? hi : nullptr, lo, out, out_copy, lse, B, T, H, D, ds->status, s)
                           : attn::launch_generic_forward(qkv, out, out_copy, lse, B, T, H, D, s);
     }
     return (int)e;

@@ -494,6 +494,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 // The 16 worker warps convert K of the next step and start its scores before they turn to the softmax of this one, and
 // convert V behind the softmax, so the tensor cores have the next scores and this step's P V ahead of them.
 //
+// The CTA of a query tile also leaves the bf16 planes of that tile's rows for the backward: Q at the start, K and V when it
+// gets to the diagonal.
+//
 // What bounds it: the tensor cores, 12 bf16 passes over both products (3200 cycles per step at D = 128), with the
 // conversions, the softmax and the additions of the workers beneath them.
 // ---------------------------------------------------------------------------------------
@@ -518,8 +521,10 @@ enum Site24 : int { SITE24_GO_S = 301, SITE24_GO_PV, SITE24_S, SITE24_PV, SITE24
 // kTma: D = 16 kK, and the copy engine fetches the rows; else the workers read them when they need them.
 template <int kK, bool kTma>
 __global__ void __launch_bounds__(attn24::kThreads, 1)
-attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ qkv, float *__restrict__ out,
-                  float *__restrict__ out_copy, float *__restrict__ lse, int T, int H, int D_arg, Scale scale_log2, int *status) {
+attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_o,
+                  const __grid_constant__ CUtensorMap map_copy, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ xhi,
+                  __nv_bfloat16 *__restrict__ xlo, float *__restrict__ out, float *__restrict__ out_copy, float *__restrict__ lse,
+                  int T, int H, int D_arg, Scale scale_log2, int *status) {
     using Smem = Fwd24Smem<kK>;
     constexpr int kPlane = Smem::kPlane, kBlocks = Smem::kBlocks;
     constexpr uint32_t kColS = 0, kColO = 192, kColQ = 192 + 16 * kK;  // S (96 columns) twice; P takes its place
@@ -549,7 +554,10 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     if (warp == kWorkWarps) {
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kCols);
     }
-    if (kTma && warp == kWorkWarps + 1 && lane == 0) tma_prefetch_desc(&map_x);
+    if (kTma && warp == kWorkWarps + 1 && lane == 0) {
+        tma_prefetch_desc(&map_x);
+        tma_prefetch_desc(&map_o);
+    }
     pdl_wait();
     const int nq = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nq;
     const int q0 = (nq - 1 - (int)blockIdx.x / nbh) * kTile;  // longest rows first
@@ -612,8 +620,7 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         const Chunk mine(tid);
         // This thread's values of a 64-row tile (rows from t0 on, the columns of one head at src) as three terms into the
         // planes at `tile`; phase: how often the buffer has been filled before.
-        auto put = [&](uint8_t *tile, int plane, int block, int kv, const float *src, int t0, int phase) {
-            float f[kBlocks][8];
+        auto put = [&](float (&f)[kBlocks][8], uint8_t *tile, int plane, int block, int kv, const float *src, int t0, int phase) {
             if (kTma) {
                 await(&sm.raw_full[kv], phase & 1, ctx, SITE24_RAW_FULL);
 #pragma unroll
@@ -630,9 +637,21 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             for (int i = 0; i < kBlocks; i++)
                 if (mine.has<kK>(i)) store_split3(tile, plane, mine.at + i * block, f[i]);
         };
+        // The same values for the backward, behind the arrival that others wait for (its fence would wait for the stores).
+        // part: 0, 1, 2 for Q, K, V
+        auto save = [&](const float (&f)[kBlocks][8], int part, int t0) {
+            const int t = t0 + mine.r;
+            if (xhi == nullptr || t0 < q0 || t >= T) return;
+            const size_t at = (size_t)b * T * C3 + (size_t)t * C3 + (size_t)part * C + (size_t)h * D;
+#pragma unroll
+            for (int i = 0; i < kBlocks; i++)
+                if (mine.has<kK>(i)) save8(xhi + at, xlo + at, mine.col(i), D, f[i], vec);
+        };
         // Q: split like K and V, 128 rows where those will be, and from there into tensor memory
+        float f[kBlocks][8], q[2][kBlocks][8];
+#pragma unroll
         for (int half = 0; half < 2; half++)
-            put(sm.k[0] + half * (kStep * 128), 2 * kPlane, kTile * 128, half, head, q0 + half * kStep, 0);
+            put(q[half], sm.k[0] + half * (kStep * 128), 2 * kPlane, kTile * 128, half, head, q0 + half * kStep, 0);
         named_sync(5, kWorkers);
 #pragma unroll
         for (int i = 0; i < kK; i++) {
@@ -647,8 +666,11 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         }
         tmem_wait_st();
         named_sync(5, kWorkers);
-        put(sm.k[0], kPlane, kStep * 128, 0, head + C, 0, 1);
+        put(f, sm.k[0], kPlane, kStep * 128, 0, head + C, 0, 1);
         warp_arrive(&sm.go_s, lane);
+        save(q[0], 0, q0);
+        save(q[1], 0, q0 + kStep);
+        save(f, 1, 0);
 
         float o[4 * kK], m = -INFINITY, l = 0.f, alpha_before = 1.f;
 #pragma unroll
@@ -656,8 +678,9 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         for (int n = 0; n < nsteps; n++) {
             await(&sm.done_s, n & 1, ctx, SITE24_S);
             if (n + 1 < nsteps) {
-                put(sm.k[0], kPlane, kStep * 128, 0, head + C, (n + 1) * kStep, n + 2);
+                put(f, sm.k[0], kPlane, kStep * 128, 0, head + C, (n + 1) * kStep, n + 2);
                 warp_arrive(&sm.go_s, lane);
+                save(f, 1, (n + 1) * kStep);
             }
             const uint32_t t_s = tmem + lane_addr + kColS + (n & 1) * 96;
             uint32_t s[16];
@@ -701,8 +724,9 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 add_columns<kK>(o, t_o, alpha_before);
             }
             alpha_before = alpha;
-            put(sm.v[0], kPlane, kStep * 128, 1, head + 2 * C, n * kStep, n + 1);
+            put(f, sm.v[0], kPlane, kStep * 128, 1, head + 2 * C, n * kStep, n + 1);
             warp_arrive(&sm.go_pv, lane);
+            save(f, 2, n * kStep);
         }
         sm.part[nsteps & 1][cq][row] = l;
         named_sync(1 + quarter, 128);
@@ -710,11 +734,33 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         await(&sm.done_pv, (nsteps - 1) & 1, ctx, SITE24_PV);
         add_columns<kK>(o, t_o, alpha_before);
         const int t = q0 + row;
+        const float inv = 1.0f / l;
+        if (kTma) {
+            // by the copy engine, from the place of the raw K and V: groups of 16 columns, 128 rows of 64 bytes, swizzled
+            uint8_t *stage = reinterpret_cast<uint8_t *>(sm.raw[0]);
+#pragma unroll
+            for (int i = 0; i < kK; i++) {
+                const int col = 4 * kK * cq + 4 * i;
+                *reinterpret_cast<float4 *>(stage + (col >> 4) * (kTile * 64) + row * 64 + ((((col >> 2) & 3) ^ ((row >> 1) & 3)) << 4)) =
+                    make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
+            }
+            fence_proxy_async_smem();
+            named_sync(5, kWorkers);
+            if (tid == 0) {
+                for (int g = 0; g < kK; g++) {
+                    tma_store_3d(stage + g * (kTile * 64), &map_o, h * D + 16 * g, q0, b);
+                    if (out_copy) tma_store_3d(stage + g * (kTile * 64), &map_copy, h * D + 16 * g, q0, b);
+                }
+                bulk_commit();
+                bulk_wait_read_all();  // shared memory stays alive until then
+            }
+        }
         if (t < T) {
-            const float inv = 1.0f / l;
             const size_t at = ((size_t)b * T + t) * C + (size_t)h * D;
-            store_columns<kK>(out + at, 4 * kK * cq, D, o, inv, vec);
-            if (out_copy) store_columns<kK>(out_copy + at, 4 * kK * cq, D, o, inv, vec);
+            if (!kTma) {
+                store_columns<kK>(out + at, 4 * kK * cq, D, o, inv, vec);
+                if (out_copy) store_columns<kK>(out_copy + at, 4 * kK * cq, D, o, inv, vec);
+            }
             // m ln 2 + ln l, ln 2 in two parts
             if (cq == 0) lse[(size_t)bh * T + t] = fmaf(m, 0.693147182464599609375f, fmaf(m, -1.904654299957768e-9f, logf(l)));
         }
@@ -768,20 +814,28 @@ cudaError_t attn24_fwd_set_attributes() {
     return cudaSuccess;
 }
 
-cudaError_t launch_attn24_forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H, int D, int *status,
-                                  cudaStream_t s) {
-    CUtensorMap map_x = {};
+cudaError_t launch_attn24_forward(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy, float *lse, int B,
+                                  int T, int H, int D, int *status, cudaStream_t s) {
+    CUtensorMap map_x = {}, map_o = {}, map_copy = {};
     const bool tma = D % 16 == 0;
     if (tma) {
-        const int rc = attn24_rows_map(&map_x, qkv, B, T, 3 * H * D, D, attn24::kStep);
+        int rc = attn24_rows_map(&map_x, qkv, B, T, 3 * H * D, D, attn24::kStep);
+        auto output = [&](CUtensorMap *map, float *to) {
+            const cuuint64_t dims[3] = {(cuuint64_t)H * D, (cuuint64_t)T, (cuuint64_t)B};
+            const cuuint64_t strides[2] = {(cuuint64_t)H * D * 4, (cuuint64_t)H * D * 4 * (cuuint64_t)T};
+            const cuuint32_t box[3] = {16, (cuuint32_t)kTile, 1};
+            return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, to, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
+        };
+        if (rc == 0) rc = output(&map_o, out);
+        if (rc == 0 && out_copy) rc = output(&map_copy, out_copy);
         if (rc != 0) return (cudaError_t)rc;
     }
     return attn24::with_groups((D + 15) / 16, [&](auto k) {
         constexpr int kK = decltype(k)::value;
         const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile)));
         return launch_after_previous(tma ? general::attn24_fwd_kernel<kK, true> : general::attn24_fwd_kernel<kK, false>, grid,
-                                     dim3(attn24::kThreads), sizeof(general::Fwd24Smem<kK>), s, map_x, qkv, out, out_copy, lse, T, H,
-                                     D, attn24::log2_scale(D), status);
+                                     dim3(attn24::kThreads), sizeof(general::Fwd24Smem<kK>), s, map_x, map_o, map_copy, qkv, hi, lo,
+                                     out, out_copy, lse, T, H, D, attn24::log2_scale(D), status);
     });
 }
 

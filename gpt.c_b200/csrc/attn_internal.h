@@ -55,8 +55,9 @@ cudaError_t launch_generic_backward(const __nv_bfloat16 *xhi, const __nv_bfloat1
 int attn24_rows_map(CUtensorMap *map, const void *base, int B, int T, int W, int D, int rows);
 cudaError_t attn24_fwd_set_attributes();
 cudaError_t attn24_bwd_set_attributes();
-cudaError_t launch_attn24_forward(const float *qkv, float *out, float *out_copy, float *lse, int B, int T, int H, int D, int *status,
-                                  cudaStream_t s);
+// hi, lo: receive the planes that launch_split would write (NULL: they are there already)
+cudaError_t launch_attn24_forward(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy, float *lse, int B,
+                                  int T, int H, int D, int *status, cudaStream_t s);
 // map_x: see launch_fast_backward below
 cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse, const float *delta,
                                    const float *dout, float *dqkv, int B, int T, int H, int D, int *status, cudaStream_t s);

@@ -119,6 +119,27 @@ def test_general_tensor_core_kernels_are_fp32_and_repeatable(pkg, gpu, oracle, T
         assert np.array_equal(d.cpu().numpy()[..., 2 * D:], dx[..., 2 * D:])
 
 
+@pytest.mark.parametrize("T,D", [(1, 3), (70, 20), (128, 48), (200, 40), (193, 128), (257, 72)])
+def test_general_forward_leaves_the_planes_of_the_split(pkg, gpu, T, D):
+    """Bit for bit what the split alone writes, whatever the alignment of the rows, and a core-only call leaves them alone."""
+    torch, B, H = gpu, 2, 3
+    x, _ = seeded(37 + T, B, T, H, D)
+    qkv = torch.from_numpy(x).cuda()
+    n, size = x.size, pkg.saved_bytes(B, T, H, D)
+    out, lse = torch.empty(B, T, H * D, device="cuda"), torch.empty((B, H, T), device="cuda")
+    planes = []
+    for flags in (pkg.FLAG_FORCE_GENERIC, pkg.FLAG_FORCE_GENERIC | pkg.FLAG_PREPARE_ONLY):
+        saved = torch.full((size,), 0x7f, device="cuda", dtype=torch.uint8)
+        pkg.forward_into(qkv, out, None, lse, saved, H, flags=flags)
+        planes.append(saved.cpu().numpy())
+    for at in (0, size // 2):
+        assert np.array_equal(planes[0][at:at + 2 * n], planes[1][at:at + 2 * n])
+    first = out.clone()
+    saved = torch.full((size,), 0x7f, device="cuda", dtype=torch.uint8)
+    pkg.forward_into(qkv, out, None, lse, saved, H, flags=pkg.FLAG_FORCE_GENERIC | pkg.FLAG_CORE_ONLY)
+    assert torch.equal(out, first) and bool((saved == 0x7f).all()) and pkg.device_status() == 0
+
+
 @pytest.mark.parametrize("T", [1, 40, 64, 65, 128])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_short_sequences_at_any_16_byte_address(pkg, gpu, oracle, T, offset):
