@@ -117,11 +117,20 @@ int encode_tiled(CUtensorMap *map, CUtensorMapDataType dtype, unsigned rank, con
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-int attn24_rows_map(CUtensorMap *map, const void *base, int B, int T, int W, int D, int rows) {
-    const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)T, (cuuint64_t)B, 1};
-    const cuuint64_t strides[3] = {(cuuint64_t)W * 4, (cuuint64_t)W * 4 * (cuuint64_t)T, (cuuint64_t)W * 4 * (cuuint64_t)T * (cuuint64_t)B};
-    const cuuint32_t box[4] = {(cuuint32_t)D, (cuuint32_t)rows, 1, 1};
-    return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+int attn24_heads_map(CUtensorMap *map, const void *base, int B, int T, int heads, int D, int cols, int rows, CUtensorMapSwizzle swizzle) {
+    const cuuint64_t row = (cuuint64_t)heads * D * 4;
+    const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)heads, (cuuint64_t)T, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {(cuuint64_t)D * 4, row, row * (cuuint64_t)T};
+    const cuuint32_t box[4] = {(cuuint32_t)cols, 1, (cuuint32_t)rows, 1};
+    return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, swizzle);
+}
+
+int attn24_planes_map(CUtensorMap *map, const void *saved, int B, int T, int H, int D) {
+    const cuuint64_t row = (cuuint64_t)3 * H * D * 2;
+    const cuuint64_t dims[5] = {(cuuint64_t)D, (cuuint64_t)3 * H, (cuuint64_t)T, (cuuint64_t)B, 2};
+    const cuuint64_t strides[4] = {(cuuint64_t)D * 2, row, row * (cuuint64_t)T, plane_bytes((size_t)B * T * 3 * H * D)};
+    const cuuint32_t box[5] = {64, 1, 64, 1, 1};
+    return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, saved, dims, strides, box);
 }
 
 int device_status_word(int **status) {
@@ -289,7 +298,7 @@ int attn_sm100_backward(const void *saved, const float *out, const float *lse, c
         }
         if (!core) return ATTN_OK;
         CUtensorMap map_x = {};
-        if (use_attn24(D) && D % 16 == 0 && (rc = encode_planes(&map_x, saved, B, T, 3 * H * D, xplane, 64)) != 0) return rc;
+        if (use_attn24(D) && D % 8 == 0 && (rc = attn::attn24_planes_map(&map_x, saved, B, T, H, D)) != 0) return rc;
         e = use_attn24(D) ? attn::launch_attn24_backward(map_x, xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, ds->status, s)
                           : attn::launch_generic_backward(xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, s);
     }

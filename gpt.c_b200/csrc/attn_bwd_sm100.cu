@@ -888,7 +888,7 @@ struct __align__(1024) Bwd24Smem {
     static constexpr int kDs = kBlocks == 1 ? 3 * kQueryPlane : 0;  // dS^T in g: behind dO, or in its place
     uint8_t k[2][kKeyPlane], v[2][kKeyPlane], q[2][kQueryPlane];
     uint8_t g[kDs + 3 * kDsPlane];  // dO [3][kQueryPlane], dS^T [3][kDsPlane]
-    // dQ on its way to memory, rows of D: [step parity][K plane, query], or half of the queries
+    // dQ on its way to memory: [step parity][K plane, query], or half of the queries
     __align__(128) float out[kOuts][kOutRows * 16 * kK];
     // dO of the next step as it comes (two blocks: in g, over the last two planes of dO itself)
     __align__(128) float raw_own[kBlocks == 1 ? kStep * 16 * kK : 32];
@@ -906,13 +906,14 @@ enum Site24 : int {
     SITE24_RAW_FREE, SITE24_STAT, SITE24_SMEM_ALIGN
 };
 
-// kTma: D = 16 kK, and the copy engine fetches Q, K, V and dO; else the workers do.
+// kTma: D is a multiple of 8, and the copy engine fetches Q, K, V and dO, whole blocks of columns of a head of which those
+// past the D-th read as zeros; else the workers do.
 template <int kK, bool kTma>
 __global__ void __launch_bounds__(attn24::kThreads, 1)
 attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_do,
                   const __grid_constant__ CUtensorMap map_dq, const __nv_bfloat16 *__restrict__ xhi,
                   const __nv_bfloat16 *__restrict__ xlo, const float *__restrict__ lse, const float *__restrict__ delta,
-                  const float *__restrict__ dout, float *__restrict__ dqkv, int T, int H, int D_arg, float scale, Scale scale_log2,
+                  const float *__restrict__ dout, float *__restrict__ dqkv, int T, int H, int D, float scale, Scale scale_log2,
                   int *status) {
     using Smem = Bwd24Smem<kK>;
     constexpr int kKeyPlane = Smem::kKeyPlane, kQueryPlane = Smem::kQueryPlane, kDsPlane = Smem::kDsPlane;
@@ -927,7 +928,6 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         return;
     }
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int D = kTma ? 16 * kK : D_arg;
     const bool vec = kTma || D % 4 == 0;
     WaitCtx ctx{&sm.abort_flag, status};
     if (tid == 0) {
@@ -976,20 +976,20 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if (warp == kWorkWarps + 1) {
         // ------------------------------ producer: K, V, Q and dO ------------------------------
         if (kTma && lane == 0) {
-            auto load_keys = [&](uint8_t *tile, uint64_t *bar, int x) {
+            auto load_keys = [&](uint8_t *tile, uint64_t *bar, int head) {
 #pragma unroll 1
                 for (int plane = 0; plane < 2; plane++)
 #pragma unroll 1
                     for (int i = 0; i < kBlocks; i++)
 #pragma unroll 1
                         for (int half = 0; half < 2; half++)
-                            tma_load_4d(tile + plane * kKeyPlane + i * (kTile * 128) + half * (kStep * 128), &map_x, bar, x + 64 * i,
+                            tma_load_5d(tile + plane * kKeyPlane + i * (kTile * 128) + half * (kStep * 128), &map_x, bar, 64 * i, head,
                                         k0 + half * kStep, b, plane);
             };
             for (int n = 0; n < nsteps; n++) {
                 auto load_do = [&]() {
                     mbar_expect_tx(&sm.raw_full, kStep * 16 * kK * 4);
-                    tma_load_4d(sm.raw(), &map_do, &sm.raw_full, h * D, k0 + n * kStep, b, 0);
+                    tma_load_4d(sm.raw(), &map_do, &sm.raw_full, 0, h, k0 + n * kStep, b);
                 };
                 if (kOne) {
                     if (n > 0 && !await_thread(&sm.raw_free, (n - 1) & 1, ctx, SITE24_RAW_FREE)) break;
@@ -1001,15 +1001,15 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 for (int plane = 0; plane < 2; plane++)
 #pragma unroll 1
                     for (int i = 0; i < kBlocks; i++)
-                        tma_load_4d(sm.q[plane] + i * (kStep * 128), &map_x, &sm.go_s, h * D + 64 * i, k0 + n * kStep, b, plane);
+                        tma_load_5d(sm.q[plane] + i * (kStep * 128), &map_x, &sm.go_s, 64 * i, h, k0 + n * kStep, b, plane);
                 if (!kOne) {  // its place is dS's
                     if (n > 0 && !await_thread(&sm.done_dq, (n - 1) & 1, ctx, SITE24_DQ)) break;
                     load_do();
                 }
                 if (n == 0) {
-                    load_keys(sm.k[0], &sm.go_s, C + h * D);
+                    load_keys(sm.k[0], &sm.go_s, H + h);
                     mbar_expect_tx(&sm.v_full, 2 * kKeyPlane);
-                    load_keys(sm.v[0], &sm.v_full, 2 * C + h * D);
+                    load_keys(sm.v[0], &sm.v_full, 2 * H + h);
                 }
             }
         }
@@ -1126,7 +1126,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 await(&sm.raw_full, n & 1, ctx, SITE24_RAW_FULL);
 #pragma unroll
                 for (int i = 0; i < kBlocks; i++)
-                    if (mine.has<kK>(i)) lds8(greg[i], sm.raw() + mine.r * D + mine.col(i), mine.c);
+                    if (mine.has<kK>(i)) lds8(greg[i], sm.raw() + mine.r * (16 * kK) + mine.col(i), mine.c);
                 if (kOne) warp_arrive(&sm.raw_free, lane);  // its fence holds the copy engine back until these values are in registers
                 else named_sync(5, kWorkers);
             }
@@ -1164,9 +1164,9 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             tmem_wait_ld();
             if (dq_col >= D) return;
             if (vec) {
-                float *dst = sm.out[n & (Smem::kOuts - 1)] + (kOne ? row / 64 * kStep + 16 * cq : 16 * (cq & 1)) * D + dq_col;
+                float *dst = sm.out[n & (Smem::kOuts - 1)] + (kOne ? row / 64 * kStep + 16 * cq : 16 * (cq & 1)) * (16 * kK) + dq_col;
 #pragma unroll
-                for (int e = 0; e < 16; e++) dst[e * D] = __uint_as_float(r[e]) * scale;
+                for (int e = 0; e < 16; e++) dst[e * 16 * kK] = __uint_as_float(r[e]) * scale;
             } else {
                 float *dst = dqkv + head + (size_t)q0 * C3 + dq_col;
 #pragma unroll
@@ -1178,7 +1178,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         auto send_dq = [&](int parity, int t) {
 #pragma unroll 1
             for (int plane = 0; t < T && plane < (kOne ? 2 : 1); plane++)
-                tma_reduce_add_3d(sm.out[parity] + plane * kStep * D, &map_dq, h * D, t, b);
+                tma_reduce_add_4d(sm.out[parity] + plane * kStep * 16 * kK, &map_dq, 0, h, t, b);
             bulk_commit();
         };
 
@@ -1398,17 +1398,13 @@ cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16
                                    const float *delta, const float *dout, float *dqkv, int B, int T, int H, int D, int *status,
                                    cudaStream_t s) {
     CUtensorMap map_do = {}, map_dq = {};
-    const bool tma = D % 16 == 0;
+    const bool tma = D % 8 == 0;
+    const int wide = (D + 15) / 16 * 16;
     int rc = 0;
-    if (tma) rc = attn24_rows_map(&map_do, dout, B, T, H * D, D, attn24::kStep);
+    if (tma) rc = attn24_heads_map(&map_do, dout, B, T, H, D, wide, attn24::kStep, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc == 0 && D % 4 == 0)
+        rc = attn24_heads_map(&map_dq, dqkv, B, T, 3 * H, D, wide, D <= 64 ? attn24::kStep : attn24::kStep / 2, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != 0) return (cudaError_t)rc;
-    if (D % 4 == 0) {  // one head's rows of dq
-        const cuuint64_t width = (cuuint64_t)3 * H * D;
-        const cuuint64_t dims[3] = {width, (cuuint64_t)T, (cuuint64_t)B}, strides[2] = {width * 4, width * 4 * (cuuint64_t)T};
-        const cuuint32_t box[3] = {(cuuint32_t)D, (cuuint32_t)(D <= 64 ? attn24::kStep : attn24::kStep / 2), 1};
-        rc = encode_tiled(&map_dq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dqkv, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
-        if (rc != 0) return (cudaError_t)rc;
-    }
     return attn24::with_groups((D + 15) / 16, [&](auto k) {
         constexpr int kK = decltype(k)::value;
         const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile)));

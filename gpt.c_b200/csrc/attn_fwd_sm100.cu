@@ -508,7 +508,7 @@ template <int kK>  // head columns in groups of 16
 struct __align__(1024) Fwd24Smem {
     static constexpr int kBlocks = (kK + 3) / 4, kPlane = kBlocks * kStep * 128;  // bytes of one term of a K or V tile
     uint8_t k[3][kPlane], v[3][kPlane];  // before the first step: the three terms of Q, 128 rows each
-    float raw[2][kStep * 16 * kK];       // K, V of the next step as they come (rows of D); first the halves of Q
+    float raw[2][kStep * 16 * kK];       // K, V of the next step as they come; first the halves of Q
     uint64_t raw_full[2], raw_free[2];
     uint64_t go_s, go_pv, done_s, done_pv;
     float part[2][4][kTile];  // [step parity][column quarter][row]: row maxima, at the end row sums
@@ -518,13 +518,14 @@ struct __align__(1024) Fwd24Smem {
 
 enum Site24 : int { SITE24_GO_S = 301, SITE24_GO_PV, SITE24_S, SITE24_PV, SITE24_RAW_FREE, SITE24_RAW_FULL, SITE24_SMEM_ALIGN };
 
-// kTma: D = 16 kK, and the copy engine fetches the rows; else the workers read them when they need them.
+// kTma: D is a multiple of 4, and the copy engine fetches and stores the rows, 16 kK columns of a head of which those past
+// the D-th read as zeros and are not written; else the workers read them when they need them.
 template <int kK, bool kTma>
 __global__ void __launch_bounds__(attn24::kThreads, 1)
 attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_o,
                   const __grid_constant__ CUtensorMap map_copy, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ xhi,
                   __nv_bfloat16 *__restrict__ xlo, float *__restrict__ out, float *__restrict__ out_copy, float *__restrict__ lse,
-                  int T, int H, int D_arg, Scale scale_log2, int *status) {
+                  int T, int H, int D, Scale scale_log2, int *status) {
     using Smem = Fwd24Smem<kK>;
     constexpr int kPlane = Smem::kPlane, kBlocks = Smem::kBlocks;
     constexpr uint32_t kColS = 0, kColO = 192, kColQ = 192 + 16 * kK;  // S (96 columns) twice; P takes its place
@@ -536,8 +537,7 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         return;
     }
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int D = kTma ? 16 * kK : D_arg;
-    const bool vec = kTma || D % 4 == 0;
+    constexpr bool vec = kTma;
     WaitCtx ctx{&sm.abort_flag, status};
     if (tid == 0) {
         sm.abort_flag = 0;
@@ -577,8 +577,8 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             for (int n = 0; n <= nsteps; n++) {
                 if (n > 0 && !await_thread(&sm.raw_free[kv], (n - 1) & 1, ctx, SITE24_RAW_FREE)) break;
                 mbar_expect_tx(&sm.raw_full[kv], kStep * 16 * kK * 4);
-                tma_load_4d(sm.raw[kv], &map_x, &sm.raw_full[kv], (n > 0 ? (kv + 1) * C : 0) + h * D,
-                            n > 0 ? (n - 1) * kStep : q0 + kv * kStep, b, 0);
+                tma_load_4d(sm.raw[kv], &map_x, &sm.raw_full[kv], 0, (n > 0 ? (kv + 1) * H : 0) + h,
+                            n > 0 ? (n - 1) * kStep : q0 + kv * kStep, b);
             }
         }
     } else if (warp == kWorkWarps) {
@@ -625,7 +625,7 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 await(&sm.raw_full[kv], phase & 1, ctx, SITE24_RAW_FULL);
 #pragma unroll
                 for (int i = 0; i < kBlocks; i++)
-                    if (mine.has<kK>(i)) lds8(f[i], sm.raw[kv] + mine.r * D + mine.col(i), mine.c);
+                    if (mine.has<kK>(i)) lds8(f[i], sm.raw[kv] + mine.r * (16 * kK) + mine.col(i), mine.c);
                 warp_arrive(&sm.raw_free[kv], lane);  // its fence holds the copy engine back until these values are in registers
             } else {
                 const float *from = src + (size_t)(t0 + mine.r) * C3;
@@ -748,8 +748,9 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             named_sync(5, kWorkers);
             if (tid == 0) {
                 for (int g = 0; g < kK; g++) {
-                    tma_store_3d(stage + g * (kTile * 64), &map_o, h * D + 16 * g, q0, b);
-                    if (out_copy) tma_store_3d(stage + g * (kTile * 64), &map_copy, h * D + 16 * g, q0, b);
+                    if (16 * g >= D) break;
+                    tma_store_4d(stage + g * (kTile * 64), &map_o, 16 * g, h, q0, b);
+                    if (out_copy) tma_store_4d(stage + g * (kTile * 64), &map_copy, 16 * g, h, q0, b);
                 }
                 bulk_commit();
                 bulk_wait_read_all();  // shared memory stays alive until then
@@ -817,17 +818,11 @@ cudaError_t attn24_fwd_set_attributes() {
 cudaError_t launch_attn24_forward(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy, float *lse, int B,
                                   int T, int H, int D, int *status, cudaStream_t s) {
     CUtensorMap map_x = {}, map_o = {}, map_copy = {};
-    const bool tma = D % 16 == 0;
+    const bool tma = D % 4 == 0;
     if (tma) {
-        int rc = attn24_rows_map(&map_x, qkv, B, T, 3 * H * D, D, attn24::kStep);
-        auto output = [&](CUtensorMap *map, float *to) {
-            const cuuint64_t dims[3] = {(cuuint64_t)H * D, (cuuint64_t)T, (cuuint64_t)B};
-            const cuuint64_t strides[2] = {(cuuint64_t)H * D * 4, (cuuint64_t)H * D * 4 * (cuuint64_t)T};
-            const cuuint32_t box[3] = {16, (cuuint32_t)kTile, 1};
-            return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, to, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
-        };
-        if (rc == 0) rc = output(&map_o, out);
-        if (rc == 0 && out_copy) rc = output(&map_copy, out_copy);
+        int rc = attn24_heads_map(&map_x, qkv, B, T, 3 * H, D, (D + 15) / 16 * 16, attn24::kStep, CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc == 0) rc = attn24_heads_map(&map_o, out, B, T, H, D, 16, kTile, CU_TENSOR_MAP_SWIZZLE_64B);
+        if (rc == 0 && out_copy) rc = attn24_heads_map(&map_copy, out_copy, B, T, H, D, 16, kTile, CU_TENSOR_MAP_SWIZZLE_64B);
         if (rc != 0) return (cudaError_t)rc;
     }
     return attn24::with_groups((D + 15) / 16, [&](auto k) {

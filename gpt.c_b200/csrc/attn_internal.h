@@ -51,14 +51,17 @@ cudaError_t launch_generic_backward(const __nv_bfloat16 *xhi, const __nv_bfloat1
                                     cudaStream_t s);
 
 // The general kernels on the tensor cores (D <= kAttn24MaxD, T <= kGenericMaxT), fp32 operands as three bf16 terms.
-// fp32 [B, T, W] as a 4-D map {W, T, B, 1} with boxes of D columns by `rows`, not swizzled.
-int attn24_rows_map(CUtensorMap *map, const void *base, int B, int T, int W, int D, int rows);
+// fp32 [B, T, heads, D] (D a multiple of 4) as a 4-D map {D, heads, T, B} with boxes of `cols` columns of one head by `rows`
+// tokens; columns past the D-th read as zeros and are not written.
+int attn24_heads_map(CUtensorMap *map, const void *base, int B, int T, int heads, int D, int cols, int rows, CUtensorMapSwizzle swizzle);
+// The bf16 planes at `saved` (D a multiple of 8) as a 5-D map {D, 3 H, T, B, plane}, boxes of 64 columns by 64 tokens.
+int attn24_planes_map(CUtensorMap *map, const void *saved, int B, int T, int H, int D);
 cudaError_t attn24_fwd_set_attributes();
 cudaError_t attn24_bwd_set_attributes();
 // hi, lo: receive the planes that launch_split would write (NULL: they are there already)
 cudaError_t launch_attn24_forward(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy, float *lse, int B,
                                   int T, int H, int D, int *status, cudaStream_t s);
-// map_x: see launch_fast_backward below
+// map_x: attn24_planes_map where D is a multiple of 8, else not looked at
 cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse, const float *delta,
                                    const float *dout, float *dqkv, int B, int T, int H, int D, int *status, cudaStream_t s);
 
