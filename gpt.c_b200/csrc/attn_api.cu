@@ -279,7 +279,7 @@ int attn_sm100_backward(const void *saved, const float *out, const float *lse, c
         e = attn::launch_fast_backward_fp32(map_x, map_dx, dout, out, lse, delta, dhi, dlo, dqkv, B, T, H, sched, ds->status, s);
     } else if (fast) {
         if (prepare) {
-            e = attn::launch_bwd_prepare(dout, out, delta, dhi, dlo, dqkv, sched, B, T, H, D, s);
+            e = attn::launch_bwd_prepare(dout, out, delta, dhi, dlo, dqkv, false, sched, B, T, H, D, s);
             if (e != cudaSuccess) return (int)e;
         }
         if (!core) return ATTN_OK;
@@ -292,14 +292,16 @@ int attn_sm100_backward(const void *saved, const float *out, const float *lse, c
         if (rc != 0) return rc;
         e = attn::launch_fast_backward(map_x, map_do, map_dx, lse, delta, dqkv, B, T, H, ds->num_sms, sched, ds->status, s);
     } else {
+        // two pieces add to dk and dv, which only a preparation of this call leaves at zero
+        const int pieces = use_attn24(D) && D % 4 == 0 && prepare && core ? attn::attn24_backward_pieces(B, T, H, ds->num_sms) : 1;
         if (prepare) {
-            e = attn::launch_bwd_prepare(dout, out, delta, nullptr, nullptr, dqkv, nullptr, B, T, H, D, s);
+            e = attn::launch_bwd_prepare(dout, out, delta, nullptr, nullptr, dqkv, pieces > 1, nullptr, B, T, H, D, s);
             if (e != cudaSuccess) return (int)e;
         }
         if (!core) return ATTN_OK;
         CUtensorMap map_x = {};
         if (use_attn24(D) && D % 8 == 0 && (rc = attn::attn24_planes_map(&map_x, saved, B, T, H, D)) != 0) return rc;
-        e = use_attn24(D) ? attn::launch_attn24_backward(map_x, xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, ds->status, s)
+        e = use_attn24(D) ? attn::launch_attn24_backward(map_x, xhi, xlo, lse, delta, dout, dqkv, pieces, B, T, H, D, ds->status, s)
                           : attn::launch_generic_backward(xhi, xlo, lse, delta, dout, dqkv, B, T, H, D, s);
     }
     return (int)e;

@@ -859,7 +859,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 // General backward: any head size up to 128; fp32 dO, P and dS as three bf16 terms (attn24.cuh), Q, K, V as the two the
 // forward saved.
 //
-// One CTA per (b, h, 128 keys), which walks the queries from the diagonal on in steps of 64:
+// One CTA per (b, h, 128 keys), which walks the queries from the diagonal on in steps of 64, or two that take half of the
+// steps each (attn24_backward_pieces):
 //     S^T = K Q^T, dP^T = V dO^T      (lanes = keys; 4 and 5 term products)
 //     dV += P^T dO, dK += dS^T Q      (P^T, dS^T from tensor memory; 6 and 5)
 //     dQ^T = K^T dS^T                 (lanes = head columns; 5)
@@ -911,9 +912,9 @@ enum Site24 : int {
 template <int kK, bool kTma>
 __global__ void __launch_bounds__(attn24::kThreads, 1)
 attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_do,
-                  const __grid_constant__ CUtensorMap map_dq, const __nv_bfloat16 *__restrict__ xhi,
+                  const __grid_constant__ CUtensorMap map_dq, const __grid_constant__ CUtensorMap map_dkv, const __nv_bfloat16 *__restrict__ xhi,
                   const __nv_bfloat16 *__restrict__ xlo, const float *__restrict__ lse, const float *__restrict__ delta,
-                  const float *__restrict__ dout, float *__restrict__ dqkv, int T, int H, int D, float scale, Scale scale_log2,
+                  const float *__restrict__ dout, float *__restrict__ dqkv, int pieces, int T, int H, int D, float scale, Scale scale_log2,
                   int *status) {
     using Smem = Bwd24Smem<kK>;
     constexpr int kKeyPlane = Smem::kKeyPlane, kQueryPlane = Smem::kQueryPlane, kDsPlane = Smem::kDsPlane;
@@ -927,6 +928,14 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE24_SMEM_ALIGN);
         return;
     }
+    const int nt = (T + kTile - 1) / kTile * pieces, nbh = (int)gridDim.x / nt;
+    const int tile = (int)blockIdx.x / nbh;  // the first keys are seen by the most queries
+    const int k0 = tile / pieces * kTile, all = (T - k0 + kStep - 1) / kStep, first_part = (all + pieces - 1) / pieces;
+    const int nsteps = tile % pieces == 0 ? first_part : all - first_part;
+    const int qs = k0 + (tile % pieces == 0 ? 0 : first_part * kStep);  // first query
+    if (nsteps == 0) return;
+    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
+    const int C = H * D;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const bool vec = kTma || D % 4 == 0;
     WaitCtx ctx{&sm.abort_flag, status};
@@ -962,10 +971,6 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (vec) tma_prefetch_desc(&map_dq);
     }
     pdl_wait();
-    const int nt = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nt;
-    const int k0 = (int)blockIdx.x / nbh * kTile;  // the first keys are seen by the most queries
-    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
-    const int C = H * D, nsteps = (T - k0 + kStep - 1) / kStep;
     const size_t C3 = 3 * (size_t)C, head = (size_t)b * T * C3 + (size_t)h * D;
     const float *dhead = dout + (size_t)b * T * C + (size_t)h * D;
     tc_fence_before_sync();
@@ -989,7 +994,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             for (int n = 0; n < nsteps; n++) {
                 auto load_do = [&]() {
                     mbar_expect_tx(&sm.raw_full, kStep * 16 * kK * 4);
-                    tma_load_4d(sm.raw(), &map_do, &sm.raw_full, 0, h, k0 + n * kStep, b);
+                    tma_load_4d(sm.raw(), &map_do, &sm.raw_full, 0, h, qs + n * kStep, b);
                 };
                 if (kOne) {
                     if (n > 0 && !await_thread(&sm.raw_free, (n - 1) & 1, ctx, SITE24_RAW_FREE)) break;
@@ -1001,7 +1006,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 for (int plane = 0; plane < 2; plane++)
 #pragma unroll 1
                     for (int i = 0; i < kBlocks; i++)
-                        tma_load_5d(sm.q[plane] + i * (kStep * 128), &map_x, &sm.go_s, 64 * i, h, k0 + n * kStep, b, plane);
+                        tma_load_5d(sm.q[plane] + i * (kStep * 128), &map_x, &sm.go_s, 64 * i, h, qs + n * kStep, b, plane);
                 if (!kOne) {  // its place is dS's
                     if (n > 0 && !await_thread(&sm.done_dq, (n - 1) & 1, ctx, SITE24_DQ)) break;
                     load_do();
@@ -1019,7 +1024,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             float v[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int t = k0 + n * kStep + 32 * (i & 1) + lane;
+                const int t = qs + n * kStep + 32 * (i & 1) + lane;
                 v[i] = t < T ? (i < 2 ? lse : delta)[(size_t)bh * T + t] : 0.f;
             }
             if (n > 1) await(&sm.stat_free[n & 1], ((n >> 1) - 1) & 1, ctx, SITE24_STAT);
@@ -1101,7 +1106,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         const Chunk mine(tid);
         auto put_q = [&](int n) {
             if (kTma) return;
-            const int t = k0 + n * kStep + mine.r;
+            const int t = qs + n * kStep + mine.r;
             const size_t from = head + (size_t)t * C3;
 #pragma unroll
             for (int i = 0; i < kBlocks; i++)
@@ -1115,7 +1120,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         float greg[kBlocks][8];
         auto request_g = [&](int n) {
             if (kTma) return;
-            const int t = k0 + n * kStep + mine.r;
+            const int t = qs + n * kStep + mine.r;
             const float *from = dhead + (size_t)t * C;
 #pragma unroll
             for (int i = 0; i < kBlocks; i++)
@@ -1158,7 +1163,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         // that are not 16-byte aligned are added to from registers.
         const int dq_col = kOne ? row % 64 : row;
         auto take_dq = [&](int n) {
-            const int q0 = k0 + n * kStep + 16 * cq;
+            const int q0 = qs + n * kStep + 16 * cq;
             uint32_t r[16];
             tmem_ld16(tmem + lane_addr + kColDQ + 16 * cq, r);
             tmem_wait_ld();
@@ -1194,7 +1199,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             *reinterpret_cast<uint4 *>(to + 2 * kDsPlane) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         };
         for (int n = 0; n < nsteps; n++) {
-            const int q0 = k0 + n * kStep;
+            const int q0 = qs + n * kStep;
             const bool more = n + 1 < nsteps;
             await(&sm.stat_full[n & 1], (n >> 1) & 1, ctx, SITE24_STAT);
             await(&sm.done_s, n & 1, ctx, SITE24_S);
@@ -1320,14 +1325,34 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 if (vec) {
                     fence_proxy_async_smem();
                     named_sync(2, kWorkers / 2);
-                    if (tid == 256) send_dq(0, k0 + nsteps * kStep - kStep / 2);
+                    if (tid == 256) send_dq(0, qs + nsteps * kStep - kStep / 2);
                 }
             }
         }
         if (tid == 0 || tid == 256) bulk_wait_all();
-        const int t = k0 + row;
-        if (t < T) {
-            float *dst = dqkv + head + (size_t)t * C3;
+        if (vec) {
+            // dK and dV by the copy engine, from where K and V were: groups of 16 columns, 128 rows of 64 bytes, swizzled
+#pragma unroll
+            for (int i = 0; i < kK; i++) {
+                const int col = 4 * kK * cq + 4 * i;
+                const int at = (col >> 4) * (kTile * 64) + row * 64 + ((((col >> 2) & 3) ^ ((row >> 1) & 3)) << 4);
+                *reinterpret_cast<float4 *>(sm.k[0] + at) = make_float4(dk[4 * i] * scale, dk[4 * i + 1] * scale, dk[4 * i + 2] * scale, dk[4 * i + 3] * scale);
+                *reinterpret_cast<float4 *>(sm.v[0] + at) = make_float4(dv[4 * i], dv[4 * i + 1], dv[4 * i + 2], dv[4 * i + 3]);
+            }
+            fence_proxy_async_smem();
+            named_sync(5, kWorkers);
+            if (tid == 0) {
+                for (int g = 0; g < kK && 16 * g < D; g++)
+                    for (int part = 0; part < 2; part++) {
+                        const uint8_t *from = (part == 0 ? sm.k[0] : sm.v[0]) + g * (kTile * 64);
+                        if (pieces == 1) tma_store_4d(from, &map_dkv, 16 * g, (part + 1) * H + h, k0, b);
+                        else tma_reduce_add_4d(from, &map_dkv, 16 * g, (part + 1) * H + h, k0, b);
+                    }
+                bulk_commit();
+                bulk_wait_all();
+            }
+        } else if (k0 + row < T) {
+            float *dst = dqkv + head + (size_t)(k0 + row) * C3;
             store_columns<kK>(dst + C, 4 * kK * cq, D, dk, scale, vec);
             store_columns<kK>(dst + 2 * C, 4 * kK * cq, D, dv, 1.f, vec);
         }
@@ -1394,23 +1419,40 @@ cudaError_t attn24_bwd_set_attributes() {
     return cudaSuccess;
 }
 
+// The CTA of the first keys has T / 64 steps, the average SM as many as there are in all divided by the SMs: where the former
+// is the longer, two CTAs share the steps of a key tile (a CTA costs about one step more than it has).  Not more than two,
+// so that the sums of dk and dv do not depend on the order of the additions.  Backward with preparation, 1 -> 2 pieces, us:
+// B=4 T=1024 H=6 D=128 114 -> 103, B=2 T=1000 H=8 D=112 105 -> 65, B=1 T=2048 H=4 D=128 187 -> 103, B=1 T=511 H=2 D=100
+// 62 -> 37, B=8 T=512 H=16 D=32 83 -> 73.
+int attn24_backward_pieces(int B, int T, int H, int sms) {
+    const long long nt = (T + kTile - 1) / kTile, longest = (T + attn24::kStep - 1) / attn24::kStep, bh = (long long)B * H;
+    long long steps = 0;
+    for (long long k0 = 0; k0 < T; k0 += kTile) steps += (T - k0 + attn24::kStep - 1) / attn24::kStep;
+    auto time = [&](int pieces) {
+        const long long one = (longest + pieces - 1) / pieces + 1, even = (bh * (steps + nt * pieces) + sms - 1) / sms + 1;
+        return one > even ? one : even;
+    };
+    return time(2) * 21 < time(1) * 20 ? 2 : 1;
+}
+
 cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse,
-                                   const float *delta, const float *dout, float *dqkv, int B, int T, int H, int D, int *status,
-                                   cudaStream_t s) {
-    CUtensorMap map_do = {}, map_dq = {};
+                                   const float *delta, const float *dout, float *dqkv, int pieces, int B, int T, int H, int D,
+                                   int *status, cudaStream_t s) {
+    CUtensorMap map_do = {}, map_dq = {}, map_dkv = {};
     const bool tma = D % 8 == 0;
     const int wide = (D + 15) / 16 * 16;
     int rc = 0;
     if (tma) rc = attn24_heads_map(&map_do, dout, B, T, H, D, wide, attn24::kStep, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc == 0 && D % 4 == 0)
         rc = attn24_heads_map(&map_dq, dqkv, B, T, 3 * H, D, wide, D <= 64 ? attn24::kStep : attn24::kStep / 2, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc == 0 && D % 4 == 0) rc = attn24_heads_map(&map_dkv, dqkv, B, T, 3 * H, D, 16, kTile, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc != 0) return (cudaError_t)rc;
     return attn24::with_groups((D + 15) / 16, [&](auto k) {
         constexpr int kK = decltype(k)::value;
-        const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile)));
+        const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile) * pieces));
         return launch_after_previous(tma ? general::attn24_bwd_kernel<kK, true> : general::attn24_bwd_kernel<kK, false>, grid,
-                                     dim3(attn24::kThreads), sizeof(general::Bwd24Smem<kK>), s, map_x, map_do, map_dq, xhi, xlo, lse,
-                                     delta, dout, dqkv, T, H, D, 1.0f / sqrtf((float)D), attn24::log2_scale(D), status);
+                                     dim3(attn24::kThreads), sizeof(general::Bwd24Smem<kK>), s, map_x, map_do, map_dq, map_dkv, xhi, xlo, lse,
+                                     delta, dout, dqkv, pieces, T, H, D, 1.0f / sqrtf((float)D), attn24::log2_scale(D), status);
     });
 }
 

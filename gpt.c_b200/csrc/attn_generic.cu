@@ -102,10 +102,10 @@ __global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ x,
 
 // ---------------------------------------------------------------------------------------
 // backward preparation for the general kernels: delta[b,h,t] = sum_d dout*out, and zero-fill of the
-// dq third of dqkv (the backward accumulates dq with atomics).  One warp per (b, t, h): D elements.
+// dq third of dqkv (the backward accumulates dq in memory), or of all of it.  One warp per (b, t, h): D elements.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) bwd_prepare_kernel(const float *__restrict__ dout, const float *__restrict__ out,
-                                                           float *__restrict__ delta, float *__restrict__ dq_zero,
+                                                           float *__restrict__ delta, float *__restrict__ dqkv, bool zero_all,
                                                            int B, int T, int H, int D) {
     tc05::pdl_launch_dependents();
     tc05::pdl_wait();
@@ -123,11 +123,33 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const float *__restric
         for (int d = lane; d < D; d += kWarp) {
             const float g = dout[base + d];
             acc += g * out[base + d];
-            dq_zero[bt * 3 * C + (size_t)h * D + d] = 0.f;
+            float *zero = dqkv + bt * 3 * C + (size_t)h * D + d;
+            zero[0] = 0.f;
+            if (zero_all) zero[C] = zero[2 * C] = 0.f;
         }
         acc = warp_sum(acc);
         if (lane == 0) delta[((size_t)b * H + h) * T + t] = acc;
     }
+}
+
+// The same for up to 64 columns, a multiple of 4: 8 or 16 lanes per row, a 16-byte word each (B=32 T=1024 H=16 D=64 118 ->
+// 84 us, B=8 T=1024 H=4 D=48 7.6 -> 6.8; at D = 128 the kernel above is faster, 6.5 against 8.2 us for B=4 T=1024 H=6).
+__global__ void __launch_bounds__(256) bwd_prepare_words_kernel(const float *__restrict__ dout, const float *__restrict__ out,
+                                                                 float *__restrict__ delta, float *__restrict__ dqkv, bool zero_all,
+                                                                 int lanes, int B, int T, int H, int D) {
+    tc05::pdl_launch_dependents();
+    tc05::pdl_wait();
+    const size_t w = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes, nrows = (size_t)B * T * H, bt = w / H;
+    const int d = 4 * (threadIdx.x % lanes), h = (int)(w % H), C = H * D;
+    float acc = 0.f;
+    if (w < nrows && d < D) {
+        const float4 g = __ldcs(reinterpret_cast<const float4 *>(dout + w * D + d)), o = __ldcs(reinterpret_cast<const float4 *>(out + w * D + d));
+        acc = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
+        for (int part = 0; part < (zero_all ? 3 : 1); part++)
+            *reinterpret_cast<float4 *>(dqkv + (bt * 3 + part) * C + (size_t)h * D + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (w < nrows && d == 0) delta[(bt / T * H + h) * T + bt % T] = acc;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -817,17 +839,22 @@ cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, s
 }
 
 cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta, __nv_bfloat16 *dhi,
-                               __nv_bfloat16 *dlo, float *dq_zero, int *sched, int B, int T, int H, int D, cudaStream_t s) {
+                               __nv_bfloat16 *dlo, float *dqkv, bool zero_all, int *sched, int B, int T, int H, int D, cudaStream_t s) {
     if (D == 64 && dhi && dlo) {
         const size_t nvec = (size_t)B * T * H * 8;
         const size_t blocks = (nvec + 255) / 256;
         return launch_after_previous(bwd_prepare64_kernel, dim3((unsigned)blocks), dim3(256), 0, s, dout, out, delta, dhi,
-                                     dlo, dq_zero, sched, B, T, H);
+                                     dlo, dqkv, sched, B, T, H);
     }
     const size_t rows = (size_t)B * T * H;
+    if (D % 4 == 0 && D <= 64) {
+        const int lanes = D > 32 ? 16 : 8;
+        return launch_after_previous(bwd_prepare_words_kernel, dim3((unsigned)((rows * lanes + 255) / 256)), dim3(256), 0, s, dout, out,
+                                     delta, dqkv, zero_all, lanes, B, T, H, D);
+    }
     const size_t most = (size_t)sm_count() * 16;
     const size_t blocks = (rows + 7) / 8 < most ? (rows + 7) / 8 : most;
-    return launch_after_previous(bwd_prepare_kernel, dim3((unsigned)blocks), dim3(256), 0, s, dout, out, delta, dq_zero, B, T,
+    return launch_after_previous(bwd_prepare_kernel, dim3((unsigned)blocks), dim3(256), 0, s, dout, out, delta, dqkv, zero_all, B, T,
                                  H, D);
 }
 

@@ -36,11 +36,11 @@ inline size_t plane_bytes(size_t n) { return align_up(n * sizeof(__nv_bfloat16),
 // fp32 -> (hi, lo) bf16 planes, hi = bf16(x), lo = bf16(x - hi).
 cudaError_t launch_split(const float *x, __nv_bfloat16 *hi, __nv_bfloat16 *lo, size_t n, cudaStream_t s);
 
-// rowsum(dout * out) per (b, h, t) -> delta [B, H, T], and zero-fill of the dq third of `dq_zero` ([B, T, 3C]);
+// rowsum(dout * out) per (b, h, t) -> delta [B, H, T], and zero-fill of the dq third of dqkv ([B, T, 3C]), or of all of it;
 // also splits dout into bf16 planes when dhi/dlo are given and zeroes the two ints at `sched` (the item counter
 // of the tensor-core backward kernel) when that is given.
 cudaError_t launch_bwd_prepare(const float *dout, const float *out, float *delta, __nv_bfloat16 *dhi,
-                               __nv_bfloat16 *dlo, float *dq_zero, int *sched, int B, int T, int H, int D, cudaStream_t s);
+                               __nv_bfloat16 *dlo, float *dqkv, bool zero_all, int *sched, int B, int T, int H, int D, cudaStream_t s);
 
 // General-shape SIMT kernels (kAttn24MaxD < D <= kGenericMaxD, T <= kGenericMaxT).
 cudaError_t generic_set_attributes();
@@ -63,7 +63,10 @@ cudaError_t launch_attn24_forward(const float *qkv, __nv_bfloat16 *hi, __nv_bflo
                                   int T, int H, int D, int *status, cudaStream_t s);
 // map_x: attn24_planes_map where D is a multiple of 8, else not looked at
 cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo, const float *lse, const float *delta,
-                                   const float *dout, float *dqkv, int B, int T, int H, int D, int *status, cudaStream_t s);
+                                   const float *dout, float *dqkv, int pieces, int B, int T, int H, int D, int *status, cudaStream_t s);
+// Into how many pieces (1 or 2, D a multiple of 4 only) the queries of a key tile are best cut: with 2 dk and dv are added to
+// memory, which has to be zero.
+int attn24_backward_pieces(int B, int T, int H, int sms);
 
 // Tensor-core (tcgen05) kernels, D == 64.  The tensor maps cover the bf16 hi/lo planes:
 //   map_x : dims {3C, T, B, 2 planes}, box {64, 128, 1, 1}, 128-byte swizzle

@@ -140,6 +140,24 @@ def test_general_forward_leaves_the_planes_of_the_split(pkg, gpu, T, D):
     assert torch.equal(out, first) and bool((saved == 0x7f).all()) and pkg.device_status() == 0
 
 
+@pytest.mark.parametrize("B,T,H,D", [(1, 65, 1, 48), (2, 200, 3, 20), (1, 513, 2, 128), (4, 300, 10, 96)])
+def test_general_backward_in_one_and_two_pieces(pkg, gpu, oracle, B, T, H, D):
+    """The stages called one by one take a key tile's queries in one piece, called together in two where SMs would be idle:
+    the same sums in another order (up to nine steps of 64 queries, each rounded once), and within the oracle's bound."""
+    torch = gpu
+    x, g = seeded(41 + T, B, T, H, D)
+    out, ctx = pkg.forward(torch.from_numpy(x).cuda(), H, flags=pkg.FLAG_FORCE_GENERIC)
+    dout = torch.from_numpy(g).cuda()
+    together = pkg.backward(ctx, dout)
+    apart = torch.full_like(together, float("nan"))
+    scratch = torch.empty(pkg.backward_scratch_bytes(B, T, H, D), device="cuda", dtype=torch.uint8)
+    for stage in (pkg.FLAG_PREPARE_ONLY, pkg.FLAG_CORE_ONLY):
+        pkg.backward_into(ctx.saved, ctx.out, ctx.lse, dout, apart, scratch, H, flags=pkg.FLAG_FORCE_GENERIC | stage)
+    assert pkg.device_status() == 0
+    assert (together - apart).norm().item() < 2.0 ** -21 * apart.norm().item()
+    assert np.abs(together.cpu().numpy() - oracle.backward(x, g, H)).max() < GENERIC_TOL
+
+
 @pytest.mark.parametrize("T", [1, 40, 64, 65, 128])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_short_sequences_at_any_16_byte_address(pkg, gpu, oracle, T, offset):
