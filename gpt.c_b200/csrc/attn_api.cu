@@ -215,16 +215,11 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
     __nv_bfloat16 *hi = static_cast<__nv_bfloat16 *>(saved);
     __nv_bfloat16 *lo = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(saved) + plane);
     cudaError_t e = cudaSuccess;
-    CUtensorMap map_o, map_copy;  // where the tensor-core kernels' result goes
-    if (fast && !(flags & ATTN_FLAG_PREPARE_ONLY)) {
-        if ((rc = encode_rows_f32(&map_o, out, B, T, H * D)) != 0) return rc;
-        if (out_copy && (rc = encode_rows_f32(&map_copy, out_copy, B, T, H * D)) != 0) return rc;
-    }
     // Both stages in one kernel for sequences of one key step and no more of them than SMs (6.7 -> 4.6 us for one of 40
     // tokens).  Beyond that the split kernel, which spreads the conversion over the whole GPU and overlaps its end with
     // the set-up of the next, is faster: B=8 T=128 H=12 9.5 us in two kernels, 14 us in one.
     if (fast && T <= attn::kShortT / 2 && B * H <= ds->num_sms && !(flags & (ATTN_FLAG_CORE_ONLY | ATTN_FLAG_PREPARE_ONLY)))
-        return (int)attn::launch_fast_forward_fp32(qkv, hi, lo, map_o, out_copy ? &map_copy : nullptr, lse, B, T, H, ds->status, s);
+        return (int)attn::launch_fast_forward_fp32(qkv, hi, lo, out, out_copy, lse, B, T, H, ds->status, s);
     // the general kernel on the tensor cores writes the planes itself
     const bool planes_too = !fast && use_attn24(D) && !(flags & (ATTN_FLAG_CORE_ONLY | ATTN_FLAG_PREPARE_ONLY));
     if (!(flags & ATTN_FLAG_CORE_ONLY) && !planes_too) {
@@ -234,10 +229,11 @@ int attn_sm100_forward(const float *qkv, float *out, float *out_copy, float *lse
     if (flags & ATTN_FLAG_PREPARE_ONLY) return ATTN_OK;
 
     if (fast) {
-        CUtensorMap map_x;
-        rc = encode_planes(&map_x, saved, B, T, 3 * H * D, plane, 64);
-        if (rc != 0) return rc;
-        e = attn::launch_fast_forward(map_x, map_o, out_copy ? &map_copy : nullptr, lse, B, T, H, ds->status, s);
+        CUtensorMap map_x, map_o, map_copy{};
+        if ((rc = encode_planes(&map_x, saved, B, T, 3 * H * D, plane, 64)) != 0) return rc;
+        if ((rc = encode_rows_f32(&map_o, out, B, T, H * D)) != 0) return rc;
+        if (out_copy && (rc = encode_rows_f32(&map_copy, out_copy, B, T, H * D)) != 0) return rc;
+        e = attn::launch_fast_forward(map_x, map_o, map_copy, out, out_copy, lse, B, T, H, ds->status, s);
     } else {
         e = use_attn24(D) ? attn::launch_attn24_forward(qkv, planes_too ? hi : nullptr, lo, out, out_copy, lse, B, T, H, D, ds->status, s)
                           : attn::launch_generic_forward(qkv, out, out_copy, lse, B, T, H, D, s);

@@ -9,7 +9,8 @@
 // addressed straight inside [B, T, 3C] by a 4-D tensor map (column, row, batch, plane).
 //
 // The grid has one CTA per item, heaviest first.  The first Q and K tiles are requested while the CTA is still being set
-// up, the finished tile leaves by the copy engine from where Q was.  A sequence of at most 64 tokens takes one key step.
+// up, the finished tile leaves by the copy engine from where Q was.  A sequence of
+// at most 64 tokens takes one key step, and its rows leave from registers.
 //
 // A CTA is deliberately small (about 100 KiB of shared memory, 256 columns of tensor memory,
 // 384 threads) so that TWO CTAs share an SM.  Inside a CTA two score buffers alternate, so the
@@ -176,60 +177,97 @@ __device__ __forceinline__ void load_k(FwdSmem &sm, const CUtensorMap &map_x, co
     tma_load_4d(sm.k[st][1], &map_x, &sm.k_full[st], C + w.h * kD, j * kStep, w.b, 1);
 }
 
-// Sequences of at most 64 tokens: the (only) item's Q, K and V come from the fp32 tensor, every thread splits its share
-// into the two bf16 planes, in shared memory where the tensor cores read them and in `saved` for the backward.
-// That takes the split kernel, its launch and a second trip through memory out of a pass that is all latency.
-struct Chunks {  // this thread's 32-byte pieces of the 3 x 64 rows
-    static constexpr int kEach = 3 * 8 * kStep / kThreads;
-    static_assert(kEach * kThreads == 3 * 8 * kStep, "every thread has the same number");
-    uint4 hi[kEach], lo[kEach];
-    __device__ static int part(int u) { return ((int)threadIdx.x + u * kThreads) >> 9; }
-    __device__ static int row(int u) { return (((int)threadIdx.x + u * kThreads) >> 3) & 63; }
-    __device__ static int col() { return (int)threadIdx.x & 7; }
-    __device__ static size_t at(int u, int b, int h, int T, int C) {
-        return ((size_t)b * T + row(u)) * 3 * C + part(u) * C + h * kD + 8 * col();
-    }
-};
-__device__ __forceinline__ void take_fp32(FwdSmem &sm, Chunks &x, const float *__restrict__ qkv, int b, int h, int T, int C) {
-    float4 a[Chunks::kEach][2];  // all on their way before the first is used
-    const bool wide = aligned32(qkv);
+// 32 columns of one row, scaled: 32 bytes per store when the pointer allows it.
+__device__ __forceinline__ void store_row(float *dst, const uint32_t (&r)[32], float by) {
+    if (aligned32(dst)) {
 #pragma unroll
-    for (int u = 0; u < Chunks::kEach; u++) {
-        a[u][0] = a[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (Chunks::row(u) < T) load_f32x8(a[u][0], a[u][1], qkv + Chunks::at(u, b, h, T, C), wide);
-    }
+        for (int c = 0; c < 32; c += 8)
+            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + c), "f"(__uint_as_float(r[c]) * by),
+                         "f"(__uint_as_float(r[c + 1]) * by), "f"(__uint_as_float(r[c + 2]) * by), "f"(__uint_as_float(r[c + 3]) * by),
+                         "f"(__uint_as_float(r[c + 4]) * by), "f"(__uint_as_float(r[c + 5]) * by), "f"(__uint_as_float(r[c + 6]) * by),
+                         "f"(__uint_as_float(r[c + 7]) * by)
+                         : "memory");
+    } else {
 #pragma unroll
-    for (int u = 0; u < Chunks::kEach; u++) {
-        split_bf16x2(a[u][0].x, a[u][0].y, x.hi[u].x, x.lo[u].x);
-        split_bf16x2(a[u][0].z, a[u][0].w, x.hi[u].y, x.lo[u].y);
-        split_bf16x2(a[u][1].x, a[u][1].y, x.hi[u].z, x.lo[u].z);
-        split_bf16x2(a[u][1].z, a[u][1].w, x.hi[u].w, x.lo[u].w);
-        const int part = Chunks::part(u), row = Chunks::row(u), at = row * 128 + ((Chunks::col() ^ (row & 7)) << 4);
-        uint8_t *dh = part == 0 ? sm.q[0] : (part == 1 ? sm.k[0][0] : sm.v[0][0]);
-        uint8_t *dl = part == 0 ? sm.q[1] : (part == 1 ? sm.k[0][1] : sm.v[0][1]);
-        *reinterpret_cast<uint4 *>(dh + at) = x.hi[u];
-        *reinterpret_cast<uint4 *>(dl + at) = x.lo[u];
-    }
-    fence_proxy_async_smem();
-}
-// The planes for the backward, once nothing waits for this thread's fence any more.
-__device__ __forceinline__ void save_planes(const Chunks &x, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, int b, int h,
-                                            int T, int C) {
-#pragma unroll
-    for (int u = 0; u < Chunks::kEach; u++) {
-        if (Chunks::row(u) >= T) continue;
-        const size_t at = Chunks::at(u, b, h, T, C);
-        *reinterpret_cast<uint4 *>(hi + at) = x.hi[u];
-        *reinterpret_cast<uint4 *>(lo + at) = x.lo[u];
+        for (int c = 0; c < 32; c += 4)
+            *reinterpret_cast<float4 *>(dst + c) = make_float4(__uint_as_float(r[c]) * by, __uint_as_float(r[c + 1]) * by,
+                                                               __uint_as_float(r[c + 2]) * by, __uint_as_float(r[c + 3]) * by);
     }
 }
 
-template <bool kFp32>
+// Sequences of at most 64 tokens: the (only) item's Q, K and V come from the fp32 tensor, every thread splits its share
+// into the two bf16 planes, in shared memory where the tensor cores read them; two warps with nothing else to do store
+// them from there in `saved` for the backward.
+// That takes the split kernel, its launch and a second trip through memory out of a pass that is all latency.
+__device__ __forceinline__ size_t piece_at(int part, int row, int col, int b, int h, int T, int C) {
+    return ((size_t)b * T + row) * 3 * C + part * C + h * kD + 8 * col;
+}
+__device__ __forceinline__ uint8_t *plane_of(FwdSmem &sm, int part, int lo) {
+    return part == 0 ? sm.q[lo] : (part == 1 ? sm.k[0][lo] : sm.v[0][lo]);
+}
+__device__ __forceinline__ void take_fp32(FwdSmem &sm, const float *__restrict__ qkv, int b, int h, int T, int C) {
+    constexpr int kEach = 3 * 8 * kStep / kThreads;  // 32-byte pieces of the 3 x 64 rows for a thread
+    static_assert(kEach * kThreads == 3 * 8 * kStep, "every thread has the same number");
+    float4 a[kEach][2];  // all on their way before the first is used
+    const bool wide = aligned32(qkv);
+#pragma unroll
+    for (int u = 0; u < kEach; u++) {
+        const int i = (int)threadIdx.x + u * kThreads, part = i >> 9, row = (i >> 3) & 63, c = i & 7;
+        a[u][0] = a[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < T) load_f32x8(a[u][0], a[u][1], qkv + piece_at(part, row, c, b, h, T, C), wide);
+    }
+#pragma unroll
+    for (int u = 0; u < kEach; u++) {
+        const int i = (int)threadIdx.x + u * kThreads, part = i >> 9, row = (i >> 3) & 63, c = i & 7;
+        uint4 vh, vl;
+        split_bf16x2(a[u][0].x, a[u][0].y, vh.x, vl.x);
+        split_bf16x2(a[u][0].z, a[u][0].w, vh.y, vl.y);
+        split_bf16x2(a[u][1].x, a[u][1].y, vh.z, vl.z);
+        split_bf16x2(a[u][1].z, a[u][1].w, vh.w, vl.w);
+        const int at = row * 128 + ((c ^ (row & 7)) << 4);
+        *reinterpret_cast<uint4 *>(plane_of(sm, part, 0) + at) = vh;
+        *reinterpret_cast<uint4 *>(plane_of(sm, part, 1) + at) = vl;
+    }
+    fence_proxy_async_smem();
+}
+// i: 0..63, one of the threads of the two warps.  Stored by every thread, the planes held up the warps that the first product
+// waits for (11 sequences of 50 tokens, 6 heads: 6.07 us, 5.28 this way).
+__device__ __forceinline__ void save_planes(FwdSmem &sm, int i, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, int b,
+                                            int h, int T, int C) {
+    const int c = i & 7;
+#pragma unroll 2
+    for (int row = i >> 3; row < T; row += 8) {
+        const int from = row * 128 + ((c ^ (row & 7)) << 4);
+#pragma unroll
+        for (int part = 0; part < 3; part++) {
+            const size_t at = piece_at(part, row, c, b, h, T, C);
+            *reinterpret_cast<uint4 *>(hi + at) = *reinterpret_cast<const uint4 *>(plane_of(sm, part, 0) + from);
+            *reinterpret_cast<uint4 *>(lo + at) = *reinterpret_cast<const uint4 *>(plane_of(sm, part, 1) + from);
+        }
+    }
+}
+
+// Where an item comes from and goes.  kShort, kFp32: sequences of at most 64 tokens, from the planes or from the fp32
+// tensor; half a tile of rows leaves from registers, since for a CTA with nothing else to do the copy engine is the longer
+// way (B=8 T=42 H=16, core and forward: 5.0 and 6.8 us by the copy engine, 4.6 and 6.1 from registers; B=8 T=128 H=12, core
+// alone, a whole tile: 6.6 and 6.8).
+enum Form : int { kLong, kShort, kFp32 };
+template <int kForm>
+struct Maps {  // no tensor map that the form does not use: a launch carries them all
+    CUtensorMap x, o, copy;
+};
+template <>
+struct Maps<kShort> {
+    CUtensorMap x;
+};
+template <>
+struct Maps<kFp32> {};
+
+template <int kForm>
 __global__ void __launch_bounds__(kThreads, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_o,
-                const __grid_constant__ CUtensorMap map_copy, bool has_copy, const float *__restrict__ qkv,
-                __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo, float *__restrict__ lse, int B, int T, int H,
-                float scale_log2, int *status) {
+attn_fwd_kernel(const __grid_constant__ Maps<kForm> maps, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ hi,
+                __nv_bfloat16 *__restrict__ lo, float *__restrict__ out, float *__restrict__ out_copy, float *__restrict__ lse, int B,
+                int T, int H, float scale_log2, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     FwdSmem &sm = *reinterpret_cast<FwdSmem *>(smem_raw);
     if ((smem_u32(smem_raw) & 1023u) != 0) {
@@ -241,10 +279,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const int C = H * kD;
     WaitCtx ctx{&sm.abort_flag, status};
 
-    if (threadIdx.x == 96) {
-        if (!kFp32) tma_prefetch_desc(&map_x);
-        tma_prefetch_desc(&map_o);
-        if (has_copy) tma_prefetch_desc(&map_copy);
+    if constexpr (kForm == kLong) {
+        if (threadIdx.x == 96) {
+            tma_prefetch_desc(&maps.x);
+            tma_prefetch_desc(&maps.o);
+            if (out_copy) tma_prefetch_desc(&maps.copy);
+        }
     }
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
@@ -265,22 +305,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         fence_barrier_init();
         // This thread is also the Q/K producer: the first Q and K tiles are requested right away, while the other
         // warps are still setting up (but not before the kernel that wrote them has completed).
-        if (!kFp32) {
+        if constexpr (kForm != kFp32) {
             pdl_wait();
             fence_proxy_async_smem();
+            if constexpr (kForm == kShort) tma_prefetch_desc(&maps.x);
             const Item w = decode((int)blockIdx.x, B, T, H);
-            load_q(sm, map_x, w);
-            for (int j = 0; j < min(2, w.nsteps); j++) load_k(sm, map_x, w, C, j, j);
+            load_q(sm, maps.x, w);
+            for (int j = 0; j < min(2, w.nsteps); j++) load_k(sm, maps.x, w, C, j, j);
         }
     }
     if (warp == 1) {
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
     pdl_wait();  // every thread, before its first access to global memory
-    Chunks chunks;
-    if (kFp32) {
+    if (kForm == kFp32) {
         const Item w = decode((int)blockIdx.x, B, T, H);
-        take_fp32(sm, chunks, qkv, w.b, w.h, T, C);
+        take_fp32(sm, qkv, w.b, w.h, T, C);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -288,33 +328,37 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
 
     const Item w = decode((int)blockIdx.x, B, T, H);
-    if (kFp32 && threadIdx.x == 0) {  // what the copy engine signals otherwise
+    if (kForm == kFp32 && threadIdx.x == 0) {  // what the copy engine signals otherwise
         mbar_arrive(&sm.q_full);
         mbar_arrive(&sm.k_full[0]);
         mbar_arrive(&sm.v_full[0]);
     }
-    if (kFp32) save_planes(chunks, hi, lo, w.b, w.h, T, C);
 
-    if (kFp32 && (warp == 0 || warp == 3)) {
-        // no loads to request
+    if (kForm == kFp32 && (warp == 0 || warp == 3)) {
+        // no loads to request; these two leave the planes for the backward
+        save_planes(sm, (warp == 0 ? 0 : 32) + lane, hi, lo, w.b, w.h, T, C);
     } else if (warp == 0) {
         // ------------------------------ TMA producer: K ------------------------------
-        if (lane == 0) {
-            for (int n = 2; n < w.nsteps; n++) {  // Q and the first two steps were requested during set-up
-                if (!mbar_wait(&sm.k_empty[n & 1], ((n >> 1) - 1) & 1, ctx, SITE_K_EMPTY)) break;
-                load_k(sm, map_x, w, C, n, n & 1);
+        if constexpr (kForm != kFp32) {
+            if (lane == 0) {
+                for (int n = 2; n < w.nsteps; n++) {  // Q and the first two steps were requested during set-up
+                    if (!mbar_wait(&sm.k_empty[n & 1], ((n >> 1) - 1) & 1, ctx, SITE_K_EMPTY)) break;
+                    load_k(sm, maps.x, w, C, n, n & 1);
+                }
             }
         }
     } else if (warp == 3) {
         // ------------------------------ TMA producer: V ------------------------------
-        if (lane == 0) {
-            const int xv = 2 * C + w.h * kD;
-            for (int n = 0; n < w.nsteps; n++) {
-                const int st = n & 1;
-                if (n >= 2 && !mbar_wait(&sm.v_empty[st], ((n >> 1) - 1) & 1, ctx, SITE_V_EMPTY)) break;
-                mbar_expect_tx(&sm.v_full[st], 2 * kPlaneStep);
-                tma_load_4d(sm.v[st][0], &map_x, &sm.v_full[st], xv, n * kStep, w.b, 0);
-                tma_load_4d(sm.v[st][1], &map_x, &sm.v_full[st], xv, n * kStep, w.b, 1);
+        if constexpr (kForm != kFp32) {
+            if (lane == 0) {
+                const int xv = 2 * C + w.h * kD;
+                for (int n = 0; n < w.nsteps; n++) {
+                    const int st = n & 1;
+                    if (n >= 2 && !mbar_wait(&sm.v_empty[st], ((n >> 1) - 1) & 1, ctx, SITE_V_EMPTY)) break;
+                    mbar_expect_tx(&sm.v_full[st], 2 * kPlaneStep);
+                    tma_load_4d(sm.v[st][0], &maps.x, &sm.v_full[st], xv, n * kStep, w.b, 0);
+                    tma_load_4d(sm.v[st][1], &maps.x, &sm.v_full[st], xv, n * kStep, w.b, 1);
+                }
             }
         }
     } else if (warp == 2) {
@@ -453,24 +497,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             tc_fence_before_sync();
             const int tok = w.qt * kTile + row;
             if (half == 0 && tok < T) lse[((size_t)w.b * H + w.h) * T + tok] = (m + __log2f(l_all)) * 0.6931471805599453f;
-            // This thread's own row and plane of Q, long in tensor memory, take its 32 columns, and the copy engine takes
-            // them from there (rows past the end are dropped).  Rows written from registers, a row per lane in 32-byte
-            // pieces, took 1640 cycles at the end of every CTA (B=8 T=128 H=12).
-            uint8_t *at = sm.q[half] + row * 128;
+            if constexpr (kForm != kLong) {
+                if (tok < T) {
+                    const size_t at = ((size_t)w.b * T + tok) * C + (size_t)w.h * kD + 32 * half;
+                    store_row(out + at, r, inv);
+                    if (out_copy) store_row(out_copy + at, r, inv);
+                }
+            } else {
+                // This thread's own row and plane of Q, long in tensor memory, take its 32 columns, and the copy engine takes
+                // them from there (rows past the end are dropped).  Rows written from registers, a row per lane in 32-byte
+                // pieces, took 1640 cycles at the end of every CTA (B=8 T=128 H=12).
+                uint8_t *at = sm.q[half] + row * 128;
 #pragma unroll
-            for (int c = 0; c < 8; c++)
-                *reinterpret_cast<float4 *>(at + ((c ^ (row & 7)) << 4)) =
-                    make_float4(__uint_as_float(r[4 * c]) * inv, __uint_as_float(r[4 * c + 1]) * inv, __uint_as_float(r[4 * c + 2]) * inv,
-                                __uint_as_float(r[4 * c + 3]) * inv);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&sm.staged[half]);
-                if (quarter == 0 && mbar_wait(&sm.staged[half], 0, ctx, SITE_STAGED)) {
-                    tma_store_3d(sm.q[half], &map_o, w.h * kD + 32 * half, w.qt * kTile, w.b);
-                    if (has_copy) tma_store_3d(sm.q[half], &map_copy, w.h * kD + 32 * half, w.qt * kTile, w.b);
-                    bulk_commit();
-                    bulk_wait_read_all();  // shared memory stays alive until then
+                for (int c = 0; c < 8; c++)
+                    *reinterpret_cast<float4 *>(at + ((c ^ (row & 7)) << 4)) =
+                        make_float4(__uint_as_float(r[4 * c]) * inv, __uint_as_float(r[4 * c + 1]) * inv, __uint_as_float(r[4 * c + 2]) * inv,
+                                    __uint_as_float(r[4 * c + 3]) * inv);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sm.staged[half]);
+                    if (quarter == 0 && mbar_wait(&sm.staged[half], 0, ctx, SITE_STAGED)) {
+                        tma_store_3d(sm.q[half], &maps.o, w.h * kD + 32 * half, w.qt * kTile, w.b);
+                        if (out_copy) tma_store_3d(sm.q[half], &maps.copy, w.h * kD + 32 * half, w.qt * kTile, w.b);
+                        bulk_commit();
+                        bulk_wait_read_all();  // shared memory stays alive until then
+                    }
                 }
             }
         }
@@ -780,25 +832,29 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 }  // namespace
 
 cudaError_t fast_fwd_set_attributes() {
-    const cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(attn_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem));
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<kLong>, a, (int)sizeof(FwdSmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_fwd_kernel<kShort>, a, (int)sizeof(FwdSmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_fwd_kernel<kFp32>, a, (int)sizeof(FwdSmem));
+    return e;
 }
 
 static const float kScaleLog2 = 0.125f * 1.4426950408889634f;  // 1/sqrt(64) * log2(e)
 
-cudaError_t launch_fast_forward(const CUtensorMap &map_x, const CUtensorMap &map_o, const CUtensorMap *map_copy, float *lse, int B,
-                                int T, int H, int *status, cudaStream_t s) {
-    const int nqt = (T + kTile - 1) / kTile;
-    return launch_after_previous(attn_fwd_kernel<false>, dim3((unsigned)(nqt * B * H)), dim3(kThreads), sizeof(FwdSmem), s, map_x, map_o,
-                                 map_copy ? *map_copy : map_o, map_copy != nullptr, nullptr, nullptr, nullptr, lse, B, T, H, kScaleLog2,
-                                 status);
+cudaError_t launch_fast_forward(const CUtensorMap &map_x, const CUtensorMap &map_o, const CUtensorMap &map_copy, float *out,
+                                float *out_copy, float *lse, int B, int T, int H, int *status, cudaStream_t s) {
+    const dim3 grid((unsigned)((T + kTile - 1) / kTile * B * H));
+    if (T <= kTile / 2)
+        return launch_after_previous(attn_fwd_kernel<kShort>, grid, dim3(kThreads), sizeof(FwdSmem), s, Maps<kShort>{map_x}, nullptr, nullptr,
+                                     nullptr, out, out_copy, lse, B, T, H, kScaleLog2, status);
+    return launch_after_previous(attn_fwd_kernel<kLong>, grid, dim3(kThreads), sizeof(FwdSmem), s, Maps<kLong>{map_x, map_o, map_copy},
+                                 nullptr, nullptr, nullptr, out, out_copy, lse, B, T, H, kScaleLog2, status);
 }
 
-cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, const CUtensorMap &map_o,
-                                     const CUtensorMap *map_copy, float *lse, int B, int T, int H, int *status, cudaStream_t s) {
-    return launch_after_previous(attn_fwd_kernel<true>, dim3((unsigned)(B * H)), dim3(kThreads), sizeof(FwdSmem), s, map_o, map_o,
-                                 map_copy ? *map_copy : map_o, map_copy != nullptr, qkv, hi, lo, lse, B, T, H, kScaleLog2, status);
+cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy, float *lse,
+                                     int B, int T, int H, int *status, cudaStream_t s) {
+    return launch_after_previous(attn_fwd_kernel<kFp32>, dim3((unsigned)(B * H)), dim3(kThreads), sizeof(FwdSmem), s,
+                                 Maps<kFp32>{}, qkv, hi, lo, out, out_copy, lse, B, T, H, kScaleLog2, status);
 }
 
 cudaError_t attn24_fwd_set_attributes() {

@@ -73,12 +73,12 @@ int attn24_backward_pieces(int B, int T, int H, int sms);
 //   map_do: dims { C, T, B, 2 planes}, same box
 cudaError_t fast_fwd_set_attributes();
 cudaError_t fast_bwd_set_attributes();
-// map_o, map_copy (may be null): the fp32 output and its copy, dims {C, T, B}, box {32, 128, 1}, 128-byte swizzle.
-cudaError_t launch_fast_forward(const CUtensorMap &map_x, const CUtensorMap &map_o, const CUtensorMap *map_copy, float *lse, int B,
-                                int T, int H, int *status, cudaStream_t s);
+// map_o, map_copy (used only if out_copy is not null): out and out_copy, dims {C, T, B}, box {32, 128, 1}, 128-byte swizzle.
+cudaError_t launch_fast_forward(const CUtensorMap &map_x, const CUtensorMap &map_o, const CUtensorMap &map_copy, float *out,
+                                float *out_copy, float *lse, int B, int T, int H, int *status, cudaStream_t s);
 // T <= kShortT / 2 only: splits qkv itself (hi, lo receive the planes), in place of launch_split and launch_fast_forward.
-cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, const CUtensorMap &map_o,
-                                     const CUtensorMap *map_copy, float *lse, int B, int T, int H, int *status, cudaStream_t s);
+cudaError_t launch_fast_forward_fp32(const float *qkv, __nv_bfloat16 *hi, __nv_bfloat16 *lo, float *out, float *out_copy, float *lse,
+                                     int B, int T, int H, int *status, cudaStream_t s);
 // T <= kShortT and B * H <= num_sms only: prepares dout itself (everything launch_bwd_prepare leaves in the scratch
 // buffer is written too), in place of launch_bwd_prepare and launch_fast_backward.
 cudaError_t launch_fast_backward_fp32(const CUtensorMap &map_x, const CUtensorMap &map_dx, const float *dout, const float *out,

@@ -118,7 +118,7 @@ extern "C" int attn_sm100_forward_static(const float *qkv, float *out, float *ls
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return (int)cudaErrorInvalidValue;
-    return (int)attn::launch_fast_forward(map_x, map_o, nullptr, lse, B, T, H, st.status, s);
+    return (int)attn::launch_fast_forward(map_x, map_o, map_o, out, nullptr, lse, B, T, H, st.status, s);
 }
 
 
