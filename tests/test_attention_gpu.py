@@ -158,6 +158,28 @@ def test_general_backward_in_one_and_two_pieces(pkg, gpu, oracle, B, T, H, D):
     assert np.abs(together.cpu().numpy() - oracle.backward(x, g, H)).max() < GENERIC_TOL
 
 
+@pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 63, 3), (5, 64, 6), (30, 33, 5), (2, 65, 3)])
+def test_short_forward_from_fp32_and_from_planes_agree(pkg, gpu, B, T, H):
+    """One kernel over the fp32 tensor (few short sequences), the split and the core, and each with and without a copy:
+    the same products in the same order, so the same bits and the same planes."""
+    import torch
+
+    qkv = torch.from_numpy(np.random.default_rng(B + T).standard_normal((B, T, 192 * H)).astype(np.float32)).cuda()
+    results = []
+    for stages in ((0,), (pkg.FLAG_PREPARE_ONLY, pkg.FLAG_CORE_ONLY)):
+        for copy in (False, True):
+            out = torch.full((B, T, 64 * H), float("nan"), device="cuda")
+            out_copy = torch.full_like(out, float("nan")) if copy else None
+            lse = torch.full((B, H, T), float("nan"), device="cuda")
+            saved = torch.zeros(pkg.saved_bytes(B, T, H, 64), device="cuda", dtype=torch.uint8)
+            for flags in stages:
+                pkg.forward_into(qkv, out, out_copy, lse, saved, H, flags=flags)
+            results.append((out, lse, saved) if out_copy is None else (out_copy, lse, saved))
+            assert out_copy is None or torch.equal(out, out_copy)
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+
+
 @pytest.mark.parametrize("T", [1, 40, 64, 65, 128])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_short_sequences_at_any_16_byte_address(pkg, gpu, oracle, T, offset):
