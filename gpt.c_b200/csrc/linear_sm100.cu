@@ -66,7 +66,6 @@ struct Problem {
     int b_shift;            // B's contraction index runs this far behind A's (see RowClass)
     int a_whole[4];         // columns in whole blocks of A's views
     int a_shift[4];         // columns of A's views before the first column of dy (dW from row classes)
-    Chain chain;
     int m_fast;  // consecutive work items walk down the rows of C (else along its columns)
 };
 
@@ -188,7 +187,6 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
         fence_barrier_init();
     }
     if (warp == 2) {
-        if (p.chain == kFirst) pdl_wait();
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
     if (warp == 3 && lane == 0) {
@@ -197,7 +195,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
             tma_prefetch_desc(&maps.b[i]);
         }
     }
-    if (p.chain != kBeside) pdl_wait();  // every thread, before its first access to global memory
+    pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -403,7 +401,6 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
         tc_fence_after_sync();
         tmem_dealloc(tmem, kTmemCols);
     }
-    if (p.chain == kBeside) pdl_wait();
 }
 
 // db[n] += sum_m dy[m, n].  A block covers 128 columns, four per lane, and every 8th row of its share of the rows; the
@@ -411,9 +408,9 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
 // else they are 32 apart and read one by one.
 template <bool kWords>
 __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict__ dy, float *__restrict__ db, int M, int N,
-                                                        int pitch, Chain chain) {
+                                                        int pitch) {
     tc05::pdl_launch_dependents();
-    if (chain != kBeside) tc05::pdl_wait();
+    tc05::pdl_wait();
     __shared__ float4 part[8][32];
     const int lane = threadIdx.x & 31, rl = threadIdx.x >> 5;
     constexpr int kApart = kWords ? 1 : 32;
@@ -449,14 +446,13 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict_
         if (kWords && col + 3 < N && (reinterpret_cast<uintptr_t>(db + col) & 15u) == 0) {
             asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(db + col), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w)
                          : "memory");
-        } else {
-            atomicAdd(db + col, t.x);
-            if (col + kApart < N) atomicAdd(db + col + kApart, t.y);
-            if (col + 2 * kApart < N) atomicAdd(db + col + 2 * kApart, t.z);
-            if (col + 3 * kApart < N) atomicAdd(db + col + 3 * kApart, t.w);
+            return;
         }
+        atomicAdd(db + col, t.x);
+        if (col + kApart < N) atomicAdd(db + col + kApart, t.y);
+        if (col + 2 * kApart < N) atomicAdd(db + col + 2 * kApart, t.z);
+        if (col + 3 * kApart < N) atomicAdd(db + col + 3 * kApart, t.w);
     }
-    if (chain == kBeside) tc05::pdl_wait();
 }
 
 // dst[M, Np] = src[M, N] with zero columns N..Np-1: a copy of dy whose rows start on 16-byte boundaries, for
@@ -528,7 +524,6 @@ Problem make_problem(int M, int N, int K, int bn, int splits) {
     p.M = M, p.N = N, p.K = K, p.bn = bn;
     p.a_one = p.b_one = 0;
     p.m_fast = 0;
-    p.chain = kAlone;
     p.ldc = (size_t)N;
     p.b_shift = 0;
     for (int i = 0; i < 4; i++) p.a_shift[i] = p.a_whole[i] = 0;
@@ -737,8 +732,7 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
 }
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
-int input_gradient(const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, Chain chain, int *status,
-                   cudaStream_t s) {
+int input_gradient(const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status, cudaStream_t s) {
     const int kb = np / kBK;
     Plan plan = plan_tiles(M, K, kb, sms);
     // Pieces of the contraction may fill the SMs better, although dx has to be zeroed first.  Any number where it is very long
@@ -750,10 +744,9 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
     cut.ns += 2500 + (int)((long long)M * K * 4 / 5500);
     if (cut.splits > 1 && (very_long ? cut.ns : at_most_int(cut.ns * 21ll / 20)) < plan.ns) plan = cut;
     int split = 1, rc;
-    if (plan_split(M, K, np, sms, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, sms, chain, status, s);
+    if (plan_split(M, K, np, sms, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, sms, status, s);
     CUtensorMap ma, mb, mc;
     Problem p = make_problem(M, K, np, plan.bn, plan.splits);
-    p.chain = chain;
     if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
     p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32) == 0;
     if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
@@ -787,7 +780,7 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     const Plan plan = plan_tiles(M, N, (K + kBK - 1) / kBK, sms);
     int split = 1;
     if (plan_split(M, N, K, sms, &split) < plan.ns)
-        return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, sms, kAlone, status, s);
+        return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, sms, status, s);
     CUtensorMap ma, mb;
     // with plain stores (N not a multiple of 4) only the widest tiles are built
     Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, 1);
@@ -836,19 +829,13 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         if (rc != 0) return rc;
         g = static_cast<const float *>(scratch);
     }
-    Chain chain = classes ? kAlone : kFirst;
-    if (!classes && dx) {
-        if ((rc = input_gradient(g, w, dx, M, N, np, K, sms, dw || db ? kFirst : kAlone, status, s)) != 0) return rc;
-        chain = kBeside;
-    }
+    if (!classes && dx && (rc = input_gradient(g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
     CUtensorMap ma, mb, mc;
     if (!classes && dw) {
         // dw[N,K] += dy[M,N]^T . x[M,K]: contraction over M, split so that every SM has work (rows of the
         // result past N are dropped by the copy engine)
         const Plan plan = plan_pieces(N, K, (M + kBK - 1) / kBK, sms, 1);
         Problem pdw = make_problem(N, K, M, plan.bn, plan.splits);
-        pdw.chain = chain == kFirst && !db ? kAlone : chain;
-        chain = kBeside;
         pdw.a_one = map_mn_major_blocks(&ma, g, M, np, 4) == 0;
         if (!pdw.a_one && (rc = map_mn_major(&ma, g, M, np)) != 0) return rc;
         pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32) == 0;
@@ -863,7 +850,7 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         const int across = (N + 127) / 128, fill = 8 * sms / across, by = (M + 31) / 32 < fill ? (M + 31) / 32 : (fill > 1 ? fill : 1);
         dim3 grid((unsigned)((N + 127) / 128), (unsigned)by);
         rc = (int)attn::launch_after_previous(classes ? bias_grad_kernel<false> : bias_grad_kernel<true>, grid, dim3(256), 0, s, g,
-                                              db, M, N, classes ? N : np, chain);
+                                              db, M, N, classes ? N : np);
     }
     return rc;
 }

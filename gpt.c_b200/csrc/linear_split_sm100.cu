@@ -43,7 +43,6 @@ struct Params {
     int tiles_m, split, kb_total, kb_per_split;
     int stages, tmem_cols;
     int w_one;         // MN-major weight tile fetched with one 3-D copy per stage
-    int first;         // Chain
     size_t plane_elems;
 };
 
@@ -88,7 +87,6 @@ __global__ void __launch_bounds__(Roles<kSplit>::kThreads, Roles<kSplit>::kPerSm
         fence_barrier_init();
     }
     if (warp == kWarpMma) {
-        if (p.first) pdl_wait();
         tmem_alloc_then_launch_dependents(&ct.tmem_base, p.tmem_cols);
     }
     if (warp == kWarpTma && lane == 0) {
@@ -275,7 +273,7 @@ int plan_split(int M, int cols, int kc, int sms, int *split) {
 }
 
 int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, const float *bias, float *out, void *planes, int M,
-                 int cols, int kc, int split, int sms, Chain chain, int *status, cudaStream_t s) {
+                 int cols, int kc, int split, int sms, int *status, cudaStream_t s) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -293,7 +291,6 @@ int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, 
     }
     Params p;
     p.M = M, p.cols = cols;
-    p.first = chain == kFirst;
     p.bm = rows_per_tile(M);
     p.tiles_m = (M + p.bm - 1) / p.bm;
     p.kb_total = (kc + kBK - 1) / kBK;

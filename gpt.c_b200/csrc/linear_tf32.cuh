@@ -74,19 +74,11 @@ inline int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows, s
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
 }
-// How a kernel of the backward stands to the one before it in the stream.  dx, dW and db read the same tensors and none
-// reads what another writes, so they may run at the same time.  For that the first of them lets the next one start only
-// after its own wait for the kernel before (whose results are complete then, for everybody); the others do not wait at
-// their start but at their end, so that the last one's completion means the completion of all.  On small layers, where each
-// kernel is a chain of latencies, the three then take little longer than one; on large ones the SMs that a kernel's last
-// round leaves idle go on with the next kernel.
-enum Chain : int { kAlone, kFirst, kBeside };
-
 // The kernel for results of few tiles (linear_split_sm100.cu): out[M, cols] = act[M, kc] . w^T + bias, with w [cols, kc],
 // or with w_mn_major [w_rows, cols] (its rows past w_rows, up to kc, read as zeros); optionally the bf16 planes of out.
 // `split` CTAs share the contraction of a tile.  Returns ATTN_OK or an error.
 int launch_split(const float *act, const float *w, bool w_mn_major, int w_rows, const float *bias, float *out, void *planes, int M,
-                 int cols, int kc, int split, int sms, Chain chain, int *status, cudaStream_t s);
+                 int cols, int kc, int split, int sms, int *status, cudaStream_t s);
 // The best `split` and the time in nanoseconds it is expected to take.
 int plan_split(int M, int cols, int kc, int sms, int *split);
 

@@ -1,41 +1,35 @@
-"""Tensor memory and programmatic dependent launch, checked in the sources.
-
-A CTA that allocates tensor memory waits until its SM has the columns.  If the kernel were to let the next one start
-before that (any one thread's griddepcontrol.launch_dependents counts for its CTA), a CTA of the next kernel could take
-the columns and then wait for this kernel to complete, which waits for the columns: neither ends.  Such a stop cannot be
-tested by running it, so the order is checked where it is written down."""
+"""Kernels that may start before the previous one of their stream has completed: what they read is only visible to a kernel
+that has waited for it itself, so each of them waits, whatever its arguments.  Read from the sources: a kernel that does not
+is a race on memory, which a run may or may not show."""
 import glob
 import os
 import re
 
+import pytest
+
 CSRC = os.path.join(os.path.dirname(__file__), "..", "gpt.c_b200", "csrc")
-
-
-def code(path):
-    text = open(path).read()
-    return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
+WAIT = re.compile(r"^    (?:tc05::)?pdl_wait\(\);", re.M)  # a statement of the kernel's own block, under no condition
+START = re.compile(r"pdl_launch_dependents\(\)|tmem_alloc_then_launch_dependents\(")
 
 
 def kernels():
-    """(file, text from one __global__ to the next) of every kernel."""
+    """(name, body) of every kernel that lets the next one of the stream start early, or is launched that way itself."""
+    found = []
     for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
-        for body in re.split(r"\b__global__\b", code(path))[1:]:
-            yield os.path.basename(path), body
+        text = open(path).read()
+        for m in re.finditer(r"__global__.*?\b(\w+_kernel)\(", text, re.S):
+            name, body = m.group(1), text[m.end():text.index("\n}\n", m.end())]
+            if START.search(body) or re.search(r"launch_\w*after_previous\([^;]*\b%s\b" % name, text):
+                found.append((name, body))
+    return found
 
 
-def test_next_kernel_is_let_start_by_the_thread_that_has_allocated():
-    allocating = [(f, body) for f, body in kernels() if re.search(r"\btmem_alloc", body)]
-    assert {f for f, _ in allocating} == {"attn_fwd_sm100.cu", "attn_bwd_sm100.cu", "linear_sm100.cu", "linear_split_sm100.cu"}
-    for f, body in allocating:
-        assert len(re.findall(r"\btmem_alloc_then_launch_dependents\(", body)) == 1, f
-        assert not re.search(r"launch_dependents\(|launch_dependents;", body.replace("tmem_alloc_then_launch_dependents(", "")), \
-            f"{f}: the next kernel is let start by something else than the allocation"
+def test_kernels_are_found():
+    names = [n for n, _ in kernels()]
+    assert {"linear_gemm_kernel", "linear_split_kernel", "bias_grad_kernel", "attn_fwd_kernel", "attn_bwd_kernel",
+            "attn24_fwd_kernel", "attn24_bwd_kernel", "split_kernel", "ln_forward_kernel"} <= set(names)
 
 
-def test_allocation_comes_before_the_signal():
-    headers = {os.path.basename(p): code(p) for p in glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.cu"))}
-    assert [f for f, text in sorted(headers.items()) if "tcgen05.alloc" in text] == ["tc05.cuh"]
-    text = headers["tc05.cuh"]
-    body = text[text.index("tmem_alloc_then_launch_dependents("):]
-    body = body[:body.index("\n}")]
-    assert text.count("tcgen05.alloc") == 1 and 0 < body.index("tcgen05.alloc") < body.index("pdl_launch_dependents();")
+@pytest.mark.parametrize("name,body", kernels(), ids=lambda v: v if len(v) < 64 else "")
+def test_kernel_waits_for_the_one_before_it(name, body):
+    assert WAIT.search(body), f"{name} can read what the previous kernel of the stream wrote without having waited for it"

@@ -199,7 +199,7 @@ def test_linear_backward_parts_can_be_skipped(pkg):
 @pytest.mark.parametrize("M,N,K", [(16, 96, 64), (37, 768, 768), (300, 2304, 768), (2048, 768, 768), (9, 16415, 32)])
 @pytest.mark.parametrize("want_dx,want_dw,want_db", [(True, True, True), (True, True, False), (True, False, True), (False, True, True)])
 def test_linear_backward_kernels_beside_each_other(pkg, M, N, K, want_dx, want_dw, want_db):
-    """dx, dW and db may run at the same time, but neither before what wrote dy, x and w nor after what reads the results:
+    """dx, dW and db read the same tensors, none of them before what wrote dy, x and w nor after what reads the results:
     back to back, with every input written by the kernel before and every result read by the kernel behind.  Small and
     large tiles, clusters, pieces that add into zeros, a padded copy."""
     L = pkg.lib()
