@@ -9,8 +9,8 @@
 // addressed straight inside [B, T, 3C] by a 4-D tensor map (column, row, batch, plane).
 //
 // The grid has one CTA per item, heaviest first.  The first Q and K tiles are requested while the CTA is still being set
-// up, the finished tile leaves by the copy engine from where Q was.  A sequence of
-// at most 64 tokens takes one key step, and its rows leave from registers.
+// up, the finished tile leaves by the copy engine from where Q was, or straight from registers where that is sooner.
+// A sequence of at most 64 tokens takes one key step.
 //
 // A CTA is deliberately small (about 100 KiB of shared memory, 256 columns of tensor memory,
 // 384 threads) so that TWO CTAs share an SM.  Inside a CTA two score buffers alternate, so the
@@ -247,17 +247,16 @@ __device__ __forceinline__ void save_planes(FwdSmem &sm, int i, __nv_bfloat16 *_
     }
 }
 
-// Where an item comes from and goes.  kShort, kFp32: sequences of at most 64 tokens, from the planes or from the fp32
-// tensor; half a tile of rows leaves from registers, since for a CTA with nothing else to do the copy engine is the longer
-// way (B=8 T=42 H=16, core and forward: 5.0 and 6.8 us by the copy engine, 4.6 and 6.1 from registers; B=8 T=128 H=12, core
-// alone, a whole tile: 6.6 and 6.8).
-enum Form : int { kLong, kShort, kFp32 };
+// Where an item comes from and goes.  kLong: the result leaves by the copy engine.  kRows: from registers, which is the
+// shorter way for a CTA that stores part of a tile, once, and has its SM to itself (rows_from_registers).  kFp32: the same,
+// and the item comes from the fp32 tensor (sequences of at most 64 tokens).
+enum Form : int { kLong, kRows, kFp32 };
 template <int kForm>
 struct Maps {  // no tensor map that the form does not use: a launch carries them all
     CUtensorMap x, o, copy;
 };
 template <>
-struct Maps<kShort> {
+struct Maps<kRows> {
     CUtensorMap x;
 };
 template <>
@@ -308,7 +307,7 @@ attn_fwd_kernel(const __grid_constant__ Maps<kForm> maps, const float *__restric
         if constexpr (kForm != kFp32) {
             pdl_wait();
             fence_proxy_async_smem();
-            if constexpr (kForm == kShort) tma_prefetch_desc(&maps.x);
+            if constexpr (kForm == kRows) tma_prefetch_desc(&maps.x);
             const Item w = decode((int)blockIdx.x, B, T, H);
             load_q(sm, maps.x, w);
             for (int j = 0; j < min(2, w.nsteps); j++) load_k(sm, maps.x, w, C, j, j);
@@ -834,18 +833,32 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 cudaError_t fast_fwd_set_attributes() {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<kLong>, a, (int)sizeof(FwdSmem));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_fwd_kernel<kShort>, a, (int)sizeof(FwdSmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_fwd_kernel<kRows>, a, (int)sizeof(FwdSmem));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_fwd_kernel<kFp32>, a, (int)sizeof(FwdSmem));
     return e;
 }
 
 static const float kScaleLog2 = 0.125f * 1.4426950408889634f;  // 1/sqrt(64) * log2(e)
 
+// Whether the result leaves from registers.  The last to end are the CTAs of the last query tile; where that tile has at most
+// 96 rows, they are stored once and no second CTA on the SM covers the way through shared memory, barrier and copy engine, the
+// rows are sooner out of registers.  Up to 64 tokens they are in any case.  Forward in us, copy engine / registers, without a
+// copy of the result:
+//     B=1 H=4:  T=65 6.7 / 6.3, 96 6.55 / 6.2, 120 7.1 / 6.9, 130 7.1 / 6.65, 192 7.2 / 6.8, 256 8.4 / 8.25, 448 10.5 / 10.2
+//     B=1 H=12: T=700 15.1 / 14.8, 832 16.9 / 16.6, 960 18.8 / 18.4, 1088 20.7 / 20.3
+//     B=6 H=12: T=96 9.45 / 9.4, 127 8.4 / 8.4, 192 9.5 / 9.3, 256 11.3 / 11.4
+// with two CTAs on an SM (T, H=12): B=16 96 11.0 / 11.25, 127 12.2 / 12.7, B=8 130 10.6 / 10.65, 256 13.5 / 13.7; with a copy,
+// core alone: B=3 T=100 H=8 6.6 / 6.7, B=6 T=192 H=12 8.15 / 8.2, B=8 T=128 H=12 7.5 / 8.6.
+static bool rows_from_registers(int T, long long items, bool copied) {
+    return T <= kTile / 2 || (!copied && T % kTile > 0 && T % kTile <= 96 && items <= sm_count());
+}
+
 cudaError_t launch_fast_forward(const CUtensorMap &map_x, const CUtensorMap &map_o, const CUtensorMap &map_copy, float *out,
                                 float *out_copy, float *lse, int B, int T, int H, int *status, cudaStream_t s) {
-    const dim3 grid((unsigned)((T + kTile - 1) / kTile * B * H));
-    if (T <= kTile / 2)
-        return launch_after_previous(attn_fwd_kernel<kShort>, grid, dim3(kThreads), sizeof(FwdSmem), s, Maps<kShort>{map_x}, nullptr, nullptr,
+    const long long items = (long long)((T + kTile - 1) / kTile) * B * H;
+    const dim3 grid((unsigned)items);
+    if (rows_from_registers(T, items, out_copy != nullptr))
+        return launch_after_previous(attn_fwd_kernel<kRows>, grid, dim3(kThreads), sizeof(FwdSmem), s, Maps<kRows>{map_x}, nullptr, nullptr,
                                      nullptr, out, out_copy, lse, B, T, H, kScaleLog2, status);
     return launch_after_previous(attn_fwd_kernel<kLong>, grid, dim3(kThreads), sizeof(FwdSmem), s, Maps<kLong>{map_x, map_o, map_copy},
                                  nullptr, nullptr, nullptr, out, out_copy, lse, B, T, H, kScaleLog2, status);

@@ -180,6 +180,27 @@ def test_short_forward_from_fp32_and_from_planes_agree(pkg, gpu, B, T, H):
         assert all(torch.equal(a, b) for a, b in zip(results[0], other))
 
 
+@pytest.mark.parametrize("B,T,H", [(1, 65, 1), (2, 96, 3), (2, 97, 3), (74, 70, 2), (75, 70, 2), (3, 130, 5), (2, 224, 4), (2, 225, 4),
+                                   (1, 700, 3)])
+def test_rows_from_registers_and_by_the_copy_engine_agree(pkg, gpu, B, T, H):
+    """Without a copy of the result the rows of a partial last tile leave from registers while every tile has its SM to itself
+    (148 of them), with one by the copy engine: the same bits, and no others are written."""
+    torch = gpu
+    qkv = torch.from_numpy(seeded(43 + T, B, T, H, 64)[0]).cuda()
+    saved = torch.empty(pkg.saved_bytes(B, T, H, 64), device="cuda", dtype=torch.uint8)
+    n, results = B * T * H * 64, []
+    for copy in (False, True):
+        buf = torch.full((n + 16384,), 1234.5, device="cuda")
+        out, lse = buf[8192:8192 + n].view(B, T, H * 64), torch.full((B, H, T), float("nan"), device="cuda")
+        out_copy = torch.full_like(out, float("nan")) if copy else None
+        pkg.forward_into(qkv, out, out_copy, lse, saved, H)
+        assert pkg.device_status() == 0
+        assert out_copy is None or torch.equal(out, out_copy)
+        results.append((buf, lse))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    assert bool((results[0][0][:8192] == 1234.5).all()) and bool((results[0][0][8192 + n:] == 1234.5).all())
+
+
 @pytest.mark.parametrize("T", [1, 40, 64, 65, 128])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_short_sequences_at_any_16_byte_address(pkg, gpu, oracle, T, offset):
