@@ -45,7 +45,9 @@ __device__ __forceinline__ float ex2f(float x) {
 }
 
 // p = hi + mid + lo for both halves: hi rounded, mid the next eight bits cut off, lo what is left.  The rounding is an
-// integer addition: conversions share the quarter-rate pipe with exp2.  (A NaN may leave hi, but not mid.)
+// integer addition: conversions share the quarter-rate pipe with exp2.  What is not finite stays so in one of the terms, but
+// not what it was: an infinity leaves inf and NaN (inf - inf), a finite value above 3.396e38 rounds up to inf, a NaN may leave
+// hi, but not mid.  Products with them are NaN, and whoever uses this looks for that.
 __device__ __forceinline__ void split3(float2 p, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
     const float2 minus = make_float2(-1.f, -1.f);
     const uint32_t a = __float_as_uint(p.x) + 0x8000u, b = __float_as_uint(p.y) + 0x8000u;

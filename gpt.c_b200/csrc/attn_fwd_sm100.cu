@@ -563,9 +563,87 @@ struct __align__(1024) Fwd24Smem {
     uint64_t raw_full[2], raw_free[2];
     uint64_t go_s, go_pv, done_s, done_pv;
     float part[2][4][kTile];  // [step parity][column quarter][row]: row maxima, at the end row sums
+    uint32_t odd[4][4];       // [column quarter][row / 32]: a bit per row of a result that is not finite
     uint32_t tmem_base;
     int abort_flag;
 };
+
+// The rows of this CTA's tile that are marked in `odd`, over again in fp32 arithmetic, a warp per row: a term of an infinite
+// operand, or of a finite one that rounds up to infinity, is not a number, and so is the product of its infinite term with a
+// zero term of the other operand.  A row that stays NaN ends at the first score that decides it, so NaN in every input costs
+// next to nothing.  A function of its own, behind the last barrier: inlined, or called from the workers' branch, it made the
+// loop over the keys up to 10 % slower.
+__device__ __noinline__ void exact_rows(const uint32_t (&odd)[4][4], const float *__restrict__ qkv, float *__restrict__ out,
+                                        float *__restrict__ out_copy, float *__restrict__ lse, int T, int H, int D, float scale) {
+    constexpr int kE = attn::kAttn24MaxD / 32, kAhead = 4;  // columns of a lane, keys whose loads are on their way together
+    if (threadIdx.x == 0) bulk_wait_all();  // the copy engine has written the tile
+    __syncthreads();
+    const int nq = (T + kTile - 1) / kTile, nbh = (int)gridDim.x / nq;
+    const int q0 = (nq - 1 - (int)blockIdx.x / nbh) * kTile, bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H, C = H * D;
+    const size_t C3 = 3 * (size_t)C;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float *head = qkv + (size_t)b * T * C3 + (size_t)h * D, *k_rows = head + C, *v_rows = head + 2 * C;
+#pragma unroll 1
+    for (int r = warp; r < kTile; r += attn24::kThreads / 32) {
+        if (!((odd[0][r >> 5] | odd[1][r >> 5] | odd[2][r >> 5] | odd[3][r >> 5]) >> (r & 31) & 1u)) continue;
+        const int t = q0 + r;
+        float q[kE], acc[kE];
+#pragma unroll
+        for (int e = 0; e < kE; e++) {
+            q[e] = lane + 32 * e < D ? __ldg(head + (size_t)t * C3 + lane + 32 * e) : 0.f;
+            acc[e] = 0.f;
+        }
+        auto scores = [&](int j0, float (&s)[kAhead]) {  // of keys j0 on; -inf past the diagonal
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                s[u] = 0.f;
+#pragma unroll
+                for (int e = 0; e < kE; e++)
+                    if (j0 + u <= t && lane + 32 * e < D) s[u] = fmaf(q[e], __ldg(k_rows + (size_t)(j0 + u) * C3 + lane + 32 * e), s[u]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) s[u] = j0 + u <= t ? s[u] * scale : -INFINITY;
+        };
+        float m = -INFINITY, l = 0.f, s[kAhead];
+        bool is_nan = false;
+#pragma unroll 1
+        for (int j = 0; j <= t && !is_nan; j += kAhead) {
+            scores(j, s);
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                is_nan = is_nan || !(s[u] < INFINITY);  // an infinite maximum is subtracted from itself
+                m = fmaxf(m, s[u]);
+            }
+        }
+        const float minus = m == -INFINITY ? 0.f : m;
+#pragma unroll 1
+        for (int j = 0; j <= t && !is_nan; j += kAhead) {
+            scores(j, s);
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                if (j + u > t) break;
+                const float p = expf(s[u] - minus);
+                l += p;
+#pragma unroll
+                for (int e = 0; e < kE; e++)
+                    if (lane + 32 * e < D) acc[e] = fmaf(p, __ldg(v_rows + (size_t)(j + u) * C3 + lane + 32 * e), acc[e]);
+            }
+        }
+        const float by = is_nan ? NAN : 1.0f / l;
+        const size_t at = ((size_t)b * T + t) * C + (size_t)h * D;
+#pragma unroll
+        for (int e = 0; e < kE; e++) {
+            if (lane + 32 * e >= D) break;
+            out[at + lane + 32 * e] = acc[e] * by;
+            if (out_copy) out_copy[at + lane + 32 * e] = acc[e] * by;
+        }
+        if (lane == 0) lse[(size_t)bh * T + t] = is_nan ? NAN : m + logf(l);
+    }
+}
 
 enum Site24 : int { SITE24_GO_S = 301, SITE24_GO_PV, SITE24_S, SITE24_PV, SITE24_RAW_FREE, SITE24_RAW_FULL, SITE24_SMEM_ALIGN };
 
@@ -576,7 +654,7 @@ __global__ void __launch_bounds__(attn24::kThreads, 1)
 attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_o,
                   const __grid_constant__ CUtensorMap map_copy, const float *__restrict__ qkv, __nv_bfloat16 *__restrict__ xhi,
                   __nv_bfloat16 *__restrict__ xlo, float *__restrict__ out, float *__restrict__ out_copy, float *__restrict__ lse,
-                  int T, int H, int D, Scale scale_log2, int *status) {
+                  int T, int H, int D, float scale, Scale scale_log2, int *status) {
     using Smem = Fwd24Smem<kK>;
     constexpr int kPlane = Smem::kPlane, kBlocks = Smem::kBlocks;
     constexpr uint32_t kColS = 0, kColO = 192, kColQ = 192 + 16 * kK;  // S (96 columns) twice; P takes its place
@@ -616,6 +694,7 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int C = H * D, nsteps = (min(q0 + kTile, T) + kStep - 1) / kStep;
     const size_t C3 = 3 * (size_t)C;
     const float *head = qkv + (size_t)b * T * C3 + (size_t)h * D;
+    int odd = 0;  // whether this thread has a value of the result that is not finite
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -786,6 +865,14 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         add_columns<kK>(o, t_o, alpha_before);
         const int t = q0 + row;
         const float inv = 1.0f / l;
+        {
+            float zero[4] = {m * 0.f, 0.f, 0.f, 0.f};  // what is finite times zero is zero
+#pragma unroll
+            for (int i = 0; i < 4 * kK; i++) zero[i & 3] = fmaf(o[i] * inv, 0.f, zero[i & 3]);
+            odd = t < T && !((zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.f);
+            const uint32_t rows = __ballot_sync(0xffffffffu, odd);
+            if (lane == 0) sm.odd[cq][quarter] = rows;
+        }
         if (kTma) {
             // by the copy engine, from the place of the raw K and V: groups of 16 columns, 128 rows of 64 bytes, swizzled
             uint8_t *stage = reinterpret_cast<uint8_t *>(sm.raw[0]);
@@ -819,11 +906,12 @@ attn24_fwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     if (sm.abort_flag) __nanosleep(50000);  // let copies and products that are still in flight end
     tc_fence_before_sync();
-    __syncthreads();
+    const int again = __syncthreads_or(odd);
     if (warp == kWorkWarps) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, kCols);
     }
+    if (again) exact_rows(sm.odd, qkv, out, out_copy, lse, T, H, D, scale);
 }
 
 }  // namespace general
@@ -899,7 +987,7 @@ cudaError_t launch_attn24_forward(const float *qkv, __nv_bfloat16 *hi, __nv_bflo
         const dim3 grid((unsigned)((size_t)B * H * ((T + kTile - 1) / kTile)));
         return launch_after_previous(tma ? general::attn24_fwd_kernel<kK, true> : general::attn24_fwd_kernel<kK, false>, grid,
                                      dim3(attn24::kThreads), sizeof(general::Fwd24Smem<kK>), s, map_x, map_o, map_copy, qkv, hi, lo,
-                                     out, out_copy, lse, T, H, D, attn24::log2_scale(D), status);
+                                     out, out_copy, lse, T, H, D, 1.0f / sqrtf((float)D), attn24::log2_scale(D), status);
     });
 }
 

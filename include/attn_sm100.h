@@ -44,6 +44,12 @@
  * product is evaluated as hi*hi + hi*lo + lo*hi on the tensor cores with fp32 accumulation;
  * softmax statistics are fp32.  Head sizes other than 64 take general kernels with fp32 operands (the
  * backward reads q, k, v as the two saved planes).
+ *
+ * Values that are not finite: the general forward gives what fp32 arithmetic gives (a score of -inf has no
+ * weight, an infinite v is infinite in every row that gives it weight), and up to head size 128 rows that
+ * do not see such a value are unaffected (above, rows of the same tile of keys may be).  Two bf16 terms
+ * have no infinities: where head size is 64, and in the planes the backward reads, an infinite value, or
+ * a finite one above 3.396e38, makes NaN of what it enters.
  */
 #ifndef ATTN_SM100_H
 #define ATTN_SM100_H

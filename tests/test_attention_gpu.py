@@ -119,6 +119,69 @@ def test_general_tensor_core_kernels_are_fp32_and_repeatable(pkg, gpu, oracle, T
         assert np.array_equal(d.cpu().numpy()[..., 2 * D:], dx[..., 2 * D:])
 
 
+def causal_forward_f64(x, H):
+    """out, lse of the definition in 64 bits, row by row over the keys a row sees: what is not finite goes where it goes."""
+    B, T, C3 = x.shape
+    D = C3 // 3 // H
+    q, k, v = (x.astype(np.float64).reshape(B, T, 3, H, D)[:, :, i] for i in range(3))
+    out, lse = np.empty((B, T, H, D)), np.empty((B, H, T))
+    with np.errstate(invalid="ignore", over="ignore"):
+        for b in range(B):
+            for h in range(H):
+                for t in range(T):
+                    s = (k[b, :t + 1, h] * q[b, t, h]).sum(1) / np.sqrt(D)
+                    e = np.exp(s - s.max())
+                    out[b, t, h] = (e[:, None] / e.sum() * v[b, :t + 1, h]).sum(0)
+                    lse[b, h, t] = -np.inf if s.max() == -np.inf else s.max() + np.log(e.sum())
+    return out.reshape(B, T, H * D), lse
+
+
+def same_but_for_rounding(got, ref, rel):
+    """NaN and infinities in the same places, the rest to `rel` of the larger of a value and one (of the typical value)."""
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    assert np.array_equal(np.isinf(got), np.isinf(ref))
+    assert np.array_equal(np.sign(got[np.isinf(ref)]), np.sign(ref[np.isinf(ref)]))
+    finite = np.isfinite(ref)
+    assert (np.abs(got[finite] - ref[finite]) <= rel * np.maximum(np.abs(ref[finite]), 1.0)).all()
+
+
+@pytest.mark.parametrize("T,D", [(1, 16), (70, 3), (130, 20), (150, 64), (140, 67), (200, 128)])
+@pytest.mark.parametrize("what", ["all scores -inf", "score -inf", "score +inf", "v inf", "v nan", "v large", "q large", "all nan"])
+def test_general_forward_of_infinities_and_the_largest_values(pkg, gpu, T, D, what):
+    """Operands in three bf16 terms have neither infinities nor the values that round up to one: such rows are what fp32
+    arithmetic makes of them, and no other row changes.  (1e-5: sums of up to 200 terms of up to five, each rounded once.)"""
+    torch, H, at = gpu, 2, T // 3
+    x, _ = seeded(47 + T + D, 2, T, H, D)
+    q, k, v = (x.reshape(2, T, 3, H, D)[:, :, i] for i in range(3))
+    if what == "all scores -inf":
+        k[0, :, 1, 0] = np.abs(k[0, :, 1, 0]) + 0.125
+        q[0, at, 1, 0] = -np.inf
+    elif what == "score -inf":
+        q[1, :, 0, D - 1] = np.abs(q[1, :, 0, D - 1]) + 0.125
+        k[1, at, 0, D - 1] = -np.inf
+    elif what == "score +inf":
+        q[0, at, 0, 0], k[0, :, 0, 0] = np.inf, np.abs(k[0, :, 0, 0]) + 0.125
+    elif what == "v inf":
+        v[0, at, 0, 0], v[1, 0, 1, D - 1] = np.inf, -np.inf
+    elif what == "v nan":
+        v[1, at, 1, D // 2] = np.nan
+    elif what == "v large":  # finite, rounds up to infinity in bf16
+        v[0, at, 1, 0], v[1, at, 0, D - 1] = 3.4028e38, -3.3999e38
+    elif what == "q large":  # scores of more than 1e37, all but one of them negative
+        k[0, :, 1, 0] = -np.abs(k[0, :, 1, 0]) - 0.125
+        k[0, 0, 1, 0] = 0.0
+        q[0, at:, 1, 0] = 3.4e38
+    else:
+        x[...] = np.nan
+    out, ctx = pkg.forward(torch.from_numpy(x).cuda(), H, flags=pkg.FLAG_FORCE_GENERIC, keep_copy=True)
+    assert pkg.device_status() == 0
+    assert torch.equal(out.view(torch.int32), ctx.out.view(torch.int32))
+    out, lse = out.cpu().numpy(), ctx.lse.cpu().numpy()
+    ref_out, ref_lse = causal_forward_f64(x, H)
+    same_but_for_rounding(out, ref_out, 1e-5)
+    same_but_for_rounding(lse, ref_lse, 1e-5)
+
+
 @pytest.mark.parametrize("T,D", [(1, 3), (70, 20), (128, 48), (200, 40), (193, 128), (257, 72)])
 def test_general_forward_leaves_the_planes_of_the_split(pkg, gpu, T, D):
     """Bit for bit what the split alone writes, whatever the alignment of the rows, and a core-only call leaves them alone."""
