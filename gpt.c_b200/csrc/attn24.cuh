@@ -47,10 +47,10 @@ __device__ __forceinline__ float ex2f(float x) {
 // p = hi + mid + lo for both halves: hi rounded, mid the next eight bits cut off, lo what is left.  The rounding is an
 // integer addition: conversions share the quarter-rate pipe with exp2.  What is not finite stays so in one of the terms, but
 // not what it was: an infinity leaves inf and NaN (inf - inf), a finite value above 3.396e38 rounds up to inf, a NaN may leave
-// hi, but not mid.  Products with them are NaN, and whoever uses this looks for that.
-__device__ __forceinline__ void split3(float2 p, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+// hi, but not mid.  Products with them are NaN, and whoever uses this looks for that.  half: 0 to cut hi off, too.
+__device__ __forceinline__ void split3(float2 p, uint32_t &hi, uint32_t &mid, uint32_t &lo, uint32_t half = 0x8000u) {
     const float2 minus = make_float2(-1.f, -1.f);
-    const uint32_t a = __float_as_uint(p.x) + 0x8000u, b = __float_as_uint(p.y) + 0x8000u;
+    const uint32_t a = __float_as_uint(p.x) + half, b = __float_as_uint(p.y) + half;
     hi = __byte_perm(a, b, 0x7632);
     const float2 r = fma2(make_float2(__uint_as_float(a & 0xFFFF0000u), __uint_as_float(b & 0xFFFF0000u)), minus, p);
     mid = __byte_perm(__float_as_uint(r.x), __float_as_uint(r.y), 0x7632);
@@ -137,11 +137,20 @@ struct Chunk {
     __device__ __forceinline__ int col(int i) const { return 8 * c + 64 * i; }
 };
 
-// Splits eight values into the three planes at `tile`, `plane` bytes apart.
+// Splits eight values into the three planes at `tile`, `plane` bytes apart.  kLarge: hi is cut off instead of rounded where one
+// of the values would round up to infinity (three terms of eight bits all the same).
+template <bool kLarge = false>
 __device__ __forceinline__ void store_split3(uint8_t *tile, int plane, int at, const float (&f)[8]) {
+    uint32_t half = 0x8000u;
+    if (kLarge) {
+        float top = fmaxf(fabsf(f[0]), fabsf(f[1]));
+#pragma unroll
+        for (int e = 2; e < 8; e += 2) top = max3(top, fabsf(f[e]), fabsf(f[e + 1]));
+        half = top >= __uint_as_float(0x7f7f8000u) ? 0u : half;
+    }
     uint32_t h[4], m[4], l[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) split3(make_float2(f[2 * e], f[2 * e + 1]), h[e], m[e], l[e]);
+    for (int e = 0; e < 4; e++) split3(make_float2(f[2 * e], f[2 * e + 1]), h[e], m[e], l[e], half);
     *reinterpret_cast<uint4 *>(tile + at) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4 *>(tile + plane + at) = make_uint4(m[0], m[1], m[2], m[3]);
     *reinterpret_cast<uint4 *>(tile + 2 * plane + at) = make_uint4(l[0], l[1], l[2], l[3]);

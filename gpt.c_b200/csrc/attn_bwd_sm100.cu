@@ -898,9 +898,109 @@ struct __align__(1024) Bwd24Smem {
     uint64_t go_s, go_dp, go_dv, go_dk, go_dq;  // operands are in place (one arrival per worker warp; Q from the copy engine)
     uint64_t done_s, done_dp, done_dv, done_dk, done_dq;
     uint64_t v_full, raw_full, raw_free, stat_full[2], stat_free[2];
+    uint32_t odd[4][4];  // [column quarter][key / 32]: a bit per key with a dK or dV that is not finite
     uint32_t tmem_base;
     int abort_flag;
 };
+
+// What this CTA does: keys from k0 on, and nsteps steps of queries from qs on.
+struct Part {
+    int bh, k0, qs, nsteps;
+    __device__ __forceinline__ Part(int pieces, int T) {
+        const int nt = (T + kTile - 1) / kTile * pieces, nbh = (int)gridDim.x / nt;
+        const int tile = (int)blockIdx.x / nbh;  // the first keys are seen by the most queries
+        bh = (int)blockIdx.x % nbh;
+        k0 = tile / pieces * kTile;
+        const int all = (T - k0 + kStep - 1) / kStep, first_part = (all + pieces - 1) / pieces;
+        nsteps = tile % pieces == 0 ? first_part : all - first_part;
+        qs = k0 + (tile % pieces == 0 ? 0 : first_part * kStep);
+    }
+};
+
+// Where column col of row `row` is in a tile that dK or dV leaves by: groups of 16 columns, 128 rows of 64 bytes, swizzled.
+__device__ __forceinline__ int key_tile_at(int row, int col) {
+    return (col >> 4) * (kTile * 64) + row * 64 + ((((col >> 2) & 3) ^ ((row >> 1) & 3)) << 4) + (col & 3) * 4;
+}
+
+// dK and dV of this CTA's keys that are marked in `odd`, over its queries, again in fp32 arithmetic, a warp per key: an infinite
+// dO is inf and NaN in its terms, and its products with keys after it are no zeros.  The other keys' are in the tiles at
+// dk_tile and dv_tile (NULL: in dqkv already).  More than one piece: another CTA adds to the same keys.
+// A function of its own, behind the last barrier, as in the forward.
+__device__ __noinline__ void exact_keys(const uint32_t (&odd)[4][4], const uint8_t *dk_tile, const uint8_t *dv_tile, int pieces,
+                                        const __nv_bfloat16 *__restrict__ xhi, const __nv_bfloat16 *__restrict__ xlo,
+                                        const float *__restrict__ lse, const float *__restrict__ delta, const float *__restrict__ dout,
+                                        float *__restrict__ dqkv, int T, int H, int D, float scale) {
+    constexpr int kE = attn::kAttn24MaxD / 32, kAhead = 4;  // columns of a lane, queries whose loads are on their way together
+    const Part part(pieces, T);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, bh = part.bh, b = bh / H, h = bh % H, C = H * D;
+    const int k0 = part.k0, q0 = part.qs, q1 = min(T, q0 + part.nsteps * kStep);
+    const size_t C3 = 3 * (size_t)C, head = (size_t)b * T * C3 + (size_t)h * D;
+    const float *dhead = dout + (size_t)b * T * C + (size_t)h * D;
+    auto at = [&](size_t i) { return __bfloat162float(xhi[i]) + __bfloat162float(xlo[i]); };
+#pragma unroll 1
+    for (int r = warp; r < min(kTile, T - k0); r += attn24::kThreads / 32) {
+        const int j = k0 + r;
+        const size_t row = head + (size_t)j * C3;
+        const bool again = (odd[0][r >> 5] | odd[1][r >> 5] | odd[2][r >> 5] | odd[3][r >> 5]) >> (r & 31) & 1u;
+        if (!again && dk_tile == nullptr) continue;
+        float k[kE], v[kE], dk[kE], dv[kE];
+#pragma unroll
+        for (int e = 0; e < kE; e++) {
+            const int col = lane + 32 * e;
+            k[e] = again && col < D ? at(row + C + col) : 0.f;
+            v[e] = again && col < D ? at(row + 2 * C + col) : 0.f;
+            dk[e] = again || col >= D ? 0.f : *reinterpret_cast<const float *>(dk_tile + key_tile_at(r, col));
+            dv[e] = again || col >= D ? 0.f : *reinterpret_cast<const float *>(dv_tile + key_tile_at(r, col));
+        }
+        bool is_nan = false;
+#pragma unroll 1
+        for (int i0 = max(j, q0); again && i0 < q1 && !is_nan; i0 += kAhead) {
+            float q[kAhead][kE], g[kAhead][kE], s[kAhead], dp[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                s[u] = dp[u] = 0.f;
+#pragma unroll
+                for (int e = 0; e < kE; e++) {
+                    const int col = lane + 32 * e;
+                    const bool in = i0 + u < q1 && col < D;
+                    q[u][e] = in ? at(head + (size_t)(i0 + u) * C3 + col) : 0.f;
+                    g[u][e] = in ? __ldg(dhead + (size_t)(i0 + u) * C + col) : 0.f;
+                    s[u] = fmaf(q[u][e], k[e], s[u]);
+                    dp[u] = fmaf(g[u][e], v[e], dp[u]);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) {
+                    s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+                    dp[u] += __shfl_xor_sync(0xffffffffu, dp[u], o);
+                }
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                if (i0 + u >= q1) break;
+                const size_t t = (size_t)bh * T + i0 + u;
+                const float p = expf(s[u] * scale - lse[t]), ds = p * (dp[u] - delta[t]);
+                is_nan = is_nan || p != p;  // every column of both is NaN
+#pragma unroll
+                for (int e = 0; e < kE; e++) dv[e] = fmaf(p, g[u][e], dv[e]), dk[e] = fmaf(ds, q[u][e], dk[e]);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < kE; e++) {
+            const int col = lane + 32 * e;
+            if (col >= D) break;
+            const float a = is_nan ? NAN : again ? dk[e] * scale : dk[e], c = is_nan ? NAN : dv[e];
+            if (pieces > 1) {
+                atomicAdd(dqkv + row + C + col, a);
+                atomicAdd(dqkv + row + 2 * C + col, c);
+            } else {
+                dqkv[row + C + col] = a;
+                dqkv[row + 2 * C + col] = c;
+            }
+        }
+    }
+}
 
 enum Site24 : int {
     SITE24_GO_S = 321, SITE24_GO_DP, SITE24_GO_DV, SITE24_GO_DK, SITE24_GO_DQ, SITE24_S, SITE24_DP, SITE24_DV, SITE24_DK, SITE24_DQ, SITE24_V, SITE24_RAW_FULL,
@@ -928,13 +1028,9 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE24_SMEM_ALIGN);
         return;
     }
-    const int nt = (T + kTile - 1) / kTile * pieces, nbh = (int)gridDim.x / nt;
-    const int tile = (int)blockIdx.x / nbh;  // the first keys are seen by the most queries
-    const int k0 = tile / pieces * kTile, all = (T - k0 + kStep - 1) / kStep, first_part = (all + pieces - 1) / pieces;
-    const int nsteps = tile % pieces == 0 ? first_part : all - first_part;
-    const int qs = k0 + (tile % pieces == 0 ? 0 : first_part * kStep);  // first query
+    const Part part(pieces, T);
+    const int bh = part.bh, b = bh / H, h = bh % H, k0 = part.k0, qs = part.qs, nsteps = part.nsteps;
     if (nsteps == 0) return;
-    const int bh = (int)blockIdx.x % nbh, b = bh / H, h = bh % H;
     const int C = H * D;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const bool vec = kTma || D % 4 == 0;
@@ -973,6 +1069,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     pdl_wait();
     const size_t C3 = 3 * (size_t)C, head = (size_t)b * T * C3 + (size_t)h * D;
     const float *dhead = dout + (size_t)b * T * C + (size_t)h * D;
+    int odd = 0;  // whether this thread has a value of dK or dV that is not finite
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -1137,7 +1234,7 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             }
 #pragma unroll
             for (int i = 0; i < kBlocks; i++)
-                if (mine.has<kK>(i)) store_split3(sm.g, kQueryPlane, mine.at + i * (kStep * 128), greg[i]);
+                if (mine.has<kK>(i)) store_split3<true>(sm.g, kQueryPlane, mine.at + i * (kStep * 128), greg[i]);
             warp_arrive(&sm.go_dp, lane);
         };
         request_g(0);
@@ -1330,18 +1427,29 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             }
         }
         if (tid == 0 || tid == 256) bulk_wait_all();
+        {
+            float zero[4] = {0.f, 0.f, 0.f, 0.f};  // what is finite times zero is zero
+#pragma unroll
+            for (int i = 0; i < 4 * kK; i++) zero[i & 3] = fmaf(dk[i], 0.f, fmaf(dv[i], 0.f, zero[i & 3]));
+            odd = k0 + row < T && !((zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.f);
+            const uint32_t keys = __ballot_sync(0xffffffffu, odd);
+            if (lane == 0) sm.odd[cq][quarter] = keys;
+        }
         if (vec) {
-            // dK and dV by the copy engine, from where K and V were: groups of 16 columns, 128 rows of 64 bytes, swizzled
+            // dK and dV by the copy engine, from where K and V were
 #pragma unroll
             for (int i = 0; i < kK; i++) {
-                const int col = 4 * kK * cq + 4 * i;
-                const int at = (col >> 4) * (kTile * 64) + row * 64 + ((((col >> 2) & 3) ^ ((row >> 1) & 3)) << 4);
+                const int at = key_tile_at(row, 4 * kK * cq + 4 * i);
                 *reinterpret_cast<float4 *>(sm.k[0] + at) = make_float4(dk[4 * i] * scale, dk[4 * i + 1] * scale, dk[4 * i + 2] * scale, dk[4 * i + 3] * scale);
                 *reinterpret_cast<float4 *>(sm.v[0] + at) = make_float4(dv[4 * i], dv[4 * i + 1], dv[4 * i + 2], dv[4 * i + 3]);
             }
             fence_proxy_async_smem();
             named_sync(5, kWorkers);
-            if (tid == 0) {
+            uint32_t any = 0;
+            if (tid == 0)
+#pragma unroll
+                for (int i = 0; i < 16; i++) any |= sm.odd[i >> 2][i & 3];
+            if (tid == 0 && any == 0) {  // else exact_keys() writes them
                 for (int g = 0; g < kK && 16 * g < D; g++)
                     for (int part = 0; part < 2; part++) {
                         const uint8_t *from = (part == 0 ? sm.k[0] : sm.v[0]) + g * (kTile * 64);
@@ -1359,11 +1467,13 @@ attn24_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     if (sm.abort_flag) __nanosleep(50000);  // let copies and products that are still in flight end
     tc_fence_before_sync();
-    __syncthreads();
+    const int again = __syncthreads_or(odd);
     if (warp == kWorkWarps) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, 512);
     }
+    if (again)
+        exact_keys(sm.odd, vec ? sm.k[0] : nullptr, sm.v[0], pieces, xhi, xlo, lse, delta, dout, dqkv, T, H, D, scale);
 }
 
 }  // namespace general

@@ -47,7 +47,8 @@
  *
  * Values that are not finite: the general forward gives what fp32 arithmetic gives (a score of -inf has no
  * weight, an infinite v is infinite in every row that gives it weight), and up to head size 128 rows that
- * do not see such a value are unaffected (above, rows of the same tile of keys may be).  Two bf16 terms
+ * do not see such a value are unaffected (above, rows of the same tile of keys may be).  The general
+ * backward does the same with dout, keys that a row does not see included.  Two bf16 terms
  * have no infinities: where head size is 64, and in the planes the backward reads, an infinite value, or
  * a finite one above 3.396e38, makes NaN of what it enters.
  */

@@ -182,6 +182,57 @@ def test_general_forward_of_infinities_and_the_largest_values(pkg, gpu, T, D, wh
     same_but_for_rounding(lse, ref_lse, 1e-5)
 
 
+def causal_backward_f64(x, g, H):
+    """dq, dk, dv of the definition in 64 bits, over the pairs of a row and a key it sees."""
+    B, T, C3 = x.shape
+    D = C3 // 3 // H
+    q, k, v = (x.astype(np.float64).reshape(B, T, 3, H, D)[:, :, i] for i in range(3))
+    g = g.astype(np.float64).reshape(B, T, H, D)
+    d = np.zeros((B, T, 3, H, D))
+    with np.errstate(invalid="ignore"):
+        for b in range(B):
+            for h in range(H):
+                for t in range(T):
+                    s = (k[b, :t + 1, h] * q[b, t, h]).sum(1) / np.sqrt(D)
+                    p = np.exp(s - s.max())
+                    p /= p.sum()
+                    o = (p[:, None] * v[b, :t + 1, h]).sum(0)
+                    ds = p * ((v[b, :t + 1, h] * g[b, t, h]).sum(1) - (o * g[b, t, h]).sum()) / np.sqrt(D)
+                    d[b, t, 0, h] = (ds[:, None] * k[b, :t + 1, h]).sum(0)
+                    d[b, :t + 1, 1, h] += ds[:, None] * q[b, t, h]
+                    d[b, :t + 1, 2, h] += p[:, None] * g[b, t, h]
+    return d.reshape(B, T, C3)
+
+
+@pytest.mark.parametrize("T,D", [(1, 16), (70, 3), (130, 20), (150, 64), (140, 67), (300, 48), (200, 128)])
+@pytest.mark.parametrize("what", ["inf", "inf at the end", "-inf in many", "nan", "large"])
+def test_general_backward_of_infinities_and_the_largest_values(pkg, gpu, T, D, what):
+    """The same for dO: q, k and v are read with 16 bits and their values stay below 2^128 there.  (Each of three factors off by
+    up to 2^-17 of the largest; both numbers of pieces: T = 300 has two.)"""
+    torch, H, at = gpu, 2, T // 3
+    x, g = seeded(53 + T + D, 2, T, H, D)
+    v, do = x.reshape(2, T, 3, H, D)[:, :, 2], g.reshape(2, T, H, D)
+    if what == "inf":
+        do[0, at, 1, 0] = np.inf
+    elif what == "inf at the end":
+        do[1, T - 1, 0, D - 1] = np.inf
+    elif what == "-inf in many":
+        do[0, at:, 0, D // 2] = -np.inf
+    elif what == "nan":
+        do[1, at, 1, D // 2] = np.nan
+    else:
+        v[..., 0] *= 0.125  # so that dO . V and what follows from it stays below the largest number
+        do[0, at, 1, 0], do[1, T - 1, 0, 0] = 3.4028e38, -3.3999e38
+    _, ctx = pkg.forward(torch.from_numpy(x).cuda(), H, flags=pkg.FLAG_FORCE_GENERIC)
+    dx = pkg.backward(ctx, torch.from_numpy(g).cuda()).cpu().numpy()
+    assert pkg.device_status() == 0
+    ref = causal_backward_f64(x, g, H)
+    finite = np.isfinite(ref)
+    assert np.array_equal(np.isnan(dx), np.isnan(ref))
+    assert np.array_equal(dx[np.isinf(ref)], ref[np.isinf(ref)].astype(np.float32))
+    assert (np.abs(dx[finite] - ref[finite]) <= 3 * 2.0 ** -17 * np.abs(ref[finite]).max()).all()
+
+
 @pytest.mark.parametrize("T,D", [(1, 3), (70, 20), (128, 48), (200, 40), (193, 128), (257, 72)])
 def test_general_forward_leaves_the_planes_of_the_split(pkg, gpu, T, D):
     """Bit for bit what the split alone writes, whatever the alignment of the rows, and a core-only call leaves them alone."""
