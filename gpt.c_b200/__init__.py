@@ -57,6 +57,7 @@ SIGNATURES = {
 
 _lib = None
 _calls_module = None
+_entry_classes = {}  # name of an entry point -> the class of its function in lib()
 
 
 class AttnError(RuntimeError):
@@ -78,8 +79,38 @@ def lib() -> ctypes.CDLL:
             fn = getattr(handle, name)
             fn.restype = res
             fn.argtypes = args
+            _entry_classes[name] = fn.__class__ = _entry_class(handle._FuncPtr)
         _lib = handle
+        _shorten_calls()
     return _lib
+
+
+def _entry_class(plain):
+    """A class for one function of the library: a ctypes function like any other, which the extension module may give a
+    shorter way from a call's arguments to the C ABI.  That way knows the signature above, so a function that is given
+    another one becomes an ordinary ctypes function."""
+
+    class Entry(plain):
+        _flags_ = plain._flags_
+        _restype_ = plain._restype_
+
+        def __setattr__(self, name, value):
+            if name in ("restype", "argtypes", "errcheck"):
+                self.__class__ = plain
+            plain.__setattr__(self, name, value)
+
+        def __delattr__(self, name):
+            if name in ("restype", "argtypes", "errcheck"):
+                self.__class__ = plain
+            plain.__delattr__(self, name)
+
+    return Entry
+
+
+def _shorten_calls():
+    if _calls_module is not None:
+        for name, method in _calls_module.entry_calls(ctypes._CFuncPtr).items():
+            _entry_classes[name].__call__ = method
 
 
 def _calls():
@@ -98,8 +129,8 @@ def _calls():
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         mod.set_error(AttnError)
-        mod.take_over(lib())
         _calls_module = mod
+        _shorten_calls()
     return _calls_module
 
 

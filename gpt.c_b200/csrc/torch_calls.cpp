@@ -6,7 +6,7 @@
 // stream, 11 to 13 converted arguments per ctypes call) around 16 us of GPU work.  Here the arguments are taken
 // from the tensor objects directly, outputs come from the caching allocator without going through the operator
 // dispatcher, and the stream is a thread-local read.  The GIL is released around the C ABI call, as ctypes does.
-// The element-wise entry points and size queries that programs call through lib() get the same treatment (Function):
+// The element-wise entry points and size queries that programs call through lib() get the same treatment (entry_calls):
 // converting their arguments took ctypes 0.5 to 1 us of the 2.8 us of a call, 2.3 of which the launch itself needs.
 #include <Python.h>
 
@@ -323,14 +323,11 @@ PyObject *layernorm_backward(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Function: a C ABI entry point called with Python numbers, in front of the ctypes function of the same name, which
-// gets every call whose arguments are not exactly as many plain numbers (or None for a pointer), and every attribute.
+// What calling a ctypes function of the library does instead (the package puts these into the classes of its function
+// objects as __call__): a call with exactly as many plain numbers (or None for a pointer) as the function has arguments goes
+// to the C ABI from here, every other one to ctypes.
 // ------------------------------------------------------------------------------------------
-struct Function {
-    PyObject_HEAD
-    vectorcallfunc call;
-    PyObject *plain;
-};
+PyTypeObject *g_plain = nullptr;  // ctypes' own class of functions
 
 template <class T>
 bool take(PyObject *o, T *&out) {
@@ -343,11 +340,22 @@ bool take(PyObject *o, int &out) { return PyLong_Check(o) && (out = static_cast<
 bool take(PyObject *o, size_t &out) { return PyLong_Check(o) && (out = static_cast<size_t>(PyLong_AsUnsignedLongLongMask(o)), true); }
 bool take(PyObject *o, float &out) { return PyFloat_Check(o) && (out = static_cast<float>(PyFloat_AS_DOUBLE(o)), true); }
 
+PyObject *call_plain(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *names) {
+    PyObject *tuple = PyTuple_New(n), *keywords = names != nullptr ? PyDict_New() : nullptr, *result = nullptr;
+    bool ok = tuple != nullptr && (names == nullptr || keywords != nullptr);
+    for (Py_ssize_t i = 0; ok && i < n; i++) PyTuple_SET_ITEM(tuple, i, Py_NewRef(args[i]));
+    for (Py_ssize_t i = 0; ok && names != nullptr && i < PyTuple_GET_SIZE(names); i++)
+        ok = PyDict_SetItem(keywords, PyTuple_GET_ITEM(names, i), args[n + i]) == 0;
+    if (ok) result = g_plain->tp_call(self, tuple, keywords);
+    Py_XDECREF(tuple);
+    Py_XDECREF(keywords);
+    return result;
+}
+
 template <class R, class... A, size_t... I>
-PyObject *invoke(R (*fn)(A...), PyObject *self, PyObject *const *args, size_t nargsf, PyObject *names, std::index_sequence<I...>) {
+PyObject *invoke(R (*fn)(A...), PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *names, std::index_sequence<I...>) {
     std::tuple<A...> v;
-    if (names != nullptr || PyVectorcall_NARGS(nargsf) != (Py_ssize_t)sizeof...(A) || !(take(args[I], std::get<I>(v)) && ...))
-        return PyObject_Vectorcall(reinterpret_cast<Function *>(self)->plain, args, nargsf, names);
+    if (names != nullptr || n != (Py_ssize_t)sizeof...(A) || !(take(args[I], std::get<I>(v)) && ...)) return call_plain(self, args, n, names);
     R rc;
     Py_BEGIN_ALLOW_THREADS
     rc = fn(std::get<I>(v)...);
@@ -357,66 +365,33 @@ PyObject *invoke(R (*fn)(A...), PyObject *self, PyObject *const *args, size_t na
 template <class R, class... A>
 constexpr size_t arity(R (*)(A...)) { return sizeof...(A); }
 template <auto kFn>
-PyObject *vectorcall(PyObject *self, PyObject *const *args, size_t nargsf, PyObject *names) {
-    return invoke(kFn, self, args, nargsf, names, std::make_index_sequence<arity(kFn)>());
+PyObject *call(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *names) {
+    return invoke(kFn, self, args, n, names, std::make_index_sequence<arity(kFn)>());
 }
 
-#define ENTRY(name) {#name, vectorcall<name>}
-const struct {
-    const char *name;
-    vectorcallfunc call;
-} kEntries[] = {ENTRY(tensor_sm100_fill),        ENTRY(tensor_sm100_arange),        ENTRY(tensor_sm100_copy),
-                ENTRY(tensor_sm100_axpy),        ENTRY(tensor_sm100_gelu_forward),  ENTRY(tensor_sm100_gelu_backward),
-                ENTRY(xent_sm100_forward),       ENTRY(xent_sm100_backward),        ENTRY(attn_sm100_saved_bytes),
-                ENTRY(attn_sm100_backward_scratch_bytes)};
+#define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call<name>)), METH_FASTCALL | METH_KEYWORDS, nullptr}
+PyMethodDef kEntries[] = {ENTRY(tensor_sm100_fill),        ENTRY(tensor_sm100_arange),        ENTRY(tensor_sm100_copy),
+                          ENTRY(tensor_sm100_axpy),        ENTRY(tensor_sm100_gelu_forward),  ENTRY(tensor_sm100_gelu_backward),
+                          ENTRY(xent_sm100_forward),       ENTRY(xent_sm100_backward),        ENTRY(attn_sm100_saved_bytes),
+                          ENTRY(attn_sm100_backward_scratch_bytes)};
 
-void function_dealloc(PyObject *self) {
-    Py_XDECREF(reinterpret_cast<Function *>(self)->plain);
-    Py_TYPE(self)->tp_free(self);
-}
-PyObject *function_getattr(PyObject *self, PyObject *name) { return PyObject_GetAttr(reinterpret_cast<Function *>(self)->plain, name); }
-int function_setattr(PyObject *self, PyObject *name, PyObject *value) {
-    return PyObject_SetAttr(reinterpret_cast<Function *>(self)->plain, name, value);
-}
-
-PyTypeObject *function_type() {
-    static PyTypeObject type = {PyVarObject_HEAD_INIT(nullptr, 0)};
-    if (type.tp_name == nullptr) {
-        type.tp_name = "gptc_b200_calls.Function";
-        type.tp_basicsize = sizeof(Function);
-        type.tp_dealloc = function_dealloc;
-        type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL;
-        type.tp_vectorcall_offset = offsetof(Function, call);
-        type.tp_call = PyVectorcall_Call;
-        type.tp_getattro = function_getattr;
-        type.tp_setattro = function_setattr;
-        if (PyType_Ready(&type) < 0) {
-            type.tp_name = nullptr;
-            return nullptr;
-        }
+// entry_calls(class of ctypes functions) -> {name of the entry point: method of that class}
+PyObject *entry_calls(PyObject *, PyObject *plain) {
+    if (!PyType_Check(plain) || reinterpret_cast<PyTypeObject *>(plain)->tp_call == nullptr) {
+        PyErr_SetString(PyExc_TypeError, "expected the class of ctypes functions");
+        return nullptr;
     }
-    return &type;
-}
-
-// take_over(library): the entry points above, in front of those of the ctypes library object
-PyObject *take_over(PyObject *, PyObject *library) {
-    PyTypeObject *type = function_type();
-    if (type == nullptr) return nullptr;
-    for (const auto &e : kEntries) {
-        PyObject *plain = PyObject_GetAttrString(library, e.name);
-        if (plain == nullptr) return nullptr;
-        Function *f = PyObject_New(Function, type);
-        if (f == nullptr) {
-            Py_DECREF(plain);
-            return nullptr;
-        }
-        f->call = e.call;
-        f->plain = plain;
-        const int rc = PyObject_SetAttrString(library, e.name, reinterpret_cast<PyObject *>(f));
-        Py_DECREF(f);
-        if (rc < 0) return nullptr;
+    Py_INCREF(plain);
+    Py_XDECREF(reinterpret_cast<PyObject *>(g_plain));
+    g_plain = reinterpret_cast<PyTypeObject *>(plain);
+    PyObject *all = PyDict_New();
+    for (PyMethodDef &e : kEntries) {
+        PyObject *method = all != nullptr ? PyDescr_NewMethod(g_plain, &e) : nullptr;
+        if (method == nullptr || PyDict_SetItemString(all, e.ml_name, method) < 0) Py_CLEAR(all);
+        Py_XDECREF(method);
+        if (all == nullptr) return nullptr;
     }
-    Py_RETURN_NONE;
+    return all;
 }
 
 // set_error(cls): the exception class raised for a non-zero status
@@ -430,7 +405,7 @@ PyObject *set_error(PyObject *, PyObject *cls) {
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(forward), FAST(backward), FAST(forward_into), FAST(backward_into), FAST(linear_forward),
                           FAST(linear_backward), FAST(layernorm_forward), FAST(layernorm_backward),
-                          {"set_error", set_error, METH_O, nullptr}, {"take_over", take_over, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                          {"set_error", set_error, METH_O, nullptr}, {"entry_calls", entry_calls, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "gptc_b200_calls", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

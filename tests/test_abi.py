@@ -96,6 +96,47 @@ def test_no_cpu_fallback_without_gpu(pkg):
         pkg.init()
 
 
+@pytest.fixture
+def fresh(pkg, monkeypatch):
+    """The library loaded anew, as in a program that has made no tensor-level call yet (the module is loaded again by one)."""
+    monkeypatch.setattr(pkg, "_lib", None)
+    monkeypatch.setattr(pkg, "_calls_module", None)
+    monkeypatch.setattr(pkg, "_entry_classes", {}, raising=False)
+    return pkg
+
+
+def test_functions_are_the_same_objects_before_and_after_the_extension_is_loaded(fresh):
+    """What lib() gives does not depend on what has been called before, and is a ctypes function in both cases."""
+    names = sorted(fresh.SIGNATURES)
+    before = [getattr(fresh.lib(), n) for n in names]
+    classes = [type(f) for f in before]
+    address = [ctypes.cast(f, ctypes.c_void_p).value for f in before]
+    assert before[names.index("tensor_sm100_axpy")](5, 1.0, None, None, None) == -1
+    fresh._calls()
+    for name, fn, cls, at in zip(names, before, classes, address):
+        assert getattr(fresh.lib(), name) is fn and type(fn) is cls and isinstance(fn, ctypes._CFuncPtr)
+        assert ctypes.cast(fn, ctypes.c_void_p).value == at and at
+        assert fn.argtypes == fresh.SIGNATURES[name][1] and fn.restype is fresh.SIGNATURES[name][0]
+    assert before[names.index("tensor_sm100_axpy")](5, 1.0, None, None, None) == -1
+
+
+@pytest.mark.parametrize("loaded_before", [False, True])
+def test_a_changed_signature_acts_on_every_call(fresh, loaded_before):
+    if loaded_before:
+        fresh._calls()
+    fn = fresh.lib().tensor_sm100_fill
+    assert fn(None, 2, 0.5, None) == -1
+    fn.errcheck = lambda result, func, args: result - 100
+    fresh._calls()
+    assert fn(None, 2, 0.5, None) == -101  # a call whose arguments are plain numbers
+    del fn.errcheck
+    fn.restype = ctypes.c_uint
+    assert fn(None, 2, 0.5, None) == 2 ** 32 - 1
+    fn.argtypes = [ctypes.c_void_p] * 4
+    with pytest.raises(ctypes.ArgumentError):
+        fn(None, 2, 0.5, None)
+
+
 def test_extension_answers_like_ctypes(pkg):
     """The entry points the extension puts in front of the ctypes functions: the same results for numbers, None, ctypes
     objects and wrong arguments (all rejected or done before the GPU is touched), the same attributes."""
