@@ -105,14 +105,6 @@ at::Tensor alloc(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &b
     return at::detail::empty_cuda(shape, type, beside.device(), std::nullopt);
 }
 
-// `count` floats of a float tensor from `offset` on, as a tensor of its own beside it in the same memory.
-at::Tensor part(const at::Tensor &of, int64_t offset, int64_t count) {
-    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(of.storage()), of.key_set(), of.dtype());
-    t.unsafeGetTensorImpl()->set_storage_offset(offset);
-    t.unsafeGetTensorImpl()->set_sizes_contiguous({count});
-    return t;
-}
-
 PyObject *value_error(const char *text) {
     PyErr_SetString(PyExc_ValueError, text);
     return nullptr;
@@ -286,10 +278,7 @@ PyObject *layernorm_forward(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (!a.ok) return nullptr;
     const int64_t C = x->size(-1), rows = x->numel() / C;
     at::Tensor y = alloc(x->sizes(), at::kFloat, *x);
-    // the row statistics live equally long: one allocation (1.2 us) for both
-    const int64_t apart = (rows + 63) / 64 * 64;
-    const at::Tensor stats = alloc({2 * apart}, at::kFloat, *x);
-    at::Tensor mean = part(stats, 0, rows), rstd = part(stats, apart, rows);
+    at::Tensor mean = alloc({rows}, at::kFloat, *x), rstd = alloc({rows}, at::kFloat, *x);
     const float *xp = static_cast<const float *>(x->data_ptr());
     float *yp = static_cast<float *>(y.data_ptr()), *mp = static_cast<float *>(mean.data_ptr()),
           *rp = static_cast<float *>(rstd.data_ptr());

@@ -53,6 +53,19 @@ def test_layernorm_forward_and_backward_vs_cpu(pkg, rows, C, with_bias):
     assert np.abs(dx.cpu().numpy() - (dx0 + dx_ref)).max() <= 2e-5 * max(1.0, np.abs(dx_ref).max())
 
 
+def test_layernorm_results_do_not_share_memory(pkg):
+    """What is kept, saved or resized is that tensor alone."""
+    x, w = torch.randn(37, 768, device="cuda"), torch.randn(768, device="cuda")
+    results = pkg.layernorm_forward(x, w)
+    assert len({t.untyped_storage().data_ptr() for t in results}) == 3
+    for t in results:
+        assert t.untyped_storage().nbytes() == 4 * t.numel() and t.storage_offset() == 0
+    y, mean, rstd = results
+    before = rstd.clone()
+    mean.resize_(5000).fill_(7.0)
+    assert torch.equal(rstd, before)
+
+
 def test_layernorm_argument_errors(pkg):
     L = pkg.lib()
     t = torch.zeros(64, device="cuda")
