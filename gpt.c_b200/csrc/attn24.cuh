@@ -24,15 +24,18 @@ constexpr int kWorkWarps = kWorkers / 32;
 constexpr int kStep = 64;  // rows of the smaller tile operand
 
 // log2(e) / sqrt(D) as the sum of two floats, both positive (a score of -inf times either is -inf), and a little more than
-// that: a score is a chain of D / 16 products that are not small, each of which truncates the sum so far.  Truncation takes
-// half a unit in the last place on average, 0.36 * 2^-23 of a value whose mantissa is spread over its logarithm, and the
-// sum after i of k products is i / k of the score on average: 0.36 * (k + 1) * 2^-24 of the score are missing.  (Without
-// that the error of the log-sum-exp was 3.6e-8 at D = 128, 3.1e-8 in fp32 arithmetic; with it 3.1e-8.)
+// that: the tensor cores truncate, so the last k = D / 16 products of a score, which are not small, leave it too small by
+// (0.18 k + 0.5) * 2^-24 of it on average.  That is what scores of 2^3 and more showed at D = 16 ... 128 against 64 bits (0.36 k
+// + 0.36 would follow from cutting off half a unit of the sum so far after each product, and is too much: the sums seem to
+// have a bit more on the way).  Relative error of the log-sum-exp without it, with twice of it and with it, and in fp32
+// arithmetic, 1e-8: D = 128, q and k of standard deviation one 3.6, 2.8, 2.8, 3.1, of two 11.0, 7.7, 4.2, 6.6; D = 64, of two
+// 6.8, 4.6, 3.3, 4.9.  In the backward, which takes its scores from 16-bit operands, it is 1 % of the error (dq at D = 128, of
+// two: 1.67e-5 without it, 1.65e-5 with it, 1.66e-5 in fp32 arithmetic).
 struct Scale {
     float hi, lo;
 };
 inline Scale log2_scale(int D) {
-    const double c = 1.4426950408889634 / sqrt((double)D) * (1.0 + 0.36 * ((D + 15) / 16 + 1) / 16777216.0);
+    const double c = 1.4426950408889634 / sqrt((double)D) * (1.0 + (0.18 * ((D + 15) / 16) + 0.5) / 16777216.0);
     float hi = (float)c;
     if ((double)hi >= c) hi = nextafterf(hi, 0.f);
     return Scale{hi, (float)(c - (double)hi)};

@@ -233,6 +233,24 @@ def test_general_backward_of_infinities_and_the_largest_values(pkg, gpu, T, D, w
     assert (np.abs(dx[finite] - ref[finite]) <= 3 * 2.0 ** -17 * np.abs(ref[finite]).max()).all()
 
 
+@pytest.mark.parametrize("D", [16, 64, 80, 96, 128])
+@pytest.mark.parametrize("std", [1.0, 2.0, 3.0])
+def test_general_forward_is_fp32_for_large_scores_too(pkg, gpu, D, std):
+    """Scores of up to 200: the log-sum-exp, above all a score there, is off by less than the half unit (2^-24, 6.0e-8) that one
+    rounding may cost (fp32 arithmetic: 3.1e-8 ... 9.0e-8), and not by the same share in one direction."""
+    torch, B, T, H = gpu, 2, 700, 4
+    torch.manual_seed(D)
+    x = torch.randn(B, T, 3 * H * D, device="cuda") * std
+    _, ctx = pkg.forward(x, H, flags=pkg.FLAG_FORCE_GENERIC)
+    assert pkg.device_status() == 0
+    q, k, _ = (x.double().view(B, T, 3, H, D)[:, :, i].transpose(1, 2) for i in range(3))
+    s = (q @ k.transpose(-1, -2)) / D ** 0.5
+    ref = torch.logsumexp(s.masked_fill(torch.ones(T, T, device="cuda", dtype=torch.bool).triu(1), -float("inf")), -1)
+    off = ctx.lse.double() - ref
+    assert (off.norm() / ref.norm()).item() < 2.0 ** -24
+    assert abs((off * ref).sum() / (ref * ref).sum()).item() < 2.0 ** -26
+
+
 @pytest.mark.parametrize("T,D", [(1, 3), (70, 20), (128, 48), (200, 40), (193, 128), (257, 72)])
 def test_general_forward_leaves_the_planes_of_the_split(pkg, gpu, T, D):
     """Bit for bit what the split alone writes, whatever the alignment of the rows, and a core-only call leaves them alone."""
