@@ -81,8 +81,8 @@ def test_generic_vs_oracle(pkg, gpu, oracle, shape):
 @pytest.mark.parametrize("D", [1, 4, 31, 32, 33, 63, 96, 100, 128, 129, 132, 200, 256])
 @pytest.mark.parametrize("T", [1, 63, 65, 130])
 def test_generic_tile_edges(pkg, gpu, oracle, T, D):
-    """Query and key tiles of 64 (32 above D = 128), head columns in blocks of 32, rows read in words of four
-    columns when D allows it."""
+    """Tiles of 128 rows in steps of 64, head columns in groups of 16 and blocks of 64 (above D = 128 tiles of 64 and 32, blocks
+    of 32), rows fetched in words of four columns when D allows it."""
     x, g = seeded(23 + T + D, 2, T, 2, D)
     out, lse, dx = run_cuda(pkg, gpu, x, g, 2, flags=pkg.FLAG_FORCE_GENERIC)
     ref_out, ref_lse = oracle.forward(x, 2, want_lse=True)
@@ -95,7 +95,7 @@ def test_generic_tile_edges(pkg, gpu, oracle, T, D):
                                  (2, 3), (64, 20), (129, 40), (191, 100), (320, 126)])
 def test_general_tensor_core_kernels_are_fp32_and_repeatable(pkg, gpu, oracle, T, D):
     """Steps of 64 keys or queries, tiles of 128, head columns in groups of 16 and blocks of 64, rows fetched by the copy
-    engine (D a multiple of 16) or by the threads (a multiple of 4, and others).
+    engine (D a multiple of 4 in the forward, of 8 in the backward) or by the threads.
 
     Operands of 24 bits: a relative error of 2^-21 in the 2-norm leaves eight roundings of 2^-24, above all those of
     exponents of up to eight and of exp2; operands of 16 bits give 4e-6.  The backward reads q, k, v with 16 bits: each of
@@ -117,6 +117,37 @@ def test_general_tensor_core_kernels_are_fp32_and_repeatable(pkg, gpu, oracle, T
         d = pkg.backward(ctx, gd)
         assert np.array_equal(o.cpu().numpy(), out) and np.array_equal(ctx.lse.cpu().numpy().reshape(lse.shape), lse)
         assert np.array_equal(d.cpu().numpy()[..., 2 * D:], dx[..., 2 * D:])
+
+
+def attention_f64(torch, x, dout, H):
+    """out, lse and dqkv in 64 bits, by torch's own products and differentiation on the GPU: nothing of this library."""
+    B, T, C3 = x.shape
+    D = C3 // 3 // H
+    qkv = x.double().requires_grad_(True)
+    q, k, v = (qkv.view(B, T, 3, H, D)[:, :, i].transpose(1, 2) for i in range(3))
+    s = (q @ k.transpose(-1, -2)) / D ** 0.5
+    s = s.masked_fill(torch.ones(T, T, device=x.device, dtype=torch.bool).triu(1), -float("inf"))
+    out = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(B, T, H * D)
+    out.backward(dout.double())
+    return out.detach(), torch.logsumexp(s.detach(), -1), qkv.grad
+
+
+@pytest.mark.parametrize("B,T,H,D", [(30, 130, 8, 20), (10, 300, 20, 48), (3, 511, 25, 67), (4, 640, 12, 128), (12, 200, 13, 64), (50, 64, 6, 16)])
+def test_general_kernels_of_more_tiles_than_sms(pkg, gpu, B, T, H, D):
+    """Thread blocks that follow others on an SM.  Bounds as for one tile: 2^-21 for operands of 24 bits, three factors of 16
+    in the backward."""
+    torch = gpu
+    torch.manual_seed(T)
+    x, g = torch.randn(B, T, 3 * H * D, device="cuda"), torch.randn(B, T, H * D, device="cuda")
+    out, ctx = pkg.forward(x, H, flags=pkg.FLAG_FORCE_GENERIC)
+    dx = pkg.backward(ctx, g)
+    assert pkg.device_status() == 0
+    ref_out, ref_lse, ref_dx = attention_f64(torch, x, g, H)
+    assert (out - ref_out).norm().item() < 2.0 ** -21 * ref_out.norm().item()
+    assert (ctx.lse - ref_lse).norm().item() < 2.0 ** -21 * ref_lse.norm().item()
+    for part in range(3):
+        a, b = (t[..., part * H * D:(part + 1) * H * D] for t in (dx, ref_dx))
+        assert (a - b).norm().item() < 3 * 2.0 ** -17 * b.norm().item()
 
 
 def causal_forward_f64(x, H):
@@ -664,11 +695,13 @@ QUEUE_EDGE_SHAPES = [
 
 @pytest.mark.parametrize("shape", QUEUE_EDGE_SHAPES, ids=lambda s: "B%d_T%d_H%d_items%d" % (s + (_items(*s),)))
 def test_backward_item_queue_edges_match_generic_kernels(pkg, gpu, shape):
-    """The tensor-core backward against the SIMT kernels of the same library (themselves checked against the
-    oracle above) where the number of work items crosses multiples of the SM count."""
+    """The backward of D = 64 against the general kernels of the same library (which share instructions and the split with it),
+    and against 64-bit arithmetic that shares nothing, where the number of work items crosses multiples of the SM count."""
     B, T, H = shape
     x, g = seeded(50 + B + T + H, B, T, H, 64)
     _, _, d1 = run_cuda(pkg, gpu, x, g, H)
     _, _, d2 = run_cuda(pkg, gpu, x, g, H, flags=pkg.FLAG_FORCE_GENERIC)
     assert np.isfinite(d1).all()
     assert np.abs(d1 - d2).max() < EXPECT_DX
+    ref = attention_f64(gpu, gpu.from_numpy(x).cuda(), gpu.from_numpy(g).cuda(), H)[2].cpu().numpy()
+    assert np.abs(d1 - ref).max() < EXPECT_DX
