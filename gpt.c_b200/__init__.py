@@ -109,8 +109,7 @@ def _entry_class(plain):
 
 def _shorten_calls():
     if _calls_module is not None:
-        for name, method in _calls_module.entry_calls(ctypes._CFuncPtr).items():
-            _entry_classes[name].__call__ = method
+        _calls_module.shorten_calls(_entry_classes)
 
 
 def _calls():

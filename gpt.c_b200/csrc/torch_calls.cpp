@@ -6,7 +6,7 @@
 // stream, 11 to 13 converted arguments per ctypes call) around 16 us of GPU work.  Here the arguments are taken
 // from the tensor objects directly, outputs come from the caching allocator without going through the operator
 // dispatcher, and the stream is a thread-local read.  The GIL is released around the C ABI call, as ctypes does.
-// The element-wise entry points and size queries that programs call through lib() get the same treatment (entry_calls):
+// The element-wise entry points and size queries that programs call through lib() get the same treatment (shorten_calls):
 // converting their arguments took ctypes 0.5 to 1 us of the 2.8 us of a call, 2.3 of which the launch itself needs.
 #include <Python.h>
 
@@ -312,12 +312,10 @@ PyObject *layernorm_backward(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 // ------------------------------------------------------------------------------------------
-// What calling a ctypes function of the library does instead (the package puts these into the classes of its function
-// objects as __call__): a call with exactly as many plain numbers (or None for a pointer) as the function has arguments goes
-// to the C ABI from here, every other one to ctypes.
+// What calling a ctypes function of the library does instead, as the tp_call of its function object's class: a call with
+// exactly as many plain numbers (or None for a pointer) as the function has arguments goes to the C ABI from here, every
+// other one to ctypes.
 // ------------------------------------------------------------------------------------------
-PyTypeObject *g_plain = nullptr;  // ctypes' own class of functions
-
 template <class T>
 bool take(PyObject *o, T *&out) {
     if (o == Py_None) out = nullptr;
@@ -329,22 +327,14 @@ bool take(PyObject *o, int &out) { return PyLong_Check(o) && (out = static_cast<
 bool take(PyObject *o, size_t &out) { return PyLong_Check(o) && (out = static_cast<size_t>(PyLong_AsUnsignedLongLongMask(o)), true); }
 bool take(PyObject *o, float &out) { return PyFloat_Check(o) && (out = static_cast<float>(PyFloat_AS_DOUBLE(o)), true); }
 
-PyObject *call_plain(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *names) {
-    PyObject *tuple = PyTuple_New(n), *keywords = names != nullptr ? PyDict_New() : nullptr, *result = nullptr;
-    bool ok = tuple != nullptr && (names == nullptr || keywords != nullptr);
-    for (Py_ssize_t i = 0; ok && i < n; i++) PyTuple_SET_ITEM(tuple, i, Py_NewRef(args[i]));
-    for (Py_ssize_t i = 0; ok && names != nullptr && i < PyTuple_GET_SIZE(names); i++)
-        ok = PyDict_SetItem(keywords, PyTuple_GET_ITEM(names, i), args[n + i]) == 0;
-    if (ok) result = g_plain->tp_call(self, tuple, keywords);
-    Py_XDECREF(tuple);
-    Py_XDECREF(keywords);
-    return result;
-}
-
 template <class R, class... A, size_t... I>
-PyObject *invoke(R (*fn)(A...), PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *names, std::index_sequence<I...>) {
+PyObject *invoke(R (*fn)(A...), ternaryfunc own, PyObject *self, PyObject *args, PyObject *keywords, std::index_sequence<I...>) {
     std::tuple<A...> v;
-    if (names != nullptr || n != (Py_ssize_t)sizeof...(A) || !(take(args[I], std::get<I>(v)) && ...)) return call_plain(self, args, n, names);
+    if (keywords != nullptr || PyTuple_GET_SIZE(args) != (Py_ssize_t)sizeof...(A) || !(take(PyTuple_GET_ITEM(args, I), std::get<I>(v)) && ...)) {
+        PyTypeObject *base = Py_TYPE(self)->tp_base;  // of the function's class, or of one derived from it
+        while (base->tp_call == own) base = base->tp_base;
+        return base->tp_call(self, args, keywords);
+    }
     R rc;
     Py_BEGIN_ALLOW_THREADS
     rc = fn(std::get<I>(v)...);
@@ -354,33 +344,32 @@ PyObject *invoke(R (*fn)(A...), PyObject *self, PyObject *const *args, Py_ssize_
 template <class R, class... A>
 constexpr size_t arity(R (*)(A...)) { return sizeof...(A); }
 template <auto kFn>
-PyObject *call(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *names) {
-    return invoke(kFn, self, args, n, names, std::make_index_sequence<arity(kFn)>());
+PyObject *call(PyObject *self, PyObject *args, PyObject *keywords) {
+    return invoke(kFn, call<kFn>, self, args, keywords, std::make_index_sequence<arity(kFn)>());
 }
 
-#define ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call<name>)), METH_FASTCALL | METH_KEYWORDS, nullptr}
-PyMethodDef kEntries[] = {ENTRY(tensor_sm100_fill),        ENTRY(tensor_sm100_arange),        ENTRY(tensor_sm100_copy),
-                          ENTRY(tensor_sm100_axpy),        ENTRY(tensor_sm100_gelu_forward),  ENTRY(tensor_sm100_gelu_backward),
-                          ENTRY(xent_sm100_forward),       ENTRY(xent_sm100_backward),        ENTRY(attn_sm100_saved_bytes),
-                          ENTRY(attn_sm100_backward_scratch_bytes)};
+#define ENTRY(name) {#name, call<name>}
+const struct {
+    const char *name;
+    ternaryfunc call;
+} kEntries[] = {ENTRY(tensor_sm100_fill),        ENTRY(tensor_sm100_arange),        ENTRY(tensor_sm100_copy),
+                ENTRY(tensor_sm100_axpy),        ENTRY(tensor_sm100_gelu_forward),  ENTRY(tensor_sm100_gelu_backward),
+                ENTRY(xent_sm100_forward),       ENTRY(xent_sm100_backward),        ENTRY(attn_sm100_saved_bytes),
+                ENTRY(attn_sm100_backward_scratch_bytes)};
 
-// entry_calls(class of ctypes functions) -> {name of the entry point: method of that class}
-PyObject *entry_calls(PyObject *, PyObject *plain) {
-    if (!PyType_Check(plain) || reinterpret_cast<PyTypeObject *>(plain)->tp_call == nullptr) {
-        PyErr_SetString(PyExc_TypeError, "expected the class of ctypes functions");
-        return nullptr;
+// shorten_calls({name of an entry point: class of its function alone, a Python class derived from ctypes' own})
+PyObject *shorten_calls(PyObject *, PyObject *classes) {
+    for (const auto &e : kEntries) {
+        PyObject *cls = PyDict_Check(classes) ? PyDict_GetItemString(classes, e.name) : nullptr;
+        if (cls == nullptr || !PyType_Check(cls) || !PyType_HasFeature(reinterpret_cast<PyTypeObject *>(cls), Py_TPFLAGS_HEAPTYPE) ||
+            reinterpret_cast<PyTypeObject *>(cls)->tp_base->tp_call == nullptr) {
+            PyErr_Format(PyExc_TypeError, "%s: expected a class derived from that of ctypes functions", e.name);
+            return nullptr;
+        }
+        reinterpret_cast<PyTypeObject *>(cls)->tp_call = e.call;
+        PyType_Modified(reinterpret_cast<PyTypeObject *>(cls));
     }
-    Py_INCREF(plain);
-    Py_XDECREF(reinterpret_cast<PyObject *>(g_plain));
-    g_plain = reinterpret_cast<PyTypeObject *>(plain);
-    PyObject *all = PyDict_New();
-    for (PyMethodDef &e : kEntries) {
-        PyObject *method = all != nullptr ? PyDescr_NewMethod(g_plain, &e) : nullptr;
-        if (method == nullptr || PyDict_SetItemString(all, e.ml_name, method) < 0) Py_CLEAR(all);
-        Py_XDECREF(method);
-        if (all == nullptr) return nullptr;
-    }
-    return all;
+    Py_RETURN_NONE;
 }
 
 // set_error(cls): the exception class raised for a non-zero status
@@ -394,7 +383,7 @@ PyObject *set_error(PyObject *, PyObject *cls) {
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(forward), FAST(backward), FAST(forward_into), FAST(backward_into), FAST(linear_forward),
                           FAST(linear_backward), FAST(layernorm_forward), FAST(layernorm_backward),
-                          {"set_error", set_error, METH_O, nullptr}, {"entry_calls", entry_calls, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                          {"set_error", set_error, METH_O, nullptr}, {"shorten_calls", shorten_calls, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "gptc_b200_calls", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
