@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const float *__restric
     }
 }
 
-// The same for up to 64 columns, a multiple of 4: 8 or 16 lanes per row, a 16-byte word each (B=32 T=1024 H=16 D=64 118 ->
-// 84 us, B=8 T=1024 H=4 D=48 7.6 -> 6.8; at D = 128 the kernel above is faster, 6.5 against 8.2 us for B=4 T=1024 H=6).
+// The same for up to 64 columns, a multiple of 4: 8 or 16 lanes per row, a 16-byte word each (B=32 T=1024 H=16 D=64 120 ->
+// 70 ... 77 us, B=8 T=1024 H=4 D=48 7.5 -> 5.4; at D = 128 the kernel above is faster, 6.5 against 8.2 us for B=4 T=1024 H=6).
 __global__ void __launch_bounds__(256) bwd_prepare_words_kernel(const float *__restrict__ dout, const float *__restrict__ out,
                                                                  float *__restrict__ delta, float *__restrict__ dqkv, bool zero_all,
                                                                  int lanes, int B, int T, int H, int D) {

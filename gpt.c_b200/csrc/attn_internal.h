@@ -69,7 +69,7 @@ cudaError_t launch_attn24_backward(const CUtensorMap &map_x, const __nv_bfloat16
 int attn24_backward_pieces(int B, int T, int H, int sms);
 
 // Tensor-core (tcgen05) kernels, D == 64.  The tensor maps cover the bf16 hi/lo planes:
-//   map_x : dims {3C, T, B, 2 planes}, box {64, 128, 1, 1}, 128-byte swizzle
+//   map_x : dims {3C, T, B, 2 planes}, box {64, 64, 1, 1}, 128-byte swizzle
 //   map_do: dims { C, T, B, 2 planes}, same box
 cudaError_t fast_fwd_set_attributes();
 cudaError_t fast_bwd_set_attributes();

@@ -737,7 +737,7 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
     Plan plan = plan_tiles(M, K, kb, sms);
     // Pieces of the contraction may fill the SMs better, although dx has to be zeroed first.  Any number where it is very long
     // (the vocabulary projection), else two, whose sum does not depend on their order, and if they are expected to save more
-    // than the estimate's error (M, N, K: 900, 5120, 1280 52 -> 33 us, 3000, 12032, 512 96 -> 80; without a margin 6000, 9999,
+    // than the estimate's error (M, N, K: 900, 5120, 1280 41 -> 26 us, 3000, 12032, 512 92 -> 78; without a margin 6000, 9999,
     // 768 214 -> 220).
     const bool very_long = kb >= 512;
     Plan cut = plan_pieces(M, K, kb, sms, 32, very_long ? 32 : 2);

@@ -75,7 +75,12 @@ extern "C" {
 /* forward and backward each enqueue a preparation kernel (the bf16 hi/lo split of qkv; the split
  * of dout with rowsum(dout*out) and the zero-fill of dq) followed by the core attention kernel.
  * These two flags enqueue only one of the two stages, e.g. to time them separately or to reuse a
- * `saved` buffer that is already filled.  Setting both is an error (ATTN_ERR_SHAPE). */
+ * `saved` buffer that is already filled.  Setting both is an error (ATTN_ERR_SHAPE).  Where one kernel does
+ * both stages' work (short sequences; general forward) a call without these flags enqueues only that one,
+ * with the same results.  The general backward of few long sequences takes a key tile's queries in two
+ * pieces only when both stages come in one call, for which the preparation also zeroes dk and dv: the core
+ * stage alone, which may be repeated on a prepared scratch buffer (dq is added to, dk and dv are written),
+ * is slower there, and dk and dv can differ in the last bits. */
 #define ATTN_FLAG_PREPARE_ONLY 2
 #define ATTN_FLAG_CORE_ONLY 4
 
