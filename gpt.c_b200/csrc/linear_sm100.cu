@@ -18,7 +18,7 @@
 //
 // What bounds the kernel: a 128 x 256 tile needs 48 KB per contraction block, and the SMs get 15 to 18 TB/s from L2
 // together (tensor pipe active 48 % in the forward with bf16 planes, 76 % in dW).  The result is written straight from
-// registers, a row per lane in 32-byte sectors: staging it for the copy engine costs shared memory that the pipeline
+// registers, 64 bytes of a row per pair of lanes: staging it for the copy engine costs shared memory that the pipeline
 // wants, bandwidth, and hand-overs between warps (QKV forward with bf16 planes 72 -> 67 us at 192 columns).
 //
 // Warp roles (384 threads, one CTA per SM, grid = number of SMs, tiles handed out round robin):
@@ -325,28 +325,47 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
                 }
-                if (kEpi == 0 && bias != nullptr) {
-                    const float mine = c == 0 ? bv[0] : c == 1 ? bv[1] : c == 2 ? bv[2 % kChunks] : bv[3 % kChunks];
-#pragma unroll
-                    for (int e = 0; e < 32; e++)
-                        r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, mine, e));
-                }
+                const float mine = c == 0 ? bv[0] : c == 1 ? bv[1] : c == 2 ? bv[2 % kChunks] : bv[3 % kChunks];
                 if (kEpi == 0 && !kDirect) {
-                    // straight from the registers: this lane's row, 32-byte sectors
-                    const int row = row0 + lane;
-                    if (row < p.M) {
-                        store_words<8>(c_direct + (size_t)row * p.ldc + col0, p.N - col0, p.wide, r);
-                        if (kPlanes) {
-                            uint32_t hp[16], lp[16];
+                    // Straight from the registers.  A pair of lanes holds two rows; they exchange halves, so that both have 16
+                    // columns of either row and a store instruction touches 16 rows instead of 32: L2 takes 32-byte pieces of
+                    // a line one by one at 4.0 TB/s, pieces of 64 bytes and more at 5.3 (K = 32, 8192 x 3072: 28 -> 22 us).
+                    const int odd = lane & 1, col = col0 + 16 * odd;
 #pragma unroll
-                            for (int e = 0; e < 16; e++)
-                                split_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]), hp[e], lp[e]);
-                            uint32_t *hi = planes + ((size_t)row * p.N + col0) / 2;
-                            store_words<4>(hi, (p.N - col0) / 2, p.wide_planes, hp);
-                            store_words<4>(hi + p.plane_words, (p.N - col0) / 2, p.wide_planes, lp);
+                    for (int e = 0; e < 16; e++) {
+                        const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? r[e] : r[16 + e], 1);
+                        r[e] = odd ? other : r[e];
+                        r[16 + e] = odd ? r[16 + e] : other;
+                    }
+                    if (bias != nullptr) {
+#pragma unroll
+                        for (int e = 0; e < 16; e++) {
+                            const float add = __shfl_sync(0xffffffffu, mine, 16 * odd + e);
+                            r[e] = __float_as_uint(__uint_as_float(r[e]) + add);
+                            r[16 + e] = __float_as_uint(__uint_as_float(r[16 + e]) + add);
+                        }
+                    }
+#pragma unroll
+                    for (int o = 0; o < 2; o++) {
+                        const int row = row0 + lane - odd + o;
+                        if (row >= p.M) continue;
+                        store_words<4>(c_direct + (size_t)row * p.ldc + col, p.N - col, p.wide, r + 16 * o);
+                        if (kPlanes) {
+                            uint32_t hp[8], lp[8];
+#pragma unroll
+                            for (int e = 0; e < 8; e++)
+                                split_bf16x2(__uint_as_float(r[16 * o + 2 * e]), __uint_as_float(r[16 * o + 2 * e + 1]), hp[e], lp[e]);
+                            uint32_t *hi = planes + ((size_t)row * p.N + col) / 2;
+                            store_words<2>(hi, (p.N - col) / 2, p.wide_planes, hp);
+                            store_words<2>(hi + p.plane_words, (p.N - col) / 2, p.wide_planes, lp);
                         }
                     }
                     continue;
+                }
+                if (kDirect && bias != nullptr) {
+#pragma unroll
+                    for (int e = 0; e < 32; e++)
+                        r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, mine, e));
                 }
                 const int up = kClasses ? p.a_shift[wk.cls] : 0;
                 if (kClasses && row0 < up) {
