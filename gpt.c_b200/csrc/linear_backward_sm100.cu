@@ -1,0 +1,499 @@
+// Backward of the Linear layer for sm_100a: dx = dy . W, dW += dy^T . x and db += column sums of dy in ONE launch.
+//
+// Replaces the two SGEMMs and the atomic bias reduction of linear_backward_cuda_kernel of gpt.c
+// (kernels/src/cuda/Linear.cu:64-92).  The products run on the tensor cores with TF32 operands read straight from the
+// fp32 tensors (linear_sm100.cu has the forward and says more about operands and pipeline).
+//
+// Why one launch: each product alone leaves SMs idle.  Tiles of dx = 8192 x 768 are 192 for 148 SMs, and every launch
+// starts with empty pipelines and ends with a last tile's way out (about 4.5 us).  dW is added into what is there, so its
+// contraction may be cut anywhere: every CTA first takes its tiles of dx, then as much of dW as makes all CTAs end together.
+// dy is read from shared memory a second time for db, in fp32, by two warps that have nothing else to do.  Before, three
+// launches, now (M, N, K in us, with db): 8192, 3072, 768 138 -> 124; 8192, 2304, 768 115 -> 95; 8192, 768, 768 51 -> 39;
+// 1500, 6400, 1600 128 -> 106; 1500, 1600, 1600 45 -> 34; 1705, 129, 4288 32 -> 25; 12, 288, 128 10.3 -> 8.4.
+// What bounds it: shared memory, which takes a block's 48 KB in and hands them to the tensor cores once (768 cycles at 128
+// bytes each, 512 of products), and the power cap: 8192 x 3072 x 768 runs at 630 TFLOP/s.
+//
+//     dx[M,K]  = dy[M,N] . W[N,K]      A: dy, K-major (over N)   B: W, MN-major
+//     dW[N,K] += dy[M,N]^T . x[M,K]    A: dy, MN-major           B: x, MN-major   (contraction over M, cut into ranges)
+//
+// Both results have K columns; a tile is 128 rows by up to 256 columns, and the columns are dealt out evenly in blocks of
+// 32 (K = 1600: six tiles of 224 and one of 256 columns).
+//
+// Warp roles (384 threads, one CTA per SM):
+//   warp 0      TMA producer
+//   warp 1      MMA issuer
+//   warp 2      tensor-memory allocation, db
+//   warp 3      db
+//   warps 4-11  epilogue: dx from registers, dW through a staging buffer to a bulk tensor reduction
+// All waits on barriers are bounded (tc05.cuh).
+#include <math.h>
+
+#include <type_traits>
+
+#include "linear_tf32.cuh"
+
+namespace lin {
+namespace {
+
+using namespace tc05;
+
+constexpr int kThreads = 384, kEpiWarps = 8;
+constexpr int kBN = 256;                             // columns of an accumulator
+constexpr int kMostStages = 6, kRingBytes = 192 * 1024;  // pipeline: as many stages as fit, of 16 KB of A and up to 32 KB of B
+
+enum Site : int { SITE_EMPTY = 231, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_DB, SITE_SMEM_ALIGN };
+
+struct __align__(1024) Smem {
+    uint8_t ring[kRingBytes];
+    uint8_t out[kEpiWarps][4096];  // output staging of the epilogue warps: 32 rows x 128 bytes
+    uint64_t full[kMostStages], empty[kMostStages];
+    uint64_t acc_full[2], acc_empty[2];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+struct Maps {
+    CUtensorMap dy_k, dy_mn;     // A of dx and of dW
+    CUtensorMap w[2], x[2];      // B of dx and of dW, for tiles of p.cols and of p.cols + 1 blocks of 32 columns
+    CUtensorMap dw;
+};
+
+// dW's tiles are cut across the contraction, and their ranges dealt out to teams of CTAs.  The members of a team work on the same
+// range of neighbouring tiles at the same time, one tile each, so that what these tiles share comes from HBM once.
+struct Problem {
+    int M, N, K;
+    int tiles_n, cols, wider;  // column tiles; blocks of 32 columns in each; the first `wider` have one more
+    int dx_tiles, dx_kb;       // tiles of dx, handed out round robin; contraction blocks of one
+    int dw_kb;                 // contraction blocks of a tile of dW
+    int team, down;            // CTAs of a team; their tiles are below (1) or beside each other (0)
+    int strips;                // groups of `team` tiles
+    int teams, fewer;          // the first `fewer` teams (those with a tile of dx more) take share_fewer of dW, the others share
+    uint32_t share_fewer, share;  // in units of 2^-32
+    int snap;
+    int uncut;                 // dW alone, whole tiles round robin
+    int stages, stage_bytes;
+    int wide;                  // rows of dx start on 32-byte boundaries
+};
+
+// Counted through all strips, team c takes the contraction blocks from range_start(c) to range_start(c + 1).  A range does not
+// begin or end within `snap` blocks of a tile's edge.
+__host__ __device__ __forceinline__ int range_start(const Problem &p, int c) {
+    const int total = p.strips * p.dw_kb;
+    if (c >= p.teams) return total;
+    const uint32_t part = c < p.fewer ? c * p.share_fewer : p.fewer * p.share_fewer + (c - p.fewer) * p.share;
+    const int u = (int)(((unsigned long long)(uint32_t)total * part) >> 32);
+    const int in = u % p.dw_kb;
+    return in < p.snap ? u - in : p.dw_kb - in < p.snap ? u + p.dw_kb - in : u;
+}
+
+// A tile of dx, or a tile of dW with a range of its contraction.
+struct Item {
+    bool dw;
+    int m0, tn, n0, cols, kb0, kb1;
+};
+struct Items {
+    int cta, ctas;
+    int i;        // tiles of dx taken so far
+    int at, end;  // the team's range
+    int member;
+    __host__ __device__ __forceinline__ Items(const Problem &p, int cta, int ctas) : cta(cta), ctas(ctas), i(0) {
+        const int team = cta / p.team;
+        member = cta - team * p.team;
+        at = range_start(p, team), end = range_start(p, team + 1);
+    }
+    __host__ __device__ __forceinline__ bool next(const Problem &p, Item &t) {
+        const int w = cta + i * ctas;
+        int tm;
+        if (p.uncut) {
+            if (w >= p.strips) return false;
+            t.dw = true;
+            tm = w / p.tiles_n, t.tn = w - tm * p.tiles_n;
+            t.kb0 = 0, t.kb1 = p.dw_kb;
+            i++;
+        } else if (w < p.dx_tiles) {
+            t.dw = false;
+            tm = w / p.tiles_n, t.tn = w - tm * p.tiles_n;
+            t.kb0 = 0, t.kb1 = p.dx_kb;
+            i++;
+        } else {
+            if (at >= end) return false;
+            t.dw = true;
+            const int strip = at / p.dw_kb;
+            t.kb0 = at - strip * p.dw_kb;
+            const int take = p.dw_kb - t.kb0 < end - at ? p.dw_kb - t.kb0 : end - at;
+            t.kb1 = t.kb0 + take;
+            at += take;
+            if (p.down) {
+                t.tn = strip, tm = member;
+            } else {
+                const int tile = strip * p.team + member;
+                tm = tile / p.tiles_n, t.tn = tile - tm * p.tiles_n;
+            }
+        }
+        t.m0 = tm * kBM;
+        t.cols = p.cols + (t.tn < p.wider ? 1 : 0);
+        t.n0 = 32 * (t.tn * p.cols + (t.tn < p.wider ? t.tn : p.wider));
+        return true;
+    }
+};
+
+// A role's place in the ring of pipeline stages.
+struct Place {
+    int st = 0;
+    uint32_t round = 0;
+    __device__ __forceinline__ void next(int stages) {
+        if (++st == stages) st = 0, round++;
+    }
+};
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    const float2 lo = add2(make_float2(a.x, a.y), make_float2(b.x, b.y)), hi = add2(make_float2(a.z, a.w), make_float2(b.z, b.w));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx, float *__restrict__ db, Problem p, int *status) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    if ((smem_u32(smem_raw) & 1023u) != 0) {
+        if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_TIMEOUT_BASE + SITE_SMEM_ALIGN);
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WaitCtx ctx{&sm.abort_flag, status};
+
+    if (threadIdx.x == 0) {
+        sm.abort_flag = 0;
+        for (int i = 0; i < kMostStages; i++) {
+            mbar_init(&sm.full[i], 1);
+            mbar_init(&sm.empty[i], db != nullptr ? 3 : 1);  // the products, and the warps that sum up db
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&sm.acc_full[i], 1);
+            mbar_init(&sm.acc_empty[i], kEpiWarps);
+        }
+        fence_barrier_init();
+    }
+    if (warp == 2) tmem_alloc_then_launch_dependents(&sm.tmem_base, 2 * kBN);
+    if (warp == 3 && lane == 0) {
+        if (p.dx_tiles > 0) {
+            tma_prefetch_desc(&maps.dy_k);
+            tma_prefetch_desc(&maps.w[0]);
+        }
+        tma_prefetch_desc(&maps.dy_mn);
+        tma_prefetch_desc(&maps.x[0]);
+        tma_prefetch_desc(&maps.dw);
+    }
+    Items items(p, (int)blockIdx.x, (int)gridDim.x);  // the first item, before the wait for the previous kernel
+    Item t;
+    bool more = items.next(p, t);
+    pdl_wait();  // every thread, before its first access to global memory
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = sm.tmem_base;
+
+    if (warp == 0) {
+        // ------------------------------ TMA producer ------------------------------
+        if (lane == 0) {
+            Place at;
+            bool ok = true;
+            for (; ok && more; more = items.next(p, t)) {
+                const int wide = t.cols - p.cols;
+                const CUtensorMap *map_b = t.dw ? &maps.x[wide] : &maps.w[wide];
+                for (int kb = t.kb0; kb < t.kb1; kb++, at.next(p.stages)) {
+                    const int st = at.st;
+                    if (at.round > 0 && !mbar_wait(&sm.empty[st], (at.round - 1) & 1, ctx, SITE_EMPTY)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t *a = sm.ring + st * p.stage_bytes;
+                    mbar_expect_tx(&sm.full[st], kATileBytes + t.cols * 4096);
+                    // K-major: map {contraction, rows}, box {32, 128}.  MN-major: blocks of 32 rows, each
+                    // [32 contraction steps x 128 bytes].
+                    if (t.dw) tma_load_4d(a, &maps.dy_mn, &sm.full[st], 0, kb * kBK, t.m0 / 32, 0);
+                    else tma_load_4d(a, &maps.dy_k, &sm.full[st], kb * kBK, t.m0, 0, 0);
+                    tma_load_4d(a + kATileBytes, map_b, &sm.full[st], 0, kb * kBK, t.n0 / 32, 0);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------ MMA issuer ------------------------------
+        const uint32_t leader = elect_leader();
+        Place at;
+        int j = 0;
+        bool ok = true;
+        for (; ok && more; more = items.next(p, t)) {
+            const int acc = j & 1;
+            if (j >= 2 && !mbar_wait_warp(&sm.acc_empty[acc], ((j >> 1) - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
+            tc_fence_after_sync();
+            const uint32_t d = tmem + (uint32_t)acc * kBN;
+            // one loop per product, so that its operands' layouts are constants: what this warp issues per cycle is what the
+            // tensor cores live on
+            auto products = [&](auto dw) {
+                constexpr bool kDW = decltype(dw)::value;
+                const uint32_t idesc = idesc_tf32(kBM, 0, kDW ? 1 : 0, 1) | (uint32_t)(t.cols * 4) << 17;
+                for (int kb = t.kb0; kb < t.kb1; kb++, at.next(p.stages)) {
+                    const int st = at.st;
+                    if (!mbar_wait_warp(&sm.full[st], at.round & 1, ctx, SITE_FULL)) return false;
+                    tc_fence_after_sync();
+                    const uint32_t a = smem_u32(sm.ring) + st * p.stage_bytes;
+                    // MN-major tiles: 32-row blocks 4096 bytes apart, groups of 4 contraction steps 512 bytes apart
+                    const uint64_t ad = kDW ? smem_desc_sw128_base32(a, 4096, 512)
+                                            : smem_desc_sw128(a, 16, 1024);
+                    const uint64_t bd = smem_desc_sw128_base32(a + kATileBytes, 4096, 512);
+#pragma unroll
+                    for (int k = 0; k < kBK / 8; k++)
+                        mma_tf32_lead(leader, d, desc_advance(ad, k * (kDW ? 1024 : 32)), desc_advance(bd, k * 1024), idesc,
+                                      (kb > t.kb0 || k > 0) ? 1u : 0u);
+                    tc_commit_lead(leader, &sm.empty[st]);
+                }
+                return true;
+            };
+            ok = t.dw ? products(std::true_type()) : products(std::false_type());
+            if (!ok) break;
+            tc_commit_lead(leader, &sm.acc_full[acc]);
+            j++;
+        }
+    } else if (warp < 4) {
+        // ------------------------------ db ------------------------------
+        // Column sums of dy, from the A tiles of dW.  The column tiles of the same 128 columns of dy share them out in blocks of
+        // 32, since it slows a tile down to have its A read twice (all four blocks by the first column tile: 8192 x 3072 x 768
+        // 134 us, shared out 131, among two warps 124, without db 122).  A lane reads 16 bytes of a row (of one value of M):
+        // rows lane / 8 + 4 i, the 16-byte word lane % 8, which the swizzle makes the columns from `col` on.  Eight rows are
+        // added up first, eight such sums next, so that long sums don't lose more than short ones.
+        if (db != nullptr) {
+            const int col = ((((lane & 7) >> 1) ^ (lane >> 3)) << 3) + ((lane & 1) << 2);
+            Place at;
+            bool ok = true;
+            for (; ok && more; more = items.next(p, t)) {
+                uint32_t mine = 0;
+#pragma unroll
+                for (int b = 0; b < 4; b++) mine |= t.dw && (b & 1) == (warp & 1) && b * (p.tiles_n < 4 ? p.tiles_n : 4) / 4 == t.tn ? 1u << b : 0u;
+                float4 all[4] = {}, some[4] = {};
+                for (int kb = t.kb0; kb < t.kb1; kb++, at.next(p.stages)) {
+                    const int st = at.st;
+                    if (!mbar_wait_warp(&sm.full[st], at.round & 1, ctx, SITE_DB)) {
+                        ok = false;
+                        break;
+                    }
+                    if (mine != 0) {
+#pragma unroll
+                        for (int b = 0; b < 4; b++) {
+                            if (!(mine >> b & 1)) continue;
+                            const float4 *rows = reinterpret_cast<const float4 *>(sm.ring + st * p.stage_bytes + b * 4096) + lane;
+                            float4 v[8];
+#pragma unroll
+                            for (int i = 0; i < 8; i++) v[i] = rows[32 * i];
+                            some[b] = add4(some[b], add4(add4(add4(v[0], v[1]), add4(v[2], v[3])), add4(add4(v[4], v[5]), add4(v[6], v[7]))));
+                        }
+                        if ((kb & 7) == 7 || kb + 1 == t.kb1) {
+#pragma unroll
+                            for (int b = 0; b < 4; b++) all[b] = add4(all[b], some[b]), some[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                    }
+                    if (lane == 0) mbar_arrive(&sm.empty[st]);
+                }
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    if (!(mine >> b & 1)) continue;
+                    float *s = reinterpret_cast<float *>(&all[b]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {  // the lanes with the same columns
+                        s[e] += __shfl_xor_sync(0xffffffffu, s[e], 10);
+                        s[e] += __shfl_xor_sync(0xffffffffu, s[e], 20);
+                    }
+                    const int n = t.m0 + 32 * b + col;
+                    if (lane < 8) {
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            if (n + e < p.N) atomicAdd(db + n + e, s[e]);
+                    }
+                }
+            }
+        }
+    } else if (warp >= 4) {
+        // ------------------------------ epilogue ------------------------------
+        // Every warp takes 32 rows (its tensor-memory lane quarter) and half of the blocks of columns.  No warp waits for
+        // another one.
+        const int quarter = warp & 3, half = (warp - 4) >> 2;
+        uint8_t *buf = sm.out[warp - 4];
+        const uint32_t lane_addr = (uint32_t)(quarter << 5) << 16;
+        int j = 0;
+        for (; more; more = items.next(p, t)) {
+            const int acc = j & 1;
+            if (!mbar_wait_warp(&sm.acc_full[acc], (j >> 1) & 1, ctx, SITE_ACC_FULL)) break;
+            tc_fence_after_sync();
+            const int row0 = t.m0 + 32 * quarter;
+            const int c0 = half ? (t.cols + 1) / 2 : 0, c1 = half ? t.cols : (t.cols + 1) / 2;
+            auto read_out = [&] {  // the tensor cores may reuse the accumulator
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
+            };
+            if (c0 == c1) read_out();
+#pragma unroll 1
+            for (int c = c0; c < c1; c++) {
+                const int col0 = t.n0 + 32 * c;
+                uint32_t r[32];
+                tmem_ld32(tmem + lane_addr + (uint32_t)acc * kBN + 32 * c, r);
+                tmem_wait_ld();
+                if (c + 1 == c1) read_out();
+                if (!t.dw) {
+                    const int odd = lane & 1, col = col0 + 16 * odd;
+                    exchange_halves(odd, r);
+#pragma unroll
+                    for (int o = 0; o < 2; o++) {
+                        const int row = row0 + lane - odd + o;
+                        if (row < p.M) store_words<4>(dx + (size_t)row * p.K + col, p.K - col, p.wide, r + 16 * o);
+                    }
+                    continue;
+                }
+                if (lane == 0) bulk_wait_read_all();  // the copy engine has read the buffer out
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; q++)  // one row of 128 bytes per lane, 16-byte words swizzled
+                    *reinterpret_cast<uint4 *>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                        make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_reduce_add_3d(buf, &maps.dw, col0, row0, 0);
+                    bulk_commit();
+                }
+            }
+            j++;
+        }
+        if (lane == 0) bulk_wait_read_all();  // shared memory stays until it has been read
+    }
+
+    // ------------------------------ tear-down ------------------------------
+    if (sm.abort_flag) __nanosleep(50000);
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 2) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, 2 * kBN);
+    }
+}
+
+// ---- host side ----
+
+// Nanoseconds of a contraction block of a tile `cols` blocks of 32 columns wide while `busy` SMs of `sms` work on such tiles,
+// of what a tile takes besides, and of adding pieces of dW to memory.  Fitted to dW alone at nine shapes, 5 widths, 1 to 11
+// pieces (2795 x 3200 x 640: cut anywhere, 7 blocks wide 24.8 us, one whole piece of 5 or 4 blocks per CTA 30.8 and 28.6;
+// 8192 x 768 x 768: 8 pieces of 18 tiles 20.3, cut anywhere 23.8).
+double block_ns(int cols, int busy, int sms) {
+    const double alone = 186 + 19 * cols, fed = (190.0 + 26 * cols) * busy / sms;
+    return fed > alone ? fed : alone;
+}
+double tile_ns(int cols) { return cols > 6 ? 2000 : cols > 4 ? 900 : 400; }
+double adding_ns(double pieces, int cols) { return pieces * cols * 16384 * 150e-6; }
+
+Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
+    Problem p = {};
+    p.M = M, p.N = N, p.K = K;
+    p.tiles_n = plan.tiles_n, p.cols = K / 32 / plan.tiles_n, p.wider = K / 32 % plan.tiles_n;
+    p.dx_tiles = plan.dx_tiles, p.dx_kb = plan.dx_kb, p.dw_kb = plan.dw_kb;
+    p.team = plan.team, p.down = plan.down, p.strips = plan.strips, p.teams = plan.teams, p.fewer = plan.fewer;
+    const double all = plan.fewer * plan.share_fewer + (plan.teams - plan.fewer) * plan.share;
+    // rounded up, so that shares of whole tiles begin where tiles do
+    p.share_fewer = (uint32_t)ceil(plan.share_fewer / all * 4294967296.0);
+    p.share = (uint32_t)fmin(ceil(plan.share / all * 4294967296.0), 4294967295.0);
+    // a few tiles of few blocks are cut anywhere, many are not
+    p.snap = p.dw_kb >= 16 ? 4 : p.strips >= p.teams ? (p.dw_kb < 8 ? p.dw_kb : 2) : 0;
+    p.uncut = p.dx_tiles == 0 && p.team == 1 && p.snap == p.dw_kb;
+    p.stage_bytes = kATileBytes + (p.cols + (p.wider > 0)) * 4096;
+    p.stages = kRingBytes / p.stage_bytes < kMostStages ? kRingBytes / p.stage_bytes : kMostStages;
+    return p;
+}
+
+}  // namespace
+
+// The split of the work and the time in nanoseconds it is expected to take: see linear_tf32.cuh.
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms) {
+    BackwardPlan best = {};
+    const int blocks = K / 32;
+    for (int width = 8; width >= 4; width--) {
+        const int tiles_n = (blocks + width - 1) / width;
+        if (tiles_n == best.tiles_n) continue;
+        BackwardPlan c = {};
+        c.tiles_n = tiles_n;
+        const int cols = (blocks + tiles_n - 1) / tiles_n;
+        const double tb = block_ns(cols, sms, sms), te = tile_ns(cols);
+        const int rows_m = (M + kBM - 1) / kBM, rows_n = (N + kBM - 1) / kBM;
+        c.dx_tiles = want_dx ? rows_m * tiles_n : 0;
+        c.dx_kb = (N + kBK - 1) / kBK;
+        c.dw_kb = (M + kBK - 1) / kBK;
+        const int dw_tiles = rows_n * tiles_n;
+        // Where dy and x don't stay in L2 together, a team shares the larger of them, if that keeps most SMs busy.
+        c.down = N < K, c.team = c.down ? rows_n : tiles_n;
+        if (4.0 * M * ((double)N + K) < (64 << 20) || c.team > sms || sms / c.team * c.team < sms * 24 / 25) c.down = 0, c.team = 1;
+        c.strips = dw_tiles / c.team;
+        c.teams = sms / c.team;
+        if (!want_dx && (long long)c.strips * c.dw_kb < c.teams) c.teams = c.strips * c.dw_kb;
+        const int ctas = c.teams * c.team;
+        const double dx_ns = c.dx_kb * tb + te;
+        // every CTA has about one piece of a tile more than its share of whole ones
+        const double even = (c.dx_tiles * dx_ns + dw_tiles * (c.dw_kb * tb + te)) / ctas + te;
+        const int most = (c.dx_tiles + ctas - 1) / ctas;
+        c.fewer = (c.dx_tiles % ctas + c.team - 1) / c.team;
+        // what is left for dW, in blocks, in a CTA with `most` tiles of dx and in one with a tile less
+        c.share_fewer = (even - most * dx_ns - te) / tb, c.share = c.share_fewer + (c.fewer ? dx_ns / tb : 0);
+        if (c.share_fewer < 3) c.share_fewer = 0;
+        if (c.share < 1) c.share = 1;
+        double time = (even > most * dx_ns ? even : most * dx_ns) + adding_ns(dw_tiles + ctas, cols);
+        const int most_pieces = want_dx ? 0 : sms / dw_tiles < c.dw_kb ? sms / dw_tiles : c.dw_kb;
+        auto as_deep = [&](int pieces) {  // fewest pieces that are no longer
+            const int depth = (c.dw_kb + pieces - 1) / pieces;
+            return (c.dw_kb + depth - 1) / depth;
+        };
+        for (int tries = 0, pieces = most_pieces > 0 ? as_deep(most_pieces) : 0; tries < 4 && pieces > 0; tries++) {
+            // whole pieces of the same size, as many as SMs or fewer: no CTA has parts of two tiles, all of them the same rows
+            const int busy = pieces * dw_tiles;
+            const double whole = (c.dw_kb + pieces - 1) / pieces * block_ns(cols, busy, sms) + te + adding_ns(busy, cols);
+            if (whole <= time) {
+                c.team = 1, c.down = 0, c.strips = dw_tiles, c.teams = busy, c.share = 1;
+                time = whole;
+            }
+            pieces = pieces > 1 ? as_deep(pieces - 1) : 0;
+        }
+        const double ns = 4470 + time;
+        c.ns = ns < 2e9 ? (int)ns : 2000000000;
+        if (best.ns == 0 || c.ns < best.ns) best = c;
+    }
+    return best;
+}
+
+int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
+                    int M, int N, int np, int K, int *status, cudaStream_t s) {
+    static bool attr_done[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear backward kernel");
+    if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+        e = cudaFuncSetAttribute(linear_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64) attr_done[dev] = true;
+    }
+    Problem p = make_problem(plan, M, N, K);
+    p.wide = (reinterpret_cast<uintptr_t>(dx) & 31u) == 0;
+    Maps maps;
+    int rc;
+    if ((rc = map_mn_major_blocks(&maps.dy_mn, dy, M, np, 4)) != 0) return rc;
+    if ((rc = map_out_f32(&maps.dw, dw, N, K)) != 0) return rc;
+    if ((rc = map_mn_major_blocks(&maps.x[0], x, M, K, p.cols)) != 0) return rc;
+    if (p.wider && (rc = map_mn_major_blocks(&maps.x[1], x, M, K, p.cols + 1)) != 0) return rc;
+    maps.w[0] = maps.x[0], maps.dy_k = maps.dy_mn;  // not looked at without dx
+    if (dx) {
+        if ((rc = map_mn_major_blocks(&maps.w[0], w, w_rows, K, p.cols)) != 0) return rc;
+        if (p.wider && (rc = map_mn_major_blocks(&maps.w[1], w, w_rows, K, p.cols + 1)) != 0) return rc;
+        if ((rc = map_k_major(&maps.dy_k, dy, M, np, 128)) != 0) return rc;
+    }
+    return (int)attn::launch_after_previous(linear_backward_kernel, dim3(plan.teams * plan.team), dim3(kThreads), sizeof(Smem), s, maps, dx, db, p, status);
+}
+
+}  // namespace lin

@@ -12,6 +12,8 @@
 //     forward  y [M,N]  = x [M,K] . W[N,K]^T        A: x, K-major          B: W,  K-major
 //     dx       dx[M,K]  = dy[M,N] . W[N,K]          A: dy, K-major (over N) B: W,  MN-major
 //     dW       dW[N,K] += dy[M,N]^T . x[M,K]        A: dy, MN-major         B: x,  MN-major  (split over M)
+// This file has the forward, dx where it is wanted alone or has few rows, and both gradients where rows of dy are not 16-byte
+// aligned; elsewhere linear_backward_sm100.cu makes them in one launch.
 // (K-major: the contraction index is the contiguous one.)  Contraction blocks are 32 fp32 values (one 128-byte
 // swizzled row).  A tile is 128 rows by 128, 192 or 256 columns, with as many pipeline stages as shared memory holds;
 // plan_tiles picks the width.
@@ -132,26 +134,6 @@ __device__ __forceinline__ void clear_leading(uint8_t *tile, int columns, int la
     }
     fence_proxy_async_smem();
     __syncwarp();
-}
-
-// Writes 4 * kQuads consecutive 32-bit words to dst, as far as `left` words go (a multiple of
-// 4): 32 bytes per store where dst allows it, else 16.
-template <int kQuads>
-__device__ __forceinline__ void store_words(void *dst, int left, int wide, const uint32_t *r) {
-    uint32_t *d = static_cast<uint32_t *>(dst);
-    if (wide) {
-#pragma unroll
-        for (int q = 0; q < kQuads / 2; q++)
-            if (8 * q < left)
-                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(d + 8 * q), "r"(r[8 * q]),
-                             "r"(r[8 * q + 1]), "r"(r[8 * q + 2]), "r"(r[8 * q + 3]), "r"(r[8 * q + 4]), "r"(r[8 * q + 5]),
-                             "r"(r[8 * q + 6]), "r"(r[8 * q + 7])
-                             : "memory");
-    } else {
-#pragma unroll
-        for (int q = 0; q < kQuads; q++)
-            if (4 * q < left) *reinterpret_cast<uint4 *>(d + 4 * q) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-    }
 }
 
 // kEpi 0: C = acc (+ bias), optional bf16 planes; kEpi 1: C += acc (bulk reduction)
@@ -327,16 +309,8 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                 }
                 const float mine = c == 0 ? bv[0] : c == 1 ? bv[1] : c == 2 ? bv[2 % kChunks] : bv[3 % kChunks];
                 if (kEpi == 0 && !kDirect) {
-                    // Straight from the registers.  A pair of lanes holds two rows; they exchange halves, so that both have 16
-                    // columns of either row and a store instruction touches 16 rows instead of 32: L2 takes 32-byte pieces of
-                    // a line one by one at 4.0 TB/s, pieces of 64 bytes and more at 5.3 (K = 32, 8192 x 3072: 28 -> 22 us).
                     const int odd = lane & 1, col = col0 + 16 * odd;
-#pragma unroll
-                    for (int e = 0; e < 16; e++) {
-                        const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? r[e] : r[16 + e], 1);
-                        r[e] = odd ? other : r[e];
-                        r[16 + e] = odd ? r[16 + e] : other;
-                    }
+                    exchange_halves(odd, r);
                     if (bias != nullptr) {
 #pragma unroll
                         for (int e = 0; e < 16; e++) {
@@ -531,13 +505,6 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(float *__restrict__ dst, 
 
 // ---- host side ----
 
-int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, size_t pitch = 0) {
-    if (pitch == 0) pitch = (size_t)cols;
-    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
-    const cuuint64_t strides[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * 4 * (cuuint64_t)rows};
-    const cuuint32_t box[3] = {32, 32, 1};
-    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
-}
 Problem make_problem(int M, int N, int K, int bn, int splits) {
     Problem p;
     p.M = M, p.N = N, p.K = K, p.bn = bn;
@@ -751,9 +718,15 @@ int gradients_by_row_class(const float *dy, const float *x, const float *w, floa
 }
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
-int input_gradient(const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status, cudaStream_t s) {
+struct InputGradient {
+    Plan tiles;
+    int split;  // > 0: the kernel for results of few tiles, with that many CTAs per tile
+    int ns;
+};
+InputGradient plan_input_gradient(int M, int np, int K, int sms) {
     const int kb = np / kBK;
-    Plan plan = plan_tiles(M, K, kb, sms);
+    InputGradient r;
+    r.tiles = plan_tiles(M, K, kb, sms);
     // Pieces of the contraction may fill the SMs better, although dx has to be zeroed first.  Any number where it is very long
     // (the vocabulary projection), else two, whose sum does not depend on their order, and if they are expected to save more
     // than the estimate's error (M, N, K: 900, 5120, 1280 41 -> 26 us, 3000, 12032, 512 92 -> 78; without a margin 6000, 9999,
@@ -761,9 +734,18 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
     const bool very_long = kb >= 512;
     Plan cut = plan_pieces(M, K, kb, sms, 32, very_long ? 32 : 2);
     cut.ns += 2500 + (int)((long long)M * K * 4 / 5500);
-    if (cut.splits > 1 && (very_long ? cut.ns : at_most_int(cut.ns * 21ll / 20)) < plan.ns) plan = cut;
-    int split = 1, rc;
-    if (plan_split(M, K, np, sms, &split) < plan.ns) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, split, sms, status, s);
+    if (cut.splits > 1 && (very_long ? cut.ns : at_most_int(cut.ns * 21ll / 20)) < r.tiles.ns) r.tiles = cut;
+    int split = 1;
+    const int split_ns = plan_split(M, K, np, sms, &split);
+    r.split = split_ns < r.tiles.ns ? split : 0;
+    r.ns = r.split ? split_ns : r.tiles.ns;
+    return r;
+}
+int input_gradient(const InputGradient &how, const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status,
+                   cudaStream_t s) {
+    if (how.split) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, how.split, sms, status, s);
+    const Plan &plan = how.tiles;
+    int rc;
     CUtensorMap ma, mb, mc;
     Problem p = make_problem(M, K, np, plan.bn, plan.splits);
     if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
@@ -774,6 +756,21 @@ int input_gradient(const float *g, const float *w, float *dx, int M, int N, int 
     if ((rc = map_out_f32(&mc, dx, M, K)) != 0) return rc;
     if ((rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
     return launch<false, true, 1>(ma, mb, mc, nullptr, dx, nullptr, p, status, s);
+}
+
+// Whether a result lies over something that another product of the same call reads or writes: then the products have to
+// follow each other, dx first and db last.
+bool overlapping(const float *dy, const float *x, const float *w, const float *dx, const float *dw, const float *db, int M, int N, int K) {
+    struct Range {
+        const float *at;
+        size_t n;
+    };
+    const Range r[6] = {{dx, (size_t)M * K}, {dw, (size_t)N * K}, {db, (size_t)N},
+                        {dy, (size_t)M * N}, {x, (size_t)M * K},  {w, (size_t)N * K}};
+    for (int i = 0; i < 3; i++)
+        for (int j = i + 1; j < 6; j++)
+            if (r[i].at && r[j].at && r[i].at < r[j].at + r[j].n && r[j].at < r[i].at + r[i].n) return true;
+    return false;
 }
 
 }  // namespace
@@ -848,20 +845,22 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         if (rc != 0) return rc;
         g = static_cast<const float *>(scratch);
     }
-    if (!classes && dx && (rc = input_gradient(g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
-    CUtensorMap ma, mb, mc;
-    if (!classes && dw) {
-        // dw[N,K] += dy[M,N]^T . x[M,K]: contraction over M, split so that every SM has work (rows of the
-        // result past N are dropped by the copy engine)
-        const Plan plan = plan_pieces(N, K, (M + kBK - 1) / kBK, sms, 1);
-        Problem pdw = make_problem(N, K, M, plan.bn, plan.splits);
-        pdw.a_one = map_mn_major_blocks(&ma, g, M, np, 4) == 0;
-        if (!pdw.a_one && (rc = map_mn_major(&ma, g, M, np)) != 0) return rc;
-        pdw.b_one = map_mn_major_blocks(&mb, x, M, K, plan.bn / 32) == 0;
-        if (!pdw.b_one && (rc = map_mn_major(&mb, x, M, K)) != 0) return rc;
-        if ((rc = map_out_f32(&mc, dw, N, K)) != 0) return rc;
-        rc = launch<true, true, 1>(ma, mb, mc, nullptr, dw, nullptr, pdw, status, s);
-        if (rc != 0) return rc;
+    if (!classes) {
+        const bool in_parts = dw && overlapping(dy, x, w, dx, dw, db, M, N, K);
+        InputGradient alone{};
+        if (dx) alone = plan_input_gradient(M, np, K, sms);
+        BackwardPlan rest{}, both{};
+        if (dw) rest = plan_backward(M, N, K, false, sms);
+        // dx has the same bits with and without dW: one launch only where dx alone would be whole tiles too
+        if (dw && dx && !in_parts && !alone.split && alone.tiles.splits == 1) both = plan_backward(M, N, K, true, sms);
+        const bool together = both.ns > 0 && both.ns < alone.ns + rest.ns;
+        if (dx && !together && (rc = input_gradient(alone, g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
+        if (dw) {
+            rc = launch_backward(together ? both : rest, g, x, w, N, together ? dx : nullptr, dw, in_parts ? nullptr : db, M, N, np, K,
+                                 status, s);
+            if (rc != 0) return rc;
+            if (!in_parts) return ATTN_OK;
+        }
     }
     if (db) {
         // eight blocks per SM, so that enough loads are on their way (six columns of 32 blocks took 9.2 us at

@@ -41,6 +41,39 @@ __device__ __forceinline__ uint64_t smem_desc_sw128_base32(uint32_t smem_addr, u
     return d;
 }
 
+// Writes 4 * kQuads consecutive 32-bit words to dst, as far as `left` words go (a multiple of
+// 4): 32 bytes per store where dst allows it, else 16.
+template <int kQuads>
+__device__ __forceinline__ void store_words(void *dst, int left, int wide, const uint32_t *r) {
+    uint32_t *d = static_cast<uint32_t *>(dst);
+    if (wide) {
+#pragma unroll
+        for (int q = 0; q < kQuads / 2; q++)
+            if (8 * q < left)
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(d + 8 * q), "r"(r[8 * q]),
+                             "r"(r[8 * q + 1]), "r"(r[8 * q + 2]), "r"(r[8 * q + 3]), "r"(r[8 * q + 4]), "r"(r[8 * q + 5]),
+                             "r"(r[8 * q + 6]), "r"(r[8 * q + 7])
+                             : "memory");
+    } else {
+#pragma unroll
+        for (int q = 0; q < kQuads; q++)
+            if (4 * q < left) *reinterpret_cast<uint4 *>(d + 4 * q) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+    }
+}
+
+// The 32 columns of a row that every lane holds leave from registers: a pair of lanes (odd: the second one) holds two rows and
+// exchanges halves, so that both have 16 columns of either row, r[0..15] of the even lane's and r[16..31] of the odd one's,
+// and a store instruction touches 16 rows instead of 32.  L2 takes 32-byte pieces of a line one by one at 4.0 TB/s, pieces of
+// 64 bytes and more at 5.3 (forward of K = 32, 8192 x 3072: 28 -> 22 us).
+__device__ __forceinline__ void exchange_halves(int odd, uint32_t (&r)[32]) {
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? r[e] : r[16 + e], 1);
+        r[e] = odd ? other : r[e];
+        r[16 + e] = odd ? r[16 + e] : other;
+    }
+}
+
 // ---- host side ----
 
 // Operand read K-major: matrix [rows, kc] row-major (kc contiguous = contraction); boxes of 32 x box_rows.
@@ -74,6 +107,27 @@ inline int map_mn_major(CUtensorMap *map, const float *base, int kc, int rows, s
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
 }
+inline int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, size_t pitch = 0) {
+    if (pitch == 0) pitch = (size_t)cols;
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * 4 * (cuuint64_t)rows};
+    const cuuint32_t box[3] = {32, 32, 1};
+    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
+}
+// All of a backward in one launch (linear_backward_sm100.cu), or dW and db alone (dx NULL).  What is cut how, and the time in
+// nanoseconds it is expected to take.
+struct BackwardPlan {
+    int tiles_n;                 // column tiles of both results
+    int dx_tiles, dx_kb, dw_kb;  // tiles of dx; contraction blocks of a tile of dx, of dW
+    int team, down, strips;      // CTAs that work on neighbouring tiles of dW, below (1) or beside each other; groups of such tiles
+    int teams, fewer;
+    double share_fewer, share;   // how much of dW the first `fewer` teams take, and the others
+    int ns;
+};
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms);
+// dy [M, np] with zeros from column N on, w [w_rows, K].
+int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
+                    int M, int N, int np, int K, int *status, cudaStream_t s);
 // The kernel for results of few tiles (linear_split_sm100.cu): out[M, cols] = act[M, kc] . w^T + bias, with w [cols, kc],
 // or with w_mn_major [w_rows, cols] (its rows past w_rows, up to kc, read as zeros); optionally the bf16 planes of out.
 // `split` CTAs share the contraction of a tile.  Returns ATTN_OK or an error.

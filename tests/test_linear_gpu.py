@@ -253,6 +253,52 @@ def test_linear_input_gradient_in_two_pieces(pkg, M, N, K):
         assert torch.equal(pkg.linear_backward(g, xt, wt, None, None), first)
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (1500, 1600, 1600),                    # seven column tiles, of 7 and 8 blocks of 32
+    (1203, 160, 736), (2373, 384, 1152),   # more tiles of dW than of dx per CTA, one tile row; ranges that end inside tiles
+    (200, 2500, 3200),                     # tiles of dW only 7 blocks deep, more than CTAs: not cut
+    (4500, 3072, 768), (4500, 768, 3072),  # dy and x larger than L2: teams of three CTAs beside, of six below each other
+    (640, 33, 32), (1025, 129, 4288),      # one column of a tile in use; long rows
+])
+@pytest.mark.parametrize("with_db", [True, False])
+def test_linear_backward_in_one_launch(pkg, M, N, K, with_db):
+    """dx, dW and db of one launch, in which every CTA takes tiles of dx and a range of dW; db starts on any address."""
+    x, w, _, dy = inputs(M, N, K, 59)
+    rng = np.random.default_rng(7)
+    dw0, db0 = rng.standard_normal((N, K), dtype=np.float32), rng.standard_normal(N, dtype=np.float32)
+    xt, wt, dyt, dw = (torch.from_numpy(a).cuda() for a in (x, w, dy, dw0.copy()))
+    db = torch.full((N + 12,), 0.5, device="cuda")
+    at = 4 if N % 32 == 0 else 3
+    db[at:at + N] = torch.from_numpy(db0).cuda()
+    dx = torch.full((M + 2, K), 3.0, device="cuda")
+    need = pkg.lib().linear_sm100_backward_scratch_bytes(M, N, K)
+    scratch = torch.empty(max(need, 1), dtype=torch.uint8, device="cuda")
+    assert pkg.lib().linear_sm100_backward(dyt.data_ptr(), xt.data_ptr(), wt.data_ptr(), dx[1:].data_ptr(), dw.data_ptr(),
+                                           db[at:].data_ptr() if with_db else None, scratch.data_ptr() if need else None, M, N, K,
+                                           torch.cuda.current_stream().cuda_stream) == 0
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, dw0, db0)
+    within(dx[1:-1].cpu().numpy(), dx_ref, dy, w)
+    within(dw.cpu().numpy(), dw_ref, dy.T, x)
+    assert bool((dx[0] == 3.0).all()) and bool((dx[-1] == 3.0).all())
+    # fp32 sums of M values, 8 at a time, then 8 such sums, then pieces: at most 2^-20 of the sum of magnitudes
+    err = np.abs(db[at:at + N].cpu().numpy() - (db_ref if with_db else db0))
+    assert (err <= 2.0 ** -20 * (np.abs(dy).sum(0) + np.abs(db0))).all()
+    assert bool((db[:at] == 0.5).all()) and bool((db[at + N:] == 0.5).all())
+
+
+def test_linear_backward_results_over_operands(pkg):
+    """Where dW lies over w, dx comes from w as it was; where db lies over dy, dW comes from dy as it was."""
+    M, N, K = 1024, 512, 512
+    x, w, _, dy = inputs(M, N, K, 67)
+    xt, wt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, dy))
+    dx = pkg.linear_backward(dyt, xt, wt, wt, dyt[0])
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, _ = ops.linear_backward(dy, x, w, w, np.zeros(N, np.float32))
+    within(dx.cpu().numpy(), dx_ref, dy, w)
+    within(wt.cpu().numpy(), dw_ref, dy.T, x)
+
+
 def test_linear_argument_errors(pkg):
     L = pkg.lib()
     assert L.linear_sm100_forward(None, None, None, None, None, 1, 4, 4, None) == -1
