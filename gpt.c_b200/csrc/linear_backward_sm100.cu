@@ -52,10 +52,33 @@ struct __align__(1024) Smem {
     int abort_flag;
 };
 
+// Rows of dy whose pitch is not a multiple of 16 bytes (the vocabulary projection: 50257 floats) cannot be tiled by the
+// copy engine as they are, but every fourth row can: the rows m = 4 i + j form a matrix with a pitch of 4 N floats, whose
+// base is moved down to a 16-byte boundary, by a_shift = (j N) mod 4 floats.  The view's column c is then column
+// c - a_shift of dy.  In dx that is the contraction index, and W is fetched at rows c - a_shift (rows before the first
+// and past the last read as zeros); one product per class, which leaves every fourth row of dx.  What the first a_shift
+// columns hold is the end of the row of dy before: the MMA warp puts zeros there in shared memory (clear_leading), since
+// the zeros of W alone would turn a value that is not finite into NaN.  In dW the view's column is the row of the
+// result: each class is a piece of the contraction, added into dW a_shift rows higher up.  What this replaces is a
+// copy of dy with padded rows, 536 us for the 1.65 GB of 8192 x 50257.
+struct RowClass {
+    const float *dy;  // base of the view
+    int rows, shift;
+};
+RowClass row_class(const float *dy, int M, int N, int j) {
+    const int shift = (int)(((long long)j * N) & 3);
+    return RowClass{dy + (size_t)j * N - shift, (M - j + 3) / 4, shift};
+}
+
+// kClasses: the four views of dy (RowClass), and what goes with them.
+template <bool kClasses>
 struct Maps {
-    CUtensorMap dy_k, dy_mn;     // A of dx and of dW
-    CUtensorMap w[2], x[2];      // B of dx and of dW, for tiles of p.cols and of p.cols + 1 blocks of 32 columns
+    static constexpr int kViews = kClasses ? 4 : 1;
+    CUtensorMap dy_k[kViews], dy_mn[kViews];  // A of dx and of dW
+    CUtensorMap x[kViews][2], w[2];           // B of dW and of dx, for tiles of p.cols and of p.cols + 1 blocks of 32 columns
     CUtensorMap dw;
+    CUtensorMap dx[kViews];        // where dx is added up from pieces
+    CUtensorMap dy_whole[kViews];  // dy_mn takes a copy per 32 columns and has the ones after the whole blocks too; this takes one per tile
 };
 
 // dW's tiles are cut across the contraction, and their ranges dealt out to teams of CTAs.  The members of a team work on the same
@@ -64,9 +87,12 @@ struct Problem {
     int M, N, K;
     int tiles_n, cols, wider;  // column tiles; blocks of 32 columns in each; the first `wider` have one more
     int dx_tiles, dx_kb;       // tiles of dx, handed out round robin; contraction blocks of one
+    int classes;               // 4: views of every fourth row of dy
+    int dx_pieces, piece_tiles, piece_kb;  // dx from so many pieces of the contraction; tiles and contraction blocks of a piece
+    int whole[4], shift[4];    // columns of the views in whole blocks; before the first column of dy
     int dw_kb;                 // contraction blocks of a tile of dW
     int team, down;            // CTAs of a team; their tiles are below (1) or beside each other (0)
-    int strips;                // groups of `team` tiles
+    int rounds, strips;        // groups of `team` tiles: whole ones dealt out round robin; the ones after them, which are cut
     int teams, fewer;          // the first `fewer` teams (those with a tile of dx more) take share_fewer of dW, the others share
     uint32_t share_fewer, share;  // in units of 2^-32
     int snap;
@@ -89,20 +115,20 @@ __host__ __device__ __forceinline__ int range_start(const Problem &p, int c) {
 // A tile of dx, or a tile of dW with a range of its contraction.
 struct Item {
     bool dw;
-    int m0, tn, n0, cols, kb0, kb1;
+    int cls, m0, tn, n0, cols, kb0, kb1;
 };
 struct Items {
     int cta, ctas;
-    int i;        // tiles of dx taken so far
-    int at, end;  // the team's range
-    int member;
-    __host__ __device__ __forceinline__ Items(const Problem &p, int cta, int ctas) : cta(cta), ctas(ctas), i(0) {
-        const int team = cta / p.team;
+    int i, whole;  // tiles of dx and whole tiles of dW taken so far
+    int at, end;   // the team's range
+    int team, member;
+    __host__ __device__ __forceinline__ Items(const Problem &p, int cta, int ctas) : cta(cta), ctas(ctas), i(0), whole(0) {
+        team = cta / p.team;
         member = cta - team * p.team;
         at = range_start(p, team), end = range_start(p, team + 1);
     }
     __host__ __device__ __forceinline__ bool next(const Problem &p, Item &t) {
-        const int w = cta + i * ctas;
+        int w = cta + i * ctas;
         int tm;
         if (p.uncut) {
             if (w >= p.strips) return false;
@@ -112,23 +138,38 @@ struct Items {
             i++;
         } else if (w < p.dx_tiles) {
             t.dw = false;
+            const int piece = p.dx_pieces > 1 ? w / p.piece_tiles : 0;
+            w -= piece * p.piece_tiles;
             tm = w / p.tiles_n, t.tn = w - tm * p.tiles_n;
-            t.kb0 = 0, t.kb1 = p.dx_kb;
+            t.kb0 = piece * p.piece_kb, t.kb1 = p.dx_kb - t.kb0 < p.piece_kb ? p.dx_kb : t.kb0 + p.piece_kb;
             i++;
         } else {
-            if (at >= end) return false;
             t.dw = true;
-            const int strip = at / p.dw_kb;
-            t.kb0 = at - strip * p.dw_kb;
-            const int take = p.dw_kb - t.kb0 < end - at ? p.dw_kb - t.kb0 : end - at;
-            t.kb1 = t.kb0 + take;
-            at += take;
+            int strip;
+            if (whole < p.rounds) {
+                strip = team + whole++ * p.teams;
+                t.kb0 = 0, t.kb1 = p.dw_kb;
+            } else {
+                if (at >= end) return false;
+                strip = at / p.dw_kb;
+                t.kb0 = at - strip * p.dw_kb;
+                const int take = p.dw_kb - t.kb0 < end - at ? p.dw_kb - t.kb0 : end - at;
+                t.kb1 = t.kb0 + take;
+                at += take;
+                strip += p.rounds * p.teams;
+            }
             if (p.down) {
                 t.tn = strip, tm = member;
             } else {
                 const int tile = strip * p.team + member;
                 tm = tile / p.tiles_n, t.tn = tile - tm * p.tiles_n;
             }
+        }
+        t.cls = 0;
+        if (p.classes > 1) {  // dW: the classes of a tile follow each other, so that what they add to stays in L2
+            const int rows = p.piece_tiles / p.tiles_n / 4;
+            t.cls = t.dw ? tm & 3 : tm / rows;
+            tm = t.dw ? tm >> 2 : tm - t.cls * rows;
         }
         t.m0 = tm * kBM;
         t.cols = p.cols + (t.tn < p.wider ? 1 : 0);
@@ -146,13 +187,28 @@ struct Place {
     }
 };
 
+// Zeros for the first `columns` (at most 3) of a K-major A tile's 128 rows: they are in the first 16 bytes of a row, which
+// the 128-byte swizzle puts at 16 * (row mod 8).  By a whole warp, one lane of which issues the tensor-core instructions
+// that read the tile.
+__device__ __forceinline__ void clear_leading(uint8_t *tile, int columns, int lane) {
+    for (int r = lane; r < kBM; r += 32) {
+        float *row = reinterpret_cast<float *>(tile + r * 128 + ((r & 7) << 4));
+        row[0] = 0.f;
+        if (columns > 1) row[1] = 0.f;
+        if (columns > 2) row[2] = 0.f;
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+}
+
 __device__ __forceinline__ float4 add4(float4 a, float4 b) {
     const float2 lo = add2(make_float2(a.x, a.y), make_float2(b.x, b.y)), hi = add2(make_float2(a.z, a.w), make_float2(b.z, b.w));
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
+template <bool kClasses>
 __global__ void __launch_bounds__(kThreads, 1)
-linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx, float *__restrict__ db, Problem p, int *status) {
+linear_backward_kernel(const __grid_constant__ Maps<kClasses> maps, float *__restrict__ dx, float *__restrict__ dw, float *__restrict__ db, Problem p, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     if ((smem_u32(smem_raw) & 1023u) != 0) {
@@ -177,11 +233,11 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
     if (warp == 2) tmem_alloc_then_launch_dependents(&sm.tmem_base, 2 * kBN);
     if (warp == 3 && lane == 0) {
         if (p.dx_tiles > 0) {
-            tma_prefetch_desc(&maps.dy_k);
+            tma_prefetch_desc(&maps.dy_k[0]);
             tma_prefetch_desc(&maps.w[0]);
         }
-        tma_prefetch_desc(&maps.dy_mn);
-        tma_prefetch_desc(&maps.x[0]);
+        tma_prefetch_desc(&maps.dy_mn[0]);
+        tma_prefetch_desc(&maps.x[0][0]);
         tma_prefetch_desc(&maps.dw);
     }
     Items items(p, (int)blockIdx.x, (int)gridDim.x);  // the first item, before the wait for the previous kernel
@@ -200,7 +256,9 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
             bool ok = true;
             for (; ok && more; more = items.next(p, t)) {
                 const int wide = t.cols - p.cols;
-                const CUtensorMap *map_b = t.dw ? &maps.x[wide] : &maps.w[wide];
+                const int view = kClasses ? t.cls : 0;
+                const CUtensorMap *map_b = t.dw ? &maps.x[view][wide] : &maps.w[wide];
+                const int behind = kClasses && !t.dw ? p.shift[view] : 0;  // W's rows run this far behind the view's columns
                 for (int kb = t.kb0; kb < t.kb1; kb++, at.next(p.stages)) {
                     const int st = at.st;
                     if (at.round > 0 && !mbar_wait(&sm.empty[st], (at.round - 1) & 1, ctx, SITE_EMPTY)) {
@@ -211,9 +269,18 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
                     mbar_expect_tx(&sm.full[st], kATileBytes + t.cols * 4096);
                     // K-major: map {contraction, rows}, box {32, 128}.  MN-major: blocks of 32 rows, each
                     // [32 contraction steps x 128 bytes].
-                    if (t.dw) tma_load_4d(a, &maps.dy_mn, &sm.full[st], 0, kb * kBK, t.m0 / 32, 0);
-                    else tma_load_4d(a, &maps.dy_k, &sm.full[st], kb * kBK, t.m0, 0, 0);
-                    tma_load_4d(a + kATileBytes, map_b, &sm.full[st], 0, kb * kBK, t.n0 / 32, 0);
+                    if (!t.dw) {
+                        tma_load_4d(a, &maps.dy_k[view], &sm.full[st], kb * kBK, t.m0, 0, 0);
+                    } else if (!kClasses) {
+                        tma_load_4d(a, &maps.dy_mn[0], &sm.full[st], 0, kb * kBK, t.m0 / 32, 0);
+                    } else if (t.m0 + kBM <= p.whole[view]) {
+                        tma_load_4d(a, &maps.dy_whole[view], &sm.full[st], 0, kb * kBK, t.m0 / 32, 0);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            tma_load_4d(a + i * 4096, &maps.dy_mn[view], &sm.full[st], t.m0 + 32 * i, kb * kBK, 0, 0);
+                    }
+                    tma_load_4d(a + kATileBytes, map_b, &sm.full[st], 0, kb * kBK - behind, t.n0 / 32, 0);
                 }
             }
         }
@@ -238,6 +305,7 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
                     if (!mbar_wait_warp(&sm.full[st], at.round & 1, ctx, SITE_FULL)) return false;
                     tc_fence_after_sync();
                     const uint32_t a = smem_u32(sm.ring) + st * p.stage_bytes;
+                    if (kClasses && !kDW && kb == 0 && p.shift[t.cls] > 0) clear_leading(sm.ring + st * p.stage_bytes, p.shift[t.cls], lane);
                     // MN-major tiles: 32-row blocks 4096 bytes apart, groups of 4 contraction steps 512 bytes apart
                     const uint64_t ad = kDW ? smem_desc_sw128_base32(a, 4096, 512)
                                             : smem_desc_sw128(a, 16, 1024);
@@ -305,11 +373,11 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
                         s[e] += __shfl_xor_sync(0xffffffffu, s[e], 10);
                         s[e] += __shfl_xor_sync(0xffffffffu, s[e], 20);
                     }
-                    const int n = t.m0 + 32 * b + col;
+                    const int n = t.m0 + 32 * b + col - (kClasses ? p.shift[t.cls] : 0);
                     if (lane < 8) {
 #pragma unroll
                         for (int e = 0; e < 4; e++)
-                            if (n + e < p.N) atomicAdd(db + n + e, s[e]);
+                            if (n + e >= 0 && n + e < p.N) atomicAdd(db + n + e, s[e]);
                     }
                 }
             }
@@ -341,13 +409,30 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
                 tmem_ld32(tmem + lane_addr + (uint32_t)acc * kBN + 32 * c, r);
                 tmem_wait_ld();
                 if (c + 1 == c1) read_out();
-                if (!t.dw) {
+                if (!t.dw && (!kClasses || p.dx_pieces == 1)) {
                     const int odd = lane & 1, col = col0 + 16 * odd;
                     exchange_halves(odd, r);
 #pragma unroll
                     for (int o = 0; o < 2; o++) {
                         const int row = row0 + lane - odd + o;
-                        if (row < p.M) store_words<4>(dx + (size_t)row * p.K + col, p.K - col, p.wide, r + 16 * o);
+                        if (row * p.classes + t.cls < p.M)
+                            store_words<4>(dx + ((size_t)row * p.classes + t.cls) * p.K + col, p.K - col, p.wide, r + 16 * o);
+                    }
+                    continue;
+                }
+                const int up = kClasses && t.dw ? p.shift[t.cls] : 0;
+                if (kClasses && row0 < up) {
+                    // The first 32 rows of the result: up to three of them do not exist, and a copy must not start at a
+                    // negative coordinate.
+                    const int row = row0 + lane - up;
+                    if (row >= 0 && row < p.N) {
+                        float *dst = dw + (size_t)row * p.K + col0;
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * q),
+                                         "f"(__uint_as_float(r[4 * q])), "f"(__uint_as_float(r[4 * q + 1])),
+                                         "f"(__uint_as_float(r[4 * q + 2])), "f"(__uint_as_float(r[4 * q + 3]))
+                                         : "memory");
                     }
                     continue;
                 }
@@ -360,7 +445,7 @@ linear_backward_kernel(const __grid_constant__ Maps maps, float *__restrict__ dx
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_reduce_add_3d(buf, &maps.dw, col0, row0, 0);
+                    tma_reduce_add_3d(buf, kClasses && !t.dw ? &maps.dx[t.cls] : &maps.dw, col0, row0 - up, 0);
                     bulk_commit();
                 }
             }
@@ -395,16 +480,18 @@ double adding_ns(double pieces, int cols) { return pieces * cols * 16384 * 150e-
 Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
     Problem p = {};
     p.M = M, p.N = N, p.K = K;
+    p.classes = plan.classes, p.dx_pieces = plan.dx_pieces;
+    p.piece_tiles = plan.dx_tiles / plan.dx_pieces, p.piece_kb = (plan.dx_kb + plan.dx_pieces - 1) / plan.dx_pieces;
     p.tiles_n = plan.tiles_n, p.cols = K / 32 / plan.tiles_n, p.wider = K / 32 % plan.tiles_n;
     p.dx_tiles = plan.dx_tiles, p.dx_kb = plan.dx_kb, p.dw_kb = plan.dw_kb;
-    p.team = plan.team, p.down = plan.down, p.strips = plan.strips, p.teams = plan.teams, p.fewer = plan.fewer;
+    p.team = plan.team, p.down = plan.down, p.rounds = plan.rounds, p.strips = plan.strips, p.teams = plan.teams, p.fewer = plan.fewer;
     const double all = plan.fewer * plan.share_fewer + (plan.teams - plan.fewer) * plan.share;
     // rounded up, so that shares of whole tiles begin where tiles do
     p.share_fewer = (uint32_t)ceil(plan.share_fewer / all * 4294967296.0);
     p.share = (uint32_t)fmin(ceil(plan.share / all * 4294967296.0), 4294967295.0);
     // a few tiles of few blocks are cut anywhere, many are not
     p.snap = p.dw_kb >= 16 ? 4 : p.strips >= p.teams ? (p.dw_kb < 8 ? p.dw_kb : 2) : 0;
-    p.uncut = p.dx_tiles == 0 && p.team == 1 && p.snap == p.dw_kb;
+    p.uncut = p.dx_tiles == 0 && p.classes == 1 && p.team == 1 && p.snap == p.dw_kb;
     p.stage_bytes = kATileBytes + (p.cols + (p.wider > 0)) * 4096;
     p.stages = kRingBytes / p.stage_bytes < kMostStages ? kRingBytes / p.stage_bytes : kMostStages;
     return p;
@@ -413,7 +500,7 @@ Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
 }  // namespace
 
 // The split of the work and the time in nanoseconds it is expected to take: see linear_tf32.cuh.
-BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms) {
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes, int dx_pieces) {
     BackwardPlan best = {};
     const int blocks = K / 32;
     for (int width = 8; width >= 4; width--) {
@@ -423,28 +510,40 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms) {
         c.tiles_n = tiles_n;
         const int cols = (blocks + tiles_n - 1) / tiles_n;
         const double tb = block_ns(cols, sms, sms), te = tile_ns(cols);
-        const int rows_m = (M + kBM - 1) / kBM, rows_n = (N + kBM - 1) / kBM;
-        c.dx_tiles = want_dx ? rows_m * tiles_n : 0;
-        c.dx_kb = (N + kBK - 1) / kBK;
-        c.dw_kb = (M + kBK - 1) / kBK;
-        const int dw_tiles = rows_n * tiles_n;
+        const int rows = (M + classes - 1) / classes;  // of a class
+        const int rows_m = (rows + kBM - 1) / kBM, rows_n = (N + classes - 1 + kBM - 1) / kBM;
+        c.dx_kb = (N + classes - 1 + kBK - 1) / kBK;
+        c.dw_kb = (rows + kBK - 1) / kBK;
+        c.classes = classes;
+        const int piece_kb = (c.dx_kb + dx_pieces - 1) / dx_pieces;
+        c.dx_pieces = (c.dx_kb + piece_kb - 1) / piece_kb;
+        c.dx_tiles = want_dx ? classes * rows_m * tiles_n * c.dx_pieces : 0;
+        const int dw_tiles = want_dw ? classes * rows_n * tiles_n : 0;
         // Where dy and x don't stay in L2 together, a team shares the larger of them, if that keeps most SMs busy.
-        c.down = N < K, c.team = c.down ? rows_n : tiles_n;
+        c.down = classes == 1 && N < K, c.team = c.down ? rows_n : tiles_n;
         if (4.0 * M * ((double)N + K) < (64 << 20) || c.team > sms || sms / c.team * c.team < sms * 24 / 25) c.down = 0, c.team = 1;
         c.strips = dw_tiles / c.team;
         c.teams = sms / c.team;
         if (!want_dx && (long long)c.strips * c.dw_kb < c.teams) c.teams = c.strips * c.dw_kb;
         const int ctas = c.teams * c.team;
-        const double dx_ns = c.dx_kb * tb + te;
+        const double dx_ns = piece_kb * tb + te;
         // every CTA has about one piece of a tile more than its share of whole ones
         const double even = (c.dx_tiles * dx_ns + dw_tiles * (c.dw_kb * tb + te)) / ctas + te;
         const int most = (c.dx_tiles + ctas - 1) / ctas;
         c.fewer = (c.dx_tiles % ctas + c.team - 1) / c.team;
         // what is left for dW, in blocks, in a CTA with `most` tiles of dx and in one with a tile less
         c.share_fewer = (even - most * dx_ns - te) / tb, c.share = c.share_fewer + (c.fewer ? dx_ns / tb : 0);
+        if (classes > 1) {
+            // Most strips whole and in turn, so that teams work on neighbouring columns of dy at the same time
+            const double least = c.fewer ? c.share_fewer : c.share;
+            c.rounds = least > 0 ? (int)(least / c.dw_kb) : 0;
+            if (c.rounds > c.strips / c.teams) c.rounds = c.strips / c.teams;
+            c.strips -= c.rounds * c.teams;
+            c.share_fewer -= c.rounds * c.dw_kb, c.share -= c.rounds * c.dw_kb;
+        }
         if (c.share_fewer < 3) c.share_fewer = 0;
         if (c.share < 1) c.share = 1;
-        double time = (even > most * dx_ns ? even : most * dx_ns) + adding_ns(dw_tiles + ctas, cols);
+        double time = (even > most * dx_ns && want_dw ? even : most * dx_ns) + adding_ns(dw_tiles + ctas, cols);
         const int most_pieces = want_dx ? 0 : sms / dw_tiles < c.dw_kb ? sms / dw_tiles : c.dw_kb;
         auto as_deep = [&](int pieces) {  // fewest pieces that are no longer
             const int depth = (c.dw_kb + pieces - 1) / pieces;
@@ -455,7 +554,7 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms) {
             const int busy = pieces * dw_tiles;
             const double whole = (c.dw_kb + pieces - 1) / pieces * block_ns(cols, busy, sms) + te + adding_ns(busy, cols);
             if (whole <= time) {
-                c.team = 1, c.down = 0, c.strips = dw_tiles, c.teams = busy, c.share = 1;
+                c.team = 1, c.down = 0, c.rounds = 0, c.strips = dw_tiles, c.teams = busy, c.share = 1;
                 time = whole;
             }
             pieces = pieces > 1 ? as_deep(pieces - 1) : 0;
@@ -467,33 +566,60 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms) {
     return best;
 }
 
-int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
-                    int M, int N, int np, int K, int *status, cudaStream_t s) {
+template <bool kClasses>
+static int launch(const Maps<kClasses> &maps, float *dx, float *dw, float *db, const Problem &p, int ctas, int *status, cudaStream_t s) {
     static bool attr_done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear backward kernel");
+    auto kernel = linear_backward_kernel<kClasses>;
     if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-        e = cudaFuncSetAttribute(linear_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return (int)e;
         if (dev >= 0 && dev < 64) attr_done[dev] = true;
     }
+    return (int)attn::launch_after_previous(kernel, dim3(ctas), dim3(kThreads), sizeof(Smem), s, maps, dx, dw, db, p, status);
+}
+
+int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
+                    int M, int N, int np, int K, int *status, cudaStream_t s) {
     Problem p = make_problem(plan, M, N, K);
     p.wide = (reinterpret_cast<uintptr_t>(dx) & 31u) == 0;
-    Maps maps;
+    Maps<false> maps;
     int rc;
-    if ((rc = map_mn_major_blocks(&maps.dy_mn, dy, M, np, 4)) != 0) return rc;
+    if ((rc = map_mn_major_blocks(&maps.dy_mn[0], dy, M, np, 4)) != 0) return rc;
     if ((rc = map_out_f32(&maps.dw, dw, N, K)) != 0) return rc;
-    if ((rc = map_mn_major_blocks(&maps.x[0], x, M, K, p.cols)) != 0) return rc;
-    if (p.wider && (rc = map_mn_major_blocks(&maps.x[1], x, M, K, p.cols + 1)) != 0) return rc;
-    maps.w[0] = maps.x[0], maps.dy_k = maps.dy_mn;  // not looked at without dx
-    if (dx) {
-        if ((rc = map_mn_major_blocks(&maps.w[0], w, w_rows, K, p.cols)) != 0) return rc;
-        if (p.wider && (rc = map_mn_major_blocks(&maps.w[1], w, w_rows, K, p.cols + 1)) != 0) return rc;
-        if ((rc = map_k_major(&maps.dy_k, dy, M, np, 128)) != 0) return rc;
+    for (int i = 0; i <= (p.wider > 0); i++) {
+        if ((rc = map_mn_major_blocks(&maps.x[0][i], x, M, K, p.cols + i)) != 0) return rc;
+        if (dx && (rc = map_mn_major_blocks(&maps.w[i], w, w_rows, K, p.cols + i)) != 0) return rc;
     }
-    return (int)attn::launch_after_previous(linear_backward_kernel, dim3(plan.teams * plan.team), dim3(kThreads), sizeof(Smem), s, maps, dx, db, p, status);
+    if (dx && (rc = map_k_major(&maps.dy_k[0], dy, M, np, 128)) != 0) return rc;
+    return launch<false>(maps, dx, dw, db, p, plan.teams * plan.team, status, s);
+}
+
+int launch_backward_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db,
+                                 int M, int N, int K, int *status, cudaStream_t s) {
+    Problem p = make_problem(plan, M, N, K);
+    p.wide = (reinterpret_cast<uintptr_t>(dx) & 31u) == 0;
+    Maps<true> maps;
+    int rc;
+    if (dw && (rc = map_out_f32(&maps.dw, dw, N, K)) != 0) return rc;
+    for (int j = 0; j < 4; j++) {
+        const RowClass c = row_class(dy, M, N, j);
+        const size_t pitch = 4 * (size_t)N;
+        p.shift[j] = c.shift, p.whole[j] = (N + c.shift) / 32 * 32;
+        if (p.whole[j] > 0 && (rc = map_mn_major_blocks(&maps.dy_whole[j], c.dy, c.rows, p.whole[j], 4, pitch)) != 0) return rc;
+        if ((rc = map_mn_major(&maps.dy_mn[j], c.dy, c.rows, N + c.shift, pitch)) != 0) return rc;
+        for (int i = 0; i <= (p.wider > 0); i++)
+            if ((rc = map_mn_major_blocks(&maps.x[j][i], x + (size_t)j * K, c.rows, K, p.cols + i, 4 * (size_t)K)) != 0) return rc;
+        if (!dx) continue;
+        if ((rc = map_k_major(&maps.dy_k[j], c.dy, c.rows, N + c.shift, 128, pitch)) != 0) return rc;
+        if (p.dx_pieces > 1 && (rc = map_out_f32(&maps.dx[j], dx + (size_t)j * K, c.rows, K, 4 * (size_t)K)) != 0) return rc;
+    }
+    for (int i = 0; dx && i <= (p.wider > 0); i++)
+        if ((rc = map_mn_major_blocks(&maps.w[i], w, N, K, p.cols + i)) != 0) return rc;
+    return launch<true>(maps, dx, dw, db, p, plan.teams * plan.team, status, s);
 }
 
 }  // namespace lin

@@ -8,12 +8,9 @@
 // epilogue adds the bias and can also emit the result as the two bf16 planes (hi, lo) the
 // attention kernels consume, which removes the attention path's own split pass.
 //
-// The three products differ only in which operand dimension is contiguous in memory:
 //     forward  y [M,N]  = x [M,K] . W[N,K]^T        A: x, K-major          B: W,  K-major
 //     dx       dx[M,K]  = dy[M,N] . W[N,K]          A: dy, K-major (over N) B: W,  MN-major
-//     dW       dW[N,K] += dy[M,N]^T . x[M,K]        A: dy, MN-major         B: x,  MN-major  (split over M)
-// This file has the forward, dx where it is wanted alone or has few rows, and both gradients where rows of dy are not 16-byte
-// aligned; elsewhere linear_backward_sm100.cu makes them in one launch.
+// dx is made here where it is wanted alone or has few rows; dW, db and elsewhere dx are linear_backward_sm100.cu's.
 // (K-major: the contraction index is the contiguous one.)  Contraction blocks are 32 fp32 values (one 128-byte
 // swizzled row).  A tile is 128 rows by 128, 192 or 256 columns, with as many pipeline stages as shared memory holds;
 // plan_tiles picks the width.
@@ -60,14 +57,11 @@ struct __align__(1024) SmemT {
 struct Problem {
     int M, N, K;  // C is [M, N]; K is the contraction length
     int bn;       // tile width
-    int a_one, b_one;  // MN-major operand fetched with one 3-D copy per stage (else one copy per 32-row block)
+    int b_one;    // MN-major B fetched with one 3-D copy per stage (else one copy per 32-row block)
     int tiles_m, tiles_n, splits, kb_total, kb_per_split, total;
     int wide, wide_planes;  // rows of C / of the planes start on 32-byte boundaries
     size_t plane_words;     // distance from the hi to the lo plane
     size_t ldc;             // floats from one row of C to the next
-    int b_shift;            // B's contraction index runs this far behind A's (see RowClass)
-    int a_whole[4];         // columns in whole blocks of A's views
-    int a_shift[4];         // columns of A's views before the first column of dy (dW from row classes)
     int m_fast;  // consecutive work items walk down the rows of C (else along its columns)
 };
 
@@ -75,35 +69,11 @@ enum Site : int {
     SITE_EMPTY = 201, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_SMEM_ALIGN
 };
 
-// Tensors the copy engine fetches from; four views of each operand for dW from row classes.
-template <bool kClasses>
 struct Maps {
-    CUtensorMap a[kClasses ? 4 : 1], b[kClasses ? 4 : 1], c;
-    // row classes: A's 32-column blocks that are whole, fetched a tile at a time (`a` has the columns after them too,
-    // but takes four copies, and the thread that requests them is then the limit)
-    CUtensorMap a_whole[kClasses ? 4 : 1];
+    CUtensorMap a, b, c;
 };
-
-// Rows of dy whose pitch is not a multiple of 16 bytes (the vocabulary projection: 50257 floats) cannot be tiled by the
-// copy engine as they are, but every fourth row can: the rows m = 4 i + j form a matrix with a pitch of 4 N floats, whose
-// base is moved down to a 16-byte boundary, by a_shift = (j N) mod 4 floats.  The view's column c is then column
-// c - a_shift of dy.  In dx that is the contraction index, and W is fetched at rows c - a_shift (rows before the first
-// and past the last read as zeros); one product per class, which leaves every fourth row of dx.  What the first a_shift
-// columns hold is the end of the row of dy before: the MMA warp puts zeros there in shared memory (clear_leading), since
-// the zeros of W alone would turn a value that is not finite into NaN.  In dW the view's column is the row of the
-// result: each class is a piece of the contraction, added into dW a_shift rows higher up.  What this replaces is a
-// copy of dy with padded rows, 536 us for the 1.65 GB of 8192 x 50257.
-struct RowClass {
-    const float *dy;  // base of the view
-    int rows, shift;
-};
-RowClass row_class(const float *dy, int M, int N, int j) {
-    const int shift = (int)(((long long)j * N) & 3);
-    return RowClass{dy + (size_t)j * N - shift, (M - j + 3) / 4, shift};
-}
 
 struct Work {
-    int cls;  // row class
     int m0, n0, kb0, kb1;  // first row of this CTA's 128, first column of the tile, contraction blocks
 };
 __device__ __forceinline__ Work decode(const Problem &p, int w) {
@@ -116,32 +86,17 @@ __device__ __forceinline__ Work decode(const Problem &p, int w) {
     Work r;
     r.m0 = tm * kBM;
     r.n0 = tn * p.bn;
-    r.cls = split;  // only looked at where the pieces of the contraction are row classes
     r.kb0 = split * p.kb_per_split;
     r.kb1 = min(p.kb_total, r.kb0 + p.kb_per_split);
     return r;
 }
 
-// Zeros for the first `columns` (at most 3) of a K-major A tile's 128 rows: they are in the first 16 bytes of a row, which
-// the 128-byte swizzle puts at 16 * (row mod 8).  By a whole warp, one lane of which issues the tensor-core instructions
-// that read the tile.
-__device__ __forceinline__ void clear_leading(uint8_t *tile, int columns, int lane) {
-    for (int r = lane; r < kBM; r += 32) {
-        float *row = reinterpret_cast<float *>(tile + r * 128 + ((r & 7) << 4));
-        row[0] = 0.f;
-        if (columns > 1) row[1] = 0.f;
-        if (columns > 2) row[2] = 0.f;
-    }
-    fence_proxy_async_smem();
-    __syncwarp();
-}
-
 // kEpi 0: C = acc (+ bias), optional bf16 planes; kEpi 1: C += acc (bulk reduction)
 // kDirect: the result goes out with plain coalesced 4-byte stores, for outputs whose row pitch is not a multiple of 16
 // bytes (the 50257-wide vocabulary projection).
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kClasses>
+template <bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect>
 __global__ void __launch_bounds__(kThreads, 1)
-linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__restrict__ bias, float *__restrict__ c_direct,
+linear_gemm_kernel(const __grid_constant__ Maps maps, const float *__restrict__ bias, float *__restrict__ c_direct,
                    uint32_t *__restrict__ planes, Problem p, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     using Smem = SmemT<kBN, kStages, kEpi == 1 || kDirect>;
@@ -172,10 +127,8 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
         tmem_alloc_then_launch_dependents(&sm.tmem_base, kTmemCols);
     }
     if (warp == 3 && lane == 0) {
-        for (int i = 0; i < (kClasses ? 4 : 1); i++) {
-            tma_prefetch_desc(&maps.a[i]);
-            tma_prefetch_desc(&maps.b[i]);
-        }
+        tma_prefetch_desc(&maps.a);
+        tma_prefetch_desc(&maps.b);
     }
     pdl_wait();  // every thread, before its first access to global memory
     tc_fence_before_sync();
@@ -189,9 +142,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
             int it = 0;
             bool ok = true;
             for (int w = first; ok && w < p.total; w += step) {
-                Work wk = decode(p, w);
-                const CUtensorMap &map_a = maps.a[kClasses ? wk.cls : 0], &map_b = maps.b[kClasses ? wk.cls : 0];
-                if (kClasses) wk.kb0 = 0, wk.kb1 = p.kb_total;
+                const Work wk = decode(p, w);
                 for (int kb = wk.kb0; kb < wk.kb1; kb++, it++) {
                     const int st = it % kStages;
                     if (it >= kStages && !mbar_wait(&sm.empty[st], ((it / kStages) - 1) & 1, ctx, SITE_EMPTY)) {
@@ -204,48 +155,34 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                     };
                     const int b0 = wk.n0;
                     // K-major: map {contraction, rows}, one box {32, 128}.  MN-major: map {rows, contraction},
-                    // four boxes {32, 32}: blocks of 32 rows, each [32 contraction steps x 128 bytes].
-                    if (kAMN) {
-                        if (kClasses && wk.m0 + kBM <= p.a_whole[wk.cls]) {
-                            load(sm.a[st], &maps.a_whole[kClasses ? wk.cls : 0], 0, kb * kBK, wk.m0 / 32);
-                        } else if (p.a_one) {
-                            load(sm.a[st], &map_a, 0, kb * kBK, wk.m0 / 32);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 4; i++)
-                                load(sm.a[st] + i * 4096, &map_a, wk.m0 + 32 * i, kb * kBK, 0);
-                        }
-                    } else {
-                        load(sm.a[st], &map_a, kb * kBK, wk.m0, 0);
-                    }
+                    // boxes {32, 32}: blocks of 32 rows, each [32 contraction steps x 128 bytes].
+                    load(sm.a[st], &maps.a, kb * kBK, wk.m0, 0);
                     if (kBMN) {
                         if (p.b_one) {
-                            load(sm.b[st], &map_b, 0, kb * kBK - p.b_shift, b0 / 32);
+                            load(sm.b[st], &maps.b, 0, kb * kBK, b0 / 32);
                         } else {
 #pragma unroll
                             for (int i = 0; i < kBN / 32; i++)
-                                load(sm.b[st] + i * 4096, &map_b, b0 + 32 * i, kb * kBK - p.b_shift, 0);
+                                load(sm.b[st] + i * 4096, &maps.b, b0 + 32 * i, kb * kBK, 0);
                         }
                     } else {
-                        load(sm.b[st], &map_b, kb * kBK, b0, 0);  // the B map's box is kBN rows
+                        load(sm.b[st], &maps.b, kb * kBK, b0, 0);  // the B map's box is kBN rows
                     }
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        constexpr uint32_t idesc = idesc_tf32(kBM, kBN, kAMN ? 1 : 0, kBMN ? 1 : 0);
+        constexpr uint32_t idesc = idesc_tf32(kBM, kBN, 0, kBMN ? 1 : 0);
         const uint32_t leader = elect_leader();
         int it = 0, j = 0;
         bool ok = true;
         for (int w = first; ok && w < p.total; w += step, j++) {
-            Work wk = decode(p, w);
-            if (kClasses) wk.kb0 = 0, wk.kb1 = p.kb_total;
+            const Work wk = decode(p, w);
             const int acc = j & 1;
             if (j >= 2 && !mbar_wait_warp(&sm.acc_empty[acc], ((j >> 1) - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
             tc_fence_after_sync();
             const uint32_t d = tmem + (uint32_t)acc * kBN;
-            bool clear = !kAMN && kBMN && wk.kb0 == 0 && p.b_shift > 0;  // tested anew for every block: 0.6 % slower
             for (int kb = wk.kb0; kb < wk.kb1; kb++, it++) {
                 const int st = it % kStages;
                 if (!mbar_wait_warp(&sm.full[st], (it / kStages) & 1, ctx, SITE_FULL)) {
@@ -253,18 +190,13 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                     break;
                 }
                 tc_fence_after_sync();
-                if (clear) {
-                    clear_leading(sm.a[st], p.b_shift, lane);
-                    clear = false;
-                }
                 // MN-major tiles: 32-row blocks 4096 bytes apart, groups of 4 contraction steps 512 bytes apart
-                const uint64_t ad = kAMN ? smem_desc_sw128_base32(smem_u32(sm.a[st]), 4096, 512)
-                                         : smem_desc_sw128(smem_u32(sm.a[st]), 16, 1024);
+                const uint64_t ad = smem_desc_sw128(smem_u32(sm.a[st]), 16, 1024);
                 const uint64_t bd = kBMN ? smem_desc_sw128_base32(smem_u32(sm.b[st]), 4096, 512)
                                          : smem_desc_sw128(smem_u32(sm.b[st]), 16, 1024);
 #pragma unroll
                 for (int k = 0; k < kBK / 8; k++) {
-                    const uint64_t ak = desc_advance(ad, k * (kAMN ? 1024 : 32)), bk = desc_advance(bd, k * (kBMN ? 1024 : 32));
+                    const uint64_t ak = desc_advance(ad, k * 32), bk = desc_advance(bd, k * (kBMN ? 1024 : 32));
                     const uint32_t add = (kb > wk.kb0 || k > 0) ? 1u : 0u;
                     mma_tf32_lead(leader, d, ak, bk, idesc, add);
                 }
@@ -341,23 +273,6 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                     for (int e = 0; e < 32; e++)
                         r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, mine, e));
                 }
-                const int up = kClasses ? p.a_shift[wk.cls] : 0;
-                if (kClasses && row0 < up) {
-                    // The first 32 rows of the result: up to three of them do not exist, and a copy must not start at a
-                    // negative coordinate.
-                    const int row = row0 + lane - up;
-                    if (row >= 0 && row < p.M) {
-                        float *dst = c_direct + (size_t)row * p.ldc + col0;
-#pragma unroll
-                        for (int q = 0; q < 8; q++)
-                            if (col0 + 4 * q < p.N)
-                                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * q),
-                                             "f"(__uint_as_float(r[4 * q])), "f"(__uint_as_float(r[4 * q + 1])),
-                                             "f"(__uint_as_float(r[4 * q + 2])), "f"(__uint_as_float(r[4 * q + 3]))
-                                             : "memory");
-                    }
-                    continue;
-                }
                 if (!kDirect && lane == 0) bulk_wait_read_all();  // the copy engine has read the buffer out
                 __syncwarp();
 #pragma unroll
@@ -378,7 +293,7 @@ linear_gemm_kernel(const __grid_constant__ Maps<kClasses> maps, const float *__r
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_reduce_add_3d(buf, &maps.c, col0, row0 - up, 0);
+                    tma_reduce_add_3d(buf, &maps.c, col0, row0, 0);
                     bulk_commit();
                 }
             }
@@ -508,11 +423,9 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(float *__restrict__ dst, 
 Problem make_problem(int M, int N, int K, int bn, int splits) {
     Problem p;
     p.M = M, p.N = N, p.K = K, p.bn = bn;
-    p.a_one = p.b_one = 0;
+    p.b_one = 0;
     p.m_fast = 0;
     p.ldc = (size_t)N;
-    p.b_shift = 0;
-    for (int i = 0; i < 4; i++) p.a_shift[i] = p.a_whole[i] = 0;
     p.tiles_m = (M + kBM - 1) / kBM;
     p.tiles_n = (N + bn - 1) / bn;
     p.kb_total = (K + kBK - 1) / kBK;
@@ -586,15 +499,15 @@ Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks, int most = 32)
     return best;
 }
 
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect, bool kClasses = false>
-int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *planes, Problem p, int *status, cudaStream_t s) {
+template <bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect>
+int launch_one(const Maps &maps, const float *bias, float *c, void *planes, Problem p, int *status, cudaStream_t s) {
     using Smem = SmemT<kBN, kStages, kEpi == 1 || kDirect>;
     static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear kernel");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    auto kernel = linear_gemm_kernel<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect, kClasses>;
+    auto kernel = linear_gemm_kernel<kBMN, kEpi, kBN, kStages, kPlanes, kDirect>;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return (int)e;
@@ -609,20 +522,12 @@ int launch_maps(const Maps<kClasses> &maps, const float *bias, float *c, void *p
                                                      static_cast<uint32_t *>(planes), p, status);
 }
 
-template <bool kAMN, bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect>
-int launch_one(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
-               const Problem &p, int *status, cudaStream_t s) {
-    const Maps<false> maps = {{ma}, {mb}, mc, {ma}};
-    return launch_maps<kAMN, kBMN, kEpi, kBN, kStages, kPlanes, kDirect>(maps, bias, c, planes, p, status, s);
-}
-
 // Pipeline depth by what fits in 227 KiB next to the output staging tile.
-template <bool kAMN, bool kBMN, int kEpi>
-int launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const float *bias, float *c, void *planes,
-           const Problem &p, int *status, cudaStream_t s) {
+template <bool kBMN, int kEpi>
+int launch(const Maps &maps, const float *bias, float *c, void *planes, const Problem &p, int *status, cudaStream_t s) {
 #define GO(bn, stages, with_planes) \
-    return launch_one<kAMN, kBMN, kEpi, bn, stages, with_planes, false>(ma, mb, mc, bias, c, planes, p, status, s)
-    constexpr bool kCanPlanes = !kAMN && !kBMN && kEpi == 0;  // only the forward product writes planes
+    return launch_one<kBMN, kEpi, bn, stages, with_planes, false>(maps, bias, c, planes, p, status, s)
+    constexpr bool kCanPlanes = !kBMN && kEpi == 0;  // only the forward product writes planes
     if constexpr (kCanPlanes) {
         if (planes && p.bn == 256) GO(256, 4, true);
         if (planes && p.bn == 192) GO(192, 5, true);
@@ -654,67 +559,25 @@ bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) ==
 // The size of the scratch buffer follows from the shape alone, so this must too.
 bool by_row_class(int M, int N) { return N % 4 != 0 && M >= 4096 && (long long)M * N >= (32 << 20); }
 
-// Tile width of dW [N, K] from views of every fourth row: 256 unless tiles of 192 columns end more than a tenth earlier;
-// 128 is only for results that narrow.  8192 x 50257, K = 384: 764 / 724 / 822 us at 128 / 192 / 256 columns,
-// 512: 1128 / 1000 / 845, 576: 1352 / 1025 / 1181, 640: 1431 / 1297 / 1165, 768: 1615 / 1372 / 1218, 1600: 3222 / 3164 / 3007.
-int class_tile_width(int K) {
-    if (K <= 128) return 128;
-    return (K + 191) / 192 * 192 * 11 / 10 < (K + 255) / 256 * 256 ? 192 : 256;
-}
-
-// dx and dW (either may be NULL) straight from a dy whose rows are not 16-byte aligned.
-int gradients_by_row_class(const float *dy, const float *x, const float *w, float *dx, float *dw, int M, int N, int K, int sms,
+// dx, dW and db (dx or dw may be NULL) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut into
+// pieces that add into zeros: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from
+// sums of 524 blocks of 32, 1.3e-5 from sums of 171).  Without dW, whose ranges make up for it, their number decides how even
+// the last round of tiles is (8192 x 50257 x 768: 1009 us from 3 pieces, 1111 from 4).
+int gradients_by_row_class(const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, int M, int N, int K, int sms,
                            int *status, cudaStream_t s) {
-    int rc;
-    CUtensorMap ma, mb, mc;
-    if (dx) {
-        const int kb = (N + 3 + kBK - 1) / kBK;
-        Plan plan = plan_tiles((M + 3) / 4, K, kb, sms), cut = plan_pieces((M + 3) / 4, K, kb, sms, 32);
-        cut.ns += (2500 + (int)((long long)M * K * 4 / 5500)) / 4;
-        if (cut.splits > 1 && cut.ns < plan.ns) plan = cut;
-        if (plan.splits > 1 && (rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
-        for (int j = 0; j < 4; j++) {
-            const RowClass c = row_class(dy, M, N, j);
-            Problem p = make_problem(c.rows, K, N + c.shift, plan.bn, plan.splits);
-            p.ldc = 4 * (size_t)K, p.b_shift = c.shift;
-            if ((rc = map_k_major(&ma, c.dy, c.rows, N + c.shift, 128, 4 * (size_t)N)) != 0) return rc;
-            p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32) == 0;
-            if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
-            float *out = dx + (size_t)j * K;
-            if (p.splits > 1) {
-                if ((rc = map_out_f32(&mc, out, c.rows, K, p.ldc)) != 0) return rc;
-                rc = launch<false, true, 1>(ma, mb, mc, nullptr, out, nullptr, p, status, s);
-            } else {
-                rc = launch<false, true, 0>(ma, mb, ma, nullptr, out, nullptr, p, status, s);
-            }
-            if (rc != 0) return rc;
-        }
+    const int kb = (N + 3 + kBK - 1) / kBK;
+    const int least = (kb + 523) / 524, by_tiles = plan_pieces((M + 3) / 4, K, kb, sms, 32).splits;
+    const int pieces = least > by_tiles ? least : by_tiles;
+    BackwardPlan plan = plan_backward(M, N, K, dx != nullptr, dw != nullptr, sms, 4, pieces);
+    for (int more = 1; dx && !dw && more <= 2; more++) {
+        const BackwardPlan other = plan_backward(M, N, K, true, false, sms, 4, pieces + more);
+        if (other.ns < plan.ns) plan = other;
     }
-    if (!dw) return ATTN_OK;
-    // the four classes of a tile follow each other, so that the tile of dW they add into stays in L2
-    Maps<true> maps;
-    Problem p = make_problem(N, K, (M + 3) / 4, class_tile_width(K), 1);
-    p.splits = 4, p.total *= 4;
-    p.a_one = 0, p.b_one = 1;
-    for (int j = 0; j < 4; j++) {
-        const RowClass c = row_class(dy, M, N, j);
-        p.a_shift[j] = c.shift;
-        p.a_whole[j] = (N + c.shift) / 32 * 32;
-        if (p.a_whole[j] > 0) {
-            if ((rc = map_mn_major_blocks(&maps.a_whole[j], c.dy, c.rows, p.a_whole[j], 4, 4 * (size_t)N)) != 0) return rc;
-        } else {
-            maps.a_whole[j] = {};
-        }
-        if ((rc = map_mn_major(&maps.a[j], c.dy, c.rows, N + c.shift, 4 * (size_t)N)) != 0) return rc;
-        if ((rc = map_mn_major_blocks(&maps.b[j], x + (size_t)j * K, c.rows, K, p.bn / 32, 4 * (size_t)K)) != 0) return rc;
+    if (dx && plan.dx_pieces > 1) {
+        const int rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s);
+        if (rc != 0) return rc;
     }
-    // up to three rows of the last tile may only be reached through the shifted views
-    p.tiles_m = (N + 3 + kBM - 1) / kBM;
-    p.total = p.tiles_m * p.tiles_n * p.splits;
-    if ((rc = map_out_f32(&maps.c, dw, N, K)) != 0) return rc;
-    if (p.bn == 192) return launch_maps<true, true, 1, 192, 4, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
-    if (p.bn == 256) return launch_maps<true, true, 1, 256, 4, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
-    return launch_maps<true, true, 1, 128, 6, false, false, true>(maps, nullptr, dw, nullptr, p, status, s);
+    return launch_backward_by_row_class(plan, dy, x, w, dx, dw, db, M, N, K, status, s);
 }
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
@@ -746,16 +609,16 @@ int input_gradient(const InputGradient &how, const float *g, const float *w, flo
     if (how.split) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, how.split, sms, status, s);
     const Plan &plan = how.tiles;
     int rc;
-    CUtensorMap ma, mb, mc;
+    Maps maps = {};
     Problem p = make_problem(M, K, np, plan.bn, plan.splits);
-    if ((rc = map_k_major(&ma, g, M, np, 128)) != 0) return rc;
-    p.b_one = map_mn_major_blocks(&mb, w, N, K, p.bn / 32) == 0;
-    if (!p.b_one && (rc = map_mn_major(&mb, w, N, K)) != 0) return rc;
-    if (p.splits == 1) return launch<false, true, 0>(ma, mb, ma, nullptr, dx, nullptr, p, status, s);
+    if ((rc = map_k_major(&maps.a, g, M, np, 128)) != 0) return rc;
+    p.b_one = map_mn_major_blocks(&maps.b, w, N, K, p.bn / 32) == 0;
+    if (!p.b_one && (rc = map_mn_major(&maps.b, w, N, K)) != 0) return rc;
+    if (p.splits == 1) return launch<true, 0>(maps, nullptr, dx, nullptr, p, status, s);
     // the pieces of the contraction add into dx with bulk reductions: start from zeros
-    if ((rc = map_out_f32(&mc, dx, M, K)) != 0) return rc;
+    if ((rc = map_out_f32(&maps.c, dx, M, K)) != 0) return rc;
     if ((rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
-    return launch<false, true, 1>(ma, mb, mc, nullptr, dx, nullptr, p, status, s);
+    return launch<true, 1>(maps, nullptr, dx, nullptr, p, status, s);
 }
 
 // Whether a result lies over something that another product of the same call reads or writes: then the products have to
@@ -797,16 +660,14 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
     int split = 1;
     if (plan_split(M, N, K, sms, &split) < plan.ns)
         return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, sms, status, s);
-    CUtensorMap ma, mb;
+    Maps maps = {};
     // with plain stores (N not a multiple of 4) only the widest tiles are built
     Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, 1);
     p.m_fast = stream_rows_of_c(M, N, K);
-    if ((rc = map_k_major(&ma, x, M, K, 128)) != 0) return rc;
-    if ((rc = map_k_major(&mb, w, N, K, p.bn)) != 0) return rc;
-    if (direct) {
-        return launch_one<false, false, 0, 256, 4, false, true>(ma, mb, ma, bias, y, nullptr, p, status, s);
-    }
-    return launch<false, false, 0>(ma, mb, ma, bias, y, planes, p, status, s);
+    if ((rc = map_k_major(&maps.a, x, M, K, 128)) != 0) return rc;
+    if ((rc = map_k_major(&maps.b, w, N, K, p.bn)) != 0) return rc;
+    if (direct) return launch_one<false, 0, 256, 4, false, true>(maps, bias, y, nullptr, p, status, s);
+    return launch<false, 0>(maps, bias, y, planes, p, status, s);
 }
 
 size_t linear_sm100_backward_scratch_bytes(int M, int N, int K) {
@@ -837,8 +698,12 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int sms = attn::sm_count();
     const float *g = dy;  // without row classes [M, np] from here on
+    const bool in_parts = dw && overlapping(dy, x, w, dx, dw, db, M, N, K);
     if (classes) {
-        if ((rc = gradients_by_row_class(dy, x, w, dx, dw, M, N, K, sms, status, s)) != 0) return rc;
+        if (dx && (!dw || in_parts)) rc = gradients_by_row_class(dy, x, w, dx, nullptr, nullptr, M, N, K, sms, status, s);
+        if (rc == 0 && dw)
+            rc = gradients_by_row_class(dy, x, w, in_parts ? nullptr : dx, dw, in_parts ? nullptr : db, M, N, K, sms, status, s);
+        if (rc != 0 || (dw && !in_parts)) return rc;
     } else if (padded) {
         rc = (int)attn::launch_after_previous(pad_rows_kernel, dim3(sms * 16), dim3(256), 0, s, static_cast<float *>(scratch), dy, M,
                                               N, np);
@@ -846,13 +711,12 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         g = static_cast<const float *>(scratch);
     }
     if (!classes) {
-        const bool in_parts = dw && overlapping(dy, x, w, dx, dw, db, M, N, K);
         InputGradient alone{};
         if (dx) alone = plan_input_gradient(M, np, K, sms);
         BackwardPlan rest{}, both{};
-        if (dw) rest = plan_backward(M, N, K, false, sms);
+        if (dw) rest = plan_backward(M, N, K, false, true, sms);
         // dx has the same bits with and without dW: one launch only where dx alone would be whole tiles too
-        if (dw && dx && !in_parts && !alone.split && alone.tiles.splits == 1) both = plan_backward(M, N, K, true, sms);
+        if (dw && dx && !in_parts && !alone.split && alone.tiles.splits == 1) both = plan_backward(M, N, K, true, true, sms);
         const bool together = both.ns > 0 && both.ns < alone.ns + rest.ns;
         if (dx && !together && (rc = input_gradient(alone, g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
         if (dw) {

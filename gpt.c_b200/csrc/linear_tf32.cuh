@@ -114,20 +114,25 @@ inline int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, 
     const cuuint32_t box[3] = {32, 32, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
 }
-// All of a backward in one launch (linear_backward_sm100.cu), or dW and db alone (dx NULL).  What is cut how, and the time in
+// All of a backward in one launch (linear_backward_sm100.cu), or dW and db alone (dx NULL), or dx alone (dw and db NULL).  What is cut how, and the time in
 // nanoseconds it is expected to take.
 struct BackwardPlan {
     int tiles_n;                 // column tiles of both results
-    int dx_tiles, dx_kb, dw_kb;  // tiles of dx; contraction blocks of a tile of dx, of dW
-    int team, down, strips;      // CTAs that work on neighbouring tiles of dW, below (1) or beside each other; groups of such tiles
+    int dx_tiles, dx_kb, dw_kb;  // tiles of dx (of all its pieces); contraction blocks of a tile of dx, of dW
+    int classes, dx_pieces;      // views of dy; pieces of the contraction of dx, which are added up in memory where there are several
+    int team, down;              // CTAs that work on neighbouring tiles of dW, below (1) or beside each other
+    int rounds, strips;          // groups of such tiles that a team takes whole; groups that are cut
     int teams, fewer;
     double share_fewer, share;   // how much of dW the first `fewer` teams take, and the others
     int ns;
 };
-BackwardPlan plan_backward(int M, int N, int K, bool want_dx, int sms);
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes = 1, int dx_pieces = 1);
 // dy [M, np] with zeros from column N on, w [w_rows, K].
 int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
                     int M, int N, int np, int K, int *status, cudaStream_t s);
+// The same from views of every fourth row of dy [M, N] (plan.classes = 4).  With plan.dx_pieces > 1 dx has to be zero.
+int launch_backward_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db,
+                                 int M, int N, int K, int *status, cudaStream_t s);
 // The kernel for results of few tiles (linear_split_sm100.cu): out[M, cols] = act[M, kc] . w^T + bias, with w [cols, kc],
 // or with w_mn_major [w_rows, cols] (its rows past w_rows, up to kc, read as zeros); optionally the bf16 planes of out.
 // `split` CTAs share the contraction of a tile.  Returns ATTN_OK or an error.
