@@ -120,7 +120,8 @@ inline cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, di
 // cuTensorMapEncodeTiled with the given swizzle, no interleave, no L2 promotion, zero fill; the encoder
 // is resolved by attn_sm100_init.  Returns 0 or a cudaError_t.
 int encode_tiled(CUtensorMap *map, CUtensorMapDataType dtype, unsigned rank, const void *base, const cuuint64_t *dims,
-                 const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
+                 const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B,
+                 CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_NONE);
 // Status word of the current device (initialises the library on first use).  Returns ATTN_OK or an error.
 int device_status_word(int **status);
 

@@ -78,12 +78,13 @@ __device__ __forceinline__ void exchange_halves(int odd, uint32_t (&r)[32]) {
 
 // Operand read K-major: matrix [rows, kc] row-major (kc contiguous = contraction); boxes of 32 x box_rows.
 // `pitch`: floats from one row to the next (0: kc).
-inline int map_k_major(CUtensorMap *map, const float *base, int rows, int kc, int box_rows, size_t pitch = 0) {
+inline int map_k_major(CUtensorMap *map, const float *base, int rows, int kc, int box_rows, size_t pitch = 0,
+                       CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_NONE) {
     if (pitch == 0) pitch = (size_t)kc;
     const cuuint64_t dims[4] = {(cuuint64_t)kc, (cuuint64_t)rows, 1, 1};
     const cuuint64_t strides[3] = {(cuuint64_t)pitch * 4, (cuuint64_t)pitch * 4 * (cuuint64_t)rows, (cuuint64_t)pitch * 4 * (cuuint64_t)rows};
     const cuuint32_t box[4] = {32, (cuuint32_t)box_rows, 1, 1};
-    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box);
+    return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, promotion);
 }
 // Operand read MN-major, whole tile in one copy: the matrix [kc, rows] seen as {32 values, kc, rows / 32 blocks}
 // with the block index as the slowest box dimension, box {32, 32, nblocks}: shared memory receives
