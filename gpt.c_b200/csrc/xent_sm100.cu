@@ -65,8 +65,9 @@ __global__ void __launch_bounds__(kThreads) xent_forward_kernel(const float *__r
             s *= __expf(m - bm);  // exp(-inf) = 0 on the first batch
             m = bm;
         }
+        const float low = m == -INFINITY ? 0.f : m;  // a thread that has seen nothing but -inf so far adds nothing
 #pragma unroll
-        for (int u = 0; u < kBatch; u++) s += __expf(v[u] - m);  // exp(-inf) = 0 past the end of the row
+        for (int u = 0; u < kBatch; u++) s += __expf(v[u] - low);  // exp(-inf) = 0 past the end of the row
     }
     // combine (m, s) pairs across the warp, then across the block
     const float wm = warp_max(m);

@@ -55,6 +55,25 @@ def test_cross_entropy_forward_backward_vs_cpu(pkg, rows, C):
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("rows,C", [(5, 50257), (9, 12000), (3, 9)])
+def test_cross_entropy_masked_classes(pkg, rows, C):
+    """Logits of -inf: probability 0, whatever their place in the row."""
+    L = pkg.lib()
+    logits = np.random.default_rng(C).standard_normal((rows, C)).astype(np.float32)
+    logits[:, : C * 8 // 9] = -np.inf
+    logits[0], logits[0, 0] = -np.inf, 1.0  # one class left
+    targets = np.full(rows, C - 1, np.float32)
+    targets[0] = 0
+    lt, tt = torch.from_numpy(logits).cuda(), torch.from_numpy(targets).cuda()
+    logsm, loss = torch.empty_like(lt), torch.zeros(1, device="cuda")
+    assert L.xent_sm100_forward(lt.data_ptr(), tt.data_ptr(), logsm.data_ptr(), loss.data_ptr(), rows, C, stream()) == 0
+    got, (ref, loss_ref) = logsm.cpu().numpy(), ops.xent_forward(logits, targets)
+    masked = np.isneginf(logits)
+    assert np.isneginf(got[masked]).all()
+    assert np.abs(got[~masked] - ref[~masked]).max() <= 2e-6 * max(1.0, np.abs(ref[~masked]).max())
+    assert abs(loss.item() - loss_ref) <= 1e-5 * max(1.0, abs(loss_ref))
+
+
 def test_cross_entropy_argument_errors(pkg):
     L = pkg.lib()
     assert L.xent_sm100_forward(None, None, None, None, 1, 1, None) == -1
