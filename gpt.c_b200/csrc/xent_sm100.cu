@@ -7,7 +7,7 @@
 //   backward  dout[r, target_r] = -g[r] / rows;  s = sum_j dout[r, j];  dout[r, j] -= exp(logsm[r, j]) * s
 // (the backward works on whatever dout holds, like the reference, whose layer hands in zeros).
 //
-// One block of 1024 threads per row; the rows of a [rows, 50257] tensor start on 4-byte boundaries only,
+// One block of 1024 threads per row (the forward of long rows: below); the rows of a [rows, 50257] tensor start on 4-byte boundaries only,
 // so loads and stores are 4 bytes wide but fully coalesced.  Forward: maximum and sum of exponentials in
 // one online pass, then the write pass re-reads the row (200 KB): 8 bytes of HBM traffic per element when the
 // re-read hits L2.  The forward loops keep eight loads per thread in flight: with one load per trip, which is
@@ -157,6 +157,186 @@ __global__ void __launch_bounds__(kThreads) xent_backward_kernel(const float *__
     }
 }
 
+// ---- forward of rows that fit in shared memory ----
+//
+// One CTA per SM goes through rows of up to kSlots * kSlot values, which the copy engine brings in pieces of 16 KB: a row is
+// read once, and while its results leave piece by piece the next rows follow into the places that become free, so that HBM
+// always has up to 200 KB of reads from every SM ahead of it (8192 x 50257: 628 -> 544 us, 6.05 TB/s).  The backward the same
+// way, its log-probabilities through registers, was no faster than its kernel above (883 and 880 us; rows of 16384 356, 270).
+constexpr int kSlot = 4096, kSlots = 13;  // floats of a piece; pieces of the ring: 208 KB
+constexpr int kWorkers = 512, kRowThreads = kWorkers + 32;
+constexpr int kPerThread = kSlot / 4 / kWorkers;  // 16-byte words of a piece per thread
+
+struct __align__(128) RowSmem {
+    float ring[kSlots][kSlot];
+    uint64_t full[kSlots], empty[kSlots];
+    float m[2][kWorkers / 32], s[2][kWorkers / 32];  // per warp, of this row and of the one before
+    int abort_flag;
+};
+enum Site : int { SITE_EMPTY = 251, SITE_FULL };
+
+// The words of a row that start on 16-byte boundaries, and the up to three values either side of them.
+struct Row {
+    int head, words;  // values before the first word, words
+    __device__ __forceinline__ Row(const float *x, int C) {
+        head = min(C, (int)((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / 4);
+        words = (C - head) / 4;
+    }
+    __device__ __forceinline__ int pieces() const { return (words * 4 + kSlot - 1) / kSlot; }
+    // the loose values, one each for the first threads: -1 for the others
+    __device__ __forceinline__ int loose(int thread, int C) const {
+        const int j = thread < head ? thread : head + 4 * words + thread - head;
+        return thread < head || (thread < 6 && j < C) ? j : -1;
+    }
+};
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tc05::smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(tc05::smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
+
+__device__ __forceinline__ void init_ring(RowSmem &sm) {
+    if (threadIdx.x == 0) {
+        sm.abort_flag = 0;
+        for (int i = 0; i < kSlots; i++) {
+            tc05::mbar_init(&sm.full[i], 1);
+            tc05::mbar_init(&sm.empty[i], kWorkers / 32);
+        }
+        tc05::fence_barrier_init();
+    }
+    __syncthreads();
+}
+// The place of a piece in the ring: pieces are counted through all rows of the CTA.
+struct Place {
+    int slot = 0;
+    uint32_t round = 0;
+    __device__ __forceinline__ void next() {
+        if (++slot == kSlots) slot = 0, round++;
+    }
+};
+// One thread: the pieces of every row of this CTA.
+__device__ __forceinline__ void load_rows(RowSmem &sm, const float *x, int rows, int C, const tc05::WaitCtx &ctx) {
+    Place at;
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+        const float *from = x + (size_t)r * C;
+        const Row row(from, C);
+        for (int c = 0; c < row.pieces(); c++, at.next()) {
+            if (at.round > 0 && !tc05::mbar_wait(&sm.empty[at.slot], (at.round - 1) & 1, ctx, SITE_EMPTY)) return;
+            const uint32_t bytes = min(kSlot, row.words * 4 - c * kSlot) * 4;
+            tc05::mbar_expect_tx(&sm.full[at.slot], bytes);
+            bulk_load(sm.ring[at.slot], from + row.head + c * kSlot, bytes, &sm.full[at.slot]);
+        }
+    }
+}
+// After a warp's last look at a piece: the copy engine may overwrite it.
+__device__ __forceinline__ void release(RowSmem &sm, int c) {
+    tc05::fence_proxy_async_smem();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) tc05::mbar_arrive(&sm.empty[c]);
+}
+
+__global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const float *__restrict__ logits, const float *__restrict__ targets,
+                                                                         float *__restrict__ logsm, float *__restrict__ loss, int rows,
+                                                                         int C, int *status) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    RowSmem &sm = *reinterpret_cast<RowSmem *>(smem_raw);
+    tc05::pdl_launch_dependents();
+    init_ring(sm);
+    tc05::pdl_wait();
+    tc05::WaitCtx ctx{&sm.abort_flag, status};
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid >= kWorkers) {
+        if (tid == kWorkers) load_rows(sm, logits, rows, C, ctx);
+        return;
+    }
+    Place first;
+    for (int r = blockIdx.x, n = 0; r < rows; r += gridDim.x, n++) {
+        const float *x = logits + (size_t)r * C;
+        float *y = logsm + (size_t)r * C;
+        const Row row(x, C);
+        const int loose = row.loose(tid, C), pieces = row.pieces();
+        const float mine = loose >= 0 ? x[loose] : -INFINITY, at_target = tid == 0 ? x[(int)targets[r]] : 0.f;
+        // maximum so far and four sums of exponentials; what is below the maximum of nothing (all -inf) adds nothing
+        float m = mine, s0 = loose >= 0 && mine != -INFINITY ? __expf(mine - m) : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        Place at = first;
+        for (int c = 0; c < pieces; c++, at.next()) {
+            if (!tc05::mbar_wait_warp(&sm.full[at.slot], at.round & 1, ctx, SITE_FULL)) break;  // the others learn of it behind workers_sync
+            const int words = min(kSlot / 4, row.words - c * (kSlot / 4));
+            const float4 *from = reinterpret_cast<const float4 *>(sm.ring[at.slot]);
+            float4 v[kPerThread];
+            float bm = -INFINITY;
+#pragma unroll
+            for (int u = 0; u < kPerThread; u++) {
+                const int i = tid + u * kWorkers;
+                v[u] = i < words ? from[i] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+                bm = fmaxf(fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)), bm);
+            }
+            if (bm > m) {
+                const float f = __expf(m - bm);  // exp(-inf) = 0 on the first piece
+                s0 *= f, s1 *= f, s2 *= f, s3 *= f;
+                m = bm;
+            }
+            const float low = m == -INFINITY ? 0.f : m;
+#pragma unroll
+            for (int u = 0; u < kPerThread; u++)
+                s0 += __expf(v[u].x - low), s1 += __expf(v[u].y - low), s2 += __expf(v[u].z - low), s3 += __expf(v[u].w - low);
+        }
+        float s = (s0 + s1) + (s2 + s3);
+        const float wm = warp_max(m);
+        s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));  // s is 0, or NaN, where there was nothing but -inf
+        if (lane == 0) sm.m[n & 1][warp] = wm, sm.s[n & 1][warp] = s;
+        workers_sync();
+        if (*ctx.cta_abort) return;
+        const float pm = lane < kWorkers / 32 ? sm.m[n & 1][lane] : -INFINITY, ps = lane < kWorkers / 32 ? sm.s[n & 1][lane] : 0.f;
+        const float top = warp_max(pm);
+        const float shift = top + logf(warp_sum(pm == -INFINITY ? ps : ps * __expf(pm - top)));
+        const bool whole = ((reinterpret_cast<uintptr_t>(x) ^ reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+        at = first;
+        for (int c = 0; c < pieces; c++, at.next()) {
+            const int words = min(kSlot / 4, row.words - c * (kSlot / 4));
+            const float4 *from = reinterpret_cast<const float4 *>(sm.ring[at.slot]);
+            float *to = y + row.head + c * kSlot;
+#pragma unroll
+            for (int u = 0; u < kPerThread; u++) {
+                const int i = tid + u * kWorkers;
+                if (i >= words) continue;
+                const float4 v = from[i];
+                const float4 o = make_float4(v.x - shift, v.y - shift, v.z - shift, v.w - shift);
+                if (whole) __stcs(reinterpret_cast<float4 *>(to) + i, o);
+                else __stcs(to + 4 * i, o.x), __stcs(to + 4 * i + 1, o.y), __stcs(to + 4 * i + 2, o.z), __stcs(to + 4 * i + 3, o.w);
+            }
+            release(sm, at.slot);
+        }
+        first = at;
+        if (loose >= 0) y[loose] = mine - shift;
+        if (tid == 0) atomicAdd(loss, -(at_target - shift) / (float)rows);
+    }
+}
+
+// Shorter rows gain nothing, several of whose blocks share an SM (8192 rows of 16384: 197 us there, 206 here, 24576: 271, 279,
+// 32000: 367, 351, 50257: 628, 544; 1 row of 50257: 9.8, 9.9, 37 rows: 12.1, 10.5).
+bool row_fits(int C) { return C >= 30000 && C <= kSlot * kSlots; }
+
+int launch_rows(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, cudaStream_t s) {
+    static bool ready[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64 || !ready[dev]) {
+        e = cudaFuncSetAttribute(xent_forward_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowSmem));
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64) ready[dev] = true;
+    }
+    int *status = nullptr;
+    const int rc = attn::device_status_word(&status);
+    if (rc != ATTN_OK) return rc;
+    const int sms = attn::sm_count();
+    return (int)attn::launch_after_previous(xent_forward_rows_kernel, dim3(rows < sms ? rows : sms), dim3(kRowThreads), sizeof(RowSmem), s,
+                                            logits, targets, logsm, loss, rows, C, status);
+}
+
 }  // namespace
 }  // namespace xent
 
@@ -165,6 +345,7 @@ extern "C" {
 int xent_sm100_forward(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, void *stream) {
     if (!logits || !targets || !logsm || !loss) return ATTN_ERR_NULL;
     if (rows <= 0 || C <= 0) return ATTN_ERR_SHAPE;
+    if (xent::row_fits(C)) return xent::launch_rows(logits, targets, logsm, loss, rows, C, static_cast<cudaStream_t>(stream));
     return (int)attn::launch_after_previous(xent::xent_forward_kernel, dim3(rows), dim3(xent::kThreads), 0,
                                             static_cast<cudaStream_t>(stream), logits, targets, logsm, loss, rows, C);
 }

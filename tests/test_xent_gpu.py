@@ -74,6 +74,73 @@ def test_cross_entropy_masked_classes(pkg, rows, C):
     assert abs(loss.item() - loss_ref) <= 1e-5 * max(1.0, abs(loss_ref))
 
 
+@pytest.mark.parametrize("rows,C,offsets", [
+    (1, 30000, (0, 0)), (3, 29999, (1, 2)),              # the shortest rows that are kept in shared memory, the longest that are not
+    (400, 50257, (0, 0)), (300, 50257, (3, 3)),          # several rows per CTA, up to three loose values either side of the words
+    (297, 31001, (1, 2)), (149, 32768, (2, 1)),          # logits and log-probabilities on different addresses modulo 16
+    (150, 53248, (0, 0)), (150, 53247, (1, 1)), (2, 53249, (0, 0)),  # every place of the ring full; a row too long for it
+])
+def test_cross_entropy_rows_in_shared_memory(pkg, rows, C, offsets):
+    """Rows on any 4-byte boundary, with values that are -inf, against the oracle; nothing is written outside."""
+    L = pkg.lib()
+    rng = np.random.default_rng(rows * 7 + C)
+    logits = (rng.standard_normal((rows, C)) * 3.0).astype(np.float32)
+    logits[rows // 2, : C // 2] = -np.inf  # masked classes, whole pieces of them
+    targets = rng.integers(C // 2, C, size=rows).astype(np.float32)
+    targets[0], targets[-1] = C - 1, C - 2
+    g = rng.standard_normal(rows).astype(np.float32)
+    with np.errstate(invalid="ignore"):
+        logsm_ref, loss_ref = ops.xent_forward(logits, targets)
+
+    def place(a, off):  # a copy that starts `off` floats past a 16-byte boundary, in a buffer of sevens
+        buf = torch.full((a.size + 16,), 7.0, device="cuda")
+        v = buf[4 + off:4 + off + a.size].view(a.shape)
+        v.copy_(torch.from_numpy(a))
+        return buf, v
+
+    def outside(buf, off, n):
+        return bool((buf[:4 + off] == 7.0).all()) and bool((buf[4 + off + n:] == 7.0).all())
+
+    _, lt = place(logits, offsets[0])
+    sbuf, logsm = place(np.zeros_like(logits), offsets[1])
+    tt, gt = torch.from_numpy(targets).cuda(), torch.from_numpy(g).cuda()
+    loss = torch.zeros(1, device="cuda")
+    assert L.xent_sm100_forward(lt.data_ptr(), tt.data_ptr(), logsm.data_ptr(), loss.data_ptr(), rows, C, stream()) == 0
+    got = logsm.cpu().numpy()
+    masked = np.isneginf(logits)
+    assert np.isneginf(got[masked]).all()
+    assert np.abs(got[~masked] - logsm_ref[~masked]).max() <= 2e-6 * np.abs(logsm_ref[~masked]).max()
+    unit = float(np.spacing(np.float32(loss_ref)))
+    assert abs(loss.item() - loss_ref) <= 1e-6 * abs(loss_ref) + 2e-6 + 6 * np.sqrt(rows / 12) * unit
+    assert outside(sbuf, offsets[1], logits.size)
+    d0 = (rng.standard_normal((rows, C)) * 0.01).astype(np.float32)
+    dbuf, dout = place(d0, offsets[0])
+    assert L.xent_sm100_backward(gt.data_ptr(), tt.data_ptr(), logsm.data_ptr(), dout.data_ptr(), rows, C, stream()) == 0
+    d_ref = ops.xent_backward(g, targets, np.where(masked, -np.inf, logsm_ref), d0)
+    assert np.abs(dout.cpu().numpy() - d_ref).max() <= 1e-6 + 1e-5 * np.abs(d_ref).max()
+    assert outside(dbuf, offsets[0], logits.size)
+    assert pkg.device_status() == 0
+
+
+def test_cross_entropy_keeps_rows_apart(pkg):
+    """A NaN or an infinity stays in its own row; a row of -inf has no probabilities."""
+    L = pkg.lib()
+    rows, C = 310, 30003
+    logits = np.random.default_rng(5).standard_normal((rows, C)).astype(np.float32)
+    bad = {3: (0, np.nan), 4: (C - 1, np.nan), 160: (7777, np.inf), 200: (slice(None), -np.inf)}
+    for row, (col, value) in bad.items():
+        logits[row, col] = value
+    lt, tt = torch.from_numpy(logits).cuda(), torch.zeros(rows, device="cuda")
+    logsm, loss = torch.empty_like(lt), torch.zeros(1, device="cuda")
+    assert L.xent_sm100_forward(lt.data_ptr(), tt.data_ptr(), logsm.data_ptr(), loss.data_ptr(), rows, C, stream()) == 0
+    got = logsm.cpu().numpy()
+    rest = np.setdiff1d(np.arange(rows), list(bad))
+    for row in bad:  # an infinite logit: log(inf) below it everywhere, inf - inf at its place
+        assert not np.isfinite(got[row]).any()
+    ref, _ = ops.xent_forward(logits[rest], np.zeros(len(rest), np.float32))
+    assert np.abs(got[rest] - ref).max() <= 2e-6 * np.abs(ref).max()
+
+
 def test_cross_entropy_argument_errors(pkg):
     L = pkg.lib()
     assert L.xent_sm100_forward(None, None, None, None, 1, 1, None) == -1
