@@ -550,14 +550,17 @@ int stream_rows_of_c(int M, int N, int K) {
 bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
 // Whether the gradients of a [M, N] result come from views of every fourth row of dy, whose rows are not 16-byte aligned,
-// and not from a copy with padded rows.  The copy is cheap as long as it stays in L2 (128 MB), and dx as four products
-// of a quarter of the rows wants at least eight row tiles in each.  dx and dW, copy -> views, in us (N, K; M):
-//     50257, 768; 1024: 398 -> 470, 2048: 675 -> 826, 4096: 1455 -> 1215, 8192: 3000 -> 2520
-//     50257, 384; 1024: 272 -> 293, 2048: 475 -> 503, 4096: 942 -> 902, 8192: 1930 -> 1662
-//     16387, 512; 1024: 102 -> 105, 2048: 186 -> 182, 4096: 349 -> 316, 8192: 720 -> 541
-//      4099, 768; 1024: 39 -> 74, 4096: 119 -> 134, 8192: 256 -> 218          1001, 768; 2048: 26 -> 63, 8192: 66 -> 87
-// The size of the scratch buffer follows from the shape alone, so this must too.
-bool by_row_class(int M, int N) { return N % 4 != 0 && M >= 4096 && (long long)M * N >= (32 << 20); }
+// and not from a copy with padded rows.  The copy is cheap as long as it stays in L2 (128 MB); the views add each tile of dW to
+// memory four times, which costs more than the copy where K is large beside M.  dx and dW, copy -> views, in us (N, K; M):
+//     50257, 768; 700: 280 -> 320, 1024: 378 -> 357, 2048: 655 -> 591      50257, 384; 1024: 291 -> 224, 2048: 537 -> 401
+//     50257, 1600; 2048: 1340 -> 1520, 4096: 2975 -> 2817                  16387, 512; 3000: 267 -> 210
+//     30001, 1024; 1500: 396 -> 394                                        13001, 768; 3000: 244 -> 242
+// From 4096 rows on it is the views in any case.  Below, dx of a contraction of less than 16384 has the same bits in every call,
+// which pieces that add into zeros would not give it.  The size of the scratch buffer follows from the shape alone, so this must too.
+bool by_row_class(int M, int N, int K) {
+    if (N % 4 == 0 || (long long)M * N < (32 << 20)) return false;
+    return M >= 4096 || (N >= 16384 && M >= 1000 && 3ll * M >= 4ll * K);
+}
 
 // dx, dW and db (dx or dw may be NULL) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut into
 // pieces that add into zeros: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from
@@ -671,8 +674,7 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
 }
 
 size_t linear_sm100_backward_scratch_bytes(int M, int N, int K) {
-    (void)K;
-    if (M <= 0 || N <= 0 || N % 32 == 0 || lin::by_row_class(M, N)) return 0;
+    if (M <= 0 || N <= 0 || N % 32 == 0 || lin::by_row_class(M, N, K)) return 0;
     const size_t np = ((size_t)N + 31) / 32 * 32;
     return (size_t)M * np * sizeof(float);
 }
@@ -683,7 +685,7 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     if (!dy || !w || (!dx && !dw) || (dw && !x)) return ATTN_ERR_NULL;
     if (M <= 0 || N <= 0 || K <= 0 || (long long)M * N > 0x7fffffffLL || (long long)M * K > 0x7fffffffLL) return ATTN_ERR_SHAPE;
     if (K % 32 != 0) return ATTN_ERR_UNSUPPORTED;
-    const bool classes = by_row_class(M, N);
+    const bool classes = by_row_class(M, N, K);
     const bool padded = N % 32 != 0 && !classes;  // dy's rows cannot be tiles of the copy engine: work on a padded copy
     const int np = (N + 31) / 32 * 32;
     if ((long long)M * np > 0x7fffffffLL) return ATTN_ERR_SHAPE;

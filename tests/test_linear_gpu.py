@@ -287,6 +287,24 @@ def test_linear_backward_in_one_launch(pkg, M, N, K, with_db):
     assert bool((db[:at] == 0.5).all()) and bool((db[at + N:] == 0.5).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(1000, 33555, 64), (1025, 32801, 96), (3001, 16387, 320), (2050, 16386, 1536)])
+def test_linear_backward_from_every_fourth_row_of_fewer(pkg, M, N, K):
+    """Below 4096 rows, with a contraction of dx that is cut into pieces: views of dy, or a copy where K is large beside M (the
+    last one)."""
+    x, w, _, dy = inputs(M, N, K, 71)
+    dw0 = np.random.default_rng(3).standard_normal((N, K), dtype=np.float32)
+    xt, wt, dyt, dw = (torch.from_numpy(a).cuda() for a in (x, w, dy, dw0))
+    db = torch.zeros(N, device="cuda")
+    need = pkg.lib().linear_sm100_backward_scratch_bytes(M, N, K)
+    assert (need == 0) == (3 * M >= 4 * K)
+    dx = pkg.linear_backward(dyt, xt, wt, dw, db)
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, dw0, np.zeros(N, np.float32))
+    within(dx.cpu().numpy(), dx_ref, dy, w)
+    within(dw.cpu().numpy(), dw_ref, dy.T, x)
+    assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+
+
 def test_linear_backward_results_over_operands(pkg):
     """Where dW lies over w, dx comes from w as it was; where db lies over dy, dW comes from dy as it was."""
     M, N, K = 1024, 512, 512
