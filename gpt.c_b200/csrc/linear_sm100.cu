@@ -12,7 +12,7 @@
 //     dx       dx[M,K]  = dy[M,N] . W[N,K]          A: dy, K-major (over N) B: W,  MN-major
 // dx is made here where it is wanted alone or has few rows; dW, db and elsewhere dx are linear_backward_sm100.cu's.
 // (K-major: the contraction index is the contiguous one.)  Contraction blocks are 32 fp32 values (one 128-byte
-// swizzled row).  A tile is 128 rows by 128, 192 or 256 columns, with as many pipeline stages as shared memory holds;
+// swizzled row).  A tile is 128 rows by 128, 192 or 256 columns, or 256 rows by 192 or 256, with as many pipeline stages as shared memory holds;
 // plan_tiles picks the width.
 //
 // What bounds the kernel: a 128 x 256 tile needs 48 KB per contraction block, and the SMs get 15 to 18 TB/s from L2
@@ -43,9 +43,9 @@ constexpr int kEpiWarps = 8;
 
 // Tile width kBN (128, 192 or 256 columns) and pipeline depth are chosen per problem: wide tiles halve the
 // shared-memory and L2 traffic per flop, narrow ones fill the SMs better when there are few tiles.
-template <int kBN, int kStages, bool kStage>
+template <int kRows, int kBN, int kStages, bool kStage>
 struct __align__(1024) SmemT {
-    uint8_t a[kStages][kATileBytes];
+    uint8_t a[kStages][kRows * kATileBytes];
     uint8_t b[kStages][kBN * kBK * 4];
     uint8_t out[kStage ? kEpiWarps : 1][kStage ? 4096 : 16];  // output staging of the epilogue warps: 32 rows x 128 bytes
     uint64_t full[kStages], empty[kStages];
@@ -56,7 +56,7 @@ struct __align__(1024) SmemT {
 
 struct Problem {
     int M, N, K;  // C is [M, N]; K is the contraction length
-    int bn;       // tile width
+    int rows, bn;  // tile height in blocks of 128 rows, width
     int b_one;    // MN-major B fetched with one 3-D copy per stage (else one copy per 32-row block)
     int tiles_m, tiles_n, splits, kb_total, kb_per_split, total;
     int wide, wide_planes;  // rows of C / of the planes start on 32-byte boundaries
@@ -84,7 +84,7 @@ __device__ __forceinline__ Work decode(const Problem &p, int w) {
     const int tn = p.m_fast ? t / p.tiles_m : t % p.tiles_n;
     const int tm = p.m_fast ? t % p.tiles_m : t / p.tiles_n;
     Work r;
-    r.m0 = tm * kBM;
+    r.m0 = tm * p.rows * kBM;
     r.n0 = tn * p.bn;
     r.kb0 = split * p.kb_per_split;
     r.kb1 = min(p.kb_total, r.kb0 + p.kb_per_split);
@@ -94,12 +94,13 @@ __device__ __forceinline__ Work decode(const Problem &p, int w) {
 // kEpi 0: C = acc (+ bias), optional bf16 planes; kEpi 1: C += acc (bulk reduction)
 // kDirect: the result goes out with plain coalesced 4-byte stores, for outputs whose row pitch is not a multiple of 16
 // bytes (the 50257-wide vocabulary projection).
-template <bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect>
+template <bool kBMN, int kEpi, int kRows, int kBN, int kStages, bool kPlanes, bool kDirect>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_gemm_kernel(const __grid_constant__ Maps maps, const float *__restrict__ bias, float *__restrict__ c_direct,
                    uint32_t *__restrict__ planes, Problem p, int *status) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    using Smem = SmemT<kBN, kStages, kEpi == 1 || kDirect>;
+    using Smem = SmemT<kRows, kBN, kStages, kEpi == 1 || kDirect>;
+    constexpr int kAccs = 2 / kRows;  // accumulators of 128 rows, one read out while the other is filled; or one of 256
     constexpr uint32_t kTmemCols = 2 * kBN <= 256 ? 256 : 512;  // a power of two that holds two accumulators
     constexpr int kBTileBytes = kBN * kBK * 4;
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
@@ -149,14 +150,15 @@ linear_gemm_kernel(const __grid_constant__ Maps maps, const float *__restrict__ 
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(&sm.full[st], kATileBytes + kBTileBytes);
+                    mbar_expect_tx(&sm.full[st], kRows * kATileBytes + kBTileBytes);
                     auto load = [&](void *dst, const CUtensorMap *map, int c0, int c1, int c2) {
                         tma_load_4d(dst, map, &sm.full[st], c0, c1, c2, 0);
                     };
                     const int b0 = wk.n0;
                     // K-major: map {contraction, rows}, one box {32, 128}.  MN-major: map {rows, contraction},
                     // boxes {32, 32}: blocks of 32 rows, each [32 contraction steps x 128 bytes].
-                    load(sm.a[st], &maps.a, kb * kBK, wk.m0, 0);
+#pragma unroll
+                    for (int h = 0; h < kRows; h++) load(sm.a[st] + h * kATileBytes, &maps.a, kb * kBK, wk.m0 + h * kBM, 0);
                     if (kBMN) {
                         if (p.b_one) {
                             load(sm.b[st], &maps.b, 0, kb * kBK, b0 / 32);
@@ -179,8 +181,8 @@ linear_gemm_kernel(const __grid_constant__ Maps maps, const float *__restrict__ 
         bool ok = true;
         for (int w = first; ok && w < p.total; w += step, j++) {
             const Work wk = decode(p, w);
-            const int acc = j & 1;
-            if (j >= 2 && !mbar_wait_warp(&sm.acc_empty[acc], ((j >> 1) - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
+            const int acc = j % kAccs;
+            if (j >= kAccs && !mbar_wait_warp(&sm.acc_empty[acc], (j / kAccs - 1) & 1, ctx, SITE_ACC_EMPTY)) break;
             tc_fence_after_sync();
             const uint32_t d = tmem + (uint32_t)acc * kBN;
             for (int kb = wk.kb0; kb < wk.kb1; kb++, it++) {
@@ -198,7 +200,8 @@ linear_gemm_kernel(const __grid_constant__ Maps maps, const float *__restrict__ 
                 for (int k = 0; k < kBK / 8; k++) {
                     const uint64_t ak = desc_advance(ad, k * 32), bk = desc_advance(bd, k * (kBMN ? 1024 : 32));
                     const uint32_t add = (kb > wk.kb0 || k > 0) ? 1u : 0u;
-                    mma_tf32_lead(leader, d, ak, bk, idesc, add);
+#pragma unroll
+                    for (int h = 0; h < kRows; h++) mma_tf32_lead(leader, d + h * kBN, desc_advance(ak, h * kATileBytes), bk, idesc, add);
                 }
                 tc_commit_lead(leader, &sm.empty[st]);
             }
@@ -218,23 +221,24 @@ linear_gemm_kernel(const __grid_constant__ Maps maps, const float *__restrict__ 
         int j = 0;
         for (int w = first; w < p.total; w += step, j++) {
             const Work wk = decode(p, w);
-            const int acc = j & 1;
-            const int row0 = wk.m0 + 32 * quarter;
+            const int acc = j % kAccs;
             float bv[kChunks];  // bias of the columns col0 + lane, fetched while the tile is still being computed
 #pragma unroll
             for (int c = 0; c < kChunks; c++) {
                 const int col = wk.n0 + half * (kBN / 2) + 32 * c + lane;
                 bv[c] = kEpi == 0 && bias != nullptr && col < p.N ? __ldg(bias + col) : 0.f;
             }
-            if (!mbar_wait_warp(&sm.acc_full[acc], (j >> 1) & 1, ctx, SITE_ACC_FULL)) break;
+            if (!mbar_wait_warp(&sm.acc_full[acc], (j / kAccs) & 1, ctx, SITE_ACC_FULL)) break;
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < kChunks; c++) {
+            for (int i = 0; i < kRows * kChunks; i++) {
+                const int h = i / kChunks, c = i % kChunks;
+                const int row0 = wk.m0 + h * kBM + 32 * quarter;
                 const int off = half * (kBN / 2) + 32 * c, col0 = wk.n0 + off;
                 uint32_t r[32];
-                tmem_ld32(tmem + lane_addr + (uint32_t)acc * kBN + off, r);
+                tmem_ld32(tmem + lane_addr + (uint32_t)(acc + h) * kBN + off, r);
                 tmem_wait_ld();
-                if (c == kChunks - 1) {  // the accumulator has been read out: the tensor cores may reuse it
+                if (i == kRows * kChunks - 1) {  // the accumulator has been read out: the tensor cores may reuse it
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
@@ -420,13 +424,13 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(float *__restrict__ dst, 
 
 // ---- host side ----
 
-Problem make_problem(int M, int N, int K, int bn, int splits) {
+Problem make_problem(int M, int N, int K, int rows, int bn, int splits) {
     Problem p;
-    p.M = M, p.N = N, p.K = K, p.bn = bn;
+    p.M = M, p.N = N, p.K = K, p.rows = rows, p.bn = bn;
     p.b_one = 0;
     p.m_fast = 0;
     p.ldc = (size_t)N;
-    p.tiles_m = (M + kBM - 1) / kBM;
+    p.tiles_m = (M + rows * kBM - 1) / (rows * kBM);
     p.tiles_n = (N + bn - 1) / bn;
     p.kb_total = (K + kBK - 1) / kBK;
     if (splits < 1) splits = 1;
@@ -443,18 +447,22 @@ Problem make_problem(int M, int N, int K, int bn, int splits) {
 // on 224 shapes of 100 to 8192 rows and 512 to 6400 columns (mean error 5 %).  Wide tiles read the least per flop and
 // win when there are many, narrow ones leave a smaller last round.
 struct Plan {
-    int bn, splits;
+    int rows, bn, splits;
     int ns;
 };
 struct Cost {
-    int bn, fixed, round, block;  // nanoseconds
+    int rows, bn, fixed, round, block;  // nanoseconds
 };
-constexpr Cost kCosts[3] = {{256, 4470, 2030, 283}, {192, 4450, 900, 232}, {128, 3920, 400, 226}};
+// Tiles of 256 rows take a third less from L2 and shared memory per product (a block of 256 x 192 in 0.52 us where two of 128 x 192
+// take 0.67), but have one accumulator: nothing is computed while a tile leaves.  They win where the contraction is long or they
+// end in fewer rounds (us, 128 rows -> 256: 8192 x 768 x 3072 66 -> 59, 8192 x 2304 x 768 with planes 60 -> 57.5, 1500 x 4800 x
+// 1600 with planes 54 -> 49; 8192 x 3072 x 768 67.7 -> 68.2, 1500 x 1600 x 6400 61 -> 99).
+constexpr Cost kCosts[5] = {{1, 256, 4470, 2030, 283}, {1, 192, 4450, 900, 232}, {1, 128, 3920, 400, 226}, {2, 256, 5000, 5600, 620}, {2, 192, 4500, 4000, 520}};
 constexpr int kL2BytesPerNs = 18190;
 
 // Time of `tiles` tiles of kb contraction blocks each, without the fixed part.
 long long rounds_ns(const Cost &c, long long tiles, int kb, int sms) {
-    const long long bytes = kATileBytes + (long long)c.bn * kBK * 4;  // a CTA's operands of one block
+    const long long bytes = c.rows * kATileBytes + (long long)c.bn * kBK * 4;  // a CTA's operands of one block
     auto round = [&](long long busy) {
         const long long fed = bytes * busy / kL2BytesPerNs;
         return c.round + kb * (fed > c.block ? fed : c.block);
@@ -467,15 +475,15 @@ int at_most_int(long long v) { return v < 0x7fffffff ? (int)v : 0x7fffffff; }
 
 // What does not fit in L2 arrives from HBM at 5.0 TB/s, after a start of 6 us.
 Plan plan_tiles(int M, int N, int kb, int sms) {
-    Plan best{128, 1, 0};
+    Plan best{1, 128, 1, 0};
     const long long bytes = 4ll * ((long long)M * N + (long long)kb * kBK * (M + N));
     const long long least = bytes > (100ll << 20) ? 6000 + bytes / 5000 : 0;
     for (const Cost &c : kCosts) {
         if (c.bn > 128 && N < c.bn) continue;
-        const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + c.bn - 1) / c.bn);
+        const long long tiles = (long long)((M + c.rows * kBM - 1) / (c.rows * kBM)) * ((N + c.bn - 1) / c.bn);
         long long t = c.fixed + rounds_ns(c, tiles, kb, sms);
         if (t < least) t = least;
-        if (best.ns == 0 || t < best.ns) best = Plan{c.bn, 1, at_most_int(t)};
+        if (best.ns == 0 || t < best.ns) best = Plan{c.rows, c.bn, 1, at_most_int(t)};
     }
     return best;
 }
@@ -483,9 +491,9 @@ Plan plan_tiles(int M, int N, int kb, int sms) {
 // The same with the contraction cut into up to 32 pieces that add into the result with bulk reductions (dW, and dx when
 // its contraction is very long); those cost 80 ns per megabyte and make a block 15 % slower.
 Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks, int most = 32) {
-    Plan best{128, 1, 0};
+    Plan best{1, 128, 1, 0};
     for (const Cost &c : kCosts) {
-        if (c.bn > 128 && N < c.bn) continue;
+        if (c.rows > 1 || (c.bn > 128 && N < c.bn)) continue;
         const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + c.bn - 1) / c.bn);
         const long long tile_bytes = (long long)kBM * c.bn * 4;
         for (int s = 1; s <= most && s <= kb; s++) {
@@ -493,21 +501,21 @@ Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks, int most = 32)
             if (s > 1 && per < least_blocks) break;
             const long long t = c.fixed + rounds_ns(c, tiles * s, per, sms) * 115 / 100 +
                                 tiles * s * tile_bytes / 1000 * 80 / 1000;
-            if (best.ns == 0 || t < best.ns) best = Plan{c.bn, s, at_most_int(t)};
+            if (best.ns == 0 || t < best.ns) best = Plan{1, c.bn, s, at_most_int(t)};
         }
     }
     return best;
 }
 
-template <bool kBMN, int kEpi, int kBN, int kStages, bool kPlanes, bool kDirect>
+template <bool kBMN, int kEpi, int kRows, int kBN, int kStages, bool kPlanes, bool kDirect>
 int launch_one(const Maps &maps, const float *bias, float *c, void *planes, Problem p, int *status, cudaStream_t s) {
-    using Smem = SmemT<kBN, kStages, kEpi == 1 || kDirect>;
+    using Smem = SmemT<kRows, kBN, kStages, kEpi == 1 || kDirect>;
     static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of the Linear kernel");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    auto kernel = linear_gemm_kernel<kBMN, kEpi, kBN, kStages, kPlanes, kDirect>;
+    auto kernel = linear_gemm_kernel<kBMN, kEpi, kRows, kBN, kStages, kPlanes, kDirect>;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
         if (e != cudaSuccess) return (int)e;
@@ -525,17 +533,23 @@ int launch_one(const Maps &maps, const float *bias, float *c, void *planes, Prob
 // Pipeline depth by what fits in 227 KiB next to the output staging tile.
 template <bool kBMN, int kEpi>
 int launch(const Maps &maps, const float *bias, float *c, void *planes, const Problem &p, int *status, cudaStream_t s) {
-#define GO(bn, stages, with_planes) \
-    return launch_one<kBMN, kEpi, bn, stages, with_planes, false>(maps, bias, c, planes, p, status, s)
+#define GO(rows, bn, stages, with_planes) \
+    return launch_one<kBMN, kEpi, rows, bn, stages, with_planes, false>(maps, bias, c, planes, p, status, s)
     constexpr bool kCanPlanes = !kBMN && kEpi == 0;  // only the forward product writes planes
     if constexpr (kCanPlanes) {
-        if (planes && p.bn == 256) GO(256, 4, true);
-        if (planes && p.bn == 192) GO(192, 5, true);
-        if (planes) GO(128, 6, true);
+        if (planes && p.rows == 2 && p.bn == 256) GO(2, 256, 3, true);
+        if (planes && p.rows == 2) GO(2, 192, 4, true);
+        if (planes && p.bn == 256) GO(1, 256, 4, true);
+        if (planes && p.bn == 192) GO(1, 192, 5, true);
+        if (planes) GO(1, 128, 6, true);
     }
-    if (p.bn == 256) GO(256, 4, false);
-    if (p.bn == 192) GO(192, kEpi == 1 ? 4 : 5, false);
-    GO(128, 6, false);
+    if constexpr (kEpi == 0) {
+        if (p.rows == 2 && p.bn == 256) GO(2, 256, 3, false);
+        if (p.rows == 2) GO(2, 192, 4, false);
+    }
+    if (p.bn == 256) GO(1, 256, 4, false);
+    if (p.bn == 192) GO(1, 192, kEpi == 1 ? 4 : 5, false);
+    GO(1, 128, 6, false);
 #undef GO
 }
 
@@ -613,7 +627,7 @@ int input_gradient(const InputGradient &how, const float *g, const float *w, flo
     const Plan &plan = how.tiles;
     int rc;
     Maps maps = {};
-    Problem p = make_problem(M, K, np, plan.bn, plan.splits);
+    Problem p = make_problem(M, K, np, plan.rows, plan.bn, plan.splits);
     if ((rc = map_k_major(&maps.a, g, M, np, 128)) != 0) return rc;
     p.b_one = map_mn_major_blocks(&maps.b, w, N, K, p.bn / 32) == 0;
     if (!p.b_one && (rc = map_mn_major(&maps.b, w, N, K)) != 0) return rc;
@@ -665,11 +679,11 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
         return launch_split(x, w, false, 0, bias, y, planes, M, N, K, split, sms, status, s);
     Maps maps = {};
     // with plain stores (N not a multiple of 4) only the widest tiles are built
-    Problem p = make_problem(M, N, K, direct ? 256 : plan.bn, 1);
+    Problem p = make_problem(M, N, K, direct ? 1 : plan.rows, direct ? 256 : plan.bn, 1);
     p.m_fast = stream_rows_of_c(M, N, K);
     if ((rc = map_k_major(&maps.a, x, M, K, 128)) != 0) return rc;
     if ((rc = map_k_major(&maps.b, w, N, K, p.bn)) != 0) return rc;
-    if (direct) return launch_one<false, 0, 256, 4, false, true>(maps, bias, y, nullptr, p, status, s);
+    if (direct) return launch_one<false, 0, 1, 256, 4, false, true>(maps, bias, y, nullptr, p, status, s);
     return launch<false, 0>(maps, bias, y, planes, p, status, s);
 }
 

@@ -305,6 +305,24 @@ def test_linear_backward_from_every_fourth_row_of_fewer(pkg, M, N, K):
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
 
 
+@pytest.mark.parametrize("M,N,K", [(1411, 4800, 1600), (2305, 2312, 1568), (8001, 760, 3072)])
+def test_linear_tiles_of_256_rows(pkg, M, N, K):
+    """Forward with bias and planes and dx alone, where tiles of 256 rows by 256 or 192 columns are taken: the last ones with
+    fewer rows and columns, one with rows in its lower half only."""
+    x, w, b, _ = inputs(M, N, K, 73)
+    xt, wt, bt = (torch.from_numpy(a).cuda() for a in (x, w, b))
+    planes = torch.zeros(2 * ((M * N * 2 + 255) // 256 * 256), dtype=torch.uint8, device="cuda")
+    y = pkg.linear_forward(xt, wt, bt, planes=planes)
+    within(y.cpu().numpy(), ops.linear_forward(x, w, b), x, w.T)
+    hi, lo = (p[: M * N * 2].view(torch.bfloat16).view(M, N) for p in planes.chunk(2))
+    assert torch.equal(hi, y.bfloat16()) and torch.equal(lo, (y - hi.float()).bfloat16())
+    # x as the gradient of a [M, K] result
+    w2 = np.ascontiguousarray(w.T[:, : N // 32 * 32])
+    dx = pkg.linear_backward(xt, torch.empty(M, w2.shape[1], device="cuda"), torch.from_numpy(w2).cuda(), None, None)
+    assert pkg.device_status() == 0
+    within(dx.cpu().numpy(), x.astype(np.float64) @ w2.astype(np.float64), x, w2)
+
+
 def test_linear_backward_results_over_operands(pkg):
     """Where dW lies over w, dx comes from w as it was; where db lies over dy, dW comes from dy as it was."""
     M, N, K = 1024, 512, 512
