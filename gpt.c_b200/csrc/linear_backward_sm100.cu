@@ -41,7 +41,7 @@ constexpr int kThreads = 384, kEpiWarps = 8;
 constexpr int kBN = 256;                             // columns of an accumulator
 constexpr int kMostStages = 6, kRingBytes = 192 * 1024;  // pipeline: as many stages as fit, of 16 KB of A and up to 32 KB of B
 
-enum Site : int { SITE_EMPTY = 231, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_DB, SITE_SMEM_ALIGN };
+enum Site : int { SITE_EMPTY = 261, SITE_FULL, SITE_ACC_EMPTY, SITE_ACC_FULL, SITE_DB, SITE_SMEM_ALIGN };
 
 struct __align__(1024) Smem {
     uint8_t ring[kRingBytes];

@@ -15,17 +15,18 @@
 // swizzled row).  A tile is 128 rows by 128, 192 or 256 columns, or 256 rows by 192 or 256, with as many pipeline stages as shared memory holds;
 // plan_tiles picks the width.
 //
-// What bounds the kernel: a 128 x 256 tile needs 48 KB per contraction block, and the SMs get 15 to 18 TB/s from L2
-// together (tensor pipe active 48 % in the forward with bf16 planes, 76 % in dW).  The result is written straight from
-// registers, 64 bytes of a row per pair of lanes: staging it for the copy engine costs shared memory that the pipeline
-// wants, bandwidth, and hand-overs between warps (QKV forward with bf16 planes 72 -> 67 us at 192 columns).
+// What bounds the kernel: shared memory takes a contraction block's operands in and hands them to the tensor cores, 128 bytes a
+// cycle in all, 2 R + n + R n / 128 cycles for R rows by n columns against R n / 64 in the tensor cores (128 x 192 60 %, 128 x 256
+// 67, 256 x 192 71, 256 x 256 80 % of their rate; ncu: 48 % busy in the forward with bf16 planes, 82 % at 8192 x 768 x 3072).
+// The result is written straight from registers, 64 bytes of a row per pair of lanes: staging it for the copy engine costs shared
+// memory that the pipeline wants, bandwidth, and hand-overs between warps (QKV forward with bf16 planes 72 -> 67 us at 192 columns).
 //
 // Warp roles (384 threads, one CTA per SM, grid = number of SMs, tiles handed out round robin):
 //   warp 0      TMA producer
 //   warp 1      MMA issuer (kind::tf32, one elected lane)
 //   warp 2      tensor-memory allocation (2 accumulators: the epilogue of one tile overlaps the main loop of the next)
 //   warps 4-11  epilogue: 32 rows and half of the columns each, (+ bias, bf16 split) -> global memory, or through a
-//               staging buffer of the warp's own to a bulk tensor reduction (dW) or unaligned rows (vocabulary)
+//               staging buffer of the warp's own to a bulk tensor reduction (dx in pieces) or unaligned rows (vocabulary)
 // The waits on barriers are bounded (tc05.cuh).  Two others end for the reasons given there and need no limit: the
 // allocation of tensor memory, and the wait for the previous kernel of the stream.
 #include "linear_tf32.cuh"
@@ -488,7 +489,7 @@ Plan plan_tiles(int M, int N, int kb, int sms) {
     return best;
 }
 
-// The same with the contraction cut into up to 32 pieces that add into the result with bulk reductions (dW, and dx when
+// The same with the contraction cut into up to 32 pieces that add into the result with bulk reductions (dx when
 // its contraction is very long); those cost 80 ns per megabyte and make a block 15 % slower.
 Plan plan_pieces(int M, int N, int kb, int sms, int least_blocks, int most = 32) {
     Plan best{1, 128, 1, 0};
@@ -570,11 +571,13 @@ bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) ==
 //     50257, 1600; 2048: 1340 -> 1520, 4096: 2975 -> 2817                  16387, 512; 3000: 267 -> 210
 //     30001, 1024; 1500: 396 -> 394                                        13001, 768; 3000: 244 -> 242
 // From 4096 rows on it is the views in any case.  Below, dx of a contraction of less than 16384 has the same bits in every call,
-// which pieces that add into zeros would not give it.  The size of the scratch buffer follows from the shape alone, so this must too.
+// which pieces that add into zeros would not give it.
 bool by_row_class(int M, int N, int K) {
     if (N % 4 == 0 || (long long)M * N < (32 << 20)) return false;
     return M >= 4096 || (N >= 16384 && M >= 1000 && 3ll * M >= 4ll * K);
 }
+// Whether a caller has to bring room for the copy: wherever it may be made.
+bool wants_scratch(int M, int N) { return N % 32 != 0 && (N % 4 == 0 || M < 4096 || (long long)M * N < (32 << 20)); }
 
 // dx, dW and db (dx or dw may be NULL) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut into
 // pieces that add into zeros: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from
@@ -688,7 +691,8 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
 }
 
 size_t linear_sm100_backward_scratch_bytes(int M, int N, int K) {
-    if (M <= 0 || N <= 0 || N % 32 == 0 || lin::by_row_class(M, N, K)) return 0;
+    (void)K;
+    if (M <= 0 || N <= 0 || !lin::wants_scratch(M, N)) return 0;
     const size_t np = ((size_t)N + 31) / 32 * 32;
     return (size_t)M * np * sizeof(float);
 }
@@ -703,7 +707,7 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     const bool padded = N % 32 != 0 && !classes;  // dy's rows cannot be tiles of the copy engine: work on a padded copy
     const int np = (N + 31) / 32 * 32;
     if ((long long)M * np > 0x7fffffffLL) return ATTN_ERR_SHAPE;
-    if (padded && !scratch) return ATTN_ERR_NULL;
+    if (wants_scratch(M, N) && !scratch) return ATTN_ERR_NULL;
     // dy itself must start on a 16-byte boundary in both cases: the padding kernel reads it in 16-byte words
     if (!aligned16(dy) || !aligned16(x) || !aligned16(w) || !aligned16(dx) || !aligned16(dw) ||
         (N % 32 == 0 && !aligned16(db)) || !aligned16(scratch))

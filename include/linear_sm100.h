@@ -42,10 +42,9 @@ int linear_sm100_forward(const float *x, const float *w, const float *bias, floa
 
 /*
  * Bytes of device scratch linear_sm100_backward needs: 0 when N is a multiple of 32, and when it is not even
- * a multiple of 4 but dy is large, M * N >= 2^25 and M >= 4096 (the vocabulary projection of a training step,
+ * a multiple of 4 but dy is large, M >= 4096 and M * N >= 2^25 (the vocabulary projection of a training step,
  * N = 50257: its rows start on 4-byte boundaries only, which the copy engine cannot tile, but every fourth row it
- * can), or N >= 16384, M >= 1000 and M >= 4/3 K.  Else room for a copy of dy whose rows are padded to the next
- * multiple of 32 columns.
+ * can).  Else room for a copy of dy whose rows are padded to the next multiple of 32 columns.
  */
 size_t linear_sm100_backward_scratch_bytes(int M, int N, int K);
 

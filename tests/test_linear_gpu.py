@@ -295,8 +295,6 @@ def test_linear_backward_from_every_fourth_row_of_fewer(pkg, M, N, K):
     dw0 = np.random.default_rng(3).standard_normal((N, K), dtype=np.float32)
     xt, wt, dyt, dw = (torch.from_numpy(a).cuda() for a in (x, w, dy, dw0))
     db = torch.zeros(N, device="cuda")
-    need = pkg.lib().linear_sm100_backward_scratch_bytes(M, N, K)
-    assert (need == 0) == (3 * M >= 4 * K)
     dx = pkg.linear_backward(dyt, xt, wt, dw, db)
     assert pkg.device_status() == 0
     dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, dw0, np.zeros(N, np.float32))
