@@ -171,9 +171,9 @@ struct __align__(128) RowSmem {
     float ring[kSlots][kSlot];
     uint64_t full[kSlots], empty[kSlots];
     float m[2][kWorkers / 32], s[2][kWorkers / 32];  // per warp, of this row and of the one before
-    int abort_flag;
+    int abort_flag, drain_flag;  // a wait has run out; so has the wait for copies on their way at the end
 };
-enum Site : int { SITE_EMPTY = 251, SITE_FULL };
+enum Site : int { SITE_EMPTY = 251, SITE_FULL, SITE_DRAIN };
 
 // The words of a row that start on 16-byte boundaries, and the up to three values either side of them.
 struct Row {
@@ -195,11 +195,21 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  "l"(src), "r"(bytes), "r"(tc05::smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
+// A barrier of the workers that tells each of them whether one has given up.  They leave together or not at all: the flag in
+// shared memory may change while they look at it, and those that stayed would wait at the next barrier for ever.
+__device__ __forceinline__ bool workers_any(bool gave_up) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"((uint32_t)gave_up), "n"(kWorkers)
+        : "memory");
+    return any != 0;
+}
 
 __device__ __forceinline__ void init_ring(RowSmem &sm) {
     if (threadIdx.x == 0) {
-        sm.abort_flag = 0;
+        sm.abort_flag = sm.drain_flag = 0;
         for (int i = 0; i < kSlots; i++) {
             tc05::mbar_init(&sm.full[i], 1);
             tc05::mbar_init(&sm.empty[i], kWorkers / 32);
@@ -216,18 +226,27 @@ struct Place {
         if (++slot == kSlots) slot = 0, round++;
     }
 };
-// One thread: the pieces of every row of this CTA.
-__device__ __forceinline__ void load_rows(RowSmem &sm, const float *x, int rows, int C, const tc05::WaitCtx &ctx) {
+// One thread: the pieces of every row of this CTA.  Returns the place behind the last one.
+__device__ __forceinline__ Place load_rows(RowSmem &sm, const float *x, int rows, int C, const tc05::WaitCtx &ctx) {
     Place at;
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const float *from = x + (size_t)r * C;
         const Row row(from, C);
         for (int c = 0; c < row.pieces(); c++, at.next()) {
-            if (at.round > 0 && !tc05::mbar_wait(&sm.empty[at.slot], (at.round - 1) & 1, ctx, SITE_EMPTY)) return;
+            if (at.round > 0 && !tc05::mbar_wait(&sm.empty[at.slot], (at.round - 1) & 1, ctx, SITE_EMPTY)) return at;
             const uint32_t bytes = min(kSlot, row.words * 4 - c * kSlot) * 4;
             tc05::mbar_expect_tx(&sm.full[at.slot], bytes);
             bulk_load(sm.ring[at.slot], from + row.head + c * kSlot, bytes, &sm.full[at.slot]);
         }
+    }
+    return at;
+}
+// The same thread, last: nothing is on its way into shared memory that the CTA gives back, also where the workers have left.
+__device__ __forceinline__ void drain(RowSmem &sm, const Place &end, const tc05::WaitCtx &ctx) {
+    const tc05::WaitCtx last{&sm.drain_flag, ctx.status, ctx.limit_ns};
+    for (int i = 0; i < kSlots; i++) {
+        const uint32_t pieces = end.round + (i < end.slot);  // that this place has been given
+        if (pieces > 0) tc05::mbar_wait(&sm.full[i], (pieces - 1) & 1, last, SITE_DRAIN);
     }
 }
 // After a warp's last look at a piece: the copy engine may overwrite it.
@@ -239,16 +258,16 @@ __device__ __forceinline__ void release(RowSmem &sm, int c) {
 
 __global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const float *__restrict__ logits, const float *__restrict__ targets,
                                                                          float *__restrict__ logsm, float *__restrict__ loss, int rows,
-                                                                         int C, int *status) {
+                                                                         int C, int loaded, uint64_t limit_ns, int *status) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     RowSmem &sm = *reinterpret_cast<RowSmem *>(smem_raw);
     tc05::pdl_launch_dependents();
     init_ring(sm);
     tc05::pdl_wait();
-    tc05::WaitCtx ctx{&sm.abort_flag, status};
+    tc05::WaitCtx ctx{&sm.abort_flag, status, limit_ns};
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid >= kWorkers) {
-        if (tid == kWorkers) load_rows(sm, logits, rows, C, ctx);
+        if (tid == kWorkers) drain(sm, load_rows(sm, logits, loaded, C, ctx), ctx);
         return;
     }
     Place first;
@@ -261,8 +280,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const
         // maximum so far and four sums of exponentials; what is below the maximum of nothing (all -inf) adds nothing
         float m = mine, s0 = loose >= 0 && mine != -INFINITY ? __expf(mine - m) : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
         Place at = first;
+        bool arrived = true;
         for (int c = 0; c < pieces; c++, at.next()) {
-            if (!tc05::mbar_wait_warp(&sm.full[at.slot], at.round & 1, ctx, SITE_FULL)) break;  // the others learn of it behind workers_sync
+            arrived = tc05::mbar_wait_warp(&sm.full[at.slot], at.round & 1, ctx, SITE_FULL);
+            if (!arrived) break;
             const int words = min(kSlot / 4, row.words - c * (kSlot / 4));
             const float4 *from = reinterpret_cast<const float4 *>(sm.ring[at.slot]);
             float4 v[kPerThread];
@@ -287,8 +308,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const
         const float wm = warp_max(m);
         s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));  // s is 0, or NaN, where there was nothing but -inf
         if (lane == 0) sm.m[n & 1][warp] = wm, sm.s[n & 1][warp] = s;
-        workers_sync();
-        if (*ctx.cta_abort) return;
+        if (workers_any(!arrived)) return;
         const float pm = lane < kWorkers / 32 ? sm.m[n & 1][lane] : -INFINITY, ps = lane < kWorkers / 32 ? sm.s[n & 1][lane] : 0.f;
         const float top = warp_max(pm);
         const float shift = top + logf(warp_sum(pm == -INFINITY ? ps : ps * __expf(pm - top)));
@@ -319,7 +339,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const
 // 32000: 367, 351, 50257: 628, 544; 1 row of 50257: 9.8, 9.9, 37 rows: 12.1, 10.5).
 bool row_fits(int C) { return C >= 30000 && C <= kSlot * kSlots; }
 
-int launch_rows(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, cudaStream_t s) {
+// `loaded` rows are fetched: all of them, or in the test of what happens when one never arrives fewer.
+int launch_rows(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, cudaStream_t s, int loaded,
+                uint64_t limit_ns = 0) {
     static bool ready[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -334,7 +356,7 @@ int launch_rows(const float *logits, const float *targets, float *logsm, float *
     if (rc != ATTN_OK) return rc;
     const int sms = attn::sm_count();
     return (int)attn::launch_after_previous(xent_forward_rows_kernel, dim3(rows < sms ? rows : sms), dim3(kRowThreads), sizeof(RowSmem), s,
-                                            logits, targets, logsm, loss, rows, C, status);
+                                            logits, targets, logsm, loss, rows, C, loaded, limit_ns, status);
 }
 
 }  // namespace
@@ -345,9 +367,16 @@ extern "C" {
 int xent_sm100_forward(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, void *stream) {
     if (!logits || !targets || !logsm || !loss) return ATTN_ERR_NULL;
     if (rows <= 0 || C <= 0) return ATTN_ERR_SHAPE;
-    if (xent::row_fits(C)) return xent::launch_rows(logits, targets, logsm, loss, rows, C, static_cast<cudaStream_t>(stream));
+    if (xent::row_fits(C)) return xent::launch_rows(logits, targets, logsm, loss, rows, C, static_cast<cudaStream_t>(stream), rows);
     return (int)attn::launch_after_previous(xent::xent_forward_kernel, dim3(rows), dim3(xent::kThreads), 0,
                                             static_cast<cudaStream_t>(stream), logits, targets, logsm, loss, rows, C);
+}
+
+int xent_sm100_selftest_wait_limit(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, int loaded,
+                                   unsigned limit_us, void *stream) {
+    if (!logits || !targets || !logsm || !loss) return ATTN_ERR_NULL;
+    if (rows <= 0 || !xent::row_fits(C) || loaded < 0 || loaded > rows || limit_us == 0 || limit_us > 100000u) return ATTN_ERR_SHAPE;
+    return xent::launch_rows(logits, targets, logsm, loss, rows, C, static_cast<cudaStream_t>(stream), loaded, limit_us * 1000ull);
 }
 
 int xent_sm100_backward(const float *g, const float *targets, const float *logsm, float *dout, int rows, int C, void *stream) {

@@ -27,6 +27,14 @@ extern "C" {
 int xent_sm100_forward(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, void *stream);
 
 /*
+ * What the forward does when rows never arrive, without a fault: the same kernel, for rows of 30000 to 53248 classes, fetches only
+ * the first `loaded` rows.  Its waits for the others run out after limit_us microseconds (at most 0.1 s), attn_sm100_device_status
+ * reports 1252, and the rows before them are complete.  (The reference has no counterpart.)
+ */
+int xent_sm100_selftest_wait_limit(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, int loaded,
+                                   unsigned limit_us, void *stream);
+
+/*
  * dout[r, target_r] = -g[r] / rows;  s = sum_j dout[r, j];  dout[r, j] -= exp(logsm[r, j]) * s.
  * Works on what dout holds (read-modify-write), like the reference, whose layer hands in zeros; g has one
  * value per row.
