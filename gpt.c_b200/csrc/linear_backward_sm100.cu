@@ -236,9 +236,11 @@ linear_backward_kernel(const __grid_constant__ Maps<kClasses> maps, float *__res
             tma_prefetch_desc(&maps.dy_k[0]);
             tma_prefetch_desc(&maps.w[0]);
         }
-        tma_prefetch_desc(&maps.dy_mn[0]);
-        tma_prefetch_desc(&maps.x[0][0]);
-        tma_prefetch_desc(&maps.dw);
+        if (dw != nullptr) {
+            tma_prefetch_desc(&maps.dy_mn[0]);
+            tma_prefetch_desc(&maps.x[0][0]);
+            tma_prefetch_desc(&maps.dw);
+        }
     }
     Items items(p, (int)blockIdx.x, (int)gridDim.x);  // the first item, before the wait for the previous kernel
     Item t;
@@ -586,7 +588,7 @@ int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, c
                     int M, int N, int np, int K, int *status, cudaStream_t s) {
     Problem p = make_problem(plan, M, N, K);
     p.wide = (reinterpret_cast<uintptr_t>(dx) & 31u) == 0;
-    Maps<false> maps;
+    Maps<false> maps = {};
     int rc;
     if ((rc = map_mn_major_blocks(&maps.dy_mn[0], dy, M, np, 4)) != 0) return rc;
     if ((rc = map_out_f32(&maps.dw, dw, N, K)) != 0) return rc;
@@ -602,17 +604,19 @@ int launch_backward_by_row_class(const BackwardPlan &plan, const float *dy, cons
                                  int M, int N, int K, int *status, cudaStream_t s) {
     Problem p = make_problem(plan, M, N, K);
     p.wide = (reinterpret_cast<uintptr_t>(dx) & 31u) == 0;
-    Maps<true> maps;
+    Maps<true> maps = {};  // those of products that are not wanted stay empty: x may be NULL without dw
     int rc;
     if (dw && (rc = map_out_f32(&maps.dw, dw, N, K)) != 0) return rc;
     for (int j = 0; j < 4; j++) {
         const RowClass c = row_class(dy, M, N, j);
         const size_t pitch = 4 * (size_t)N;
         p.shift[j] = c.shift, p.whole[j] = (N + c.shift) / 32 * 32;
-        if (p.whole[j] > 0 && (rc = map_mn_major_blocks(&maps.dy_whole[j], c.dy, c.rows, p.whole[j], 4, pitch)) != 0) return rc;
-        if ((rc = map_mn_major(&maps.dy_mn[j], c.dy, c.rows, N + c.shift, pitch)) != 0) return rc;
-        for (int i = 0; i <= (p.wider > 0); i++)
-            if ((rc = map_mn_major_blocks(&maps.x[j][i], x + (size_t)j * K, c.rows, K, p.cols + i, 4 * (size_t)K)) != 0) return rc;
+        if (dw) {
+            if (p.whole[j] > 0 && (rc = map_mn_major_blocks(&maps.dy_whole[j], c.dy, c.rows, p.whole[j], 4, pitch)) != 0) return rc;
+            if ((rc = map_mn_major(&maps.dy_mn[j], c.dy, c.rows, N + c.shift, pitch)) != 0) return rc;
+            for (int i = 0; i <= (p.wider > 0); i++)
+                if ((rc = map_mn_major_blocks(&maps.x[j][i], x + (size_t)j * K, c.rows, K, p.cols + i, 4 * (size_t)K)) != 0) return rc;
+        }
         if (!dx) continue;
         if ((rc = map_k_major(&maps.dy_k[j], c.dy, c.rows, N + c.shift, 128, pitch)) != 0) return rc;
         if (p.dx_pieces > 1 && (rc = map_out_f32(&maps.dx[j], dx + (size_t)j * K, c.rows, K, 4 * (size_t)K)) != 0) return rc;

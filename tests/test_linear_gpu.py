@@ -303,6 +303,33 @@ def test_linear_backward_from_every_fourth_row_of_fewer(pkg, M, N, K):
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
 
 
+@pytest.mark.parametrize("M,N,K", [(4096, 8195, 64), (1000, 33555, 64), (5001, 16386, 160)])
+def test_linear_backward_from_every_fourth_row_in_part(pkg, M, N, K):
+    """dx without dW, which needs no x; dW that lies over w, so that the products follow each other."""
+    L = pkg.lib()
+    x, w, _, dy = inputs(M, N, K, 79)
+    xt, wt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, dy))
+    st = torch.cuda.current_stream().cuda_stream
+    need = L.linear_sm100_backward_scratch_bytes(M, N, K)
+    scratch = torch.empty(max(need, 1), dtype=torch.uint8, device="cuda")
+    sp = scratch.data_ptr() if need else None
+    dx = torch.full((M + 2, K), 3.0, device="cuda")
+    db = torch.zeros(N, device="cuda")
+    assert L.linear_sm100_backward(dyt.data_ptr(), None, wt.data_ptr(), dx[1:].data_ptr(), None, db.data_ptr(), sp, M, N, K, st) == 0
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, w, np.zeros(N, np.float32))
+    within(dx[1:-1].cpu().numpy(), dx_ref, dy, w)
+    assert bool((dx[0] == 3.0).all()) and bool((dx[-1] == 3.0).all())
+    assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+    dx.fill_(3.0), db.zero_()
+    assert L.linear_sm100_backward(dyt.data_ptr(), xt.data_ptr(), wt.data_ptr(), dx[1:].data_ptr(), wt.data_ptr(), db.data_ptr(), sp,
+                                   M, N, K, st) == 0
+    assert pkg.device_status() == 0
+    within(dx[1:-1].cpu().numpy(), dx_ref, dy, w)
+    within(wt.cpu().numpy(), dw_ref, dy.T, x)
+    assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+
+
 @pytest.mark.parametrize("M,N,K", [(1411, 4800, 1600), (2305, 2312, 1568), (8001, 760, 3072)])
 def test_linear_tiles_of_256_rows(pkg, M, N, K):
     """Forward with bias and planes and dx alone, where tiles of 256 rows by 256 or 192 columns are taken: the last ones with
