@@ -23,6 +23,9 @@ struct DeviceState {
     int num_sms = 0;        // the persistent backward kernel runs one CTA per SM
 };
 DeviceState g_dev[kMaxDevices];
+// The status word of each device that loads this: part of the module, because the first call may be one that a stream captures,
+// where neither an allocation nor a memset is allowed.
+__device__ int g_status_word;
 std::mutex g_init_lock;  // per-device set-up may be entered by several host threads at once
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -178,10 +181,9 @@ int attn_sm100_init(void) {
     int sms = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
     g_dev[dev].num_sms = sms;
-    int *st = nullptr;
-    if ((e = cudaMalloc(&st, sizeof(int))) != cudaSuccess) return (int)e;
-    if ((e = cudaMemset(st, 0, sizeof(int))) != cudaSuccess) return (int)e;
-    g_dev[dev].status = st;
+    void *st = nullptr;
+    if ((e = cudaGetSymbolAddress(&st, g_status_word)) != cudaSuccess) return (int)e;
+    g_dev[dev].status = static_cast<int *>(st);
     g_dev[dev].ready.store(true, std::memory_order_release);
     return ATTN_OK;
 }

@@ -89,9 +89,10 @@ int attn_sm100_version(void);
 
 /*
  * Prepares the current device: checks that it is compute capability 10.x, resolves the driver's
- * tensor-map encoder, raises the dynamic shared-memory limit of the kernels and allocates the
- * 4-byte device status word.  Idempotent; forward/backward call it on first use of a device, but
- * that first call allocates, so call it yourself before timing or capturing anything.
+ * tensor-map encoder, raises the dynamic shared-memory limit of the kernels and looks up the
+ * 4-byte device status word.  Idempotent; forward/backward call it on first use of a device, also under
+ * stream capture (nothing is allocated), but that first call takes longer, so call it yourself before
+ * timing anything.
  */
 int attn_sm100_init(void);
 
