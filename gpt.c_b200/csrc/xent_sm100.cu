@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kThreads) xent_forward_kernel(const float *__r
     }
     // combine (m, s) pairs across the warp, then across the block
     const float wm = warp_max(m);
-    s = warp_sum(m == -INFINITY ? 0.f : s * __expf(m - wm));
+    s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));  // s is 0, or NaN, where there was nothing but -inf
     if ((threadIdx.x & 31) == 0) {
         s_m[threadIdx.x >> 5] = wm;
         s_s[threadIdx.x >> 5] = s;
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kThreads) xent_forward_kernel(const float *__r
         const float pm = threadIdx.x < kThreads / 32 ? s_m[threadIdx.x] : -INFINITY;
         const float ps = threadIdx.x < kThreads / 32 ? s_s[threadIdx.x] : 0.f;
         const float bm = warp_max(pm);
-        const float bs = warp_sum(pm == -INFINITY ? 0.f : ps * __expf(pm - bm));
+        const float bs = warp_sum(pm == -INFINITY ? ps : ps * __expf(pm - bm));
         if (threadIdx.x == 0) s_shift = bm + logf(bs);
     }
     __syncthreads();
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const
         }
         float s = (s0 + s1) + (s2 + s3);
         const float wm = warp_max(m);
-        s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));  // s is 0, or NaN, where there was nothing but -inf
+        s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));  // as in the kernel above
         if (lane == 0) sm.m[n & 1][warp] = wm, sm.s[n & 1][warp] = s;
         if (workers_any(!arrived)) return;
         const float pm = lane < kWorkers / 32 ? sm.m[n & 1][lane] : -INFINITY, ps = lane < kWorkers / 32 ? sm.s[n & 1][lane] : 0.f;

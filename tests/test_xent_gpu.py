@@ -141,6 +141,23 @@ def test_cross_entropy_keeps_rows_apart(pkg):
     assert np.abs(got[rest] - ref).max() <= 2e-6 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("rows,C", [(7, 9), (5, 1000), (5, 1024), (5, 12000), (3, 29999), (4, 50257)])
+def test_cross_entropy_passes_nan_on(pkg, rows, C):
+    """One NaN makes its row and the loss NaN, also where a thread sees no other value, or only -inf beside it."""
+    L = pkg.lib()
+    logits = np.random.default_rng(C).standard_normal((rows, C)).astype(np.float32)
+    for row, col in enumerate((0, C - 1, C // 2)[:rows - 1]):
+        logits[row, col] = np.nan
+    logits[1, : C - 2] = -np.inf
+    lt, tt = torch.from_numpy(logits).cuda(), torch.full((rows,), C - 2.0, device="cuda")
+    logsm, loss = torch.empty_like(lt), torch.zeros(1, device="cuda")
+    assert L.xent_sm100_forward(lt.data_ptr(), tt.data_ptr(), logsm.data_ptr(), loss.data_ptr(), rows, C, stream()) == 0
+    got = logsm.cpu().numpy()
+    bad = np.isnan(logits).any(1)
+    assert np.isnan(got[bad]).all() and np.isfinite(got[~bad]).all() and np.isnan(loss.item())
+    assert pkg.device_status() == 0
+
+
 def test_cross_entropy_argument_errors(pkg):
     L = pkg.lib()
     assert L.xent_sm100_forward(None, None, None, None, 1, 1, None) == -1
