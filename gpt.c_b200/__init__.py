@@ -42,6 +42,7 @@ SIGNATURES = {
     "linear_sm100_forward": (_c.c_int, [_c.c_void_p] * 5 + [_c.c_int] * 3 + [_c.c_void_p]),
     "linear_sm100_backward_scratch_bytes": (_c.c_size_t, [_c.c_int] * 3),
     "linear_sm100_backward": (_c.c_int, [_c.c_void_p] * 7 + [_c.c_int] * 3 + [_c.c_void_p]),
+    "linear_sm100_backward_plan": (_c.c_int, [_c.c_int] * 6 + [_c.POINTER(_c.c_int)]),
     "layernorm_sm100_forward": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_float] + [_c.c_void_p] * 3 + [_c.c_int] * 2 + [_c.c_void_p]),
     "layernorm_sm100_backward": (_c.c_int, [_c.c_void_p] * 8 + [_c.c_int] * 2 + [_c.c_void_p]),
     "tensor_sm100_fill": (_c.c_int, [_c.c_void_p, _c.c_size_t, _c.c_float, _c.c_void_p]),

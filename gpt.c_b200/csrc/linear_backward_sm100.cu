@@ -568,6 +568,24 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
     return best;
 }
 
+DwLoad dw_load(const BackwardPlan &plan, int M, int N, int K) {
+    DwLoad most = {};
+    const int ctas = plan.teams * plan.team;
+    if (ctas == 0) return most;
+    const Problem p = make_problem(plan, M, N, K);
+    for (int cta = 0; cta < ctas; cta++) {
+        Items items(p, cta, ctas);
+        int blocks = 0;
+        for (Item t; items.next(p, t);) {
+            if (!t.dw) continue;
+            blocks += t.kb1 - t.kb0;
+            if (t.kb1 - t.kb0 > most.sum) most.sum = t.kb1 - t.kb0;
+        }
+        if (blocks > most.cta) most.cta = blocks;
+    }
+    return most;
+}
+
 template <bool kClasses>
 static int launch(const Maps<kClasses> &maps, float *dx, float *dw, float *db, const Problem &p, int ctas, int *status, cudaStream_t s) {
     static bool attr_done[64] = {};

@@ -579,20 +579,23 @@ bool by_row_class(int M, int N, int K) {
 // Whether a caller has to bring room for the copy: wherever it may be made.
 bool wants_scratch(int M, int N) { return N % 32 != 0 && (N % 4 == 0 || M < 4096 || (long long)M * N < (32 << 20)); }
 
-// dx, dW and db (dx or dw may be NULL) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut into
-// pieces that add into zeros: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from
+// dx, dW and db (not all of them need be wanted) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut
+// into pieces that add into zeros: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from
 // sums of 524 blocks of 32, 1.3e-5 from sums of 171).  Without dW, whose ranges make up for it, their number decides how even
 // the last round of tiles is (8192 x 50257 x 768: 1009 us from 3 pieces, 1111 from 4).
-int gradients_by_row_class(const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, int M, int N, int K, int sms,
-                           int *status, cudaStream_t s) {
+BackwardPlan plan_by_row_class(int M, int N, int K, bool want_dx, bool want_dw, int sms) {
     const int kb = (N + 3 + kBK - 1) / kBK;
     const int least = (kb + 523) / 524, by_tiles = plan_pieces((M + 3) / 4, K, kb, sms, 32).splits;
     const int pieces = least > by_tiles ? least : by_tiles;
-    BackwardPlan plan = plan_backward(M, N, K, dx != nullptr, dw != nullptr, sms, 4, pieces);
-    for (int more = 1; dx && !dw && more <= 2; more++) {
+    BackwardPlan plan = plan_backward(M, N, K, want_dx, want_dw, sms, 4, pieces);
+    for (int more = 1; want_dx && !want_dw && more <= 2; more++) {
         const BackwardPlan other = plan_backward(M, N, K, true, false, sms, 4, pieces + more);
         if (other.ns < plan.ns) plan = other;
     }
+    return plan;
+}
+int gradients_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, int M,
+                           int N, int K, int *status, cudaStream_t s) {
     if (dx && plan.dx_pieces > 1) {
         const int rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s);
         if (rc != 0) return rc;
@@ -639,6 +642,32 @@ int input_gradient(const InputGradient &how, const float *g, const float *w, flo
     if ((rc = map_out_f32(&maps.c, dx, M, K)) != 0) return rc;
     if ((rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s)) != 0) return rc;
     return launch<true, 1>(maps, nullptr, dx, nullptr, p, status, s);
+}
+
+// How the backward makes dx and dW; np: columns of a padded dy.  `in_parts`: one product after the other.
+struct Gradients {
+    bool classes, together;  // views of dy; dx and dW in one launch
+    InputGradient alone;     // dx in a launch of its own, not from views
+    BackwardPlan dx, dw;     // dx in a launch of its own, from views; the launch that makes dW, and dx if together
+};
+Gradients plan_gradients(int M, int N, int K, int np, bool want_dx, bool want_dw, bool in_parts, int sms) {
+    Gradients g = {};
+    g.classes = by_row_class(M, N, K);
+    if (g.classes) {
+        g.together = want_dx && want_dw && !in_parts;
+        if (want_dx && !g.together) g.dx = plan_by_row_class(M, N, K, true, false, sms);
+        if (want_dw) g.dw = plan_by_row_class(M, N, K, g.together, true, sms);
+        return g;
+    }
+    if (want_dx) g.alone = plan_input_gradient(M, np, K, sms);
+    if (!want_dw) return g;
+    g.dw = plan_backward(M, N, K, false, true, sms);
+    // dx has the same bits with and without dW: one launch only where dx alone would be whole tiles too
+    if (!want_dx || in_parts || g.alone.split || g.alone.tiles.splits > 1) return g;
+    const BackwardPlan both = plan_backward(M, N, K, true, true, sms);
+    g.together = both.ns < g.alone.ns + g.dw.ns;
+    if (g.together) g.dw = both;
+    return g;
 }
 
 // Whether a result lies over something that another product of the same call reads or writes: then the products have to
@@ -717,34 +746,25 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     if (rc != ATTN_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int sms = attn::sm_count();
-    const float *g = dy;  // without row classes [M, np] from here on
     const bool in_parts = dw && overlapping(dy, x, w, dx, dw, db, M, N, K);
-    if (classes) {
-        if (dx && (!dw || in_parts)) rc = gradients_by_row_class(dy, x, w, dx, nullptr, nullptr, M, N, K, sms, status, s);
-        if (rc == 0 && dw)
-            rc = gradients_by_row_class(dy, x, w, in_parts ? nullptr : dx, dw, in_parts ? nullptr : db, M, N, K, sms, status, s);
-        if (rc != 0 || (dw && !in_parts)) return rc;
-    } else if (padded) {
+    const Gradients how = plan_gradients(M, N, K, np, dx != nullptr, dw != nullptr, in_parts, sms);
+    float *dx_too = how.together ? dx : nullptr, *db_too = in_parts ? nullptr : db;
+    const float *g = dy;  // without row classes [M, np] from here on
+    if (padded) {
         rc = (int)attn::launch_after_previous(pad_rows_kernel, dim3(sms * 16), dim3(256), 0, s, static_cast<float *>(scratch), dy, M,
                                               N, np);
         if (rc != 0) return rc;
         g = static_cast<const float *>(scratch);
     }
-    if (!classes) {
-        InputGradient alone{};
-        if (dx) alone = plan_input_gradient(M, np, K, sms);
-        BackwardPlan rest{}, both{};
-        if (dw) rest = plan_backward(M, N, K, false, true, sms);
-        // dx has the same bits with and without dW: one launch only where dx alone would be whole tiles too
-        if (dw && dx && !in_parts && !alone.split && alone.tiles.splits == 1) both = plan_backward(M, N, K, true, true, sms);
-        const bool together = both.ns > 0 && both.ns < alone.ns + rest.ns;
-        if (dx && !together && (rc = input_gradient(alone, g, w, dx, M, N, np, K, sms, status, s)) != 0) return rc;
-        if (dw) {
-            rc = launch_backward(together ? both : rest, g, x, w, N, together ? dx : nullptr, dw, in_parts ? nullptr : db, M, N, np, K,
-                                 status, s);
-            if (rc != 0) return rc;
-            if (!in_parts) return ATTN_OK;
-        }
+    if (dx && !how.together) {
+        rc = classes ? gradients_by_row_class(how.dx, dy, x, w, dx, nullptr, nullptr, M, N, K, status, s)
+                     : input_gradient(how.alone, g, w, dx, M, N, np, K, sms, status, s);
+        if (rc != 0) return rc;
+    }
+    if (dw) {
+        rc = classes ? gradients_by_row_class(how.dw, dy, x, w, dx_too, dw, db_too, M, N, K, status, s)
+                     : launch_backward(how.dw, g, x, w, N, dx_too, dw, db_too, M, N, np, K, status, s);
+        if (rc != 0 || !in_parts) return rc;
     }
     if (db) {
         // eight blocks per SM, so that enough loads are on their way (six columns of 32 blocks took 9.2 us at
@@ -755,6 +775,21 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
                                               db, M, N, classes ? N : np);
     }
     return rc;
+}
+
+int linear_sm100_backward_plan(int M, int N, int K, int want_dx, int want_dw, int sms, int *plan) {
+    using namespace lin;
+    if (!plan) return ATTN_ERR_NULL;
+    if (M <= 0 || N <= 0 || K <= 0 || sms <= 0 || (!want_dx && !want_dw) || (long long)M * N > 0x7fffffffLL || (long long)M * K > 0x7fffffffLL)
+        return ATTN_ERR_SHAPE;
+    if (K % 32 != 0) return ATTN_ERR_UNSUPPORTED;
+    const Gradients how = plan_gradients(M, N, K, (N + 31) / 32 * 32, want_dx, want_dw, false, sms);
+    const BackwardPlan &one = want_dw ? how.dw : how.dx;  // nothing in it for dx alone, not from views
+    const int pieces = !want_dx ? 0 : how.classes ? one.dx_pieces : how.alone.split ? 1 : how.alone.tiles.splits;
+    const DwLoad load = dw_load(one, M, N, K);
+    const int out[9] = {how.together, how.classes ? 4 : 1, one.teams * one.team, one.team, one.down, pieces, pieces <= 2, load.cta, load.sum};
+    for (int i = 0; i < 9; i++) plan[i] = out[i];
+    return ATTN_OK;
 }
 
 }  // extern "C"

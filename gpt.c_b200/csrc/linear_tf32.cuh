@@ -128,6 +128,11 @@ struct BackwardPlan {
     int ns;
 };
 BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes = 1, int dx_pieces = 1);
+// Contraction blocks of dW: the most that one CTA takes, and the most that one accumulator sums up.
+struct DwLoad {
+    int cta, sum;
+};
+DwLoad dw_load(const BackwardPlan &plan, int M, int N, int K);
 // dy [M, np] with zeros from column N on, w [w_rows, K].
 int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
                     int M, int N, int np, int K, int *status, cudaStream_t s);

@@ -63,6 +63,16 @@ size_t linear_sm100_backward_scratch_bytes(int M, int N, int K);
 int linear_sm100_backward(const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, void *scratch,
                           int M, int N, int K, void *stream);
 
+/*
+ * How linear_sm100_backward cuts its work on a GPU of `sms` SMs, for tests and to read timings by.  Host arithmetic only.  plan[0..8]:
+ *   0  1: dx and dW in one launch                       5  pieces of the contraction of dx (0 without dx)
+ *   1  4: from views of every fourth row of dy, else 1  6  1: their sum has a fixed order, the same bits in every call
+ *   2  CTAs of the launch that makes dW                 7  most contraction blocks (32 rows) of dW that one CTA takes
+ *   3  CTAs that work on neighbouring tiles of dW       8  most of them in one accumulator
+ *   4  1: these tiles are below each other, 0: beside
+ */
+int linear_sm100_backward_plan(int M, int N, int K, int want_dx, int want_dw, int sms, int *plan);
+
 #ifdef __cplusplus
 }
 #endif

@@ -14,6 +14,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 from oracle import ops_oracle as ops  # noqa: E402
+from test_linear_plan import SMS, TEAMS, plan  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -285,6 +286,16 @@ def test_linear_backward_in_one_launch(pkg, M, N, K, with_db):
     err = np.abs(db[at:at + N].cpu().numpy() - (db_ref if with_db else db0))
     assert (err <= 2.0 ** -20 * (np.abs(dy).sum(0) + np.abs(db0))).all()
     assert bool((db[:at] == 0.5).all()) and bool((db[at + N:] == 0.5).all())
+
+
+@pytest.mark.parametrize("M,N,K,team,down", TEAMS)
+@pytest.mark.parametrize("with_db", [True, False])
+def test_linear_backward_in_one_launch_by_teams(pkg, M, N, K, team, down, with_db):
+    """The same at sizes of which tests/test_linear_plan.py says that they run that way, by teams of every kind."""
+    assert torch.cuda.get_device_properties(0).multi_processor_count == SMS
+    p = plan(pkg, M, N, K)
+    assert (p["together"], p["views"], p["team"], p["down"]) == (1, 1, team, down)
+    test_linear_backward_in_one_launch(pkg, M, N, K, with_db)
 
 
 @pytest.mark.parametrize("M,N,K", [(1000, 33555, 64), (1025, 32801, 96), (3001, 16387, 320), (2050, 16386, 1536)])

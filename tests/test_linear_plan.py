@@ -1,0 +1,42 @@
+"""How the Linear backward cuts its work, as linear_sm100_backward_plan (include/linear_sm100.h) says it does: host arithmetic."""
+import ctypes
+
+import pytest
+
+SMS = 148
+
+
+def plan(pkg, M, N, K, want_dx=1, want_dw=1, sms=SMS):
+    out = (ctypes.c_int * 9)()
+    assert pkg.lib().linear_sm100_backward_plan(M, N, K, want_dx, want_dw, sms, out) == 0
+    names = ("together", "views", "ctas", "team", "down", "dx_pieces", "dx_fixed_order", "dw_of_a_cta", "dw_sum")
+    return dict(zip(names, out))
+
+
+# shapes that dx, dW and db share one launch at, and its teams: (M, N, K, CTAs of a team, below each other)
+TEAMS = [
+    (8001, 760, 3072, 6, 1), (6867, 243, 2208, 2, 1),  # a padded copy of dy; its last tile has one row in use
+    (5420, 3326, 160, 2, 0), (4500, 3072, 768, 3, 0),
+    (173, 1365, 5216, 1, 0),                           # tiles of dW only 6 blocks deep
+    (7146, 8, 288, 1, 0), (8776, 344, 32, 1, 0),       # one tile row, one block of columns
+    (1025, 129, 4288, 1, 0),
+]
+
+
+@pytest.mark.parametrize("M,N,K,team,down", TEAMS)
+def test_one_launch(pkg, M, N, K, team, down):
+    p = plan(pkg, M, N, K)
+    assert (p["together"], p["views"], p["team"], p["down"]) == (1, 1, team, down)
+
+
+@pytest.mark.parametrize("M,N,K,views", [(8192, 50257, 768, 4), (1024, 50257, 768, 4), (37, 50257, 768, 1), (8192, 50304, 768, 1)])
+def test_views(pkg, M, N, K, views):
+    assert plan(pkg, M, N, K)["views"] == views
+
+
+def test_plan_arguments(pkg):
+    L, out = pkg.lib(), (ctypes.c_int * 9)()
+    assert L.linear_sm100_backward_plan(8, 8, 32, 1, 1, SMS, None) == -1
+    for bad in ((0, 8, 32, 1, 1, SMS), (8, 8, 32, 0, 0, SMS), (8, 8, 32, 1, 1, 0), (65536, 65536, 32, 1, 1, SMS)):
+        assert L.linear_sm100_backward_plan(*bad, out) == -2
+    assert L.linear_sm100_backward_plan(8, 8, 40, 1, 1, SMS, out) == -3
