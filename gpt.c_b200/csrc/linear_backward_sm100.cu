@@ -88,7 +88,8 @@ struct Problem {
     int tiles_n, cols, wider;  // column tiles; blocks of 32 columns in each; the first `wider` have one more
     int dx_tiles, dx_kb;       // tiles of dx, handed out round robin; contraction blocks of one
     int classes;               // 4: views of every fourth row of dy
-    int dx_pieces, piece_tiles, piece_kb;  // dx from so many pieces of the contraction; tiles and contraction blocks of a piece
+    int dx_pieces, piece_tiles, piece_kb;  // dx from so many pieces of the contraction, added up in memory; tiles and contraction blocks of a piece
+    int dx_sums;               // or from so many in turn, added up by the CTA whose tile it is
     int whole[4], shift[4];    // columns of the views in whole blocks; before the first column of dy
     int dw_kb;                 // contraction blocks of a tile of dW
     int team, down;            // CTAs of a team; their tiles are below (1) or beside each other (0)
@@ -112,7 +113,7 @@ __host__ __device__ __forceinline__ int range_start(const Problem &p, int c) {
     return in < p.snap ? u - in : p.dw_kb - in < p.snap ? u + p.dw_kb - in : u;
 }
 
-// A tile of dx, or a tile of dW with a range of its contraction.
+// A tile of dx or of dW with a range of its contraction: what goes through one accumulator.
 struct Item {
     bool dw;
     int cls, m0, tn, n0, cols, kb0, kb1;
@@ -122,39 +123,51 @@ struct Items {
     int i, whole;  // tiles of dx and whole tiles of dW taken so far
     int at, end;   // the team's range
     int team, member;
-    __host__ __device__ __forceinline__ Items(const Problem &p, int cta, int ctas) : cta(cta), ctas(ctas), i(0), whole(0) {
+    int from, to, sums;  // what is left of the tile's range, and the accumulators it goes through
+    __host__ __device__ __forceinline__ Items(const Problem &p, int cta, int ctas) : cta(cta), ctas(ctas), i(0), whole(0), sums(0) {
         team = cta / p.team;
         member = cta - team * p.team;
         at = range_start(p, team), end = range_start(p, team + 1);
     }
+    // `t` is the item before, which the next one may continue.
     __host__ __device__ __forceinline__ bool next(const Problem &p, Item &t) {
+        if (sums == 0 && !next_tile(p, t)) return false;
+        t.kb0 = from;
+        from = sums == 1 ? to : from + (to - from + sums - 1) / sums;
+        t.kb1 = from;
+        sums--;
+        return true;
+    }
+    __host__ __device__ __forceinline__ bool next_tile(const Problem &p, Item &t) {
         int w = cta + i * ctas;
         int tm;
+        sums = 1;
         if (p.uncut) {
             if (w >= p.strips) return false;
             t.dw = true;
             tm = w / p.tiles_n, t.tn = w - tm * p.tiles_n;
-            t.kb0 = 0, t.kb1 = p.dw_kb;
+            from = 0, to = p.dw_kb;
             i++;
         } else if (w < p.dx_tiles) {
             t.dw = false;
             const int piece = p.dx_pieces > 1 ? w / p.piece_tiles : 0;
             w -= piece * p.piece_tiles;
             tm = w / p.tiles_n, t.tn = w - tm * p.tiles_n;
-            t.kb0 = piece * p.piece_kb, t.kb1 = p.dx_kb - t.kb0 < p.piece_kb ? p.dx_kb : t.kb0 + p.piece_kb;
+            from = piece * p.piece_kb, to = p.dx_kb - from < p.piece_kb ? p.dx_kb : from + p.piece_kb;
+            sums = p.dx_sums;
             i++;
         } else {
             t.dw = true;
             int strip;
             if (whole < p.rounds) {
                 strip = team + whole++ * p.teams;
-                t.kb0 = 0, t.kb1 = p.dw_kb;
+                from = 0, to = p.dw_kb;
             } else {
                 if (at >= end) return false;
                 strip = at / p.dw_kb;
-                t.kb0 = at - strip * p.dw_kb;
-                const int take = p.dw_kb - t.kb0 < end - at ? p.dw_kb - t.kb0 : end - at;
-                t.kb1 = t.kb0 + take;
+                from = at - strip * p.dw_kb;
+                const int take = p.dw_kb - from < end - at ? p.dw_kb - from : end - at;
+                to = from + take;
                 at += take;
                 strip += p.rounds * p.teams;
             }
@@ -199,6 +212,21 @@ __device__ __forceinline__ void clear_leading(uint8_t *tile, int columns, int la
     }
     fence_proxy_async_smem();
     __syncwarp();
+}
+
+// r += what is at src, 4 * kQuads floats as far as `left` go (a multiple of 4).
+template <int kQuads>
+__device__ __forceinline__ void add_words(const float *src, int left, uint32_t *r) {
+#pragma unroll
+    for (int q = 0; q < kQuads; q++) {
+        if (4 * q >= left) continue;
+        float4 v;
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(src + 4 * q) : "memory");
+        r[4 * q] = __float_as_uint(v.x + __uint_as_float(r[4 * q]));
+        r[4 * q + 1] = __float_as_uint(v.y + __uint_as_float(r[4 * q + 1]));
+        r[4 * q + 2] = __float_as_uint(v.z + __uint_as_float(r[4 * q + 2]));
+        r[4 * q + 3] = __float_as_uint(v.w + __uint_as_float(r[4 * q + 3]));
+    }
 }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) {
@@ -417,8 +445,10 @@ linear_backward_kernel(const __grid_constant__ Maps<kClasses> maps, float *__res
 #pragma unroll
                     for (int o = 0; o < 2; o++) {
                         const int row = row0 + lane - odd + o;
-                        if (row * p.classes + t.cls < p.M)
-                            store_words<4>(dx + ((size_t)row * p.classes + t.cls) * p.K + col, p.K - col, p.wide, r + 16 * o);
+                        if (row * p.classes + t.cls >= p.M) continue;
+                        float *to = dx + ((size_t)row * p.classes + t.cls) * p.K + col;
+                        if (kClasses && t.kb0 > 0) add_words<4>(to, p.K - col, r + 16 * o);  // what this thread wrote for the range before
+                        store_words<4>(to, p.K - col, p.wide, r + 16 * o);
                     }
                     continue;
                 }
@@ -482,8 +512,9 @@ double adding_ns(double pieces, int cols) { return pieces * cols * 16384 * 150e-
 Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
     Problem p = {};
     p.M = M, p.N = N, p.K = K;
-    p.classes = plan.classes, p.dx_pieces = plan.dx_pieces;
-    p.piece_tiles = plan.dx_tiles / plan.dx_pieces, p.piece_kb = (plan.dx_kb + plan.dx_pieces - 1) / plan.dx_pieces;
+    p.classes = plan.classes;
+    p.dx_pieces = plan.dx_in_turn ? 1 : plan.dx_pieces, p.dx_sums = plan.dx_in_turn ? plan.dx_pieces : 1;
+    p.piece_tiles = plan.dx_tiles / p.dx_pieces, p.piece_kb = (plan.dx_kb + p.dx_pieces - 1) / p.dx_pieces;
     p.tiles_n = plan.tiles_n, p.cols = K / 32 / plan.tiles_n, p.wider = K / 32 % plan.tiles_n;
     p.dx_tiles = plan.dx_tiles, p.dx_kb = plan.dx_kb, p.dw_kb = plan.dw_kb;
     p.team = plan.team, p.down = plan.down, p.rounds = plan.rounds, p.strips = plan.strips, p.teams = plan.teams, p.fewer = plan.fewer;
@@ -502,7 +533,7 @@ Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
 }  // namespace
 
 // The split of the work and the time in nanoseconds it is expected to take: see linear_tf32.cuh.
-BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes, int dx_pieces) {
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes, int dx_pieces, bool in_turn) {
     BackwardPlan best = {};
     const int blocks = K / 32;
     for (int width = 8; width >= 4; width--) {
@@ -519,7 +550,8 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
         c.classes = classes;
         const int piece_kb = (c.dx_kb + dx_pieces - 1) / dx_pieces;
         c.dx_pieces = (c.dx_kb + piece_kb - 1) / piece_kb;
-        c.dx_tiles = want_dx ? classes * rows_m * tiles_n * c.dx_pieces : 0;
+        c.dx_in_turn = in_turn;
+        c.dx_tiles = want_dx ? classes * rows_m * tiles_n * (in_turn ? 1 : c.dx_pieces) : 0;
         const int dw_tiles = want_dw ? classes * rows_n * tiles_n : 0;
         // Where dy and x don't stay in L2 together, a team shares the larger of them, if that keeps most SMs busy.
         c.down = classes == 1 && N < K, c.team = c.down ? rows_n : tiles_n;
@@ -528,7 +560,7 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
         c.teams = sms / c.team;
         if (!want_dx && (long long)c.strips * c.dw_kb < c.teams) c.teams = c.strips * c.dw_kb;
         const int ctas = c.teams * c.team;
-        const double dx_ns = piece_kb * tb + te;
+        const double dx_ns = (piece_kb * tb + te) * (in_turn ? c.dx_pieces : 1);
         // every CTA has about one piece of a tile more than its share of whole ones
         const double even = (c.dx_tiles * dx_ns + dw_tiles * (c.dw_kb * tb + te)) / ctas + te;
         const int most = (c.dx_tiles + ctas - 1) / ctas;

@@ -564,44 +564,8 @@ int stream_rows_of_c(int M, int N, int K) {
 
 bool aligned16(const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
-// Whether the gradients of a [M, N] result come from views of every fourth row of dy, whose rows are not 16-byte aligned,
-// and not from a copy with padded rows.  The copy is cheap as long as it stays in L2 (128 MB); the views add each tile of dW to
-// memory four times, which costs more than the copy where K is large beside M.  dx and dW, copy -> views, in us (N, K; M):
-//     50257, 768; 700: 280 -> 320, 1024: 378 -> 357, 2048: 655 -> 591      50257, 384; 1024: 291 -> 224, 2048: 537 -> 401
-//     50257, 1600; 2048: 1340 -> 1520, 4096: 2975 -> 2817                  16387, 512; 3000: 267 -> 210
-//     30001, 1024; 1500: 396 -> 394                                        13001, 768; 3000: 244 -> 242
-// From 4096 rows on it is the views in any case.  Below, dx of a contraction of less than 16384 has the same bits in every call,
-// which pieces that add into zeros would not give it.
-bool by_row_class(int M, int N, int K) {
-    if (N % 4 == 0 || (long long)M * N < (32 << 20)) return false;
-    return M >= 4096 || (N >= 16384 && M >= 1000 && 3ll * M >= 4ll * K);
-}
 // Whether a caller has to bring room for the copy: wherever it may be made.
 bool wants_scratch(int M, int N) { return N % 32 != 0 && (N % 4 == 0 || M < 4096 || (long long)M * N < (32 << 20)); }
-
-// dx, dW and db (not all of them need be wanted) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut
-// into pieces that add into zeros: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from
-// sums of 524 blocks of 32, 1.3e-5 from sums of 171).  Without dW, whose ranges make up for it, their number decides how even
-// the last round of tiles is (8192 x 50257 x 768: 1009 us from 3 pieces, 1111 from 4).
-BackwardPlan plan_by_row_class(int M, int N, int K, bool want_dx, bool want_dw, int sms) {
-    const int kb = (N + 3 + kBK - 1) / kBK;
-    const int least = (kb + 523) / 524, by_tiles = plan_pieces((M + 3) / 4, K, kb, sms, 32).splits;
-    const int pieces = least > by_tiles ? least : by_tiles;
-    BackwardPlan plan = plan_backward(M, N, K, want_dx, want_dw, sms, 4, pieces);
-    for (int more = 1; want_dx && !want_dw && more <= 2; more++) {
-        const BackwardPlan other = plan_backward(M, N, K, true, false, sms, 4, pieces + more);
-        if (other.ns < plan.ns) plan = other;
-    }
-    return plan;
-}
-int gradients_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, int M,
-                           int N, int K, int *status, cudaStream_t s) {
-    if (dx && plan.dx_pieces > 1) {
-        const int rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s);
-        if (rc != 0) return rc;
-    }
-    return launch_backward_by_row_class(plan, dy, x, w, dx, dw, db, M, N, K, status, s);
-}
 
 // dx[M,K] = g[M,np] . w[N,K]: contraction over N (rows of w past N read as zeros)
 struct InputGradient {
@@ -627,6 +591,61 @@ InputGradient plan_input_gradient(int M, int np, int K, int sms) {
     r.ns = r.split ? split_ns : r.tiles.ns;
     return r;
 }
+// Whether dx as a product of its own, over a copy of dy or over every fourth row, would be whole tiles or two pieces.
+bool few_pieces(int M, int N, int K, int sms) {
+    if (M < 4096) {
+        const InputGradient how = plan_input_gradient(M, (N + 31) / 32 * 32, K, sms);
+        return how.split || how.tiles.splits <= 2;
+    }
+    const int kb = (N + 3 + kBK - 1) / kBK;
+    const Plan cut = plan_pieces((M + 3) / 4, K, kb, sms, 32);
+    return cut.splits <= 2 || cut.ns + (2500 + (int)((long long)M * K * 4 / 5500)) / 4 >= plan_tiles((M + 3) / 4, K, kb, sms).ns;
+}
+// Whether the gradients of a [M, N] result come from views of every fourth row of dy, whose rows are not 16-byte aligned,
+// and not from a copy with padded rows.  The copy is cheap as long as it stays in L2 (128 MB); the views add each tile of dW to
+// memory four times, which costs more than the copy where K is large.  From 4096 rows on it is the views in any case.  Below, dx keeps
+// its bits from call to call where the copy's would (few_pieces), which costs the views a part of what they save: there from 2800 rows
+// on.  Copy -> views, dx and dW | dx alone, in us (M, N, K), with pieces in no fixed order:
+//     1024, 50257, 768: 406 -> 400 | 250 -> 155       3000, 50257, 384: 717 -> 586 | 456 -> 275     1500, 30001, 768: 357 -> 346 | 222 -> 144
+//     1500, 22441, 960: 325 -> 340                    2700, 50257, 1024: 1192 -> 1291 | 755 -> 579
+// and with pieces in turn:
+//     3250, 50257, 768: 1226 -> 1067 | 806 -> 612     4050, 50257, 512: 1140 -> 896 | 723 -> 568    3100, 50257, 1024: 1497 -> 1423 | 898 -> 750
+//     2300, 50257, 768: 835 -> 916 | 535 -> 552       2200, 50257, 1024: 948 -> 1044 | 554 -> 629   2400, 50257, 1600: 1593 -> 1831 | 867 -> 816
+//     4090, 50257, 1600: 2644 -> 2986 | 1521 -> 1489
+bool by_row_class(int M, int N, int K, int sms) {
+    if (N % 4 == 0 || (long long)M * N < (32 << 20)) return false;
+    if (M >= 4096) return true;
+    if (N < 16384 || M < 1000 || 3ll * M < 4ll * K) return false;
+    return few_pieces(M, N, K, sms) ? M >= 2800 && K <= 1024 : K <= 896;
+}
+
+// dx, dW and db (not all of them need be wanted) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut
+// into pieces: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from sums of 524 blocks
+// of 32, 1.3e-5 from sums of 171).  They add into zeros, and three or more of them in no fixed order; where tiles of whole sums keep the
+// SMs as busy, a CTA takes a tile's pieces in turn, and dx has the same bits in every call, with and without dW.  Elsewhere and without
+// dW, whose ranges make up for it, the number of pieces decides how even the last round of tiles is (8192 x 50257 x 768: 1009 us from
+// 3 pieces, 1111 from 4).
+BackwardPlan plan_by_row_class(int M, int N, int K, bool want_dx, bool want_dw, int sms) {
+    const int kb = (N + 3 + kBK - 1) / kBK;
+    const int least = (kb + 523) / 524, by_tiles = plan_pieces((M + 3) / 4, K, kb, sms, 32).splits;
+    const int pieces = least > by_tiles ? least : by_tiles;
+    const bool in_turn = pieces > 2 && few_pieces(M, N, K, sms);
+    BackwardPlan plan = plan_backward(M, N, K, want_dx, want_dw, sms, 4, pieces, in_turn);
+    for (int more = 1; want_dx && !want_dw && pieces > 2 && !in_turn && more <= 2; more++) {
+        const BackwardPlan other = plan_backward(M, N, K, true, false, sms, 4, pieces + more);
+        if (other.ns < plan.ns) plan = other;
+    }
+    return plan;
+}
+int gradients_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, int M,
+                           int N, int K, int *status, cudaStream_t s) {
+    if (dx && plan.dx_pieces > 1 && !plan.dx_in_turn) {
+        const int rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s);
+        if (rc != 0) return rc;
+    }
+    return launch_backward_by_row_class(plan, dy, x, w, dx, dw, db, M, N, K, status, s);
+}
+
 int input_gradient(const InputGradient &how, const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status,
                    cudaStream_t s) {
     if (how.split) return launch_split(g, w, true, N, nullptr, dx, nullptr, M, K, np, how.split, sms, status, s);
@@ -652,7 +671,7 @@ struct Gradients {
 };
 Gradients plan_gradients(int M, int N, int K, int np, bool want_dx, bool want_dw, bool in_parts, int sms) {
     Gradients g = {};
-    g.classes = by_row_class(M, N, K);
+    g.classes = by_row_class(M, N, K, sms);
     if (g.classes) {
         g.together = want_dx && want_dw && !in_parts;
         if (want_dx && !g.together) g.dx = plan_by_row_class(M, N, K, true, false, sms);
@@ -732,8 +751,6 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     if (!dy || !w || (!dx && !dw) || (dw && !x)) return ATTN_ERR_NULL;
     if (M <= 0 || N <= 0 || K <= 0 || (long long)M * N > 0x7fffffffLL || (long long)M * K > 0x7fffffffLL) return ATTN_ERR_SHAPE;
     if (K % 32 != 0) return ATTN_ERR_UNSUPPORTED;
-    const bool classes = by_row_class(M, N, K);
-    const bool padded = N % 32 != 0 && !classes;  // dy's rows cannot be tiles of the copy engine: work on a padded copy
     const int np = (N + 31) / 32 * 32;
     if ((long long)M * np > 0x7fffffffLL) return ATTN_ERR_SHAPE;
     if (wants_scratch(M, N) && !scratch) return ATTN_ERR_NULL;
@@ -749,8 +766,9 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
     const bool in_parts = dw && overlapping(dy, x, w, dx, dw, db, M, N, K);
     const Gradients how = plan_gradients(M, N, K, np, dx != nullptr, dw != nullptr, in_parts, sms);
     float *dx_too = how.together ? dx : nullptr, *db_too = in_parts ? nullptr : db;
+    const bool classes = how.classes;
     const float *g = dy;  // without row classes [M, np] from here on
-    if (padded) {
+    if (N % 32 != 0 && !classes) {  // dy's rows cannot be tiles of the copy engine: work on a padded copy
         rc = (int)attn::launch_after_previous(pad_rows_kernel, dim3(sms * 16), dim3(256), 0, s, static_cast<float *>(scratch), dy, M,
                                               N, np);
         if (rc != 0) return rc;
@@ -787,7 +805,7 @@ int linear_sm100_backward_plan(int M, int N, int K, int want_dx, int want_dw, in
     const BackwardPlan &one = want_dw ? how.dw : how.dx;  // nothing in it for dx alone, not from views
     const int pieces = !want_dx ? 0 : how.classes ? one.dx_pieces : how.alone.split ? 1 : how.alone.tiles.splits;
     const DwLoad load = dw_load(one, M, N, K);
-    const int out[9] = {how.together, how.classes ? 4 : 1, one.teams * one.team, one.team, one.down, pieces, pieces <= 2, load.cta, load.sum};
+    const int out[9] = {how.together, how.classes ? 4 : 1, one.teams * one.team, one.team, one.down, pieces, pieces <= 2 || (how.classes && one.dx_in_turn), load.cta, load.sum};
     for (int i = 0; i < 9; i++) plan[i] = out[i];
     return ATTN_OK;
 }

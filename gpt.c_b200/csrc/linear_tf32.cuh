@@ -120,14 +120,15 @@ inline int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, 
 struct BackwardPlan {
     int tiles_n;                 // column tiles of both results
     int dx_tiles, dx_kb, dw_kb;  // tiles of dx (of all its pieces); contraction blocks of a tile of dx, of dW
-    int classes, dx_pieces;      // views of dy; pieces of the contraction of dx, which are added up in memory where there are several
+    int classes, dx_pieces;      // views of dy; pieces of the contraction of dx, which are added up in memory where there are several,
+    int dx_in_turn;              // 1: by the CTA that takes them in turn
     int team, down;              // CTAs that work on neighbouring tiles of dW, below (1) or beside each other
     int rounds, strips;          // groups of such tiles that a team takes whole; groups that are cut
     int teams, fewer;
     double share_fewer, share;   // how much of dW the first `fewer` teams take, and the others
     int ns;
 };
-BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes = 1, int dx_pieces = 1);
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes = 1, int dx_pieces = 1, bool in_turn = false);
 // Contraction blocks of dW: the most that one CTA takes, and the most that one accumulator sums up.
 struct DwLoad {
     int cta, sum;
@@ -136,7 +137,7 @@ DwLoad dw_load(const BackwardPlan &plan, int M, int N, int K);
 // dy [M, np] with zeros from column N on, w [w_rows, K].
 int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
                     int M, int N, int np, int K, int *status, cudaStream_t s);
-// The same from views of every fourth row of dy [M, N] (plan.classes = 4).  With plan.dx_pieces > 1 dx has to be zero.
+// The same from views of every fourth row of dy [M, N] (plan.classes = 4).  With plan.dx_pieces > 1 not in turn dx has to be zero.
 int launch_backward_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db,
                                  int M, int N, int K, int *status, cudaStream_t s);
 // The kernel for results of few tiles (linear_split_sm100.cu): out[M, cols] = act[M, kc] . w^T + bias, with w [cols, kc],

@@ -58,7 +58,8 @@ size_t linear_sm100_backward_scratch_bytes(int M, int N, int K);
  * boundaries (dy too when N is not a multiple of 4: only its later rows are unaligned then); else
  * ATTN_ERR_ALIGN.
  * dw and db are built from fp32 additions whose order is not fixed (split over M): results can differ
- * in the last bits between runs.
+ * in the last bits between runs.  So can dx where its contraction is cut into three or more pieces that add in memory: with N above
+ * 16000, or an N that is no multiple of 4, and too few tiles for the SMs (plan[6] below is 0 there).
  */
 int linear_sm100_backward(const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, void *scratch,
                           int M, int N, int K, void *stream);

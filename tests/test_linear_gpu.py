@@ -14,7 +14,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 from oracle import ops_oracle as ops  # noqa: E402
-from test_linear_plan import SMS, TEAMS, plan  # noqa: E402
+from test_linear_plan import FIXED, SMS, TEAMS, plan  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -339,6 +339,38 @@ def test_linear_backward_from_every_fourth_row_in_part(pkg, M, N, K):
     within(dx[1:-1].cpu().numpy(), dx_ref, dy, w)
     within(wt.cpu().numpy(), dw_ref, dy.T, x)
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+
+
+@pytest.mark.parametrize("M,N,K", FIXED)
+def test_linear_input_gradient_in_turn(pkg, M, N, K):
+    """From views of dy, in pieces that one CTA adds up: the same bits in every call, with and without dW, on either alignment of dx;
+    nothing outside it is written."""
+    L = pkg.lib()
+    p = plan(pkg, M, N, K)
+    assert p["views"] == 4 and p["dx_pieces"] > 2 and p["dx_fixed_order"]
+    x, w, _, dy = inputs(M, N, K, 83)
+    xt, wt, dyt = (torch.from_numpy(a).cuda() for a in (x, w, dy))
+    need = L.linear_sm100_backward_scratch_bytes(M, N, K)
+    scratch = torch.empty(max(need, 1), dtype=torch.uint8, device="cuda")
+    dw, db = torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda")
+
+    def dx(with_dw, off):
+        buf = torch.full((M * K + 32,), float("nan"), device="cuda")
+        out = buf[16 + off:16 + off + M * K].view(M, K)
+        assert L.linear_sm100_backward(dyt.data_ptr(), xt.data_ptr(), wt.data_ptr(), out.data_ptr(), dw.data_ptr() if with_dw else None,
+                                       db.data_ptr() if with_dw else None, scratch.data_ptr() if need else None, M, N, K,
+                                       torch.cuda.current_stream().cuda_stream) == 0
+        assert bool(buf[:16 + off].isnan().all()) and bool(buf[16 + off + M * K:].isnan().all())
+        return out
+
+    first = dx(True, 0)
+    assert pkg.device_status() == 0
+    dx_ref, dw_ref, db_ref = ops.linear_backward(dy, x, w, np.zeros((N, K), np.float32), np.zeros(N, np.float32))
+    within(first.cpu().numpy(), dx_ref, dy, w)
+    within(dw.cpu().numpy(), dw_ref, dy.T, x)
+    assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+    for with_dw, off in ((True, 0), (False, 0), (True, 4), (False, 4), (False, 0)):
+        assert torch.equal(dx(with_dw, off), first)
 
 
 @pytest.mark.parametrize("M,N,K", [(1411, 4800, 1600), (2305, 2312, 1568), (8001, 760, 3072)])

@@ -34,6 +34,18 @@ def test_views(pkg, M, N, K, views):
     assert plan(pkg, M, N, K)["views"] == views
 
 
+# dx as whole tiles, or the sum of two pieces, by products of its own: the same bits in every call, and with and without dW
+FIXED = [(3838, 16861, 160), (3250, 20003, 384), (24797, 3050, 160), (9695, 20359, 864)]
+
+
+@pytest.mark.parametrize("M,N,K", FIXED + [(16384, 50257, 768), (32768, 50257, 768), (14839, 12887, 896), (2300, 50257, 768),
+                                           (900, 5120, 1280)])
+def test_dx_in_a_fixed_order(pkg, M, N, K):
+    both, alone = plan(pkg, M, N, K), plan(pkg, M, N, K, want_dw=0)
+    assert both["dx_fixed_order"] == alone["dx_fixed_order"] == 1
+    assert both["dx_pieces"] == alone["dx_pieces"]
+
+
 def test_plan_arguments(pkg):
     L, out = pkg.lib(), (ctypes.c_int * 9)()
     assert L.linear_sm100_backward_plan(8, 8, 32, 1, 1, SMS, None) == -1
