@@ -91,7 +91,7 @@ struct Problem {
     int dx_pieces, piece_tiles, piece_kb;  // dx from so many pieces of the contraction, added up in memory; tiles and contraction blocks of a piece
     int dx_sums;               // or from so many in turn, added up by the CTA whose tile it is
     int whole[4], shift[4];    // columns of the views in whole blocks; before the first column of dy
-    int dw_kb;                 // contraction blocks of a tile of dW
+    int dw_kb, dw_most;        // contraction blocks of a tile of dW; the most that go through one accumulator
     int team, down;            // CTAs of a team; their tiles are below (1) or beside each other (0)
     int rounds, strips;        // groups of `team` tiles: whole ones dealt out round robin; the ones after them, which are cut
     int teams, fewer;          // the first `fewer` teams (those with a tile of dx more) take share_fewer of dW, the others share
@@ -177,6 +177,7 @@ struct Items {
                 const int tile = strip * p.team + member;
                 tm = tile / p.tiles_n, t.tn = tile - tm * p.tiles_n;
             }
+            if (to - from > p.dw_most) sums = (to - from + p.dw_most - 1) / p.dw_most;
         }
         t.cls = 0;
         if (p.classes > 1) {  // dW: the classes of a tile follow each other, so that what they add to stays in L2
@@ -516,7 +517,7 @@ Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
     p.dx_pieces = plan.dx_in_turn ? 1 : plan.dx_pieces, p.dx_sums = plan.dx_in_turn ? plan.dx_pieces : 1;
     p.piece_tiles = plan.dx_tiles / p.dx_pieces, p.piece_kb = (plan.dx_kb + p.dx_pieces - 1) / p.dx_pieces;
     p.tiles_n = plan.tiles_n, p.cols = K / 32 / plan.tiles_n, p.wider = K / 32 % plan.tiles_n;
-    p.dx_tiles = plan.dx_tiles, p.dx_kb = plan.dx_kb, p.dw_kb = plan.dw_kb;
+    p.dx_tiles = plan.dx_tiles, p.dx_kb = plan.dx_kb, p.dw_kb = plan.dw_kb, p.dw_most = plan.dw_most;
     p.team = plan.team, p.down = plan.down, p.rounds = plan.rounds, p.strips = plan.strips, p.teams = plan.teams, p.fewer = plan.fewer;
     const double all = plan.fewer * plan.share_fewer + (plan.teams - plan.fewer) * plan.share;
     // rounded up, so that shares of whole tiles begin where tiles do
@@ -546,7 +547,7 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
         const int rows = (M + classes - 1) / classes;  // of a class
         const int rows_m = (rows + kBM - 1) / kBM, rows_n = (N + classes - 1 + kBM - 1) / kBM;
         c.dx_kb = (N + classes - 1 + kBK - 1) / kBK;
-        c.dw_kb = (rows + kBK - 1) / kBK;
+        c.dw_kb = c.dw_most = (rows + kBK - 1) / kBK;
         c.classes = classes;
         const int piece_kb = (c.dx_kb + dx_pieces - 1) / dx_pieces;
         c.dx_pieces = (c.dx_kb + piece_kb - 1) / piece_kb;

@@ -663,6 +663,15 @@ int input_gradient(const InputGradient &how, const float *g, const float *w, flo
     return launch<true, 1>(maps, nullptr, dx, nullptr, p, status, s);
 }
 
+// Contraction blocks of dW that one accumulator sums up at most; it loses precision with them, since the tensor cores truncate.  As many
+// as where every CTA had one piece of the same size, or 160: ranges of 158 blocks in two sums cost 8192 x 3072 x 768 139 -> 142 us, and
+// one sum adds 1.2e-5 to the 7.7e-4 of the operands.  A longer range takes several sums, which add up in memory (18917 x
+// 6368 x 544: four of 148 blocks, 1.0e-5 and 332 us, where one of 592 gives 3.2e-5 and 320).
+int longest_dw_sum(int N, int K, int kb, int sms) {
+    const int pieces = plan_pieces(N, K, kb, sms, 1).splits, even = (kb + pieces - 1) / pieces;
+    return even > 160 ? even : 160;
+}
+
 // How the backward makes dx and dW; np: columns of a padded dy.  `in_parts`: one product after the other.
 struct Gradients {
     bool classes, together;  // views of dy; dx and dW in one launch
@@ -681,11 +690,13 @@ Gradients plan_gradients(int M, int N, int K, int np, bool want_dx, bool want_dw
     if (want_dx) g.alone = plan_input_gradient(M, np, K, sms);
     if (!want_dw) return g;
     g.dw = plan_backward(M, N, K, false, true, sms);
+    const int most = longest_dw_sum(N, K, g.dw.dw_kb, sms);
+    g.dw.dw_most = most;
     // dx has the same bits with and without dW: one launch only where dx alone would be whole tiles too
     if (!want_dx || in_parts || g.alone.split || g.alone.tiles.splits > 1) return g;
     const BackwardPlan both = plan_backward(M, N, K, true, true, sms);
     g.together = both.ns < g.alone.ns + g.dw.ns;
-    if (g.together) g.dw = both;
+    if (g.together) g.dw = both, g.dw.dw_most = most;
     return g;
 }
 

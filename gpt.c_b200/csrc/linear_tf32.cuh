@@ -125,6 +125,7 @@ struct BackwardPlan {
     int team, down;              // CTAs that work on neighbouring tiles of dW, below (1) or beside each other
     int rounds, strips;          // groups of such tiles that a team takes whole; groups that are cut
     int teams, fewer;
+    int dw_most;                 // contraction blocks of dW that go through one accumulator
     double share_fewer, share;   // how much of dW the first `fewer` teams take, and the others
     int ns;
 };

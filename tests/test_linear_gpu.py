@@ -14,7 +14,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 from oracle import ops_oracle as ops  # noqa: E402
-from test_linear_plan import FIXED, SMS, TEAMS, plan  # noqa: E402
+from test_linear_plan import FIXED, LONG, SMS, TEAMS, plan  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -339,6 +339,14 @@ def test_linear_backward_from_every_fourth_row_in_part(pkg, M, N, K):
     within(dx[1:-1].cpu().numpy(), dx_ref, dy, w)
     within(wt.cpu().numpy(), dw_ref, dy.T, x)
     assert np.abs(db.cpu().numpy() - db_ref).max() <= 1e-5 * np.sqrt(M) * 8
+
+
+@pytest.mark.parametrize("M,N,K", LONG)
+def test_linear_weight_gradient_in_several_sums(pkg, M, N, K):
+    assert torch.cuda.get_device_properties(0).multi_processor_count == SMS
+    p = plan(pkg, M, N, K)
+    assert p["dw_sum"] <= 160 < p["dw_of_a_cta"]
+    test_linear_backward_in_one_launch(pkg, M, N, K, True)
 
 
 @pytest.mark.parametrize("M,N,K", FIXED)

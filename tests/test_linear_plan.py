@@ -46,6 +46,17 @@ def test_dx_in_a_fixed_order(pkg, M, N, K):
     assert both["dx_pieces"] == alone["dx_pieces"]
 
 
+# a CTA takes longer ranges of dW's contraction than one accumulator sums up
+LONG = [(40998, 3796, 32), (11087, 2470, 672)]
+
+
+@pytest.mark.parametrize("M,N,K", LONG + [(18917, 6368, 544)])
+def test_sums_of_dw_stay_short(pkg, M, N, K):
+    """At most 160 contraction blocks of 32 rows, where pieces of one size for all SMs would be no longer."""
+    assert plan(pkg, M, N, K)["dw_of_a_cta"] > 160
+    assert max(plan(pkg, M, N, K, want_dx=want_dx)["dw_sum"] for want_dx in (0, 1)) <= 160
+
+
 def test_plan_arguments(pkg):
     L, out = pkg.lib(), (ctypes.c_int * 9)()
     assert L.linear_sm100_backward_plan(8, 8, 32, 1, 1, SMS, None) == -1
