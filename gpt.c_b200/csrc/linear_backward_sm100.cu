@@ -523,8 +523,8 @@ Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
     // rounded up, so that shares of whole tiles begin where tiles do
     p.share_fewer = (uint32_t)ceil(plan.share_fewer / all * 4294967296.0);
     p.share = (uint32_t)fmin(ceil(plan.share / all * 4294967296.0), 4294967295.0);
-    // a few tiles of few blocks are cut anywhere, many are not
-    p.snap = p.dw_kb >= 16 ? 4 : p.strips >= p.teams ? (p.dw_kb < 8 ? p.dw_kb : 2) : 0;
+    // pieces of the same size stay as they are; a few tiles of few blocks are cut anywhere, many are not
+    p.snap = plan.even && p.strips < p.teams ? 0 : p.dw_kb >= 16 ? 4 : p.strips >= p.teams ? (p.dw_kb < 8 ? p.dw_kb : 2) : 0;
     p.uncut = p.dx_tiles == 0 && p.classes == 1 && p.team == 1 && p.snap == p.dw_kb;
     p.stage_bytes = kATileBytes + (p.cols + (p.wider > 0)) * 4096;
     p.stages = kRingBytes / p.stage_bytes < kMostStages ? kRingBytes / p.stage_bytes : kMostStages;
@@ -589,7 +589,7 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
             const int busy = pieces * dw_tiles;
             const double whole = (c.dw_kb + pieces - 1) / pieces * block_ns(cols, busy, sms) + te + adding_ns(busy, cols);
             if (whole <= time) {
-                c.team = 1, c.down = 0, c.rounds = 0, c.strips = dw_tiles, c.teams = busy, c.share = 1;
+                c.team = 1, c.down = 0, c.rounds = 0, c.strips = dw_tiles, c.teams = busy, c.share = 1, c.even = 1;
                 time = whole;
             }
             pieces = pieces > 1 ? as_deep(pieces - 1) : 0;

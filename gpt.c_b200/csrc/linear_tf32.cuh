@@ -124,7 +124,7 @@ struct BackwardPlan {
     int dx_in_turn;              // 1: by the CTA that takes them in turn
     int team, down;              // CTAs that work on neighbouring tiles of dW, below (1) or beside each other
     int rounds, strips;          // groups of such tiles that a team takes whole; groups that are cut
-    int teams, fewer;
+    int teams, fewer, even;      // even: whole pieces of the same size, one per team
     int dw_most;                 // contraction blocks of dW that go through one accumulator
     double share_fewer, share;   // how much of dW the first `fewer` teams take, and the others
     int ns;

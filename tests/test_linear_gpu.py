@@ -14,7 +14,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 from oracle import ops_oracle as ops  # noqa: E402
-from test_linear_plan import FIXED, LONG, SMS, TEAMS, plan  # noqa: E402
+from test_linear_plan import EVEN, FIXED, LONG, SMS, TEAMS, plan  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -346,6 +346,12 @@ def test_linear_weight_gradient_in_several_sums(pkg, M, N, K):
     assert torch.cuda.get_device_properties(0).multi_processor_count == SMS
     p = plan(pkg, M, N, K)
     assert p["dw_sum"] <= 160 < p["dw_of_a_cta"]
+    test_linear_backward_in_one_launch(pkg, M, N, K, True)
+
+
+@pytest.mark.parametrize("M,N,K,blocks", EVEN)
+def test_linear_weight_gradient_in_pieces_of_one_size(pkg, M, N, K, blocks):
+    assert plan(pkg, M, N, K)["dw_of_a_cta"] == blocks
     test_linear_backward_in_one_launch(pkg, M, N, K, True)
 
 

@@ -57,6 +57,16 @@ def test_sums_of_dw_stay_short(pkg, M, N, K):
     assert max(plan(pkg, M, N, K, want_dx=want_dx)["dw_sum"] for want_dx in (0, 1)) <= 160
 
 
+# few tiles, so that every CTA has one piece of dW of the same size, in contraction blocks
+EVEN = [(640, 33, 32, 1), (506, 384, 384, 2), (700, 512, 512, 4), (2187, 44, 768, 4), (1205, 160, 736, 4), (512, 768, 768, 4)]
+
+
+@pytest.mark.parametrize("M,N,K,blocks", EVEN)
+def test_pieces_of_one_size(pkg, M, N, K, blocks):
+    for want_dx in (0, 1):
+        assert plan(pkg, M, N, K, want_dx=want_dx)["dw_of_a_cta"] == blocks
+
+
 def test_plan_arguments(pkg):
     L, out = pkg.lib(), (ctypes.c_int * 9)()
     assert L.linear_sm100_backward_plan(8, 8, 32, 1, 1, SMS, None) == -1
