@@ -338,6 +338,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) xent_forward_rows_kernel(const
 // Shorter rows gain nothing, several of whose blocks share an SM (8192 rows of 16384: 197 us there, 206 here, 24576: 271, 279,
 // 32000: 367, 351, 50257: 628, 544; 1 row of 50257: 9.8, 9.9, 37 rows: 12.1, 10.5).
 bool row_fits(int C) { return C >= 30000 && C <= kSlot * kSlots; }
+// Nor do more rows than SMs, up to two for each, which the kernel above takes all at once and this one in two turns, unless their
+// addresses modulo 16 differ (214 rows of 30000: 13.6 us there, 15.6 here, 34000: 16.1, 17.1, 36001: 18.3, 17.7, 50257: 25.1, 24.0).
+bool in_two_turns(int rows, int C) { return C % 4 == 0 && rows > attn::sm_count() && rows <= 2 * attn::sm_count(); }
 
 // `loaded` rows are fetched: all of them, or in the test of what happens when one never arrives fewer.
 int launch_rows(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, cudaStream_t s, int loaded,
@@ -367,7 +370,8 @@ extern "C" {
 int xent_sm100_forward(const float *logits, const float *targets, float *logsm, float *loss, int rows, int C, void *stream) {
     if (!logits || !targets || !logsm || !loss) return ATTN_ERR_NULL;
     if (rows <= 0 || C <= 0) return ATTN_ERR_SHAPE;
-    if (xent::row_fits(C)) return xent::launch_rows(logits, targets, logsm, loss, rows, C, static_cast<cudaStream_t>(stream), rows);
+    if (xent::row_fits(C) && !xent::in_two_turns(rows, C))
+        return xent::launch_rows(logits, targets, logsm, loss, rows, C, static_cast<cudaStream_t>(stream), rows);
     return (int)attn::launch_after_previous(xent::xent_forward_kernel, dim3(rows), dim3(xent::kThreads), 0,
                                             static_cast<cudaStream_t>(stream), logits, targets, logsm, loss, rows, C);
 }

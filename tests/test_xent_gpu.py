@@ -122,6 +122,15 @@ def test_cross_entropy_rows_in_shared_memory(pkg, rows, C, offsets):
     assert pkg.device_status() == 0
 
 
+@pytest.mark.parametrize("rows,C,offsets", [
+    (148, 53248, (0, 0)), (149, 53248, (0, 0)), (296, 30000, (0, 0)), (297, 53248, (0, 0)),  # one row per SM, up to two, more
+    (299, 32768, (2, 1)),
+])
+def test_cross_entropy_rows_on_even_addresses(pkg, rows, C, offsets):
+    """Either side of where up to two rows per SM, all on the same address modulo 16, are taken at once."""
+    test_cross_entropy_rows_in_shared_memory(pkg, rows, C, offsets)
+
+
 def test_cross_entropy_keeps_rows_apart(pkg):
     """A NaN or an infinity stays in its own row; a row of -inf has no probabilities."""
     L = pkg.lib()
