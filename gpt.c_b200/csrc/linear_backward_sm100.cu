@@ -88,8 +88,9 @@ struct Problem {
     int tiles_n, cols, wider;  // column tiles; blocks of 32 columns in each; the first `wider` have one more
     int dx_tiles, dx_kb;       // tiles of dx, handed out round robin; contraction blocks of one
     int classes;               // 4: views of every fourth row of dy
-    int dx_pieces, piece_tiles, piece_kb;  // dx from so many pieces of the contraction, added up in memory; tiles and contraction blocks of a piece
+    int dx_pieces, piece_tiles, piece_kb;  // dx from so many pieces of the contraction; tiles and contraction blocks of a piece
     int dx_sums;               // or from so many in turn, added up by the CTA whose tile it is
+    size_t dx_apart;           // from one piece of dx to the next, which are not added up here (0: they are)
     int whole[4], shift[4];    // columns of the views in whole blocks; before the first column of dy
     int dw_kb, dw_most;        // contraction blocks of a tile of dW; the most that go through one accumulator
     int team, down;            // CTAs of a team; their tiles are below (1) or beside each other (0)
@@ -440,15 +441,16 @@ linear_backward_kernel(const __grid_constant__ Maps<kClasses> maps, float *__res
                 tmem_ld32(tmem + lane_addr + (uint32_t)acc * kBN + 32 * c, r);
                 tmem_wait_ld();
                 if (c + 1 == c1) read_out();
-                if (!t.dw && (!kClasses || p.dx_pieces == 1)) {
+                if (!t.dw && (!kClasses || p.dx_pieces == 1 || p.dx_apart)) {
                     const int odd = lane & 1, col = col0 + 16 * odd;
+                    float *piece = kClasses ? dx + t.kb0 / p.piece_kb * p.dx_apart : dx;
                     exchange_halves(odd, r);
 #pragma unroll
                     for (int o = 0; o < 2; o++) {
                         const int row = row0 + lane - odd + o;
                         if (row * p.classes + t.cls >= p.M) continue;
-                        float *to = dx + ((size_t)row * p.classes + t.cls) * p.K + col;
-                        if (kClasses && t.kb0 > 0) add_words<4>(to, p.K - col, r + 16 * o);  // what this thread wrote for the range before
+                        float *to = piece + ((size_t)row * p.classes + t.cls) * p.K + col;
+                        if (kClasses && p.dx_sums > 1 && t.kb0 > 0) add_words<4>(to, p.K - col, r + 16 * o);  // what this thread wrote for the range before
                         store_words<4>(to, p.K - col, p.wide, r + 16 * o);
                     }
                     continue;
@@ -514,7 +516,8 @@ Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
     Problem p = {};
     p.M = M, p.N = N, p.K = K;
     p.classes = plan.classes;
-    p.dx_pieces = plan.dx_in_turn ? 1 : plan.dx_pieces, p.dx_sums = plan.dx_in_turn ? plan.dx_pieces : 1;
+    p.dx_pieces = plan.dx_how == kDxInTurn ? 1 : plan.dx_pieces, p.dx_sums = plan.dx_how == kDxInTurn ? plan.dx_pieces : 1;
+    p.dx_apart = plan.dx_how == kDxApart ? (size_t)M * K : 0;
     p.piece_tiles = plan.dx_tiles / p.dx_pieces, p.piece_kb = (plan.dx_kb + p.dx_pieces - 1) / p.dx_pieces;
     p.tiles_n = plan.tiles_n, p.cols = K / 32 / plan.tiles_n, p.wider = K / 32 % plan.tiles_n;
     p.dx_tiles = plan.dx_tiles, p.dx_kb = plan.dx_kb, p.dw_kb = plan.dw_kb, p.dw_most = plan.dw_most;
@@ -534,7 +537,7 @@ Problem make_problem(const BackwardPlan &plan, int M, int N, int K) {
 }  // namespace
 
 // The split of the work and the time in nanoseconds it is expected to take: see linear_tf32.cuh.
-BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes, int dx_pieces, bool in_turn) {
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes, int dx_pieces, DxPieces how) {
     BackwardPlan best = {};
     const int blocks = K / 32;
     for (int width = 8; width >= 4; width--) {
@@ -551,8 +554,8 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
         c.classes = classes;
         const int piece_kb = (c.dx_kb + dx_pieces - 1) / dx_pieces;
         c.dx_pieces = (c.dx_kb + piece_kb - 1) / piece_kb;
-        c.dx_in_turn = in_turn;
-        c.dx_tiles = want_dx ? classes * rows_m * tiles_n * (in_turn ? 1 : c.dx_pieces) : 0;
+        c.dx_how = how;
+        c.dx_tiles = want_dx ? classes * rows_m * tiles_n * (how == kDxInTurn ? 1 : c.dx_pieces) : 0;
         const int dw_tiles = want_dw ? classes * rows_n * tiles_n : 0;
         // Where dy and x don't stay in L2 together, a team shares the larger of them, if that keeps most SMs busy.
         c.down = classes == 1 && N < K, c.team = c.down ? rows_n : tiles_n;
@@ -561,7 +564,7 @@ BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int 
         c.teams = sms / c.team;
         if (!want_dx && (long long)c.strips * c.dw_kb < c.teams) c.teams = c.strips * c.dw_kb;
         const int ctas = c.teams * c.team;
-        const double dx_ns = (piece_kb * tb + te) * (in_turn ? c.dx_pieces : 1);
+        const double dx_ns = (piece_kb * tb + te) * (how == kDxInTurn ? c.dx_pieces : 1);
         // every CTA has about one piece of a tile more than its share of whole ones
         const double even = (c.dx_tiles * dx_ns + dw_tiles * (c.dw_kb * tb + te)) / ctas + te;
         const int most = (c.dx_tiles + ctas - 1) / ctas;
@@ -670,7 +673,7 @@ int launch_backward_by_row_class(const BackwardPlan &plan, const float *dy, cons
         }
         if (!dx) continue;
         if ((rc = map_k_major(&maps.dy_k[j], c.dy, c.rows, N + c.shift, 128, pitch)) != 0) return rc;
-        if (p.dx_pieces > 1 && (rc = map_out_f32(&maps.dx[j], dx + (size_t)j * K, c.rows, K, 4 * (size_t)K)) != 0) return rc;
+        if (p.dx_pieces > 1 && !p.dx_apart && (rc = map_out_f32(&maps.dx[j], dx + (size_t)j * K, c.rows, K, 4 * (size_t)K)) != 0) return rc;
     }
     for (int i = 0; dx && i <= (p.wider > 0); i++)
         if ((rc = map_mn_major_blocks(&maps.w[i], w, N, K, p.cols + i)) != 0) return rc;

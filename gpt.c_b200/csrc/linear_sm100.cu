@@ -368,6 +368,23 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict_
     }
 }
 
+// A matrix as the sum of its pieces, `words` 16-byte words each, in their order: they come from L2, four at a time.
+__global__ void __launch_bounds__(256) sum_pieces_kernel(float4 *__restrict__ out, const float4 *__restrict__ parts, size_t words, int pieces) {
+    tc05::pdl_launch_dependents();
+    tc05::pdl_wait();
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (size_t)gridDim.x * 256) {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int p0 = 0; p0 < pieces; p0 += 4) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = p0 + u < pieces ? __ldcs(parts + (p0 + u) * words + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; u++) sum = make_float4(sum.x + v[u].x, sum.y + v[u].y, sum.z + v[u].z, sum.w + v[u].w);
+        }
+        out[i] = sum;
+    }
+}
+
 // dst[M, Np] = src[M, N] with zero columns N..Np-1: a copy of dy whose rows start on 16-byte boundaries, for
 // outputs of layers whose feature count is not a multiple of 4 (the vocabulary projection).
 __global__ void __launch_bounds__(256) pad_rows_kernel(float *__restrict__ dst, const float *__restrict__ src, int M, int N,
@@ -591,7 +608,7 @@ InputGradient plan_input_gradient(int M, int np, int K, int sms) {
     r.ns = r.split ? split_ns : r.tiles.ns;
     return r;
 }
-// Whether dx as a product of its own, over a copy of dy or over every fourth row, would be whole tiles or two pieces.
+// Whether dx as a product of its own, below 4096 rows over a copy of dy, else over every fourth row, would be whole tiles or two pieces.
 bool few_pieces(int M, int N, int K, int sms) {
     if (M < 4096) {
         const InputGradient how = plan_input_gradient(M, (N + 31) / 32 * 32, K, sms);
@@ -603,47 +620,50 @@ bool few_pieces(int M, int N, int K, int sms) {
 }
 // Whether the gradients of a [M, N] result come from views of every fourth row of dy, whose rows are not 16-byte aligned,
 // and not from a copy with padded rows.  The copy is cheap as long as it stays in L2 (128 MB); the views add each tile of dW to
-// memory four times, which costs more than the copy where K is large.  From 4096 rows on it is the views in any case.  Below, dx keeps
-// its bits from call to call where the copy's would (few_pieces), which costs the views a part of what they save: there from 2800 rows
-// on.  Copy -> views, dx and dW | dx alone, in us (M, N, K), with pieces in no fixed order:
-//     1024, 50257, 768: 406 -> 400 | 250 -> 155       3000, 50257, 384: 717 -> 586 | 456 -> 275     1500, 30001, 768: 357 -> 346 | 222 -> 144
-//     1500, 22441, 960: 325 -> 340                    2700, 50257, 1024: 1192 -> 1291 | 755 -> 579
-// and with pieces in turn:
-//     3250, 50257, 768: 1226 -> 1067 | 806 -> 612     4050, 50257, 512: 1140 -> 896 | 723 -> 568    3100, 50257, 1024: 1497 -> 1423 | 898 -> 750
-//     2300, 50257, 768: 835 -> 916 | 535 -> 552       2200, 50257, 1024: 948 -> 1044 | 554 -> 629   2400, 50257, 1600: 1593 -> 1831 | 867 -> 816
-//     4090, 50257, 1600: 2644 -> 2986 | 1521 -> 1489
-bool by_row_class(int M, int N, int K, int sms) {
+// memory four times, which costs more than the copy where K is large.  From 4096 rows on it is the views in any case.  Copy -> views,
+// dx and dW | dx alone, in us (M, N, K):
+//     1024, 50257, 768: 409 -> 402 | 251 -> 157       3000, 50257, 384: 712 -> 577 | 447 -> 269     1500, 30001, 768: 356 -> 338 | 222 -> 140
+//     2300, 50257, 768: 857 -> 795 | 530 -> 351       3500, 50257, 384: 863 -> 662 | 546 -> 328     3100, 50257, 1024: 1482 -> 1401 | 892 -> 740
+//     1800, 30001, 896: 497 -> 528 | 292 -> 250       1500, 22441, 960: 325 -> 340                  2700, 50257, 1024: 1192 -> 1291 | 755 -> 579
+//     2400, 50257, 1600: 1644 -> 1807 | 840 -> 827    4090, 50257, 1600: 2481 -> 2986 | 1521 -> 1489
+bool by_row_class(int M, int N, int K) {
     if (N % 4 == 0 || (long long)M * N < (32 << 20)) return false;
-    if (M >= 4096) return true;
-    if (N < 16384 || M < 1000 || 3ll * M < 4ll * K) return false;
-    return few_pieces(M, N, K, sms) ? M >= 2800 && K <= 1024 : K <= 896;
+    return M >= 4096 || (N >= 16384 && M >= 1000 && 3ll * M >= 4ll * K && K <= (M < 2800 ? 768 : 1024));
 }
 
 // dx, dW and db (not all of them need be wanted) straight from a dy whose rows are not 16-byte aligned.  The contraction of dx is cut
 // into pieces: long sums on the tensor cores, which truncate, lose precision (dx of N = 50257 is 3.9e-5 off from sums of 524 blocks
-// of 32, 1.3e-5 from sums of 171).  They add into zeros, and three or more of them in no fixed order; where tiles of whole sums keep the
-// SMs as busy, a CTA takes a tile's pieces in turn, and dx has the same bits in every call, with and without dW.  Elsewhere and without
-// dW, whose ranges make up for it, the number of pieces decides how even the last round of tiles is (8192 x 50257 x 768: 1009 us from
-// 3 pieces, 1111 from 4).
+// of 32, 1.3e-5 from sums of 171).  They add into zeros, three or more of them in no fixed order.  But dx has the same bits in every
+// call, with and without dW, where tiles of whole sums would keep the SMs as busy: below 4096 rows the pieces are kept apart, where
+// the padded copy would be, and added up behind the launch (2300 x 50257 x 768 774 -> 795 us, elsewhere more: 1500 x 30001 x 768 338 ->
+// 361); above, where there is no such room, a CTA takes a tile's pieces in turn (16384 x 50257 x 768 4609 -> 4583, dx alone 2118 -> 2374).
+// In no order and without dW, whose ranges make up for it, their number decides how even the last round of tiles is (8192 x 50257 x 768:
+// 1009 us from 3 pieces, 1111 from 4).
 BackwardPlan plan_by_row_class(int M, int N, int K, bool want_dx, bool want_dw, int sms) {
     const int kb = (N + 3 + kBK - 1) / kBK;
     const int least = (kb + 523) / 524, by_tiles = plan_pieces((M + 3) / 4, K, kb, sms, 32).splits;
-    const int pieces = least > by_tiles ? least : by_tiles;
-    const bool in_turn = pieces > 2 && few_pieces(M, N, K, sms);
-    BackwardPlan plan = plan_backward(M, N, K, want_dx, want_dw, sms, 4, pieces, in_turn);
-    for (int more = 1; want_dx && !want_dw && pieces > 2 && !in_turn && more <= 2; more++) {
+    int pieces = least > by_tiles ? least : by_tiles;
+    const DxPieces how = pieces <= 2 || !few_pieces(M, N, K, sms) ? kDxAdded : M < 4096 ? kDxApart : kDxInTurn;
+    if (how == kDxApart && pieces > (N + 31) / 32 * 32 / K) pieces = (N + 31) / 32 * 32 / K;  // as many as there is room for
+    BackwardPlan plan = plan_backward(M, N, K, want_dx, want_dw, sms, 4, pieces, how);
+    for (int more = 1; want_dx && !want_dw && pieces > 2 && how == kDxAdded && more <= 2; more++) {
         const BackwardPlan other = plan_backward(M, N, K, true, false, sms, 4, pieces + more);
         if (other.ns < plan.ns) plan = other;
     }
     return plan;
 }
-int gradients_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db, int M,
-                           int N, int K, int *status, cudaStream_t s) {
-    if (dx && plan.dx_pieces > 1 && !plan.dx_in_turn) {
+int gradients_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db,
+                           void *scratch, int M, int N, int K, int sms, int *status, cudaStream_t s) {
+    const bool apart = dx && plan.dx_how == kDxApart;
+    float *parts = static_cast<float *>(scratch);
+    if (dx && plan.dx_how == kDxAdded && plan.dx_pieces > 1) {
         const int rc = tensor_sm100_fill(dx, (size_t)M * K, 0.f, s);
         if (rc != 0) return rc;
     }
-    return launch_backward_by_row_class(plan, dy, x, w, dx, dw, db, M, N, K, status, s);
+    const int rc = launch_backward_by_row_class(plan, dy, x, w, apart ? parts : dx, dw, db, M, N, K, status, s);
+    if (rc != 0 || !apart) return rc;
+    return (int)attn::launch_after_previous(sum_pieces_kernel, dim3(sms * 8), dim3(256), 0, s, reinterpret_cast<float4 *>(dx),
+                                            reinterpret_cast<const float4 *>(parts), (size_t)M * K / 4, plan.dx_pieces);
 }
 
 int input_gradient(const InputGradient &how, const float *g, const float *w, float *dx, int M, int N, int np, int K, int sms, int *status,
@@ -680,7 +700,7 @@ struct Gradients {
 };
 Gradients plan_gradients(int M, int N, int K, int np, bool want_dx, bool want_dw, bool in_parts, int sms) {
     Gradients g = {};
-    g.classes = by_row_class(M, N, K, sms);
+    g.classes = by_row_class(M, N, K);
     if (g.classes) {
         g.together = want_dx && want_dw && !in_parts;
         if (want_dx && !g.together) g.dx = plan_by_row_class(M, N, K, true, false, sms);
@@ -786,12 +806,12 @@ int linear_sm100_backward(const float *dy, const float *x, const float *w, float
         g = static_cast<const float *>(scratch);
     }
     if (dx && !how.together) {
-        rc = classes ? gradients_by_row_class(how.dx, dy, x, w, dx, nullptr, nullptr, M, N, K, status, s)
+        rc = classes ? gradients_by_row_class(how.dx, dy, x, w, dx, nullptr, nullptr, scratch, M, N, K, sms, status, s)
                      : input_gradient(how.alone, g, w, dx, M, N, np, K, sms, status, s);
         if (rc != 0) return rc;
     }
     if (dw) {
-        rc = classes ? gradients_by_row_class(how.dw, dy, x, w, dx_too, dw, db_too, M, N, K, status, s)
+        rc = classes ? gradients_by_row_class(how.dw, dy, x, w, dx_too, dw, db_too, scratch, M, N, K, sms, status, s)
                      : launch_backward(how.dw, g, x, w, N, dx_too, dw, db_too, M, N, np, K, status, s);
         if (rc != 0 || !in_parts) return rc;
     }
@@ -816,7 +836,8 @@ int linear_sm100_backward_plan(int M, int N, int K, int want_dx, int want_dw, in
     const BackwardPlan &one = want_dw ? how.dw : how.dx;  // nothing in it for dx alone, not from views
     const int pieces = !want_dx ? 0 : how.classes ? one.dx_pieces : how.alone.split ? 1 : how.alone.tiles.splits;
     const DwLoad load = dw_load(one, M, N, K);
-    const int out[9] = {how.together, how.classes ? 4 : 1, one.teams * one.team, one.team, one.down, pieces, pieces <= 2 || (how.classes && one.dx_in_turn), load.cta, load.sum};
+    const int out[9] = {how.together, how.classes ? 4 : 1, one.teams * one.team, one.team, one.down, pieces,
+                        pieces <= 2 || (how.classes && one.dx_how != kDxAdded), load.cta, load.sum};
     for (int i = 0; i < 9; i++) plan[i] = out[i];
     return ATTN_OK;
 }

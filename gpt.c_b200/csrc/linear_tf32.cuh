@@ -115,13 +115,16 @@ inline int map_out_f32(CUtensorMap *map, const float *base, int rows, int cols, 
     const cuuint32_t box[3] = {32, 32, 1};
     return attn::encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box);
 }
+// Pieces of the contraction of dx: added to zeros in memory, in no fixed order; added up by one CTA, which takes them in turn; left
+// apart, one matrix behind the other.
+enum DxPieces : int { kDxAdded, kDxInTurn, kDxApart };
 // All of a backward in one launch (linear_backward_sm100.cu), or dW and db alone (dx NULL), or dx alone (dw and db NULL).  What is cut how, and the time in
 // nanoseconds it is expected to take.
 struct BackwardPlan {
     int tiles_n;                 // column tiles of both results
     int dx_tiles, dx_kb, dw_kb;  // tiles of dx (of all its pieces); contraction blocks of a tile of dx, of dW
-    int classes, dx_pieces;      // views of dy; pieces of the contraction of dx, which are added up in memory where there are several,
-    int dx_in_turn;              // 1: by the CTA that takes them in turn
+    int classes, dx_pieces;      // views of dy; pieces of the contraction of dx,
+    DxPieces dx_how;             // and what becomes of them
     int team, down;              // CTAs that work on neighbouring tiles of dW, below (1) or beside each other
     int rounds, strips;          // groups of such tiles that a team takes whole; groups that are cut
     int teams, fewer, even;      // even: whole pieces of the same size, one per team
@@ -129,7 +132,7 @@ struct BackwardPlan {
     double share_fewer, share;   // how much of dW the first `fewer` teams take, and the others
     int ns;
 };
-BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes = 1, int dx_pieces = 1, bool in_turn = false);
+BackwardPlan plan_backward(int M, int N, int K, bool want_dx, bool want_dw, int sms, int classes = 1, int dx_pieces = 1, DxPieces how = kDxAdded);
 // Contraction blocks of dW: the most that one CTA takes, and the most that one accumulator sums up.
 struct DwLoad {
     int cta, sum;
@@ -138,7 +141,8 @@ DwLoad dw_load(const BackwardPlan &plan, int M, int N, int K);
 // dy [M, np] with zeros from column N on, w [w_rows, K].
 int launch_backward(const BackwardPlan &plan, const float *dy, const float *x, const float *w, int w_rows, float *dx, float *dw, float *db,
                     int M, int N, int np, int K, int *status, cudaStream_t s);
-// The same from views of every fourth row of dy [M, N] (plan.classes = 4).  With plan.dx_pieces > 1 not in turn dx has to be zero.
+// The same from views of every fourth row of dy [M, N] (plan.classes = 4).  With several pieces that are added dx has to be zero, with pieces
+// apart it has room for them all.
 int launch_backward_by_row_class(const BackwardPlan &plan, const float *dy, const float *x, const float *w, float *dx, float *dw, float *db,
                                  int M, int N, int K, int *status, cudaStream_t s);
 // The kernel for results of few tiles (linear_split_sm100.cu): out[M, cols] = act[M, kc] . w^T + bias, with w [cols, kc],

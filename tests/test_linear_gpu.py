@@ -357,8 +357,8 @@ def test_linear_weight_gradient_in_pieces_of_one_size(pkg, M, N, K, blocks):
 
 @pytest.mark.parametrize("M,N,K", FIXED)
 def test_linear_input_gradient_in_turn(pkg, M, N, K):
-    """From views of dy, in pieces that one CTA adds up: the same bits in every call, with and without dW, on either alignment of dx;
-    nothing outside it is written."""
+    """From views of dy, in pieces that one CTA takes in turn, or below 4096 rows in pieces apart that are added up behind the launch:
+    the same bits in every call, with and without dW, on either alignment of dx; nothing outside it is written."""
     L = pkg.lib()
     p = plan(pkg, M, N, K)
     assert p["views"] == 4 and p["dx_pieces"] > 2 and p["dx_fixed_order"]
