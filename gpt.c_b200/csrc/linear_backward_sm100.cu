@@ -9,7 +9,7 @@
 // contraction may be cut anywhere: every CTA first takes its tiles of dx, then as much of dW as makes all CTAs end together.
 // dy is read from shared memory a second time for db, in fp32, by two warps that have nothing else to do.  Before, three
 // launches, now (M, N, K in us, with db): 8192, 3072, 768 138 -> 124; 8192, 2304, 768 115 -> 95; 8192, 768, 768 51 -> 39;
-// 1500, 6400, 1600 128 -> 106; 1500, 1600, 1600 45 -> 34; 1705, 129, 4288 32 -> 25; 12, 288, 128 10.3 -> 8.4.
+// 1500, 6400, 1600 128 -> 106; 1500, 1600, 1600 45 -> 34; 1705, 129, 4288 32 -> 25.
 // What bounds it: shared memory, which takes a block's 48 KB in and hands them to the tensor cores once (768 cycles at 128
 // bytes each, 512 of products), and the power cap: 8192 x 3072 x 768 runs at 630 TFLOP/s.
 //

@@ -461,8 +461,9 @@ Problem make_problem(int M, int N, int K, int rows, int bn, int splits) {
 
 // Tile shape and number of pieces of the contraction for a [M, N] result of kb contraction blocks, chosen by expected
 // time: a fixed part, and for every round over the SMs a charge and kb blocks at the slower of what one CTA takes when
-// it is alone (`block`) and what L2 needs to feed all CTAs of the round.  The constants are a fit to the kernel's times
-// on 224 shapes of 100 to 8192 rows and 512 to 6400 columns (mean error 5 %).  Wide tiles read the least per flop and
+// it is alone (`block`) and what L2 needs to feed all CTAs of the round.  The constants of 128 rows were fitted to the kernel's times
+// on 224 shapes of 100 to 8192 rows and 512 to 6400 columns (mean error 5 %) before results left in pieces of 64 bytes of a row, which
+// made the rounds of short contractions shorter; those of 256 rows come from the shapes below.  Wide tiles read the least per flop and
 // win when there are many, narrow ones leave a smaller last round.
 struct Plan {
     int rows, bn, splits;
